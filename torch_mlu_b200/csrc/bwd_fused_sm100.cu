@@ -303,14 +303,14 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     reg_decrease<kRegsUtil>();
     if (warp == 8) {
       // ------------------------------------------------------------------ TMA producer (rest of the ring)
-      if (lane == 0 && n_items > 0) {
+      if (n_items > 0 && elect_one()) {
         for (int idx = kPreloaded; idx < 2 * n_items; ++idx)
           if (!load_tile(idx)) break;
         drain_after_abort(abort_flag);
       }
     } else if (warp == 9) {
       // ------------------------------------------------------------------ score GEMMs: S = K Q^T, dP = V dO^T
-      if (lane == 0 && n_items > 0) {
+      if (n_items > 0 && elect_one()) {
         auto y_full = [&](int idx) { return mbar_wait(bar + kFBarYFull + 8 * (idx & 3), (idx >> 2) & 1, abort_flag); };
         auto y_slot = [&](int idx) { return base + kFSmemY + (idx & 3) * kTileBytes; };
 #ifdef SDPA_BWD_STAMPS
@@ -353,7 +353,7 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     } else if (warp == 10) {
       // ------------------------------------------------------------------ dV += P^T dO, dQ = dS K, dK += dS^T Q
-      if (lane == 0 && n_items > 0) {
+      if (n_items > 0 && elect_one()) {
         bool ok = mbar_wait(bar + kFBarXFull, 0, abort_flag);
         for (int i = 0; ok && i < n_items; ++i) {
           const int s0 = (2 * i) & 3;

@@ -263,7 +263,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer (rest of the ring)
-    if (lane == 0 && n_items > 0) {
+    if (n_items > 0 && elect_one()) {
       for (int idx = kPreloaded; idx < 2 * n_items; ++idx)
         if (!load_tile(idx)) break;
       drain_after_abort(abort_flag);
@@ -280,7 +280,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // overwrites that item's P / dS buffer). There is one per item parity, so that the barrier a wait
     // looks at cannot be a whole phase further on: its next phase belongs to item i+2, whose scores
     // only exist after this wait.
-    if (lane == 0 && n_items > 0) {
+    if (n_items > 0 && elect_one()) {
       // Where the score GEMMs of item i land:
       //   dK/dV: S(i) in T[i&1], dP(i) in T[(i&1)^1]. The compute warpgroups put BOTH 16-bit results
       //          (P and dS) into the S buffer, so the dP buffer is free once it has been read and

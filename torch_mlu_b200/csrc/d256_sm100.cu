@@ -194,7 +194,7 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer: K(0) V(0) K(1) V(1) ...
-    if (lane == 0) {
+    if (elect_one()) {
       for (int t = 0; t < 2 * n_blocks; ++t) {
         const int s = t % kSlots;
         const uint32_t lap = static_cast<uint32_t>(t / kSlots);
@@ -211,7 +211,7 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_blocks > 0) {
+    if (n_blocks > 0 && elect_one()) {
       auto slot_of = [&](int t) { return base + kSmemRing + (t % kSlots) * kSlotBytes; };
       auto wait_full = [&](int t) { return mbar_wait(bar + kBFull + 8 * (t % kSlots), (t / kSlots) & 1, abort_flag); };
       auto issue_qk = [&](int j) {
@@ -642,7 +642,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       for (int t = 0; t < 2 * n_items; ++t) {
         const int i = t >> 1;
         const int s = slot_index(t);
@@ -677,7 +677,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     // memory): a single issuer would hold the pipe back. So warp 9 issues the score GEMMs and warp 10 the accumulations;
     // what the pipe's own order would guarantee between the two is the `W read` barrier (warp 10 commits it behind an item's
     // accumulation, warp 9 waits for it before a score GEMM overwrites that item's P / dS).
-    if (lane == 0 && n_items > 0) {
+    if (n_items > 0 && elect_one()) {
       auto wait_full = [&](int t) { return mbar_wait(bar + kBFull + 8 * slot_index(t), (t / kRing) & 1, abort_flag); };
       auto release = [&](int t) { umma_commit(bar + kBEmpty + 8 * slot_index(t)); };
       auto t_buf = [&](int k) { return (k & 1) ? t_b : t_a; };

@@ -332,7 +332,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     reg_decrease<kRegsOther>();
     if (warp == kProducerWarp) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
+      if (elect_one()) {
         tma_prefetch_desc(&tm_q);
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
@@ -378,7 +378,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
     } else if (warp == kMmaWarp) {
       // ------------------------------------------------------------------ MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t kv_base = 0;          // ring position of this unit's K(0)
         uint32_t ucnt = 0;             // units started so far
         uint32_t cnt0 = 0, cnt1 = 0;   // key blocks issued so far per Q tile (phase of the S/P/O barriers)
