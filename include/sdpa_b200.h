@@ -257,6 +257,15 @@ SDPA_B200_API int sdpa_b200_transpose_bias(const void* bias, int64_t batch_strid
                                            int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, void* out,
                                            int64_t out_row_stride, void* stream);
 
+/* Writes a boolean attention mask (one byte per element, non-zero = the pair takes part, element strides, 0 for a broadcast
+ * dimension) as the additive bias of 0 / -inf that sdpa_b200_params.bias takes: out is
+ * [batch][heads][seqlen_q][out_row_stride] 16-bit elements of `dtype`, contiguous, out_row_stride a multiple of 8 that holds
+ * seqlen_k; the padding is zero-filled. Pass 1 for a dimension the mask is broadcast along and give the bias the stride 0
+ * there. */
+SDPA_B200_API int sdpa_b200_mask_to_bias(const void* mask, int64_t batch_stride, int64_t head_stride, int64_t row_stride,
+                                         int64_t key_stride, int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k,
+                                         void* out, int64_t out_row_stride, int32_t dtype, void* stream);
+
 /* How many of this library's kernels the calling process has launched so far. */
 SDPA_B200_API uint64_t sdpa_b200_launch_count(void);
 

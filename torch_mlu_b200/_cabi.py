@@ -32,6 +32,7 @@ EXPORTED_SYMBOLS = (
     "sdpa_b200_dropout_keep_mask",
     "sdpa_b200_dropout_keep_mask_varlen",
     "sdpa_b200_transpose_bias",
+    "sdpa_b200_mask_to_bias",
     "sdpa_b200_launch_count",
 )
 STATIC_SCRATCH_BYTES = 16 << 20
@@ -118,6 +119,9 @@ def load() -> ctypes.CDLL:
     lib.sdpa_b200_transpose_bias.restype = c_int
     lib.sdpa_b200_transpose_bias.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32, c_void_p,
                                              c_int64, c_void_p]
+    lib.sdpa_b200_mask_to_bias.restype = c_int
+    lib.sdpa_b200_mask_to_bias.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32, c_void_p,
+                                           c_int64, c_int32, c_void_p]
     _lib = lib
     return lib
 

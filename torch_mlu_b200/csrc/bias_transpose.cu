@@ -1,4 +1,5 @@
-// Transposed copy of an attention bias for the backward pass: [.., Lq, Lk] -> [.., Lk, ld >= Lq].
+// Preparation of attention biases: a boolean mask as a bias (mask_to_bias_kernel), and the transposed copy for the backward
+// pass: [.., Lq, Lk] -> [.., Lk, ld >= Lq].
 //
 // The dK/dV kernel's threads own keys and walk over queries, so it reads a bias stored query-major two bytes
 // at a time; with this copy (sdpa_b200_params.bias_t) it reads 16 bytes at a time. HBM-bound: every element is
@@ -52,10 +53,79 @@ __global__ void __launch_bounds__(256) bias_transpose_kernel(const TransposePara
   }
 }
 
+// Boolean mask -> 0 / -inf bias, eight keys (16 bytes of output) per thread. Launch-bound for the usual padding masks (a few
+// KB); one kernel where the tensor-library route took three (fill, invert, masked fill) and a copy for unaligned rows.
+struct MaskParams {
+  const uint8_t* mask;
+  uint4* out;
+  int64_t batch_stride, head_stride, row_stride, key_stride;
+  int heads, seqlen_q, seqlen_k, groups;  // groups: 8-key groups per output row
+  uint32_t neg_inf;                       // -inf in both halves
+};
+
+__global__ void __launch_bounds__(256) mask_to_bias_kernel(const MaskParams p, int64_t total) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const int64_t row = i / p.groups;
+  const int k0 = static_cast<int>(i - row * p.groups) * 8;
+  const int64_t bh = row / p.seqlen_q;
+  const int64_t b = bh / p.heads;
+  const uint8_t* src = p.mask + b * p.batch_stride + (bh - b * p.heads) * p.head_stride + (row - bh * p.seqlen_q) * p.row_stride;
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int k = k0 + 2 * j;
+    uint32_t x = 0u;
+    if (k < p.seqlen_k && src[k * p.key_stride] == 0) x |= p.neg_inf & 0x0000ffffu;
+    if (k + 1 < p.seqlen_k && src[(k + 1) * p.key_stride] == 0) x |= p.neg_inf & 0xffff0000u;
+    w[j] = x;
+  }
+  p.out[i] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 }  // namespace
 }  // namespace sdpa_b200
 
 using namespace sdpa_b200;
+
+extern "C" SDPA_B200_API int sdpa_b200_mask_to_bias(const void* mask, int64_t batch_stride, int64_t head_stride, int64_t row_stride,
+                                                    int64_t key_stride, int32_t batch, int32_t heads, int32_t seqlen_q,
+                                                    int32_t seqlen_k, void* out, int64_t out_row_stride, int32_t dtype,
+                                                    void* stream) {
+  if (mask == nullptr || out == nullptr || (reinterpret_cast<uintptr_t>(out) & 15u) || batch <= 0 || heads <= 0 || seqlen_q <= 0 ||
+      seqlen_k <= 0 || batch_stride < 0 || head_stride < 0 || row_stride < 0 || key_stride < 0 || (out_row_stride % 8) != 0 ||
+      out_row_stride < seqlen_k || (dtype != SDPA_B200_BF16 && dtype != SDPA_B200_F16)) {
+    set_error("mask_to_bias: non-NULL pointers, a 16-byte aligned output, positive sizes, strides that are not negative and "
+              "an output row stride that is a multiple of 8 and holds seqlen_k");
+    return SDPA_B200_INVALID_ARG;
+  }
+  MaskParams m;
+  m.mask = static_cast<const uint8_t*>(mask);
+  m.out = static_cast<uint4*>(out);
+  m.batch_stride = batch_stride;
+  m.head_stride = head_stride;
+  m.row_stride = row_stride;
+  m.key_stride = key_stride;
+  m.heads = heads;
+  m.seqlen_q = seqlen_q;
+  m.seqlen_k = seqlen_k;
+  m.groups = static_cast<int>(out_row_stride / 8);
+  m.neg_inf = dtype == SDPA_B200_F16 ? 0xfc00fc00u : 0xff80ff80u;
+  const int64_t total = static_cast<int64_t>(batch) * heads * seqlen_q * m.groups;
+  const int64_t blocks = (total + 255) / 256;
+  if (blocks > 0x7fffffff) {
+    set_error("mask_to_bias: too many elements");
+    return SDPA_B200_INVALID_ARG;
+  }
+  mask_to_bias_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(m, total);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) {
+    set_error("mask_to_bias: launch failed: %s", cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
+  }
+  count_launch();
+  return SDPA_B200_OK;
+}
 
 extern "C" SDPA_B200_API int sdpa_b200_transpose_bias(const void* bias, int64_t batch_stride, int64_t head_stride,
                                                       int64_t row_stride, int32_t batch, int32_t heads, int32_t seqlen_q,

@@ -1,0 +1,318 @@
+// Autograd formulas of the attention operators and the scaled_dot_product_attention front end, in C++: a training step on
+// short sequences is bound by the host work around four kernels of a few microseconds each, and the Python versions of
+// these wrappers (torch.library.register_autograd, a torch.autograd.Function, the choice function's twenty checks) took
+// 200 to 300 us per step where this file takes about 20.
+#include <ATen/ExpandUtils.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+#include <torch/library.h>
+
+#include "torch_glue.h"
+
+namespace b200_glue {
+
+using at::Tensor;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+void check_status(int st, const char* what) {
+  if (C10_LIKELY(st == SDPA_B200_OK)) return;
+  throw StatusError(st, c10::str(what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error()));
+}
+
+// ------------------------------------------------------------------------- additive bias
+int64_t ceil8(int64_t n) { return (n + 7) / 8 * 8; }
+
+// The additive bias as a [B, H, Lq, Lk] view the kernels can read: broadcast dimensions keep stride 0, rows start 16-byte
+// aligned and are readable up to the next multiple of 8 keys. A bias that already has that layout is used in place; any
+// other is copied once into rows padded to a multiple of 8.
+Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k) {
+  TORCH_CHECK(attn_bias.scalar_type() == q.scalar_type() && attn_bias.device() == q.device(),
+              "attn_bias must have the dtype and device of query");
+  const int64_t full[4] = {q.size(0), q.size(1), q.size(2), seqlen_k};
+  Tensor view = attn_bias.expand(full);
+  if (view.stride(3) == 1 && seqlen_k % 8 == 0 && reinterpret_cast<uintptr_t>(view.data_ptr()) % 16 == 0 &&
+      view.stride(0) % 8 == 0 && view.stride(1) % 8 == 0 && view.stride(2) % 8 == 0)
+    return view;
+  std::vector<int64_t> sizes(attn_bias.sizes().begin(), attn_bias.sizes().end());
+  sizes.back() = seqlen_k;
+  Tensor src = attn_bias.expand(sizes);
+  sizes.back() = ceil8(seqlen_k);
+  Tensor buf = at::zeros(sizes, q.options());
+  buf.narrow(-1, 0, seqlen_k).copy_(src);
+  return buf.narrow(-1, 0, seqlen_k).expand(full);
+}
+
+// A boolean attn_mask (true = take part) as a bias of 0 / -inf in the layout of prepare_bias: one kernel over the mask's own
+// elements (broadcast dimensions stay broadcast).
+Tensor bias_of_mask(const Tensor& mask, const Tensor& q, int64_t seqlen_k) {
+  const int64_t full[4] = {q.size(0), q.size(1), q.size(2), seqlen_k};
+  const Tensor m = mask.expand(full);
+  int64_t own[4];
+  for (int i = 0; i < 3; ++i) own[i] = m.stride(i) == 0 ? 1 : full[i];
+  own[3] = ceil8(seqlen_k);
+  Tensor buf = at::detail::empty_cuda(own, q.scalar_type(), q.device(), c10::nullopt);
+  check_status(sdpa_b200_mask_to_bias(m.data_ptr(), m.stride(0), m.stride(1), m.stride(2), m.stride(3), static_cast<int32_t>(own[0]),
+                                      static_cast<int32_t>(own[1]), static_cast<int32_t>(own[2]), static_cast<int32_t>(seqlen_k),
+                                      buf.data_ptr(), own[3], q.scalar_type() == at::kHalf ? SDPA_B200_F16 : SDPA_B200_BF16,
+                                      at::cuda::getCurrentCUDAStream(q.get_device()).stream()),
+               "sdpa_b200_mask_to_bias");
+  return buf.narrow(-1, 0, seqlen_k).expand(full);
+}
+
+// [B, H, Lk, Lq] view of a copy of `bias` with keys and queries exchanged, for the dK/dV kernel, whose threads own keys and
+// read consecutive queries; undefined for a bias that does not depend on the query.
+Tensor transposed_bias(const Tensor& bias) {
+  if (bias.stride(2) == 0) return {};
+  const int64_t B = bias.size(0), H = bias.size(1), Lq = bias.size(2), Lk = bias.size(3);
+  const int64_t nb = bias.stride(0) == 0 ? 1 : B, nh = bias.stride(1) == 0 ? 1 : H, lq8 = ceil8(Lq);
+  Tensor buf = at::detail::empty_cuda({nb, nh, Lk, lq8}, bias.scalar_type(), bias.device(), c10::nullopt);
+  check_status(sdpa_b200_transpose_bias(bias.data_ptr(), bias.stride(0), bias.stride(1), bias.stride(2), static_cast<int32_t>(nb),
+                                        static_cast<int32_t>(nh), static_cast<int32_t>(Lq), static_cast<int32_t>(Lk),
+                                        buf.data_ptr(), lq8, at::cuda::getCurrentCUDAStream(bias.get_device()).stream()),
+               "sdpa_b200_transpose_bias");
+  return buf.narrow(-1, 0, Lq).expand({B, H, Lk, Lq});
+}
+
+// ------------------------------------------------------------------------- autograd
+using DenseBackwardOp = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
+                                                           const Tensor&, const Tensor&, const Tensor&, int64_t, int64_t, double,
+                                                           bool, const Tensor&, const Tensor&, c10::optional<double>);
+
+// One node for all forms: dense, dense with an additive bias, packed.
+struct AttentionBackward : public torch::autograd::Node {
+  SavedVariable q, k, v, out, lse, cu_q, cu_k, seed, offset;
+  Tensor bias;                       // dense with bias: the prepared view
+  std::vector<int64_t> bias_sizes;   // shape of the attn_mask argument, when its gradient is wanted
+  bool packed = false, causal = false, want_dbias = false;
+  int64_t max_q = 0, max_k = 0;
+  double scale = 1.0, dropout_p = 0.0;
+
+  std::string name() const override { return "B200AttentionBackward"; }
+
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* s : {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset}) s->reset_data();
+    bias.reset();
+  }
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list result(num_outputs());
+    if (!grads[0].defined()) return result;
+    const Tensor& go = grads[0];
+    const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), out_ = out.unpack(shared_from_this()), lse_ = lse.unpack();
+    const Tensor seed_ = seed.unpack(), offset_ = offset.unpack();
+    Tensor dq, dk, dv;
+    if (bias.defined()) {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      c10::cuda::CUDAGuard device_guard(q_.device());
+      Tensor dbias;
+      if (want_dbias)  // zero-filled: the kernels skip what the causal mask hides
+        dbias = at::zeros({q_.size(0), q_.size(1), q_.size(2), ceil8(k_.size(2))}, q_.options()).narrow(-1, 0, k_.size(2));
+      const Tensor bias_t = transposed_bias(bias);
+      BackwardOptions opt;
+      opt.bias = &bias;
+      opt.dbias = &dbias;
+      opt.bias_t = &bias_t;
+      std::tie(dq, dk, dv) = dense_backward(go, q_, k_, v_, out_, lse_, causal, scale, opt);
+      if (want_dbias) result[3] = at::sum_to(dbias, bias_sizes);
+    } else if (at::GradMode::is_enabled()) {
+      // create_graph=True: through the operators, so that whatever autograd knows about them applies
+      if (packed) {
+        static auto op = c10::Dispatcher::singleton()
+                             .findSchemaOrThrow("b200_sdpa::_flash_attention_backward", "").typed<DenseBackwardOp>();
+        std::tie(dq, dk, dv) = op.call(go, q_, k_, v_, out_, lse_, cu_q.unpack(), cu_k.unpack(), max_q, max_k, dropout_p, causal,
+                                       seed_, offset_, scale);
+      } else {
+        static auto op = c10::Dispatcher::singleton()
+                             .findSchemaOrThrow("b200_sdpa::_scaled_dot_product_flash_attention_backward", "").typed<DenseBackwardOp>();
+        const Tensor none = at::empty({0}, q_.options().dtype(at::kInt));
+        std::tie(dq, dk, dv) = op.call(go, q_, k_, v_, out_, lse_, none, none, max_q, max_k, dropout_p, causal, seed_, offset_, scale);
+      }
+    } else {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      if (packed)
+        std::tie(dq, dk, dv) = varlen_backward_with_dropout(go, q_, k_, v_, out_, lse_, cu_q.unpack(), cu_k.unpack(), max_q, max_k,
+                                                            dropout_p, causal, seed_, offset_, scale);
+      else
+        std::tie(dq, dk, dv) = dense_backward_with_dropout(go, q_, k_, v_, out_, lse_, dropout_p, causal, seed_, offset_, scale);
+    }
+    if (task_should_compute_output(0)) result[0] = dq;
+    if (task_should_compute_output(1)) result[1] = dk;
+    if (task_should_compute_output(2)) result[2] = dv;
+    return result;
+  }
+};
+
+bool any_requires_grad(std::initializer_list<const Tensor*> tensors) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : tensors)
+    if (t->defined() && t->requires_grad()) return true;
+  return false;
+}
+
+// Hangs a node behind `out` (a fresh tensor). `bias_arg`: the attn_mask the caller gave, or undefined.
+std::shared_ptr<AttentionBackward> new_node(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& bias_arg, bool causal,
+                                            double scale, double dropout_p) {
+  std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(bias_arg.defined() ? torch::autograd::collect_next_edges(q, k, v, bias_arg)
+                                          : torch::autograd::collect_next_edges(q, k, v));
+  node->q = SavedVariable(q, false);
+  node->k = SavedVariable(k, false);
+  node->v = SavedVariable(v, false);
+  node->causal = causal;
+  node->scale = scale;
+  node->dropout_p = dropout_p;
+  return node;
+}
+
+void finish_node(const std::shared_ptr<AttentionBackward>& node, Tensor& out, const Tensor& lse, const Tensor& seed,
+                 const Tensor& offset) {
+  torch::autograd::set_history(out, node);
+  node->out = SavedVariable(out, true);
+  node->lse = SavedVariable(lse, false);
+  node->seed = SavedVariable(seed, false);
+  node->offset = SavedVariable(offset, false);
+}
+
+using DenseOp = std::tuple<Tensor, Tensor, Tensor, Tensor, int64_t, int64_t, Tensor, Tensor, Tensor>(
+    const Tensor&, const Tensor&, const Tensor&, double, bool, bool, c10::optional<double>);
+using PackedOp = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&,
+                                                                    const Tensor&, int64_t, int64_t, double, bool, bool,
+                                                                    c10::optional<double>);
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, int64_t, int64_t, Tensor, Tensor, Tensor> dense_with_grad(
+    const Tensor& q, const Tensor& k, const Tensor& v, double dropout_p, bool is_causal, bool return_debug_mask,
+    c10::optional<double> scale) {
+  static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_scaled_dot_product_flash_attention", "").typed<DenseOp>();
+  auto r = [&] {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    return op.call(q, k, v, dropout_p, is_causal, return_debug_mask, scale);
+  }();
+  if (any_requires_grad({&q, &k, &v})) {
+    auto node = new_node(q, k, v, Tensor(), is_causal, scale_or_default(q, scale), dropout_p);
+    node->max_q = q.size(2);
+    node->max_k = k.size(2);
+    Tensor lse = std::get<1>(r);
+    if (lse.size(2) != q.size(2)) lse = lse.slice(2, 0, q.size(2)).contiguous();
+    finish_node(node, std::get<0>(r), lse, std::get<6>(r), std::get<7>(r));
+  }
+  return r;
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> packed_with_grad(const Tensor& q, const Tensor& k, const Tensor& v,
+                                                                    const Tensor& cu_q, const Tensor& cu_k, int64_t max_q,
+                                                                    int64_t max_k, double dropout_p, bool is_causal,
+                                                                    bool return_debug_mask, c10::optional<double> scale) {
+  static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_flash_attention_forward", "").typed<PackedOp>();
+  auto r = [&] {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    return op.call(q, k, v, cu_q, cu_k, max_q, max_k, dropout_p, is_causal, return_debug_mask, scale);
+  }();
+  if (any_requires_grad({&q, &k, &v})) {
+    auto node = new_node(q, k, v, Tensor(), is_causal, scale_or_default(q, scale), dropout_p);
+    node->packed = true;
+    node->max_q = max_q;
+    node->max_k = max_k;
+    node->cu_q = SavedVariable(cu_q, false);
+    node->cu_k = SavedVariable(cu_k, false);
+    finish_node(node, std::get<0>(r), std::get<1>(r), std::get<2>(r), std::get<3>(r));
+  }
+  return r;
+}
+
+bool broadcasts_to(const Tensor& t, const int64_t (&full)[4]) {
+  const int64_t d = t.dim();
+  for (int64_t i = 0; i < d; ++i) {
+    const int64_t n = t.size(d - 1 - i);
+    if (n != 1 && n != full[3 - i]) return false;
+  }
+  return true;
+}
+
+}  // namespace
+
+// The checks are those of sdp_choice.py (sdp_utils.h:99-455): a call that fails one of them, or whose answer depends on more
+// than they say (autocast, tensor subclasses, a top-left causal mask over unequal lengths), gets an undefined tensor, and
+// the Python function goes through the whole procedure with its warnings and errors.
+Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::optional<Tensor>& attn_mask, double dropout_p,
+            bool is_causal, c10::optional<double> scale) {
+  const auto& ctx = at::globalContext();
+  const bool flash = ctx.userEnabledFlashSDP(), efficient = ctx.userEnabledMemEfficientSDP();
+  const bool has_mask = attn_mask.has_value() && attn_mask->defined();
+  if (!(efficient || (flash && !has_mask))) return {};
+  if (at::autocast::is_autocast_enabled(at::kCUDA) || c10::impl::TorchDispatchModeTLS::any_modes_set()) return {};
+  for (const Tensor* t : {&q, &k, &v}) {
+    if (!t->is_cuda() || t->is_nested() || t->dim() != 4 || t->layout() != at::kStrided ||
+        t->unsafeGetTensorImpl()->is_python_dispatch() || t->stride(-1) != 1 || t->scalar_type() != q.scalar_type() ||
+        t->size(0) != q.size(0) || t->size(1) != q.size(1) || t->size(3) != q.size(3) || t->device() != q.device())
+      return {};
+  }
+  const auto dtype = q.scalar_type();
+  const int64_t D = q.size(3), Lq = q.size(2), Lk = k.size(2);
+  if ((dtype != at::kHalf && dtype != at::kBFloat16) || D < 64 || D > 256 || D % 8 != 0 || Lq == 0 || Lk == 0 || v.size(2) != Lk ||
+      q.size(0) == 0 || q.size(1) == 0 || (is_causal && Lq != Lk))
+    return {};
+  if (at::cuda::getDeviceProperties(q.get_device())->major != 10) return {};
+  const double sc = scale_or_default(q, scale);
+
+  if (!has_mask) {
+    DropoutResult r = [&] {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      return dense_forward_with_dropout(q, k, v, dropout_p, is_causal, false, sc, /*allow_gqa=*/false);
+    }();
+    if (any_requires_grad({&q, &k, &v})) {
+      auto node = new_node(q, k, v, Tensor(), is_causal, sc, dropout_p);
+      node->max_q = Lq;
+      node->max_k = Lk;
+      finish_node(node, r.out, r.lse, r.seed, r.offset);
+    }
+    return r.out;
+  }
+
+  const Tensor& mask = *attn_mask;
+  const int64_t full[4] = {q.size(0), q.size(1), Lq, Lk};
+  if (!efficient || D > 128 || dropout_p != 0.0 || mask.dim() < 1 || mask.dim() > 4 || !broadcasts_to(mask, full) || mask.stride(-1) != 1 ||
+      !mask.is_cuda() || mask.device() != q.device() || mask.unsafeGetTensorImpl()->is_python_dispatch() ||
+      !(mask.scalar_type() == at::kBool || at::isFloatingType(mask.scalar_type())))
+    return {};
+  c10::cuda::CUDAGuard device_guard(q.device());
+  const bool boolean = mask.scalar_type() == at::kBool;
+  const Tensor bias_arg = boolean ? Tensor() : mask.to(dtype);  // (differentiable) conversion of a bias of another type
+  Tensor bias, out, lse;
+  {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    bias = boolean ? bias_of_mask(mask, q, Lk) : prepare_bias(bias_arg, q, Lk);
+    ForwardOptions opt;
+    opt.bias = &bias;
+    std::tie(out, lse) = dense_forward(q, k, v, is_causal, sc, /*allow_gqa=*/false, opt);
+  }
+  if (any_requires_grad({&q, &k, &v, &bias_arg})) {
+    auto node = new_node(q, k, v, bias_arg, is_causal, sc, 0.0);
+    node->bias = bias;
+    if (bias_arg.defined() && bias_arg.requires_grad()) {
+      node->want_dbias = true;
+      node->bias_sizes = bias_arg.sizes().vec();
+    }
+    finish_node(node, out, lse, Tensor(), Tensor());
+  }
+  return out;
+}
+
+}  // namespace b200_glue
+
+TORCH_LIBRARY_IMPL(b200_sdpa, AutogradCUDA, m) {
+  m.impl("_scaled_dot_product_flash_attention", b200_glue::dense_with_grad);
+  m.impl("_flash_attention_forward", b200_glue::packed_with_grad);
+}

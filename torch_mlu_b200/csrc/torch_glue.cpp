@@ -15,6 +15,8 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGeneratorImpl.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
@@ -24,13 +26,29 @@
 #include <tuple>
 
 #include "../../include/sdpa_b200.h"
+#include "torch_glue.h"
 
-namespace {
+namespace b200_glue {
 
 using at::Tensor;
 
+namespace {
+
 void check_status(int st, const char* what) {
-  TORCH_CHECK(st == SDPA_B200_OK, what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error());
+  if (C10_LIKELY(st == SDPA_B200_OK)) return;
+  throw StatusError(st, c10::str(what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error()));
+}
+
+// Uninitialised device tensors without the dispatcher round trip of at::empty (a few hundred nanoseconds each, of calls
+// whose kernels run for a few microseconds).
+Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor& like) {
+  return at::detail::empty_cuda(sizes, dtype, like.device(), c10::nullopt);
+}
+
+// [B, H, L, D] tensor in the memory order of a [B, L, H, D] buffer, which the reference returns (attention.cpp:146-148)
+Tensor new_heads_second(int64_t B, int64_t H, int64_t L, int64_t D, const Tensor& like) {
+  const int64_t sizes[4] = {B, H, L, D}, strides[4] = {L * H * D, D, H * D, 1};
+  return at::detail::empty_strided_cuda(sizes, strides, like.scalar_type(), like.device());
 }
 
 // FlashAttention_internal.cpp:73-108: device, dtype and last-dim stride checks
@@ -41,9 +59,6 @@ void check_input(const Tensor& t, const char* name) {
   TORCH_CHECK(t.stride(-1) == 1, "Input tensor must have contiguous last dimension (", name, ")");
 }
 
-double scale_or_default(const Tensor& q, c10::optional<double> scale) {  // sdp_utils.h:40-47
-  return scale.has_value() ? *scale : 1.0 / std::sqrt(static_cast<double>(q.size(-1)));
-}
 
 void set_bhld(int64_t& bs, int64_t& hs, int64_t& rs, const Tensor& t) {
   bs = t.stride(0);
@@ -112,6 +127,8 @@ void varlen_params(sdpa_b200_params& p, const Tensor& q, const Tensor& k, const 
 // One int32 per device that every call made through this glue hands to the kernels (sdpa_b200_params.device_status):
 // a kernel whose bounded wait runs out leaves SDPA_B200_DEVICE_TIMEOUT in it, and it stays there, whatever happens
 // to the per-call workspaces, until b200_sdpa::_device_status reads and clears it.
+}  // namespace
+
 Tensor& status_word(int device) {
   static std::mutex mu;
   static Tensor words[64];
@@ -121,6 +138,12 @@ Tensor& status_word(int device) {
     words[device] = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
   return words[device];
 }
+
+double scale_or_default(const Tensor& q, c10::optional<double> scale) {  // sdp_utils.h:40-47
+  return scale.has_value() ? *scale : 1.0 / std::sqrt(static_cast<double>(q.size(-1)));
+}
+
+namespace {
 
 int64_t device_status(int64_t device) {
   if (device < 0) device = at::cuda::current_device();
@@ -133,17 +156,15 @@ int64_t device_status(int64_t device) {
   return st;
 }
 
-void run(const sdpa_b200_params& params, bool backward, const Tensor& like) {
-  sdpa_b200_params p = params;
+void run(sdpa_b200_params& p, bool backward, const Tensor& like) {
   p.device_status = reinterpret_cast<uint32_t*>(status_word(like.get_device()).data_ptr());
-  // torch.use_deterministic_algorithms(True) selects the backward with a fixed summation order
-  p.deterministic = at::globalContext().deterministicAlgorithms() ? 1 : 0;
   size_t bytes = 0;
   check_status(backward ? sdpa_b200_bwd_workspace_bytes(&p, &bytes) : sdpa_b200_fwd_workspace_bytes(&p, &bytes),
-               "sdpa_b200 workspace query");
-  Tensor ws = at::empty({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
+               "workspace query");
+  // from torch's stream-ordered pool, and back to it at the end of this call
+  const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
   void* stream = at::cuda::getCurrentCUDAStream(like.get_device()).stream();
-  check_status(backward ? sdpa_b200_bwd(&p, ws.data_ptr(), bytes, stream) : sdpa_b200_fwd(&p, ws.data_ptr(), bytes, stream),
+  check_status(backward ? sdpa_b200_bwd(&p, ws.get(), bytes, stream) : sdpa_b200_fwd(&p, ws.get(), bytes, stream),
                backward ? "sdpa_b200_bwd" : "sdpa_b200_fwd");
 }
 
@@ -158,6 +179,8 @@ void check_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   TORCH_CHECK(cu_q.numel() == cu_k.numel() && cu_q.numel() >= 2, "cu_seqlens_q and cu_seqlens_k must have batch+1 entries");
   TORCH_CHECK(k.size(1) == v.size(1) && q.size(1) % k.size(1) == 0,
               "Number of heads in key/value must divide number of heads in query");
+  TORCH_CHECK(q.size(2) == k.size(2) && q.size(2) == v.size(2), "query, key and value must have the same head_dim");
+  TORCH_CHECK(k.size(0) == v.size(0), "Key and Value must have the same number of tokens");
   check_input(q, "query");
   check_input(k, "key");
   check_input(v, "value");
@@ -167,11 +190,6 @@ void check_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
 // One bit per (query, key) pair in both orientations, written by the library from a Philox seed / offset pair
 // (the reference draws the pattern inside its kernel from such a pair and hands the pair to the backward
 // operator, FlashAttention_internal.cpp:190-214).
-struct KeepMasks {
-  Tensor rows, cols;  // int32 [B*H, Lq_pad, Lk_pad/32] and [B*H, Lk_pad, Lq_pad/32]
-  double p = 0.0;
-};
-
 KeepMasks make_keep_masks(const Tensor& q, int64_t seqlen_k, double dropout_p, uint64_t seed, uint64_t offset, bool causal) {
   TORCH_CHECK(dropout_p > 0.0 && dropout_p < 1.0, "dropout_p must be inside [0, 1)");
   c10::cuda::CUDAGuard guard(q.device());
@@ -279,6 +297,14 @@ Tensor debug_mask_of(const KeepMasks& m, const Tensor& q, int64_t seqlen_k) {
       .to(q.scalar_type());
 }
 
+void set_bias(sdpa_b200_params& p, const Tensor* bias) {
+  if (bias == nullptr || !bias->defined()) return;
+  p.bias = bias->data_ptr();
+  p.bias_batch_stride = bias->stride(0);
+  p.bias_head_stride = bias->stride(1);
+  p.bias_row_stride = bias->stride(2);
+}
+
 void set_dropout(sdpa_b200_params& p, const KeepMasks* keep) {
   if (keep == nullptr) return;
   p.dropout_p = static_cast<float>(keep->p);
@@ -286,9 +312,29 @@ void set_dropout(sdpa_b200_params& p, const KeepMasks* keep) {
   p.keep_cols = reinterpret_cast<const uint32_t*>(keep->cols.data_ptr());
 }
 
+void set_backward_options(sdpa_b200_params& p, const BackwardOptions& opt) {
+  set_bias(p, opt.bias);
+  if (opt.dbias != nullptr && opt.dbias->defined()) {
+    p.dbias = opt.dbias->data_ptr();
+    p.dbias_batch_stride = opt.dbias->stride(0);
+    p.dbias_head_stride = opt.dbias->stride(1);
+    p.dbias_row_stride = opt.dbias->stride(2);
+  }
+  if (opt.bias_t != nullptr && opt.bias_t->defined()) {
+    p.bias_t = opt.bias_t->data_ptr();
+    p.bias_t_batch_stride = opt.bias_t->stride(0);
+    p.bias_t_head_stride = opt.bias_t->stride(1);
+    p.bias_t_row_stride = opt.bias_t->stride(2);
+  }
+  // torch.use_deterministic_algorithms(True) selects the backward with a fixed summation order
+  p.deterministic = opt.deterministic >= 0 ? opt.deterministic : (at::globalContext().deterministicAlgorithms() ? 1 : 0);
+}
+
+}  // namespace
+
 // ------------------------------------------------------------------------- dense [B,H,L,D]
 std::tuple<Tensor, Tensor> dense_forward(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale,
-                                         bool allow_gqa, const KeepMasks* keep = nullptr) {
+                                         bool allow_gqa, const ForwardOptions& opt) {
   // attention.cpp:70-100
   TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && v.dim() == 4,
               "query, key and value must be 4-dimensional [batch, heads, seq_len, head_dim]");
@@ -306,33 +352,38 @@ std::tuple<Tensor, Tensor> dense_forward(const Tensor& q, const Tensor& k, const
   check_input(v, "value");
   c10::cuda::CUDAGuard guard(q.device());
   const int64_t B = q.size(0), H = q.size(1), L = q.size(2), D = q.size(3);
-  // [B,H,L,D] view of a [B,L,H,D] buffer, as the reference returns (attention.cpp:146-148)
-  Tensor out = at::empty({B, L, H, D}, q.options()).transpose(1, 2);
-  Tensor lse = at::empty({B, H, L}, q.options().dtype(at::kFloat));
+  Tensor out = new_heads_second(B, H, L, D, q);
+  Tensor lse = new_tensor({B, H, L}, at::kFloat, q);
   sdpa_b200_params p;
   dense_params(p, q, k, v, out, lse, causal, scale);
-  set_dropout(p, keep);
+  p.kernel = opt.kernel;
+  p.num_splits = opt.num_splits;
+  p.sm_margin = opt.sm_margin;
+  set_dropout(p, opt.keep);
+  set_bias(p, opt.bias);
   run(p, false, q);
   return {out, lse};
 }
 
 std::tuple<Tensor, Tensor, Tensor> dense_backward(const Tensor& dout_in, const Tensor& q, const Tensor& k, const Tensor& v,
                                                   const Tensor& out, const Tensor& lse, bool causal, double scale,
-                                                  const KeepMasks* keep = nullptr) {
+                                                  const BackwardOptions& opt) {
   Tensor dout = dout_in.stride(-1) == 1 ? dout_in : dout_in.contiguous();
   check_input(dout, "grad_out");
   check_input(q, "query");
   check_input(k, "key");
   check_input(v, "value");
   check_input(out, "out");
+  TORCH_CHECK(dout.scalar_type() == q.scalar_type() && out.scalar_type() == q.scalar_type(),
+              "query, key, and value must have the same dtype");
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.dim() == 3 && lse.size(0) == q.size(0) &&
                   lse.size(1) == q.size(1) && lse.size(2) == q.size(2),
               "logsumexp must be contiguous fp32 [batch, heads, seqlen_q]");
   c10::cuda::CUDAGuard guard(q.device());
   const int64_t B = q.size(0), D = q.size(3);
-  Tensor dq = at::empty({B, q.size(2), q.size(1), D}, q.options()).transpose(1, 2);
-  Tensor dk = at::empty({B, k.size(2), k.size(1), D}, k.options()).transpose(1, 2);
-  Tensor dv = at::empty({B, v.size(2), v.size(1), D}, v.options()).transpose(1, 2);
+  Tensor dq = new_heads_second(B, q.size(1), q.size(2), D, q);
+  Tensor dk = new_heads_second(B, k.size(1), k.size(2), D, k);
+  Tensor dv = new_heads_second(B, k.size(1), k.size(2), D, v);
   sdpa_b200_params p;
   dense_params(p, q, k, v, out, lse, causal, scale);
   p.dout = dout.data_ptr();
@@ -343,36 +394,42 @@ std::tuple<Tensor, Tensor, Tensor> dense_backward(const Tensor& dout_in, const T
   set_bhld(p.dq_batch_stride, p.dq_head_stride, p.dq_row_stride, dq);
   set_bhld(p.dk_batch_stride, p.dk_head_stride, p.dk_row_stride, dk);
   set_bhld(p.dv_batch_stride, p.dv_head_stride, p.dv_row_stride, dv);
-  set_dropout(p, keep);
+  set_dropout(p, opt.keep);
+  set_backward_options(p, opt);
   run(p, true, q);
   return {dq, dk, dv};
 }
 
+namespace {
+// what the Philox and debug slots of a result hold when there is no dropout (FlashAttention_internal.cpp:212-213)
+void no_dropout_slots(DropoutResult& r, const Tensor& q) {
+  r.seed = new_tensor({0}, at::kLong, q);
+  r.offset = new_tensor({0}, at::kLong, q);
+  r.debug = new_tensor({0}, q.scalar_type(), q);
+}
+}  // namespace
+
 // The dense operator pair with dropout: the forward draws a Philox pair, returns it as two CPU int64 scalars
 // (and the pattern on request); the backward draws the same pattern again from them.
-struct DenseDropoutResult {
-  Tensor out, lse, seed, offset, debug;
-};
-
-DenseDropoutResult dense_forward_with_dropout(const Tensor& q, const Tensor& k, const Tensor& v, double dropout_p,
-                                              bool causal, bool return_debug_mask, double scale, bool allow_gqa) {
+DropoutResult dense_forward_with_dropout(const Tensor& q, const Tensor& k, const Tensor& v, double dropout_p,
+                                         bool causal, bool return_debug_mask, double scale, bool allow_gqa) {
   TORCH_CHECK(dropout_p >= 0.0 && dropout_p < 1.0, "dropout_p must be inside [0, 1)");
-  DenseDropoutResult r;
-  r.seed = at::empty({0}, q.options().dtype(at::kLong));
-  r.offset = at::empty({0}, q.options().dtype(at::kLong));
-  r.debug = at::empty({0}, q.options());
+  DropoutResult r;
   if (dropout_p == 0.0) {
     std::tie(r.out, r.lse) = dense_forward(q, k, v, causal, scale, allow_gqa);
+    no_dropout_slots(r, q);
     return r;
   }
   TORCH_CHECK(q.dim() == 4 && k.dim() == 4, "query, key and value must be 4-dimensional [batch, heads, seq_len, head_dim]");
   auto [seed, offset] = draw_philox(q, q.size(0) * q.size(1) * q.size(2) * k.size(2));
   KeepMasks keep = make_keep_masks(q, k.size(2), dropout_p, seed, offset, causal);
-  std::tie(r.out, r.lse) = dense_forward(q, k, v, causal, scale, allow_gqa, &keep);
+  ForwardOptions opt;
+  opt.keep = &keep;
+  std::tie(r.out, r.lse) = dense_forward(q, k, v, causal, scale, allow_gqa, opt);
   g_keep_cache.put(dense_keep_key(q, k.size(2), dropout_p, seed, offset, causal), keep);
   r.seed = cpu_i64(seed);
   r.offset = cpu_i64(offset);
-  if (return_debug_mask) r.debug = debug_mask_of(keep, q, k.size(2));
+  r.debug = return_debug_mask ? debug_mask_of(keep, q, k.size(2)) : new_tensor({0}, q.scalar_type(), q);
   return r;
 }
 
@@ -389,8 +446,12 @@ std::tuple<Tensor, Tensor, Tensor> dense_backward_with_dropout(const Tensor& gra
   KeepMasks keep;
   if (!g_keep_cache.take(dense_keep_key(q, k.size(2), dropout_p, seed, offset, causal), &keep))
     keep = make_keep_masks(q, k.size(2), dropout_p, seed, offset, causal);
-  return dense_backward(grad_out, q, k, v, out, lse, causal, scale, &keep);
+  BackwardOptions opt;
+  opt.keep = &keep;
+  return dense_backward(grad_out, q, k, v, out, lse, causal, scale, opt);
 }
+
+namespace {
 
 // ------------------------------------------------------------------ packed [total,H,D]
 // packed form of the pattern: rows by packed token index, see sdpa_b200_dropout_keep_mask_varlen
@@ -413,16 +474,19 @@ KeepMasks make_keep_masks_varlen(const Tensor& q, const Tensor& k, const Tensor&
   return m;
 }
 
+}  // namespace
+
 std::tuple<Tensor, Tensor> varlen_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q,
                                           const Tensor& cu_k, int64_t max_q, int64_t max_k, bool causal, double scale,
-                                          const KeepMasks* keep = nullptr) {
+                                          const ForwardOptions& opt) {
   check_varlen(q, k, v, cu_q, cu_k);
   c10::cuda::CUDAGuard guard(q.device());
-  Tensor out = at::empty(q.sizes(), q.options());
-  Tensor lse = at::empty({q.size(1), q.size(0)}, q.options().dtype(at::kFloat));  // FlashAttention_internal.cpp:129
+  Tensor out = new_tensor(q.sizes(), q.scalar_type(), q);
+  Tensor lse = new_tensor({q.size(1), q.size(0)}, at::kFloat, q);  // FlashAttention_internal.cpp:129
   sdpa_b200_params p;
   varlen_params(p, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, causal, scale);
-  set_dropout(p, keep);
+  set_dropout(p, opt.keep);
+  set_bias(p, opt.bias);
   run(p, false, q);
   return {out, lse};
 }
@@ -430,18 +494,20 @@ std::tuple<Tensor, Tensor> varlen_forward(const Tensor& q, const Tensor& k, cons
 std::tuple<Tensor, Tensor, Tensor> varlen_backward(const Tensor& dout_in, const Tensor& q, const Tensor& k, const Tensor& v,
                                                    const Tensor& out, const Tensor& lse, const Tensor& cu_q,
                                                    const Tensor& cu_k, int64_t max_q, int64_t max_k, bool causal,
-                                                   double scale, const KeepMasks* keep = nullptr) {
+                                                   double scale, const BackwardOptions& opt) {
   check_varlen(q, k, v, cu_q, cu_k);
   Tensor dout = dout_in.stride(-1) == 1 ? dout_in : dout_in.contiguous();
   check_input(dout, "grad_out");
   check_input(out, "out");
+  TORCH_CHECK(dout.scalar_type() == q.scalar_type() && out.scalar_type() == q.scalar_type(),
+              "query, key, and value must have the same dtype");
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.dim() == 2 && lse.size(0) == q.size(1) &&
                   lse.size(1) == q.size(0),
               "logsumexp must be contiguous fp32 [heads_q, total_q]");
   c10::cuda::CUDAGuard guard(q.device());
-  Tensor dq = at::empty(q.sizes(), q.options());
-  Tensor dk = at::empty(k.sizes(), k.options());
-  Tensor dv = at::empty(v.sizes(), v.options());
+  Tensor dq = new_tensor(q.sizes(), q.scalar_type(), q);
+  Tensor dk = new_tensor(k.sizes(), k.scalar_type(), k);
+  Tensor dv = new_tensor(v.sizes(), v.scalar_type(), v);
   sdpa_b200_params p;
   varlen_params(p, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, causal, scale);
   p.dout = dout.data_ptr();
@@ -452,10 +518,13 @@ std::tuple<Tensor, Tensor, Tensor> varlen_backward(const Tensor& dout_in, const 
   set_thd(p.dq_batch_stride, p.dq_head_stride, p.dq_row_stride, dq);
   set_thd(p.dk_batch_stride, p.dk_head_stride, p.dk_row_stride, dk);
   set_thd(p.dv_batch_stride, p.dv_head_stride, p.dv_row_stride, dv);
-  set_dropout(p, keep);
+  set_dropout(p, opt.keep);
+  set_backward_options(p, opt);
   run(p, true, q);
   return {dq, dk, dv};
 }
+
+namespace {
 
 // The debug mask of a packed call: [B, Hq, max_q, max_k] in q's dtype, > 0 where a pair was kept and 0 outside a
 // sequence (attention.cpp:178-196 normalises the vendor kernel's mask to the same form). Reads cu_seqlens back
@@ -478,29 +547,27 @@ Tensor debug_mask_of_varlen(const KeepMasks& m, const Tensor& q, const Tensor& c
   return out;
 }
 
-// The packed operator pair with dropout.
-struct VarlenDropoutResult {
-  Tensor out, lse, seed, offset, debug;
-};
+}  // namespace
 
-VarlenDropoutResult varlen_forward_with_dropout(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q,
-                                                const Tensor& cu_k, int64_t max_q, int64_t max_k, double dropout_p, bool causal,
-                                                double scale, bool return_debug_mask = false) {
+// The packed operator pair with dropout.
+DropoutResult varlen_forward_with_dropout(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q,
+                                          const Tensor& cu_k, int64_t max_q, int64_t max_k, double dropout_p, bool causal,
+                                          double scale, bool return_debug_mask) {
   TORCH_CHECK(dropout_p >= 0.0 && dropout_p < 1.0, "dropout_p must be inside [0, 1)");
-  VarlenDropoutResult r;
-  r.seed = at::empty({0}, q.options().dtype(at::kLong));
-  r.offset = at::empty({0}, q.options().dtype(at::kLong));
-  r.debug = at::empty({0}, q.options());
+  DropoutResult r;
   if (dropout_p == 0.0) {
     std::tie(r.out, r.lse) = varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, causal, scale);
+    no_dropout_slots(r, q);
     return r;
   }
   check_varlen(q, k, v, cu_q, cu_k);
   auto [seed, offset] = draw_philox(q, (cu_q.numel() - 1) * q.size(1) * max_q * max_k);
   KeepMasks keep = make_keep_masks_varlen(q, k, cu_q, cu_k, max_q, max_k, dropout_p, seed, offset, causal);
-  std::tie(r.out, r.lse) = varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, causal, scale, &keep);
+  ForwardOptions opt;
+  opt.keep = &keep;
+  std::tie(r.out, r.lse) = varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, causal, scale, opt);
   g_keep_cache.put(packed_keep_key(q, k, cu_q, max_q, max_k, dropout_p, seed, offset, causal), keep);
-  if (return_debug_mask) r.debug = debug_mask_of_varlen(keep, q, cu_q, cu_k, max_q, max_k);
+  r.debug = return_debug_mask ? debug_mask_of_varlen(keep, q, cu_q, cu_k, max_q, max_k) : new_tensor({0}, q.scalar_type(), q);
   r.seed = cpu_i64(seed);
   r.offset = cpu_i64(offset);
   return r;
@@ -522,8 +589,12 @@ std::tuple<Tensor, Tensor, Tensor> varlen_backward_with_dropout(const Tensor& gr
   KeepMasks keep;
   if (!g_keep_cache.take(packed_keep_key(q, k, cu_q, max_q, max_k, dropout_p, seed, offset, causal), &keep))
     keep = make_keep_masks_varlen(q, k, cu_q, cu_k, max_q, max_k, dropout_p, seed, offset, causal);
-  return varlen_backward(grad_out, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, causal, scale, &keep);
+  BackwardOptions opt;
+  opt.keep = &keep;
+  return varlen_backward(grad_out, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, causal, scale, opt);
 }
+
+namespace {
 
 // ------------------------------------------------ operators with the reference's schemas
 std::tuple<Tensor, Tensor, Tensor, Tensor, int64_t, int64_t, Tensor, Tensor, Tensor> ref_sdpa_flash(
@@ -690,6 +761,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> autocast_flash_forward(
 }
 
 }  // namespace
+}  // namespace b200_glue
+
+using namespace b200_glue;
 
 TORCH_LIBRARY(b200_sdpa, m) {
   // codegen/mlu_functions.yaml:1313-1316, verbatim argument lists

@@ -17,6 +17,10 @@ strides (any [B,H,L,D] / [B,L,H,D] view with unit head_dim stride), so the five
 
 torch is used for device memory and the current stream only. There is no CPU path: a call
 on a machine without the built library or without an sm_100 GPU raises.
+
+The calls themselves are made by csrc/py_calls.cpp (checks, outputs, parameter block and launch in one native call: a short
+decode or prefill is host-bound otherwise); the ``_*_params`` / ``_run_*`` helpers drive the C ABI field by field, for
+callers that bring their own output buffers.
 """
 from __future__ import annotations
 
@@ -26,7 +30,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _cabi, dropout
+from . import _cabi, dropout, torch_glue
 
 __all__ = [
     "_scaled_dot_product_flash_attention",
@@ -46,20 +50,14 @@ def calculate_scale(query: torch.Tensor, scale: Optional[float]) -> float:
     return float(scale) if scale is not None else 1.0 / math.sqrt(query.size(-1))
 
 
+def _calls():
+    """The module of direct native calls (loaded on first use)."""
+    return torch_glue.calls or torch_glue.load()
+
+
 def _check(cond: bool, msg: str) -> None:
     if not cond:
         raise RuntimeError(msg)
-
-
-def _check_inputs(*tensors: torch.Tensor) -> None:
-    for t in tensors:
-        _check(t.is_cuda, "Input tensor must be on a CUDA device (this path has no CPU fallback)")
-        # FlashAttention_internal.cpp:74-80
-        _check(t.dtype in (torch.bfloat16, torch.float16),
-               f"FlashAttention only support fp16 and bf16 data type (got {t.dtype})")
-        _check(t.dtype == tensors[0].dtype, "query, key, and value must have the same dtype")
-        # FlashAttention_internal.cpp:100-108
-        _check(t.stride(-1) == 1, "Input tensor must have contiguous last dimension")
 
 
 def _stream_ptr(device: Optional[torch.device] = None) -> int:
@@ -102,8 +100,7 @@ class _Workspace:
         bounded wait runs out leaves DEVICE_TIMEOUT in it, and it stays there until device_status() reads it."""
         word = cls._status.get(device.index)
         if word is None:
-            word = torch.zeros(1, dtype=torch.int32, device=device)
-            cls._status[device.index] = word
+            word = cls._status[device.index] = _calls().status_word(device.index)
         return word
 
 
@@ -252,31 +249,13 @@ def _new_bias_grad(query, key):
 
 def _dense_forward(query, key, value, is_causal, scale, allow_gqa, kernel=_cabi.KERNEL_AUTO, num_splits=0, keep=None,
                    bias=None, sm_margin=0):
-    # attention.cpp:70-100; `keep`: dropout.KeepMasks of this call, or None; `bias`: from _prepare_bias, or None
-    _check(query.dim() == 4 and key.dim() == 4 and value.dim() == 4,
-           "query, key and value must be 4-dimensional [batch, heads, seq_len, head_dim]")
-    _check(query.size(0) == key.size(0) == value.size(0), "query, key and value must have the same batch size")
-    _check(key.size(2) == value.size(2), "Key and Value must have the same sequence length")
-    if allow_gqa:
-        _check(key.size(1) == value.size(1) and query.size(1) % key.size(1) == 0,
-               "Number of heads in key/value must divide number of heads in query")
-    else:
-        _check(query.size(1) == key.size(1) == value.size(1),
-               "query, key and value must have the same number of heads")
-    _check(query.size(3) == key.size(3) == value.size(3), "query, key and value must have the same head_dim")
-    _check_inputs(query, key, value)
-    B, H, Lq, D = query.shape
-    # the reference returns a [B,H,L,D] view of a [B,L,H,D] buffer (attention.cpp:146-148)
-    out = torch.empty((B, Lq, H, D), dtype=query.dtype, device=query.device).transpose(1, 2)
-    lse = torch.empty((B, H, Lq), dtype=torch.float32, device=query.device)
-    p = _dense_params(query, key, value, out, lse, is_causal, scale, kernel, num_splits)
-    if keep is not None:
-        p.dropout_p = keep.dropout_p
-        p.keep_rows, p.keep_cols = keep.rows.data_ptr(), keep.cols.data_ptr()
-    _set_bias(p, bias)
-    p.sm_margin = int(sm_margin)
-    _run_fwd(p, query.device)
-    return out, lse
+    """(out [B,H,Lq,D] in the memory order of [B,Lq,H,D], lse [B,H,Lq]). `keep`: dropout.KeepMasks of this call, or None;
+    `bias`: from _prepare_bias, or None; `scale` None: 1/sqrt(head_dim)."""
+    if keep is None:
+        return _calls().dense_forward(query, key, value, is_causal, scale, allow_gqa, kernel, num_splits, sm_margin, None, None, 0.0,
+                                      bias)
+    return _calls().dense_forward(query, key, value, is_causal, scale, allow_gqa, kernel, num_splits, sm_margin, keep.rows, keep.cols,
+                                  keep.dropout_p, bias)
 
 
 def _scaled_dot_product_flash_attention(query, key, value, dropout_p: float = 0.0, is_causal: bool = False,
@@ -314,38 +293,21 @@ def _scaled_dot_product_flash_attention(query, key, value, dropout_p: float = 0.
 
 
 def _deterministic(flag: Optional[bool]) -> int:
-    """The backward's `deterministic` switch: an explicit choice, else torch's global setting."""
-    return int(torch.are_deterministic_algorithms_enabled() if flag is None else bool(flag))
+    """The backward's `deterministic` switch: an explicit choice (0 / 1), else -1 for torch's global setting."""
+    return -1 if flag is None else int(bool(flag))
 
 
 def _dense_backward(grad_out, query, key, value, out, logsumexp, is_causal, scale, keep=None, bias=None, dbias=None,
                     bias_t=None, deterministic: Optional[bool] = None):
     # bias_t: a transposed copy of the bias (see _transposed_bias) kept by the caller; made here when missing
     # deterministic: True = the kernels with a fixed summation order; None = torch.are_deterministic_algorithms_enabled()
-    _check_inputs(grad_out, query, key, value, out)
-    _check(logsumexp.dtype == torch.float32 and logsumexp.is_contiguous(), "logsumexp must be contiguous fp32")
-    B, H, Lq, D = query.shape
-    _check(tuple(logsumexp.shape) == (B, H, Lq), "logsumexp must be [batch, heads, seqlen_q]")
-    dq = torch.empty((B, Lq, H, D), dtype=query.dtype, device=query.device).transpose(1, 2)
-    dk = torch.empty((B, key.size(2), key.size(1), D), dtype=key.dtype, device=key.device).transpose(1, 2)
-    dv = torch.empty((B, key.size(2), key.size(1), D), dtype=key.dtype, device=key.device).transpose(1, 2)
-    p = _dense_params(query, key, value, out, logsumexp, is_causal, scale)
-    p.dout, p.dq, p.dk, p.dv = grad_out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    _set_strides_bhld(p, "do", grad_out)
-    _set_strides_bhld(p, "dq", dq)
-    _set_strides_bhld(p, "dk", dk)
-    _set_strides_bhld(p, "dv", dv)
-    if keep is not None:
-        p.dropout_p = keep.dropout_p
-        p.keep_rows, p.keep_cols = keep.rows.data_ptr(), keep.cols.data_ptr()
     if bias_t is False:
         bias_t = None  # the caller wants the strided reads (tests compare the two paths)
     elif bias is not None and bias_t is None:
         bias_t = _transposed_bias(bias)  # one HBM pass; the dK/dV kernel then reads the bias 16 bytes at a time
-    _set_bias(p, bias, dbias, bias_t)
-    p.deterministic = _deterministic(deterministic)
-    _run_bwd(p, query.device)
-    return dq, dk, dv
+    rows, cols, p = (None, None, 0.0) if keep is None else (keep.rows, keep.cols, keep.dropout_p)
+    return _calls().dense_backward(grad_out, query, key, value, out, logsumexp, is_causal, scale, rows, cols, p, bias, dbias, bias_t,
+                                   _deterministic(deterministic))
 
 
 def _scaled_dot_product_flash_attention_backward(grad_out, query, key, value, out, logsumexp, cum_seq_q, cum_seq_k,
@@ -505,62 +467,30 @@ def _varlen_params(query, key, value, out, lse, cu_q, cu_k, max_q, max_k, is_cau
     return p
 
 
-def _check_varlen(query, key, value, cu_q, cu_k):
-    # FlashAttention_internal.cpp:81-84, 112-127
+def _check_packed(query, key, value, cu_q, cu_k):
+    # what drawing a dropout pattern needs to be true; the native call makes all the checks of
+    # FlashAttention_internal.cpp:81-127
     _check(query.dim() == 3 and key.dim() == 3 and value.dim() == 3,
            "varlen query, key and value must be packed [total_tokens, heads, head_dim]")
-    _check(cu_q.dtype == torch.int32, "cu_seqlens_q must have dtype int32")
-    _check(cu_k.dtype == torch.int32, "cu_seqlens_k must have dtype int32")
-    _check(cu_q.is_cuda and cu_k.is_cuda, "cu_seqlens must be on the device")
-    _check(cu_q.is_contiguous() and cu_k.is_contiguous(), "cu_seqlens must be contiguous")
+    for name, cu in (("cu_seqlens_q", cu_q), ("cu_seqlens_k", cu_k)):
+        _check(cu.dtype == torch.int32, f"{name} must have dtype int32")
+        _check(cu.is_cuda and cu.is_contiguous(), "cu_seqlens must be contiguous device tensors")
     _check(cu_q.numel() == cu_k.numel() and cu_q.numel() >= 2, "cu_seqlens_q and cu_seqlens_k must have batch+1 entries")
-    _check(key.size(1) == value.size(1) and query.size(1) % key.size(1) == 0,
-           "Number of heads in key/value must divide number of heads in query")
-    _check(query.size(2) == key.size(2) == value.size(2), "query, key and value must have the same head_dim")
-    _check(key.size(0) == value.size(0), "Key and Value must have the same number of tokens")
-    _check_inputs(query, key, value)
 
 
 def _varlen_forward(query, key, value, cu_q, cu_k, max_q, max_k, is_causal, scale, keep=None, bias=None):
     """Packed forward: (out [total_q, Hq, D], lse [Hq, total_q]). `keep`: dropout.KeepMasksVarlen or None; `bias`: a
     [B, Hq, max_q, max_k] view from _prepare_bias or None (sequence b reads bias[b] by positions inside the sequence)."""
-    _check_varlen(query, key, value, cu_q, cu_k)
-    out = torch.empty_like(query, memory_format=torch.contiguous_format)
-    lse = torch.empty((query.size(1), query.size(0)), dtype=torch.float32, device=query.device)
-    p = _varlen_params(query, key, value, out, lse, cu_q, cu_k, max_q, max_k, is_causal, scale)
-    if keep is not None:
-        p.dropout_p = keep.dropout_p
-        p.keep_rows, p.keep_cols = keep.rows.data_ptr(), keep.cols.data_ptr()
-    _set_bias(p, bias)
-    _run_fwd(p, query.device)
-    return out, lse
+    rows, cols, p = (None, None, 0.0) if keep is None else (keep.rows, keep.cols, keep.dropout_p)
+    return _calls().varlen_forward(query, key, value, cu_q, cu_k, int(max_q), int(max_k), is_causal, scale, rows, cols, p, bias)
 
 
 def _varlen_backward(grad_out, query, key, value, out, logsumexp, cu_q, cu_k, max_q, max_k, is_causal, scale, keep=None,
                      bias=None, dbias=None, deterministic: Optional[bool] = None):
-    _check_varlen(query, key, value, cu_q, cu_k)
-    if grad_out.stride(-1) != 1:
-        grad_out = grad_out.contiguous()
-    _check_inputs(grad_out, out)
-    _check(logsumexp.dtype == torch.float32 and logsumexp.is_contiguous()
-           and tuple(logsumexp.shape) == (query.size(1), query.size(0)),
-           "logsumexp must be contiguous fp32 [heads_q, total_q]")
-    dq = torch.empty_like(query, memory_format=torch.contiguous_format)
-    dk = torch.empty_like(key, memory_format=torch.contiguous_format)
-    dv = torch.empty_like(value, memory_format=torch.contiguous_format)
-    p = _varlen_params(query, key, value, out, logsumexp, cu_q, cu_k, max_q, max_k, is_causal, scale)
-    p.dout, p.dq, p.dk, p.dv = grad_out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    _set_strides_thd(p, "do", grad_out)
-    _set_strides_thd(p, "dq", dq)
-    _set_strides_thd(p, "dk", dk)
-    _set_strides_thd(p, "dv", dv)
-    if keep is not None:
-        p.dropout_p = keep.dropout_p
-        p.keep_rows, p.keep_cols = keep.rows.data_ptr(), keep.cols.data_ptr()
-    _set_bias(p, bias, dbias, None if bias is None else _transposed_bias(bias))
-    p.deterministic = _deterministic(deterministic)
-    _run_bwd(p, query.device)
-    return dq, dk, dv
+    rows, cols, p = (None, None, 0.0) if keep is None else (keep.rows, keep.cols, keep.dropout_p)
+    return _calls().varlen_backward(grad_out, query, key, value, out, logsumexp, cu_q, cu_k, int(max_q), int(max_k), is_causal, scale,
+                                    rows, cols, p, bias, dbias, None if bias is None else _transposed_bias(bias),
+                                    _deterministic(deterministic))
 
 
 def _flash_attention_forward(query, key, value, cum_seq_q, cum_seq_k, max_q: int, max_k: int, dropout_p: float,
@@ -573,18 +503,15 @@ def _flash_attention_forward(query, key, value, cum_seq_q, cum_seq_k, max_q: int
     keep the packed layout here.
     """
     _check(0.0 <= dropout_p < 1.0, "dropout_p must be inside [0, 1)")
-    _check_varlen(query, key, value, cum_seq_q, cum_seq_k)
-    seed, offset = _philox_placeholders(query)
-    debug = _empty_like_debug(query)
-    keep = None
-    if dropout_p > 0.0:
-        # the Philox pair as two CPU int64 scalars; on request the pattern as [B, Hq, max_q, max_k], > 0 = kept
-        s, o = dropout.draw_seed_and_offset(query.device, (cum_seq_q.numel() - 1) * query.size(1) * int(max_q) * int(max_k))
-        keep = dropout.packed_masks(s, o, dropout_p, query.size(1), cum_seq_q, cum_seq_k, query.size(0), key.size(0),
-                                    int(max_q), int(max_k), is_causal, forward=True)
-        seed, offset = torch.tensor(s, dtype=torch.int64), torch.tensor(o, dtype=torch.int64)
-        if return_debug_mask:
-            debug = keep.dense().to(query.dtype)
+    if dropout_p == 0.0:
+        return _calls().flash_attention_forward(query, key, value, cum_seq_q, cum_seq_k, int(max_q), int(max_k), is_causal, scale)
+    _check_packed(query, key, value, cum_seq_q, cum_seq_k)
+    # the Philox pair as two CPU int64 scalars; on request the pattern as [B, Hq, max_q, max_k], > 0 = kept
+    s, o = dropout.draw_seed_and_offset(query.device, (cum_seq_q.numel() - 1) * query.size(1) * int(max_q) * int(max_k))
+    keep = dropout.packed_masks(s, o, dropout_p, query.size(1), cum_seq_q, cum_seq_k, query.size(0), key.size(0),
+                                int(max_q), int(max_k), is_causal, forward=True)
+    seed, offset = torch.tensor(s, dtype=torch.int64), torch.tensor(o, dtype=torch.int64)
+    debug = keep.dense().to(query.dtype) if return_debug_mask else _empty_like_debug(query)
     out, lse = _varlen_forward(query, key, value, cum_seq_q, cum_seq_k, max_q, max_k, is_causal, calculate_scale(query, scale),
                                keep=keep)
     return out, lse, seed, offset, debug
@@ -597,9 +524,9 @@ def _flash_attention_backward(grad_out, query, key, value, out, logsumexp, cum_s
     inside the kernel (the reference's shape check at FlashAttention_internal.cpp:363-364
     cannot pass for Hq != Hkv; here it can)."""
     _check(0.0 <= dropout_p < 1.0, "dropout_p must be inside [0, 1)")
-    _check_varlen(query, key, value, cum_seq_q, cum_seq_k)
     keep = None
     if dropout_p > 0.0:
+        _check_packed(query, key, value, cum_seq_q, cum_seq_k)
         s, o = _philox_ints(philox_seed, philox_offset)
         keep = dropout.packed_masks(s, o, dropout_p, query.size(1), cum_seq_q, cum_seq_k, query.size(0), key.size(0),
                                     int(max_q), int(max_k), is_causal, forward=False)
@@ -743,14 +670,11 @@ def decode_attention(query, key_cache, value_cache, *, scale: Optional[float] = 
 
     Split-KV streaming kernel; the key range is cut into ``num_splits`` pieces (0 = choose)."""
     _check(query.dim() == 4 and query.size(2) == 1, "decode_attention needs query of shape [B, Hq, 1, D]")
-    out, lse = _dense_forward(query, key_cache, value_cache, False, calculate_scale(query, scale),
-                              allow_gqa=True, kernel=_cabi.KERNEL_DECODE, num_splits=num_splits)
-    return out, lse
+    return _dense_forward(query, key_cache, value_cache, False, scale, True, _cabi.KERNEL_DECODE, num_splits)
 
 
 def gqa_prefill(query, key, value, *, is_causal: bool = False, scale: Optional[float] = None, sm_margin: int = 0):
     """Dense [B,Hq,L,D] x [B,Hkv,L,D] prefill with head broadcast (the dense reference op
     refuses Hq != Hkv, attention.cpp:82-83; the kernel underneath does not). ``sm_margin`` SMs are left free
     for a kernel that runs beside this one on another stream (a collective, for example)."""
-    return _dense_forward(query, key, value, is_causal, calculate_scale(query, scale), allow_gqa=True,
-                          kernel=_cabi.KERNEL_PREFILL, sm_margin=sm_margin)
+    return _dense_forward(query, key, value, is_causal, scale, True, _cabi.KERNEL_PREFILL, 0, None, None, int(sm_margin))

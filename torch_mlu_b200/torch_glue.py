@@ -1,4 +1,4 @@
-"""Builds and loads the dispatcher glue (csrc/torch_glue.cpp -> lib/libsdpa_b200_torch.so).
+"""Builds and loads the torch glue (csrc/torch_glue.cpp, sdpa_autograd.cpp, py_calls.cpp -> lib/libsdpa_b200_torch.so).
 
 After ``load()``:
 * ``torch.ops.b200_sdpa._scaled_dot_product_flash_attention`` (+ ``_backward``) and
@@ -19,9 +19,11 @@ import torch
 from . import _cabi, build as native_build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = os.path.join(HERE, "csrc", "torch_glue.cpp")
+CSRC = os.path.join(HERE, "csrc")
+SOURCES = ["torch_glue.cpp", "sdpa_autograd.cpp", "py_calls.cpp"]
+OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(_cabi.LIB_DIR, "libsdpa_b200_torch.so")
-_loaded = False
+calls = None  # the module of csrc/py_calls.cpp, once load() has run
 
 
 def build(verbose: bool = False) -> str:
@@ -30,76 +32,55 @@ def build(verbose: bool = False) -> str:
     # then load the new file as a second copy with its own state (error text, launch counter).
     if _cabi._lib is None:
         native_build.build_native()
-    newest = max(os.path.getmtime(SRC), os.path.getmtime(os.path.join(os.path.dirname(HERE), "include", "sdpa_b200.h")))
+    headers = [os.path.join(CSRC, "torch_glue.h"), os.path.join(os.path.dirname(HERE), "include", "sdpa_b200.h")]
+    newest = max(os.path.getmtime(p) for p in headers + [os.path.join(CSRC, f) for f in SOURCES])
     if os.path.exists(LIB) and os.path.getmtime(LIB) >= newest:
         return LIB
+    import sysconfig
+    from concurrent.futures import ThreadPoolExecutor
     from torch.utils import cpp_extension
     inc = [f"-I{p}" for p in cpp_extension.include_paths()]
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    inc.append(f"-I{cuda_home}/include")
+    inc += [f"-I{cuda_home}/include", f"-I{sysconfig.get_paths()['include']}"]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-DTORCH_API_INCLUDE_EXTENSION_H",
-           *inc, SRC, "-o", LIB, f"-L{_cabi.LIB_DIR}", "-lsdpa_b200", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10",
-           "-ltorch_cuda", "-lc10_cuda", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or r.returncode != 0:
-        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-    if r.returncode != 0:
-        raise RuntimeError("building the torch glue failed")
+    os.makedirs(OBJ_DIR, exist_ok=True)
+
+    def run(cmd):
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        if r.returncode != 0:
+            raise RuntimeError("building the torch glue failed")
+
+    objs = [os.path.join(OBJ_DIR, f.replace(".cpp", ".glue.o")) for f in SOURCES]
+    stale = [(f, o) for f, o in zip(SOURCES, objs) if not os.path.exists(o) or
+             os.path.getmtime(o) < max(os.path.getmtime(p) for p in headers + [os.path.join(CSRC, f)])]
+    with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
+        list(ex.map(lambda fo: run(["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+                                    "-DTORCH_API_INCLUDE_EXTENSION_H", *inc, "-c", os.path.join(CSRC, fo[0]), "-o", fo[1]]), stale))
+    run(["g++", "-shared", *objs, "-o", LIB, f"-L{_cabi.LIB_DIR}", "-lsdpa_b200", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10",
+         "-ltorch_cuda", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"])
     return LIB
 
 
-def _register_autograd() -> None:
-    """Autograd formulas for the b200_sdpa operators: the forward saves q, k, v, out and the
-    logsumexp, the backward is the matching *_backward operator (what upstream derivatives.yaml
-    wires for the aten operators the reference registers)."""
-    ns = torch.ops.b200_sdpa
-
-    def dense_setup(ctx, inputs, keyword_only_inputs, output):
-        query, key, value, dropout_p, is_causal, _dbg = inputs[:6]
-        out, lse, cum_q, cum_k, max_q, max_k, seed, offset, _ = output
-        ctx.save_for_backward(query, key, value, out, lse, cum_q, cum_k, seed, offset)
-        ctx.args = (max_q, max_k, dropout_p, is_causal)
-        ctx.scale = keyword_only_inputs.get("scale")
-
-    def dense_backward(ctx, grad_out, *ignored):
-        query, key, value, out, lse, cum_q, cum_k, seed, offset = ctx.saved_tensors
-        max_q, max_k, dropout_p, is_causal = ctx.args
-        dq, dk, dv = ns._scaled_dot_product_flash_attention_backward(grad_out, query, key, value, out, lse, cum_q, cum_k,
-                                                                      max_q, max_k, dropout_p, is_causal, seed, offset,
-                                                                      scale=ctx.scale)
-        return dq, dk, dv, None, None, None
-
-    def varlen_setup(ctx, inputs, keyword_only_inputs, output):
-        query, key, value, cum_q, cum_k, max_q, max_k, dropout_p, is_causal, _dbg = inputs[:10]
-        out, lse, seed, offset, _ = output
-        ctx.save_for_backward(query, key, value, out, lse, cum_q, cum_k, seed, offset)
-        ctx.args = (max_q, max_k, dropout_p, is_causal)
-        ctx.scale = keyword_only_inputs.get("scale")
-
-    def varlen_backward(ctx, grad_out, *ignored):
-        query, key, value, out, lse, cum_q, cum_k, seed, offset = ctx.saved_tensors
-        max_q, max_k, dropout_p, is_causal = ctx.args
-        dq, dk, dv = ns._flash_attention_backward(grad_out, query, key, value, out, lse, cum_q, cum_k, max_q, max_k,
-                                                  dropout_p, is_causal, seed, offset, scale=ctx.scale)
-        return dq, dk, dv, None, None, None, None, None, None, None
-
-    torch.library.register_autograd("b200_sdpa::_scaled_dot_product_flash_attention", dense_backward,
-                                    setup_context=dense_setup)
-    torch.library.register_autograd("b200_sdpa::_flash_attention_forward", varlen_backward, setup_context=varlen_setup)
-
-
-def load() -> None:
-    """Load the glue library (building it first if needed). Raises if it cannot be built."""
-    global _loaded
-    if _loaded:
-        return
+def load():
+    """Load the glue library (building it first if needed) and return its module of direct calls. Raises if it cannot
+    be built."""
+    global calls
+    if calls is not None:
+        return calls
+    import importlib.machinery
+    import importlib.util
     build()
     _cabi.load()
     torch.ops.load_library(LIB)
-    _register_autograd()
-    _loaded = True
+    loader = importlib.machinery.ExtensionFileLoader("libsdpa_b200_torch", LIB)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("libsdpa_b200_torch", loader))
+    loader.exec_module(module)
+    module.set_status_error(_cabi.SdpaError)
+    calls = module
+    return calls
 
 
 def install_aten_overrides() -> None:
@@ -108,7 +89,7 @@ def install_aten_overrides() -> None:
 
 
 def remove_aten_overrides() -> None:
-    if _loaded:
+    if calls is not None:
         torch.ops.b200_sdpa._remove_aten_overrides()
 
 
