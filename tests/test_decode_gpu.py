@@ -32,6 +32,25 @@ def test_decode_matches_oracle(cuda_device, native_lib, B, Hq, Hkv, Lk, splits):
     orc.assert_close_lse(lse, l_ref)
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Lk,D", [
+    (1, 8, 1, 20000, 128),    # one unit over every CTA of the grid
+    (5, 24, 1, 130, 64),      # head chunks of 16 and 8, a tile of two keys
+    (75, 8, 4, 64, 128),      # one tile per unit, more units than CTAs: nothing is shared
+    (50, 8, 8, 65, 64),       # 400 units of two tiles: shares that begin and end inside units
+    (37, 12, 12, 700, 128),   # 444 units: CTAs with whole units between two shared ones
+])
+def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D):
+    """The automatic split deals 64-key tiles of all (batch, kv head) units out in equal contiguous shares: shapes whose
+    shares begin, end or lie entirely inside units. Tolerances as above (16-bit output, fp32 logsumexp)."""
+    q, k, v = rand((B, Hq, 1, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3)
+    dev = cuda_device
+    out, lse = ops.decode_attention(q.to(dev), k.to(dev), v.to(dev))
+    assert ops.device_status() == 0
+    o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=False)
+    orc.assert_close_bf16(out, o_ref, "out")
+    orc.assert_close_lse(lse, l_ref)
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,Lk,splits", [(2, 8, 2, 1000, 4), (1, 32, 2, 777, 3), (1, 4, 4, 4096, 0)])
 def test_decode_head_dim_64(cuda_device, native_lib, B, Hq, Hkv, Lk, splits):
     g = torch.Generator().manual_seed(8)

@@ -3,13 +3,19 @@
 // the fused kernel (torch_mlu/csrc/aten/operators/cnnl/transformers/sdp_utils.h:510-521) -
 // so semantics follow mha_varlen_fwd (FlashAttention_internal.cpp:57-267) with one query row.
 //
-// Work unit: (batch, kv head, split of the key range). A CTA of 4 warps streams its keys
-// once; each thread reads K and V rows with 128-bit loads straight into mma.sync fragments
-// (the contraction index of Q K^T is permuted so a 16-byte load IS a B fragment pair; V
-// pairs of keys are interleaved with two byte-permutes per word). All query heads of the
-// GQA group ride in the M dimension of m16n8k16, so K/V bytes are read once per group.
-// Per-split partial (O, lse) go to the workspace; a second kernel merges the splits with
-// warp shuffles.
+// A unit is one (batch, kv head, chunk of up to 16 query heads of its group): all those heads ride in the M dimension of
+// mma.sync.m16n8k16, so K/V bytes are read once per group. The keys of all units, cut into tiles of 64, form one list that is
+// dealt out in equal contiguous shares to a grid that fits the GPU in one wave (two CTAs per SM): every SM streams the same
+// number of bytes whatever the batch, the number of heads and the length are, and the loads of a CTA run on across unit
+// boundaries. (One CTA per (unit, split) left the last wave nearly empty - 512 CTAs on 444 places ran at 4.3 TB/s - and paid
+// the pipeline's fill and the merge of four warps once per split.) A unit whose tiles belong to several CTAs leaves partial
+// (O, lse) rows in the workspace, at most two per CTA, and a second kernel merges them.
+//
+// Inside a CTA each of the four warps owns 16 keys of every tile and a ring of shared-memory stages that its own elected lane
+// fills by TMA (two 16 x 64-column boxes each of K and V, 128-byte swizzle: ldmatrix reads them without bank conflicts), so
+// the warps never wait for one another inside a unit. 96 KB per CTA are in flight. Measured against register-fed loads and
+// fixed splits (Hq 32, Hkv 8, D 128): B 64 Lk 32768 1355 -> 1223 us (7.0 TB/s; a bare read kernel reaches 7.4), B 16 Lk 8192
+// 126 -> 89 us, B 1 Lk 32768 67 -> 31 us, B 1 Lk 1000 18.5 -> 8.7 us (both kernels, back to back).
 #include <cuda_bf16.h>
 
 #include <mutex>
@@ -22,33 +28,63 @@ namespace {
 
 constexpr int kDecWarps = 4;
 constexpr int kDecThreads = kDecWarps * 32;
-constexpr int kKeysPerStep = 16;  // keys one warp handles per loop iteration
-constexpr int kMaxD = 128;  // head_dim 64 and 128 are built
+constexpr int kKeysPerStep = 16;                        // keys one warp handles per tile
+constexpr int kTileKeys = kDecWarps * kKeysPerStep;     // 64
 constexpr int kMaxSplits = 128;
+constexpr int kCtasPerSm = 2;
+constexpr uint32_t kBoxRowBytes = 128;                  // one 64-column box row
+constexpr uint32_t kBoxBytes = kKeysPerStep * kBoxRowBytes;
 
 struct DecodeParams {
   const uint16_t* q;  // bf16 or f16 bits (f16 != 0)
-  const uint16_t* k;
-  const uint16_t* v;
   uint16_t* out;
   float* lse;
-  float* part_o;    // [batch, heads_q, splits, head_dim] fp32, normalised per split
-  float* part_lse;  // [batch, heads_q, splits] fp32, log2 domain
+  float* part_o;    // rows of head_dim fp32 values, normalised per share; the order of the rows: part_row()
+  float* part_lse;  // one fp32 value per row, log2 domain
+  uint32_t* status;
   int64_t q_batch_stride, q_head_stride;
-  int64_t k_batch_stride, k_head_stride, k_row_stride;
-  int64_t v_batch_stride, v_head_stride, v_row_stride;
   int64_t o_batch_stride, o_head_stride;
-  int heads_q, heads_kv, group, chunks, len_k, num_splits, keys_per_split, head_dim;
+  int heads_q, heads_kv, group, chunks, len_k, head_dim, rows;  // rows: query heads per unit, min(group, 16)
+  int units, tiles_per_unit, grid;
+  int num_splits, tiles_per_split;  // num_splits > 0: the caller fixed the shares, CTA = (unit, split)
   float scale_log2;
   int f16;
 };
 
-__device__ __forceinline__ uint4 ld_stream_16(const void* p) {
-  uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(p));
-  return r;
+// Tiles [first, last) of the list (tile = unit * tiles_per_unit + tile in unit) that CTA `i` works on.
+__host__ __device__ __forceinline__ void cta_share(const DecodeParams& p, int i, int64_t& first, int64_t& last) {
+  if (p.num_splits > 0) {
+    const int u = i / p.num_splits, sp = i - u * p.num_splits;
+    const int lo = sp * p.tiles_per_split, hi = lo + p.tiles_per_split;
+    first = static_cast<int64_t>(u) * p.tiles_per_unit + (lo < p.tiles_per_unit ? lo : p.tiles_per_unit);
+    last = static_cast<int64_t>(u) * p.tiles_per_unit + (hi < p.tiles_per_unit ? hi : p.tiles_per_unit);
+  } else {
+    const int64_t total = static_cast<int64_t>(p.units) * p.tiles_per_unit;
+    first = i * total / p.grid;
+    last = (i + 1) * total / p.grid;
+  }
+}
+
+// The CTA whose share holds `tile` (equal shares only).
+__device__ __forceinline__ int cta_of(const DecodeParams& p, int64_t tile) {
+  const int64_t total = static_cast<int64_t>(p.units) * p.tiles_per_unit;
+  return static_cast<int>(((tile + 1) * p.grid - 1) / total);
+}
+
+// Row of the partial results for one query head: with fixed splits [batch * heads_q][splits]; with equal shares two slots of
+// `rows` heads per CTA, slot 0 for the unit its share begins in and slot 1 for the unit it ends in (`r`: head in the unit).
+__device__ __forceinline__ int64_t part_row(const DecodeParams& p, int cta, int slot, int head_row, int r) {
+  if (p.num_splits > 0) return static_cast<int64_t>(head_row) * p.num_splits + cta % p.num_splits;
+  return (2 * static_cast<int64_t>(cta) + slot) * p.rows + r;
+}
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
 template <bool kF16>
@@ -106,359 +142,512 @@ __device__ __forceinline__ float quad_sum(float x) {
   return x;
 }
 
-// Shared scratch for the 4-warp merge: per warp 16 rows x (128 O + m + l).
+// Stages of each warp's ring: what lets two CTAs share an SM's 228 KB.
+template <bool kHi, int kD>
+__host__ __device__ constexpr int decode_stages() { return (kHi ? 2 : 3) * (128 / kD); }
 template <int kD>
-struct DecodeSmem {
-  float o[kDecWarps][16][kD];
-  float m[kDecWarps][16];
-  float l[kDecWarps][16];
-};
+__host__ __device__ constexpr uint32_t decode_stage_bytes() { return 2u * (kD / 64) * kBoxBytes; }
+// per merging warp: accumulators in fragment order [value][lane], then row maxima and sums
+template <bool kHi, int kD>
+__host__ __device__ constexpr int decode_merge_floats() { return ((kHi ? 4 : 2) * (kD / 8) + (kHi ? 4 : 2)) * 32; }
+template <bool kHi, int kD>
+__host__ __device__ constexpr uint32_t decode_smem_bytes() {
+  return 1024 + kDecWarps * decode_stages<kHi, kD>() * decode_stage_bytes<kD>() +
+         (kDecWarps - 1) * decode_merge_floats<kHi, kD>() * 4 + kDecWarps * decode_stages<kHi, kD>() * 8 + 16;
+}
 
-// kHi: the GQA group has more than 8 query heads, so fragment rows 8-15 are in use too.
+// kHi: a unit has more than 8 query heads, so fragment rows 8-15 are in use too.
 template <bool kHi, int kD, bool kF16>
-__global__ void __launch_bounds__(kDecThreads, 3) decode_splitkv_kernel(const DecodeParams p) {
-  __shared__ DecodeSmem<kD> sm;
+__global__ void __launch_bounds__(kDecThreads, kCtasPerSm)
+decode_splitkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const DecodeParams p) {
   constexpr int kKSteps = kD / 16;   // MMAs over head_dim for Q K^T
-  constexpr int kLoads = kD / 32;    // 16-byte K loads per thread and key
-  constexpr int kHalves = kD / 64;   // 64-column halves of V / O
   constexpr int kNBlocks = kD / 8;   // 8-column output blocks of P V
+  constexpr int kBoxes = kD / 64;    // 64-column boxes per operand and stage
+  constexpr int kSt = decode_stages<kHi, kD>();
+  constexpr uint32_t kStageBytes = decode_stage_bytes<kD>();
+  constexpr int kMergeFloats = decode_merge_floats<kHi, kD>();
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  const uint32_t base = (raw_addr + 1023u) & ~1023u;
+  float* merge = reinterpret_cast<float*>(smem_raw + (base - raw_addr) + kDecWarps * kSt * kStageBytes);
+  const uint32_t bars = smem_u32(merge + (kDecWarps - 1) * kMergeFloats);
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(merge + (kDecWarps - 1) * kMergeFloats + kDecWarps * kSt * 2);
+
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int g = lane >> 2;  // fragment row (query head within the chunk) / key within a block
+  const int g = lane >> 2;  // fragment row (query head within the unit) / key within a block of 8
   const int t = lane & 3;
-  const int split = blockIdx.x;
-  const int hkv = blockIdx.y / p.chunks;
-  const int chunk = blockIdx.y % p.chunks;
-  const int b = blockIdx.z;
-  const int head0 = hkv * p.group + chunk * 16;        // first query head of this CTA
-  const int nheads = min(16, p.group - chunk * 16);    // query heads this CTA serves
+  const uint32_t ring = base + warp * (kSt * kStageBytes);
+  const uint32_t bar = bars + warp * (kSt * 8);
 
-  const int k_begin = split * p.keys_per_split;
-  const int k_end = min(p.len_k, k_begin + p.keys_per_split);
+  // the merge kernel behind this one may be launched as soon as every CTA is running (it waits for this grid's results)
+  if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  // ---- Q fragments. MMA i (0..7) contracts over d = (i/2)*32 + 8t + 4(i&1) + {0,1 | 2,3}.
-  uint32_t qa[kKSteps][4];
-  {
-    const uint16_t* qb = p.q + b * p.q_batch_stride;
-#pragma unroll
-    for (int i = 0; i < kKSteps; ++i) {
-      const int d0 = (i >> 1) * 32 + 8 * t + 4 * (i & 1);
-      uint2 lo = make_uint2(0u, 0u), hi = make_uint2(0u, 0u);
-      if (g < nheads) lo = *reinterpret_cast<const uint2*>(qb + (head0 + g) * p.q_head_stride + d0);
-      if (kHi && g + 8 < nheads) hi = *reinterpret_cast<const uint2*>(qb + (head0 + g + 8) * p.q_head_stride + d0);
-      qa[i][0] = lo.x;  // row g,   k 2t..2t+1
-      qa[i][1] = hi.x;  // row g+8, k 2t..2t+1
-      qa[i][2] = lo.y;  // row g,   k 2t+8..2t+9
-      qa[i][3] = hi.y;  // row g+8, k 2t+8..2t+9
-    }
-  }
+  int64_t first, last;
+  cta_share(p, blockIdx.x, first, last);
+  const int n_tiles = static_cast<int>(last - first);
+  const int unit0 = static_cast<int>(first / p.tiles_per_unit);
+  const int tile0 = static_cast<int>(first - static_cast<int64_t>(unit0) * p.tiles_per_unit);
 
-  const uint16_t* kbase = p.k + b * p.k_batch_stride + hkv * p.k_head_stride;
-  const uint16_t* vbase = p.v + b * p.v_batch_stride + hkv * p.v_head_stride;
-  const int last_key = p.len_k - 1;
-
-  float o[kNBlocks][4];
-#pragma unroll
-  for (int nb = 0; nb < kNBlocks; ++nb) o[nb][0] = o[nb][1] = o[nb][2] = o[nb][3] = 0.f;
-  float m_lo = -INFINITY, m_hi = kHi ? -INFINITY : 0.f;  // running max (log2 domain) of rows g and g+8
-  float l_lo = 0.f, l_hi = 0.f;              // this thread's share of the running sums
-  const float c = p.scale_log2;
-
-  uint4 kbuf[2][kLoads];
-  auto load_k = [&](int key0) {
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      const int key = min(key0 + blk * 8 + g, last_key);
-      const uint16_t* row = kbase + static_cast<int64_t>(key) * p.k_row_stride + 8 * t;
-#pragma unroll
-      for (int l4 = 0; l4 < kLoads; ++l4) kbuf[blk][l4] = ld_stream_16(row + l4 * 32);
-    }
-  };
-
-  int key0 = k_begin + warp * kKeysPerStep;
-  if (key0 < k_end) load_k(key0);
-  for (; key0 < k_end; key0 += kDecWarps * kKeysPerStep) {
-    // ---- V rows of this step: keys 2t, 2t+1, 2t+8, 2t+9 at d = half*64 + 8g .. +7
-    uint4 vbuf[kHalves][4];
-    {
-      const int r0 = key0 + 2 * t;
-#pragma unroll
-      for (int half = 0; half < kHalves; ++half) {
-        const uint16_t* col = vbase + half * 64 + 8 * g;
-        vbuf[half][0] = ld_stream_16(col + static_cast<int64_t>(min(r0, last_key)) * p.v_row_stride);
-        vbuf[half][1] = ld_stream_16(col + static_cast<int64_t>(min(r0 + 1, last_key)) * p.v_row_stride);
-        vbuf[half][2] = ld_stream_16(col + static_cast<int64_t>(min(r0 + 8, last_key)) * p.v_row_stride);
-        vbuf[half][3] = ld_stream_16(col + static_cast<int64_t>(min(r0 + 9, last_key)) * p.v_row_stride);
-      }
-    }
-    // ---- S = Q K^T for two blocks of 8 keys
-    float s[2][4];
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      s[blk][0] = s[blk][1] = s[blk][2] = s[blk][3] = 0.f;
-#pragma unroll
-      for (int l4 = 0; l4 < kLoads; ++l4) {
-        const uint4 w = kbuf[blk][l4];
-        mma_rows<kHi, kF16>(s[blk], qa[2 * l4], w.x, w.y);
-        mma_rows<kHi, kF16>(s[blk], qa[2 * l4 + 1], w.z, w.w);
-      }
-    }
-    const int next = key0 + kDecWarps * kKeysPerStep;
-    if (next < k_end) load_k(next);
-
-    // ---- mask the tail, online softmax (thread holds keys key0 + blk*8 + 2t + {0,1})
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      const int kk = key0 + blk * 8 + 2 * t;
-      if (kk >= k_end) { s[blk][0] = -INFINITY; s[blk][2] = -INFINITY; }
-      if (kk + 1 >= k_end) { s[blk][1] = -INFINITY; s[blk][3] = -INFINITY; }
-    }
-    const float mx_lo = quad_max(fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]))) * c;
-    const float mx_hi = kHi ? quad_max(fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]))) * c : 0.f;
-    const float mn_lo = fmaxf(m_lo, mx_lo);
-    const float mn_hi = fmaxf(m_hi, mx_hi);
-    if (__any_sync(0xffffffffu, (mn_lo > m_lo) || (mn_hi > m_hi))) {
-      // every key0 < k_end step has at least one visible key, so mn_* is finite here
-      const float a_lo = ex2_approx(m_lo - mn_lo);
-      const float a_hi = ex2_approx(m_hi - mn_hi);
-      l_lo *= a_lo;
-      l_hi *= a_hi;
-#pragma unroll
-      for (int nb = 0; nb < kNBlocks; ++nb) {
-        o[nb][0] *= a_lo;
-        o[nb][1] *= a_lo;
-        if (kHi) {
-          o[nb][2] *= a_hi;
-          o[nb][3] *= a_hi;
-        }
-      }
-      m_lo = mn_lo;
-      m_hi = mn_hi;
-    }
-    float pr[2][4];
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      pr[blk][0] = ex2_approx(fmaf(s[blk][0], c, -m_lo));
-      pr[blk][1] = ex2_approx(fmaf(s[blk][1], c, -m_lo));
-      pr[blk][2] = kHi ? ex2_approx(fmaf(s[blk][2], c, -m_hi)) : 0.f;
-      pr[blk][3] = kHi ? ex2_approx(fmaf(s[blk][3], c, -m_hi)) : 0.f;
-      l_lo += pr[blk][0] + pr[blk][1];
-      l_hi += pr[blk][2] + pr[blk][3];
-    }
-    const uint32_t pa0 = pack_16x2<kF16>(pr[0][0], pr[0][1]);  // row g,   keys 2t, 2t+1
-    const uint32_t pa1 = pack_16x2<kF16>(pr[0][2], pr[0][3]);  // row g+8
-    const uint32_t pa2 = pack_16x2<kF16>(pr[1][0], pr[1][1]);  // row g,   keys 8+2t, 9+2t
-    const uint32_t pa3 = pack_16x2<kF16>(pr[1][2], pr[1][3]);  // row g+8
-
-    // ---- O += P V. n-block (half, q) covers d = half*64 + 8*n + q for fragment column n.
-#pragma unroll
-    for (int half = 0; half < kHalves; ++half) {
-      const uint32_t x0[4] = {vbuf[half][0].x, vbuf[half][0].y, vbuf[half][0].z, vbuf[half][0].w};
-      const uint32_t x1[4] = {vbuf[half][1].x, vbuf[half][1].y, vbuf[half][1].z, vbuf[half][1].w};
-      const uint32_t x2[4] = {vbuf[half][2].x, vbuf[half][2].y, vbuf[half][2].z, vbuf[half][2].w};
-      const uint32_t x3[4] = {vbuf[half][3].x, vbuf[half][3].y, vbuf[half][3].z, vbuf[half][3].w};
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const uint32_t sel = (q & 1) ? 0x7632u : 0x5410u;
-        const uint32_t b0 = __byte_perm(x0[q >> 1], x1[q >> 1], sel);
-        const uint32_t b1 = __byte_perm(x2[q >> 1], x3[q >> 1], sel);
-        const uint32_t pa[4] = {pa0, pa1, pa2, pa3};
-        mma_rows<kHi, kF16>(o[half * 8 + q], pa, b0, b1);
-      }
-    }
-  }
-
-  // ---- merge the 4 warps. Fragment column n = 2t + e of n-block (half, q) is
-  //      d = half*64 + 8*(2t+e) + q.
-  l_lo = quad_sum(l_lo);
-  l_hi = quad_sum(l_hi);
-  if (t == 0) {
-    sm.m[warp][g] = m_lo;
-    sm.m[warp][g + 8] = m_hi;
-    sm.l[warp][g] = l_lo;
-    sm.l[warp][g + 8] = l_hi;
-  }
-#pragma unroll
-  for (int half = 0; half < kHalves; ++half) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int nb = half * 8 + q;
-      const int d = half * 64 + 16 * t + q;
-      sm.o[warp][g][d] = o[nb][0];
-      sm.o[warp][g][d + 8] = o[nb][1];
-      if (kHi) {
-        sm.o[warp][g + 8][d] = o[nb][2];
-        sm.o[warp][g + 8][d + 8] = o[nb][3];
-      }
-    }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kDecWarps * kSt; ++i) mbar_init(bars + 8 * i, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
   }
   __syncthreads();
 
-  const int d = threadIdx.x;  // thread <-> output column (threads beyond head_dim idle)
-  for (int r = 0; d < kD && r < nheads; ++r) {
-    float mm = -INFINITY;
+  // ---- the load side of the warp's ring: its own step, tile and unit, kSt steps ahead of the arithmetic
+  int ld_unit = unit0, ld_tile = tile0, ld_step = 0;
+  int ld_b, ld_hk;
+  auto load_unit = [&]() {
+    const int hc = ld_unit / p.chunks;
+    ld_b = hc / p.heads_kv;
+    ld_hk = hc - ld_b * p.heads_kv;
+  };
+  load_unit();
+  auto issue_load = [&]() {  // called by one lane
+    const uint32_t st = ld_step % kSt;
+    const uint32_t dst = ring + st * kStageBytes, full = bar + 8 * st;
+    const int row = ld_tile * kTileKeys + warp * kKeysPerStep;
+    mbar_arrive_expect_tx(full, kStageBytes);
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) mm = fmaxf(mm, sm.m[w][r]);
-    float ll = 0.f, acc = 0.f;
+    for (int c = 0; c < kBoxes; ++c) tma_load_4d(dst + c * kBoxBytes, &tm_k, full, c * 64, row, ld_hk, ld_b);
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) {
-      const float mw = sm.m[w][r];
-      const float sc = (mw == -INFINITY) ? 0.f : ex2_approx(mw - mm);
-      ll += sm.l[w][r] * sc;
-      acc += sm.o[w][r][d] * sc;
+    for (int c = 0; c < kBoxes; ++c) tma_load_4d(dst + (kBoxes + c) * kBoxBytes, &tm_v, full, c * 64, row, ld_hk, ld_b);
+  };
+  auto next_load = [&]() {
+    ++ld_step;
+    if (++ld_tile == p.tiles_per_unit) {
+      ld_tile = 0;
+      ++ld_unit;
+      load_unit();
     }
-    const int hq = head0 + r;
-    const float inv = (ll > 0.f) ? 1.f / ll : 0.f;
-    const float lse2 = (ll > 0.f) ? mm + log2f(ll) : -INFINITY;
-    if (p.num_splits == 1) {
-      p.out[b * p.o_batch_stride + hq * p.o_head_stride + d] = to_16<kF16>(acc * inv);
-      if (d == 0)
-        p.lse[static_cast<int64_t>(b) * p.heads_q + hq] = (ll > 0.f) ? lse2 * 0.6931471805599453f : INFINITY;
-    } else {
-      const int64_t slot = (static_cast<int64_t>(b) * p.heads_q + hq) * p.num_splits + split;
-      p.part_o[slot * kD + d] = acc * inv;
-      if (d == 0) p.part_lse[slot] = lse2;
+  };
+  if (elect_one()) {
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  for (int i = 0; i < kSt && i < n_tiles; ++i) {
+    if (elect_one()) issue_load();
+    next_load();
+  }
+
+  // ---- Q fragments of a unit
+  uint32_t qa[kKSteps][4], qn[kKSteps][4];
+  auto load_q = [&](int unit, uint32_t (&dst)[kKSteps][4]) {
+    const int hc = unit / p.chunks, b = hc / p.heads_kv;
+    const int head0 = (hc - b * p.heads_kv) * p.group + (unit - hc * p.chunks) * 16;
+    const int nheads = min(16, p.group - (unit - hc * p.chunks) * 16);
+    const uint16_t* q0 = p.q + b * p.q_batch_stride + (head0 + g) * p.q_head_stride + 2 * t;
+    const uint16_t* q8 = q0 + 8 * p.q_head_stride;
+#pragma unroll
+    for (int i = 0; i < kKSteps; ++i) {
+      dst[i][0] = dst[i][1] = dst[i][2] = dst[i][3] = 0u;
+      if (g < nheads) {
+        dst[i][0] = *reinterpret_cast<const uint32_t*>(q0 + i * 16);      // row g,   k 2t..2t+1
+        dst[i][2] = *reinterpret_cast<const uint32_t*>(q0 + i * 16 + 8);  // row g,   k 2t+8..2t+9
+      }
+      if (kHi && g + 8 < nheads) {
+        dst[i][1] = *reinterpret_cast<const uint32_t*>(q8 + i * 16);
+        dst[i][3] = *reinterpret_cast<const uint32_t*>(q8 + i * 16 + 8);
+      }
+    }
+  };
+  if (n_tiles > 0) load_q(unit0, qn);
+
+  const float c = p.scale_log2;
+  // ldmatrix row addresses inside a box: this lane's row of each of the four 8x8 matrices
+  const int mrow = lane & 7, mat = lane >> 3;
+  bool ok = true;
+  int step = 0;
+  for (int unit = unit0, tile = tile0; step < n_tiles; ++unit, tile = 0) {
+    const int seg_tiles = min(n_tiles - step, p.tiles_per_unit - tile);
+    const bool whole = seg_tiles == p.tiles_per_unit && p.num_splits <= 1;
+#pragma unroll
+    for (int i = 0; i < kKSteps; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) qa[i][j] = qn[i][j];
+    if (step + seg_tiles < n_tiles) load_q(unit + 1, qn);  // in flight under this unit's tiles
+
+    float o[kNBlocks][4];
+#pragma unroll
+    for (int nb = 0; nb < kNBlocks; ++nb) o[nb][0] = o[nb][1] = o[nb][2] = o[nb][3] = 0.f;
+    float m_lo = -INFINITY, m_hi = -INFINITY;  // running max (log2 domain) of rows g and g+8
+    float l_lo = 0.f, l_hi = 0.f;              // this thread's share of the running sums
+
+    for (int i = 0; i < seg_tiles; ++i, ++step) {
+      const uint32_t st = step % kSt;
+      const uint32_t k_smem = ring + st * kStageBytes, v_smem = k_smem + kBoxes * kBoxBytes;
+      if (ok) ok = mbar_wait(bar + 8 * st, (step / kSt) & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+
+      // ---- S = Q K^T for two blocks of 8 keys
+      float s[2][4];
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk) {
+        s[blk][0] = s[blk][1] = s[blk][2] = s[blk][3] = 0.f;
+#pragma unroll
+        for (int ch = 0; ch < kD / 8; ch += 4) {  // four 16-byte chunks of 8 keys = the B fragments of two K steps
+          uint32_t kf[4];
+          const int chunk = ch + mat;
+          ldmatrix_x4(k_smem + (chunk >> 3) * kBoxBytes + (blk * 8 + mrow) * kBoxRowBytes + (((chunk & 7) ^ mrow) << 4), kf);
+          mma_rows<kHi, kF16>(s[blk], qa[ch / 2], kf[0], kf[1]);
+          mma_rows<kHi, kF16>(s[blk], qa[ch / 2 + 1], kf[2], kf[3]);
+        }
+      }
+
+      // ---- mask the tail, online softmax (thread holds keys key0 + blk*8 + 2t + {0,1})
+      const int key0 = (tile + i) * kTileKeys + warp * kKeysPerStep;
+      if (key0 + kKeysPerStep > p.len_k) {
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk) {
+          const int kk = key0 + blk * 8 + 2 * t;
+          if (kk >= p.len_k) { s[blk][0] = -INFINITY; s[blk][2] = -INFINITY; }
+          if (kk + 1 >= p.len_k) { s[blk][1] = -INFINITY; s[blk][3] = -INFINITY; }
+        }
+      }
+      const float mn_lo = fmaxf(m_lo, quad_max(fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]))) * c);
+      const float mn_hi = kHi ? fmaxf(m_hi, quad_max(fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]))) * c) : m_hi;
+      if (__any_sync(0xffffffffu, (mn_lo > m_lo) || (mn_hi > m_hi))) {
+        // a row that has seen no key yet (m = -inf) has o = l = 0: any finite factor will do
+        const float a_lo = (mn_lo == -INFINITY) ? 1.f : ex2_approx(m_lo - mn_lo);
+        const float a_hi = (mn_hi == -INFINITY) ? 1.f : ex2_approx(m_hi - mn_hi);
+        l_lo *= a_lo;
+        l_hi *= a_hi;
+#pragma unroll
+        for (int nb = 0; nb < kNBlocks; ++nb) {
+          o[nb][0] *= a_lo;
+          o[nb][1] *= a_lo;
+          if (kHi) {
+            o[nb][2] *= a_hi;
+            o[nb][3] *= a_hi;
+          }
+        }
+        m_lo = mn_lo;
+        m_hi = mn_hi;
+      }
+      const float u_lo = (m_lo == -INFINITY) ? 0.f : m_lo, u_hi = (m_hi == -INFINITY) ? 0.f : m_hi;
+      float pr[2][4];
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk) {
+        pr[blk][0] = ex2_approx(fmaf(s[blk][0], c, -u_lo));
+        pr[blk][1] = ex2_approx(fmaf(s[blk][1], c, -u_lo));
+        pr[blk][2] = kHi ? ex2_approx(fmaf(s[blk][2], c, -u_hi)) : 0.f;
+        pr[blk][3] = kHi ? ex2_approx(fmaf(s[blk][3], c, -u_hi)) : 0.f;
+        l_lo += pr[blk][0] + pr[blk][1];
+        l_hi += pr[blk][2] + pr[blk][3];
+      }
+      uint32_t pa[4];
+      pa[0] = pack_16x2<kF16>(pr[0][0], pr[0][1]);  // row g,   keys 2t, 2t+1
+      pa[1] = pack_16x2<kF16>(pr[0][2], pr[0][3]);  // row g+8
+      pa[2] = pack_16x2<kF16>(pr[1][0], pr[1][1]);  // row g,   keys 8+2t, 9+2t
+      pa[3] = pack_16x2<kF16>(pr[1][2], pr[1][3]);  // row g+8
+
+      // ---- O += P V: matrices (keys 0-7, chunk), (keys 8-15, chunk), the same for the next chunk
+#pragma unroll
+      for (int ch = 0; ch < kD / 8; ch += 2) {
+        uint32_t vf[4];
+        const int chunk = ch + (mat >> 1);
+        ldmatrix_x4_trans(v_smem + (chunk >> 3) * kBoxBytes + ((mat & 1) * 8 + mrow) * kBoxRowBytes + (((chunk & 7) ^ mrow) << 4), vf);
+        mma_rows<kHi, kF16>(o[ch], pa, vf[0], vf[1]);
+        mma_rows<kHi, kF16>(o[ch + 1], pa, vf[2], vf[3]);
+      }
+      // the stage has been read by every lane: refill it
+      __syncwarp();
+      if (ld_step < n_tiles) {
+        if (ok && elect_one()) issue_load();
+        next_load();
+      }
+    }
+
+    // ---- merge the four warps: 1-3 hand their state over in fragment order, warp 0 folds it into its own
+    l_lo = quad_sum(l_lo);
+    l_hi = quad_sum(l_hi);
+    __syncthreads();  // warp 0 has read what the previous unit left here
+    if (warp > 0) {
+      float* dst = merge + (warp - 1) * kMergeFloats + lane;
+#pragma unroll
+      for (int nb = 0; nb < kNBlocks; ++nb) {
+#pragma unroll
+        for (int e = 0; e < (kHi ? 4 : 2); ++e) dst[(nb * (kHi ? 4 : 2) + e) * 32] = o[nb][e];
+      }
+      dst += kNBlocks * (kHi ? 4 : 2) * 32;
+      dst[0] = m_lo;
+      dst[32] = l_lo;
+      if (kHi) {
+        dst[64] = m_hi;
+        dst[96] = l_hi;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      constexpr int kTail = kNBlocks * (kHi ? 4 : 2) * 32;
+      float mm_lo = m_lo, mm_hi = m_hi;
+#pragma unroll
+      for (int w = 0; w < kDecWarps - 1; ++w) {
+        mm_lo = fmaxf(mm_lo, merge[w * kMergeFloats + kTail + lane]);
+        if (kHi) mm_hi = fmaxf(mm_hi, merge[w * kMergeFloats + kTail + 64 + lane]);
+      }
+      auto weight = [](float m, float mm) { return (m == -INFINITY) ? 0.f : ex2_approx(m - mm); };
+      float f_lo = weight(m_lo, mm_lo), f_hi = kHi ? weight(m_hi, mm_hi) : 0.f;
+      l_lo *= f_lo;
+      l_hi *= f_hi;
+#pragma unroll
+      for (int nb = 0; nb < kNBlocks; ++nb) {
+        o[nb][0] *= f_lo;
+        o[nb][1] *= f_lo;
+        o[nb][2] *= f_hi;
+        o[nb][3] *= f_hi;
+      }
+#pragma unroll
+      for (int w = 0; w < kDecWarps - 1; ++w) {
+        const float* src = merge + w * kMergeFloats + lane;
+        f_lo = weight(src[kTail], mm_lo);
+        l_lo += src[kTail + 32] * f_lo;
+        if (kHi) {
+          f_hi = weight(src[kTail + 64], mm_hi);
+          l_hi += src[kTail + 96] * f_hi;
+        }
+#pragma unroll
+        for (int nb = 0; nb < kNBlocks; ++nb) {
+#pragma unroll
+          for (int e = 0; e < (kHi ? 4 : 2); ++e) o[nb][e] += src[(nb * (kHi ? 4 : 2) + e) * 32] * (e < 2 ? f_lo : f_hi);
+        }
+      }
+      const int hc = unit / p.chunks, b = hc / p.heads_kv;
+      const int head0 = (hc - b * p.heads_kv) * p.group + (unit - hc * p.chunks) * 16;
+      const int nheads = min(16, p.group - (unit - hc * p.chunks) * 16);
+#pragma unroll
+      for (int hi = 0; hi < (kHi ? 2 : 1); ++hi) {
+        const int r = g + 8 * hi;
+        if (r >= nheads) continue;
+        const float l = hi ? l_hi : l_lo, mm = hi ? mm_hi : mm_lo;
+        const float inv = (l > 0.f) ? 1.f / l : 0.f;
+        const float lse2 = (l > 0.f) ? mm + log2f(l) : -INFINITY;
+        if (whole) {
+          uint16_t* dst = p.out + b * p.o_batch_stride + (head0 + r) * p.o_head_stride + 2 * t;
+#pragma unroll
+          for (int nb = 0; nb < kNBlocks; ++nb)
+            *reinterpret_cast<uint32_t*>(dst + nb * 8) = pack_16x2<kF16>(o[nb][2 * hi] * inv, o[nb][2 * hi + 1] * inv);
+          if (t == 0) p.lse[static_cast<int64_t>(b) * p.heads_q + head0 + r] = (l > 0.f) ? lse2 * 0.6931471805599453f : INFINITY;
+        } else {
+          const int64_t row = part_row(p, blockIdx.x, unit == unit0 ? 0 : 1, b * p.heads_q + head0 + r, r);
+          float* dst = p.part_o + row * kD + 2 * t;
+#pragma unroll
+          for (int nb = 0; nb < kNBlocks; ++nb)
+            *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(o[nb][2 * hi] * inv, o[nb][2 * hi + 1] * inv);
+          if (t == 0) p.part_lse[row] = lse2;
+        }
+      }
     }
   }
+  // a fixed split without keys (more splits than tiles): its merge partner finds an empty part
+  if (n_tiles == 0 && p.num_splits > 1) {
+    const int u = blockIdx.x / p.num_splits, hc = u / p.chunks, b = hc / p.heads_kv;
+    const int chunk = u - hc * p.chunks;
+    if (static_cast<int>(threadIdx.x) < min(16, p.group - chunk * 16))
+      p.part_lse[part_row(p, blockIdx.x, 0, b * p.heads_q + (hc - b * p.heads_kv) * p.group + chunk * 16 + threadIdx.x, 0)] = -INFINITY;
+  }
+  if (lane == 0) drain_after_abort(abort_flag);
+  if (threadIdx.x == 0 && *abort_flag != 0) atomicExch(p.status, static_cast<uint32_t>(SDPA_B200_DEVICE_TIMEOUT));
 }
 
-// One warp per (batch, query head): merge the per-split partials.
-__global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams p, int rows) {
-  const int kD = p.head_dim;
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp_global >= rows) return;
-  const int b = warp_global / p.heads_q;
-  const int hq = warp_global % p.heads_q;
-  const float* pl = p.part_lse + static_cast<int64_t>(warp_global) * p.num_splits;
-  const float* po = p.part_o + static_cast<int64_t>(warp_global) * p.num_splits * kD;
-
-  // lane-strided pass over the split lse values, then a shuffle tree
-  float mx = -INFINITY;
-  for (int s = lane; s < p.num_splits; s += 32) mx = fmaxf(mx, pl[s]);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  float sum = 0.f;
-  for (int s = lane; s < p.num_splits; s += 32) {
-    const float v = pl[s];
-    sum += (v == -INFINITY) ? 0.f : exp2f(v - mx);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float inv = (sum > 0.f) ? 1.f / sum : 0.f;
-  const bool active = lane * 4 < kD;
-  for (int s = 0; active && s < p.num_splits; ++s) {
-    const float v = pl[s];
-    const float w = (v == -INFINITY) ? 0.f : exp2f(v - mx) * inv;
-    const float4 x = *reinterpret_cast<const float4*>(po + static_cast<int64_t>(s) * kD + lane * 4);
-    acc.x += w * x.x;
-    acc.y += w * x.y;
-    acc.z += w * x.z;
-    acc.w += w * x.w;
-  }
-  if (active) {
-    uint16_t* dst = p.out + b * p.o_batch_stride + hq * p.o_head_stride + lane * 4;
-    const uint2 packed = p.f16 ? make_uint2(pack_f16x2(acc.x, acc.y), pack_f16x2(acc.z, acc.w))
-                               : make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
-    *reinterpret_cast<uint2*>(dst) = packed;
-  }
-  if (lane == 0)
-    p.lse[warp_global] = (sum > 0.f) ? (mx + log2f(sum)) * 0.6931471805599453f : INFINITY;
-}
-
-template <int kD, bool kF16>
-void launch_decode_kernel_t(const DecodeParams& d, dim3 grid, cudaStream_t stream) {
-  if (d.group > 8) decode_splitkv_kernel<true, kD, kF16><<<grid, kDecThreads, 0, stream>>>(d);
-  else decode_splitkv_kernel<false, kD, kF16><<<grid, kDecThreads, 0, stream>>>(d);
-}
-
-void launch_decode_kernel(const DecodeParams& d, dim3 grid, cudaStream_t stream) {
-  if (d.head_dim == 64) {
-    if (d.f16) launch_decode_kernel_t<64, true>(d, grid, stream);
-    else launch_decode_kernel_t<64, false>(d, grid, stream);
+// Merges the parts of the units that several CTAs worked on: one CTA of four warps per (batch, query head), each warp a
+// quarter of the parts, lanes over head_dim.
+template <int kD>
+__global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams p) {
+  __shared__ float sm_o[3][kD], sm_m[4], sm_l[4];
+  const int row = blockIdx.x;  // batch * heads_q + query head
+  const int b = row / p.heads_q, hq = row - b * p.heads_q;
+  const int hk = hq / p.group, in_group = hq - hk * p.group;
+  const int unit = (b * p.heads_kv + hk) * p.chunks + in_group / 16, r = in_group % 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int c0, c1;  // CTAs [c0, c1] hold the unit's tiles
+  const int64_t u0 = static_cast<int64_t>(unit) * p.tiles_per_unit;
+  if (p.num_splits > 0) {
+    c0 = unit * p.num_splits;
+    c1 = c0 + p.num_splits - 1;
   } else {
-    if (d.f16) launch_decode_kernel_t<128, true>(d, grid, stream);
-    else launch_decode_kernel_t<128, false>(d, grid, stream);
+    c0 = cta_of(p, u0);
+    c1 = cta_of(p, u0 + p.tiles_per_unit - 1);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the parts are written
+  if (c0 == c1) return;  // one CTA had all of it and wrote the result itself
+  const int64_t total = static_cast<int64_t>(p.units) * p.tiles_per_unit;
+  // the unit's part of CTA c is its slot 0 unless c began in an earlier unit (only c0 can have)
+  const int first_slot = (p.num_splits == 0 && c0 * total / p.grid < u0) ? 1 : 0;
+
+  float m = -INFINITY, l = 0.f;
+  constexpr int kPer = kD / 32;  // floats per lane
+  float acc[kPer];
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) acc[e] = 0.f;
+  for (int c = c0 + warp * 4; c <= c1; c += 16) {
+    float ls[4], x[4][kPer];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool have = c + j <= c1;
+      const int cj = have ? c + j : c;
+      const int64_t pr = part_row(p, cj, cj == c0 ? first_slot : 0, row, r);
+      ls[j] = have ? p.part_lse[pr] : -INFINITY;
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) x[j][e] = (ls[j] == -INFINITY) ? 0.f : p.part_o[pr * kD + e * 32 + lane];
+    }
+    const float mn = fmaxf(fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3])), m);
+    if (mn == -INFINITY) continue;
+    const float a = exp2f(m - mn);
+    l *= a;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) acc[e] *= a;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float w = exp2f(ls[j] - mn);
+      l += w;
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) acc[e] += w * x[j][e];
+    }
+    m = mn;
+  }
+  if (lane == 0) {
+    sm_m[warp] = m;
+    sm_l[warp] = l;
+  }
+  if (warp > 0) {
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) sm_o[warp - 1][e * 32 + lane] = acc[e];
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  const float mm = fmaxf(fmaxf(sm_m[0], sm_m[1]), fmaxf(sm_m[2], sm_m[3]));
+  float sum = 0.f, f[4];
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    f[w] = (sm_m[w] == -INFINITY) ? 0.f : exp2f(sm_m[w] - mm);
+    sum += sm_l[w] * f[w];
+  }
+  const float inv = (sum > 0.f) ? 1.f / sum : 0.f;
+  uint16_t* dst = p.out + b * p.o_batch_stride + hq * p.o_head_stride;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    float v = acc[e] * f[0];
+#pragma unroll
+    for (int w = 1; w < 4; ++w) v += sm_o[w - 1][e * 32 + lane] * f[w];
+    dst[e * 32 + lane] = p.f16 ? to_16<true>(v * inv) : to_16<false>(v * inv);
+  }
+  if (lane == 0) p.lse[row] = (sum > 0.f) ? (mm + log2f(sum)) * 0.6931471805599453f : INFINITY;
+}
+
+// How the keys are shared out: by the caller's num_splits, or in equal shares over one wave of CTAs.
+void plan_decode(const sdpa_b200_params& p, int sms, DecodeParams& d) {
+  d.group = p.heads_q / p.heads_kv;
+  d.chunks = (d.group + 15) / 16;
+  d.rows = d.group < 16 ? d.group : 16;
+  d.units = p.batch * p.heads_kv * d.chunks;
+  d.tiles_per_unit = (p.max_seqlen_k + kTileKeys - 1) / kTileKeys;
+  d.num_splits = 0;
+  d.tiles_per_split = 0;
+  if (p.num_splits > 0) {
+    d.num_splits = p.num_splits > kMaxSplits ? kMaxSplits : p.num_splits;
+    d.tiles_per_split = (d.tiles_per_unit + d.num_splits - 1) / d.num_splits;
+    d.grid = d.units * d.num_splits;
+  } else {
+    const int64_t total = static_cast<int64_t>(d.units) * d.tiles_per_unit;
+    const int64_t wave = static_cast<int64_t>(kCtasPerSm) * sms;
+    d.grid = static_cast<int>(total < wave ? total : wave);
   }
 }
 
-int choose_splits(const sdpa_b200_params& p) {
-  if (p.num_splits > 0) return p.num_splits > kMaxSplits ? kMaxSplits : p.num_splits;
-  const int group = p.heads_q / p.heads_kv;
-  const int chunks = (group + 15) / 16;
-  const long units = static_cast<long>(p.batch) * p.heads_kv * chunks;
-  // about 2048 keys per split, but enough CTAs for several waves of 148 SMs x 3 CTAs
-  int splits = (p.max_seqlen_k + 2047) / 2048;
-  const long want = 4L * 148 * 3;
-  while (units * splits < want && p.max_seqlen_k / (splits * 2) >= 256) splits *= 2;
-  if (splits < 1) splits = 1;
-  if (splits > kMaxSplits) splits = kMaxSplits;
-  return splits;
+// Rows of partial results the workspace must hold (0: every unit stays whole).
+size_t partial_rows(const sdpa_b200_params& p, const DecodeParams& d) {
+  if (d.num_splits == 1) return 0;
+  if (d.num_splits > 1) return static_cast<size_t>(p.batch) * p.heads_q * d.num_splits;
+  return static_cast<size_t>(d.grid) * 2 * d.rows;
 }
+
+constexpr int kPlanSms = 160;  // workspace sizes do not ask the device: an upper bound of its SMs (148)
 
 }  // namespace
 
-size_t decode_workspace_bytes(const sdpa_b200_params& p, int* num_splits_out) {
-  const int splits = choose_splits(p);
-  if (num_splits_out) *num_splits_out = splits;
-  if (splits == 1) return 0;
-  const size_t rows = static_cast<size_t>(p.batch) * p.heads_q * splits;
-  return rows * sizeof(float) * (p.head_dim + 1) + 256;
+size_t decode_workspace_bytes(const sdpa_b200_params& p) {
+  DecodeParams d;
+  plan_decode(p, kPlanSms, d);
+  const size_t rows = partial_rows(p, d);
+  return rows == 0 ? 0 : rows * sizeof(float) * (p.head_dim + 1) + 256;
 }
 
 namespace {
 
-// Kernel arguments for one decode call; the split partials go to part_o / part_lse
-// (rows = batch * heads_q * splits slots of head_dim and of one float).
-DecodeParams fill_decode_params(const sdpa_b200_params& p, int splits, float* part_o, float* part_lse) {
-  DecodeParams d;
+template <bool kHi, int kD, bool kF16>
+cudaError_t launch_split(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const DecodeParams& d, cudaStream_t stream) {
+  constexpr uint32_t kSmem = decode_smem_bytes<kHi, kD>();
+  auto kernel = decode_splitkv_kernel<kHi, kD, kF16>;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (err != cudaSuccess) return err;
+  kernel<<<d.grid, kDecThreads, kSmem, stream>>>(tm_k, tm_v, d);
+  return cudaGetLastError();
+}
+
+template <int kD>
+cudaError_t launch_combine(const DecodeParams& d, int rows, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows);
+  cfg.blockDim = dim3(128);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, decode_combine_kernel<kD>, d);
+}
+
+// The split kernel and, where units are shared between CTAs, the merge kernel. Partial results go to `scratch`
+// (partial_rows() rows of head_dim + 1 floats).
+int launch_decode(const sdpa_b200_params& p, DecodeParams& d, float* scratch, uint32_t* status, const char* who, cudaStream_t stream) {
+  const bool f16 = p.dtype == SDPA_B200_F16;
+  const size_t rows = partial_rows(p, d);
   d.q = static_cast<const uint16_t*>(p.q);
-  d.k = static_cast<const uint16_t*>(p.k);
-  d.v = static_cast<const uint16_t*>(p.v);
   d.out = static_cast<uint16_t*>(p.out);
   d.lse = p.lse;
-  d.part_o = part_o;
-  d.part_lse = part_lse;
+  d.part_o = scratch;
+  d.part_lse = scratch + rows * p.head_dim;
+  d.status = status;
   d.q_batch_stride = p.q_batch_stride;
   d.q_head_stride = p.q_head_stride;
-  d.k_batch_stride = p.k_batch_stride;
-  d.k_head_stride = p.k_head_stride;
-  d.k_row_stride = p.k_row_stride;
-  d.v_batch_stride = p.v_batch_stride;
-  d.v_head_stride = p.v_head_stride;
-  d.v_row_stride = p.v_row_stride;
   d.o_batch_stride = p.o_batch_stride;
   d.o_head_stride = p.o_head_stride;
   d.heads_q = p.heads_q;
   d.heads_kv = p.heads_kv;
-  d.group = p.heads_q / p.heads_kv;
-  d.chunks = (d.group + 15) / 16;
   d.len_k = p.max_seqlen_k;
-  d.num_splits = splits;
   d.head_dim = p.head_dim;
-  const int kps = (p.max_seqlen_k + splits - 1) / splits;
-  d.keys_per_split = ((kps + 63) / 64) * 64;  // whole 4-warp steps
   d.scale_log2 = p.softmax_scale * 1.4426950408889634f;
-  d.f16 = p.dtype == SDPA_B200_F16;
-  return d;
-}
-
-// The split kernel and, with more than one split, the merge kernel.
-int launch_decode_pair(const DecodeParams& d, int batch, const char* who, cudaStream_t stream) {
-  dim3 grid(d.num_splits, d.heads_kv * d.chunks, batch);
-  launch_decode_kernel(d, grid, stream);
-  cudaError_t err = cudaGetLastError();
+  d.f16 = f16;
+  CUtensorMap tm_k, tm_v;
+  int st = make_tensor_map_16(f16, &tm_k, p.k, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.k_row_stride, p.k_head_stride,
+                              p.k_batch_stride, kKeysPerStep);
+  if (st != SDPA_B200_OK) return st;
+  st = make_tensor_map_16(f16, &tm_v, p.v, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.v_row_stride, p.v_head_stride,
+                          p.v_batch_stride, kKeysPerStep);
+  if (st != SDPA_B200_OK) return st;
+  const bool hi = d.rows > 8;
+  cudaError_t err;
+  if (p.head_dim == 64) {
+    err = hi ? (f16 ? launch_split<true, 64, true>(tm_k, tm_v, d, stream) : launch_split<true, 64, false>(tm_k, tm_v, d, stream))
+             : (f16 ? launch_split<false, 64, true>(tm_k, tm_v, d, stream) : launch_split<false, 64, false>(tm_k, tm_v, d, stream));
+  } else {
+    err = hi ? (f16 ? launch_split<true, 128, true>(tm_k, tm_v, d, stream) : launch_split<true, 128, false>(tm_k, tm_v, d, stream))
+             : (f16 ? launch_split<false, 128, true>(tm_k, tm_v, d, stream) : launch_split<false, 128, false>(tm_k, tm_v, d, stream));
+  }
   if (err != cudaSuccess) {
     set_error("%s: launch failed: %s", who, cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
   }
   count_launch();
-  if (d.num_splits > 1) {
-    const int nrows = batch * d.heads_q;
-    decode_combine_kernel<<<(nrows + 3) / 4, 128, 0, stream>>>(d, nrows);
-    err = cudaGetLastError();
+  // no merge when the shares' borders coincide with the units'
+  const bool shared = d.num_splits > 0 ? d.num_splits > 1 : (d.tiles_per_unit > 1 && d.units % d.grid != 0);
+  if (shared) {
+    const int out_rows = p.batch * p.heads_q;
+    err = p.head_dim == 64 ? launch_combine<64>(d, out_rows, stream) : launch_combine<128>(d, out_rows, stream);
     if (err != cudaSuccess) {
       set_error("%s merge: launch failed: %s", who, cudaGetErrorString(err));
       return SDPA_B200_LAUNCH_FAILED;
@@ -499,16 +688,21 @@ int launch_fwd_decode(const sdpa_b200_params& p, void* workspace, size_t workspa
                       cudaStream_t stream) {
   int st = check_decode_request(p);
   if (st != SDPA_B200_OK) return st;
-  int splits = 1;
-  const size_t need = decode_workspace_bytes(p, &splits);
+  const size_t need = decode_workspace_bytes(p);
   if (workspace_bytes < kWorkspaceHeaderBytes + need) {
     set_error("decode workspace too small: %zu < %zu", workspace_bytes, kWorkspaceHeaderBytes + need);
     return SDPA_B200_INVALID_ARG;
   }
-  const size_t rows = static_cast<size_t>(p.batch) * p.heads_q * splits;
-  float* ws = reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes);
-  const DecodeParams d = fill_decode_params(p, splits, ws, ws + rows * p.head_dim);
-  return launch_decode_pair(d, p.batch, "decode", stream);
+  const int sms = sm_count();
+  if (sms <= 0 || sms > kPlanSms) {
+    set_error("decode: cannot use a device with %d SMs", sms);
+    return SDPA_B200_NO_DEVICE;
+  }
+  DecodeParams d;
+  plan_decode(p, sms, d);
+  float* scratch = reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes);
+  uint32_t* status = p.device_status != nullptr ? p.device_status : static_cast<uint32_t*>(workspace);
+  return launch_decode(p, d, scratch, status, "decode", stream);
 }
 
 }  // namespace sdpa_b200
@@ -536,7 +730,8 @@ int launch_fwd_decode(const sdpa_b200_params& p, void* workspace, size_t workspa
 namespace sdpa_b200 {
 namespace {
 
-static __device__ __align__(256) unsigned char g_decode_static_scratch[SDPA_B200_STATIC_SCRATCH_BYTES];
+constexpr size_t kStaticHeaderBytes = 256;  // in front of the partials: takes a time-out when the caller gives no status word
+static __device__ __align__(256) unsigned char g_decode_static_scratch[SDPA_B200_STATIC_SCRATCH_BYTES + kStaticHeaderBytes];
 
 constexpr int kMaxDevices = 64;
 void* g_static_scratch_ptr[kMaxDevices] = {};
@@ -580,21 +775,27 @@ extern "C" SDPA_B200_API int sdpa_b200_decode_static(const sdpa_b200_params* p, 
   }
   st = check_decode_request(*p);
   if (st != SDPA_B200_OK) return st;
-  const int splits = choose_splits(*p);
-  const size_t rows = static_cast<size_t>(p->batch) * p->heads_q * splits;
-  const size_t need = rows * sizeof(float) * (p->head_dim + 1);
+  DecodeParams d;
+  plan_decode(*p, kPlanSms, d);
+  const size_t need = partial_rows(*p, d) * sizeof(float) * (p->head_dim + 1);
   if (need > SDPA_B200_STATIC_SCRATCH_BYTES) {
     set_error("decode_static: batch %d x heads_q %d x %d splits needs %zu bytes of split partials, more than the "
               "%u bytes built into the library; lower num_splits or use sdpa_b200_fwd with a workspace",
-              p->batch, p->heads_q, splits, need, static_cast<unsigned>(SDPA_B200_STATIC_SCRATCH_BYTES));
+              p->batch, p->heads_q, p->num_splits, need, static_cast<unsigned>(SDPA_B200_STATIC_SCRATCH_BYTES));
     return SDPA_B200_INVALID_ARG;
   }
   st = check_device();
   if (st != SDPA_B200_OK) return st;
+  const int sms = sm_count();
+  if (sms <= 0 || sms > kPlanSms) {
+    set_error("decode_static: cannot use a device with %d SMs", sms);
+    return SDPA_B200_NO_DEVICE;
+  }
   void* scratch = nullptr;
   st = static_scratch_address(&scratch);
   if (st != SDPA_B200_OK) return st;
-  float* part_o = static_cast<float*>(scratch);
-  const DecodeParams d = fill_decode_params(*p, splits, part_o, part_o + rows * p->head_dim);
-  return launch_decode_pair(d, p->batch, "decode_static", static_cast<cudaStream_t>(stream));
+  plan_decode(*p, sms, d);
+  uint32_t* status = p->device_status != nullptr ? p->device_status : static_cast<uint32_t*>(scratch);
+  return launch_decode(*p, d, reinterpret_cast<float*>(static_cast<char*>(scratch) + kStaticHeaderBytes), status, "decode_static",
+                       static_cast<cudaStream_t>(stream));
 }

@@ -36,7 +36,7 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
 int sm_count();
 
 // Split-KV decode forward. Workspace layout is private to decode_splitkv.cu.
-size_t decode_workspace_bytes(const sdpa_b200_params& p, int* num_splits_out);
+size_t decode_workspace_bytes(const sdpa_b200_params& p);
 int launch_fwd_decode(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes,
                       cudaStream_t stream);
 

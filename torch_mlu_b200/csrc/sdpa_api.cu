@@ -354,7 +354,7 @@ int sdpa_b200_fwd_workspace_bytes(const sdpa_b200_params* p, size_t* bytes) {
   int st = validate_common(p);
   if (st != SDPA_B200_OK) return st;
   size_t need = kWorkspaceHeaderBytes;
-  if (use_decode(p)) need += decode_workspace_bytes(*p, nullptr);
+  if (use_decode(p)) need += decode_workspace_bytes(*p);
   *bytes = need;
   return SDPA_B200_OK;
 }
@@ -382,7 +382,8 @@ int sdpa_b200_fwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
   st = check_device();
   if (st != SDPA_B200_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, s) != cudaSuccess) {
+  // the header holds the unit counter of the persistent prefill kernel and, without a device_status, the status word
+  if (!(use_decode(p) && p->device_status != nullptr) && cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, s) != cudaSuccess) {
     set_error("clearing the workspace header failed: %s", cudaGetErrorString(cudaGetLastError()));
     return SDPA_B200_LAUNCH_FAILED;
   }
