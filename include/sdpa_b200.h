@@ -156,7 +156,8 @@ typedef struct sdpa_b200_params {
    * fp32 workspace with floating-point reductions whose order varies between launches (dK and dV are still summed
    * in a fixed order); non-zero = separate dK/dV and dQ kernels with fixed summation order throughout, so that the
    * same call gives the same bits every time, at about 1.4x the time. A call with a bias always takes the second
-   * path. Ignored by the forward. */
+   * path, unless the bias is the same for every query (bias_row_stride == 0) and dbias is NULL. Ignored by the
+   * forward. */
   int32_t deterministic;
   /* Forward (tile kernel): number of SMs the persistent kernel leaves free, for a kernel that is to run beside it on
    * another stream - a collective that reassembles the previous step's outputs, say. 0 = one CTA on every SM, which

@@ -323,3 +323,38 @@ def test_backward_with_a_transposed_bias_copy_gives_the_same_gradients(cuda_devi
     for a, b in zip(plain, fast):
         assert torch.equal(a, b)
     assert ops._transposed_bias(bias[:, :, :1].expand(B, H, Lq, Lk)) is None   # no query dependence: nothing to copy
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Lq,Lk,Hq,Hkv,D,causal,shape", [
+    (130, 200, 2, 2, 64, False, (2, 1, 1, 200)),    # a key-padding mask per sequence
+    (257, 129, 4, 2, 128, False, (1, 4, 1, 129)),   # one row per query head of a group; ragged keys
+    (300, 300, 3, 1, 64, True, (2, 3, 1, 300)),
+    (2, 72, 2, 2, 96, False, (2, 2, 1, 72)),
+    (640, 513, 2, 2, 64, False, (1, 1, 1, 513)),    # five items per CTA: dQ's own buffer is reused
+])
+def test_backward_with_a_bias_that_is_the_same_for_every_query(cuda_device, native_lib, dtype, Lq, Lk, Hq, Hkv, D, causal, shape):
+    """Without a bias gradient such a call takes the fused kernel, and the two kernels where a fixed order is asked for:
+    both against autograd through the fp32 math, held to the reference suite's own rule, with hidden (-inf) keys."""
+    dev = cuda_device
+    g = torch.Generator().manual_seed(11)
+    q, k, v = (torch.randn(s, generator=g).to(dtype) for s in ((2, Hq, Lq, D), (2, Hkv, Lk, D), (2, Hkv, Lk, D)))
+    bias = torch.randn(shape, generator=g).to(dtype)
+    bias[0, 0, 0, Lk // 2:Lk // 2 + 9] = float("-inf")
+    do = torch.randn((2, Hq, Lq, D), generator=g).to(dtype)
+    qd, kd, vd = q.to(dev), k.to(dev), v.to(dev)
+    sc = ops.calculate_scale(qd, None)
+    bd = ops._prepare_bias(bias.to(dev), qd, kd)
+    assert bd.stride(2) == 0
+    out, lse = ops._dense_forward(qd, kd, vd, causal, sc, allow_gqa=True, bias=bd)
+    grads = [ops._dense_backward(do.to(dev), qd, kd, vd, out, lse, causal, sc, bias=bd, deterministic=d) for d in (False, True, True)]
+    assert ops.device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(grads[1], grads[2]))  # the fixed order is still there for the asking
+    ke, ve = (t.repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+    true = _bias_reference(q, ke, ve, bias, do, causal)
+    lowp = _bias_reference(q, ke, ve, bias, do, causal, dtype)
+    fold = lambda t: t.view(2, Hkv, Hq // Hkv, Lk, D).sum(2)
+    for got in grads[:2]:
+        for name, x, t, l, fudge in (("dq", got[0], true[2], lowp[2], 4), ("dk", got[1], fold(true[3]), fold(lowp[3]), 2),
+                                     ("dv", got[2], fold(true[4]), fold(lowp[4]), 2)):
+            orc.assert_close_reference_rule(x, t, l, name, fudge=fudge)

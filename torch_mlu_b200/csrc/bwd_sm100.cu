@@ -947,9 +947,12 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 
 }  // namespace
 
-// The fused kernel serves every call that does not ask for a fixed summation order and has no bias (the bias gradient
-// is written by the dQ kernel, whose threads own query rows).
-bool use_fused_backward(const sdpa_b200_params& p) { return p.deterministic == 0 && p.bias == nullptr; }
+// The fused kernel serves every call that does not ask for a fixed summation order and has no bias, or one that is the
+// same for every query and needs no gradient (a key-padding mask). Any other bias takes the two kernels: its gradient is
+// written by the dQ kernel, whose threads own query rows, and its values would not fit the fused kernel's registers.
+bool use_fused_backward(const sdpa_b200_params& p) {
+  return p.deterministic == 0 && (p.bias == nullptr || (p.bias_row_stride == 0 && p.dbias == nullptr));
+}
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
   const size_t bytes = 2 * static_cast<size_t>(p.batch) * p.heads_q * lq_padded(p) * sizeof(float);
