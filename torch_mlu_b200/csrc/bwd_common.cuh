@@ -65,7 +65,9 @@ struct BwdKernelParams {
 };
 
 // bwd_fused_sm100.cu: the fused kernel and the dQ conversion behind it. `grid` and the CTA-order fields of `kp` are
-// those of the dK/dV kernel (one CTA per key block); dq_acc holds bwd_fused_workspace_bytes() bytes.
+// those of the dK/dV kernel (one CTA per key block); dq_acc holds bwd_fused_workspace_bytes() bytes, the rows of existing
+// queries cleared.
+size_t bwd_fused_acc_rows(const sdpa_b200_params& p, int lq_pad);
 size_t bwd_fused_workspace_bytes(const sdpa_b200_params& p, int lq_pad);
 int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_acc, int grid, cudaStream_t stream,
                      const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,

@@ -687,17 +687,12 @@ int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_ac
   const bool f16 = p.dtype == SDPA_B200_F16;
   const int kd = p.head_dim <= 64 ? 64 : 128;
   const size_t acc_rows = bwd_fused_acc_rows(p, kp.lq_pad);
-  cudaError_t err = cudaMemsetAsync(dq_acc, 0, acc_rows * kd * sizeof(float), stream);
-  if (err != cudaSuccess) {
-    set_error("backward: clearing the dQ accumulator failed: %s", cudaGetErrorString(err));
-    return SDPA_B200_LAUNCH_FAILED;
-  }
   kp.dq_acc = dq_acc;
   kp.dq_acc_rows = p.cu_seqlens_q != nullptr ? static_cast<int>(acc_rows / p.heads_q) : 0;
   const bool drop = kp.keep_cols != nullptr, key_bias = p.bias != nullptr;
   FusedKernel kernel = drop ? (key_bias ? pick_fused<true, true>(p.head_dim, f16) : pick_fused<true, false>(p.head_dim, f16))
                             : (key_bias ? pick_fused<false, true>(p.head_dim, f16) : pick_fused<false, false>(p.head_dim, f16));
-  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmemRequest);
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmemRequest);
   if (err != cudaSuccess) {
     set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", kFSmemRequest, cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;

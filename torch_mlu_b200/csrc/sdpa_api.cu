@@ -382,8 +382,8 @@ int sdpa_b200_fwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
   st = check_device();
   if (st != SDPA_B200_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the header holds the unit counter of the persistent prefill kernel and, without a device_status, the status word
-  if (!(use_decode(p) && p->device_status != nullptr) && cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, s) != cudaSuccess) {
+  // without a device_status the header holds the status word (launch_fwd_prefill clears its unit counter there itself)
+  if (p->device_status == nullptr && cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, s) != cudaSuccess) {
     set_error("clearing the workspace header failed: %s", cudaGetErrorString(cudaGetLastError()));
     return SDPA_B200_LAUNCH_FAILED;
   }
@@ -437,7 +437,7 @@ int sdpa_b200_bwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
   st = check_device();
   if (st != SDPA_B200_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, s) != cudaSuccess) {
+  if (p->device_status == nullptr && cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, s) != cudaSuccess) {
     set_error("clearing the workspace header failed: %s", cudaGetErrorString(cudaGetLastError()));
     return SDPA_B200_LAUNCH_FAILED;
   }
