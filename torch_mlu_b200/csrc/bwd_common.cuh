@@ -115,9 +115,4 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src,
 // the overlap. (A no-op for a grid launched the ordinary way.)
 __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// both halves of a packed 16-bit pair survive or die by two keep bits (bit 0 -> low half)
-__device__ __forceinline__ uint32_t keep_pair_mask(uint32_t two_bits) {
-  return ((two_bits & 1u) ? 0x0000ffffu : 0u) | ((two_bits & 2u) ? 0xffff0000u : 0u);
-}
-
 }  // namespace sdpa_b200

@@ -462,8 +462,12 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         uint32_t pw[32];
 #pragma unroll
         for (int j2 = 0; j2 < 32; ++j2) {
-          pw[j2] = pack_16x2<kF16>(pr[2 * j2], pr[2 * j2 + 1]);
-          if constexpr (kDrop) pw[j2] &= keep_pair_mask((j2 < 16 ? keep.x : keep.y) >> ((2 * j2) & 31));
+          if constexpr (kDrop) {
+            const uint32_t word = j2 < 16 ? keep.x : keep.y;
+            pw[j2] = pack_16x2<kF16>(kept(word, (2 * j2) & 31, pr[2 * j2]), kept(word, (2 * j2 + 1) & 31, pr[2 * j2 + 1]));
+          } else {
+            pw[j2] = pack_16x2<kF16>(pr[2 * j2], pr[2 * j2 + 1]);
+          }
         }
         tmem_st_x16(sbuf, pw);
         tmem_st_x16(sbuf + 16, pw + 16);
@@ -489,13 +493,17 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         uint32_t dw[32];
 #pragma unroll
         for (int j2 = 0; j2 < 32; ++j2) {
-          float dp0 = __uint_as_float(d[2 * j2]), dp1 = __uint_as_float(d[2 * j2 + 1]);
+          const float dp0 = __uint_as_float(d[2 * j2]), dp1 = __uint_as_float(d[2 * j2 + 1]);
+          float e0, e1;  // (M o dP / (1 - p)) - delta
           if constexpr (kDrop) {
-            const uint32_t two = (j2 < 16 ? keep.x : keep.y) >> ((2 * j2) & 31);
-            dp0 = (two & 1u) ? dp0 * p.keep_scale : 0.f;
-            dp1 = (two & 2u) ? dp1 * p.keep_scale : 0.f;
+            const uint32_t word = j2 < 16 ? keep.x : keep.y;
+            e0 = fmaf(kept(word, (2 * j2) & 31, dp0), p.keep_scale, -vec_delta[2 * j2]);
+            e1 = fmaf(kept(word, (2 * j2 + 1) & 31, dp1), p.keep_scale, -vec_delta[2 * j2 + 1]);
+          } else {
+            e0 = dp0 - vec_delta[2 * j2];
+            e1 = dp1 - vec_delta[2 * j2 + 1];
           }
-          dw[j2] = pack_16x2<kF16>(pr[2 * j2] * (dp0 - vec_delta[2 * j2]), pr[2 * j2 + 1] * (dp1 - vec_delta[2 * j2 + 1]));
+          dw[j2] = pack_16x2<kF16>(pr[2 * j2] * e0, pr[2 * j2 + 1] * e1);
         }
         // the dS tile is free once dK(i-1), its last reader, is done (the commit that also releases that item's ring slots)
         if (i > 0) {

@@ -67,11 +67,6 @@ struct D256Params {
   float keep_scale;           // 1 / (1 - dropout_p)
 };
 
-// both halves of a packed 16-bit pair survive or die by two keep bits (bit 0 -> low half)
-__device__ __forceinline__ uint32_t keep_pair(uint32_t two_bits) {
-  return ((two_bits & 1u) ? 0x0000ffffu : 0u) | ((two_bits & 2u) ? 0xffff0000u : 0u);
-}
-
 template <bool kF16>
 constexpr uint32_t kIdescS64 = umma_idesc_16(kRowsA, kRowsB, false, false, kF16);   // scores: N = 64, B K-major
 template <bool kF16>
@@ -332,9 +327,13 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
         const float2 x = fma2(make_float2(s[2 * i], s[2 * i + 1]), c2, nm2);
         const float2 pr = make_float2(ex2_approx(x.x), ex2_approx(x.y));
         if (i & 1) lb = add2(lb, pr); else la = add2(la, pr);
-        pk[i] = pack_16x2<kF16>(pr.x, pr.y);
-        // the row sum keeps every pair (softmax is normalised before dropout); only P V loses the dropped ones
-        if constexpr (kDrop) pk[i] &= keep_pair((i < 16 ? keep.x : keep.y) >> ((2 * i) & 31));
+        if constexpr (kDrop) {
+          // the row sum keeps every pair (softmax is normalised before dropout); only P V loses the dropped ones
+          const uint32_t word = i < 16 ? keep.x : keep.y;
+          pk[i] = pack_16x2<kF16>(kept(word, (2 * i) & 31, pr.x), kept(word, (2 * i + 1) & 31, pr.y));
+        } else {
+          pk[i] = pack_16x2<kF16>(pr.x, pr.y);
+        }
       }
       l_run += (la.x + la.y) + (lb.x + lb.y);
       // Every phase of the PV barrier is observed, in order, and before this block's P is handed over (PV(j) cannot end
@@ -829,8 +828,8 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
       if (kMode == kDV) {
 #pragma unroll
         for (int j2 = 0; j2 < kCols / 2; ++j2) {
-          w[j2] = pack_16x2<kF16>(pr[2 * j2], pr[2 * j2 + 1]);
-          if constexpr (kDrop) w[j2] &= keep_pair(keep >> (2 * j2));
+          if constexpr (kDrop) w[j2] = pack_16x2<kF16>(kept(keep, 2 * j2, pr[2 * j2]), kept(keep, 2 * j2 + 1, pr[2 * j2 + 1]));
+          else w[j2] = pack_16x2<kF16>(pr[2 * j2], pr[2 * j2 + 1]);
         }
       } else {
         ok = __all_sync(0xffffffffu, mbar_wait(bar + kBTFull + 8 * db, seen[db] & 1u, abort_flag));
@@ -847,13 +846,16 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
         for (int j2 = 0; j2 < kCols / 2; ++j2) {
           const float dl0 = kKeys ? vec_delta[2 * j2] : my_delta;
           const float dl1 = kKeys ? vec_delta[2 * j2 + 1] : my_delta;
-          float dp0 = __uint_as_float(d[2 * j2]), dp1 = __uint_as_float(d[2 * j2 + 1]);
+          const float dp0 = __uint_as_float(d[2 * j2]), dp1 = __uint_as_float(d[2 * j2 + 1]);
+          float e0, e1;  // (M o dP / (1 - p)) - delta
           if constexpr (kDrop) {
-            const uint32_t two = keep >> (2 * j2);
-            dp0 = (two & 1u) ? dp0 * p.keep_scale : 0.f;
-            dp1 = (two & 2u) ? dp1 * p.keep_scale : 0.f;
+            e0 = fmaf(kept(keep, 2 * j2, dp0), p.keep_scale, -dl0);
+            e1 = fmaf(kept(keep, 2 * j2 + 1, dp1), p.keep_scale, -dl1);
+          } else {
+            e0 = dp0 - dl0;
+            e1 = dp1 - dl1;
           }
-          w[j2] = pack_16x2<kF16>(pr[2 * j2] * (dp0 - dl0), pr[2 * j2 + 1] * (dp1 - dl1));
+          w[j2] = pack_16x2<kF16>(pr[2 * j2] * e0, pr[2 * j2 + 1] * e1);
         }
       }
       // the 16-bit result over the front of this thread's OWN score columns (16 columns = 32 streamed rows): the other

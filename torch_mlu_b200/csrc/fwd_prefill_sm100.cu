@@ -270,11 +270,6 @@ __device__ __forceinline__ void write_unit(uint8_t* smem, uint32_t e, const Unit
   dst[3] = make_uint4(u.n_iter, u.done, 0, 0);
 }
 
-// both halves of a packed 16-bit pair survive or die by two keep bits (bit 0 -> low half)
-__device__ __forceinline__ uint32_t keep_pair_mask(uint32_t two_bits) {
-  return ((two_bits & 1u) ? 0x0000ffffu : 0u) | ((two_bits & 2u) ? 0xffff0000u : 0u);
-}
-
 template <int kD, bool kF16, bool kDrop, bool kBias>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
@@ -683,11 +678,13 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
             const float2 x = fma2(make_float2(s[cc * 16 + 2 * i], s[cc * 16 + 2 * i + 1]), c2, nm2);
             const float2 pr = make_float2(ex2_approx(x.x), ex2_approx(x.y));
             if (i & 1) lb = add2(lb, pr); else la = add2(la, pr);
-            pk[i] = pack_16x2<kF16>(pr.x, pr.y);
             if constexpr (kDrop) {
               // the row sum above keeps every pair (softmax is normalised before dropout); only P.V loses them
               const uint32_t word = (cc >> 1) == 0 ? keep.x : (cc >> 1) == 1 ? keep.y : (cc >> 1) == 2 ? keep.z : keep.w;
-              pk[i] &= keep_pair_mask(word >> ((cc & 1) * 16 + 2 * i));
+              const int bit = (cc & 1) * 16 + 2 * i;
+              pk[i] = pack_16x2<kF16>(kept(word, bit, pr.x), kept(word, bit + 1, pr.y));
+            } else {
+              pk[i] = pack_16x2<kF16>(pr.x, pr.y);
             }
           }
           if (cc == 4) {
