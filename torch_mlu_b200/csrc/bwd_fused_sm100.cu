@@ -205,8 +205,8 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (first) {
       mbar_arrive_expect_tx(full, kLoadBytes + 1024);
       const size_t vec = (static_cast<size_t>(b) * p.heads_q + hy) * p.lq_pad + static_cast<size_t>(yt) * kTile;
-      bulk_load_1d(base + kFSmemVec + (s >> 1) * 1024, p.lse2 + vec, 512, full);
-      bulk_load_1d(base + kFSmemVec + (s >> 1) * 1024 + 512, p.delta + vec, 512, full);
+      bulk_load_1d(base + kFSmemVec + (s >> 1) * 1024, p.nlse2 + vec, 512, full);
+      bulk_load_1d(base + kFSmemVec + (s >> 1) * 1024 + 512, p.ndelta + vec, 512, full);
     } else {
       mbar_arrive_expect_tx(full, kLoadBytes);
     }
@@ -424,8 +424,8 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (!ok) break;
       tc_fence_after_sync();
       FSTAMP(half, i, 1);
-      const float* vec_lse = reinterpret_cast<const float*>(smem + kFSmemVec + (i & 1) * 1024) + half * 64;
-      const float* vec_delta = vec_lse + 128;
+      const float* vec_nlse = reinterpret_cast<const float*>(smem + kFSmemVec + (i & 1) * 1024) + half * 64;
+      const float* vec_ndelta = vec_nlse + 128;
       // key xr sees query y0 + j iff xr <= y0 + j + off  <=>  j >= xr - off - y0. A row past the last key sees nothing:
       // in a packed tensor it holds the next sequence's key, whose dS must not reach this sequence's dQ.
       int j_lo = p.is_causal ? xr - causal_off - y0 - half * 64 : 0;
@@ -441,20 +441,26 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         float key_bias = 0.f;
         if constexpr (kKeyBias) key_bias = unpack_16x2<kF16>(bias_raw).x * 1.4426950408889634f;
 #pragma unroll
-        for (int j = 0; j < 64; j += 2) {
-          const float x0v = fmaf(__uint_as_float(a[j]), c, kKeyBias ? key_bias - vec_lse[j] : -vec_lse[j]);
-          const float x1v = fmaf(__uint_as_float(a[j + 1]), c, kKeyBias ? key_bias - vec_lse[j + 1] : -vec_lse[j + 1]);
-          if (((j >> 1) & 3) < SDPA_BWD_POLY_FUSED) {
-            const float2 e = exp2_poly3_x2(make_float2(x0v, x1v));
-            pr[j] = e.x;
-            pr[j + 1] = e.y;
-          } else {
-            pr[j] = ex2_approx(x0v);
-            pr[j + 1] = ex2_approx(x1v);
+        for (int j4 = 0; j4 < 16; ++j4) {
+          const float4 l = read_vec4<kDrop>(vec_nlse + 4 * j4);
+          float2 nl[2] = {make_float2(l.x, l.y), make_float2(l.z, l.w)};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = 4 * j4 + 2 * h;
+            if constexpr (kKeyBias) nl[h] = add2(nl[h], make_float2(key_bias, key_bias));
+            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl[h]);
+            if (((j >> 1) & 3) < SDPA_BWD_POLY_FUSED) {
+              const float2 e = exp2_poly3_x2(x);
+              pr[j] = e.x;
+              pr[j + 1] = e.y;
+            } else {
+              pr[j] = ex2_approx(x.x);
+              pr[j + 1] = ex2_approx(x.y);
+            }
           }
         }
         // only tiles on the causal diagonal or past the end of the keys need the element mask (queries past the end
-        // have lse2 = +inf, i.e. P = 0)
+        // have lse = +inf, i.e. P = 0)
         if (__any_sync(0xffffffffu, j_lo > 0)) {
 #pragma unroll
           for (int j = 0; j < 64; ++j) pr[j] = (j >= j_lo) ? pr[j] : 0.f;
@@ -492,18 +498,22 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         FSTAMP(half, i, 5);
         uint32_t dw[32];
 #pragma unroll
-        for (int j2 = 0; j2 < 32; ++j2) {
-          const float dp0 = __uint_as_float(d[2 * j2]), dp1 = __uint_as_float(d[2 * j2 + 1]);
-          float e0, e1;  // (M o dP / (1 - p)) - delta
-          if constexpr (kDrop) {
-            const uint32_t word = j2 < 16 ? keep.x : keep.y;
-            e0 = fmaf(kept(word, (2 * j2) & 31, dp0), p.keep_scale, -vec_delta[2 * j2]);
-            e1 = fmaf(kept(word, (2 * j2 + 1) & 31, dp1), p.keep_scale, -vec_delta[2 * j2 + 1]);
-          } else {
-            e0 = dp0 - vec_delta[2 * j2];
-            e1 = dp1 - vec_delta[2 * j2 + 1];
+        for (int j4 = 0; j4 < 16; ++j4) {
+          const float4 l = read_vec4<kDrop>(vec_ndelta + 4 * j4);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = 4 * j4 + 2 * h;
+            const float2 nd = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
+            float2 e = make_float2(__uint_as_float(d[j]), __uint_as_float(d[j + 1]));
+            if constexpr (kDrop) {  // M o dP / (1 - p) in the place of dP
+              const uint32_t word = j < 32 ? keep.x : keep.y;
+              e.x = pr[j] * fmaf(kept(word, j & 31, e.x), p.keep_scale, nd.x);
+              e.y = pr[j + 1] * fmaf(kept(word, (j + 1) & 31, e.y), p.keep_scale, nd.y);
+            } else {
+              e = mul2(make_float2(pr[j], pr[j + 1]), add2(e, nd));
+            }
+            dw[j >> 1] = pack_16x2<kF16>(e.x, e.y);
           }
-          dw[j2] = pack_16x2<kF16>(pr[2 * j2] * e0, pr[2 * j2 + 1] * e1);
         }
         // the dS tile is free once dK(i-1), its last reader, is done (the commit that also releases that item's ring slots)
         if (i > 0) {

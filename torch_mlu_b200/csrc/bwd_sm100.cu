@@ -199,8 +199,8 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (kMode == kModeDKDV && first) {
           mbar_arrive_expect_tx(full, kLoadBytes + 1024);
           const size_t vec = (static_cast<size_t>(b) * p.heads_q + hy) * p.lq_pad + static_cast<size_t>(yt) * kTile;
-          bulk_load_1d(base + kSmemVec + s * 1024, p.lse2 + vec, 512, full);
-          bulk_load_1d(base + kSmemVec + s * 1024 + 512, p.delta + vec, 512, full);
+          bulk_load_1d(base + kSmemVec + s * 1024, p.nlse2 + vec, 512, full);
+          bulk_load_1d(base + kSmemVec + s * 1024 + 512, p.ndelta + vec, 512, full);
         } else {
           mbar_arrive_expect_tx(full, kLoadBytes);
         }
@@ -454,11 +454,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t lane_base = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * 64;
     const float c = p.scale_log2;
     bool ok = true;
-    float my_lse2 = 0.f, my_delta = 0.f;
+    float my_nlse2 = 0.f, my_ndelta = 0.f;
     if (kMode == kModeDQ) {
       const size_t vec = (static_cast<size_t>(b) * p.heads_q + hx) * p.lq_pad + xr;
-      my_lse2 = p.lse2[vec];
-      my_delta = p.delta[vec];
+      my_nlse2 = p.nlse2[vec];
+      my_ndelta = p.ndelta[vec];
     }
     for (int i = 0; i < n_items; ++i) {
       const int s = (2 * i) % kStages;  // ring slot of Y1(i), which carries the per-query vectors
@@ -550,8 +550,8 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!ok) break;
       tc_fence_after_sync();
       BWD_STAMP(half, i, 1);
-      const float* vec_lse = reinterpret_cast<const float*>(smem + kSmemVec + s * 1024) + half * 64;
-      const float* vec_delta = vec_lse + 128;
+      const float* vec_nlse = reinterpret_cast<const float*>(smem + kSmemVec + s * 1024) + half * 64;
+      const float* vec_ndelta = vec_nlse + 128;
       // visibility of element (row xr, column y0 + j)
       //   dK/dV: key xr, query y0+j : visible iff xr <= y0 + j + off  <=>  j >= xr - off - y0
       //   dQ   : query xr, key y0+j : visible iff y0 + j <= xr + off and y0 + j < len_k
@@ -615,18 +615,20 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // pair in four is the measured optimum (two of four already cost time), here two of four.
         constexpr int kPolyOf4 = (kMode == kModeDKDV) ? SDPA_BWD_POLY_DKDV : SDPA_BWD_POLY_DQ;
 #pragma unroll
-        for (int j = 0; j < 64; j += 2) {
-          const float l0 = (kMode == kModeDKDV) ? vec_lse[j] : my_lse2;
-          const float l1 = (kMode == kModeDKDV) ? vec_lse[j + 1] : my_lse2;
-          const float x0 = fmaf(__uint_as_float(a[j]), c, -l0);
-          const float x1 = fmaf(__uint_as_float(a[j + 1]), c, -l1);
-          if (((j >> 1) & 3) < kPolyOf4) {
-            const float2 e = exp2_poly3_x2(make_float2(x0, x1));
-            pr[j] = e.x;
-            pr[j + 1] = e.y;
-          } else {
-            pr[j] = ex2_approx(x0);
-            pr[j + 1] = ex2_approx(x1);
+        for (int j4 = 0; j4 < 16; ++j4) {
+          const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = 4 * j4 + 2 * h;
+            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w));
+            if (((j >> 1) & 3) < kPolyOf4) {
+              const float2 e = exp2_poly3_x2(x);
+              pr[j] = e.x;
+              pr[j + 1] = e.y;
+            } else {
+              pr[j] = ex2_approx(x.x);
+              pr[j + 1] = ex2_approx(x.y);
+            }
           }
         }
         // only tiles on the causal diagonal or past the end of the keys need the element mask
@@ -670,20 +672,22 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         BWD_STAMP(half, i, 5);
         uint32_t dw[32];
 #pragma unroll
-        for (int j2 = 0; j2 < 32; ++j2) {
-          const float dl0 = (kMode == kModeDKDV) ? vec_delta[2 * j2] : my_delta;
-          const float dl1 = (kMode == kModeDKDV) ? vec_delta[2 * j2 + 1] : my_delta;
-          const float dp0 = __uint_as_float(d[2 * j2]), dp1 = __uint_as_float(d[2 * j2 + 1]);
-          float e0, e1;  // (M o dP / (1 - p)) - delta
-          if constexpr (kDrop) {
-            const uint32_t word = j2 < 16 ? keep.x : keep.y;
-            e0 = fmaf(kept(word, (2 * j2) & 31, dp0), p.keep_scale, -dl0);
-            e1 = fmaf(kept(word, (2 * j2 + 1) & 31, dp1), p.keep_scale, -dl1);
-          } else {
-            e0 = dp0 - dl0;
-            e1 = dp1 - dl1;
+        for (int j4 = 0; j4 < 16; ++j4) {
+          const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_ndelta + 4 * j4) : make_float4(my_ndelta, my_ndelta, my_ndelta, my_ndelta);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = 4 * j4 + 2 * h;
+            const float2 nd = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
+            float2 e = make_float2(__uint_as_float(d[j]), __uint_as_float(d[j + 1]));
+            if constexpr (kDrop) {  // M o dP / (1 - p) in the place of dP
+              const uint32_t word = j < 32 ? keep.x : keep.y;
+              e.x = pr[j] * fmaf(kept(word, j & 31, e.x), p.keep_scale, nd.x);
+              e.y = pr[j + 1] * fmaf(kept(word, (j + 1) & 31, e.y), p.keep_scale, nd.y);
+            } else {
+              e = mul2(make_float2(pr[j], pr[j + 1]), add2(e, nd));
+            }
+            dw[j >> 1] = pack_16x2<kF16>(e.x, e.y);
           }
-          dw[j2] = pack_16x2<kF16>(pr[2 * j2] * e0, pr[2 * j2 + 1] * e1);
         }
         tmem_st_x16(sbuf + 32, dw);
         tmem_st_x16(sbuf + 48, dw + 16);
@@ -815,14 +819,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (kMode == kModeDQ && threadIdx.x == 0) wait_for_previous_grid();
 }
 
-// delta[row] = sum_d dO[row,d] * O[row,d]; lse2[row] = lse[row] * log2(e);
-// rows padded to lq_pad per (batch, head): padding rows get lse2 = +inf, delta = 0.
+// ndelta[row] = -sum_d dO[row,d] * O[row,d]; nlse2[row] = -lse[row] * log2(e);
+// rows padded to lq_pad per (batch, head): padding rows get nlse2 = -inf, ndelta = 0.
 struct PreParams {
   const uint16_t* out;
   const uint16_t* dout;
   const float* lse;
-  float* lse2;
-  float* delta;
+  float* nlse2;
+  float* ndelta;
   const int32_t* cu_q;
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int64_t do_batch_stride, do_head_stride, do_row_stride;
@@ -900,11 +904,11 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
       if (row < len_q) {
         const float lse = (p.cu_q != nullptr) ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + row]
                                               : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + row];
-        p.lse2[dst] = lse * 1.4426950408889634f;  // +inf stays +inf
-        p.delta[dst] = acc;
+        p.nlse2[dst] = lse * -1.4426950408889634f;
+        p.ndelta[dst] = -acc;
       } else {
-        p.lse2[dst] = INFINITY;
-        p.delta[dst] = 0.f;
+        p.nlse2[dst] = -INFINITY;
+        p.ndelta[dst] = 0.f;
       }
     }
   }
@@ -992,15 +996,15 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   const bool varlen = p.cu_seqlens_q != nullptr;
   const int lq_pad = lq_padded(p);
   const size_t vec_elems = static_cast<size_t>(p.batch) * p.heads_q * lq_pad;
-  float* lse2 = reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes);
-  float* delta = lse2 + vec_elems;
+  float* nlse2 = reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes);
+  float* ndelta = nlse2 + vec_elems;
 
   PreParams pre;
   pre.out = static_cast<const uint16_t*>(p.out);
   pre.dout = static_cast<const uint16_t*>(p.dout);
   pre.lse = p.lse;
-  pre.lse2 = lse2;
-  pre.delta = delta;
+  pre.nlse2 = nlse2;
+  pre.ndelta = ndelta;
   pre.cu_q = p.cu_seqlens_q;
   pre.o_batch_stride = p.o_batch_stride;
   pre.o_head_stride = p.o_head_stride;
@@ -1057,8 +1061,8 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
     return st;
 
   BwdKernelParams kp;
-  kp.lse2 = lse2;
-  kp.delta = delta;
+  kp.nlse2 = nlse2;
+  kp.ndelta = ndelta;
   kp.dq = static_cast<uint16_t*>(p.dq);
   kp.dk = static_cast<uint16_t*>(p.dk);
   kp.dv = static_cast<uint16_t*>(p.dv);

@@ -905,7 +905,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   const int usable = sms - p.sm_margin > 1 ? sms - p.sm_margin : 1;
   dim3 grid(kp.num_slots < usable ? kp.num_slots : usable, 1, 1);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
-  // launch that clears it, a fifth of the smallest calls' time, is left out. (Without a device_status the header has been
+  // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
   // cleared already.)
   kp.unit_counter = nullptr;
   if (kp.num_slots > usable) {

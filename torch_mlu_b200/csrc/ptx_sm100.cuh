@@ -92,6 +92,20 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   return d;
 }
 
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t"
+      ".reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\t"
+      "mov.b64 rb, {%4, %5};\n\t"
+      "mul.rn.f32x2 rd, ra, rb;\n\t"
+      "mov.b64 {%0, %1}, rd;\n\t"
+      "}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 // 2^x for two values on the FMA pipe instead of the exponential unit (4 results/clk/SMSP, the scarce
 // resource of the backward's recomputation). x is clamped to >= -125, split as n + f with n = round(x),
 // |f| <= 0.5 (adding 1.5*2^23 leaves n in the low mantissa bits), 2^f is a cubic with relative error
