@@ -160,3 +160,23 @@ def test_dropout_with_head_dims_above_128(cuda_device, native_lib, B, Hq, Hkv, L
     orc.assert_close_grad_bf16(dq, qf.grad, "dq")
     orc.assert_close_grad_bf16(dk, kf.grad, "dk")
     orc.assert_close_grad_bf16(dv, vf.grad, "dv")
+
+
+@pytest.mark.parametrize("D,G,Lq,Lk,causal", [
+    (256, 1, 65, 130, False),    # two streamed items per key tile, three per query tile
+    (256, 1, 192, 64, False),    # three; one
+    (256, 3, 64, 129, True),     # three items of one block in three heads
+    (200, 2, 193, 320, False),   # eight in two heads; padded columns in the second half of every block
+    (256, 1, 449, 577, False),   # the rings wrap several times
+    (256, 1, 700, 700, True),    # every count from two to eleven
+])
+def test_backward_item_counts(cuda_device, native_lib, D, G, Lq, Lk, causal):
+    """Item counts around the lengths of the streamed rings (three whole and three half blocks). Tolerances as above."""
+    dev = cuda_device
+    q, k, v, dout = rand((1, 2 * G, Lq, D), 1), rand((1, 2, Lk, D), 2), rand((1, 2, Lk, D), 3), rand((1, 2 * G, Lq, D), 4)
+    qd, kd, vd, dd = q.to(dev), k.to(dev), v.to(dev), dout.to(dev)
+    out, lse = ops.gqa_prefill(qd, kd, vd, is_causal=causal)
+    grads = ops._dense_backward(dd, qd, kd, vd, out, lse, causal, D ** -0.5)
+    assert ops.device_status() == 0
+    o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=causal)
+    check_grads(grads, orc.cpu_sdpa_backward(dout, q, k, v, o_ref, l_ref, causal=causal))
