@@ -199,3 +199,36 @@ def test_reference_tests_own_tolerance_rule(cuda_device, native_lib, dtype, B, H
     orc.assert_close_reference_rule(dq, g_true[0], g_lp[0], "dq", fudge=4)
     orc.assert_close_reference_rule(dk, g_true[1], g_lp[1], "dk")
     orc.assert_close_reference_rule(dv, g_true[2], g_lp[2], "dv")
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,D,causal", [
+    ([200, 200], 38, 38, 128, True),          # dense, one key block past a tile, 152 key blocks
+    ([129, 129], 74, 37, 128, False),         # dense, grouped queries: 148 key blocks, one short of the fused kernel
+    ([257, 257], 100, 25, 64, True),          # dense, grouped queries at head_dim 64: 150
+    ([1, 300, 513, 64], 32, 8, 128, True),    # packed, grouped queries
+    ([70, 700, 129], 16, 16, 64, True),       # packed, ragged ends, most tiles of the grid empty
+    ([513, 2, 385], 12, 12, 104, False),      # packed, padded head_dim: 180
+])
+def test_backward_on_both_sides_of_the_dispatch(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
+    """Calls with more key blocks than SMs, which the fused kernel serves (except grouped queries at head_dim 128), and calls
+    just below, against the oracle; dense ones in the fixed order too; tolerances as above."""
+    dev = cuda_device
+    total, cu = sum(lens), [sum(lens[:i]) for i in range(len(lens) + 1)]
+    q, k, v, dout = rand((total, Hq, D), 1), rand((total, Hkv, D), 2), rand((total, Hkv, D), 3), rand((total, Hq, D), 4)
+    want = orc.varlen_backward(dout, q, k, v, cu, cu, causal=causal)
+    qd, kd, vd, dd = (t.to(dev) for t in (q, k, v, dout))
+    if len(set(lens)) == 1:
+        split = lambda t: t.view(len(lens), lens[0], -1, D).transpose(1, 2)
+        qd, kd, vd, dd = (split(t) for t in (qd, kd, vd, dd))
+        out, lse = ops.gqa_prefill(qd, kd, vd, is_causal=causal)
+        run = lambda det: [t.transpose(1, 2).reshape(total, -1, D)
+                           for t in ops._dense_backward(dd, qd, kd, vd, out, lse, causal, D ** -0.5, deterministic=det)]
+    else:
+        cu_t = torch.tensor(cu, dtype=torch.int32, device=dev)
+        out, lse, seed, off, _ = ops._flash_attention_forward(qd, kd, vd, cu_t, cu_t, max(lens), max(lens), 0.0, causal, False)
+        run = lambda _: ops._flash_attention_backward(dd, qd, kd, vd, out, lse, cu_t, cu_t, max(lens), max(lens), 0.0, causal,
+                                                      seed, off)
+    check_grads(run(False), want)
+    if len(set(lens)) == 1:
+        check_grads(run(True), want)
+    assert ops.device_status() == 0

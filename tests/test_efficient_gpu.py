@@ -327,15 +327,16 @@ def test_backward_with_a_transposed_bias_copy_gives_the_same_gradients(cuda_devi
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("Lq,Lk,Hq,Hkv,D,causal,shape", [
-    (130, 200, 2, 2, 64, False, (2, 1, 1, 200)),    # a key-padding mask per sequence
-    (257, 129, 4, 2, 128, False, (1, 4, 1, 129)),   # one row per query head of a group; ragged keys
-    (300, 300, 3, 1, 64, True, (2, 3, 1, 300)),
-    (2, 72, 2, 2, 96, False, (2, 2, 1, 72)),
-    (640, 513, 2, 2, 64, False, (1, 1, 1, 513)),    # five items per CTA: dQ's own buffer is reused
+    (130, 200, 40, 40, 64, False, (2, 1, 1, 200)),    # a key-padding mask per sequence
+    (257, 129, 80, 40, 128, False, (1, 80, 1, 129)),  # one row per query head of a group; ragged keys
+    (300, 300, 75, 25, 64, True, (2, 75, 1, 300)),
+    (2, 72, 80, 80, 96, False, (2, 80, 1, 72)),
+    (640, 513, 15, 15, 64, False, (1, 1, 1, 513)),    # five items per CTA
+    (130, 200, 2, 2, 64, False, (2, 1, 1, 200)),      # fewer key blocks than SMs: the two kernels
 ])
 def test_backward_with_a_bias_that_is_the_same_for_every_query(cuda_device, native_lib, dtype, Lq, Lk, Hq, Hkv, D, causal, shape):
-    """Without a bias gradient such a call takes the fused kernel, and the two kernels where a fixed order is asked for:
-    both against autograd through the fp32 math, held to the reference suite's own rule, with hidden (-inf) keys."""
+    """Without a bias gradient such a call takes the fused kernel from more key blocks than SMs on, and the two kernels where a
+    fixed order is asked for: both against autograd through the fp32 math, held to the reference suite's own rule, with hidden (-inf) keys."""
     dev = cuda_device
     g = torch.Generator().manual_seed(11)
     q, k, v = (torch.randn(s, generator=g).to(dtype) for s in ((2, Hq, Lq, D), (2, Hkv, Lk, D), (2, Hkv, Lk, D)))

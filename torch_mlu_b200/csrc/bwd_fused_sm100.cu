@@ -20,8 +20,9 @@
 // the accumulator; with every SM sending them, the L2 takes about 20 bytes per clock and SM (a stand-alone test reaches
 // 5.5 TB/s = 706 floats per clock over the chip with red.v4 and with cp.reduce.async.bulk alike, 3.6 TB/s once the
 // accumulator exceeds L2), i.e. ~3400 cycles per item against 2560 cycles of tensor work, and a reduce warp needs
-// ~90 cycles per red.v4. Item period ~5600 cycles: level with the two-kernel path on B8 H16 L2048 causal (0.540 ms
-// against 0.536 ms for the whole backward), 5-9 % ahead at L = 8192 causal and at large unmasked shapes.
+// ~90 cycles per red.v4. With the issuers at the pipe's rate and packed arithmetic the kernel takes 438 us at B8 H16 L2048
+// causal, whether none or three quarters of the exponentials run on the FMA pipe: the compute warps no longer bound it.
+// When it is the faster path, with figures: use_fused_backward() in bwd_sm100.cu.
 //
 // TMEM (512 columns): T1 [0,128) T2 [128,256) dV [256,384) dK [384,512). Item i has S in T[i&1] and dP in the other
 // buffer. Life of one buffer: S(i) -> P(i) (16-bit, front of each half) -> dQ(i) -> dP(i+1) -> S(i+2) ...:

@@ -973,11 +973,24 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 
 }  // namespace
 
-// The fused kernel serves every call that does not ask for a fixed summation order and has no bias, or one that is the
-// same for every query and needs no gradient (a key-padding mask). Any other bias takes the two kernels: its gradient is
-// written by the dQ kernel, whose threads own query rows, and its values would not fit the fused kernel's registers.
+// Fused kernel or the two with a fixed summation order? A bias with a query dependence or a gradient always takes the two (the
+// gradient is written by the dQ kernel, whose threads own query rows). Otherwise (us, back-to-back calls, fused | two):
+//  * up to one CTA per SM, fused leaves SMs idle for a whole chain of items, while the two kernels run side by side and need
+//    no clearing and no conversion: two. (B1 H8 L300 D128 31.9 | 22.0, B2 H8 L700 D64 26.6 | 20.5, B4 H8/1 L4096 D128 812 | 564,
+//    B1 H12 L200 with a padding mask 24.7 | 17.0, B4 H8 L500 D64 31.8 | 30.4)
+//  * head_dim 128 with grouped queries: a fused CTA chains the items of every query head of its group: two. (B8 H32/8 L2048
+//    causal 1125 | 1097; packed 12 x 64..2048 H16/4, whole step 420 | 408). Not with dropout, whose masks the two expand twice.
+//  * else fused: at head_dim 64 its items are cheap against the second pass over the scores (B8 H16 L2048 387 | 438, B16 H8 L300
+//    47 | 51); at 128 it is level, and under the power cap its 5 GEMMs for 7 decide (whole step B8 H16 L2048 769 | 776, with
+//    dropout 660 | 677; B2 H16 L8192 1758 | 1747).
+// The number of SMs is the B200's, not the current device's: workspace queries and launches must agree.
 bool use_fused_backward(const sdpa_b200_params& p) {
-  return p.deterministic == 0 && (p.bias == nullptr || (p.bias_row_stride == 0 && p.dbias == nullptr));
+  if (p.deterministic != 0) return false;
+  if (p.bias != nullptr && (p.bias_row_stride != 0 || p.dbias != nullptr)) return false;
+  constexpr int64_t kSms = 148;
+  const int64_t ctas = static_cast<int64_t>(p.batch) * p.heads_kv * ((static_cast<int64_t>(p.max_seqlen_k) + kTile - 1) / kTile);
+  if (ctas <= kSms) return false;
+  return p.head_dim <= 64 || p.heads_q == p.heads_kv || p.bias != nullptr || p.dropout_p > 0.f;
 }
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
