@@ -202,3 +202,29 @@ def test_decode_writes_nothing_outside_its_outputs(cuda_device, native_lib, D, s
     out2.assert_bands_intact("decode_static out")
     lse2.assert_bands_intact("decode_static lse")
     assert torch.equal(out2.view, out.view) and torch.equal(lse2.view, lse.view)
+
+
+def test_backward_with_a_key_bias_in_a_workspace_without_accumulator(cuda_device, native_lib):
+    """A workspace sized as for the two kernels is accepted for a bias that is the same for every query, and gives their bits."""
+    dev = cuda_device
+    q, k, v, dout = (rand((2, 40, 200, 64), s).to(dev) for s in (1, 2, 3, 4))
+    bias = torch.zeros(2, 1, 1, 200, device=dev, dtype=torch.bfloat16)
+    bias[1, ..., 150:] = float("-inf")
+    bias = bias.expand(2, 40, 200, 200)
+    out, lse = ops._dense_forward(q, k, v, False, 0.125, allow_gqa=True, bias=bias)
+    want = ops._dense_backward(dout, q, k, v, out, lse, False, 0.125, bias=bias, deterministic=True)
+    grads = [torch.empty_like(t) for t in (q, k, v)]
+    p = ops._dense_params(q, k, v, out, lse, False, 0.125)
+    set_bwd(p, dout, *grads, packed=False)
+    ops._set_bias(p, bias)
+    sizes = []
+    for p.deterministic in (1, 0):
+        need = ctypes.c_size_t(0)
+        _cabi.check(native_lib.sdpa_b200_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(need)), "workspace query")
+        sizes.append(need.value)
+    assert sizes[0] < sizes[1]
+    ws = torch.empty(sizes[0], dtype=torch.uint8, device=dev)
+    _cabi.check(native_lib.sdpa_b200_bwd(ctypes.byref(p), ws.data_ptr(), sizes[0], torch.cuda.current_stream(dev).cuda_stream), "bwd")
+    torch.cuda.synchronize(dev)
+    for got, ref in zip(grads, want):
+        assert torch.equal(got, ref)

@@ -998,13 +998,21 @@ size_t bwd_vector_bytes(const sdpa_b200_params& p) {
   return (bytes + 255) / 256 * 256;
 }
 
+// lse2 and delta, then the fp32 dQ accumulator of the fused kernel: for every call without a bias that does not ask for a fixed
+// order, whatever path its sizes take, so that one workspace serves calls that differ in dropout or sizes.
+size_t bwd_workspace_required(const sdpa_b200_params& p) {
+  const bool acc = p.deterministic == 0 && p.bias == nullptr;
+  return bwd_vector_bytes(p) + (acc ? bwd_fused_workspace_bytes(p, lq_padded(p)) : 0);
+}
+
+// What a workspace query answers. A call with a bias that the fused kernel can take is better off with the accumulator, but
+// runs in the two kernels without it.
 size_t bwd_workspace_bytes(const sdpa_b200_params& p) {
-  // lse2 and delta, then (fused kernel) the fp32 dQ accumulator
-  return bwd_vector_bytes(p) + (use_fused_backward(p) ? bwd_fused_workspace_bytes(p, lq_padded(p)) : 0);
+  return p.bias != nullptr && use_fused_backward(p) ? bwd_vector_bytes(p) + bwd_fused_workspace_bytes(p, lq_padded(p))
+                                                    : bwd_workspace_required(p);
 }
 
 int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  (void)workspace_bytes;
   const bool f16 = p.dtype == SDPA_B200_F16;
   const bool varlen = p.cu_seqlens_q != nullptr;
   const int lq_pad = lq_padded(p);
@@ -1030,7 +1038,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   pre.heads_q = p.heads_q;
   pre.lq_pad = lq_pad;
   pre.head_dim = p.head_dim;
-  const bool fused = use_fused_backward(p);
+  const bool fused = use_fused_backward(p) && workspace_bytes >= kWorkspaceHeaderBytes + bwd_workspace_bytes(p);
   float* dq_acc = fused ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p)) : nullptr;
   pre.dq_acc = dq_acc;
   pre.dq_acc_rows = fused && varlen ? static_cast<int>(bwd_fused_acc_rows(p, lq_pad) / p.heads_q) : 0;
