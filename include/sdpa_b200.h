@@ -156,8 +156,7 @@ typedef struct sdpa_b200_params {
    * its dQ contributions into an fp32 workspace with floating-point reductions whose order varies between launches (dK
    * and dV are still summed in a fixed order), or the separate dK/dV and dQ kernels with a fixed summation order
    * throughout. Non-zero = always the latter, so that the same call gives the same bits every time. A call with a bias
-   * always takes the latter too, unless the bias is the same for every query (bias_row_stride == 0) and dbias is NULL.
-   * Ignored by the forward. */
+   * always takes the latter too. Ignored by the forward. */
   int32_t deterministic;
   /* Forward (tile kernel): number of SMs the persistent kernel leaves free, for a kernel that is to run beside it on
    * another stream - a collective that reassembles the previous step's outputs, say. 0 = one CTA on every SM, which

@@ -123,10 +123,7 @@ __device__ __forceinline__ size_t dq_acc_index(size_t row) {
   return (row >> 7) * (static_cast<size_t>(kD / 4) * 512) + (row & 127) * 4;
 }
 
-// kKeyBias: an additive bias that does not depend on the query (a key-padding mask, ALiBi-like slopes): a thread owns a
-// key, so it is one value per thread and head, added to the exponent. B8 H12 L512 D64 with a padding mask: 45.5 us and 8 for
-// the accumulator, where the two kernels with general bias loads take 81.
-template <int kD, bool kF16, bool kDrop, bool kKeyBias>
+template <int kD, bool kF16, bool kDrop>
 __global__ void __launch_bounds__(kFThreads, 1)
 bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -414,9 +411,6 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                               (p.keep_lq_pad >> 5);
         keep = *reinterpret_cast<const uint2*>(words + ((y0 + half * 64) >> 5));
       }
-      uint16_t bias_raw = 0;
-      if constexpr (kKeyBias)
-        if (xr < len_k) bias_raw = p.bias[b * p.bias_batch_stride + (hx * p.kv_group + hi) * p.bias_head_stride + xr];
       // `ok` is made warp-uniform after every wait: the warp-level arrivals below need all 32 lanes
       FSTAMP(half, i, 0);
       ok = mbar_wait(bar + kFBarSFull, i & 1, abort_flag) &&
@@ -439,17 +433,13 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tmem_ld_x64(sbuf, a);
         tmem_wait_ld();
         FSTAMP(half, i, 2);
-        float key_bias = 0.f;
-        if constexpr (kKeyBias) key_bias = unpack_16x2<kF16>(bias_raw).x * 1.4426950408889634f;
 #pragma unroll
         for (int j4 = 0; j4 < 16; ++j4) {
           const float4 l = read_vec4<kDrop>(vec_nlse + 4 * j4);
-          float2 nl[2] = {make_float2(l.x, l.y), make_float2(l.z, l.w)};
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int j = 4 * j4 + 2 * h;
-            if constexpr (kKeyBias) nl[h] = add2(nl[h], make_float2(key_bias, key_bias));
-            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl[h]);
+            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w));
             if (((j >> 1) & 3) < SDPA_BWD_POLY_FUSED) {
               const float2 e = exp2_poly3_x2(x);
               pr[j] = e.x;
@@ -681,10 +671,10 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const DqConvertPara
 using FusedKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                              const CUtensorMap, const BwdKernelParams);
 
-template <bool kDrop, bool kKeyBias>
+template <bool kDrop>
 FusedKernel pick_fused(int head_dim, bool f16) {
-  if (head_dim <= 64) return f16 ? bwd_fused_kernel<64, true, kDrop, kKeyBias> : bwd_fused_kernel<64, false, kDrop, kKeyBias>;
-  return f16 ? bwd_fused_kernel<128, true, kDrop, kKeyBias> : bwd_fused_kernel<128, false, kDrop, kKeyBias>;
+  if (head_dim <= 64) return f16 ? bwd_fused_kernel<64, true, kDrop> : bwd_fused_kernel<64, false, kDrop>;
+  return f16 ? bwd_fused_kernel<128, true, kDrop> : bwd_fused_kernel<128, false, kDrop>;
 }
 
 }  // namespace
@@ -708,9 +698,7 @@ int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_ac
   const size_t acc_rows = bwd_fused_acc_rows(p, kp.lq_pad);
   kp.dq_acc = dq_acc;
   kp.dq_acc_rows = p.cu_seqlens_q != nullptr ? static_cast<int>(acc_rows / p.heads_q) : 0;
-  const bool drop = kp.keep_cols != nullptr, key_bias = p.bias != nullptr;
-  FusedKernel kernel = drop ? (key_bias ? pick_fused<true, true>(p.head_dim, f16) : pick_fused<true, false>(p.head_dim, f16))
-                            : (key_bias ? pick_fused<false, true>(p.head_dim, f16) : pick_fused<false, false>(p.head_dim, f16));
+  FusedKernel kernel = kp.keep_cols != nullptr ? pick_fused<true>(p.head_dim, f16) : pick_fused<false>(p.head_dim, f16);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmemRequest);
   if (err != cudaSuccess) {
     set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", kFSmemRequest, cudaGetErrorString(err));

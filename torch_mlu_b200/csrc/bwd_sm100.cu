@@ -45,7 +45,11 @@ constexpr uint32_t kSmemY = 2 * kTileBytes;                      // stages x 32 
 __host__ __device__ constexpr uint32_t smem_vec_off(int mode) { return kSmemY + stages_for(mode) * kTileBytes; }
 // per-slot (lse2[128], delta[128]), dK/dV only
 __host__ __device__ constexpr uint32_t smem_bar_off(int mode) { return smem_vec_off(mode) + (mode == 1 ? 0 : stages_for(mode) * 1024); }
-__host__ __device__ constexpr uint32_t smem_bytes_for(int mode) { return smem_bar_off(mode) + 256 + 1024; }
+// behind the barriers, dQ with a key bias only: 64 16-bit bias values per compute warp
+__host__ __device__ constexpr uint32_t smem_key_bias_off(int mode) { return smem_bar_off(mode) + 256; }
+__host__ __device__ constexpr uint32_t smem_bytes_for(int mode, bool key_bias) {
+  return smem_key_bias_off(mode) + (mode == 1 && key_bias ? 8 * 128 : 0) + 1024;
+}
 constexpr uint32_t kBarXFull = 0;
 constexpr uint32_t kBarYFull = 8;
 constexpr uint32_t kBarYEmpty = kBarYFull + 8 * kMaxStages;
@@ -73,7 +77,14 @@ constexpr uint32_t kSmemAbort = kSmemTmemPtr + 4;
 #define BWD_STAMP(role, item, ev) do {} while (0)
 #endif
 
-template <int kMode, int kD, bool kF16, bool kDrop, bool kBias>
+// What a tile kernel instance does about an additive bias. kKeyBias: one that is the same for every query (a key-padding mask,
+// ALiBi-like slopes) and whose gradient nobody wants. It joins the per-row addend of the exponent: one value per thread in the
+// dK/dV kernel; in the dQ kernel 64 values per warp and item, fetched as one word per lane under the waits and read back
+// as broadcasts. The general loads keep 32 more registers alive per thread. Backward of B8 H12 L512 D64 with a padding mask, all
+// launches: 61.5 us; in the fused kernel, whose dQ varies in its last bits from call to call, 60.3.
+enum BiasKind { kNoBias = 0, kFullBias = 1, kKeyBias = 2 };
+
+template <int kMode, int kD, bool kF16, bool kDrop, int kBias>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -481,7 +492,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                                     (p.keep_lq_pad >> 5);
         keep = *reinterpret_cast<const uint2*>(words + ((y0 + half * 64) >> 5));
       }
-      if constexpr (kBias) {
+      uint32_t key_bias_raw = 0u;  // dK/dV: this key's value; dQ: the values of two of the 64 keys
+      if constexpr (kBias == kKeyBias) {
+        const uint16_t* head = p.bias + b * p.bias_batch_stride + (kMode == kModeDQ ? hx : hx * p.kv_group + hi) * p.bias_head_stride;
+        const int key = y0 + half * 64 + 2 * lane;
+        if (kMode == kModeDQ && key < len_k) key_bias_raw = *reinterpret_cast<const uint32_t*>(head + key);
+        if (kMode == kModeDKDV && xr < len_k) key_bias_raw = head[xr];
+      }
+      if constexpr (kBias == kFullBias) {
         // the next item's bias values of this thread's row: into L2 now (dQ: 128 contiguous bytes of the query
         // row; dK/dV: 64 query rows, two per lane, 64 bytes each around this warp's keys)
         if (i + 1 < n_items && xr < len_x) {
@@ -495,9 +513,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               prefetch_l2(nx + min(63, len_k - 1 - cn));
             }
           } else {
-            if (p.bias_row_stride == 0) {
-              // one value per key: nothing worth fetching ahead
-            } else if (p.bias_t != nullptr) {
+            if (p.bias_t != nullptr) {
               const uint16_t* nx = p.bias_t + b * p.bias_t_batch_stride + (hx * p.kv_group + hn) * p.bias_t_head_stride +
                                    static_cast<int64_t>(xr) * p.bias_t_row_stride + cn;
               if (cn < len_q) {
@@ -516,16 +532,16 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // This item's bias values where they are contiguous for this thread (dQ: its query row; dK/dV: its key's row
       // of the transposed copy): eight 16-byte loads issued before the waits, so their latency passes under the
       // score GEMM. A chunk that starts past the end is skipped (zeros); one that straddles it reads row padding.
-      uint4 bw[kBias ? 8 : 1];
+      uint4 bw[kBias == kFullBias ? 8 : 1];
       bool bias_in_regs = false;
-      if constexpr (kBias) {
+      if constexpr (kBias == kFullBias) {
         const int col0 = y0 + half * 64;
         const uint16_t* vrow = nullptr;
         int vlen = 0;
         if (kMode == kModeDQ) {
           vrow = p.bias + b * p.bias_batch_stride + hx * p.bias_head_stride + static_cast<int64_t>(xr) * p.bias_row_stride;
           vlen = len_k;
-        } else if (p.bias_row_stride != 0 && p.bias_t != nullptr) {
+        } else if (p.bias_t != nullptr) {
           vrow = p.bias_t + b * p.bias_t_batch_stride + (hx * p.kv_group + hi) * p.bias_t_head_stride +
                  static_cast<int64_t>(xr) * p.bias_t_row_stride;
           vlen = len_q;
@@ -573,7 +589,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tmem_ld_x32_at<32>(sbuf + 32, a);
         tmem_wait_ld();
         BWD_STAMP(half, i, 2);
-        if constexpr (kBias) {
+        if constexpr (kBias == kFullBias) {
           // S <- S + bias / scale (then x = S c - lse2 as without bias)
           const int col0 = y0 + half * 64;
           if (bias_in_regs) {
@@ -588,24 +604,28 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               }
             }
           } else if (kMode == kModeDKDV && xr < len_x) {
+            // no transposed copy: this key in 64 consecutive query rows, 64 two-byte loads (consecutive lanes on
+            // consecutive keys)
             const uint16_t* bcol = p.bias + b * p.bias_batch_stride + (hx * p.kv_group + hi) * p.bias_head_stride + xr;
-            if (p.bias_row_stride == 0) {
-              // the bias does not depend on the query (ALiBi-like): one value for this thread's key
-              const float bs = unpack_16x2<kF16>(static_cast<uint32_t>(bcol[0])).x * p.inv_scale;
 #pragma unroll
-              for (int j = 0; j < 64; ++j) a[j] = __float_as_uint(__uint_as_float(a[j]) + bs);
-            } else {
-              // no transposed copy: this key in 64 consecutive query rows, 64 two-byte loads (consecutive lanes on
-              // consecutive keys)
-#pragma unroll
-              for (int j = 0; j < 64; ++j) {
-                if (col0 + j < len_q) {
-                  const uint32_t raw = bcol[static_cast<int64_t>(col0 + j) * p.bias_row_stride];
-                  const float bv = unpack_16x2<kF16>(raw).x;
-                  a[j] = __float_as_uint(fmaf(bv, p.inv_scale, __uint_as_float(a[j])));
-                }
+            for (int j = 0; j < 64; ++j) {
+              if (col0 + j < len_q) {
+                const uint32_t raw = bcol[static_cast<int64_t>(col0 + j) * p.bias_row_stride];
+                const float bv = unpack_16x2<kF16>(raw).x;
+                a[j] = __float_as_uint(fmaf(bv, p.inv_scale, __uint_as_float(a[j])));
               }
             }
+          }
+        }
+        constexpr float kLog2e = 1.4426950408889634f;
+        float key_bias = 0.f;  // dK/dV
+        uint32_t* key_bias_row = reinterpret_cast<uint32_t*>(smem + smem_key_bias_off(kMode) + warp * 128);  // dQ
+        if constexpr (kBias == kKeyBias) {
+          if (kMode == kModeDKDV) {
+            key_bias = unpack_16x2<kF16>(key_bias_raw).x * kLog2e;
+          } else {
+            key_bias_row[lane] = key_bias_raw;  // the previous item's values were read before this warp's last __syncwarp
+            __syncwarp();
           }
         }
         // x = S c - lse2. In the dK/dV kernel this pass sits on the critical chain (score GEMM ->
@@ -617,10 +637,16 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
         for (int j4 = 0; j4 < 16; ++j4) {
           const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
+          uint2 kb = make_uint2(0u, 0u);
+          if constexpr (kBias == kKeyBias && kMode == kModeDQ) kb = *reinterpret_cast<const uint2*>(key_bias_row + 2 * j4);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int j = 4 * j4 + 2 * h;
-            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w));
+            float2 nl = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
+            if constexpr (kBias == kKeyBias)
+              nl = kMode == kModeDKDV ? add2(nl, make_float2(key_bias, key_bias))
+                                      : fma2(unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), make_float2(kLog2e, kLog2e), nl);
+            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl);
             if (((j >> 1) & 3) < kPolyOf4) {
               const float2 e = exp2_poly3_x2(x);
               pr[j] = e.x;
@@ -691,7 +717,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         tmem_st_x16(sbuf + 32, dw);
         tmem_st_x16(sbuf + 48, dw + 16);
-        if constexpr (kBias && kMode == kModeDQ) {
+        if constexpr (kBias == kFullBias && kMode == kModeDQ) {
           // dbias = dS: this thread's 64 keys of its query row, already packed for the dQ GEMM
           const int col0 = y0 + half * 64;
           if (p.dbias != nullptr && xr < len_x) {
@@ -918,17 +944,23 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
 using TileKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                             const CUtensorMap, const CUtensorMap, const BwdKernelParams);
 
-template <int kMode, bool kDrop, bool kBias>
+template <int kMode, bool kDrop, int kBias>
 TileKernel pick_tile_kernel(int head_dim, bool f16) {
   if (head_dim <= 64)
     return f16 ? bwd_tile_kernel<kMode, 64, true, kDrop, kBias> : bwd_tile_kernel<kMode, 64, false, kDrop, kBias>;
   return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias>;
 }
 
+template <int kMode, bool kDrop>
+TileKernel pick_tile_kernel(BiasKind bias, int head_dim, bool f16) {
+  if (bias == kKeyBias) return pick_tile_kernel<kMode, kDrop, kKeyBias>(head_dim, f16);
+  return bias == kFullBias ? pick_tile_kernel<kMode, kDrop, kFullBias>(head_dim, f16)
+                           : pick_tile_kernel<kMode, kDrop, kNoBias>(head_dim, f16);
+}
+
 template <int kMode>
-TileKernel pick_tile_kernel(bool drop, bool bias, int head_dim, bool f16) {
-  if (drop) return bias ? pick_tile_kernel<kMode, true, true>(head_dim, f16) : pick_tile_kernel<kMode, true, false>(head_dim, f16);
-  return bias ? pick_tile_kernel<kMode, false, true>(head_dim, f16) : pick_tile_kernel<kMode, false, false>(head_dim, f16);
+TileKernel pick_tile_kernel(bool drop, BiasKind bias, int head_dim, bool f16) {
+  return drop ? pick_tile_kernel<kMode, true>(bias, head_dim, f16) : pick_tile_kernel<kMode, false>(bias, head_dim, f16);
 }
 
 // `overlap_previous`: launch with programmatic stream serialization, so that this grid's CTAs may start as soon as
@@ -940,10 +972,13 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
                        const CUtensorMap& tm_o1, const CUtensorMap& tm_o2, const BwdKernelParams& kp,
                        bool overlap_previous = false) {
   const bool drop = kp.keep_rows != nullptr;
-  const bool bias = kp.bias != nullptr;
+  // the dK/dV kernel writes no bias gradient
+  const BiasKind bias = kp.bias == nullptr                                                                    ? kNoBias
+                        : kp.bias_row_stride == 0 && (mode == kModeDKDV || kp.dbias == nullptr) ? kKeyBias
+                                                                                                              : kFullBias;
   TileKernel kernel = mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16)
                                         : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16);
-  const uint32_t smem = smem_bytes_for(mode);
+  const uint32_t smem = smem_bytes_for(mode, bias == kKeyBias);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) {
     set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", smem, cudaGetErrorString(err));
@@ -973,11 +1008,12 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 
 }  // namespace
 
-// Fused kernel or the two with a fixed summation order? A bias with a query dependence or a gradient always takes the two (the
-// gradient is written by the dQ kernel, whose threads own query rows). Otherwise (us, back-to-back calls, fused | two):
+// Fused kernel or the two with a fixed summation order? A bias always takes the two: masked training gives the same bits every
+// time (and a bias gradient is written by the dQ kernel, whose threads own query rows). Otherwise (us, back-to-back calls, fused
+// | two):
 //  * up to one CTA per SM, fused leaves SMs idle for a whole chain of items, while the two kernels run side by side and need
 //    no clearing and no conversion: two. (B1 H8 L300 D128 31.9 | 22.0, B2 H8 L700 D64 26.6 | 20.5, B4 H8/1 L4096 D128 812 | 564,
-//    B1 H12 L200 with a padding mask 24.7 | 17.0, B4 H8 L500 D64 31.8 | 30.4)
+//    B4 H8 L500 D64 31.8 | 30.4)
 //  * head_dim 128 with grouped queries: a fused CTA chains the items of every query head of its group: two. (B8 H32/8 L2048
 //    causal 1125 | 1097; packed 12 x 64..2048 H16/4, whole step 420 | 408). Not with dropout, whose masks the two expand twice.
 //  * else fused: at head_dim 64 its items are cheap against the second pass over the scores (B8 H16 L2048 387 | 438, B16 H8 L300
@@ -985,12 +1021,11 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 //    dropout 660 | 677; B2 H16 L8192 1758 | 1747).
 // The number of SMs is the B200's, not the current device's: workspace queries and launches must agree.
 bool use_fused_backward(const sdpa_b200_params& p) {
-  if (p.deterministic != 0) return false;
-  if (p.bias != nullptr && (p.bias_row_stride != 0 || p.dbias != nullptr)) return false;
+  if (p.deterministic != 0 || p.bias != nullptr) return false;
   constexpr int64_t kSms = 148;
   const int64_t ctas = static_cast<int64_t>(p.batch) * p.heads_kv * ((static_cast<int64_t>(p.max_seqlen_k) + kTile - 1) / kTile);
   if (ctas <= kSms) return false;
-  return p.head_dim <= 64 || p.heads_q == p.heads_kv || p.bias != nullptr || p.dropout_p > 0.f;
+  return p.head_dim <= 64 || p.heads_q == p.heads_kv || p.dropout_p > 0.f;
 }
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
@@ -1000,19 +1035,13 @@ size_t bwd_vector_bytes(const sdpa_b200_params& p) {
 
 // lse2 and delta, then the fp32 dQ accumulator of the fused kernel: for every call without a bias that does not ask for a fixed
 // order, whatever path its sizes take, so that one workspace serves calls that differ in dropout or sizes.
-size_t bwd_workspace_required(const sdpa_b200_params& p) {
+size_t bwd_workspace_bytes(const sdpa_b200_params& p) {
   const bool acc = p.deterministic == 0 && p.bias == nullptr;
   return bwd_vector_bytes(p) + (acc ? bwd_fused_workspace_bytes(p, lq_padded(p)) : 0);
 }
 
-// What a workspace query answers. A call with a bias that the fused kernel can take is better off with the accumulator, but
-// runs in the two kernels without it.
-size_t bwd_workspace_bytes(const sdpa_b200_params& p) {
-  return p.bias != nullptr && use_fused_backward(p) ? bwd_vector_bytes(p) + bwd_fused_workspace_bytes(p, lq_padded(p))
-                                                    : bwd_workspace_required(p);
-}
-
 int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  (void)workspace_bytes;
   const bool f16 = p.dtype == SDPA_B200_F16;
   const bool varlen = p.cu_seqlens_q != nullptr;
   const int lq_pad = lq_padded(p);
@@ -1038,7 +1067,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   pre.heads_q = p.heads_q;
   pre.lq_pad = lq_pad;
   pre.head_dim = p.head_dim;
-  const bool fused = use_fused_backward(p) && workspace_bytes >= kWorkspaceHeaderBytes + bwd_workspace_bytes(p);
+  const bool fused = use_fused_backward(p);
   float* dq_acc = fused ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p)) : nullptr;
   pre.dq_acc = dq_acc;
   pre.dq_acc_rows = fused && varlen ? static_cast<int>(bwd_fused_acc_rows(p, lq_pad) / p.heads_q) : 0;

@@ -54,7 +54,6 @@ uint32_t dropout_drop_byte(float dropout_p);
 
 // Backward: delta pre-pass + dK/dV kernel + dQ kernel.
 size_t bwd_workspace_bytes(const sdpa_b200_params& p);
-size_t bwd_workspace_required(const sdpa_b200_params& p);  // the least a call accepts
 int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes,
                cudaStream_t stream);
 

@@ -431,7 +431,7 @@ int sdpa_b200_bwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
   if ((st = check_tensor("dv", p->dv, p->dv_batch_stride, p->dv_head_stride, p->dv_row_stride, varlen, p->batch,
                          p->heads_kv)) != SDPA_B200_OK)
     return st;
-  const size_t need = kWorkspaceHeaderBytes + (p->head_dim > 128 ? bwd_d256_workspace_bytes(*p) : bwd_workspace_required(*p));
+  const size_t need = kWorkspaceHeaderBytes + (p->head_dim > 128 ? bwd_d256_workspace_bytes(*p) : bwd_workspace_bytes(*p));
   st = validate_workspace(workspace, workspace_bytes, need);
   if (st != SDPA_B200_OK) return st;
   st = check_device();
