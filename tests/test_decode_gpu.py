@@ -51,6 +51,42 @@ def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D):
     orc.assert_close_lse(lse, l_ref)
 
 
+@pytest.mark.parametrize("what", ["query", "key", "value", "score"])
+@pytest.mark.parametrize("B,Hq,Hkv,Lk,splits,D", [
+    (1, 8, 2, 4096, 0, 128),    # every unit shared between CTAs
+    (1, 40, 2, 1000, 0, 64),    # shared, head chunks of 16 and 4
+    (1, 8, 2, 4096, 4, 128),    # fixed splits
+    (1, 8, 2, 200, 6, 64),      # fixed splits, some of them without keys
+    (2, 8, 2, 4096, 1, 128),    # one CTA per unit
+    (160, 8, 2, 64, 0, 128),    # whole units
+])
+def test_decode_shows_nan_and_overflow(cuda_device, native_lib, B, Hq, Hkv, Lk, splits, D, what):
+    """One NaN in an input, or one score that overflows to +inf, makes the rows that see it NaN however the keys are dealt
+    out, as the softmax of the same values does; the other rows are not touched."""
+    q, k, v = rand((B, Hq, 1, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3)
+    at = 7 if Lk < 1000 else 300  # a key in the first share, the others hold none
+    if what == "query":
+        q[0, 1, 0, 5] = float("nan")
+    elif what == "key":
+        k[0, 1, at, 5] = float("nan")
+    elif what == "value":
+        v[0, 1, at, 5] = float("nan")
+    else:
+        q[0, :, 0, 0] = 0.0  # the other heads' scores stay ordinary
+        q[0, 1, 0, 0] = k[0, 0, at, 0] = 1e20
+    s = torch.einsum("bhqd,bhkd->bhqk", q.float(), k.float().repeat_interleave(Hq // Hkv, 1)) * D ** -0.5
+    want = torch.einsum("bhqk,bhkd->bhqd", torch.softmax(s, -1), v.float().repeat_interleave(Hq // Hkv, 1))
+    bad = want.isnan()
+    assert bad.any() and not bad.all()
+    dev = cuda_device
+    out, lse = ops.decode_attention(q.to(dev), k.to(dev), v.to(dev), num_splits=splits)
+    assert ops.device_status() == 0
+    out = out.float().cpu()
+    assert torch.equal(out.isnan(), bad)
+    orc.assert_close_bf16(out.masked_fill(bad, 0.0).bfloat16(), want.masked_fill(bad, 0.0), "out")
+    assert torch.equal(lse.cpu().isfinite(), ~s.softmax(-1).isnan().any(-1))
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,Lk,splits", [(2, 8, 2, 1000, 4), (1, 32, 2, 777, 3), (1, 4, 4, 4096, 0)])
 def test_decode_head_dim_64(cuda_device, native_lib, B, Hq, Hkv, Lk, splits):
     g = torch.Generator().manual_seed(8)

@@ -40,7 +40,7 @@ struct DecodeParams {
   uint16_t* out;
   float* lse;
   float* part_o;    // rows of head_dim fp32 values, normalised per share; the order of the rows: part_row()
-  float* part_lse;  // one fp32 value per row, log2 domain
+  float* part_lse;  // one fp32 value per row, log2 domain; -inf: no key seen; NaN where the row's sum is NaN
   uint32_t* status;
   int64_t q_batch_stride, q_head_stride;
   int64_t o_batch_stride, o_head_stride;
@@ -423,7 +423,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         if (r >= nheads) continue;
         const float l = hi ? l_hi : l_lo, mm = hi ? mm_hi : mm_lo;
         const float inv = (l > 0.f) ? 1.f / l : 0.f;
-        const float lse2 = (l > 0.f) ? mm + log2f(l) : -INFINITY;
+        const float lse2 = (l == 0.f) ? -INFINITY : mm + log2f(l);  // a NaN sum stays visible to the merge
         if (whole) {
           uint16_t* dst = p.out + b * p.o_batch_stride + (head0 + r) * p.o_head_stride + 2 * t;
 #pragma unroll
@@ -493,15 +493,16 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams 
 #pragma unroll
       for (int e = 0; e < kPer; ++e) x[j][e] = (ls[j] == -INFINITY) ? 0.f : p.part_o[pr * kD + e * 32 + lane];
     }
+    // empty parts are left out by their own weight: a NaN part is not one, and fmaxf does not return it
+    if (ls[0] == -INFINITY && ls[1] == -INFINITY && ls[2] == -INFINITY && ls[3] == -INFINITY) continue;
     const float mn = fmaxf(fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3])), m);
-    if (mn == -INFINITY) continue;
-    const float a = exp2f(m - mn);
+    const float a = (m == -INFINITY) ? 1.f : exp2f(m - mn);  // nothing summed yet, or NaN
     l *= a;
 #pragma unroll
     for (int e = 0; e < kPer; ++e) acc[e] *= a;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float w = exp2f(ls[j] - mn);
+      const float w = (ls[j] == -INFINITY) ? 0.f : exp2f(ls[j] - mn);
       l += w;
 #pragma unroll
       for (int e = 0; e < kPer; ++e) acc[e] += w * x[j][e];
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams 
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
     f[w] = (sm_m[w] == -INFINITY) ? 0.f : exp2f(sm_m[w] - mm);
-    sum += sm_l[w] * f[w];
+    sum += sm_l[w] * f[w];  // 0 * NaN is NaN: a quarter of NaN parts only counts as well
   }
   const float inv = (sum > 0.f) ? 1.f / sum : 0.f;
   uint16_t* dst = p.out + b * p.o_batch_stride + hq * p.o_head_stride;
