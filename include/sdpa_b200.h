@@ -94,6 +94,8 @@ typedef struct sdpa_b200_params {
   float* lse; /* fp32, layout above */
   /* backward only */
   const void* dout; /* bf16, same shape/strides family as out */
+  /* Gradients. Packed: rows of tokens that belong to no sequence (in front of cu_seqlens[0], behind cu_seqlens[batch]) are
+   * set to zero. */
   void* dq;         /* bf16, shape of q */
   void* dk;         /* bf16, shape of k */
   void* dv;         /* bf16, shape of v */

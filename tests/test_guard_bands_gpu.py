@@ -228,3 +228,43 @@ def test_backward_with_a_key_bias_needs_no_accumulator(cuda_device, native_lib):
     torch.cuda.synchronize(dev)
     for got, ref in zip(grads, want):
         assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("deterministic", [0, 1])
+@pytest.mark.parametrize("Hq,Hkv,D,lens,front,tail", [
+    (4, 4, 128, (100, 60), 3, 70),         # few key blocks
+    (16, 16, 64, (300, 1, 129) * 6, 5, 1),  # more key blocks than SMs
+    (40, 8, 128, (200, 300) * 8, 1, 200),   # grouped query heads
+    (4, 2, 256, (100, 60), 9, 130),
+    (2, 1, 72, (100, 60), 0, 0),            # no such rows
+])
+def test_packed_gradients_of_tokens_outside_every_sequence_are_zero(cuda_device, native_lib, Hq, Hkv, D, lens, front, tail, deterministic):
+    """A packed batch padded to a number of tokens: the outputs and the workspace hold NaN before the call, the rows of the padding
+    hold zeros after it, and the other rows the gradients of the same batch without padding."""
+    dev = cuda_device
+    n, longest = sum(lens), max(lens)
+    total = front + n + tail
+    ends = [front + sum(lens[:i]) for i in range(len(lens) + 1)]
+    cu = torch.tensor(ends, dtype=torch.int32, device=dev)
+    q, k, v, dout = (rand((total, h, D), s).to(dev) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
+    scale = D ** -0.5
+    cut = slice(front, front + n)
+    o_cut, lse_cut = ops._varlen_forward(q[cut], k[cut], v[cut], cu - front, cu - front, longest, longest, True, scale)
+    want = ops._varlen_backward(dout[cut], q[cut], k[cut], v[cut], o_cut, lse_cut, cu - front, cu - front, longest, longest, True, scale,
+                                deterministic=bool(deterministic))
+    out, lse = torch.full_like(q, NAN), torch.full((Hq, total), NAN, device=dev)
+    out[cut], lse[:, cut] = o_cut, lse_cut
+    grads = [torch.full_like(t, NAN) for t in (q, k, v)]
+    p = ops._varlen_params(q, k, v, out, lse, cu, cu, longest, longest, True, scale)
+    set_bwd(p, dout, *grads, packed=True)
+    p.deterministic = deterministic
+    need = ctypes.c_size_t(0)
+    _cabi.check(native_lib.sdpa_b200_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(need)), "workspace query")
+    ws = torch.full(((need.value + 3) // 4,), NAN, device=dev)
+    _cabi.check(native_lib.sdpa_b200_bwd(ctypes.byref(p), ws.data_ptr(), need.value, torch.cuda.current_stream(dev).cuda_stream), "bwd")
+    torch.cuda.synchronize(dev)
+    for name, got, ref in zip(("dq", "dk", "dv"), grads, want):
+        assert not got[:front].any() and not got[front + n:].any(), name
+        # the fused kernel sums dQ in a varying order: two roundings to 16 bits of nearly the same sum
+        err = (got[cut].float() - ref.float()).norm() / ref.float().norm()
+        assert float(err) <= (0.0 if deterministic or name != "dq" else 1e-3), (name, float(err))

@@ -625,7 +625,7 @@ struct DqConvertParams {
   uint16_t* dq;
   const int32_t* cu_q;  // null for dense
   int64_t dq_batch_stride, dq_head_stride, dq_row_stride;
-  int heads_q, seqlen_q, lq_pad, total_q, acc_rows, head_dim;
+  int batch, heads_q, seqlen_q, lq_pad, acc_rows, head_dim;
   float scale;
 };
 
@@ -639,7 +639,8 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const DqConvertPara
     const int tiles_per_head = p.acc_rows >> 7;
     const int h = static_cast<int>(tile / tiles_per_head);
     const int tok = static_cast<int>(tile - static_cast<size_t>(h) * tiles_per_head) * 128 + r;
-    if (tok >= p.total_q) return;
+    // the pre-pass clears the accumulator rows of the sequences, and dq itself outside them
+    if (tok < p.cu_q[0] || tok >= p.cu_q[p.batch]) return;
     dst = p.dq + static_cast<int64_t>(tok) * p.dq_row_stride + h * p.dq_head_stride;
   } else {
     const int tiles_per_head = p.lq_pad >> 7;
@@ -719,10 +720,10 @@ int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_ac
   cp.dq_batch_stride = p.dq_batch_stride;
   cp.dq_head_stride = p.dq_head_stride;
   cp.dq_row_stride = p.dq_row_stride;
+  cp.batch = p.batch;
   cp.heads_q = p.heads_q;
   cp.seqlen_q = p.max_seqlen_q;
   cp.lq_pad = kp.lq_pad;
-  cp.total_q = p.total_q;
   cp.acc_rows = kp.dq_acc_rows;
   cp.head_dim = p.head_dim;
   cp.scale = p.softmax_scale;

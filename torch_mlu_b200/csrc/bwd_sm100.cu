@@ -28,6 +28,7 @@
 #include <cstdlib>
 
 #include "bwd_common.cuh"
+#include "packed_grads.cuh"
 
 namespace sdpa_b200 {
 namespace {
@@ -859,13 +860,18 @@ struct PreParams {
   int seqlen_q, total_q, heads_q, lq_pad, head_dim;
   float* dq_acc;    // fused kernel: its dQ accumulator, whose existing rows are cleared here; else null
   int dq_acc_rows;  // as in BwdKernelParams
+  PackedGrads grads;
 };
 
 // 16 bytes (8 elements) per thread and head_dim / 8 threads per row; a 256-thread block covers 64 rows of
 // the padded sequence in up to four passes whose loads are all issued before the first use.
 constexpr int kPreRows = 64;
-template <bool kF16>
+template <bool kF16, bool kPacked>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) {
+  if (kPacked && static_cast<int>(blockIdx.x) == p.heads_q) {
+    clear_uncovered_rows(p.grads, p.heads_q);
+    return;
+  }
   // heads vary fastest across the grid: with the usual [batch, row, head, dim] memory order the blocks
   // that run together then read neighbouring 256-byte pieces of the same rows
   const int h = blockIdx.x, b = blockIdx.z;
@@ -875,7 +881,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   const int sub = threadIdx.x % tpr;
   const int r_in_pass = threadIdx.x / tpr;
   int q_off = 0, len_q = p.seqlen_q;
-  if (p.cu_q != nullptr) {
+  if (kPacked) {
     q_off = p.cu_q[b];
     len_q = p.cu_q[b + 1] - q_off;
   }
@@ -885,7 +891,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     const int groups = p.head_dim <= 64 ? 16 : 32;
     const int row = blockIdx.y * kPreRows + (threadIdx.x & (kPreRows - 1));
     if (row < len_q) {
-      const size_t acc_row = p.cu_q != nullptr ? static_cast<size_t>(h) * p.dq_acc_rows + q_off + row
+      const size_t acc_row = kPacked ? static_cast<size_t>(h) * p.dq_acc_rows + q_off + row
                                                : (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
       float4* dst = reinterpret_cast<float4*>(p.dq_acc + (acc_row >> 7) * (static_cast<size_t>(groups) * 512)) + (acc_row & 127);
       for (int g = threadIdx.x / kPreRows; g < groups; g += 256 / kPreRows) dst[g * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -900,7 +906,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     if (ps < passes && row < len_q) {
       const uint16_t* o;
       const uint16_t* dout;
-      if (p.cu_q != nullptr) {
+      if (kPacked) {
         o = p.out + static_cast<int64_t>(q_off + row) * p.o_row_stride + h * p.o_head_stride;
         dout = p.dout + static_cast<int64_t>(q_off + row) * p.do_row_stride + h * p.do_head_stride;
       } else {
@@ -928,7 +934,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     if (sub == 0 && row < p.lq_pad) {
       const size_t dst = (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
       if (row < len_q) {
-        const float lse = (p.cu_q != nullptr) ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + row]
+        const float lse = (kPacked) ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + row]
                                               : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + row];
         p.nlse2[dst] = lse * -1.4426950408889634f;
         p.ndelta[dst] = -acc;
@@ -1067,14 +1073,15 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   pre.heads_q = p.heads_q;
   pre.lq_pad = lq_pad;
   pre.head_dim = p.head_dim;
+  pre.grads = packed_grads(p);
   const bool fused = use_fused_backward(p);
   float* dq_acc = fused ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p)) : nullptr;
   pre.dq_acc = dq_acc;
   pre.dq_acc_rows = fused && varlen ? static_cast<int>(bwd_fused_acc_rows(p, lq_pad) / p.heads_q) : 0;
-  if (f16)
-    bwd_preprocess_kernel<true><<<dim3(p.heads_q, lq_pad / kPreRows, p.batch), 256, 0, stream>>>(pre);
-  else
-    bwd_preprocess_kernel<false><<<dim3(p.heads_q, lq_pad / kPreRows, p.batch), 256, 0, stream>>>(pre);
+  const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), lq_pad / kPreRows, p.batch);
+  auto pre_kernel = varlen ? (f16 ? bwd_preprocess_kernel<true, true> : bwd_preprocess_kernel<false, true>)
+                           : (f16 ? bwd_preprocess_kernel<true, false> : bwd_preprocess_kernel<false, false>);
+  pre_kernel<<<pre_grid, 256, 0, stream>>>(pre);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("backward preprocess: launch failed: %s", cudaGetErrorString(err));

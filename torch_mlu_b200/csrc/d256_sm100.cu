@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.h"
+#include "packed_grads.cuh"
 #include "ptx_sm100.cuh"
 
 namespace sdpa_b200 {
@@ -1053,23 +1054,28 @@ struct Pre256Params {
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int64_t do_batch_stride, do_head_stride, do_row_stride;
   int seqlen_q, total_q, heads_q, lq_pad, head_dim;
+  PackedGrads grads;
 };
 
 // Each warp takes four rows whose loads are all issued before the first use: 57 -> 48 us at B4 H16 L4096 (268 MB).
 constexpr int kPre256Rows = 4;
-template <bool kF16>
+template <bool kF16, bool kPacked>
 __global__ void __launch_bounds__(256) bwd_d256_preprocess_kernel(const Pre256Params p) {
+  if (kPacked && static_cast<int>(blockIdx.x) == p.heads_q) {
+    clear_uncovered_rows(p.grads, p.heads_q);
+    return;
+  }
   const int h = blockIdx.x, b = blockIdx.z;
   const int lane = threadIdx.x & 31;
   const int row0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * kPre256Rows;
   int q_off = 0, len_q = p.seqlen_q;
-  if (p.cu_q != nullptr) {
+  if (kPacked) {
     q_off = p.cu_q[b];
     len_q = p.cu_q[b + 1] - q_off;
   }
-  const uint16_t* o = p.out + h * p.o_head_stride + (p.cu_q != nullptr ? q_off * p.o_row_stride : b * p.o_batch_stride) + lane * 8;
+  const uint16_t* o = p.out + h * p.o_head_stride + (kPacked ? q_off * p.o_row_stride : b * p.o_batch_stride) + lane * 8;
   const uint16_t* dout =
-      p.dout + h * p.do_head_stride + (p.cu_q != nullptr ? q_off * p.do_row_stride : b * p.do_batch_stride) + lane * 8;
+      p.dout + h * p.do_head_stride + (kPacked ? q_off * p.do_row_stride : b * p.do_batch_stride) + lane * 8;
   uint4 ov[kPre256Rows], dv[kPre256Rows];
 #pragma unroll
   for (int i = 0; i < kPre256Rows; ++i) {
@@ -1094,7 +1100,7 @@ __global__ void __launch_bounds__(256) bwd_d256_preprocess_kernel(const Pre256Pa
     if (lane == 0 && row < p.lq_pad) {
       const size_t dst = (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
       if (row < len_q) {
-        const float lse = (p.cu_q != nullptr) ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + row]
+        const float lse = (kPacked) ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + row]
                                               : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + row];
         p.lse2[dst] = lse * 1.4426950408889634f;  // +inf stays +inf
         p.delta[dst] = acc;
@@ -1155,9 +1161,11 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   pre.heads_q = p.heads_q;
   pre.lq_pad = lq_pad;
   pre.head_dim = p.head_dim;
-  const dim3 pre_grid(p.heads_q, lq_pad / (8 * kPre256Rows), p.batch);
-  if (f16) bwd_d256_preprocess_kernel<true><<<pre_grid, 256, 0, stream>>>(pre);
-  else bwd_d256_preprocess_kernel<false><<<pre_grid, 256, 0, stream>>>(pre);
+  pre.grads = packed_grads(p);
+  const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), lq_pad / (8 * kPre256Rows), p.batch);
+  auto pre_kernel = varlen ? (f16 ? bwd_d256_preprocess_kernel<true, true> : bwd_d256_preprocess_kernel<false, true>)
+                           : (f16 ? bwd_d256_preprocess_kernel<true, false> : bwd_d256_preprocess_kernel<false, false>);
+  pre_kernel<<<pre_grid, 256, 0, stream>>>(pre);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("head_dim 256 backward pre-pass: launch failed: %s", cudaGetErrorString(err));
