@@ -2,9 +2,10 @@
 reference's schemas and the backend toggles behave like the reference's."""
 import re
 
+import pytest
 import torch
 
-from torch_mlu_b200 import backends, torch_glue
+from torch_mlu_b200 import backends, ops, torch_glue
 
 # codegen/mlu_functions.yaml:1313-1316 of the reference
 REFERENCE_SCHEMAS = {
@@ -34,3 +35,19 @@ def test_sdp_kernel_toggles_restore_state():
         assert not backends.mem_efficient_sdp_enabled()
     assert (backends.flash_sdp_enabled(), backends.mem_efficient_sdp_enabled(), backends.math_sdp_enabled()) == before
     assert int(backends.SDPBackend.FLASH_ATTENTION) == 1 and int(backends.SDPBackend.ERROR) == -1
+
+
+def test_keys_without_heads_raise():
+    """The check comes before the devices are looked at, and is not a division by the number of heads."""
+    q, kv = torch.zeros(1, 8, 1, 128, dtype=torch.bfloat16), torch.zeros(1, 0, 64, 128, dtype=torch.bfloat16)
+    for call in (ops.decode_attention, ops.gqa_prefill):
+        with pytest.raises(RuntimeError, match="must divide"):
+            call(q, kv, kv)
+
+
+@pytest.mark.gpu
+def test_packed_keys_without_heads_raise(cuda_device):
+    q, kv = (torch.zeros(16, h, 128, dtype=torch.bfloat16, device=cuda_device) for h in (8, 0))
+    cu = torch.tensor([0, 16], dtype=torch.int32, device=cuda_device)
+    with pytest.raises(RuntimeError, match="must divide"):
+        ops._flash_attention_forward(q, kv, kv, cu, cu, 16, 16, 0.0, False, False)

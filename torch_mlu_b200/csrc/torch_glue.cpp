@@ -177,7 +177,7 @@ void check_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   TORCH_CHECK(cu_q.is_cuda() && cu_k.is_cuda() && cu_q.is_contiguous() && cu_k.is_contiguous(),
               "cu_seqlens must be contiguous device tensors");
   TORCH_CHECK(cu_q.numel() == cu_k.numel() && cu_q.numel() >= 2, "cu_seqlens_q and cu_seqlens_k must have batch+1 entries");
-  TORCH_CHECK(k.size(1) == v.size(1) && q.size(1) % k.size(1) == 0,
+  TORCH_CHECK(k.size(1) == v.size(1) && k.size(1) > 0 && q.size(1) % k.size(1) == 0,
               "Number of heads in key/value must divide number of heads in query");
   TORCH_CHECK(q.size(2) == k.size(2) && q.size(2) == v.size(2), "query, key and value must have the same head_dim");
   TORCH_CHECK(k.size(0) == v.size(0), "Key and Value must have the same number of tokens");
@@ -341,7 +341,7 @@ std::tuple<Tensor, Tensor> dense_forward(const Tensor& q, const Tensor& k, const
   TORCH_CHECK(q.size(0) == k.size(0) && q.size(0) == v.size(0), "query, key and value must have the same batch size");
   TORCH_CHECK(k.size(2) == v.size(2), "Key and Value must have the same sequence length");
   if (allow_gqa) {
-    TORCH_CHECK(k.size(1) == v.size(1) && q.size(1) % k.size(1) == 0,
+    TORCH_CHECK(k.size(1) == v.size(1) && k.size(1) > 0 && q.size(1) % k.size(1) == 0,
                 "Number of heads in key/value must divide number of heads in query");
   } else {
     TORCH_CHECK(q.size(1) == k.size(1) && q.size(1) == v.size(1), "query, key and value must have the same number of heads");
