@@ -2,6 +2,8 @@
 as the flash operators, but a causal mask aligned to the TOP-LEFT corner (sdp_utils.h:32-37). torch's CPU
 scaled_dot_product_attention uses the same convention, so it is the fp32 reference here (forward and, by
 autograd, backward). Tolerances as everywhere: out / grads max-abs 2e-2, mean-abs 2e-3; lse 1e-5."""
+import contextlib
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -358,3 +360,39 @@ def test_backward_with_a_bias_that_is_the_same_for_every_query(cuda_device, nati
     for name, x, t, l, fudge in (("dq", grads[0][0], true[2], lowp[2], 4), ("dk", grads[0][1], fold(true[3]), fold(lowp[3]), 2),
                                  ("dv", grads[0][2], fold(true[4]), fold(lowp[4]), 2)):
         orc.assert_close_reference_rule(x, t, l, name, fudge=fudge)
+
+
+@pytest.mark.parametrize("Lk,rows", [(128, 128), (128, 1), (77, 77)])   # used in place, broadcast, copied into padded rows
+@pytest.mark.parametrize("learned", [False, True])
+def test_bias_changed_between_forward_and_backward_raises(cuda_device, native_lib, Lk, rows, learned):
+    dev = cuda_device
+    with backends.sdp_kernel(enable_flash=False, enable_math=False, enable_mem_efficient=True):
+        q, k, v = (torch.randn(2, 4, n, 64, device=dev, dtype=torch.bfloat16, requires_grad=True) for n in (rows if rows > 1 else 96, Lk, Lk))
+        bias = torch.randn(1, 4, rows, Lk, device=dev, dtype=torch.bfloat16, requires_grad=learned)
+        out = sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=bias)
+        with torch.no_grad():
+            bias.mul_(2)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            out.float().sum().backward()
+
+
+@pytest.mark.parametrize("Lk", [128, 77])
+@pytest.mark.parametrize("boolean", [False, True])
+def test_bias_goes_through_saved_tensor_hooks(cuda_device, native_lib, Lk, boolean):
+    """Offloading the saved tensors covers the bias, and gradients do not depend on it."""
+    dev = cuda_device
+    with backends.sdp_kernel(enable_flash=False, enable_math=False, enable_mem_efficient=True):
+        q, k, v = (torch.randn(2, 4, n, 64, device=dev, dtype=torch.bfloat16, requires_grad=True) for n in (96, Lk, Lk))
+        bias = torch.randn(2, 1, 96, Lk, device=dev, dtype=torch.bfloat16)
+        mask = bias > -1 if boolean else bias
+        go = torch.randn(2, 4, 96, 64, device=dev, dtype=torch.bfloat16)
+        grads = []
+        for hooked in (False, True):
+            packed = []
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(tuple(t.shape)), t.cpu())[1],
+                                                          lambda t: t.to(dev)) if hooked else contextlib.nullcontext():
+                out = sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=mask)
+            grads.append(torch.autograd.grad(out, (q, k, v), go))
+        assert any(s[:3] == (2, 1, 96) for s in packed), packed
+        for a, b in zip(*grads):
+            assert torch.equal(a, b)

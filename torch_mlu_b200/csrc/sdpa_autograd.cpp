@@ -35,27 +35,28 @@ int64_t ceil8(int64_t n) { return (n + 7) / 8 * 8; }
 
 // The additive bias as a [B, H, Lq, Lk] view the kernels can read: broadcast dimensions keep stride 0, rows start 16-byte
 // aligned and are readable up to the next multiple of 8 keys. A bias that already has that layout is used in place; any
-// other is copied once into rows padded to a multiple of 8.
-Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k) {
+// other is copied once into rows padded to a multiple of 8. `padded`: its rows are already that long, as mask_bias() makes them.
+Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, bool padded = false) {
   TORCH_CHECK(attn_bias.scalar_type() == q.scalar_type() && attn_bias.device() == q.device(),
               "attn_bias must have the dtype and device of query");
   const int64_t full[4] = {q.size(0), q.size(1), q.size(2), seqlen_k};
-  Tensor view = attn_bias.expand(full);
-  if (view.stride(3) == 1 && seqlen_k % 8 == 0 && reinterpret_cast<uintptr_t>(view.data_ptr()) % 16 == 0 &&
+  const Tensor given = padded ? attn_bias.narrow(-1, 0, seqlen_k) : attn_bias;
+  Tensor view = given.expand(full);
+  if (view.stride(3) == 1 && (padded || seqlen_k % 8 == 0) && reinterpret_cast<uintptr_t>(view.data_ptr()) % 16 == 0 &&
       view.stride(0) % 8 == 0 && view.stride(1) % 8 == 0 && view.stride(2) % 8 == 0)
     return view;
-  std::vector<int64_t> sizes(attn_bias.sizes().begin(), attn_bias.sizes().end());
+  std::vector<int64_t> sizes(given.sizes().begin(), given.sizes().end());
   sizes.back() = seqlen_k;
-  Tensor src = attn_bias.expand(sizes);
+  Tensor src = given.expand(sizes);
   sizes.back() = ceil8(seqlen_k);
   Tensor buf = at::zeros(sizes, q.options());
   buf.narrow(-1, 0, seqlen_k).copy_(src);
   return buf.narrow(-1, 0, seqlen_k).expand(full);
 }
 
-// A boolean attn_mask (true = take part) as a bias of 0 / -inf in the layout of prepare_bias: one kernel over the mask's own
-// elements (broadcast dimensions stay broadcast).
-Tensor bias_of_mask(const Tensor& mask, const Tensor& q, int64_t seqlen_k) {
+// A boolean attn_mask (true = take part) as a bias of 0 / -inf with rows padded to a multiple of 8: one kernel over the mask's
+// own elements (broadcast dimensions have size 1).
+Tensor mask_bias(const Tensor& mask, const Tensor& q, int64_t seqlen_k) {
   const int64_t full[4] = {q.size(0), q.size(1), q.size(2), seqlen_k};
   const Tensor m = mask.expand(full);
   int64_t own[4];
@@ -67,7 +68,7 @@ Tensor bias_of_mask(const Tensor& mask, const Tensor& q, int64_t seqlen_k) {
                                       buf.data_ptr(), own[3], q.scalar_type() == at::kHalf ? SDPA_B200_F16 : SDPA_B200_BF16,
                                       at::cuda::getCurrentCUDAStream(q.get_device()).stream()),
                "sdpa_b200_mask_to_bias");
-  return buf.narrow(-1, 0, seqlen_k).expand(full);
+  return buf;
 }
 
 // [B, H, Lk, Lq] view of a copy of `bias` with keys and queries exchanged, for the dK/dV kernel, whose threads own keys and
@@ -92,9 +93,10 @@ using DenseBackwardOp = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const 
 // One node for all forms: dense, dense with an additive bias, packed.
 struct AttentionBackward : public torch::autograd::Node {
   SavedVariable q, k, v, out, lse, cu_q, cu_k, seed, offset;
-  Tensor bias;                       // dense with bias: the prepared view
+  // dense with a bias: the caller's own tensor (a change in place before the backward is noticed), or what mask_bias() made
+  SavedVariable bias;
   std::vector<int64_t> bias_sizes;   // shape of the attn_mask argument, when its gradient is wanted
-  bool packed = false, causal = false, want_dbias = false;
+  bool packed = false, causal = false, has_bias = false, bias_padded = false, want_dbias = false;
   int64_t max_q = 0, max_k = 0;
   double scale = 1.0, dropout_p = 0.0;
 
@@ -102,8 +104,7 @@ struct AttentionBackward : public torch::autograd::Node {
 
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset}) s->reset_data();
-    bias.reset();
+    for (SavedVariable* s : {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset, &bias}) s->reset_data();
   }
 
   variable_list apply(variable_list&& grads) override {
@@ -114,15 +115,17 @@ struct AttentionBackward : public torch::autograd::Node {
     const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), out_ = out.unpack(shared_from_this()), lse_ = lse.unpack();
     const Tensor seed_ = seed.unpack(), offset_ = offset.unpack();
     Tensor dq, dk, dv;
-    if (bias.defined()) {
+    if (has_bias) {
+      const Tensor saved_bias = bias.unpack();
       at::AutoDispatchBelowADInplaceOrView guard;
       c10::cuda::CUDAGuard device_guard(q_.device());
+      const Tensor bias_ = prepare_bias(saved_bias, q_, k_.size(2), bias_padded);
       Tensor dbias;
       if (want_dbias)  // zero-filled: the kernels skip what the causal mask hides
         dbias = at::zeros({q_.size(0), q_.size(1), q_.size(2), ceil8(k_.size(2))}, q_.options()).narrow(-1, 0, k_.size(2));
-      const Tensor bias_t = transposed_bias(bias);
+      const Tensor bias_t = transposed_bias(bias_);
       BackwardOptions opt;
-      opt.bias = &bias;
+      opt.bias = &bias_;
       opt.dbias = &dbias;
       opt.bias_t = &bias_t;
       std::tie(dq, dk, dv) = dense_backward(go, q_, k_, v_, out_, lse_, causal, scale, opt);
@@ -290,17 +293,20 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
   c10::cuda::CUDAGuard device_guard(q.device());
   const bool boolean = mask.scalar_type() == at::kBool;
   const Tensor bias_arg = boolean ? Tensor() : mask.to(dtype);  // (differentiable) conversion of a bias of another type
-  Tensor bias, out, lse;
+  Tensor mask_buf, out, lse;
   {
     at::AutoDispatchBelowADInplaceOrView guard;
-    bias = boolean ? bias_of_mask(mask, q, Lk) : prepare_bias(bias_arg, q, Lk);
+    if (boolean) mask_buf = mask_bias(mask, q, Lk);
+    const Tensor bias = prepare_bias(boolean ? mask_buf : bias_arg, q, Lk, boolean);
     ForwardOptions opt;
     opt.bias = &bias;
     std::tie(out, lse) = dense_forward(q, k, v, is_causal, sc, /*allow_gqa=*/false, opt);
   }
   if (any_requires_grad({&q, &k, &v, &bias_arg})) {
     auto node = new_node(q, k, v, bias_arg, is_causal, sc, 0.0);
-    node->bias = bias;
+    node->has_bias = true;
+    node->bias_padded = boolean;
+    node->bias = SavedVariable(boolean ? mask_buf : bias_arg, false);
     if (bias_arg.defined() && bias_arg.requires_grad()) {
       node->want_dbias = true;
       node->bias_sizes = bias_arg.sizes().vec();
