@@ -210,3 +210,31 @@ def test_packed_operator_with_dropout_and_autograd(cuda_device, native_lib):
         orc.assert_close_grad_bf16(one(qd.grad), qf.grad, f"dq[{b}]")
         orc.assert_close_grad_bf16(one(kd.grad), kf.grad, f"dk[{b}]")
         orc.assert_close_grad_bf16(one(vd.grad), vf.grad, f"dv[{b}]")
+
+
+@pytest.mark.parametrize("which", ["query", "value", "mask"])
+@pytest.mark.parametrize("requires_grad", [False, True])
+def test_forward_mode_raises(cuda_device, native_lib, which, requires_grad):
+    """A tangent is not dropped in silence, by the package's function or by the registered operators."""
+    import torch.autograd.forward_ad as fwd
+    dev = cuda_device
+    q, k, v = (torch.randn(2, 4, 128, 64, device=dev, dtype=torch.bfloat16, requires_grad=requires_grad) for _ in range(3))
+    bias = torch.randn(1, 4, 128, 128, device=dev, dtype=torch.bfloat16)
+    cu = torch.tensor([0, 128], dtype=torch.int32, device=dev)
+    from torch_mlu_b200 import sdp_choice
+    with fwd.dual_level():
+        dual = lambda t: fwd.make_dual(t, torch.ones_like(t))
+        if which == "query":
+            q = dual(q)
+        elif which == "value":
+            v = dual(v)
+        with pytest.raises(NotImplementedError):
+            sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=dual(bias) if which == "mask" else bias)
+        if which != "mask":
+            with pytest.raises(NotImplementedError):
+                sdp_choice.scaled_dot_product_attention(q, k, v)
+            with pytest.raises(NotImplementedError):
+                torch.ops.b200_sdpa._scaled_dot_product_flash_attention(q, k, v)
+            with pytest.raises(NotImplementedError):
+                torch.ops.b200_sdpa._flash_attention_forward(q[0].transpose(0, 1), k[0].transpose(0, 1), v[0].transpose(0, 1), cu, cu,
+                                                             128, 128, 0.0, False, False)

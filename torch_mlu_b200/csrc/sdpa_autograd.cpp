@@ -165,6 +165,13 @@ bool any_requires_grad(std::initializer_list<const Tensor*> tensors) {
   return false;
 }
 
+// There is no forward-mode formula: an input with a tangent must not lose it in silence.
+void refuse_tangents(std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
+                                "forward-mode differentiation of the attention operators is not implemented");
+}
+
 // Hangs a node behind `out` (a fresh tensor). `bias_arg`: the attn_mask the caller gave, or undefined.
 std::shared_ptr<AttentionBackward> new_node(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& bias_arg, bool causal,
                                             double scale, double dropout_p) {
@@ -198,6 +205,7 @@ using PackedOp = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>(const Tensor
 std::tuple<Tensor, Tensor, Tensor, Tensor, int64_t, int64_t, Tensor, Tensor, Tensor> dense_with_grad(
     const Tensor& q, const Tensor& k, const Tensor& v, double dropout_p, bool is_causal, bool return_debug_mask,
     c10::optional<double> scale) {
+  refuse_tangents({&q, &k, &v});
   static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_scaled_dot_product_flash_attention", "").typed<DenseOp>();
   auto r = [&] {
     at::AutoDispatchBelowADInplaceOrView guard;
@@ -218,6 +226,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> packed_with_grad(const Tensor
                                                                     const Tensor& cu_q, const Tensor& cu_k, int64_t max_q,
                                                                     int64_t max_k, double dropout_p, bool is_causal,
                                                                     bool return_debug_mask, c10::optional<double> scale) {
+  refuse_tangents({&q, &k, &v});
   static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_flash_attention_forward", "").typed<PackedOp>();
   auto r = [&] {
     at::AutoDispatchBelowADInplaceOrView guard;
@@ -269,6 +278,7 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
     return {};
   if (at::cuda::getDeviceProperties(q.get_device())->major != 10) return {};
   const double sc = scale_or_default(q, scale);
+  refuse_tangents({&q, &k, &v});
 
   if (!has_mask) {
     DropoutResult r = [&] {
@@ -290,6 +300,7 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
       !mask.is_cuda() || mask.device() != q.device() || mask.unsafeGetTensorImpl()->is_python_dispatch() ||
       !(mask.scalar_type() == at::kBool || at::isFloatingType(mask.scalar_type())))
     return {};
+  refuse_tangents({&mask});
   c10::cuda::CUDAGuard device_guard(q.device());
   const bool boolean = mask.scalar_type() == at::kBool;
   const Tensor bias_arg = boolean ? Tensor() : mask.to(dtype);  // (differentiable) conversion of a bias of another type
