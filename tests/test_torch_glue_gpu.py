@@ -238,3 +238,66 @@ def test_forward_mode_raises(cuda_device, native_lib, which, requires_grad):
             with pytest.raises(NotImplementedError):
                 torch.ops.b200_sdpa._flash_attention_forward(q[0].transpose(0, 1), k[0].transpose(0, 1), v[0].transpose(0, 1), cu, cu,
                                                              128, 128, 0.0, False, False)
+
+
+def _qkv_and_bias(dev, requires_grad=False):
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(2, 4, 128, 64, generator=g).bfloat16().to(dev).requires_grad_(requires_grad) for _ in range(3))
+    return q, k, v, torch.randn(1, 4, 128, 128, generator=g).bfloat16().to(dev)
+
+
+class _Logged(torch.Tensor):
+    seen = []
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        cls.seen.append(getattr(func, "__name__", str(func)))
+        return super().__torch_function__(func, types, args, kwargs or {})
+
+
+class _FunctionLog(torch.overrides.TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(str(func))
+        return func(*args, **(kwargs or {}))
+
+
+def test_package_function_is_seen_by_torch_function(cuda_device, native_lib):
+    """Subclasses and modes with __torch_function__ see the attention operator, and a subclass comes back as one."""
+    from torch_mlu_b200 import sdp_choice
+    q, k, v, _ = _qkv_and_bias(cuda_device)
+    want = sdp_choice.scaled_dot_product_attention(q, k, v)
+    out = sdp_choice.scaled_dot_product_attention(q.as_subclass(_Logged), k, v)
+    assert type(out) is _Logged and "_scaled_dot_product_flash_attention" in _Logged.seen and torch.equal(out.as_subclass(torch.Tensor), want)
+    with _FunctionLog() as log:
+        assert torch.equal(sdp_choice.scaled_dot_product_attention(q, k, v), want)
+    assert any("_scaled_dot_product_flash_attention" in f for f in log.seen)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+def test_package_function_under_transforms_and_tracing(cuda_device, native_lib, masked):
+    """Wrapped tensors do not reach the kernels: what has no rule for them raises, as the operators do, or gives the same result."""
+    from torch_mlu_b200 import sdp_choice
+    q, k, v, bias = _qkv_and_bias(cuda_device)
+    mask = bias if masked else None
+    f = lambda q, k, v: sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=mask)
+    want = f(q, k, v)
+    if masked:
+        with pytest.raises(RuntimeError, match="setup_context"):
+            torch.func.functionalize(f)(q, k, v)
+        traced = torch.jit.trace(f, (q, k, v), check_trace=False)
+        q2 = torch.flip(q, [0])
+        assert torch.equal(traced(q2, k, v), f(q2, k, v))
+    else:
+        assert torch.equal(torch.func.functionalize(f)(q, k, v), want)
+        with pytest.raises(RuntimeError, match="[Bb]atching rule"):
+            torch.func.vmap(f)(*(torch.stack([t, t]) for t in (q, k, v)))
+    with pytest.raises((RuntimeError, NotImplementedError)):
+        torch.func.jvp(lambda q: f(q, k, v), (q,), (torch.ones_like(q),))
+    with pytest.raises(RuntimeError, match="torch.func|functorch"):
+        torch.func.grad(lambda q: f(q, k, v).float().sum())(q)
+    neg = torch._neg_view(q)  # a lazily negated view of q: its memory holds q, not -q
+    assert torch.equal(f(neg, k, v), f(-q, k, v)) or masked

@@ -2,6 +2,7 @@
 // tensors to launched kernels. The calls these functions serve run for 5 to 20 us on the GPU when the problem is small (a
 // decode step, a short prompt), and building the 90-field parameter block field by field through ctypes took the host
 // 50 to 60 us per call; here a call costs 5 to 10 us, most of it the CUDA launches.
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
@@ -197,9 +198,12 @@ PyObject* py_flash_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t n
 PyObject* py_sdpa(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect_args(n, 7);
-  for (int i = 0; i < 3; ++i)
-    if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
-  if (a[3] != Py_None && !THPVariable_Check(a[3])) Py_RETURN_NONE;
+  // a subclass, or a mode with __torch_function__, sees the operators of the Python procedure
+  if (at::impl::torch_function_mode_enabled()) Py_RETURN_NONE;
+  for (int i = 0; i < 4; ++i)
+    if (!(i == 3 && a[3] == Py_None) && !THPVariable_CheckExact(a[i])) Py_RETURN_NONE;
+  auto number = [](PyObject* o) { return PyFloat_Check(o) || PyLong_Check(o); };
+  if (!number(a[4]) || (a[6] != Py_None && !number(a[6]))) Py_RETURN_NONE;
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
   const c10::optional<Tensor> mask = optional_tensor(a[3], "attn_mask");
   const double p = float_arg(a[4]);

@@ -7,12 +7,14 @@
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/library.h>
 
 #include "torch_glue.h"
@@ -165,11 +167,34 @@ bool any_requires_grad(std::initializer_list<const Tensor*> tensors) {
   return false;
 }
 
+// An ordinary CUDA tensor, without wrappers, lazy conjugate or negative bits or a Python dispatch of its own: what the kernels
+// may be handed without the dispatcher.
+bool plain(const Tensor& t) {
+  constexpr c10::DispatchKeySet ordinary(
+      {c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::AutocastCUDA});
+  return ordinary.has_all(t.key_set());
+}
+
+// Nobody wants to see the operators of this thread: no dispatch mode, functional transform, functionalisation or tracing, and
+// autograd not switched off below the dispatcher.
+bool dispatcher_may_be_skipped() {
+  const auto tls = c10::impl::tls_local_dispatch_key_set();
+  return c10::default_included_set.has_all(tls.included_) && !tls.excluded_.has_all(c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA)) &&
+         !c10::impl::TorchDispatchModeTLS::any_modes_set() && !torch::jit::tracer::isTracing();
+}
+
 // There is no forward-mode formula: an input with a tangent must not lose it in silence.
 void refuse_tangents(std::initializer_list<const Tensor*> tensors) {
   for (const Tensor* t : tensors)
     TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
                                 "forward-mode differentiation of the attention operators is not implemented");
+}
+
+// The nodes below are not made for the levels of torch.func: a second derivative would be lost.
+void refuse_transforms(std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors)
+    TORCH_CHECK(!t->key_set().has(c10::DispatchKey::FuncTorchGradWrapper),
+                "the attention operators cannot be differentiated with torch.func transforms (grad, vjp, jacrev, ...)");
 }
 
 // Hangs a node behind `out` (a fresh tensor). `bias_arg`: the attn_mask the caller gave, or undefined.
@@ -212,6 +237,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, int64_t, int64_t, Tensor, Tensor, Ten
     return op.call(q, k, v, dropout_p, is_causal, return_debug_mask, scale);
   }();
   if (any_requires_grad({&q, &k, &v})) {
+    refuse_transforms({&q, &k, &v});
     auto node = new_node(q, k, v, Tensor(), is_causal, scale_or_default(q, scale), dropout_p);
     node->max_q = q.size(2);
     node->max_k = k.size(2);
@@ -233,6 +259,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> packed_with_grad(const Tensor
     return op.call(q, k, v, cu_q, cu_k, max_q, max_k, dropout_p, is_causal, return_debug_mask, scale);
   }();
   if (any_requires_grad({&q, &k, &v})) {
+    refuse_transforms({&q, &k, &v});
     auto node = new_node(q, k, v, Tensor(), is_causal, scale_or_default(q, scale), dropout_p);
     node->packed = true;
     node->max_q = max_q;
@@ -256,18 +283,17 @@ bool broadcasts_to(const Tensor& t, const int64_t (&full)[4]) {
 }  // namespace
 
 // The checks are those of sdp_choice.py (sdp_utils.h:99-455): a call that fails one of them, or whose answer depends on more
-// than they say (autocast, tensor subclasses, a top-left causal mask over unequal lengths), gets an undefined tensor, and
-// the Python function goes through the whole procedure with its warnings and errors.
+// than they say (autocast, wrapped tensors, dispatch modes, transforms, tracing, a top-left causal mask over unequal lengths), gets
+// an undefined tensor, and the Python function goes through the whole procedure with its warnings and errors.
 Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::optional<Tensor>& attn_mask, double dropout_p,
             bool is_causal, c10::optional<double> scale) {
   const auto& ctx = at::globalContext();
   const bool flash = ctx.userEnabledFlashSDP(), efficient = ctx.userEnabledMemEfficientSDP();
   const bool has_mask = attn_mask.has_value() && attn_mask->defined();
   if (!(efficient || (flash && !has_mask))) return {};
-  if (at::autocast::is_autocast_enabled(at::kCUDA) || c10::impl::TorchDispatchModeTLS::any_modes_set()) return {};
+  if (at::autocast::is_autocast_enabled(at::kCUDA) || !dispatcher_may_be_skipped()) return {};
   for (const Tensor* t : {&q, &k, &v}) {
-    if (!t->is_cuda() || t->is_nested() || t->dim() != 4 || t->layout() != at::kStrided ||
-        t->unsafeGetTensorImpl()->is_python_dispatch() || t->stride(-1) != 1 || t->scalar_type() != q.scalar_type() ||
+    if (!plain(*t) || t->dim() != 4 || t->layout() != at::kStrided || t->stride(-1) != 1 || t->scalar_type() != q.scalar_type() ||
         t->size(0) != q.size(0) || t->size(1) != q.size(1) || t->size(3) != q.size(3) || t->device() != q.device())
       return {};
   }
@@ -297,7 +323,7 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
   const Tensor& mask = *attn_mask;
   const int64_t full[4] = {q.size(0), q.size(1), Lq, Lk};
   if (!efficient || D > 128 || dropout_p != 0.0 || mask.dim() < 1 || mask.dim() > 4 || !broadcasts_to(mask, full) || mask.stride(-1) != 1 ||
-      !mask.is_cuda() || mask.device() != q.device() || mask.unsafeGetTensorImpl()->is_python_dispatch() ||
+      !plain(mask) || mask.device() != q.device() ||
       !(mask.scalar_type() == at::kBool || at::isFloatingType(mask.scalar_type())))
     return {};
   refuse_tangents({&mask});
