@@ -301,3 +301,70 @@ def test_package_function_under_transforms_and_tracing(cuda_device, native_lib, 
         torch.func.grad(lambda q: f(q, k, v).float().sum())(q)
     neg = torch._neg_view(q)  # a lazily negated view of q: its memory holds q, not -q
     assert torch.equal(f(neg, k, v), f(-q, k, v)) or masked
+
+
+class _DispatchLog(torch.utils._python_dispatch.TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(str(func))
+        return func(*args, **(kwargs or {}))
+
+
+def _call(form, q, k, v, bias, dropout_p=0.0):
+    """The package's function or a registered operator on the same values; `form` also names the backward operator's suffix."""
+    from torch_mlu_b200 import sdp_choice
+    if form == "packed":
+        cu = torch.arange(q.size(0) + 1, device=q.device, dtype=torch.int32) * q.size(2)
+        tokens = [t.transpose(1, 2).flatten(0, 1) for t in (q, k, v)]
+        return torch.ops.b200_sdpa._flash_attention_forward(*tokens, cu, cu, q.size(2), q.size(2), dropout_p, False, False)[0]
+    return sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=bias if form == "bias" else None, dropout_p=dropout_p)
+
+
+BACKWARD_OPS = {"dense": "b200_sdpa._scaled_dot_product_flash_attention_backward.default",
+                "packed": "b200_sdpa._flash_attention_backward.default", "bias": "b200_sdpa._bias_attention_backward.default"}
+
+
+@pytest.mark.parametrize("form", ["dense", "packed", "bias"])
+def test_dispatch_modes_see_the_backward(cuda_device, native_lib, form):
+    q, k, v, bias = _qkv_and_bias(cuda_device, requires_grad=True)
+    bias.requires_grad_()
+    inputs = (q, k, v, bias) if form == "bias" else (q, k, v)
+    out = _call(form, q, k, v, bias)
+    go = torch.randn_like(out)
+    want = torch.autograd.grad(out, inputs, go, retain_graph=True)
+    with _DispatchLog() as log:
+        got = torch.autograd.grad(out, inputs, go)
+    assert BACKWARD_OPS[form] in log.seen, log.seen
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dropout_p", [0.0, 0.1])
+@pytest.mark.parametrize("form", ["dense", "packed"])
+def test_make_fx_records_the_backward(cuda_device, native_lib, form, dropout_p):
+    """The traced program computes the gradients of the inputs it is given, not those of the tracing call."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    q, k, v, _ = _qkv_and_bias(cuda_device, requires_grad=True)
+
+    def step(q, k, v):
+        out = _call(form, q, k, v, None, dropout_p)
+        return torch.autograd.grad(out, (q, k, v), torch.ones_like(out))
+
+    traced = make_fx(step)(q, k, v)
+    assert BACKWARD_OPS[form] in [str(n.target) for n in traced.graph.nodes]
+    if dropout_p == 0.0:
+        q2, k2, v2 = (torch.flip(t.detach(), [0]).requires_grad_() for t in (q, k, v))
+        for a, b in zip(traced(q2, k2, v2), step(q2, k2, v2)):
+            assert torch.equal(a, b)
+
+
+def test_batched_gradients(cuda_device, native_lib):
+    q, k, v, _ = _qkv_and_bias(cuda_device, requires_grad=True)
+    out = _call("dense", q, k, v, None)
+    go = torch.randn(2, *out.shape, device=cuda_device, dtype=out.dtype)
+    got = torch.autograd.grad(out, (q, k, v), go, is_grads_batched=True, retain_graph=True)
+    for i in range(2):
+        for a, b in zip(got, torch.autograd.grad(out, (q, k, v), go[i], retain_graph=True)):
+            assert torch.equal(a[i], b)

@@ -32,6 +32,22 @@ void check_status(int st, const char* what) {
   throw StatusError(st, c10::str(what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error()));
 }
 
+// An ordinary CUDA tensor, without wrappers, lazy conjugate or negative bits or a Python dispatch of its own: what the kernels
+// may be handed without the dispatcher.
+bool plain(const Tensor& t) {
+  constexpr c10::DispatchKeySet ordinary(
+      {c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::AutocastCUDA});
+  return ordinary.has_all(t.key_set());
+}
+
+// Nobody wants to see the operators of this thread: no dispatch mode, functional transform, functionalisation or tracing, and
+// autograd not switched off below the dispatcher.
+bool dispatcher_may_be_skipped() {
+  const auto tls = c10::impl::tls_local_dispatch_key_set();
+  return c10::default_included_set.has_all(tls.included_) && !tls.excluded_.has_all(c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA)) &&
+         !c10::impl::TorchDispatchModeTLS::any_modes_set() && !torch::jit::tracer::isTracing();
+}
+
 // ------------------------------------------------------------------------- additive bias
 int64_t ceil8(int64_t n) { return (n + 7) / 8 * 8; }
 
@@ -87,6 +103,26 @@ Tensor transposed_bias(const Tensor& bias) {
   return buf.narrow(-1, 0, Lq).expand({B, H, Lk, Lq});
 }
 
+// The backward of a dense call with a bias: dq, dk, dv and, when it is wanted, the gradient of the bias before it is summed over
+// the dimensions the bias is broadcast along.
+std::tuple<Tensor, Tensor, Tensor, Tensor> bias_backward(const Tensor& grad_out, const Tensor& q, const Tensor& k, const Tensor& v,
+                                                         const Tensor& bias, const Tensor& out, const Tensor& lse, bool bias_padded,
+                                                         bool causal, bool want_dbias, double scale) {
+  c10::cuda::CUDAGuard device_guard(q.device());
+  const Tensor view = prepare_bias(bias, q, k.size(2), bias_padded);
+  Tensor dbias;
+  if (want_dbias)  // zero-filled: the kernels skip what the causal mask hides
+    dbias = at::zeros({q.size(0), q.size(1), q.size(2), ceil8(k.size(2))}, q.options()).narrow(-1, 0, k.size(2));
+  const Tensor bias_t = transposed_bias(view);
+  BackwardOptions opt;
+  opt.bias = &view;
+  opt.dbias = &dbias;
+  opt.bias_t = &bias_t;
+  auto [dq, dk, dv] = dense_backward(grad_out, q, k, v, out, lse, causal, scale, opt);
+  if (!want_dbias) dbias = at::empty({0}, q.options());
+  return {dq, dk, dv, dbias};
+}
+
 // ------------------------------------------------------------------------- autograd
 using DenseBackwardOp = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
                                                            const Tensor&, const Tensor&, const Tensor&, int64_t, int64_t, double,
@@ -117,23 +153,21 @@ struct AttentionBackward : public torch::autograd::Node {
     const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), out_ = out.unpack(shared_from_this()), lse_ = lse.unpack();
     const Tensor seed_ = seed.unpack(), offset_ = offset.unpack();
     Tensor dq, dk, dv;
+    // Through the operators where somebody wants to see them: create_graph=True, dispatch modes, tracing, wrapped gradients
+    bool direct = !at::GradMode::is_enabled() && dispatcher_may_be_skipped();
+    for (const Tensor* t : {&go, &q_, &k_, &v_, &out_, &lse_}) direct = direct && plain(*t);
     if (has_bias) {
-      const Tensor saved_bias = bias.unpack();
-      at::AutoDispatchBelowADInplaceOrView guard;
-      c10::cuda::CUDAGuard device_guard(q_.device());
-      const Tensor bias_ = prepare_bias(saved_bias, q_, k_.size(2), bias_padded);
+      const Tensor bias_ = bias.unpack();
       Tensor dbias;
-      if (want_dbias)  // zero-filled: the kernels skip what the causal mask hides
-        dbias = at::zeros({q_.size(0), q_.size(1), q_.size(2), ceil8(k_.size(2))}, q_.options()).narrow(-1, 0, k_.size(2));
-      const Tensor bias_t = transposed_bias(bias_);
-      BackwardOptions opt;
-      opt.bias = &bias_;
-      opt.dbias = &dbias;
-      opt.bias_t = &bias_t;
-      std::tie(dq, dk, dv) = dense_backward(go, q_, k_, v_, out_, lse_, causal, scale, opt);
+      if (direct && plain(bias_)) {
+        at::AutoDispatchBelowADInplaceOrView guard;
+        std::tie(dq, dk, dv, dbias) = bias_backward(go, q_, k_, v_, bias_, out_, lse_, bias_padded, causal, want_dbias, scale);
+      } else {
+        static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_bias_attention_backward", "").typed<decltype(bias_backward)>();
+        std::tie(dq, dk, dv, dbias) = op.call(go, q_, k_, v_, bias_, out_, lse_, bias_padded, causal, want_dbias, scale);
+      }
       if (want_dbias) result[3] = at::sum_to(dbias, bias_sizes);
-    } else if (at::GradMode::is_enabled()) {
-      // create_graph=True: through the operators, so that whatever autograd knows about them applies
+    } else if (!direct) {
       if (packed) {
         static auto op = c10::Dispatcher::singleton()
                              .findSchemaOrThrow("b200_sdpa::_flash_attention_backward", "").typed<DenseBackwardOp>();
@@ -165,22 +199,6 @@ bool any_requires_grad(std::initializer_list<const Tensor*> tensors) {
   for (const Tensor* t : tensors)
     if (t->defined() && t->requires_grad()) return true;
   return false;
-}
-
-// An ordinary CUDA tensor, without wrappers, lazy conjugate or negative bits or a Python dispatch of its own: what the kernels
-// may be handed without the dispatcher.
-bool plain(const Tensor& t) {
-  constexpr c10::DispatchKeySet ordinary(
-      {c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::AutocastCUDA});
-  return ordinary.has_all(t.key_set());
-}
-
-// Nobody wants to see the operators of this thread: no dispatch mode, functional transform, functionalisation or tracing, and
-// autograd not switched off below the dispatcher.
-bool dispatcher_may_be_skipped() {
-  const auto tls = c10::impl::tls_local_dispatch_key_set();
-  return c10::default_included_set.has_all(tls.included_) && !tls.excluded_.has_all(c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA)) &&
-         !c10::impl::TorchDispatchModeTLS::any_modes_set() && !torch::jit::tracer::isTracing();
 }
 
 // There is no forward-mode formula: an input with a tangent must not lose it in silence.
@@ -354,6 +372,15 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
 }
 
 }  // namespace b200_glue
+
+TORCH_LIBRARY_FRAGMENT(b200_sdpa, m) {
+  m.def("_bias_attention_backward(Tensor grad_out, Tensor query, Tensor key, Tensor value, Tensor bias, Tensor out, Tensor logsumexp, "
+        "bool bias_padded, bool is_causal, bool want_dbias, float scale) -> (Tensor, Tensor, Tensor, Tensor)");
+}
+
+TORCH_LIBRARY_IMPL(b200_sdpa, CUDA, m) {
+  m.impl("_bias_attention_backward", b200_glue::bias_backward);
+}
 
 TORCH_LIBRARY_IMPL(b200_sdpa, AutogradCUDA, m) {
   m.impl("_scaled_dot_product_flash_attention", b200_glue::dense_with_grad);
