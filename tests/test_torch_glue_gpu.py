@@ -368,3 +368,36 @@ def test_batched_gradients(cuda_device, native_lib):
     for i in range(2):
         for a, b in zip(got, torch.autograd.grad(out, (q, k, v), go[i], retain_graph=True)):
             assert torch.equal(a[i], b)
+
+
+@pytest.mark.parametrize("dropout_p", [0.0, 0.1])
+@pytest.mark.parametrize("form", ["dense", "packed", "bias", "mask"])
+def test_compiled_autograd(cuda_device, native_lib, form, dropout_p):
+    """The recorded backward, run again on other values, gives what the eager one does."""
+    from torch._dynamo import compiled_autograd
+    from torch_mlu_b200 import sdp_choice
+    if dropout_p > 0.0 and form in ("bias", "mask"):
+        pytest.skip("dropout with an attn_mask has its own Python autograd function")
+    torch._dynamo.reset()
+    graphs = []
+
+    def grads(seed, compiled):
+        q, k, v, bias = (torch.flip(t, [0]) if seed else t.clone() for t in _qkv_and_bias(cuda_device))
+        inputs = [t.requires_grad_() for t in ((q, k, v, bias) if form == "bias" else (q, k, v))]
+        torch.cuda.manual_seed(seed)
+        if form == "mask":
+            out = sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=bias > -1)
+        else:
+            out = _call(form, q, k, v, bias, dropout_p)
+        if compiled:
+            with compiled_autograd._enable(lambda gm: (graphs.append(gm), gm)[1]):
+                out.float().sum().backward()
+        else:
+            out.float().sum().backward()
+        return [t.grad for t in inputs]
+
+    for seed in (0, 1):
+        for a, b in zip(grads(seed, True), grads(seed, False)):
+            assert torch.equal(a, b)
+    names = [str(n.target) for gm in graphs for n in gm.graph.nodes]
+    assert any("B200AttentionBackward" in n for n in names), names

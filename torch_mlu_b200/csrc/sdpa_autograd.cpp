@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/library.h>
 
@@ -128,68 +129,140 @@ using DenseBackwardOp = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const 
                                                            const Tensor&, const Tensor&, const Tensor&, int64_t, int64_t, double,
                                                            bool, const Tensor&, const Tensor&, c10::optional<double>);
 
-// One node for all forms: dense, dense with an additive bias, packed.
+// What a backward needs besides the incoming gradient. One form for all calls: dense, dense with an additive bias, packed.
+struct BackwardCall {
+  bool packed = false, causal = false, has_bias = false, bias_padded = false, want_dbias = false;
+  int64_t max_q = 0, max_k = 0;
+  double scale = 1.0, dropout_p = 0.0;
+  std::vector<int64_t> bias_sizes;  // shape of the attn_mask argument, when its gradient is wanted
+};
+struct BackwardTensors {
+  Tensor q, k, v, out, lse;
+  Tensor cu_q, cu_k;    // packed
+  Tensor seed, offset;  // without a bias
+  Tensor bias;          // as saved by the node
+
+  // those the form has, in a fixed order
+  std::vector<Tensor*> used(const BackwardCall& c) {
+    std::vector<Tensor*> t = {&q, &k, &v, &out, &lse};
+    if (c.packed) t.insert(t.end(), {&cu_q, &cu_k});
+    if (c.has_bias) t.push_back(&bias);
+    else t.insert(t.end(), {&seed, &offset});
+    return t;
+  }
+};
+
+// Gradients of query, key, value and (with a bias) the bias, undefined where `needs` says so.
+variable_list run_backward(const Tensor& go, const BackwardCall& c, const BackwardTensors& t, const std::vector<bool>& needs) {
+  variable_list result(needs.size());
+  if (!go.defined()) return result;
+  Tensor dq, dk, dv;
+  // Through the operators where somebody wants to see them: create_graph=True, dispatch modes, tracing, wrapped gradients
+  bool direct = !at::GradMode::is_enabled() && dispatcher_may_be_skipped();
+  for (const Tensor* x : {&go, &t.q, &t.k, &t.v, &t.out, &t.lse}) direct = direct && plain(*x);
+  if (c.has_bias) {
+    Tensor dbias;
+    if (direct && plain(t.bias)) {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      std::tie(dq, dk, dv, dbias) = bias_backward(go, t.q, t.k, t.v, t.bias, t.out, t.lse, c.bias_padded, c.causal, c.want_dbias, c.scale);
+    } else {
+      static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_bias_attention_backward", "").typed<decltype(bias_backward)>();
+      std::tie(dq, dk, dv, dbias) = op.call(go, t.q, t.k, t.v, t.bias, t.out, t.lse, c.bias_padded, c.causal, c.want_dbias, c.scale);
+    }
+    if (c.want_dbias) result[3] = at::sum_to(dbias, c.bias_sizes);
+  } else if (!direct) {
+    if (c.packed) {
+      static auto op = c10::Dispatcher::singleton()
+                           .findSchemaOrThrow("b200_sdpa::_flash_attention_backward", "").typed<DenseBackwardOp>();
+      std::tie(dq, dk, dv) = op.call(go, t.q, t.k, t.v, t.out, t.lse, t.cu_q, t.cu_k, c.max_q, c.max_k, c.dropout_p, c.causal, t.seed,
+                                     t.offset, c.scale);
+    } else {
+      static auto op = c10::Dispatcher::singleton()
+                           .findSchemaOrThrow("b200_sdpa::_scaled_dot_product_flash_attention_backward", "").typed<DenseBackwardOp>();
+      const Tensor none = at::empty({0}, t.q.options().dtype(at::kInt));
+      std::tie(dq, dk, dv) = op.call(go, t.q, t.k, t.v, t.out, t.lse, none, none, c.max_q, c.max_k, c.dropout_p, c.causal, t.seed,
+                                     t.offset, c.scale);
+    }
+  } else {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    if (c.packed)
+      std::tie(dq, dk, dv) = varlen_backward_with_dropout(go, t.q, t.k, t.v, t.out, t.lse, t.cu_q, t.cu_k, c.max_q, c.max_k, c.dropout_p,
+                                                          c.causal, t.seed, t.offset, c.scale);
+    else
+      std::tie(dq, dk, dv) = dense_backward_with_dropout(go, t.q, t.k, t.v, t.out, t.lse, c.dropout_p, c.causal, t.seed, t.offset,
+                                                         c.scale);
+  }
+  if (needs[0]) result[0] = dq;
+  if (needs[1]) result[1] = dk;
+  if (needs[2]) result[2] = dv;
+  return result;
+}
+
 struct AttentionBackward : public torch::autograd::Node {
   SavedVariable q, k, v, out, lse, cu_q, cu_k, seed, offset;
   // dense with a bias: the caller's own tensor (a change in place before the backward is noticed), or what mask_bias() made
   SavedVariable bias;
-  std::vector<int64_t> bias_sizes;   // shape of the attn_mask argument, when its gradient is wanted
-  bool packed = false, causal = false, has_bias = false, bias_padded = false, want_dbias = false;
-  int64_t max_q = 0, max_k = 0;
-  double scale = 1.0, dropout_p = 0.0;
+  BackwardCall call;
 
   std::string name() const override { return "B200AttentionBackward"; }
+  std::array<SavedVariable*, 10> saved() { return {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset, &bias}; }
+
+  BackwardTensors unpack() {
+    return {q.unpack(), k.unpack(), v.unpack(), out.unpack(shared_from_this()), lse.unpack(), cu_q.unpack(),
+            cu_k.unpack(), seed.unpack(), offset.unpack(), bias.unpack()};
+  }
+
+  std::vector<bool> needs() const {
+    std::vector<bool> n(num_outputs());
+    for (size_t i = 0; i < n.size(); ++i) n[i] = task_should_compute_output(i);
+    return n;
+  }
 
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset, &bias}) s->reset_data();
+    for (SavedVariable* s : saved()) s->reset_data();
   }
 
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    variable_list result(num_outputs());
-    if (!grads[0].defined()) return result;
-    const Tensor& go = grads[0];
-    const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), out_ = out.unpack(shared_from_this()), lse_ = lse.unpack();
-    const Tensor seed_ = seed.unpack(), offset_ = offset.unpack();
-    Tensor dq, dk, dv;
-    // Through the operators where somebody wants to see them: create_graph=True, dispatch modes, tracing, wrapped gradients
-    bool direct = !at::GradMode::is_enabled() && dispatcher_may_be_skipped();
-    for (const Tensor* t : {&go, &q_, &k_, &v_, &out_, &lse_}) direct = direct && plain(*t);
-    if (has_bias) {
-      const Tensor bias_ = bias.unpack();
-      Tensor dbias;
-      if (direct && plain(bias_)) {
-        at::AutoDispatchBelowADInplaceOrView guard;
-        std::tie(dq, dk, dv, dbias) = bias_backward(go, q_, k_, v_, bias_, out_, lse_, bias_padded, causal, want_dbias, scale);
-      } else {
-        static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_bias_attention_backward", "").typed<decltype(bias_backward)>();
-        std::tie(dq, dk, dv, dbias) = op.call(go, q_, k_, v_, bias_, out_, lse_, bias_padded, causal, want_dbias, scale);
-      }
-      if (want_dbias) result[3] = at::sum_to(dbias, bias_sizes);
-    } else if (!direct) {
-      if (packed) {
-        static auto op = c10::Dispatcher::singleton()
-                             .findSchemaOrThrow("b200_sdpa::_flash_attention_backward", "").typed<DenseBackwardOp>();
-        std::tie(dq, dk, dv) = op.call(go, q_, k_, v_, out_, lse_, cu_q.unpack(), cu_k.unpack(), max_q, max_k, dropout_p, causal,
-                                       seed_, offset_, scale);
-      } else {
-        static auto op = c10::Dispatcher::singleton()
-                             .findSchemaOrThrow("b200_sdpa::_scaled_dot_product_flash_attention_backward", "").typed<DenseBackwardOp>();
-        const Tensor none = at::empty({0}, q_.options().dtype(at::kInt));
-        std::tie(dq, dk, dv) = op.call(go, q_, k_, v_, out_, lse_, none, none, max_q, max_k, dropout_p, causal, seed_, offset_, scale);
-      }
-    } else {
-      at::AutoDispatchBelowADInplaceOrView guard;
-      if (packed)
-        std::tie(dq, dk, dv) = varlen_backward_with_dropout(go, q_, k_, v_, out_, lse_, cu_q.unpack(), cu_k.unpack(), max_q, max_k,
-                                                            dropout_p, causal, seed_, offset_, scale);
-      else
-        std::tie(dq, dk, dv) = dense_backward_with_dropout(go, q_, k_, v_, out_, lse_, dropout_p, causal, seed_, offset_, scale);
+    if (!grads[0].defined()) return variable_list(num_outputs());
+    return run_backward(grads[0], call, unpack(), needs());
+  }
+
+  // Compiled autograd: everything a recorded call depends on, then the call itself, recorded as a function of the incoming
+  // gradient and the saved tensors.
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    for (SavedVariable* s : const_cast<AttentionBackward*>(this)->saved()) args.collect(*s, /*is_output=*/s == &out);
+    args.collect(call.bias_sizes);
+    for (const bool flag : {call.packed, call.causal, call.has_bias, call.bias_padded, call.want_dbias}) args.collect(flag);
+    args.collect(call.max_q);
+    args.collect(call.max_k);
+    args.collect(call.scale);
+    args.collect(call.dropout_p);
+  }
+
+  variable_list apply_with_saved(const variable_list& inputs, torch::dynamo::autograd::SwapSavedVariables& swap) override {
+    namespace ca = torch::dynamo::autograd;
+    for (SavedVariable* s : saved()) swap.before(*s);
+    BackwardTensors tensors = unpack();
+    ca::ivalue_list args;
+    std::vector<at::TypePtr> types;
+    for (const Tensor* t : tensors.used(call)) {
+      args.push_back(ca::IValuePacker<Tensor>::pack(*t));
+      types.push_back(ca::IValuePacker<Tensor>::packed_type());
     }
-    if (task_should_compute_output(0)) result[0] = dq;
-    if (task_should_compute_output(1)) result[1] = dk;
-    if (task_should_compute_output(2)) result[2] = dv;
+    auto recorded = [c = call, n = needs()](const variable_list& grads, const ca::ivalue_list& a) {
+      BackwardTensors t;
+      size_t i = 0;
+      for (Tensor* x : t.used(c)) *x = a[i++].toTensor();
+      return run_backward(grads[0], c, t, n);
+    };
+    const auto& compiler = ca::getPyCompilerInterface();
+    const std::string fn = compiler->bind_function(swap.get_py_compiler(), name(), recorded, types, /*is_custom_function=*/true);
+    variable_list result = compiler->call_function(
+        swap.get_py_compiler(), "apply_functional", fn, inputs, args,
+        ca::IValuePacker<std::vector<std::optional<torch::autograd::InputMetadata>>>::pack(ca::get_input_metadata(next_edges())));
+    for (SavedVariable* s : saved()) swap.after(*s);
     return result;
   }
 };
@@ -224,9 +297,9 @@ std::shared_ptr<AttentionBackward> new_node(const Tensor& q, const Tensor& k, co
   node->q = SavedVariable(q, false);
   node->k = SavedVariable(k, false);
   node->v = SavedVariable(v, false);
-  node->causal = causal;
-  node->scale = scale;
-  node->dropout_p = dropout_p;
+  node->call.causal = causal;
+  node->call.scale = scale;
+  node->call.dropout_p = dropout_p;
   return node;
 }
 
@@ -257,8 +330,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, int64_t, int64_t, Tensor, Tensor, Ten
   if (any_requires_grad({&q, &k, &v})) {
     refuse_transforms({&q, &k, &v});
     auto node = new_node(q, k, v, Tensor(), is_causal, scale_or_default(q, scale), dropout_p);
-    node->max_q = q.size(2);
-    node->max_k = k.size(2);
+    node->call.max_q = q.size(2);
+    node->call.max_k = k.size(2);
     Tensor lse = std::get<1>(r);
     if (lse.size(2) != q.size(2)) lse = lse.slice(2, 0, q.size(2)).contiguous();
     finish_node(node, std::get<0>(r), lse, std::get<6>(r), std::get<7>(r));
@@ -279,14 +352,38 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> packed_with_grad(const Tensor
   if (any_requires_grad({&q, &k, &v})) {
     refuse_transforms({&q, &k, &v});
     auto node = new_node(q, k, v, Tensor(), is_causal, scale_or_default(q, scale), dropout_p);
-    node->packed = true;
-    node->max_q = max_q;
-    node->max_k = max_k;
+    node->call.packed = true;
+    node->call.max_q = max_q;
+    node->call.max_k = max_k;
     node->cu_q = SavedVariable(cu_q, false);
     node->cu_k = SavedVariable(cu_k, false);
     finish_node(node, std::get<0>(r), std::get<1>(r), std::get<2>(r), std::get<3>(r));
   }
   return r;
+}
+
+// Shapes of the backward operators' results, for recorders that call them on tensors without data
+Tensor meta_like(const Tensor& t) {  // memory order of the kernels' outputs: [B, L, H, D] for a dense [B, H, L, D]
+  if (t.dim() != 4) return at::empty_symint(t.sym_sizes(), t.options());
+  const auto H = t.sym_size(1), L = t.sym_size(2), D = t.sym_size(3);
+  return at::empty_strided_symint(t.sym_sizes(), {L * H * D, D, H * D, 1}, t.options());
+}
+
+std::tuple<Tensor, Tensor, Tensor> meta_backward(const Tensor&, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&,
+                                                 const Tensor&, const Tensor&, const Tensor&, int64_t, int64_t, double, bool, const Tensor&,
+                                                 const Tensor&, c10::optional<double>) {
+  return {meta_like(q), meta_like(k), meta_like(v)};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> meta_bias_backward(const Tensor&, const Tensor& q, const Tensor& k, const Tensor& v,
+                                                              const Tensor&, const Tensor&, const Tensor&, bool, bool, bool want_dbias,
+                                                              double) {
+  Tensor dbias = at::empty({0}, q.options());
+  if (want_dbias) {
+    const auto Lk = k.sym_size(2);
+    dbias = at::empty_symint({q.sym_size(0), q.sym_size(1), q.sym_size(2), (Lk + 7) / 8 * 8}, q.options()).narrow_symint(-1, 0, Lk);
+  }
+  return {meta_like(q), meta_like(k), meta_like(v), dbias};
 }
 
 bool broadcasts_to(const Tensor& t, const int64_t (&full)[4]) {
@@ -331,8 +428,8 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
     }();
     if (any_requires_grad({&q, &k, &v})) {
       auto node = new_node(q, k, v, Tensor(), is_causal, sc, dropout_p);
-      node->max_q = Lq;
-      node->max_k = Lk;
+      node->call.max_q = Lq;
+      node->call.max_k = Lk;
       finish_node(node, r.out, r.lse, r.seed, r.offset);
     }
     return r.out;
@@ -359,12 +456,12 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
   }
   if (any_requires_grad({&q, &k, &v, &bias_arg})) {
     auto node = new_node(q, k, v, bias_arg, is_causal, sc, 0.0);
-    node->has_bias = true;
-    node->bias_padded = boolean;
+    node->call.has_bias = true;
+    node->call.bias_padded = boolean;
     node->bias = SavedVariable(boolean ? mask_buf : bias_arg, false);
     if (bias_arg.defined() && bias_arg.requires_grad()) {
-      node->want_dbias = true;
-      node->bias_sizes = bias_arg.sizes().vec();
+      node->call.want_dbias = true;
+      node->call.bias_sizes = bias_arg.sizes().vec();
     }
     finish_node(node, out, lse, Tensor(), Tensor());
   }
@@ -380,6 +477,12 @@ TORCH_LIBRARY_FRAGMENT(b200_sdpa, m) {
 
 TORCH_LIBRARY_IMPL(b200_sdpa, CUDA, m) {
   m.impl("_bias_attention_backward", b200_glue::bias_backward);
+}
+
+TORCH_LIBRARY_IMPL(b200_sdpa, Meta, m) {
+  m.impl("_scaled_dot_product_flash_attention_backward", b200_glue::meta_backward);
+  m.impl("_flash_attention_backward", b200_glue::meta_backward);
+  m.impl("_bias_attention_backward", b200_glue::meta_bias_backward);
 }
 
 TORCH_LIBRARY_IMPL(b200_sdpa, AutogradCUDA, m) {
