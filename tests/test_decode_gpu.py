@@ -134,3 +134,14 @@ def test_decode_split_count_does_not_change_the_answer_much(cuda_device, native_
     o_ref, l_ref = orc.cpu_sdpa_forward(c.q[1:2], c.k[1:2], c.v[1:2], scale=c.softmax_scale)
     orc.assert_close_bf16(base_o[1:2], o_ref, "out")
     orc.assert_close_lse(base_l[1:2], l_ref)
+
+
+@pytest.mark.parametrize("head_stride", [3, 12345])
+def test_decode_with_one_head_takes_any_head_stride(cuda_device, native_lib, head_stride):
+    dev = cuda_device
+    q, buf = rand((2, 4, 1, 128), 1).to(dev), rand((2, 70, 128), 2).to(dev)
+    k = buf[:, :64].unsqueeze(1)
+    odd = k.as_strided(k.shape, (k.stride(0), head_stride, k.stride(2), 1))
+    out, lse = ops.decode_attention(q, odd, odd)
+    want, want_lse = ops.decode_attention(q, k, k)
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)

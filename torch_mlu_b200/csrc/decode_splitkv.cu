@@ -624,11 +624,13 @@ int launch_decode(const sdpa_b200_params& p, DecodeParams& d, float* scratch, ui
   d.scale_log2 = p.softmax_scale * 1.4426950408889634f;
   d.f16 = f16;
   CUtensorMap tm_k, tm_v;
-  int st = make_tensor_map_16(f16, &tm_k, p.k, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.k_row_stride, p.k_head_stride,
-                              p.k_batch_stride, kKeysPerStep);
+  // the stride of a single head means nothing and may be any number, but the tensor map wants a legal one
+  const bool one_head = p.heads_kv == 1;
+  int st = make_tensor_map_16(f16, &tm_k, p.k, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.k_row_stride,
+                              one_head ? p.k_row_stride : p.k_head_stride, p.k_batch_stride, kKeysPerStep);
   if (st != SDPA_B200_OK) return st;
-  st = make_tensor_map_16(f16, &tm_v, p.v, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.v_row_stride, p.v_head_stride,
-                          p.v_batch_stride, kKeysPerStep);
+  st = make_tensor_map_16(f16, &tm_v, p.v, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.v_row_stride,
+                          one_head ? p.v_row_stride : p.v_head_stride, p.v_batch_stride, kKeysPerStep);
   if (st != SDPA_B200_OK) return st;
   const bool hi = d.rows > 8;
   cudaError_t err;
