@@ -401,3 +401,30 @@ def test_compiled_autograd(cuda_device, native_lib, form, dropout_p):
             assert torch.equal(a, b)
     names = [str(n.target) for gm in graphs for n in gm.graph.nodes]
     assert any("B200AttentionBackward" in n for n in names), names
+
+
+@pytest.mark.parametrize("view", ["expanded_rows", "expanded_all", "one_row", "odd_rows", "unaligned", "columns"])
+@pytest.mark.parametrize("form,D", [("dense", 64), ("dense", 256), ("packed", 128), ("bias", 64)])
+def test_gradients_of_any_layout(cuda_device, native_lib, form, D, view):
+    """What autograd hands back for sums, slices of concatenations and transposed consumers gives the gradients of its copy."""
+    B, H, L = 2, 4, 1 if view == "one_row" else 96
+    g = torch.Generator().manual_seed(2)
+    q, k, v = (torch.randn(B, H, L, D, generator=g).bfloat16().to(cuda_device).requires_grad_() for _ in range(3))
+    bias = torch.randn(1, H, L, L, generator=g).bfloat16().to(cuda_device)
+    out = _call(form, q, k, v, bias)
+    shape = out.shape
+    rows = 0 if form == "packed" else 2
+    if view in ("expanded_rows", "one_row"):
+        go = torch.randn([1 if i == rows else n for i, n in enumerate(shape)], generator=g).bfloat16().to(cuda_device).expand(shape)
+        go = go.as_strided(shape, [0 if i == rows else s for i, s in enumerate(go.stride())])
+    elif view == "expanded_all":
+        go = torch.randn([], generator=g).bfloat16().to(cuda_device).expand(shape)
+    elif view == "odd_rows":
+        go = torch.randn(*shape[:-1], D + 3, generator=g).bfloat16().to(cuda_device)[..., :D]
+    elif view == "unaligned":
+        go = torch.randn(*shape[:-1], D + 8, generator=g).bfloat16().to(cuda_device)[..., 1:D + 1]
+    else:
+        go = torch.randn(*shape[:-2], D, shape[-2], generator=g).bfloat16().to(cuda_device).transpose(-1, -2)
+    want = torch.autograd.grad(out, (q, k, v), go.clone(memory_format=torch.contiguous_format), retain_graph=True)
+    for a, b in zip(torch.autograd.grad(out, (q, k, v), go), want):
+        assert torch.equal(a, b)

@@ -60,6 +60,15 @@ void check_input(const Tensor& t, const char* name) {
 }
 
 
+// The incoming gradient as the kernels can read it. Autograd hands over views that they cannot: an expanded gradient (of a sum)
+// with strides of 0, a slice of the gradient of a concatenation with any strides and any address.
+Tensor readable_gradient(const Tensor& g) {
+  const int64_t rows = g.dim() - (g.dim() == 4 ? 2 : 3);  // [B, H, L, D] or [total, H, D]
+  bool ok = g.dim() >= 3 && g.stride(-1) == 1 && reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
+  for (int64_t i = 0; ok && i < g.dim() - 1; ++i) ok = (g.size(i) == 1 && i != rows) || (g.stride(i) > 0 && g.stride(i) % 8 == 0);
+  return ok ? g : g.clone(at::MemoryFormat::Contiguous);
+}
+
 void set_bhld(int64_t& bs, int64_t& hs, int64_t& rs, const Tensor& t) {
   bs = t.stride(0);
   hs = t.stride(1);
@@ -368,7 +377,7 @@ std::tuple<Tensor, Tensor> dense_forward(const Tensor& q, const Tensor& k, const
 std::tuple<Tensor, Tensor, Tensor> dense_backward(const Tensor& dout_in, const Tensor& q, const Tensor& k, const Tensor& v,
                                                   const Tensor& out, const Tensor& lse, bool causal, double scale,
                                                   const BackwardOptions& opt) {
-  Tensor dout = dout_in.stride(-1) == 1 ? dout_in : dout_in.contiguous();
+  const Tensor dout = readable_gradient(dout_in);
   check_input(dout, "grad_out");
   check_input(q, "query");
   check_input(k, "key");
@@ -496,7 +505,7 @@ std::tuple<Tensor, Tensor, Tensor> varlen_backward(const Tensor& dout_in, const 
                                                    const Tensor& cu_k, int64_t max_q, int64_t max_k, bool causal,
                                                    double scale, const BackwardOptions& opt) {
   check_varlen(q, k, v, cu_q, cu_k);
-  Tensor dout = dout_in.stride(-1) == 1 ? dout_in : dout_in.contiguous();
+  const Tensor dout = readable_gradient(dout_in);
   check_input(dout, "grad_out");
   check_input(out, "out");
   TORCH_CHECK(dout.scalar_type() == q.scalar_type() && out.scalar_type() == q.scalar_type(),
