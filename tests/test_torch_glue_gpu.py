@@ -428,3 +428,16 @@ def test_gradients_of_any_layout(cuda_device, native_lib, form, D, view):
     want = torch.autograd.grad(out, (q, k, v), go.clone(memory_format=torch.contiguous_format), retain_graph=True)
     for a, b in zip(torch.autograd.grad(out, (q, k, v), go), want):
         assert torch.equal(a, b)
+
+
+def test_outputs_are_filled_under_deterministic_algorithms(cuda_device, native_lib):
+    """torch fills memory that an operator leaves unwritten: here the rows of tokens that belong to no sequence."""
+    from torch_mlu_b200 import ops
+    q = torch.randn(300, 4, 64, device=cuda_device).bfloat16()
+    cu = torch.tensor([0, 100, 200], dtype=torch.int32, device=cuda_device)
+    torch.use_deterministic_algorithms(True)
+    try:
+        out, lse = ops._flash_attention_forward(q, q, q, cu, cu, 100, 100, 0.0, False, False)[:2]
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert out[200:].isnan().all() and lse[:, 200:].isnan().all() and not out[:200].isnan().any()

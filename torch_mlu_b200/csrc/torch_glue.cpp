@@ -40,14 +40,21 @@ void check_status(int st, const char* what) {
 }
 
 // Uninitialised device tensors without the dispatcher round trip of at::empty (a few hundred nanoseconds each, of calls
-// whose kernels run for a few microseconds).
+// whose kernels run for a few microseconds). Where torch promises a value for uninitialised memory (deterministic algorithms),
+// the dispatcher's functions are used, which write it.
+bool fills_uninitialised() {
+  return at::globalContext().deterministicAlgorithms() && at::globalContext().deterministicFillUninitializedMemory();
+}
+
 Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor& like) {
+  if (fills_uninitialised()) return at::empty(sizes, like.options().dtype(dtype));
   return at::detail::empty_cuda(sizes, dtype, like.device(), c10::nullopt);
 }
 
 // [B, H, L, D] tensor in the memory order of a [B, L, H, D] buffer, which the reference returns (attention.cpp:146-148)
 Tensor new_heads_second(int64_t B, int64_t H, int64_t L, int64_t D, const Tensor& like) {
   const int64_t sizes[4] = {B, H, L, D}, strides[4] = {L * H * D, D, H * D, 1};
+  if (fills_uninitialised()) return at::empty_strided(sizes, strides, like.options());
   return at::detail::empty_strided_cuda(sizes, strides, like.scalar_type(), like.device());
 }
 
