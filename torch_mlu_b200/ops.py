@@ -20,7 +20,7 @@ on a machine without the built library or without an sm_100 GPU raises.
 
 The calls themselves are made by csrc/py_calls.cpp (checks, outputs, parameter block and launch in one native call: a short
 decode or prefill is host-bound otherwise); the ``_*_params`` / ``_run_*`` helpers drive the C ABI field by field, for
-callers that bring their own output buffers.
+callers that bring their own output buffers and, in _FieldCalls, where that module is not available.
 """
 from __future__ import annotations
 
@@ -51,8 +51,8 @@ def calculate_scale(query: torch.Tensor, scale: Optional[float]) -> float:
 
 
 def _calls():
-    """The module of direct native calls (loaded on first use)."""
-    return torch_glue.calls or torch_glue.load()
+    """The module of direct native calls (loaded on first use), or the same calls through ctypes."""
+    return torch_glue.calls or torch_glue.calls_or_none() or _FieldCalls
 
 
 def _check(cond: bool, msg: str) -> None:
@@ -100,7 +100,9 @@ class _Workspace:
         bounded wait runs out leaves DEVICE_TIMEOUT in it, and it stays there until device_status() reads it."""
         word = cls._status.get(device.index)
         if word is None:
-            word = cls._status[device.index] = _calls().status_word(device.index)
+            native = torch_glue.calls_or_none()
+            word = cls._status[device.index] = (torch.zeros(1, dtype=torch.int32, device=device) if native is None
+                                                else native.status_word(device.index))
         return word
 
 
@@ -465,6 +467,121 @@ def _varlen_params(query, key, value, out, lse, cu_q, cu_k, max_q, max_k, is_cau
     p.dtype = _cabi.DTYPE_F16 if query.dtype == torch.float16 else _cabi.DTYPE_BF16
     p.kernel = _cabi.KERNEL_PREFILL
     return p
+
+
+def _check_inputs(*tensors: torch.Tensor) -> None:
+    for t in tensors:
+        _check(t.is_cuda, "Input tensor must be on a CUDA device (this path has no CPU fallback)")
+        # FlashAttention_internal.cpp:74-80
+        _check(t.dtype in (torch.bfloat16, torch.float16),
+               f"FlashAttention only support fp16 and bf16 data type (got {t.dtype})")
+        _check(t.dtype == tensors[0].dtype, "query, key, and value must have the same dtype")
+        # FlashAttention_internal.cpp:100-108
+        _check(t.stride(-1) == 1, "Input tensor must have contiguous last dimension")
+
+
+def _readable_gradient(g: torch.Tensor) -> torch.Tensor:
+    rows = g.dim() - (2 if g.dim() == 4 else 3)  # [B, H, L, D] or [total, H, D]
+    ok = g.stride(-1) == 1 and g.data_ptr() % 16 == 0 and all(
+        (g.size(i) == 1 and i != rows) or (g.stride(i) > 0 and g.stride(i) % 8 == 0) for i in range(g.dim() - 1))
+    return g if ok else g.clone(memory_format=torch.contiguous_format)
+
+
+class _FieldCalls:
+    """The functions of csrc/py_calls.cpp, with their arguments, on the C library alone: the parameter block is filled field by
+    field through ctypes, 50 to 60 us of host time per call."""
+
+    @staticmethod
+    def _heads_divide(query, key, value):
+        _check(key.size(1) == value.size(1) and key.size(1) > 0 and query.size(1) % key.size(1) == 0,
+               "Number of heads in key/value must divide number of heads in query")
+
+    @staticmethod
+    def _options(p, keep_rows, keep_cols, dropout_p, bias, dbias=None, bias_t=None):
+        if keep_rows is not None:
+            p.dropout_p, p.keep_rows, p.keep_cols = dropout_p, keep_rows.data_ptr(), keep_cols.data_ptr()
+        _set_bias(p, bias, dbias, bias_t)
+
+    @staticmethod
+    def _backward(p, set_strides, dout, grads, deterministic, device):
+        p.dout, p.dq, p.dk, p.dv = (t.data_ptr() for t in (dout, *grads))
+        for name, t in zip(("do", "dq", "dk", "dv"), (dout, *grads)):
+            set_strides(p, name, t)
+        p.deterministic = int(torch.are_deterministic_algorithms_enabled()) if deterministic < 0 else deterministic
+        _run_bwd(p, device)
+        return grads
+
+    @staticmethod
+    def dense_forward(query, key, value, is_causal, scale, allow_gqa, kernel, num_splits, sm_margin, keep_rows, keep_cols, dropout_p, bias):
+        # attention.cpp:70-100
+        _check(query.dim() == 4 and key.dim() == 4 and value.dim() == 4,
+               "query, key and value must be 4-dimensional [batch, heads, seq_len, head_dim]")
+        _check(query.size(0) == key.size(0) == value.size(0), "query, key and value must have the same batch size")
+        _check(key.size(2) == value.size(2), "Key and Value must have the same sequence length")
+        if allow_gqa:
+            _FieldCalls._heads_divide(query, key, value)
+        else:
+            _check(query.size(1) == key.size(1) == value.size(1), "query, key and value must have the same number of heads")
+        _check(query.size(3) == key.size(3) == value.size(3), "query, key and value must have the same head_dim")
+        _check_inputs(query, key, value)
+        B, H, Lq, D = query.shape
+        out = torch.empty((B, Lq, H, D), dtype=query.dtype, device=query.device).transpose(1, 2)
+        lse = torch.empty((B, H, Lq), dtype=torch.float32, device=query.device)
+        p = _dense_params(query, key, value, out, lse, is_causal, calculate_scale(query, scale), kernel, num_splits)
+        _FieldCalls._options(p, keep_rows, keep_cols, dropout_p, bias)
+        p.sm_margin = sm_margin
+        _run_fwd(p, query.device)
+        return out, lse
+
+    @staticmethod
+    def dense_backward(grad_out, query, key, value, out, logsumexp, is_causal, scale, keep_rows, keep_cols, dropout_p, bias, dbias, bias_t,
+                       deterministic):
+        dout = _readable_gradient(grad_out)
+        _check_inputs(dout, query, key, value, out)
+        _check(logsumexp.dtype == torch.float32 and logsumexp.is_contiguous() and tuple(logsumexp.shape) == tuple(query.shape[:3]),
+               "logsumexp must be contiguous fp32 [batch, heads, seqlen_q]")
+        grads = tuple(torch.empty((t.size(0), t.size(2), t.size(1), t.size(3)), dtype=t.dtype, device=t.device).transpose(1, 2)
+                      for t in (query, key, value))
+        p = _dense_params(query, key, value, out, logsumexp, is_causal, scale)
+        _FieldCalls._options(p, keep_rows, keep_cols, dropout_p, bias, dbias, bias_t)
+        return _FieldCalls._backward(p, _set_strides_bhld, dout, grads, deterministic, query.device)
+
+    @staticmethod
+    def _check_varlen(query, key, value, cu_q, cu_k):
+        _check_packed(query, key, value, cu_q, cu_k)
+        _FieldCalls._heads_divide(query, key, value)
+        _check(query.size(2) == key.size(2) == value.size(2), "query, key and value must have the same head_dim")
+        _check(key.size(0) == value.size(0), "Key and Value must have the same number of tokens")
+        _check_inputs(query, key, value)
+
+    @staticmethod
+    def varlen_forward(query, key, value, cu_q, cu_k, max_q, max_k, is_causal, scale, keep_rows, keep_cols, dropout_p, bias):
+        _FieldCalls._check_varlen(query, key, value, cu_q, cu_k)
+        out = torch.empty_like(query, memory_format=torch.contiguous_format)
+        lse = torch.empty((query.size(1), query.size(0)), dtype=torch.float32, device=query.device)
+        p = _varlen_params(query, key, value, out, lse, cu_q, cu_k, max_q, max_k, is_causal, calculate_scale(query, scale))
+        _FieldCalls._options(p, keep_rows, keep_cols, dropout_p, bias)
+        _run_fwd(p, query.device)
+        return out, lse
+
+    @staticmethod
+    def varlen_backward(grad_out, query, key, value, out, logsumexp, cu_q, cu_k, max_q, max_k, is_causal, scale, keep_rows, keep_cols,
+                        dropout_p, bias, dbias, bias_t, deterministic):
+        _FieldCalls._check_varlen(query, key, value, cu_q, cu_k)
+        dout = _readable_gradient(grad_out)
+        _check_inputs(query, dout, out)
+        _check(logsumexp.dtype == torch.float32 and logsumexp.is_contiguous()
+               and tuple(logsumexp.shape) == (query.size(1), query.size(0)), "logsumexp must be contiguous fp32 [heads_q, total_q]")
+        grads = tuple(torch.empty_like(t, memory_format=torch.contiguous_format) for t in (query, key, value))
+        p = _varlen_params(query, key, value, out, logsumexp, cu_q, cu_k, max_q, max_k, is_causal, scale)
+        _FieldCalls._options(p, keep_rows, keep_cols, dropout_p, bias, dbias, bias_t)
+        return _FieldCalls._backward(p, _set_strides_thd, dout, grads, deterministic, query.device)
+
+    @staticmethod
+    def flash_attention_forward(query, key, value, cu_q, cu_k, max_q, max_k, is_causal, scale):
+        out, lse = _FieldCalls.varlen_forward(query, key, value, cu_q, cu_k, max_q, max_k, is_causal, scale, None, None, 0.0, None)
+        seed, offset = _philox_placeholders(query)
+        return out, lse, seed, offset, _empty_like_debug(query)
 
 
 def _check_packed(query, key, value, cu_q, cu_k):

@@ -264,9 +264,11 @@ def scaled_dot_product_attention(query, key, value, attn_mask=None, dropout_p: f
     efficient one runs them with an attn_mask as additive bias, the math backend is torch's composite
     implementation. The plain cases are decided and run in one native call (csrc/sdpa_autograd.cpp); what it does not take
     comes back as None and goes through the procedure below."""
-    out = (torch_glue.calls or torch_glue.load()).sdpa(query, key, value, attn_mask, dropout_p, is_causal, scale)
-    if out is not None:
-        return out
+    calls = torch_glue.calls or (torch_glue.calls_or_none() if getattr(query, "is_cuda", False) else None)
+    if calls is not None:
+        out = calls.sdpa(query, key, value, attn_mask, dropout_p, is_causal, scale)
+        if out is not None:
+            return out
     choice = _fused_sdp_choice(query, key, value, attn_mask, dropout_p, is_causal, scale=scale)
     if choice == int(SDPBackend.ERROR):
         raise RuntimeError("No viable backend for scaled_dot_product_attention was found.")
@@ -275,6 +277,7 @@ def scaled_dot_product_attention(query, key, value, attn_mask=None, dropout_p: f
     if choice == int(SDPBackend.FLASH_ATTENTION) or (
             choice == int(SDPBackend.EFFICIENT_ATTENTION) and (not is_causal or query.size(-2) == key.size(-2))):
         # same kernels, same mask when Lq == Lk: the registered operator also carries autograd
+        torch_glue.load()
         return torch.ops.b200_sdpa._scaled_dot_product_flash_attention(query, key, value, dropout_p, is_causal, False,
                                                                        scale=scale)[0]
     if choice == int(SDPBackend.EFFICIENT_ATTENTION):

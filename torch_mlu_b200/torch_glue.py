@@ -24,6 +24,7 @@ SOURCES = ["torch_glue.cpp", "sdpa_autograd.cpp", "py_calls.cpp"]
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(_cabi.LIB_DIR, "libsdpa_b200_torch.so")
 calls = None  # the module of csrc/py_calls.cpp, once load() has run
+_load_error = None  # why calls_or_none() has none
 
 
 def build(verbose: bool = False) -> str:
@@ -81,6 +82,23 @@ def load():
     module.set_status_error(_cabi.SdpaError)
     calls = module
     return calls
+
+
+def calls_or_none():
+    """The module of direct calls, loaded on first use; None where it cannot be built or loaded (no compiler or torch headers),
+    which is said once. The C library and everything that needs only it work without the glue."""
+    global _load_error
+    if calls is not None:
+        return calls
+    if _load_error is None:
+        try:
+            return load()
+        except Exception as e:  # a failed build, a library that does not fit this torch
+            import warnings
+            _load_error = e
+            warnings.warn(f"the torch glue of torch_mlu_b200 is not available ({e}): calls go through ctypes, which costs some tens of "
+                          "microseconds each", RuntimeWarning, stacklevel=3)
+    return None
 
 
 def install_aten_overrides() -> None:
