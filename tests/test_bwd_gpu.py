@@ -132,6 +132,11 @@ def test_backward_is_deterministic(cuda_device, native_lib):
     d = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=False)
     assert torch.equal(c[3], d[3]) and torch.equal(c[4], d[4])
     assert orc.error_stats(c[2], d[2])[0] <= 2e-2 and orc.error_stats(c[2], a[2])[0] <= 2e-2
+    # the same with 300 key blocks, which the fused kernel serves
+    many = [rand((1, 60, 640, 128), s) for s in (5, 6, 7, 8)]
+    f, h, i = (run_fwd_bwd(cuda_device, *many, True, deterministic=det) for det in (False, False, True))
+    assert torch.equal(f[3], h[3]) and torch.equal(f[4], h[4])
+    assert orc.error_stats(f[2], h[2])[0] <= 2e-2 and orc.error_stats(f[2], i[2])[0] <= 2e-2
     # torch's global switch selects the same path
     torch.use_deterministic_algorithms(True)
     try:
@@ -140,6 +145,31 @@ def test_backward_is_deterministic(cuda_device, native_lib):
         torch.use_deterministic_algorithms(False)
     for x, y in zip(a, e):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,L,D,dropout,bias,deterministic,fused", [
+    (1, 148, 148, 128, 128, False, False, False, False),   # as many key blocks as SMs
+    (1, 149, 149, 128, 128, False, False, False, True),
+    (1, 149, 149, 128, 128, False, False, True, False),
+    (2, 80, 40, 256, 128, False, False, False, False),     # grouped queries at head_dim 128
+    (2, 80, 40, 256, 128, True, False, False, True),
+    (2, 80, 40, 256, 64, False, False, False, True),
+    (2, 80, 80, 256, 64, False, True, False, False),
+])
+def test_which_backward_kernels_run(cuda_device, native_lib, B, Hq, Hkv, L, D, dropout, bias, deterministic, fused):
+    """The tests of the fused kernel rely on this choice: read from the names of the kernels that ran."""
+    from torch.profiler import ProfilerActivity, profile
+    from torch_mlu_b200.dropout import KeepMasks
+    dev = cuda_device
+    q, k, v, do = (rand((B, h, L, D), s).to(dev) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
+    keep = KeepMasks(1, 2, 0.1, B, Hq, L, L, dev) if dropout else None
+    b = torch.zeros(B, 1, 1, L, dtype=torch.bfloat16, device=dev).expand(B, Hq, L, L) if bias else None
+    out, lse = ops._dense_forward(q, k, v, False, None, True, keep=keep, bias=b)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        ops._dense_backward(do, q, k, v, out, lse, False, D ** -0.5, keep=keep, bias=b, deterministic=deterministic)
+        torch.cuda.synchronize()
+    names = " ".join(e.name for e in prof.events())
+    assert ("bwd_fused_kernel" in names, "bwd_tile_kernel" in names) == (fused, not fused), names
 
 
 def test_config3_sampled_heads_and_linearity(cuda_device, native_lib):

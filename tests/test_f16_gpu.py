@@ -78,6 +78,25 @@ def test_f16_varlen(cuda_device, native_lib):
         orc.assert_close_grad_bf16(g, w, name)
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D,causal", [
+    (2, 40, 40, 200, 257, 128, True),
+    (1, 150, 75, 129, 257, 64, True),
+    (3, 26, 26, 130, 129, 104, False),
+])
+def test_f16_backward_with_more_key_blocks_than_sms(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
+    """The fused backward kernel."""
+    dev = cuda_device
+    q, k, v, dout = rand((B, Hq, Lq, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3), rand((B, Hq, Lq, D), 4)
+    qd, kd, vd = q.to(dev), k.to(dev), v.to(dev)
+    out, lse = ops.gqa_prefill(qd, kd, vd, is_causal=causal)
+    grads = ops._dense_backward(dout.to(dev), qd, kd, vd, out, lse, causal, D ** -0.5)
+    assert ops.device_status() == 0
+    o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=causal)
+    orc.assert_close_bf16(out, o_ref, "out")
+    for name, g, w in zip(("dq", "dk", "dv"), grads, orc.cpu_sdpa_backward(dout, q, k, v, o_ref, l_ref, causal=causal)):
+        orc.assert_close_grad_bf16(g, w, name)
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,Lk,D,splits", [
     (2, 8, 2, 1000, 128, 4), (2, 32, 2, 777, 128, 3), (1, 4, 4, 4096, 64, 0), (3, 8, 8, 1, 128, 1),
 ])

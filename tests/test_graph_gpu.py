@@ -8,10 +8,14 @@ from torch_mlu_b200 import ops
 pytestmark = pytest.mark.gpu
 
 
-def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib):
+@pytest.mark.parametrize("B,H", [
+    (2, 4),
+    (4, 26),   # 312 forward units and 624 key blocks: the forward's unit counter, the fused backward and its accumulator's clearing
+])
+def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib, B, H):
     dev = cuda_device
     g = torch.Generator().manual_seed(41)
-    B, H, L, D = 2, 4, 768, 128
+    L, D = 768, 128
     scale = D ** -0.5
     make = lambda: torch.randn(B, H, L, D, generator=g).bfloat16().to(dev)
     q, k, v, do = make(), make(), make(), make()
@@ -35,5 +39,9 @@ def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib):
         o2, l2 = ops.gqa_prefill(q, k, v, is_causal=True)
         want = [o2, l2, *ops._dense_backward(do, q, k, v, o2, l2, True, scale)]
         assert ops.device_status() == 0
-        for a, b in zip(got, want):
-            assert torch.equal(a, b)
+        for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), got, want):
+            if name == "dq" and B * H * (L // 128) > 148:
+                # the fused kernel sums dQ in a varying order: two roundings to 16 bits of nearly the same sum
+                assert float((a.float() - b.float()).norm() / b.float().norm()) <= 1e-3
+            else:
+                assert torch.equal(a, b), name

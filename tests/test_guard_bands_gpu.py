@@ -82,6 +82,9 @@ def set_bwd(p, dout, dq, dk, dv, packed):
     (2, 2, 2, 1, 300, 128, False),     # one query row: the tile kernel's smallest case
     (1, 4, 2, 200, 333, 160, True),    # head dims above 128: the kernels that stage 256-column tiles
     (2, 2, 1, 129, 70, 256, False),
+    (2, 40, 40, 200, 257, 128, True),   # more key blocks than SMs: the fused backward, and more units than SMs in the forward
+    (3, 26, 26, 333, 130, 80, False),
+    (1, 150, 75, 129, 257, 64, True),
 ])
 def test_dense_forward_and_backward_write_nothing_outside_their_outputs(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
     dev = cuda_device
@@ -119,6 +122,9 @@ def test_dense_forward_and_backward_write_nothing_outside_their_outputs(cuda_dev
     ([300, 45], 8, 2, 96, True),
     ([130, 70, 1, 255], 4, 2, 256, True),
     ([128, 129], 2, 2, 136, False),
+    ([130, 70, 1, 255], 20, 20, 128, True),   # more key blocks than SMs: the fused backward
+    ([128, 129, 127], 26, 26, 64, False),
+    ([300, 45], 50, 25, 64, True),
 ])
 def test_packed_forward_and_backward_write_nothing_outside_their_outputs(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
     dev = cuda_device

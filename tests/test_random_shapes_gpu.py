@@ -31,17 +31,29 @@ def draw_case(rng: random.Random):
                 scale=rng.choice([None, None, 0.05, 0.2]))
 
 
+def draw_case_with_many_heads(rng: random.Random):
+    """As draw_case, with enough key blocks for the fused backward (more than SMs) and the forward's unit counter."""
+    c = draw_case(rng)
+    group = rng.choice([1, 1, 2])
+    c["Hkv"] = rng.choice([50, 75])
+    c["Hq"] = c["Hkv"] * group
+    c["B"] = 3
+    if group > 1:
+        c["D"] = rng.choice([64, 32])  # grouped queries at head_dim 128 take the two kernels
+    return c
+
+
 def tensors(shape_list, seed, dtype):
     g = torch.Generator().manual_seed(seed)
     return [torch.randn(s, generator=g).to(dtype) for s in shape_list]
 
 
-@pytest.mark.parametrize("block", range(12))
-def test_dense_random_shapes(cuda_device, native_lib, block):
+@pytest.mark.parametrize("draw,block,cases", [(draw_case, b, 8) for b in range(12)] + [(draw_case_with_many_heads, b, 2) for b in range(12, 16)])
+def test_dense_random_shapes(cuda_device, native_lib, draw, block, cases):
     dev = cuda_device
     rng = random.Random(1000 + block)
-    for i in range(8):
-        c = draw_case(rng)
+    for i in range(cases):
+        c = draw(rng)
         B, Hq, Hkv, Lq, Lk, D = c["B"], c["Hq"], c["Hkv"], c["Lq"], c["Lk"], c["D"]
         q, k, v, dout = tensors([(B, Hq, Lq, D), (B, Hkv, Lk, D), (B, Hkv, Lk, D), (B, Hq, Lq, D)], 17 * block + i, c["dtype"])
         qd, kd, vd, dd = q.to(dev), k.to(dev), v.to(dev), dout.to(dev)
@@ -58,12 +70,12 @@ def test_dense_random_shapes(cuda_device, native_lib, block):
             orc.assert_close_reference_rule(g, w, lp, name + " " + tag, fudge=fudge)
 
 
-@pytest.mark.parametrize("block", range(8))
-def test_varlen_random_shapes(cuda_device, native_lib, block):
+@pytest.mark.parametrize("draw,block,cases", [(draw_case, b, 4) for b in range(8)] + [(draw_case_with_many_heads, b, 1) for b in range(8, 12)])
+def test_varlen_random_shapes(cuda_device, native_lib, draw, block, cases):
     dev = cuda_device
     rng = random.Random(2000 + block)
-    for i in range(4):
-        c = draw_case(rng)
+    for i in range(cases):
+        c = draw(rng)
         Hq, Hkv, D = c["Hq"], c["Hkv"], c["D"]
         n_seq = rng.choice([1, 2, 5])
         lens_q = [rng.choice(EDGE_LENGTHS) for _ in range(n_seq)]
