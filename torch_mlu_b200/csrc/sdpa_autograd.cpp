@@ -59,11 +59,17 @@ Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, 
   TORCH_CHECK(attn_bias.scalar_type() == q.scalar_type() && attn_bias.device() == q.device(),
               "attn_bias must have the dtype and device of query");
   const int64_t full[4] = {q.size(0), q.size(1), q.size(2), seqlen_k};
+  // the view at once: narrowing and expanding are two calls of a microsecond, here and in the backward
+  int64_t strides[4] = {0, 0, 0, 0};
+  bool ok = attn_bias.dim() >= 1 && attn_bias.size(-1) == (padded ? ceil8(seqlen_k) : seqlen_k) && attn_bias.stride(-1) == 1 &&
+            (padded || seqlen_k % 8 == 0) && reinterpret_cast<uintptr_t>(attn_bias.data_ptr()) % 16 == 0;
+  for (int64_t i = 4 - attn_bias.dim(), j = 0; ok && i < 4; ++i, ++j) {
+    const int64_t n = attn_bias.size(j);
+    strides[i] = n == 1 && i < 3 ? 0 : attn_bias.stride(j);
+    ok = i == 3 || ((n == 1 || n == full[i]) && strides[i] % 8 == 0);
+  }
+  if (ok) return attn_bias.as_strided(full, strides);
   const Tensor given = padded ? attn_bias.narrow(-1, 0, seqlen_k) : attn_bias;
-  Tensor view = given.expand(full);
-  if (view.stride(3) == 1 && (padded || seqlen_k % 8 == 0) && reinterpret_cast<uintptr_t>(view.data_ptr()) % 16 == 0 &&
-      view.stride(0) % 8 == 0 && view.stride(1) % 8 == 0 && view.stride(2) % 8 == 0)
-    return view;
   std::vector<int64_t> sizes(given.sizes().begin(), given.sizes().end());
   sizes.back() = seqlen_k;
   Tensor src = given.expand(sizes);
