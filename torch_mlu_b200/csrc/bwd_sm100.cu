@@ -1015,17 +1015,22 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 }  // namespace
 
 // Fused kernel or the two with a fixed summation order? A bias always takes the two: masked training gives the same bits every
-// time (and a bias gradient is written by the dQ kernel, whose threads own query rows). Otherwise (us, back-to-back calls, fused
-// | two):
+// time (and a bias gradient is written by the dQ kernel, whose threads own query rows). Otherwise, with figures in us, fused | two
+// ("step": forward and backward in turn over seconds; the others the backward alone, calls back to back):
 //  * up to one CTA per SM, fused leaves SMs idle for a whole chain of items, while the two kernels run side by side and need
-//    no clearing and no conversion: two. (B1 H8 L300 D128 31.9 | 22.0, B2 H8 L700 D64 26.6 | 20.5, B4 H8/1 L4096 D128 812 | 564,
-//    B4 H8 L500 D64 31.8 | 30.4)
-//  * head_dim 128 with grouped queries: a fused CTA chains the items of every query head of its group: two. (B8 H32/8 L2048
-//    causal 1125 | 1097; packed 12 x 64..2048 H16/4, whole step 420 | 408). Not with dropout, whose masks the two expand twice.
-//  * else fused: at head_dim 64 its items are cheap against the second pass over the scores (B8 H16 L2048 387 | 438, B16 H8 L300
-//    47 | 51); at 128 it is level, and under the power cap its 5 GEMMs for 7 decide (whole step B8 H16 L2048 769 | 776, with
-//    dropout 660 | 677; B2 H16 L8192 1758 | 1747).
-// The number of SMs is the B200's, not the current device's: workspace queries and launches must agree.
+//    no clearing and no conversion: two. (B1 H8 L300 D128 25.6 | 18.4, B1 H16 L1024 D128 45.1 | 29.8, B4 H8/1 L4096 D128 794 | 544,
+//    B2 H8 L700 D64 26.6 | 20.5, B4 H8 L500 D64 24.6 | 24.6; with dropout B1 H8 L2048 D128 78.3 | 50.2)
+//  * head_dim 64: fused, whose items are cheap against the second pass over the scores. (B8 H16 L2048 357 | 409, B16 H8 L300 47 | 51,
+//    grouped B8 H32/8 L2048 623 | 735, B16 H16/4 L700 194 | 218; with dropout 468 | 493, grouped 821 | 874)
+//  * head_dim 128 with grouped queries: a fused CTA chains the items of every query head of its group: two. (B8 H32/8 L2048 causal
+//    1127 | 1032, B8 H64/8 L1024 711 | 658, B16 H16/4 L700 317 | 305)
+//  * head_dim 128 otherwise: alone and at the power cap the two are ahead (B8 H16 L2048 572 | 560, B2 H16 L8192 1789 | 1656, B4 H40
+//    L300 80 | 76; with dropout 662 | 648), but in a training step the fused kernel's 5 GEMMs for 7 leave the forward more of the
+//    power: fused. (Step of B8 H16 L2048 745 | 757, with dropout 919 | 935; B2 H16 L8192 2281 | 2289, B16 H32 L512 361 | 368; the
+//    smallest of these grids loses: B4 H40 L300 111 | 108.) Grouped queries with dropout are with these although the two kernels
+//    are ahead alone (B8 H32/8 L2048 1311 | 1184).
+// A packed call counts the key blocks of its grid, every sequence at the longest length, whether they have keys or not. The number
+// of SMs is the B200's, not the current device's: workspace queries and launches must agree.
 bool use_fused_backward(const sdpa_b200_params& p) {
   if (p.deterministic != 0 || p.bias != nullptr) return false;
   constexpr int64_t kSms = 148;

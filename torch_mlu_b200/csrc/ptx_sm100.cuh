@@ -26,9 +26,7 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
-// One lane of a converged warp. Threads that issue tcgen05.mma / TMA copies are picked with it, not with `lane == 0`: those
-// instructions take their descriptors and addresses from uniform registers, and only behind elect.sync does the compiler
-// know that a single lane is active and emit them once, without a loop over the active lanes around each one. Measured
+// One lane of a converged warp. Threads that issue tcgen05.mma / TMA copies are picked with it, not with `lane == 0`. Measured
 // (all SMs, sixteen MMAs issued back to back): 28 cycles of issue per M128 N64 MMA with A in TMEM instead of 58, and the
 // pipe's own 32 cycles per MMA sustained instead of 45; N128 MMAs 43-50 instead of 58-64.
 __device__ __forceinline__ bool elect_one() {
