@@ -203,9 +203,9 @@ SDPA_B200_API int sdpa_b200_selftest_wait_timeout(uint32_t* device_status, uint3
  * frozen its memory plan. No counterpart in the reference: its attention calls always take a
  * workspace from the caching allocator (FlashAttention_internal.cpp:215-230). The caller passes
  * inputs and outputs only; the split partials live in a fixed SDPA_B200_STATIC_SCRATCH_BYTES
- * array inside the library (held by every GPU that loads it). Requests whose partials
- * (batch * heads_q * splits * 516 bytes) exceed it are refused with SDPA_B200_INVALID_ARG. The
- * first call on each device looks the array's address up; make it outside stream capture. Calls
+ * array inside the library (held by every GPU that loads it). Requests whose partials exceed it
+ * (batch * heads_q * num_splits * (head_dim + 1) * 4 bytes with num_splits > 1; with num_splits 0
+ * they always fit) are refused with SDPA_B200_INVALID_ARG. The first call on each device looks the array's address up; make it outside stream capture. Calls
  * that overlap on one GPU race on the shared array - order them on one stream. */
 #define SDPA_B200_STATIC_SCRATCH_BYTES (16u << 20)
 SDPA_B200_API int sdpa_b200_decode_static(const sdpa_b200_params* p, void* stream);

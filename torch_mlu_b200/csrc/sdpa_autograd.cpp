@@ -28,11 +28,6 @@ using torch::autograd::variable_list;
 
 namespace {
 
-void check_status(int st, const char* what) {
-  if (C10_LIKELY(st == SDPA_B200_OK)) return;
-  throw StatusError(st, c10::str(what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error()));
-}
-
 // An ordinary CUDA tensor, without wrappers, lazy conjugate or negative bits or a Python dispatch of its own: what the kernels
 // may be handed without the dispatcher.
 bool plain(const Tensor& t) {

@@ -34,11 +34,6 @@ using at::Tensor;
 
 namespace {
 
-void check_status(int st, const char* what) {
-  if (C10_LIKELY(st == SDPA_B200_OK)) return;
-  throw StatusError(st, c10::str(what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error()));
-}
-
 // Uninitialised device tensors without the dispatcher round trip of at::empty (a few hundred nanoseconds each, of calls
 // whose kernels run for a few microseconds). Where torch promises a value for uninitialised memory (deterministic algorithms),
 // the dispatcher's functions are used, which write it.

@@ -22,6 +22,11 @@ class StatusError : public c10::Error {
   int status_;
 };
 
+inline void check_status(int st, const char* what) {
+  if (C10_LIKELY(st == SDPA_B200_OK)) return;
+  throw StatusError(st, c10::str(what, ": ", sdpa_b200_status_string(st), ": ", sdpa_b200_last_error()));
+}
+
 // One bit per (query, key) pair in both orientations, written by the library from a Philox seed / offset pair
 // (the reference draws the pattern inside its kernel from such a pair and hands the pair to the backward
 // operator, FlashAttention_internal.cpp:190-214).
