@@ -299,6 +299,11 @@ def test_package_function_under_transforms_and_tracing(cuda_device, native_lib, 
         torch.func.jvp(lambda q: f(q, k, v), (q,), (torch.ones_like(q),))
     with pytest.raises(RuntimeError, match="torch.func|functorch"):
         torch.func.grad(lambda q: f(q, k, v).float().sum())(q)
+    qg = q.clone().requires_grad_()
+    assert f(qg, k, v).requires_grad
+    if not masked:
+        with torch._C._AutoDispatchBelowAutograd():
+            assert not f(qg, k, v).requires_grad
     neg = torch._neg_view(q)  # a lazily negated view of q: its memory holds q, not -q
     assert torch.equal(f(neg, k, v), f(-q, k, v)) or masked
 

@@ -40,17 +40,28 @@ bool plain(const Tensor& t) {
 // autograd not switched off below the dispatcher.
 bool dispatcher_may_be_skipped() {
   const auto tls = c10::impl::tls_local_dispatch_key_set();
-  return c10::default_included_set.has_all(tls.included_) && !tls.excluded_.has_all(c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA)) &&
+  return c10::default_included_set.has_all(tls.included_) && !tls.excluded_.has(c10::DispatchKey::AutogradFunctionality) &&
          !c10::impl::TorchDispatchModeTLS::any_modes_set() && !torch::jit::tracer::isTracing();
 }
 
 // ------------------------------------------------------------------------- additive bias
 int64_t ceil8(int64_t n) { return (n + 7) / 8 * 8; }
 
+// A copy of the bias with rows padded to a multiple of 8 keys.
+Tensor padded_copy(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k) {
+  std::vector<int64_t> sizes(attn_bias.sizes().begin(), attn_bias.sizes().end());
+  sizes.back() = seqlen_k;
+  const Tensor src = attn_bias.expand(sizes);
+  sizes.back() = ceil8(seqlen_k);
+  Tensor buf = at::zeros(sizes, q.options());
+  buf.narrow(-1, 0, seqlen_k).copy_(src);
+  return buf;
+}
+
 // The additive bias as a [B, H, Lq, Lk] view the kernels can read: broadcast dimensions keep stride 0, rows start 16-byte
-// aligned and are readable up to the next multiple of 8 keys. A bias that already has that layout is used in place; any
-// other is copied once into rows padded to a multiple of 8. `padded`: its rows are already that long, as mask_bias() makes them.
-Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, bool padded = false) {
+// aligned and are readable up to the next multiple of 8 keys. Undefined for a bias without that layout. `padded`: its rows are
+// as long as padded_copy() and mask_bias() make them.
+Tensor readable_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, bool padded) {
   TORCH_CHECK(attn_bias.scalar_type() == q.scalar_type() && attn_bias.device() == q.device(),
               "attn_bias must have the dtype and device of query");
   const int64_t full[4] = {q.size(0), q.size(1), q.size(2), seqlen_k};
@@ -63,15 +74,13 @@ Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, 
     strides[i] = n == 1 && i < 3 ? 0 : attn_bias.stride(j);
     ok = i == 3 || ((n == 1 || n == full[i]) && strides[i] % 8 == 0);
   }
-  if (ok) return attn_bias.as_strided(full, strides);
-  const Tensor given = padded ? attn_bias.narrow(-1, 0, seqlen_k) : attn_bias;
-  std::vector<int64_t> sizes(given.sizes().begin(), given.sizes().end());
-  sizes.back() = seqlen_k;
-  Tensor src = given.expand(sizes);
-  sizes.back() = ceil8(seqlen_k);
-  Tensor buf = at::zeros(sizes, q.options());
-  buf.narrow(-1, 0, seqlen_k).copy_(src);
-  return buf.narrow(-1, 0, seqlen_k).expand(full);
+  return ok ? attn_bias.as_strided(full, strides) : Tensor();
+}
+
+Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, bool padded) {
+  const Tensor view = readable_bias(attn_bias, q, seqlen_k, padded);
+  if (view.defined()) return view;
+  return readable_bias(padded_copy(padded ? attn_bias.narrow(-1, 0, seqlen_k) : attn_bias, q, seqlen_k), q, seqlen_k, true);
 }
 
 // A boolean attn_mask (true = take part) as a bias of 0 / -inf with rows padded to a multiple of 8: one kernel over the mask's
@@ -201,14 +210,16 @@ variable_list run_backward(const Tensor& go, const BackwardCall& c, const Backwa
 
 struct AttentionBackward : public torch::autograd::Node {
   SavedVariable q, k, v, out, lse, cu_q, cu_k, seed, offset;
-  // dense with a bias: the caller's own tensor (a change in place before the backward is noticed), or what mask_bias() made
-  SavedVariable bias;
+  // dense with a bias: the caller's own tensor (a change in place before the backward is noticed), or the padded buffer made from
+  // it, beside which a floating-point one is kept for the same check
+  SavedVariable bias, bias_given;
   BackwardCall call;
 
   std::string name() const override { return "B200AttentionBackward"; }
-  std::array<SavedVariable*, 10> saved() { return {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset, &bias}; }
+  std::array<SavedVariable*, 11> saved() { return {&q, &k, &v, &out, &lse, &cu_q, &cu_k, &seed, &offset, &bias, &bias_given}; }
 
   BackwardTensors unpack() {
+    bias_given.unpack();  // raises when it has been changed
     return {q.unpack(), k.unpack(), v.unpack(), out.unpack(shared_from_this()), lse.unpack(), cu_q.unpack(),
             cu_k.unpack(), seed.unpack(), offset.unpack(), bias.unpack()};
   }
@@ -446,11 +457,14 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
   c10::cuda::CUDAGuard device_guard(q.device());
   const bool boolean = mask.scalar_type() == at::kBool;
   const Tensor bias_arg = boolean ? Tensor() : mask.to(dtype);  // (differentiable) conversion of a bias of another type
-  Tensor mask_buf, out, lse;
+  Tensor padded, out, lse;  // `padded`: the buffer the bias is read from where the argument itself cannot be
   {
     at::AutoDispatchBelowADInplaceOrView guard;
-    if (boolean) mask_buf = mask_bias(mask, q, Lk);
-    const Tensor bias = prepare_bias(boolean ? mask_buf : bias_arg, q, Lk, boolean);
+    Tensor bias = boolean ? Tensor() : readable_bias(bias_arg, q, Lk, false);
+    if (!bias.defined()) {
+      padded = boolean ? mask_bias(mask, q, Lk) : padded_copy(bias_arg, q, Lk);
+      bias = readable_bias(padded, q, Lk, true);
+    }
     ForwardOptions opt;
     opt.bias = &bias;
     std::tie(out, lse) = dense_forward(q, k, v, is_causal, sc, /*allow_gqa=*/false, opt);
@@ -458,8 +472,9 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const c10::option
   if (any_requires_grad({&q, &k, &v, &bias_arg})) {
     auto node = new_node(q, k, v, bias_arg, is_causal, sc, 0.0);
     node->call.has_bias = true;
-    node->call.bias_padded = boolean;
-    node->bias = SavedVariable(boolean ? mask_buf : bias_arg, false);
+    node->call.bias_padded = padded.defined();
+    node->bias = SavedVariable(padded.defined() ? padded : bias_arg, false);
+    if (padded.defined() && !boolean) node->bias_given = SavedVariable(bias_arg, false);
     if (bias_arg.defined() && bias_arg.requires_grad()) {
       node->call.want_dbias = true;
       node->call.bias_sizes = bias_arg.sizes().vec();
