@@ -1,0 +1,105 @@
+"""The backward whose dQ comes from a GEMM over dS tiles left in the workspace (head_dim 65 to 128, more key blocks than SMs)."""
+import ctypes
+
+import pytest
+import torch
+
+from torch_mlu_b200 import _cabi, ops
+from tests.test_guard_bands_gpu import set_bwd
+
+pytestmark = pytest.mark.gpu
+NAN = float("nan")
+
+
+def run(lib, p, q, k, v, dout, packed, short_by):
+    """dq, dk, dv through the C entry point, with a workspace full of NaN that is `short_by` bytes below the recommended size."""
+    grads = [torch.full_like(t, NAN) for t in (q, k, v)]
+    set_bwd(p, dout, *grads, packed=packed)
+    p.deterministic = 1  # both paths are; without it the least workspace has room for an accumulator, which may be as large as dS
+    need = ctypes.c_size_t(0)
+    _cabi.check(lib.sdpa_b200_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(need)), "workspace query")
+    ws = torch.full(((need.value + 3) // 4,), NAN, device=q.device)
+    stream = torch.cuda.current_stream(q.device).cuda_stream
+    _cabi.check(lib.sdpa_b200_bwd(ctypes.byref(p), ws.data_ptr(), need.value - short_by, stream), "bwd")
+    torch.cuda.synchronize()
+    return grads
+
+
+def gradients_in_64_bits(q, k, v, dout, causal):
+    """[heads, length, head_dim] each."""
+    q, k, v = (t.double().requires_grad_() for t in (q, k, v))
+    group = q.size(0) // k.size(0)
+    s = q @ k.repeat_interleave(group, 0).transpose(1, 2) * q.size(-1) ** -0.5
+    if causal:
+        s = s.masked_fill(~torch.ones_like(s[0], dtype=torch.bool).tril(k.size(1) - q.size(1)), float("-inf"))
+    out = torch.softmax(s, -1).nan_to_num(0.0) @ v.repeat_interleave(group, 0)
+    return torch.autograd.grad(out, (q, k, v), dout.double())
+
+
+def distance(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+def check(with_ds, two_kernels, want):
+    # the same dK/dV kernel in both; dQ sums the same dS products in fp32, in the two kernels with a quarter of the exponentials off
+    # by up to 7.5e-5: at least as close to 64 bits, up to what the rounding of the results scatters
+    assert torch.equal(with_ds[1], two_kernels[1]) and torch.equal(with_ds[2], two_kernels[2])
+    for name, a, b, w in zip(("dq", "dk", "dv"), with_ds, two_kernels, want):
+        assert distance(a, w) <= 1.01 * distance(b, w) and distance(a, w) < 4e-3, (name, distance(a, w), distance(b, w))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D,causal", [
+    (1, 60, 60, 257, 257, 128, True),     # one row in the third tile of queries and of keys
+    (2, 28, 28, 257, 384, 128, True),     # mask offset 127
+    (1, 80, 80, 384, 255, 72, True),      # more queries than keys: rows, and whole tiles of rows, that see nothing
+    (1, 80, 80, 300, 129, 128, True),
+    (1, 100, 50, 385, 385, 96, False),    # grouped queries, an odd number of 128-row tiles per unit pair
+    (1, 160, 40, 130, 513, 128, False),
+    (3, 60, 60, 128, 128, 128, True),     # one tile per head
+])
+def test_dense(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal, dtype):
+    gen = torch.Generator().manual_seed(5)
+    q, k, v, dout = (torch.randn(B, h, n, D, generator=gen).to(cuda_device, dtype)
+                     for h, n in ((Hq, Lq), (Hkv, Lk), (Hkv, Lk), (Hq, Lq)))
+    out, lse = ops.gqa_prefill(q, k, v, is_causal=causal)
+    p = ops._dense_params(q, k, v, out, lse, causal, D ** -0.5)
+    want = [torch.stack(g) for g in zip(*(gradients_in_64_bits(q[b], k[b], v[b], dout[b], causal) for b in range(B)))]
+    check(run(native_lib, p, q, k, v, dout, False, 0), run(native_lib, p, q, k, v, dout, False, 1), want)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("lens_q,lens_k,Hq,Hkv", [
+    ((257, 0, 1, 128, 130), (257, 5, 1, 128, 130), 40, 20),
+    ((100, 300, 129), (400, 300, 65), 60, 60),   # shorter and longer keys than queries
+])
+def test_packed(cuda_device, native_lib, lens_q, lens_k, Hq, Hkv, causal):
+    D, dev = 128, cuda_device
+    gen = torch.Generator().manual_seed(6)
+    q, k, v, dout = (torch.randn(sum(n), h, D, generator=gen).to(dev, torch.bfloat16)
+                     for n, h in ((lens_q, Hq), (lens_k, Hkv), (lens_k, Hkv), (lens_q, Hq)))
+    ends_q, ends_k = ([sum(n[:i]) for i in range(len(n) + 1)] for n in (lens_q, lens_k))
+    cu_q, cu_k = (torch.tensor(e, dtype=torch.int32, device=dev) for e in (ends_q, ends_k))
+    args = (cu_q, cu_k, max(lens_q), max(lens_k), causal, D ** -0.5)
+    out, lse = ops._varlen_forward(q, k, v, *args)
+    p = ops._varlen_params(q, k, v, out, lse, *args)
+    want = [torch.zeros_like(t, dtype=torch.float64) for t in (q, k, v)]
+    for i, n in enumerate(lens_q):
+        a, b = slice(ends_q[i], ends_q[i + 1]), slice(ends_k[i], ends_k[i + 1])
+        if n > 0:
+            one = gradients_in_64_bits(*(t.transpose(0, 1) for t in (q[a], k[b], v[b], dout[a])), causal)
+            for w, g, rows in zip(want, one, (a, b, b)):
+                w[rows] = g.transpose(0, 1)
+    check(run(native_lib, p, q, k, v, dout, True, 0), run(native_lib, p, q, k, v, dout, True, 1), want)
+
+
+def test_several_passes_over_the_workspace(cuda_device, native_lib):
+    """2.7 GB of dS: two passes of ten heads give the bits of two calls with ten heads each."""
+    gen = torch.Generator(device=cuda_device).manual_seed(7)
+    q, k, v, dout = (torch.randn(1, 20, 8192, 128, generator=gen, device=cuda_device, dtype=torch.bfloat16) for _ in range(4))
+    out, lse = ops.gqa_prefill(q, k, v, is_causal=False)
+    whole = ops._dense_backward(dout, q, k, v, out, lse, False, 128 ** -0.5)
+    for part in (slice(0, 10), slice(10, 20)):
+        half = ops._dense_backward(*(t[:, part] for t in (dout, q, k, v, out)), lse[:, part].contiguous(), False, 128 ** -0.5)
+        for a, b in zip(whole, half):
+            assert torch.equal(a[:, part], b)

@@ -4,17 +4,11 @@
 
 #include <cuda_bf16.h>
 
+#include "ds_tiles.cuh"
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
 namespace sdpa_b200 {
-
-#ifndef SDPA_BWD_POLY_DKDV
-#define SDPA_BWD_POLY_DKDV 2  // of every 4 column pairs, how many use the polynomial 2^x (dK/dV kernel)
-#endif
-#ifndef SDPA_BWD_POLY_DQ
-#define SDPA_BWD_POLY_DQ 1    // the same for the dQ kernel
-#endif
 
 constexpr int kTile = 128;  // rows per tile (queries or keys)
 constexpr uint32_t kTileBytes = kTile * 128 * 2;  // one shared-memory slot (head_dim 64 uses half of it)
@@ -59,6 +53,10 @@ struct BwdKernelParams {
   // 4-column group are 512 contiguous bytes). Row index: dense (batch * heads_q + head) * lq_pad + query, packed
   // head * dq_acc_rows + token.
   float* dq_acc;
+  // dK/dV kernel: where dS goes for the dQ GEMM, and that GEMM's unit counter
+  DsTiles ds;
+  uint32_t* ds_counter;
+  int bh0;  // first (batch, head) pair of this launch
   int dq_acc_rows;  // packed: rows per head (total_q rounded up to 128, plus 128)
 #ifdef SDPA_BWD_STAMPS
   float* stamps;  // [mode 2][role 4][item 24][event 8] SM cycles since CTA start, one CTA per mode

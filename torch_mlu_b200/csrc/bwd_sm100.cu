@@ -19,15 +19,20 @@
 //      row = TMEM lane, one warpgroup per 64-query half of the tile) form P^T and dS^T, write
 //      them back to TMEM as bf16, and MMAs with the TMEM operand accumulate dV += P^T dO and
 //      dK += dS^T Q half by half (the streamed tiles are re-read in place as MN-major operands).
-//   3. bwd_tile_kernel<kModeDQ>: one CTA per (batch, query head, 128-query block); Q and dO
-//      stay, (K, V) stream; S = Q K^T, dP = dO V^T, dS -> TMEM, dQ += dS K.
+//   3. dQ, one of: bwd_tile_kernel<kModeDQ>, one CTA per (batch, query head, 128-query block); Q and dO
+//      stay, (K, V) stream; S = Q K^T, dP = dO V^T, dS -> TMEM, dQ += dS K. Or, where launch 2 has left its dS
+//      in the workspace as well (8 stores of 16 bytes per thread and item: 281 -> 315 us at B8 H16 L2048 D128
+//      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> about 120).
 // TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512). The bf16 P and dS of an item both
 // live in the item's score buffer, so the buffer that held dP is free as soon as it has been read;
 // the MMA issuer uses that (and, for dQ, the unused ACC2) to run the next item's score GEMMs and
 // exponentials under the current item's accumulation MMAs (buffer schedule at the issuer).
+#ifdef SDPA_BWD_STAMPS
 #include <cstdlib>
+#endif
 
 #include "bwd_common.cuh"
+#include "bwd_ds_gemm.h"
 #include "packed_grads.cuh"
 
 namespace sdpa_b200 {
@@ -102,7 +107,10 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int lane = threadIdx.x & 31;
   // The dQ kernel follows in the stream and depends on nothing written here: once every dK/dV CTA has begun (this
   // signal), its CTAs may take over SMs as they free up, instead of waiting for the last dK/dV CTA to finish.
-  if (kMode == kModeDKDV && threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (kMode == kModeDKDV && threadIdx.x == 0) {
+    if (kD > 64 && p.ds.data != nullptr && blockIdx.x == 0) *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
   constexpr int kStages = stages_for(kMode);
   constexpr uint32_t kSmemVec = smem_vec_off(kMode);
   constexpr uint32_t kSmemBar = smem_bar_off(kMode);
@@ -118,7 +126,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int w = blockIdx.x - grp * per_group;
     const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
     const int rank = w / size;
-    const int bh = grp * p.heads_per_wave + (w - rank * size);
+    const int bh = p.bh0 + grp * p.heads_per_wave + (w - rank * size);
     if (rank >= p.num_row_blocks) {  // padding slots of a short last group
       if (kMode == kModeDQ) wait_for_previous_grid();
       return;
@@ -472,6 +480,17 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       my_nlse2 = p.nlse2[vec];
       my_ndelta = p.ndelta[vec];
     }
+    // dK/dV with a dQ GEMM behind it: tile (query tile 0, this key block) of the group's first query head, and what leads from it
+    // to the others
+    uint32_t ds_tile0 = 0, ds_per_head = 0;
+    int ds_key_tiles = 0, ds_shift_rows = 0;
+    if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) {
+      const DsHead dh = ds_head(p.ds, b, hx * p.kv_group, p.heads_q, len_q, len_k, p.is_causal != 0);
+      ds_tile0 = static_cast<uint32_t>(dh.base + xb);
+      ds_per_head = static_cast<uint32_t>(ds_tiles_per_head(len_q, len_k, p.is_causal != 0));
+      ds_key_tiles = dh.key_tiles;
+      ds_shift_rows = dh.shift;
+    }
     for (int i = 0; i < n_items; ++i) {
       const int s = (2 * i) % kStages;  // ring slot of Y1(i), which carries the per-query vectors
       const int hi = i / tiles_per_head;
@@ -575,6 +594,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       int j_lo = 0, j_hi = kTile;
       if (kMode == kModeDKDV) {
         if (p.is_causal) j_lo = xr - causal_off - y0;
+        if (kD > 64 && xr >= len_x) j_lo = kTile;  // a row past the last key: its dS must be zero
       } else {
         j_hi = len_k - y0;
         if (p.is_causal) j_hi = min(j_hi, xr + causal_off + 1 - y0);
@@ -629,12 +649,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             __syncwarp();
           }
         }
-        // x = S c - lse2. In the dK/dV kernel this pass sits on the critical chain (score GEMM ->
-        // exponentials -> dP read -> next score GEMM) and the exponential unit alone would bound it, so
-        // kPolyOf4 of every four column pairs take their 2^x from the FMA pipe (exp2_poly3_x2). The dQ
-        // kernel's compute warps are bound by issue slots as much as by the exponential unit; there one
-        // pair in four is the measured optimum (two of four already cost time), here two of four.
-        constexpr int kPolyOf4 = (kMode == kModeDKDV) ? SDPA_BWD_POLY_DKDV : SDPA_BWD_POLY_DQ;
+        // x = S c - lse2. kPolyOf4 of every four column pairs take their 2^x from the FMA pipe (exp2_poly3_x2). dQ: one; two already
+        // cost issue slots. dK/dV at head_dim 64, where a quarter of the MMAs' time hides as many exponentials: two (step of B8 H12
+        // L512 with a mask 96.3 us, without any 97.5). At 128, none: at the power cap none to two take the same time (step of B8 H16
+        // L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed 64 to 2048 tokens 369, 368, 364), and none is the most exact.
+        constexpr int kPolyOf4 = kMode == kModeDQ ? 1 : (kD == 64 ? 2 : 0);
 #pragma unroll
         for (int j4 = 0; j4 < 16; ++j4) {
           const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
@@ -688,6 +707,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!ok) break;
       tc_fence_after_sync();
       BWD_STAMP(half, i, 4);
+      uint32_t dw[32];
       {
         uint32_t d[64];
         tmem_ld_x32_at<0>(dbuf, d);
@@ -697,7 +717,6 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         __syncwarp();
         if (lane == 0) mbar_arrive(bar + kBarDFree);  // the dP buffer may be overwritten
         BWD_STAMP(half, i, 5);
-        uint32_t dw[32];
 #pragma unroll
         for (int j4 = 0; j4 < 16; ++j4) {
           const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_ndelta + 4 * j4) : make_float4(my_ndelta, my_ndelta, my_ndelta, my_ndelta);
@@ -737,6 +756,18 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(bar + kBarPFull);
       BWD_STAMP(half, i, 7);
+      if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) {
+        // dS for the dQ GEMM: 16 bytes (8 queries) per store, 512 contiguous bytes per warp. Behind the arrival, so that the
+        // dK GEMM does not wait for the stores to issue
+        const uint32_t tile = ds_tile0 + static_cast<uint32_t>(hi) * ds_per_head +
+                              static_cast<uint32_t>(ds_row_start(y0 / kTile, ds_key_tiles, ds_shift_rows));
+        if (tile < p.ds.capacity) {
+          uint4* dst = ds_group(p.ds, tile, half * 8, r);
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch)
+            dst[ch * kDsTile] = make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]);
+        }
+      }
     }
 
     // ---- epilogue: accumulators -> scale -> 16-bit -> global
@@ -860,6 +891,9 @@ struct PreParams {
   int seqlen_q, total_q, heads_q, lq_pad, head_dim;
   float* dq_acc;    // fused kernel: its dQ accumulator, whose existing rows are cleared here; else null
   int dq_acc_rows;  // as in BwdKernelParams
+  int32_t* ds_seq_base;  // packed, dS for a dQ GEMM: DsTiles::seq_base, written here; else null
+  const int32_t* cu_k;
+  int is_causal;
   PackedGrads grads;
 };
 
@@ -884,6 +918,17 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   if (kPacked) {
     q_off = p.cu_q[b];
     len_q = p.cu_q[b + 1] - q_off;
+  }
+  if (kPacked && p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0) {
+    __shared__ int tiles_before;
+    if (threadIdx.x == 0) tiles_before = 0;
+    __syncthreads();
+    int mine = 0;
+    for (int i = threadIdx.x; i < b; i += 256)
+      mine += static_cast<int>(ds_tiles_per_head(p.cu_q[i + 1] - p.cu_q[i], p.cu_k[i + 1] - p.cu_k[i], p.is_causal != 0));
+    if (mine != 0) atomicAdd(&tiles_before, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) p.ds_seq_base[b] = tiles_before;
   }
   if (p.dq_acc != nullptr) {
     // 64 rows of an accumulator tile: per 4-column group 1 KB of consecutive floats, a thread per row. The stores need no
@@ -1014,29 +1059,78 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 
 }  // namespace
 
-// Fused kernel or the two with a fixed summation order? A bias always takes the two: masked training gives the same bits every
-// time (and a bias gradient is written by the dQ kernel, whose threads own query rows). Otherwise, with figures in us, fused | two
-// ("step": forward and backward in turn over seconds; the others the backward alone, calls back to back):
-//  * up to one CTA per SM, fused leaves SMs idle for a whole chain of items, while the two kernels run side by side and need
-//    no clearing and no conversion: two. (B1 H8 L300 D128 25.6 | 18.4, B1 H16 L1024 D128 45.1 | 29.8, B4 H8/1 L4096 D128 794 | 544,
-//    B2 H8 L700 D64 26.6 | 20.5, B4 H8 L500 D64 24.6 | 24.6; with dropout B1 H8 L2048 D128 78.3 | 50.2)
-//  * head_dim 64: fused, whose items are cheap against the second pass over the scores. (B8 H16 L2048 357 | 409, B16 H8 L300 47 | 51,
-//    grouped B8 H32/8 L2048 623 | 735, B16 H16/4 L700 194 | 218; with dropout 468 | 493, grouped 821 | 874)
-//  * head_dim 128 with grouped queries: a fused CTA chains the items of every query head of its group: two. (B8 H32/8 L2048 causal
-//    1127 | 1032, B8 H64/8 L1024 711 | 658, B16 H16/4 L700 317 | 305)
-//  * head_dim 128 otherwise: alone and at the power cap the two are ahead (B8 H16 L2048 572 | 560, B2 H16 L8192 1789 | 1656, B4 H40
-//    L300 80 | 76; with dropout 662 | 648), but in a training step the fused kernel's 5 GEMMs for 7 leave the forward more of the
-//    power: fused. (Step of B8 H16 L2048 745 | 757, with dropout 919 | 935; B2 H16 L8192 2281 | 2289, B16 H32 L512 361 | 368; the
-//    smallest of these grids loses: B4 H40 L300 111 | 108.) Grouped queries with dropout are with these although the two kernels
-//    are ahead alone (B8 H32/8 L2048 1311 | 1184).
+// Which kernels a call takes, with figures in us ("step": forward and backward in turn over seconds; the others the backward alone,
+// calls back to back):
+//  * up to one CTA per SM for the key blocks: the dK/dV and the dQ kernel side by side (bwd_tile_kernel twice). Whatever waits for
+//    the dK/dV kernel waits for a whole chain of items while SMs are idle. (B1 H8 L2048 D128 step 85, through dS 95, fused 103; B4
+//    H8/1 L4096 545, 564, 800; the other way round only where few key blocks meet many queries: B2 H32/8 L1024 unmasked 124, 112.)
+//  * a bias gradient: the same two, since the dQ kernel, whose threads own query rows, writes it.
+//  * head_dim 64, more key blocks, no bias, no fixed order asked for: the fused kernel. Its items are cheap against a second pass over
+//    the scores or over dS, whose traffic is the same as at 128 for half the work. (Step of B8 H16 L2048 490, through dS 530, two
+//    kernels 554; B4 H16 L1024 unmasked 141, 146, 142; grouped B8 H32/8 L2048 623, two kernels 735.) With a bias or in a fixed order:
+//    the two kernels (B8 H12 L512 with a mask 61.5; fused 60.3, and through dS level).
+//  * head_dim 65 to 128, more key blocks: dS through the workspace and a GEMM for dQ (use_ds_backward). One pass over the scores where
+//    the two kernels make two, and no reductions. (Step of B8 H16 L2048 695, two kernels 757, fused 752; with dropout 875, 940, 925;
+//    B2 H16 L8192 2115, 2295, 2290; B16 H32 L512 310, 365, 360; D80 B8 H16 L2048 alone 438, 533, 545; grouped B8 H32/8 L2048 alone
+//    860, 1100, 1130, B16 H16/4 L700 165, 208, 206; B3 H50 L128, the smallest of these grids, 28.8, 28.8, 32.8.)
+//    Short sequences that fill the SMs about once (up to 160 key blocks of at most two tiles) stay with the fused kernel, or, grouped
+//    and without dropout, the two: nothing but launches shows in a step there (B3 H50 L128 77.3 each way).
 // A packed call counts the key blocks of its grid, every sequence at the longest length, whether they have keys or not. The number
 // of SMs is the B200's, not the current device's: workspace queries and launches must agree.
+int64_t key_blocks(const sdpa_b200_params& p) {
+  return static_cast<int64_t>(p.batch) * p.heads_kv * ((static_cast<int64_t>(p.max_seqlen_k) + kTile - 1) / kTile);
+}
+constexpr int64_t kSms = 148;
+
+bool use_ds_backward(const sdpa_b200_params& p) {
+  if (p.head_dim <= 64 || p.dbias != nullptr || key_blocks(p) <= kSms) return false;
+  const bool one_round = key_blocks(p) <= 160 && p.max_seqlen_q <= 2 * kTile && p.max_seqlen_k <= 2 * kTile;
+  return !one_round;
+}
+
 bool use_fused_backward(const sdpa_b200_params& p) {
-  if (p.deterministic != 0 || p.bias != nullptr) return false;
-  constexpr int64_t kSms = 148;
-  const int64_t ctas = static_cast<int64_t>(p.batch) * p.heads_kv * ((static_cast<int64_t>(p.max_seqlen_k) + kTile - 1) / kTile);
-  if (ctas <= kSms) return false;
-  return p.head_dim <= 64 || p.heads_q == p.heads_kv || p.dropout_p > 0.f;
+  if (p.deterministic != 0 || p.bias != nullptr || key_blocks(p) <= kSms) return false;
+  return p.head_dim <= 64 || (!use_ds_backward(p) && (p.heads_q == p.heads_kv || p.dropout_p > 0.f));
+}
+
+// dS of a call (half of B H Lq Lk elements of two bytes under a causal mask) may take this much of the workspace; a dense call with
+// more of it goes through it in several passes over its KV heads. One pass is best (step of B8 H16 L2048, 0.57 GB of dS: 673 us in
+// one pass, 709 in two, 766 in six, where a pass's dS would stay in L2; B2 H16 L8192, 2.1 GB: 2115 in one, 2189 in two).
+constexpr size_t kDsBytesMax = size_t{2} << 30;
+
+// How a call's dS goes through the workspace: `kv_heads` (batch * heads_kv indexes) per pass, `tiles` of room, none if 0.
+struct DsPlan {
+  int kv_heads = 0;
+  uint32_t tiles = 0;
+};
+
+DsPlan ds_plan(const sdpa_b200_params& p) {
+  DsPlan plan;
+  if (!use_ds_backward(p)) return plan;
+  const int64_t cap = static_cast<int64_t>(kDsBytesMax / kDsTileBytes);
+  const int64_t key_tiles = (static_cast<int64_t>(p.max_seqlen_k) + kDsTile - 1) / kDsTile;
+  const int64_t kv_heads = static_cast<int64_t>(p.batch) * p.heads_kv;
+  if (p.cu_seqlens_q != nullptr) {
+    // the lengths are on the device: every query tile there can be, against the longest keys
+    const int64_t tiles = (p.total_q / kDsTile + p.batch) * key_tiles * p.heads_q;
+    if (tiles > cap) return plan;
+    plan.kv_heads = static_cast<int>(kv_heads);
+    plan.tiles = static_cast<uint32_t>(tiles);
+    return plan;
+  }
+  const int64_t per_kv_head = p.heads_q / p.heads_kv * ds_tiles_per_head(p.max_seqlen_q, p.max_seqlen_k, p.is_causal != 0);
+  if (per_kv_head <= 0 || per_kv_head > cap) return plan;
+  const int64_t passes = (kv_heads * per_kv_head + cap - 1) / cap;
+  int64_t per_pass = (kv_heads + passes - 1) / passes;
+  if (per_pass * per_kv_head > cap) per_pass = cap / per_kv_head;
+  if (passes > 1 && per_pass * key_tiles < 3 * 148) return plan;  // a pass must fill the SMs a few times over
+  plan.kv_heads = static_cast<int>(per_pass);
+  plan.tiles = static_cast<uint32_t>(per_pass * per_kv_head);
+  return plan;
+}
+
+size_t ds_table_bytes(const sdpa_b200_params& p) {
+  return p.cu_seqlens_q != nullptr ? (static_cast<size_t>(p.batch) * sizeof(int32_t) + 255) / 256 * 256 : 0;
 }
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
@@ -1044,15 +1138,22 @@ size_t bwd_vector_bytes(const sdpa_b200_params& p) {
   return (bytes + 255) / 256 * 256;
 }
 
-// lse2 and delta, then the fp32 dQ accumulator of the fused kernel: for every call without a bias that does not ask for a fixed
-// order, whatever path its sizes take, so that one workspace serves calls that differ in dropout or sizes.
-size_t bwd_workspace_bytes(const sdpa_b200_params& p) {
+// What a call needs: lse2 and delta, then the fp32 dQ accumulator of the fused kernel: for every call without a bias that does not ask
+// for a fixed order, whatever path its sizes take, so that one workspace serves calls that differ in dropout or sizes.
+size_t bwd_workspace_min_bytes(const sdpa_b200_params& p) {
   const bool acc = p.deterministic == 0 && p.bias == nullptr;
   return bwd_vector_bytes(p) + (acc ? bwd_fused_workspace_bytes(p, lq_padded(p)) : 0);
 }
 
+// What it is best given: room for dS too. A call that is given less takes the two kernels.
+size_t bwd_workspace_bytes(const sdpa_b200_params& p) {
+  const DsPlan plan = ds_plan(p);
+  const size_t with_ds = plan.tiles > 0 ? bwd_vector_bytes(p) + ds_table_bytes(p) + plan.tiles * kDsTileBytes : 0;
+  const size_t least = bwd_workspace_min_bytes(p);
+  return with_ds > least ? with_ds : least;
+}
+
 int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  (void)workspace_bytes;
   const bool f16 = p.dtype == SDPA_B200_F16;
   const bool varlen = p.cu_seqlens_q != nullptr;
   const int lq_pad = lq_padded(p);
@@ -1080,6 +1181,12 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   pre.head_dim = p.head_dim;
   pre.grads = packed_grads(p);
   const bool fused = use_fused_backward(p);
+  const DsPlan plan = ds_plan(p);
+  const bool through_ds = plan.tiles > 0 && workspace_bytes >= kWorkspaceHeaderBytes + bwd_workspace_bytes(p);
+  char* behind_vectors = static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p);
+  pre.ds_seq_base = through_ds && varlen ? reinterpret_cast<int32_t*>(behind_vectors) : nullptr;
+  pre.cu_k = p.cu_seqlens_k;
+  pre.is_causal = p.is_causal;
   float* dq_acc = fused ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p)) : nullptr;
   pre.dq_acc = dq_acc;
   pre.dq_acc_rows = fused && varlen ? static_cast<int>(bwd_fused_acc_rows(p, lq_pad) / p.heads_q) : 0;
@@ -1179,9 +1286,9 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
 #endif
 
   // heads per group: streamed bytes per head (q + dO of the group, or k + v) within ~48 MB of L2
-  auto set_order = [&](int heads_x, int rows_streamed, int streams_per_head) {
+  auto set_order = [&](int heads_x, int rows_streamed, int streams_per_head, int num_bh) {
     kp.heads_x = heads_x;
-    kp.num_bh = p.batch * heads_x;
+    kp.num_bh = num_bh;
     const double bytes = 2.0 * rows_streamed * p.head_dim * 2 * streams_per_head;
     int hpw = static_cast<int>((48.0 * 1024 * 1024) / bytes);
     hpw = hpw < 1 ? 1 : (hpw > 32 ? 32 : hpw);
@@ -1191,13 +1298,33 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
     return groups * hpw * kp.num_row_blocks;
   };
   kp.num_row_blocks = (p.max_seqlen_k + kTile - 1) / kTile;
-  const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group);
+  kp.bh0 = 0;
+  kp.ds.data = nullptr;
+  if (through_ds) {
+    kp.ds.data = reinterpret_cast<uint16_t*>(behind_vectors + ds_table_bytes(p));
+    kp.ds.seq_base = pre.ds_seq_base;
+    kp.ds.capacity = plan.tiles;
+    kp.ds_counter = static_cast<uint32_t*>(workspace) + 2;
+    const int kv_heads = p.batch * p.heads_kv;
+    for (int first = 0; first < kv_heads; first += plan.kv_heads) {
+      const int n = kv_heads - first < plan.kv_heads ? kv_heads - first : plan.kv_heads;
+      kp.bh0 = first;
+      kp.ds.head0 = first * kp.kv_group;
+      const int grid = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, n);
+      if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp)) !=
+          SDPA_B200_OK)
+        return st;
+      if ((st = launch_bwd_ds_gemm(p, kp.ds, first, n, false, kp.ds_counter, kp.status, stream)) != SDPA_B200_OK) return st;
+    }
+    return SDPA_B200_OK;
+  }
+  const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, p.batch * p.heads_kv);
   if (fused) return launch_bwd_fused(p, kp, dq_acc, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk);
   if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp)) !=
       SDPA_B200_OK)
     return st;
   kp.num_row_blocks = (p.max_seqlen_q + kTile - 1) / kTile;
-  const int grid_dq = set_order(p.heads_q, p.max_seqlen_k, 1);
+  const int grid_dq = set_order(p.heads_q, p.max_seqlen_k, 1, p.batch * p.heads_q);
   return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kp,
                             /*overlap_previous=*/true);
 }

@@ -52,7 +52,9 @@ int check_decode_request(const sdpa_b200_params& p);
 // round(dropout_p * 256), the byte threshold of the dropout keep-masks (dropout_mask.cu)
 uint32_t dropout_drop_byte(float dropout_p);
 
-// Backward: delta pre-pass + dK/dV kernel + dQ kernel.
+// Backward up to head_dim 128: delta pre-pass, then the kernels that bwd_sm100.cu chooses. A call that is given at least the least
+// workspace runs; with less than bwd_workspace_bytes() on other kernels.
+size_t bwd_workspace_min_bytes(const sdpa_b200_params& p);
 size_t bwd_workspace_bytes(const sdpa_b200_params& p);
 int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes,
                cudaStream_t stream);

@@ -9,6 +9,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "bwd_ds_gemm.h"
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
@@ -72,6 +73,26 @@ int make_tensor_map_16(bool f16, CUtensorMap* map, const void* base, int head_di
               "{row %lld, head %lld, batch %lld}",
               static_cast<int>(r), head_dim, (long long)rows, (long long)heads, (long long)batch,
               (long long)row_stride, (long long)head_stride, (long long)batch_stride);
+    return SDPA_B200_INVALID_ARG;
+  }
+  return SDPA_B200_OK;
+}
+
+int make_ds_tensor_map(CUtensorMap* map, const void* base, uint32_t tiles, int box_words, int box_rows) {
+  EncodeTiledFn encode = get_encode_fn();
+  if (encode == nullptr) {
+    set_error("cuTensorMapEncodeTiled is not available from the CUDA driver");
+    return SDPA_B200_NO_DEVICE;
+  }
+  cuuint64_t dims[4] = {256, static_cast<cuuint64_t>(tiles) * 16, 1, 1};
+  cuuint64_t strides[3] = {2048, 2048, 2048};
+  cuuint32_t box[4] = {static_cast<cuuint32_t>(box_words), static_cast<cuuint32_t>(box_rows), 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void*>(base), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (CUresult %d) for %u dS tiles", static_cast<int>(r), tiles);
     return SDPA_B200_INVALID_ARG;
   }
   return SDPA_B200_OK;
@@ -431,7 +452,7 @@ int sdpa_b200_bwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
   if ((st = check_tensor("dv", p->dv, p->dv_batch_stride, p->dv_head_stride, p->dv_row_stride, varlen, p->batch,
                          p->heads_kv)) != SDPA_B200_OK)
     return st;
-  const size_t need = kWorkspaceHeaderBytes + (p->head_dim > 128 ? bwd_d256_workspace_bytes(*p) : bwd_workspace_bytes(*p));
+  const size_t need = kWorkspaceHeaderBytes + (p->head_dim > 128 ? bwd_d256_workspace_bytes(*p) : bwd_workspace_min_bytes(*p));
   st = validate_workspace(workspace, workspace_bytes, need);
   if (st != SDPA_B200_OK) return st;
   st = check_device();
