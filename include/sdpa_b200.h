@@ -154,11 +154,11 @@ typedef struct sdpa_b200_params {
    * bias does not depend on the query (bias_row_stride == 0). NULL = not given. */
   const void* bias_t;
   int64_t bias_t_batch_stride, bias_t_head_stride, bias_t_row_stride;
-  /* Backward: 0 = whichever is faster for the sizes: the fused kernel, which forms every tile's scores once and adds
-   * its dQ contributions into an fp32 workspace with floating-point reductions whose order varies between launches (dK
-   * and dV are still summed in a fixed order), or the separate dK/dV and dQ kernels with a fixed summation order
-   * throughout. Non-zero = always the latter, so that the same call gives the same bits every time. A call with a bias
-   * always takes the latter too. Ignored by the forward. */
+  /* Backward: 0 = whichever is faster for the sizes. That may be the fused kernel (up to head_dim 64 in the main), which forms
+   * every tile's scores once and adds its dQ contributions into an fp32 workspace with floating-point reductions whose
+   * order varies between launches (dK and dV are still summed in a fixed order). Non-zero = only kernels with a fixed
+   * summation order throughout, so that the same call with the same workspace size gives the same bits every time. A call
+   * with a bias takes only those too. Ignored by the forward. */
   int32_t deterministic;
   /* Forward (tile kernel): number of SMs the persistent kernel leaves free, for a kernel that is to run beside it on
    * another stream - a collective that reassembles the previous step's outputs, say. 0 = one CTA on every SM, which
@@ -176,10 +176,12 @@ SDPA_B200_API const char* sdpa_b200_status_string(int status);
 /* Text of the last error raised on the calling thread (what was wrong and where). */
 SDPA_B200_API const char* sdpa_b200_last_error(void);
 
-/* Workspace size the matching call needs for these params (>= 256 bytes; 256-byte aligned
- * base required). */
+/* Workspace size the matching call is best given for these params (>= 256 bytes; 256-byte aligned base required).
+ * For the forward it is also the least it needs. The backward may leave dS there (up to 2 GiB; head dims above 64) and runs
+ * with less as well, on slower kernels: sdpa_b200_bwd_workspace_least_bytes is the size below which it is refused. */
 SDPA_B200_API int sdpa_b200_fwd_workspace_bytes(const sdpa_b200_params* p, size_t* bytes);
 SDPA_B200_API int sdpa_b200_bwd_workspace_bytes(const sdpa_b200_params* p, size_t* bytes);
+SDPA_B200_API int sdpa_b200_bwd_workspace_least_bytes(const sdpa_b200_params* p, size_t* bytes);
 
 /* out, lse <- attention(q, k, v). `stream` is a cudaStream_t passed as void*. */
 SDPA_B200_API int sdpa_b200_fwd(const sdpa_b200_params* p, void* workspace, size_t workspace_bytes, void* stream);

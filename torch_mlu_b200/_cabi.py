@@ -23,6 +23,7 @@ EXPORTED_SYMBOLS = (
     "sdpa_b200_last_error",
     "sdpa_b200_fwd_workspace_bytes",
     "sdpa_b200_bwd_workspace_bytes",
+    "sdpa_b200_bwd_workspace_least_bytes",
     "sdpa_b200_fwd",
     "sdpa_b200_bwd",
     "sdpa_b200_read_device_status",
@@ -93,7 +94,7 @@ def load() -> ctypes.CDLL:
     lib.sdpa_b200_status_string.argtypes = [c_int]
     lib.sdpa_b200_last_error.restype = c_char_p
     lib.sdpa_b200_launch_count.restype = c_uint64
-    for name in ("sdpa_b200_fwd_workspace_bytes", "sdpa_b200_bwd_workspace_bytes"):
+    for name in ("sdpa_b200_fwd_workspace_bytes", "sdpa_b200_bwd_workspace_bytes", "sdpa_b200_bwd_workspace_least_bytes"):
         fn = getattr(lib, name)
         fn.restype = c_int
         fn.argtypes = [POINTER(SdpaParams), POINTER(c_size_t)]

@@ -6,6 +6,16 @@
 
 namespace sdpa_b200 {
 
+// How a call's dS goes through the workspace: `kv_heads` (batch * heads_kv indexes) per pass, `tiles` of room, none if 0.
+struct DsPlan {
+  int kv_heads = 0;
+  uint32_t tiles = 0;
+};
+
+DsPlan ds_plan(const sdpa_b200_params& p);
+size_t ds_table_bytes(const sdpa_b200_params& p);  // DsTiles::seq_base, in front of the tiles
+size_t ds_workspace_bytes(const sdpa_b200_params& p, const DsPlan& plan);
+
 struct DsGemmParams {
   DsTiles ds;
   const int32_t* cu_q;

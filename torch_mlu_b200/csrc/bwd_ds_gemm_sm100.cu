@@ -387,6 +387,43 @@ Kernel pick_kernel(int head_dim, bool f16) {
 
 }  // namespace
 
+// dS of a call (half of B H Lq Lk elements of two bytes under a causal mask) may take this much of the workspace; a dense call with
+// more of it goes through it in several passes over its KV heads. One pass is best (step of B8 H16 L2048, 0.57 GB of dS: 673 us in
+// one pass, 709 in two, 766 in six, where a pass's dS would stay in L2; B2 H16 L8192, 2.1 GB: 2115 in one, 2189 in two).
+constexpr size_t kDsBytesMax = size_t{2} << 30;
+
+DsPlan ds_plan(const sdpa_b200_params& p) {
+  DsPlan plan;
+  const int64_t cap = static_cast<int64_t>(kDsBytesMax / kDsTileBytes);
+  const int64_t key_tiles = (static_cast<int64_t>(p.max_seqlen_k) + kDsTile - 1) / kDsTile;
+  const int64_t kv_heads = static_cast<int64_t>(p.batch) * p.heads_kv;
+  if (p.cu_seqlens_q != nullptr) {
+    // the lengths are on the device: every query tile there can be, against the longest keys
+    const int64_t tiles = (p.total_q / kDsTile + p.batch) * key_tiles * p.heads_q;
+    if (tiles > cap) return plan;
+    plan.kv_heads = static_cast<int>(kv_heads);
+    plan.tiles = static_cast<uint32_t>(tiles);
+    return plan;
+  }
+  const int64_t per_kv_head = p.heads_q / p.heads_kv * ds_tiles_per_head(p.max_seqlen_q, p.max_seqlen_k, p.is_causal != 0);
+  if (per_kv_head <= 0 || per_kv_head > cap) return plan;
+  const int64_t passes = (kv_heads * per_kv_head + cap - 1) / cap;
+  int64_t per_pass = (kv_heads + passes - 1) / passes;
+  if (per_pass * per_kv_head > cap) per_pass = cap / per_kv_head;
+  if (passes > 1 && per_pass * key_tiles < 3 * 148) return plan;  // a pass must fill the SMs a few times over
+  plan.kv_heads = static_cast<int>(per_pass);
+  plan.tiles = static_cast<uint32_t>(per_pass * per_kv_head);
+  return plan;
+}
+
+size_t ds_table_bytes(const sdpa_b200_params& p) {
+  return p.cu_seqlens_q != nullptr ? (static_cast<size_t>(p.batch) * sizeof(int32_t) + 255) / 256 * 256 : 0;
+}
+
+size_t ds_workspace_bytes(const sdpa_b200_params& p, const DsPlan& plan) {
+  return plan.tiles > 0 ? ds_table_bytes(p) + plan.tiles * kDsTileBytes : 0;
+}
+
 int launch_bwd_ds_gemm(const sdpa_b200_params& p, const DsTiles& ds, int kv_head0, int num_kv_heads, bool with_dk,
                        uint32_t* counter, uint32_t* status, cudaStream_t stream) {
   const bool f16 = p.dtype == SDPA_B200_F16;
@@ -436,9 +473,9 @@ int launch_bwd_ds_gemm(const sdpa_b200_params& p, const DsTiles& ds, int kv_head
   kp.num_kv_heads = num_kv_heads;
   kp.query_pairs = (p.max_seqlen_q + kPair - 1) / kPair;
   kp.key_pairs = (p.max_seqlen_k + kPair - 1) / kPair;
-  // heads per group: with dK, the dS of a group stays in L2 for its second reader; without, only the B operand is re-read
-  const double per_head = with_dk ? 2.0 * kp.kv_group * p.max_seqlen_q * p.max_seqlen_k / (p.is_causal ? 2 : 1)
-                                  : 2.0 * p.max_seqlen_k * p.head_dim;
+  // heads per group: the rows of the B operands are re-read by every unit of their head. (With dK too, groups of 1 to 8 heads, whose
+  // dS might come from L2 the second time, make no difference: B4 H16 L4096 D256 576 to 580 us.)
+  const double per_head = 2.0 * p.head_dim * (p.max_seqlen_k + (with_dk ? kp.kv_group * static_cast<double>(p.max_seqlen_q) : 0.0));
   int hpg = static_cast<int>(48.0 * 1024 * 1024 / per_head);
   hpg = hpg < 1 ? 1 : (hpg > 32 ? 32 : hpg);
   if (hpg > num_kv_heads) hpg = num_kv_heads;

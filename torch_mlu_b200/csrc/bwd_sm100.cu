@@ -920,15 +920,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     len_q = p.cu_q[b + 1] - q_off;
   }
   if (kPacked && p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0) {
-    __shared__ int tiles_before;
-    if (threadIdx.x == 0) tiles_before = 0;
-    __syncthreads();
-    int mine = 0;
-    for (int i = threadIdx.x; i < b; i += 256)
-      mine += static_cast<int>(ds_tiles_per_head(p.cu_q[i + 1] - p.cu_q[i], p.cu_k[i + 1] - p.cu_k[i], p.is_causal != 0));
-    if (mine != 0) atomicAdd(&tiles_before, mine);
-    __syncthreads();
-    if (threadIdx.x == 0) p.ds_seq_base[b] = tiles_before;
+    write_seq_base(p.ds_seq_base, p.cu_q, p.cu_k, b, p.is_causal != 0);
   }
   if (p.dq_acc != nullptr) {
     // 64 rows of an accumulator tile: per 4-column group 1 KB of consecutive floats, a thread per row. The stores need no
@@ -1093,46 +1085,6 @@ bool use_fused_backward(const sdpa_b200_params& p) {
   return p.head_dim <= 64 || (!use_ds_backward(p) && (p.heads_q == p.heads_kv || p.dropout_p > 0.f));
 }
 
-// dS of a call (half of B H Lq Lk elements of two bytes under a causal mask) may take this much of the workspace; a dense call with
-// more of it goes through it in several passes over its KV heads. One pass is best (step of B8 H16 L2048, 0.57 GB of dS: 673 us in
-// one pass, 709 in two, 766 in six, where a pass's dS would stay in L2; B2 H16 L8192, 2.1 GB: 2115 in one, 2189 in two).
-constexpr size_t kDsBytesMax = size_t{2} << 30;
-
-// How a call's dS goes through the workspace: `kv_heads` (batch * heads_kv indexes) per pass, `tiles` of room, none if 0.
-struct DsPlan {
-  int kv_heads = 0;
-  uint32_t tiles = 0;
-};
-
-DsPlan ds_plan(const sdpa_b200_params& p) {
-  DsPlan plan;
-  if (!use_ds_backward(p)) return plan;
-  const int64_t cap = static_cast<int64_t>(kDsBytesMax / kDsTileBytes);
-  const int64_t key_tiles = (static_cast<int64_t>(p.max_seqlen_k) + kDsTile - 1) / kDsTile;
-  const int64_t kv_heads = static_cast<int64_t>(p.batch) * p.heads_kv;
-  if (p.cu_seqlens_q != nullptr) {
-    // the lengths are on the device: every query tile there can be, against the longest keys
-    const int64_t tiles = (p.total_q / kDsTile + p.batch) * key_tiles * p.heads_q;
-    if (tiles > cap) return plan;
-    plan.kv_heads = static_cast<int>(kv_heads);
-    plan.tiles = static_cast<uint32_t>(tiles);
-    return plan;
-  }
-  const int64_t per_kv_head = p.heads_q / p.heads_kv * ds_tiles_per_head(p.max_seqlen_q, p.max_seqlen_k, p.is_causal != 0);
-  if (per_kv_head <= 0 || per_kv_head > cap) return plan;
-  const int64_t passes = (kv_heads * per_kv_head + cap - 1) / cap;
-  int64_t per_pass = (kv_heads + passes - 1) / passes;
-  if (per_pass * per_kv_head > cap) per_pass = cap / per_kv_head;
-  if (passes > 1 && per_pass * key_tiles < 3 * 148) return plan;  // a pass must fill the SMs a few times over
-  plan.kv_heads = static_cast<int>(per_pass);
-  plan.tiles = static_cast<uint32_t>(per_pass * per_kv_head);
-  return plan;
-}
-
-size_t ds_table_bytes(const sdpa_b200_params& p) {
-  return p.cu_seqlens_q != nullptr ? (static_cast<size_t>(p.batch) * sizeof(int32_t) + 255) / 256 * 256 : 0;
-}
-
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
   const size_t bytes = 2 * static_cast<size_t>(p.batch) * p.heads_q * lq_padded(p) * sizeof(float);
   return (bytes + 255) / 256 * 256;
@@ -1147,8 +1099,8 @@ size_t bwd_workspace_min_bytes(const sdpa_b200_params& p) {
 
 // What it is best given: room for dS too. A call that is given less takes the two kernels.
 size_t bwd_workspace_bytes(const sdpa_b200_params& p) {
-  const DsPlan plan = ds_plan(p);
-  const size_t with_ds = plan.tiles > 0 ? bwd_vector_bytes(p) + ds_table_bytes(p) + plan.tiles * kDsTileBytes : 0;
+  const DsPlan plan = use_ds_backward(p) ? ds_plan(p) : DsPlan();
+  const size_t with_ds = plan.tiles > 0 ? bwd_vector_bytes(p) + ds_workspace_bytes(p, plan) : 0;
   const size_t least = bwd_workspace_min_bytes(p);
   return with_ds > least ? with_ds : least;
 }
@@ -1181,7 +1133,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   pre.head_dim = p.head_dim;
   pre.grads = packed_grads(p);
   const bool fused = use_fused_backward(p);
-  const DsPlan plan = ds_plan(p);
+  const DsPlan plan = use_ds_backward(p) ? ds_plan(p) : DsPlan();
   const bool through_ds = plan.tiles > 0 && workspace_bytes >= kWorkspaceHeaderBytes + bwd_workspace_bytes(p);
   char* behind_vectors = static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p);
   pre.ds_seq_base = through_ds && varlen ? reinterpret_cast<int32_t*>(behind_vectors) : nullptr;

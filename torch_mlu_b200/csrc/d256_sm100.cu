@@ -20,6 +20,7 @@
 // behind PV(j), so the next block's scores are formed while this block is exponentiated.
 #include <cuda_bf16.h>
 
+#include "bwd_ds_gemm.h"
 #include "kernels.h"
 #include "packed_grads.cuh"
 #include "ptx_sm100.cuh"
@@ -427,7 +428,12 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Backward. Three kernels from one template, all with 128 stationary rows in tensor memory and 64-row streamed blocks:
+// Backward. One kernel and two GEMMs, or three kernels; the kernels come from one template, all with 128 stationary rows in tensor
+// memory and 64-row streamed blocks:
+//   kDVS: CTA = 128 keys. X1 = K (TMEM), X2 = V (shared memory, 64 KB). Streams (Q, dO) blocks of 64 queries of every query head of the
+//        KV head. S^T = K Q^T, dP^T = V dO^T; P^T = exp2(S^T c - lse2[q]), dV += P^T dO; dS^T = P^T o (dP^T - delta[q]) goes to
+//        the workspace (ds_tiles.cuh), from where bwd_ds_gemm_sm100.cu forms dK = scale dS^T Q and dQ = scale dS K.
+//                                                                                               TMEM: K | S dP | dV
 //   kDV: CTA = 128 keys. X1 = K (TMEM). Streams (Q, dO) blocks of 64 queries of every query head of the KV head.
 //        S^T = K Q^T; P^T = exp2(S^T c - lse2[q]); dV += P^T dO.                                TMEM: K | S0 S1 | dV
 //   kDK: CTA = 128 keys. X1 = K (TMEM), X2 = V (shared memory, 64 KB). Streams (Q, dO).
@@ -436,24 +442,28 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
 //        S = Q K^T, dP = dO V^T; dS = P o (dP - delta[row]); dQ += dS K.                          TMEM: Q | TA TB | dQ
 // A 128 x 256 fp32 accumulator is half the tensor memory, so every kernel owns exactly one; dK and dV therefore come from
 // two kernels that both form S (9 GEMM-equivalents per tile pair against the 5 of the algorithm). The score GEMM with X2
-// reads both operands from shared memory (N = 64: 48 cycles per MMA instead of 32).
+// reads both operands from shared memory (N = 64: 48 cycles per MMA instead of 32). So the three run only where there is no room
+// for dS (launch_bwd_d256): B4 H16 L4096 causal dV 541, dK 725, dQ 718 us against kDVS 837 and both GEMMs 580.
 // kDV: S(i) in T[i&1], the 16-bit P over its front; S(i+2) follows the accumulation of item i.
-// kDK, kDQ: S always in TA, dP in TB; both are free once the compute warps have read them, because the 16-bit dS goes to a
+// kDVS, kDK, kDQ: S always in TA, dP in TB; both are free once the compute warps have read them, because the 16-bit dS (kDVS: P) goes to a
 // shared-memory tile (N = 256 MMAs run at full rate with both operands there). In the pipe S(i+2) and dP(i+1) stand in front
 // of ACC(i), so it works while the compute warps form dS(i).
+// kDVS: what bounds it is shared memory: per item 32 KB of B for S, 96 KB for dP, 48 KB for ACC, 64 KB from TMA, 16 KB of P and the
+// compute warps' 16-byte reads of lse2 and delta (128 instructions of four cycles): 2560 of about 2900 cycles. A second pair of
+// compute warpgroups that took every other item changed nothing (855 us).
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kDV = 0, kDK = 1, kDQ = 2;
+constexpr int kDV = 0, kDK = 1, kDQ = 2, kDVS = 3;
 // warps 0-3 / 4-7: two compute warpgroups, one per 32-row half of every streamed block (thread = stationary row);
 // warp 8 TMA producer, warps 9 and 10 MMA issuers
 constexpr int kBwdThreads = 352;
 
 // Shared memory. kDV: a ring of six 32 KB slots (Q, dO, Q, dO ...), then the per-query vectors of each dO slot.
-// kDK, kDQ: X2 | three slots for the Y1 blocks | three half slots for the Y2 blocks | dS tile | vectors of each Y1 slot.
+// kDVS, kDK, kDQ: X2 | three slots for the Y1 blocks | three half slots for the Y2 blocks | dS tile | vectors of each Y1 slot.
 // A Y1 block is held from its score GEMM to its accumulation, more than one item later; a Y2 block only for its own score
 // GEMM, and its two halves (128 columns each) are released one by one. Three slots and three half slots leave every load at
 // least one period of about 1800 tensor cycles to arrive, which two and two whole slots do not.
 constexpr int kRingDV = 6;
-constexpr int kY1Slots = 3, kY2Halves = 3;
+constexpr int kY1Slots = 3, kY2Halves = 3;  // kDVS: Y1 = dO, Y2 = Q
 constexpr uint32_t kHalfSlotBytes = kSlotBytes / 2;
 constexpr uint32_t kSmemY1 = 2 * kSlotBytes;                             // behind X2
 constexpr uint32_t kSmemY2 = kSmemY1 + kY1Slots * kSlotBytes;
@@ -496,10 +506,24 @@ struct Bwd256Params {
   const uint32_t* keep_cols;  // [batch*heads_q][keep_k_rows][keep_lq_pad / 32]: kDV, kDK
   int keep_lq_pad, keep_lk_pad, keep_q_rows, keep_k_rows;
   float keep_scale;
+  // kDVS: where dS goes for the dK and dQ GEMMs, their unit counter, and the first (batch, KV head) of this launch
+  DsTiles ds;
+  uint32_t* ds_counter;
+  int bh0;
 };
 
 template <bool kF16>
 constexpr uint32_t kIdescS64SS = umma_idesc_16(kRowsA, kRowsB, false, false, kF16);
+
+// half kHalf of issue_scores(): the 128 columns that one half of a streamed block (two boxes) holds
+template <bool kF16, int kHalf>
+__device__ __forceinline__ void issue_scores_half(uint32_t t_s, uint32_t a_tmem, uint32_t y_half) {
+#pragma unroll
+  for (int ks = 0; ks < kWide / 32; ++ks) {
+    const uint32_t b_lo = umma_desc_lo_kmajor(y_half + (ks >> 2) * kBoxBytes + (ks & 3) * 32);
+    umma_ts_lo<kIdescS64<kF16>>(t_s, a_tmem + (kHalf * 8 + ks) * 8, b_lo, (kHalf > 0 || ks > 0) ? 1u : 0u);
+  }
+}
 
 // ACC (128 x 256) (+)= W * B with W written by two warpgroups, each over the front of its own 32 score columns: the 16-bit
 // rows 0-31 of the block sit in columns [0,16) of the buffer, rows 32-63 in columns [32,48)
@@ -567,6 +591,11 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   constexpr bool kKeys = kMode != kDQ;  // the stationary rows are keys
+  if (kMode == kDVS && threadIdx.x == 0) {
+    // the GEMMs behind wait for this grid before they read the counter or dS; their set-up may run under its tail
+    if (blockIdx.x == 0) *p.ds_counter = 0u;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
 
   // CTA order as in the forward: groups of heads whose streamed tensors fit L2, heaviest row blocks first
   // (key block 0 sees every query; the last query block sees every key)
@@ -577,7 +606,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     const int w = blockIdx.x - grp * per_group;
     const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
     const int rank = w / size;
-    const int bh = grp * p.heads_per_wave + (w - rank * size);
+    const int bh = (kMode == kDVS ? p.bh0 : 0) + grp * p.heads_per_wave + (w - rank * size);
     if (rank >= p.num_row_blocks) return;
     xb = kKeys ? rank : p.num_row_blocks - 1 - rank;
     b = bh / p.heads_x;
@@ -605,6 +634,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     if (p.is_causal) {
       y_lo = max(0, (x0 - causal_off) / kRowsB);  // first query block with a row >= x0 - off
       if (x0 - causal_off > len_q - 1) y_lo = y_hi;
+      else if (kMode == kDVS) y_lo &= ~1;  // a dS tile has two blocks: both are written, the hidden one with zeros
     }
   } else {
     int vis_end = len_k;
@@ -625,7 +655,8 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     tma_prefetch_desc(&tm_y2);
     for (int s = 0; s < kSlots; ++s) {
       mbar_init(bar + kBFull + 8 * s, 1);
-      mbar_init(bar + kBEmpty + 8 * s, 1);
+      // kDVS: delta rides with a dO block, and the compute warps read it after the accumulation may have released the block
+      mbar_init(bar + kBEmpty + 8 * s, kMode == kDVS && s < kY1Slots ? 9 : 1);
     }
     mbar_init(bar + kBAReady, 8);
     mbar_init(bar + kBX2Full, 1);
@@ -694,8 +725,8 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
         int hy, yb;
         item_pos(i, hy, yb);
         const uint32_t full = bar + kBFull + 8 * s, dst = y1_addr(i);
-        mbar_arrive_expect_tx(full, kSlotBytes + (kMode == kDK ? 512 : 0));
-        if constexpr (kMode == kDK) load_vectors(hy, yb, s, full);
+        mbar_arrive_expect_tx(full, kSlotBytes + (kMode == kDK || kMode == kDVS ? 512 : 0));
+        if constexpr (kMode == kDK || kMode == kDVS) load_vectors(hy, yb, s, full);
 #pragma unroll
         for (int c = 0; c < 4; ++c) tma_load_4d(dst + c * kBoxBytes, &tm_y1, full, c * 64, y_off + yb * kRowsB, hy, bcoord);
         return true;
@@ -727,15 +758,27 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
             tma_load_4d(dst + c * kBoxBytes, &tm_y2, full, (n & 1) * 128 + c * 64, y_off + yb * kRowsB, hy, bcoord);
           return true;
         };
-        // what fits at once, then in the order in which the slots come free: half of dP(i), its end, the end of ACC(i-1)
         bool ok = true;
-        if (n_items > 0) ok = load_y1(0) && load_y2(0) && load_y2(1);
-        if (n_items > 1) ok = ok && load_y1(1) && load_y2(2);
-        if (n_items > 2) ok = ok && load_y1(2);
-        for (int i = 0; ok && i + 1 < n_items; ++i) {
-          ok = load_y2(2 * i + 3);
-          if (ok && i + 2 < n_items) ok = load_y2(2 * i + 4);
-          if (ok && i > 0 && i + 2 < n_items) ok = load_y1(i + 2);
+        if constexpr (kMode == kDVS) {
+          // Q halves come free with S, dO blocks with the accumulation of P and the last read of delta
+          if (n_items > 0) ok = load_y2(0) && load_y2(1) && load_y1(0);
+          if (n_items > 1) ok = ok && load_y2(2) && load_y1(1);
+          if (n_items > 2) ok = ok && load_y1(2);
+          for (int i = 0; ok && i + 1 < n_items; ++i) {
+            ok = load_y2(2 * i + 3);
+            if (ok && i + 2 < n_items) ok = load_y2(2 * i + 4);
+            if (ok && i + 3 < n_items) ok = load_y1(i + 3);
+          }
+        } else {
+          // what fits at once, then in the order in which the slots come free: half of dP(i), its end, the end of ACC(i-1)
+          if (n_items > 0) ok = load_y1(0) && load_y2(0) && load_y2(1);
+          if (n_items > 1) ok = ok && load_y1(1) && load_y2(2);
+          if (n_items > 2) ok = ok && load_y1(2);
+          for (int i = 0; ok && i + 1 < n_items; ++i) {
+            ok = load_y2(2 * i + 3);
+            if (ok && i + 2 < n_items) ok = load_y2(2 * i + 4);
+            if (ok && i > 0 && i + 2 < n_items) ok = load_y1(i + 2);
+          }
         }
       }
       drain_after_abort(abort_flag);
@@ -784,7 +827,23 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
         // ---------------- scores: S(0) dP(0) S(1), then dP(i+1) as soon as dP(i) has been read and S(i+2) as soon as S(i+1)
         // has. The pipe thus always holds work that does not wait for the dS of item i, which the compute warps form
         // meanwhile. With dP(i+1) behind ACC(i) instead it stood still under them: 3300 cycles per item, 1800 of tensor work.
+        auto wait_y2 = [&](int n) {
+          return mbar_wait(bar + kBFull + 8 * (kY1Slots + y2_index(n)), static_cast<uint32_t>(n / kY2Halves) & 1u, abort_flag);
+        };
+        auto release_y2 = [&](int n) { umma_commit(bar + kBEmpty + 8 * (kY1Slots + y2_index(n))); };
         auto scores = [&](int i) -> bool {
+          if constexpr (kMode == kDVS) {
+            if (!wait_y2(2 * i)) return false;
+            tc_fence_after_sync();
+            issue_scores_half<kF16, 0>(t_a, t_x1, y2_addr(2 * i));
+            release_y2(2 * i);
+            if (!wait_y2(2 * i + 1)) return false;
+            tc_fence_after_sync();
+            issue_scores_half<kF16, 1>(t_a, t_x1, y2_addr(2 * i + 1));
+            release_y2(2 * i + 1);
+            umma_commit(bar + kBTFull);
+            return true;
+          }
           if (!wait_y1(i)) return false;
           tc_fence_after_sync();
           issue_scores<kF16>(t_a, t_x1, y1_addr(i));
@@ -793,14 +852,22 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
         };
         auto half_dp = [&](int i, auto kHalf) -> bool {
           constexpr int h = decltype(kHalf)::value;
-          const int n = 2 * i + h, s = kY1Slots + y2_index(n);
-          if (!mbar_wait(bar + kBFull + 8 * s, static_cast<uint32_t>(n / kY2Halves) & 1u, abort_flag)) return false;
+          const int n = 2 * i + h;
+          if (!wait_y2(n)) return false;
           tc_fence_after_sync();
           issue_scores_ss<kF16, h>(t_b, base, y2_addr(n));
-          umma_commit(bar + kBEmpty + 8 * s);
+          release_y2(n);
           return true;
         };
         auto dp = [&](int i) -> bool {
+          if constexpr (kMode == kDVS) {
+            if (!wait_y1(i)) return false;
+            tc_fence_after_sync();
+            issue_scores_ss<kF16, 0>(t_b, base, y1_addr(i));
+            issue_scores_ss<kF16, 1>(t_b, base, y1_addr(i) + 2 * kBoxBytes);
+            umma_commit(bar + kBTFull + 8);
+            return true;
+          }
           if (!half_dp(i, std::integral_constant<int, 0>{}) || !half_dp(i, std::integral_constant<int, 1>{})) return false;
           umma_commit(bar + kBTFull + 8);
           return true;
@@ -812,7 +879,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
           if (i + 2 < n_items) ok = ok && mbar_wait(bar + kBSFree, (i + 1) & 1, abort_flag) && scores(i + 2);
         }
       } else {
-        // ---------------- accumulations: ACC += dS(i) Y1(i)
+        // ---------------- accumulations: ACC += dS(i) Y1(i); kDVS: P^T(i) dO(i)
         for (int i = 0; ok && i < n_items; ++i) {
           ok = mbar_wait(bar + kBWFull, i & 1, abort_flag) && wait_y1(i);
           if (!ok) break;
@@ -849,6 +916,16 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
       const size_t vec = (static_cast<size_t>(b) * p.heads_q + hx) * p.lq_pad + xr;
       my_lse2 = p.lse2[vec];
       my_delta = p.delta[vec];
+    }
+    // kDVS: tile (query tile 0, this key block) of the group's first query head, and what leads from it to the others
+    uint32_t ds_tile0 = 0, ds_per_head = 0;
+    int ds_key_tiles = 0, ds_shift_rows = 0;
+    if constexpr (kMode == kDVS) {
+      const DsHead dh = ds_head(p.ds, b, hx * p.kv_group, p.heads_q, len_q, len_k, p.is_causal != 0);
+      ds_tile0 = static_cast<uint32_t>(dh.base + xb);
+      ds_per_head = static_cast<uint32_t>(ds_tiles_per_head(len_q, len_k, p.is_causal != 0));
+      ds_key_tiles = dh.key_tiles;
+      ds_shift_rows = dh.shift;
     }
     bool ok = true;
     for (int i = 0; i < n_items; ++i) {
@@ -918,15 +995,17 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
         }
       }
       uint32_t w[kCols / 2];
-      if (kMode == kDV) {
+      // the 16-bit P, for dV
+      auto pack_p = [&]() {
 #pragma unroll
         for (int j2 = 0; j2 < kCols / 2; ++j2) {
           if constexpr (kDrop) w[j2] = pack_16x2<kF16>(kept(keep, 2 * j2, pr[2 * j2]), kept(keep, 2 * j2 + 1, pr[2 * j2 + 1]));
           else w[j2] = pack_16x2<kF16>(pr[2 * j2], pr[2 * j2 + 1]);
         }
-      } else {
-        ok = __all_sync(0xffffffffu, mbar_wait(bar + kBTFull + 8, i & 1, abort_flag));
-        if (!ok) break;
+      };
+      // dP out of TMEM, dS = P o (dP - delta) into w
+      auto form_ds = [&]() -> bool {
+        if (!__all_sync(0xffffffffu, mbar_wait(bar + kBTFull + 8, i & 1, abort_flag))) return false;
         tc_fence_after_sync();
         uint32_t d[kCols];
         tmem_ld_x32(t_b + lane_base + half * 32, d);
@@ -949,36 +1028,61 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
           }
           w[j2] = pack_16x2<kF16>(pr[2 * j2] * e0, pr[2 * j2 + 1] * e1);
         }
-      }
-      if (kMode == kDV) {
-        // the 16-bit P over the front of this thread's OWN score columns (16 columns = 32 streamed rows): the other
-        // warpgroup may still be reading its half of the scores
-        tmem_st_x16(t_s, w);
-        tmem_wait_st();
-      } else {
-        // the dS tile is free once ACC(i-1) has read it
-        if (i > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(bar + kBWRead, (i - 1) & 1, abort_flag));
-          if (!ok) break;
-        }
-        // the 16-bit dS into the shared tile: row r of 128 bytes, 16-byte chunks XOR-swizzled by (row % 8)
+        return true;
+      };
+      // w into the shared A tile of the accumulation, once ACC(i-1) has read it: row r of 128 bytes, 16-byte chunks XOR-swizzled
+      // by (row % 8)
+      auto w_to_smem = [&]() -> bool {
+        if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(bar + kBWRead, (i - 1) & 1, abort_flag))) return false;
         uint8_t* wrow = smem + kSmemW + r * 128;
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch)
           *reinterpret_cast<uint4*>(wrow + (((half * 4 + ch) ^ (r & 7)) << 4)) =
               make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
         fence_proxy_async_smem();
+        return true;
+      };
+      auto w_full = [&]() {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar + kBWFull);
+      };
+      if constexpr (kMode == kDV) {
+        // over the front of this thread's OWN score columns (16 columns = 32 streamed rows): the other warpgroup may still be
+        // reading its half of the scores
+        pack_p();
+        tmem_st_x16(t_s, w);
+        tmem_wait_st();
+        w_full();
+      } else if constexpr (kMode == kDVS) {
+        pack_p();
+        ok = w_to_smem();
+        if (!ok) break;
+        w_full();
+        ok = form_ds();
+        if (!ok) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar + kBEmpty + 8 * vec_slot);  // delta(i) has been read
+        // 16 bytes (8 queries) per store, 512 contiguous bytes per warp
+        const uint32_t tile = ds_tile0 + static_cast<uint32_t>(hi) * ds_per_head +
+                              static_cast<uint32_t>(ds_row_start(y0 / kDsTile, ds_key_tiles, ds_shift_rows));
+        if (tile < p.ds.capacity) {
+          uint4* dst = ds_group(p.ds, tile, ((y0 & (kDsTile - 1)) >> 3) + half * 4, r);
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) dst[ch * kDsTile] = make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+        }
+      } else {
+        ok = form_ds() && w_to_smem();
+        if (!ok) break;
+        w_full();
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar + kBWFull);
     }
 
     // ---- epilogue: accumulator -> scale -> 16 bit -> global
     if (ok && n_items > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar + kBAccFull, 0, abort_flag));
     if (ok) {
       tc_fence_after_sync();
-      const float mul = (kMode == kDV) ? (kDrop ? p.keep_scale : 1.f) : p.scale;
+      const float mul = (kMode == kDV || kMode == kDVS) ? (kDrop ? p.keep_scale : 1.f) : p.scale;
       constexpr uint32_t kStageBase = kMode == kDV ? 0u : kSmemY1;
       const bool use_tma = (p.cu_q == nullptr) || (x0 + kRowsA <= len_x);
       uint16_t* orow = p.out + ((p.cu_q != nullptr) ? static_cast<int64_t>(x_off + xr) * p.o_row_stride
@@ -1055,6 +1159,9 @@ struct Pre256Params {
   int64_t do_batch_stride, do_head_stride, do_row_stride;
   int seqlen_q, total_q, heads_q, lq_pad, head_dim;
   PackedGrads grads;
+  int32_t* ds_seq_base;  // packed, dS through the workspace: DsTiles::seq_base, written here; else null
+  const int32_t* cu_k;
+  int is_causal;
 };
 
 // Each warp takes four rows whose loads are all issued before the first use: 57 -> 48 us at B4 H16 L4096 (268 MB).
@@ -1072,6 +1179,7 @@ __global__ void __launch_bounds__(256) bwd_d256_preprocess_kernel(const Pre256Pa
   if (kPacked) {
     q_off = p.cu_q[b];
     len_q = p.cu_q[b + 1] - q_off;
+    if (p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0) write_seq_base(p.ds_seq_base, p.cu_q, p.cu_k, b, p.is_causal != 0);
   }
   const uint16_t* o = p.out + h * p.o_head_stride + (kPacked ? q_off * p.o_row_stride : b * p.o_batch_stride) + lane * 8;
   const uint16_t* dout =
@@ -1130,12 +1238,17 @@ Bwd256Kernel pick_bwd256(bool f16, bool drop) {
 }
 }  // namespace
 
-size_t bwd_d256_workspace_bytes(const sdpa_b200_params& p) {
+size_t bwd_d256_workspace_min_bytes(const sdpa_b200_params& p) {
   const size_t lq_pad = (static_cast<size_t>(p.max_seqlen_q) + kRowsA - 1) / kRowsA * kRowsA;
   return 2 * static_cast<size_t>(p.batch) * p.heads_q * lq_pad * sizeof(float);
 }
 
-int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t stream) {
+// lse2 and delta, then room for dS. A call that is given less takes the three kernels that each form the scores.
+size_t bwd_d256_workspace_bytes(const sdpa_b200_params& p) {
+  return (bwd_d256_workspace_min_bytes(p) + 255) / 256 * 256 + ds_workspace_bytes(p, ds_plan(p));
+}
+
+int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   const bool f16 = p.dtype == SDPA_B200_F16;
   const bool varlen = p.cu_seqlens_q != nullptr;
   const int lq_pad = (p.max_seqlen_q + kRowsA - 1) / kRowsA * kRowsA;
@@ -1162,6 +1275,12 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   pre.lq_pad = lq_pad;
   pre.head_dim = p.head_dim;
   pre.grads = packed_grads(p);
+  const DsPlan plan = ds_plan(p);
+  const bool through_ds = plan.tiles > 0 && workspace_bytes >= kWorkspaceHeaderBytes + bwd_d256_workspace_bytes(p);
+  char* behind_vectors = static_cast<char*>(workspace) + kWorkspaceHeaderBytes + (bwd_d256_workspace_min_bytes(p) + 255) / 256 * 256;
+  pre.ds_seq_base = through_ds && varlen ? reinterpret_cast<int32_t*>(behind_vectors) : nullptr;
+  pre.cu_k = p.cu_seqlens_k;
+  pre.is_causal = p.is_causal;
   const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), lq_pad / (8 * kPre256Rows), p.batch);
   auto pre_kernel = varlen ? (f16 ? bwd_d256_preprocess_kernel<true, true> : bwd_d256_preprocess_kernel<false, true>)
                            : (f16 ? bwd_d256_preprocess_kernel<true, false> : bwd_d256_preprocess_kernel<false, false>);
@@ -1217,10 +1336,12 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   kp.keep_k_rows = varlen ? p.total_k + 128 : kp.keep_lk_pad;
   kp.keep_scale = drop ? 1.f / (1.f - p.dropout_p) : 1.f;
 
-  auto launch = [&](int mode, const CUtensorMap& x2, const CUtensorMap& y1, const CUtensorMap& y2, const CUtensorMap& out) {
+  // `kv_heads`: batch * heads_kv indexes from kp.bh0 on, kDVS only
+  auto launch = [&](int mode, const CUtensorMap& x2, const CUtensorMap& y1, const CUtensorMap& y2, const CUtensorMap& out, int kv_heads) {
     void (*kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const Bwd256Params);
     if (mode == kDV) kernel = pick_bwd256<kDV>(f16, drop);
     else if (mode == kDK) kernel = pick_bwd256<kDK>(f16, drop);
+    else if (mode == kDVS) kernel = pick_bwd256<kDVS>(f16, drop);
     else kernel = pick_bwd256<kDQ>(f16, drop);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesBwd256);
     if (e != cudaSuccess) {
@@ -1229,7 +1350,7 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
     }
     const bool keys = mode != kDQ;
     kp.heads_x = keys ? p.heads_kv : p.heads_q;
-    kp.num_bh = p.batch * kp.heads_x;
+    kp.num_bh = mode == kDVS ? kv_heads : p.batch * kp.heads_x;
     kp.num_row_blocks = ((keys ? p.max_seqlen_k : p.max_seqlen_q) + kRowsA - 1) / kRowsA;
     // bytes one stationary head streams: Q + dO of its group (keys), or K + V (queries)
     const double streamed = 2.0 * (keys ? p.max_seqlen_q : p.max_seqlen_k) * p.head_dim * 2 * (keys ? kp.kv_group : 1);
@@ -1256,11 +1377,26 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
     kp.o_row_stride = ors;
   };
   set_io(p.k, p.k_batch_stride, p.k_head_stride, p.k_row_stride, p.dv, p.dv_batch_stride, p.dv_head_stride, p.dv_row_stride);
-  if ((st = launch(kDV, v128 /*unused*/, q64, do64, dv128)) != SDPA_B200_OK) return st;
+  if (through_ds) {
+    kp.ds.data = reinterpret_cast<uint16_t*>(behind_vectors + ds_table_bytes(p));
+    kp.ds.seq_base = pre.ds_seq_base;
+    kp.ds.capacity = plan.tiles;
+    kp.ds_counter = static_cast<uint32_t*>(workspace) + 2;
+    const int kv_heads = p.batch * p.heads_kv;
+    for (int first = 0; first < kv_heads; first += plan.kv_heads) {
+      const int n = kv_heads - first < plan.kv_heads ? kv_heads - first : plan.kv_heads;
+      kp.bh0 = first;
+      kp.ds.head0 = first * kp.kv_group;
+      if ((st = launch(kDVS, v128, do64, q64, dv128, n)) != SDPA_B200_OK) return st;
+      if ((st = launch_bwd_ds_gemm(p, kp.ds, first, n, true, kp.ds_counter, kp.status, stream)) != SDPA_B200_OK) return st;
+    }
+    return SDPA_B200_OK;
+  }
+  if ((st = launch(kDV, v128 /*unused*/, q64, do64, dv128, 0)) != SDPA_B200_OK) return st;
   set_io(p.k, p.k_batch_stride, p.k_head_stride, p.k_row_stride, p.dk, p.dk_batch_stride, p.dk_head_stride, p.dk_row_stride);
-  if ((st = launch(kDK, v128, q64, do64, dk128)) != SDPA_B200_OK) return st;
+  if ((st = launch(kDK, v128, q64, do64, dk128, 0)) != SDPA_B200_OK) return st;
   set_io(p.q, p.q_batch_stride, p.q_head_stride, p.q_row_stride, p.dq, p.dq_batch_stride, p.dq_head_stride, p.dq_row_stride);
-  return launch(kDQ, do128, k64, v64, dq128);
+  return launch(kDQ, do128, k64, v64, dq128, 0);
 }
 
 int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t stream) {

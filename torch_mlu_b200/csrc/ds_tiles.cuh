@@ -63,4 +63,17 @@ __device__ __forceinline__ uint4* ds_group(const DsTiles& ds, uint32_t tile, int
   return reinterpret_cast<uint4*>(ds.data) + static_cast<size_t>(tile) * (kDsTileBytes / 16) + query_group * kDsTile + key;
 }
 
+// Entry b of DsTiles::seq_base, by one block of a pre-pass: the tiles of one head of the sequences in front of sequence b.
+__device__ __forceinline__ void write_seq_base(int32_t* seq_base, const int32_t* cu_q, const int32_t* cu_k, int b, bool causal) {
+  __shared__ int tiles_before;
+  if (threadIdx.x == 0) tiles_before = 0;
+  __syncthreads();
+  int mine = 0;
+  for (int i = threadIdx.x; i < b; i += blockDim.x)
+    mine += static_cast<int>(ds_tiles_per_head(cu_q[i + 1] - cu_q[i], cu_k[i + 1] - cu_k[i], causal));
+  if (mine != 0) atomicAdd(&tiles_before, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) seq_base[b] = tiles_before;
+}
+
 }  // namespace sdpa_b200

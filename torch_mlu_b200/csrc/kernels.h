@@ -28,9 +28,11 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
 
 // Forward for head dims above 128 (up to 256): one CTA per 128 query rows, Q in tensor memory (d256_sm100.cu).
 int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t stream);
-// Backward for the same head dims: a pre-pass and one kernel each for dV, dK and dQ (d256_sm100.cu).
+// Backward for the same head dims: a pre-pass, a kernel for dV and dS and the GEMMs for dK and dQ, or, without room for dS, one
+// kernel each for dV, dK and dQ (d256_sm100.cu).
+size_t bwd_d256_workspace_min_bytes(const sdpa_b200_params& p);
 size_t bwd_d256_workspace_bytes(const sdpa_b200_params& p);
-int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t stream);
+int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
 // Number of SMs of the current device (cached per device), <= 0 on error.
 int sm_count();

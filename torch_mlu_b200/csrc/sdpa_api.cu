@@ -391,6 +391,17 @@ int sdpa_b200_bwd_workspace_bytes(const sdpa_b200_params* p, size_t* bytes) {
   return SDPA_B200_OK;
 }
 
+int sdpa_b200_bwd_workspace_least_bytes(const sdpa_b200_params* p, size_t* bytes) {
+  if (bytes == nullptr) {
+    set_error("bytes is NULL");
+    return SDPA_B200_INVALID_ARG;
+  }
+  int st = validate_common(p);
+  if (st != SDPA_B200_OK) return st;
+  *bytes = kWorkspaceHeaderBytes + (p->head_dim > 128 ? bwd_d256_workspace_min_bytes(*p) : bwd_workspace_min_bytes(*p));
+  return SDPA_B200_OK;
+}
+
 int sdpa_b200_fwd(const sdpa_b200_params* p, void* workspace, size_t workspace_bytes, void* stream) {
   int st = validate_common(p);
   if (st != SDPA_B200_OK) return st;
@@ -452,7 +463,8 @@ int sdpa_b200_bwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
   if ((st = check_tensor("dv", p->dv, p->dv_batch_stride, p->dv_head_stride, p->dv_row_stride, varlen, p->batch,
                          p->heads_kv)) != SDPA_B200_OK)
     return st;
-  const size_t need = kWorkspaceHeaderBytes + (p->head_dim > 128 ? bwd_d256_workspace_bytes(*p) : bwd_workspace_min_bytes(*p));
+  size_t need = 0;
+  if ((st = sdpa_b200_bwd_workspace_least_bytes(p, &need)) != SDPA_B200_OK) return st;
   st = validate_workspace(workspace, workspace_bytes, need);
   if (st != SDPA_B200_OK) return st;
   st = check_device();
@@ -462,7 +474,7 @@ int sdpa_b200_bwd(const sdpa_b200_params* p, void* workspace, size_t workspace_b
     set_error("clearing the workspace header failed: %s", cudaGetErrorString(cudaGetLastError()));
     return SDPA_B200_LAUNCH_FAILED;
   }
-  if (p->head_dim > 128) return launch_bwd_d256(*p, workspace, s);
+  if (p->head_dim > 128) return launch_bwd_d256(*p, workspace, workspace_bytes, s);
   return launch_bwd(*p, workspace, workspace_bytes, s);
 }
 

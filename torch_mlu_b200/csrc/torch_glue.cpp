@@ -173,7 +173,16 @@ void run(sdpa_b200_params& p, bool backward, const Tensor& like) {
   check_status(backward ? sdpa_b200_bwd_workspace_bytes(&p, &bytes) : sdpa_b200_fwd_workspace_bytes(&p, &bytes),
                "workspace query");
   // from torch's stream-ordered pool, and back to it at the end of this call
-  const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+  c10::DataPtr ws;
+  try {
+    ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+  } catch (const c10::OutOfMemoryError&) {
+    // the backward runs without room for dS too
+    const size_t best = bytes;
+    if (backward) check_status(sdpa_b200_bwd_workspace_least_bytes(&p, &bytes), "workspace query");
+    if (bytes >= best) throw;
+    ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+  }
   void* stream = at::cuda::getCurrentCUDAStream(like.get_device()).stream();
   check_status(backward ? sdpa_b200_bwd(&p, ws.get(), bytes, stream) : sdpa_b200_fwd(&p, ws.get(), bytes, stream),
                backward ? "sdpa_b200_bwd" : "sdpa_b200_fwd");

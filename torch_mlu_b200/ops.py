@@ -80,8 +80,9 @@ def _set_strides_thd(p: _cabi.SdpaParams, prefix: str, t: torch.Tensor) -> None:
 
 class _Workspace:
     """Per-device cache of one growing workspace buffer per stream, and of the device's status word (torch owns
-    the memory)."""
+    the memory). Larger buffers (a backward's dS) go back to torch's pool behind the call."""
 
+    _KEEP_BYTES = 256 << 20
     _bufs: dict = {}
     _status: dict = {}
 
@@ -91,7 +92,8 @@ class _Workspace:
         buf = cls._bufs.get(key)
         if buf is None or buf.numel() < nbytes:
             buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-            cls._bufs[key] = buf
+            if nbytes <= cls._KEEP_BYTES:
+                cls._bufs[key] = buf
         return buf
 
     @classmethod
@@ -111,6 +113,15 @@ def workspace_for(params: _cabi.SdpaParams, backward: bool, device: torch.device
     need = ctypes.c_size_t(0)
     fn = lib.sdpa_b200_bwd_workspace_bytes if backward else lib.sdpa_b200_fwd_workspace_bytes
     _cabi.check(fn(ctypes.byref(params), ctypes.byref(need)), "workspace query")
+    try:
+        return _Workspace.get(device, need.value)
+    except torch.cuda.OutOfMemoryError:
+        # the backward runs without room for dS too
+        best = need.value
+        if backward:
+            _cabi.check(lib.sdpa_b200_bwd_workspace_least_bytes(ctypes.byref(params), ctypes.byref(need)), "workspace query")
+        if need.value >= best:
+            raise
     return _Workspace.get(device, need.value)
 
 
