@@ -650,33 +650,38 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         // x = S c - lse2. kPolyOf4 of every four column pairs take their 2^x from the FMA pipe (exp2_poly3_x2). dQ: one; two already
-        // cost issue slots. dK/dV at head_dim 64, where a quarter of the MMAs' time hides as many exponentials: two (step of B8 H12
-        // L512 with a mask 96.3 us, without any 97.5). At 128, none: at the power cap none to two take the same time (step of B8 H16
-        // L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed 64 to 2048 tokens 369, 368, 364), and none is the most exact.
-        constexpr int kPolyOf4 = kMode == kModeDQ ? 1 : (kD == 64 ? 2 : 0);
+        // cost issue slots. dK/dV: two, which shortens the chain of an item (step of B8 H12 L512 D64 with a mask 96.3 us, without any
+        // 97.5; B1 H8 L2048 D128 78.7, 82.0) - but none where dS goes through the workspace: those grids are full and run at the power
+        // cap, where none to two take the same time (step of B8 H16 L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed
+        // 64 to 2048 tokens 369, 368, 364), and none is the most exact.
+        auto exponentials = [&](auto kPoly) {
+          constexpr int kPolyOf4 = decltype(kPoly)::value;
 #pragma unroll
-        for (int j4 = 0; j4 < 16; ++j4) {
-          const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
-          uint2 kb = make_uint2(0u, 0u);
-          if constexpr (kBias == kKeyBias && kMode == kModeDQ) kb = *reinterpret_cast<const uint2*>(key_bias_row + 2 * j4);
+          for (int j4 = 0; j4 < 16; ++j4) {
+            const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
+            uint2 kb = make_uint2(0u, 0u);
+            if constexpr (kBias == kKeyBias && kMode == kModeDQ) kb = *reinterpret_cast<const uint2*>(key_bias_row + 2 * j4);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int j = 4 * j4 + 2 * h;
-            float2 nl = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
-            if constexpr (kBias == kKeyBias)
-              nl = kMode == kModeDKDV ? add2(nl, make_float2(key_bias, key_bias))
-                                      : fma2(unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), make_float2(kLog2e, kLog2e), nl);
-            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl);
-            if (((j >> 1) & 3) < kPolyOf4) {
-              const float2 e = exp2_poly3_x2(x);
-              pr[j] = e.x;
-              pr[j + 1] = e.y;
-            } else {
-              pr[j] = ex2_approx(x.x);
-              pr[j + 1] = ex2_approx(x.y);
+            for (int h = 0; h < 2; ++h) {
+              const int j = 4 * j4 + 2 * h;
+              float2 nl = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
+              if constexpr (kBias == kKeyBias)
+                nl = kMode == kModeDKDV ? add2(nl, make_float2(key_bias, key_bias))
+                                        : fma2(unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), make_float2(kLog2e, kLog2e), nl);
+              const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl);
+              if (((j >> 1) & 3) < kPolyOf4) {
+                const float2 e = exp2_poly3_x2(x);
+                pr[j] = e.x;
+                pr[j + 1] = e.y;
+              } else {
+                pr[j] = ex2_approx(x.x);
+                pr[j + 1] = ex2_approx(x.y);
+              }
             }
           }
-        }
+        };
+        if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) exponentials(std::integral_constant<int, 0>{});
+        else exponentials(std::integral_constant<int, kMode == kModeDQ ? 1 : 2>{});
         // only tiles on the causal diagonal or past the end of the keys need the element mask
         if (__any_sync(0xffffffffu, j_lo > 0 || j_hi < 64)) {
 #pragma unroll
