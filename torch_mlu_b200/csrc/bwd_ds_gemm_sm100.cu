@@ -153,7 +153,6 @@ bwd_ds_gemm_kernel(const __grid_constant__ CUtensorMap tm_ds_q, const __grid_con
         const int size = keys ? kv_heads : kv_heads * p.kv_group;
         const int rank = w / size, pairs = keys ? p.key_pairs : p.query_pairs;
         if (rank < pairs) {  // else: padding of a short last group
-          const int pair = keys ? rank : pairs - 1 - rank;
           const int hx = w - rank * size;  // head within the group
           const int kvh = p.kv_head0 + grp * p.heads_per_group + (keys ? hx : hx / p.kv_group);  // batch * heads_kv + head
           const int b = kvh / p.heads_kv;
@@ -168,8 +167,11 @@ bwd_ds_gemm_kernel(const __grid_constant__ CUtensorMap tm_ds_q, const __grid_con
             bcoord = 0;
           }
           const int off = len_k - len_q;
-          const int row0 = pair * kPair, rows = keys ? len_k : len_q;
-          if (row0 < rows) {
+          // heaviest first: key pair 0 (of a packed sequence: by the pairs behind it), the last query pair
+          const int rows = keys ? len_k : len_q;
+          const int pair = keys ? rank - (pairs - (len_k + kPair - 1) / kPair) : pairs - 1 - rank;
+          const int row0 = pair * kPair;
+          if (row0 >= 0 && row0 < rows) {
             // steps [lo, hi) of 64 contraction rows that contribute to tile t
             int lo[2] = {0, 0}, hi[2] = {0, 0};
 #pragma unroll
@@ -476,9 +478,8 @@ int launch_bwd_ds_gemm(const sdpa_b200_params& p, const DsTiles& ds, int kv_head
   // heads per group: the rows of the B operands are re-read by every unit of their head. (With dK too, groups of 1 to 8 heads, whose
   // dS might come from L2 the second time, make no difference: B4 H16 L4096 D256 576 to 580 us.)
   const double per_head = 2.0 * p.head_dim * (p.max_seqlen_k + (with_dk ? kp.kv_group * static_cast<double>(p.max_seqlen_q) : 0.0));
-  int hpg = static_cast<int>(48.0 * 1024 * 1024 / per_head);
-  hpg = hpg < 1 ? 1 : (hpg > 32 ? 32 : hpg);
-  if (hpg > num_kv_heads) hpg = num_kv_heads;
+  const double all = 2.0 * p.head_dim * (static_cast<double>(p.total_k) * p.heads_kv + (with_dk ? static_cast<double>(p.total_q) * p.heads_q : 0.0));
+  const int hpg = varlen ? heads_per_packed_group(all, num_kv_heads) : heads_per_l2_group(per_head, num_kv_heads);
   kp.heads_per_group = hpg;
   kp.key_units_per_group = with_dk ? hpg * kp.key_pairs : 0;
   kp.units_per_group = kp.key_units_per_group + hpg * kp.kv_group * kp.query_pairs;

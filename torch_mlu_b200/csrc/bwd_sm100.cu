@@ -118,7 +118,8 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // CTA order (1-D grid): (batch, head) pairs in groups of `heads_per_wave` whose streamed tensors
   // fit L2 together; inside a group the 128-row blocks go heaviest first across all its heads
   // (dK/dV: key block 0 sees every query; dQ: the last query block sees every key), so the launch
-  // ends on its lightest blocks.
+  // ends on its lightest blocks. Packed: blocks with the same number of blocks behind (dQ: in front of) them in their own
+  // sequence count as equally heavy, so that a short sequence's first key block does not go before a long one's second.
   int b, hx, xb;
   {
     const int per_group = p.heads_per_wave * p.num_row_blocks;
@@ -142,11 +143,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
+    if (kMode == kModeDKDV) xb -= p.num_row_blocks - (len_k + kTile - 1) / kTile;
   }
   const int causal_off = len_k - len_q;
   const int len_x = (kMode == kModeDKDV) ? len_k : len_q;
   const int x0 = xb * kTile;
-  if (x0 >= len_x) {
+  if (x0 < 0 || x0 >= len_x) {
     if (kMode == kModeDQ) wait_for_previous_grid();
     return;
   }
@@ -1242,18 +1244,17 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   }
 #endif
 
-  // heads per group: streamed bytes per head (q + dO of the group, or k + v) within ~48 MB of L2
-  auto set_order = [&](int heads_x, int rows_streamed, int streams_per_head, int num_bh) {
+  // streamed: q + dO of the group, or k + v
+  auto set_order = [&](int heads_x, int rows_streamed, int streams_per_head, int num_bh, double packed_rows) {
     kp.heads_x = heads_x;
     kp.num_bh = num_bh;
-    const double bytes = 2.0 * rows_streamed * p.head_dim * 2 * streams_per_head;
-    int hpw = static_cast<int>((48.0 * 1024 * 1024) / bytes);
-    hpw = hpw < 1 ? 1 : (hpw > 32 ? 32 : hpw);
-    if (hpw > kp.num_bh) hpw = kp.num_bh;
-    kp.heads_per_wave = hpw;
-    const int groups = (kp.num_bh + hpw - 1) / hpw;
-    return groups * hpw * kp.num_row_blocks;
+    const double row_bytes = 2.0 * p.head_dim * 2;
+    kp.heads_per_wave = varlen && !fused ? heads_per_packed_group(row_bytes * packed_rows, num_bh)
+                                         : heads_per_l2_group(row_bytes * rows_streamed * streams_per_head, num_bh);
+    const int groups = (num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
+    return groups * kp.heads_per_wave * kp.num_row_blocks;
   };
+  const double rows_q_all = static_cast<double>(p.total_q) * p.heads_q, rows_k_all = static_cast<double>(p.total_k) * p.heads_kv;
   kp.num_row_blocks = (p.max_seqlen_k + kTile - 1) / kTile;
   kp.bh0 = 0;
   kp.ds.data = nullptr;
@@ -1267,7 +1268,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
       const int n = kv_heads - first < plan.kv_heads ? kv_heads - first : plan.kv_heads;
       kp.bh0 = first;
       kp.ds.head0 = first * kp.kv_group;
-      const int grid = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, n);
+      const int grid = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, n, rows_q_all);
       if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp)) !=
           SDPA_B200_OK)
         return st;
@@ -1275,13 +1276,13 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
     }
     return SDPA_B200_OK;
   }
-  const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, p.batch * p.heads_kv);
+  const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, p.batch * p.heads_kv, rows_q_all);
   if (fused) return launch_bwd_fused(p, kp, dq_acc, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk);
   if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp)) !=
       SDPA_B200_OK)
     return st;
   kp.num_row_blocks = (p.max_seqlen_q + kTile - 1) / kTile;
-  const int grid_dq = set_order(p.heads_q, p.max_seqlen_k, 1, p.batch * p.heads_q);
+  const int grid_dq = set_order(p.heads_q, p.max_seqlen_k, 1, p.batch * p.heads_q, rows_k_all);
   return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kp,
                             /*overlap_previous=*/true);
 }

@@ -598,7 +598,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
   }
 
   // CTA order as in the forward: groups of heads whose streamed tensors fit L2, heaviest row blocks first
-  // (key block 0 sees every query; the last query block sees every key)
+  // (key block 0 sees every query; the last query block sees every key; packed key blocks by the number of blocks behind them)
   int b, hx, xb;
   {
     const int per_group = p.heads_per_wave * p.num_row_blocks;
@@ -619,11 +619,12 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
+    if (kKeys) xb -= p.num_row_blocks - (len_k + kRowsA - 1) / kRowsA;
   }
   const int causal_off = len_k - len_q;
   const int len_x = kKeys ? len_k : len_q;
   const int x0 = xb * kRowsA;
-  if (x0 >= len_x) return;
+  if (x0 < 0 || x0 >= len_x) return;
   const int x_off = kKeys ? k_off : q_off;
   const int y_off = kKeys ? q_off : k_off;
 
@@ -1220,13 +1221,6 @@ __global__ void __launch_bounds__(256) bwd_d256_preprocess_kernel(const Pre256Pa
   }
 }
 
-// heads per group so that the streamed K + V of a group stay within ~48 MB of L2
-int heads_per_wave_for(double bytes_per_head, int num_bh) {
-  int hpw = static_cast<int>((48.0 * 1024 * 1024) / bytes_per_head);
-  hpw = hpw < 1 ? 1 : (hpw > 32 ? 32 : hpw);
-  return hpw > num_bh ? num_bh : hpw;
-}
-
 }  // namespace
 
 namespace {
@@ -1354,7 +1348,8 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace
     kp.num_row_blocks = ((keys ? p.max_seqlen_k : p.max_seqlen_q) + kRowsA - 1) / kRowsA;
     // bytes one stationary head streams: Q + dO of its group (keys), or K + V (queries)
     const double streamed = 2.0 * (keys ? p.max_seqlen_q : p.max_seqlen_k) * p.head_dim * 2 * (keys ? kp.kv_group : 1);
-    kp.heads_per_wave = heads_per_wave_for(streamed, kp.num_bh);
+    const double packed = 2.0 * p.head_dim * 2 * (keys ? static_cast<double>(p.total_q) * p.heads_q : static_cast<double>(p.total_k) * p.heads_kv);
+    kp.heads_per_wave = varlen ? heads_per_packed_group(packed, kp.num_bh) : heads_per_l2_group(streamed, kp.num_bh);
     const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
     const int grid = groups * kp.heads_per_wave * kp.num_row_blocks;
     kernel<<<grid, kBwdThreads, kSmemBytesBwd256, stream>>>(x2, y1, y2, out, kp);
@@ -1437,7 +1432,9 @@ int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   kp.head_dim = p.head_dim;
   kp.num_m_blocks = (p.max_seqlen_q + kRowsA - 1) / kRowsA;
   kp.num_bh = p.batch * p.heads_q;
-  kp.heads_per_wave = heads_per_wave_for(2.0 * p.max_seqlen_k * p.head_dim * 2 / kp.kv_group, kp.num_bh);
+  const double kv_row_bytes = 2.0 * p.head_dim * 2;
+  kp.heads_per_wave = heads_per_forward_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh, varlen,
+                                              kv_row_bytes * p.total_k * p.heads_kv);
   kp.scale_log2 = p.softmax_scale * 1.4426950408889634f;
   kp.is_causal = p.is_causal;
   const bool drop = p.dropout_p > 0.f;

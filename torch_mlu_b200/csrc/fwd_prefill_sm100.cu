@@ -886,14 +886,10 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   }
   kp.num_m_blocks = (p.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM);
   kp.num_bh = p.batch * p.heads_q;
-  {
-    // K+V bytes one query head streams, shared by the heads of its GQA group
-    const double kv_bytes = 2.0 * p.max_seqlen_k * p.head_dim * 2 / kp.kv_group;
-    int hpw = static_cast<int>((48.0 * 1024 * 1024) / kv_bytes);
-    hpw = hpw < 1 ? 1 : (hpw > 32 ? 32 : hpw);
-    if (hpw > kp.num_bh) hpw = kp.num_bh;
-    kp.heads_per_wave = hpw;
-  }
+  // K+V bytes one query head streams, shared by the heads of its GQA group
+  const double kv_row_bytes = 2.0 * p.head_dim * 2;
+  kp.heads_per_wave = heads_per_forward_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh, varlen,
+                                              kv_row_bytes * p.total_k * p.heads_kv);
   const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
   kp.num_slots = groups * kp.heads_per_wave * kp.num_m_blocks;
   const int sms = sm_count();

@@ -34,6 +34,28 @@ size_t bwd_d256_workspace_min_bytes(const sdpa_b200_params& p);
 size_t bwd_d256_workspace_bytes(const sdpa_b200_params& p);
 int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
+// Kernels take (batch, head) pairs in groups whose streamed tensors stay in L2 together, and the blocks of a group heaviest first.
+// Heads per group, from the bytes that one head streams (packed: at the longest length).
+inline int heads_per_l2_group(double bytes_per_head, int num_heads) {
+  int n = static_cast<int>((48.0 * 1024 * 1024) / bytes_per_head);
+  n = n > 32 ? 32 : (n < 1 ? 1 : n);
+  return n > num_heads ? num_heads : n;
+}
+
+// Packed, from what all sequences together stream: the longest one says little about it, and in fewer and larger groups fewer long
+// chains start late. The backward's groups stream 112 MB, except in the fused kernel, which also adds into its accumulator (20 sequences of
+// 100 to 3000 tokens, D64: step 1048 us by the longest, 1074 so) (dK/dV kernel of 12 sequences of 64 to 2048 tokens, 16/4 heads: 153 us in
+// five groups, the last 50 of them with idle SMs, 134 in one; step 365 -> 350, with 64 MB 360). The forward, whose dynamic units
+// leave no such tail, takes one group if K and V are at most 48 MB and otherwise goes by the longest sequence (16 sequences of 512
+// to 4096 tokens, 139 MB: 16 groups 907 us, three 921, two 929, one 958).
+inline int heads_per_packed_group(double all_bytes, int num_heads) {
+  const int groups = 1 + static_cast<int>(all_bytes / (112.0 * 1024 * 1024));
+  return (num_heads + groups - 1) / groups;
+}
+inline int heads_per_forward_group(double bytes_per_head, int num_heads, bool packed, double all_bytes) {
+  return packed && all_bytes <= 48.0 * 1024 * 1024 ? num_heads : heads_per_l2_group(bytes_per_head, num_heads);
+}
+
 // Number of SMs of the current device (cached per device), <= 0 on error.
 int sm_count();
 
