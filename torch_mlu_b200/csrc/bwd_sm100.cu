@@ -105,12 +105,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* smem = smem_raw + (base - raw_addr);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // The dQ kernel follows in the stream and depends on nothing written here: once every dK/dV CTA has begun (this
-  // signal), its CTAs may take over SMs as they free up, instead of waiting for the last dK/dV CTA to finish.
-  if (kMode == kModeDKDV && threadIdx.x == 0) {
-    if (kD > 64 && p.ds.data != nullptr && blockIdx.x == 0) *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  }
+  // dK/dV: the pre-pass in front signals at once that this grid may start, so its set-up and the first K and V loads run under the
+  // pre-pass's tail; its vectors are read behind the wait for it. The kernel behind (the dQ kernel, which depends on nothing
+  // written here, or the dQ GEMM, which waits for this grid) is let in by every CTA behind that wait, so that it too finds the
+  // vectors complete. CTAs without work wait as well: a grid must not complete before the one in front of it.
+  if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
+    *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid; here, since block 0 may be one without work
   constexpr int kStages = stages_for(kMode);
   constexpr uint32_t kSmemVec = smem_vec_off(kMode);
   constexpr uint32_t kSmemBar = smem_bar_off(kMode);
@@ -129,7 +129,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int rank = w / size;
     const int bh = p.bh0 + grp * p.heads_per_wave + (w - rank * size);
     if (rank >= p.num_row_blocks) {  // padding slots of a short last group
-      if (kMode == kModeDQ) wait_for_previous_grid();
+      wait_for_previous_grid();
       return;
     }
     xb = (kMode == kModeDKDV) ? rank : p.num_row_blocks - 1 - rank;
@@ -149,7 +149,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int len_x = (kMode == kModeDKDV) ? len_k : len_q;
   const int x0 = xb * kTile;
   if (x0 < 0 || x0 >= len_x) {
-    if (kMode == kModeDQ) wait_for_previous_grid();
+    wait_for_previous_grid();
     return;
   }
 
@@ -262,8 +262,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (kD > 64) tma_load_4d(base + kSmemX + kHalfBytes, tmx1, bar + kBarXFull, 64, x_row, hx, bcoord);
       tma_load_4d(base + kSmemX + kTileBytes, tmx2, bar + kBarXFull, 0, x_row, hx, bcoord);
       if (kD > 64) tma_load_4d(base + kSmemX + kTileBytes + kHalfBytes, tmx2, bar + kBarXFull, 64, x_row, hx, bcoord);
-      for (int idx = 0; idx < kPreloaded && idx < 2 * n_items; ++idx) load_tile(idx);
     }
+    if (kMode == kModeDKDV) {
+      wait_for_previous_grid();
+      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+    for (int idx = 0; idx < kPreloaded && idx < 2 * n_items; ++idx) load_tile(idx);
   }
   if (warp == 0) {
     __syncwarp();
@@ -487,6 +491,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     uint32_t ds_tile0 = 0, ds_per_head = 0;
     int ds_key_tiles = 0, ds_shift_rows = 0;
     if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) {
+      wait_for_previous_grid();  // DsTiles::seq_base comes from the pre-pass
       const DsHead dh = ds_head(p.ds, b, hx * p.kv_group, p.heads_q, len_q, len_k, p.is_causal != 0);
       ds_tile0 = static_cast<uint32_t>(dh.base + xb);
       ds_per_head = static_cast<uint32_t>(ds_tiles_per_head(len_q, len_k, p.is_causal != 0));
@@ -913,6 +918,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     clear_uncovered_rows(p.grads, p.heads_q);
     return;
   }
+  if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // see bwd_tile_kernel
   // heads vary fastest across the grid: with the usual [batch, row, head, dim] memory order the blocks
   // that run together then read neighbouring 256-byte pieces of the same rows
   const int h = blockIdx.x, b = blockIdx.z;
@@ -1014,9 +1020,9 @@ TileKernel pick_tile_kernel(bool drop, BiasKind bias, int head_dim, bool f16) {
 }
 
 // `overlap_previous`: launch with programmatic stream serialization, so that this grid's CTAs may start as soon as
-// every CTA of the kernel before it in the stream has begun (see the launch_dependents signal at the top of the
-// dK/dV kernel) and an SM has room. Used for the dQ kernel, which needs nothing the dK/dV kernel writes: its CTAs
-// fill the SMs the last, partly empty wave of dK/dV CTAs leaves idle.
+// every CTA of the kernel before it in the stream has signalled launch_dependents and an SM has room. Used for the dK/dV kernel
+// behind the pre-pass, and for the dQ kernel, which needs nothing the dK/dV kernel writes: its CTAs fill the SMs the last, partly
+// empty wave of dK/dV CTAs leaves idle.
 int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t stream, const CUtensorMap& tm_q,
                        const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                        const CUtensorMap& tm_o1, const CUtensorMap& tm_o2, const BwdKernelParams& kp,
@@ -1269,8 +1275,8 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
       kp.bh0 = first;
       kp.ds.head0 = first * kp.kv_group;
       const int grid = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, n, rows_q_all);
-      if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp)) !=
-          SDPA_B200_OK)
+      if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
+                                   /*overlap_previous=*/first == 0)) != SDPA_B200_OK)
         return st;
       if ((st = launch_bwd_ds_gemm(p, kp.ds, first, n, false, kp.ds_counter, kp.status, stream)) != SDPA_B200_OK) return st;
     }
@@ -1278,8 +1284,8 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   }
   const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, p.batch * p.heads_kv, rows_q_all);
   if (fused) return launch_bwd_fused(p, kp, dq_acc, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk);
-  if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp)) !=
-      SDPA_B200_OK)
+  if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
+                               /*overlap_previous=*/true)) != SDPA_B200_OK)
     return st;
   kp.num_row_blocks = (p.max_seqlen_q + kTile - 1) / kTile;
   const int grid_dq = set_order(p.heads_q, p.max_seqlen_k, 1, p.batch * p.heads_q, rows_k_all);
