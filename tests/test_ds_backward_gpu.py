@@ -100,6 +100,30 @@ def test_packed(cuda_device, native_lib, lens_q, lens_k, Hq, Hkv, D, causal):
     check(run(native_lib, p, q, k, v, dout, True, False), run(native_lib, p, q, k, v, dout, True, True), want)
 
 
+@pytest.mark.parametrize("packed", [False, True])
+def test_infinite_gradient_of_hidden_queries(cuda_device, native_lib, packed):
+    """Keys from 128 on do not see queries 0 to 63, the first half of a dS tile: an infinite dO there leaves their gradients alone."""
+    gen = torch.Generator().manual_seed(8)
+    Lq, Lk, H, D = 128, 192, 3, 256
+    q, k, v, dout = (torch.randn(1, H, n, D, generator=gen).to(cuda_device, torch.bfloat16) for n in (Lq, Lk, Lk, Lq))
+    dout[0, :, 10] = float("inf")
+    if packed:
+        q, k, v, dout = (t[0].transpose(0, 1).contiguous() for t in (q, k, v, dout))
+        cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=cuda_device) for n in (Lq, Lk))
+        args = (cu_q, cu_k, Lq, Lk, True, D ** -0.5)
+        out, lse = ops._varlen_forward(q, k, v, *args)
+        p = ops._varlen_params(q, k, v, out, lse, *args)
+    else:
+        out, lse = ops.gqa_prefill(q, k, v, is_causal=True)
+        p = ops._dense_params(q, k, v, out, lse, True, D ** -0.5)
+    for least in (False, True):
+        dq, dk, dv = run(native_lib, p, q, k, v, dout, packed, least)
+        if not packed:
+            dq, dk, dv = (t[0].transpose(0, 1) for t in (dq, dk, dv))
+        assert torch.isfinite(dk[128:]).all() and torch.isfinite(dv[128:]).all()
+        assert torch.isfinite(torch.cat((dq[:10], dq[11:]))).all()
+
+
 def test_several_passes_over_the_workspace(cuda_device, native_lib):
     """2.7 GB of dS: two passes of ten heads give the bits of two calls with ten heads each."""
     gen = torch.Generator(device=cuda_device).manual_seed(7)

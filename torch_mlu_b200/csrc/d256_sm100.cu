@@ -635,7 +635,6 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     if (p.is_causal) {
       y_lo = max(0, (x0 - causal_off) / kRowsB);  // first query block with a row >= x0 - off
       if (x0 - causal_off > len_q - 1) y_lo = y_hi;
-      else if (kMode == kDVS) y_lo &= ~1;  // a dS tile has two blocks: both are written, the hidden one with zeros
     }
   } else {
     int vis_end = len_k;
@@ -1071,6 +1070,13 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
           uint4* dst = ds_group(p.ds, tile, ((y0 & (kDsTile - 1)) >> 3) + half * 4, r);
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch) dst[ch * kDsTile] = make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+          // A dS tile has two query blocks. Where the mask hides the first one, the head starts with the second: the hidden block's
+          // half of the tile is zeros. (Streaming it would multiply its dO by zeros into dV, and a hidden infinity into NaN.)
+          if (y0 == y_lo * kRowsB && (y_lo & 1) != 0) {
+            uint4* hidden = ds_group(p.ds, tile, half * 4, r);
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch) hidden[ch * kDsTile] = make_uint4(0u, 0u, 0u, 0u);
+          }
         }
       } else {
         ok = form_ds() && w_to_smem();
