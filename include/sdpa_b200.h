@@ -157,8 +157,8 @@ typedef struct sdpa_b200_params {
   /* Backward: 0 = whichever is faster for the sizes. That may be the fused kernel (up to head_dim 64 in the main), which forms
    * every tile's scores once and adds its dQ contributions into an fp32 workspace with floating-point reductions whose
    * order varies between launches (dK and dV are still summed in a fixed order). Non-zero = only kernels with a fixed
-   * summation order throughout, so that the same call with the same workspace size gives the same bits every time. A call
-   * with a bias takes only those too. Ignored by the forward. */
+   * summation order throughout, so that the same call gives the same bits every time, with any workspace size. A call with
+   * a bias takes only those too. Ignored by the forward. */
   int32_t deterministic;
   /* Forward (tile kernel): number of SMs the persistent kernel leaves free, for a kernel that is to run beside it on
    * another stream - a collective that reassembles the previous step's outputs, say. 0 = one CTA on every SM, which

@@ -646,11 +646,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         constexpr float kLog2e = 1.4426950408889634f;
-        float key_bias = 0.f;  // dK/dV
+        float key_bias = 0.f, key_bias_log2 = 0.f;  // dK/dV
         uint32_t* key_bias_row = reinterpret_cast<uint32_t*>(smem + smem_key_bias_off(kMode) + warp * 128);  // dQ
         if constexpr (kBias == kKeyBias) {
           if (kMode == kModeDKDV) {
-            key_bias = unpack_16x2<kF16>(key_bias_raw).x * kLog2e;
+            key_bias = unpack_16x2<kF16>(key_bias_raw).x;
+            key_bias_log2 = key_bias * kLog2e;
           } else {
             key_bias_row[lane] = key_bias_raw;  // the previous item's values were read before this warp's last __syncwarp
             __syncwarp();
@@ -660,9 +661,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // cost issue slots. dK/dV: two, which shortens the chain of an item (step of B8 H12 L512 D64 with a mask 96.3 us, without any
         // 97.5; B1 H8 L2048 D128 78.7, 82.0) - but none where dS goes through the workspace: those grids are full and run at the power
         // cap, where none to two take the same time (step of B8 H16 L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed
-        // 64 to 2048 tokens 369, 368, 364), and none is the most exact.
-        auto exponentials = [&](auto kPoly) {
-          constexpr int kPolyOf4 = decltype(kPoly)::value;
+        // 64 to 2048 tokens 369, 368, 364), and none is the most exact. Such a call without room for dS takes these two kernels, and its
+        // bits must not tell: none here either, and the same roundings in both kernels (a key bias joins with one).
+        const bool ds_call = kD > 64 && p.ds_call != 0;
+        auto exponentials = [&](auto kDsCall) {
+          constexpr bool kOfDsCall = decltype(kDsCall)::value;
+          constexpr int kPolyOf4 = kOfDsCall ? 0 : kMode == kModeDQ ? 1 : 2;
 #pragma unroll
           for (int j4 = 0; j4 < 16; ++j4) {
             const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
@@ -672,9 +676,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int h = 0; h < 2; ++h) {
               const int j = 4 * j4 + 2 * h;
               float2 nl = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
-              if constexpr (kBias == kKeyBias)
-                nl = kMode == kModeDKDV ? add2(nl, make_float2(key_bias, key_bias))
-                                        : fma2(unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), make_float2(kLog2e, kLog2e), nl);
+              if constexpr (kBias == kKeyBias) {
+                const float2 kb2 = unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), log2e = make_float2(kLog2e, kLog2e);
+                nl = kMode == kModeDQ ? fma2(kb2, log2e, nl)
+                     : kOfDsCall      ? fma2(make_float2(key_bias, key_bias), log2e, nl)
+                                      : add2(nl, make_float2(key_bias_log2, key_bias_log2));
+              }
               const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl);
               if (((j >> 1) & 3) < kPolyOf4) {
                 const float2 e = exp2_poly3_x2(x);
@@ -687,8 +694,8 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
           }
         };
-        if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) exponentials(std::integral_constant<int, 0>{});
-        else exponentials(std::integral_constant<int, kMode == kModeDQ ? 1 : 2>{});
+        if (ds_call) exponentials(std::true_type{});
+        else exponentials(std::false_type{});
         // only tiles on the causal diagonal or past the end of the keys need the element mask
         if (__any_sync(0xffffffffu, j_lo > 0 || j_hi < 64)) {
 #pragma unroll
@@ -1264,6 +1271,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   kp.num_row_blocks = (p.max_seqlen_k + kTile - 1) / kTile;
   kp.bh0 = 0;
   kp.ds.data = nullptr;
+  kp.ds_call = plan.tiles > 0;
   if (through_ds) {
     kp.ds.data = reinterpret_cast<uint16_t*>(behind_vectors + ds_table_bytes(p));
     kp.ds.seq_base = pre.ds_seq_base;
