@@ -154,7 +154,7 @@ typedef struct sdpa_b200_params {
    * bias does not depend on the query (bias_row_stride == 0). NULL = not given. */
   const void* bias_t;
   int64_t bias_t_batch_stride, bias_t_head_stride, bias_t_row_stride;
-  /* Backward: 0 = whichever is faster for the sizes. That may be the fused kernel (up to head_dim 64 in the main), which forms
+  /* Backward: 0 = whichever is faster for the sizes. That may be the fused kernel (up to head_dim 64), which forms
    * every tile's scores once and adds its dQ contributions into an fp32 workspace with floating-point reductions whose
    * order varies between launches (dK and dV are still summed in a fixed order). Non-zero = only kernels with a fixed
    * summation order throughout, so that the same call gives the same bits every time, with any workspace size. A call with

@@ -147,17 +147,21 @@ def test_backward_is_deterministic(cuda_device, native_lib):
         assert torch.equal(x, y)
 
 
-@pytest.mark.parametrize("B,Hq,Hkv,L,D,dropout,bias,deterministic,fused", [
-    (1, 148, 148, 128, 128, False, False, False, False),   # as many key blocks as SMs
-    (1, 149, 149, 128, 128, False, False, False, True),
-    (1, 149, 149, 128, 128, False, False, True, False),
-    (2, 80, 40, 256, 128, False, False, False, False),     # grouped queries at head_dim 128
-    (2, 80, 40, 256, 128, True, False, False, True),
-    (2, 80, 40, 256, 64, False, False, False, True),
-    (2, 80, 80, 256, 64, False, True, False, False),
+@pytest.mark.parametrize("B,Hq,Hkv,L,D,dropout,bias,deterministic,path", [
+    (1, 148, 148, 128, 128, False, False, False, "two"),   # as many key blocks as SMs
+    (1, 149, 149, 128, 128, False, False, False, "dS"),
+    (1, 149, 149, 128, 128, False, False, True, "dS"),
+    (2, 80, 40, 256, 128, False, False, False, "dS"),      # grouped queries
+    (2, 80, 40, 256, 128, True, False, False, "dS"),
+    (2, 80, 80, 256, 80, False, True, False, "dS"),
+    (2, 80, 40, 256, 64, False, False, False, "fused"),
+    (2, 80, 40, 256, 64, True, False, False, "fused"),
+    (2, 80, 40, 256, 64, False, False, True, "two"),
+    (2, 80, 80, 256, 64, False, True, False, "two"),
+    (1, 1, 1, 128, 256, False, False, False, "dS"),
 ])
-def test_which_backward_kernels_run(cuda_device, native_lib, B, Hq, Hkv, L, D, dropout, bias, deterministic, fused):
-    """The tests of the fused kernel rely on this choice: read from the names of the kernels that ran."""
+def test_which_backward_kernels_run(cuda_device, native_lib, B, Hq, Hkv, L, D, dropout, bias, deterministic, path):
+    """The tests of one path rely on this choice: read from the names of the kernels that ran."""
     from torch.profiler import ProfilerActivity, profile
     from torch_mlu_b200.dropout import KeepMasks
     dev = cuda_device
@@ -169,7 +173,9 @@ def test_which_backward_kernels_run(cuda_device, native_lib, B, Hq, Hkv, L, D, d
         ops._dense_backward(do, q, k, v, out, lse, False, D ** -0.5, keep=keep, bias=b, deterministic=deterministic)
         torch.cuda.synchronize()
     names = " ".join(e.name for e in prof.events())
-    assert ("bwd_fused_kernel" in names, "bwd_tile_kernel" in names) == (fused, not fused), names
+    tile = "bwd_d256_kernel" if D > 128 else "bwd_tile_kernel"
+    ran = ("bwd_fused_kernel" in names, tile in names, "bwd_ds_gemm_kernel" in names)
+    assert ran == {"fused": (True, False, False), "two": (False, True, False), "dS": (False, True, True)}[path], names
 
 
 def test_config3_sampled_heads_and_linearity(cuda_device, native_lib):

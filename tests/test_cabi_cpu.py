@@ -98,6 +98,21 @@ def test_workspace_query_and_validation_codes(native_lib):
     assert st == _cabi.INVALID_ARG
 
 
+@pytest.mark.parametrize("head_dim,batch", [(128, 2), (128, 20), (80, 20), (64, 2), (64, 20)])
+def test_backward_workspace_has_an_accumulator_only_where_a_kernel_adds_into_one(native_lib, head_dim, batch):
+    """The fp32 dQ accumulator belongs to head dims up to 64. Above, a call needs its vectors; with more key blocks (heads_kv x two of
+    128) than SMs it is best given room for dS too, also where that is less than an accumulator would take."""
+    p = _valid_params()
+    p.head_dim, p.batch, p.heads_kv, p.is_causal = head_dim, batch, 8, 1
+    vectors = 2 * batch * 8 * 256 * 4
+    accumulator = batch * 8 * 256 * 64 * 4 if head_dim <= 64 else 0
+    dS = batch * 8 * 3 * 128 * 128 * 2 if head_dim > 64 and batch * 8 * 2 > 148 else 0  # three of four tiles are visible
+    least = ctypes.c_size_t(0)
+    assert native_lib.sdpa_b200_bwd_workspace_least_bytes(ctypes.byref(p), ctypes.byref(least)) == _cabi.OK
+    assert least.value - 256 == vectors + accumulator
+    assert _ws_bytes(native_lib, p, bwd=True)[1] - 256 == vectors + max(accumulator, dS)
+
+
 def test_decode_workspace_grows_with_splits(native_lib):
     p = _valid_params()
     p.max_seqlen_q, p.max_seqlen_k, p.kernel = 1, 32768, _cabi.KERNEL_DECODE

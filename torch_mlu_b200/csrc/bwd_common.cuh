@@ -49,7 +49,7 @@ struct BwdKernelParams {
   uint16_t* dbias;  // or null
   int64_t dbias_batch_stride, dbias_head_stride, dbias_row_stride;
   float inv_scale;  // 1 / softmax_scale
-  // fused kernel: fp32 dQ accumulator, 128-row tiles of [head_dim / 4][128 rows][4] floats (a warp's 32 rows of one
+  // fused kernel: fp32 dQ accumulator, 128-row tiles of [16 column groups][128 rows][4] floats (a warp's 32 rows of one
   // 4-column group are 512 contiguous bytes). Row index: dense (batch * heads_q + head) * lq_pad + query, packed
   // head * dq_acc_rows + token.
   float* dq_acc;

@@ -39,6 +39,7 @@ namespace {
 #define SDPA_BWD_POLY_FUSED 2  // of every 4 column pairs, how many take 2^x from the FMA pipe (see exp2_poly3_x2)
 #endif
 
+constexpr int kD = 64;  // head_dim, rounded up
 constexpr int kFThreads = 512;  // warps 0-3 / 4-7 compute, 8 TMA, 9 score GEMMs, 10 accumulation GEMMs, 11 idle, 12-15 dQ reduce
 // Register hand-over (setmaxnreg): compiled for 65536 / 512 = 128 registers per thread; the compute and reduce warpgroups
 // grow, the fourth (producer, issuers) shrinks. The increase waits - without a time limit - until the pool holds enough registers, so what
@@ -88,24 +89,24 @@ constexpr uint32_t kFSmemAbort = 132;
 #define FSTAMP(role, item, ev) do {} while (0)
 #endif
 
-template <int kD, bool kF16>
+template <bool kF16>
 constexpr uint32_t kIdescDQ = umma_idesc_16(kTile, kD, true, true, kF16);  // A = dS (MN-major), B = K (MN-major)
 
 // dQ_tile[q][d] = sum_key dS[q][key] K[key][d]. The dS tile is stored [key][query]: the query index is the contiguous
 // one, i.e. the tile is an MN-major A operand (64-query chunks kHalfBytes apart); 16 keys are 2048 bytes in both tiles.
-template <int kD, bool kF16>
+template <bool kF16>
 __device__ __forceinline__ void issue_dq(uint32_t t, uint32_t ds_smem, uint32_t k_smem) {
   const uint32_t a_lo = umma_desc_lo_mnmajor(ds_smem, kHalfBytes);
   const uint32_t b_lo = umma_desc_lo_mnmajor(k_smem, kHalfBytes);
-  umma_ss_lo<kIdescDQ<kD, kF16>, false>(t, a_lo, b_lo);
+  umma_ss_lo<kIdescDQ<kF16>, false>(t, a_lo, b_lo);
 #pragma unroll
   for (int ks = 1; ks < kTile / 16; ++ks)
-    umma_ss_lo<kIdescDQ<kD, kF16>, true>(t, a_lo + ks * (2048 >> 4), b_lo + ks * (2048 >> 4));
+    umma_ss_lo<kIdescDQ<kF16>, true>(t, a_lo + ks * (2048 >> 4), b_lo + ks * (2048 >> 4));
 }
 
 // dK[key][d] += sum_q dS^T[key][q] Q[q][d]: the same dS tile as a K-major A operand (the contraction index, the query,
 // is contiguous: 16 queries are 32 bytes inside a 64-query half), Q as MN-major B.
-template <int kD, bool kF16>
+template <bool kF16>
 __device__ __forceinline__ void issue_dk(uint32_t acc, uint32_t ds_smem, uint32_t q_smem, bool accumulate) {
   const uint32_t a_lo = umma_desc_lo_kmajor(ds_smem);
   const uint32_t b_lo = umma_desc_lo_mnmajor(q_smem, kHalfBytes);
@@ -118,12 +119,11 @@ __device__ __forceinline__ void issue_dk(uint32_t acc, uint32_t ds_smem, uint32_
 
 // Index of the first float of `row` in the tiled fp32 dQ accumulator (see BwdKernelParams::dq_acc); the row's 4-column
 // group g is 512 * g floats further on.
-template <int kD>
 __device__ __forceinline__ size_t dq_acc_index(size_t row) {
   return (row >> 7) * (static_cast<size_t>(kD / 4) * 512) + (row & 127) * 4;
 }
 
-template <int kD, bool kF16, bool kDrop>
+template <bool kF16, bool kDrop>
 __global__ void __launch_bounds__(kFThreads, 1)
 bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -210,7 +210,6 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     const CUtensorMap* tm = first ? &tm_q : &tm_do;
     tma_load_4d(dst, tm, full, 0, row, hy, bcoord);
-    if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, full, 64, row, hy, bcoord);
     return true;
   };
 
@@ -238,9 +237,7 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int x_row = k_off + x0;
       mbar_arrive_expect_tx(bar + kFBarXFull, 2 * kLoadBytes);
       tma_load_4d(base + kFSmemX, &tm_k, bar + kFBarXFull, 0, x_row, hx, bcoord);
-      if (kD > 64) tma_load_4d(base + kFSmemX + kHalfBytes, &tm_k, bar + kFBarXFull, 64, x_row, hx, bcoord);
       tma_load_4d(base + kFSmemX + kTileBytes, &tm_v, bar + kFBarXFull, 0, x_row, hx, bcoord);
-      if (kD > 64) tma_load_4d(base + kFSmemX + kTileBytes + kHalfBytes, &tm_v, bar + kFBarXFull, 64, x_row, hx, bcoord);
       for (int idx = 0; idx < kPreloaded && idx < 2 * n_items; ++idx) load_tile(idx);
     }
   }
@@ -274,7 +271,7 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int qrow = yt * kTile + r;
       const size_t row = (p.cu_q != nullptr) ? static_cast<size_t>(hy) * p.dq_acc_rows + q_off + qrow
                                              : (static_cast<size_t>(b) * p.heads_q + hy) * p.lq_pad + qrow;
-      float* dst = p.dq_acc + dq_acc_index<kD>(row);
+      float* dst = p.dq_acc + dq_acc_index(row);
       const bool valid = qrow < len_q;
       FSTAMP(4, i, 0);
       ok = __all_sync(0xffffffffu, mbar_wait(bar + kFBarQFull, i & 1, abort_flag));
@@ -376,10 +373,10 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           FSTAMP(3, i, 3);
           tc_fence_after_sync();
           // dQ first: its read-out by the reduce warps then runs under the dK GEMM
-          issue_dq<kD, kF16>(sb, ds_smem, k_smem);
+          issue_dq<kF16>(sb, ds_smem, k_smem);
           umma_commit(bar + kFBarQFull);
           FSTAMP(3, i, 4);
-          issue_dk<kD, kF16>(acc_dk, ds_smem, y_q, i > 0);
+          issue_dk<kF16>(acc_dk, ds_smem, y_q, i > 0);
           umma_commit(bar + kFBarYEmpty + 8 * (s0 >> 1));  // Q(i), dO(i) and the dS tile may be overwritten
           if (i == n_items - 1) umma_commit(bar + kFBarAccFull);
           FSTAMP(3, i, 5);
@@ -629,7 +626,7 @@ struct DqConvertParams {
   float scale;
 };
 
-template <int kD, bool kF16>
+template <bool kF16>
 __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const DqConvertParams p) {
   const int r = threadIdx.x & 127;
   const int part = threadIdx.x >> 7;  // 0 / 1: first or second half of the 4-column groups
@@ -673,9 +670,8 @@ using FusedKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtenso
                              const CUtensorMap, const BwdKernelParams);
 
 template <bool kDrop>
-FusedKernel pick_fused(int head_dim, bool f16) {
-  if (head_dim <= 64) return f16 ? bwd_fused_kernel<64, true, kDrop> : bwd_fused_kernel<64, false, kDrop>;
-  return f16 ? bwd_fused_kernel<128, true, kDrop> : bwd_fused_kernel<128, false, kDrop>;
+FusedKernel pick_fused(bool f16) {
+  return f16 ? bwd_fused_kernel<true, kDrop> : bwd_fused_kernel<false, kDrop>;
 }
 
 }  // namespace
@@ -687,19 +683,17 @@ size_t bwd_fused_acc_rows(const sdpa_b200_params& p, int lq_pad) {
 }
 
 size_t bwd_fused_workspace_bytes(const sdpa_b200_params& p, int lq_pad) {
-  const int kd = p.head_dim <= 64 ? 64 : 128;
-  return bwd_fused_acc_rows(p, lq_pad) * kd * sizeof(float);
+  return bwd_fused_acc_rows(p, lq_pad) * kD * sizeof(float);
 }
 
 int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_acc, int grid, cudaStream_t stream,
                      const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                      const CUtensorMap& tm_dv, const CUtensorMap& tm_dk) {
   const bool f16 = p.dtype == SDPA_B200_F16;
-  const int kd = p.head_dim <= 64 ? 64 : 128;
   const size_t acc_rows = bwd_fused_acc_rows(p, kp.lq_pad);
   kp.dq_acc = dq_acc;
   kp.dq_acc_rows = p.cu_seqlens_q != nullptr ? static_cast<int>(acc_rows / p.heads_q) : 0;
-  FusedKernel kernel = kp.keep_cols != nullptr ? pick_fused<true>(p.head_dim, f16) : pick_fused<false>(p.head_dim, f16);
+  FusedKernel kernel = kp.keep_cols != nullptr ? pick_fused<true>(f16) : pick_fused<false>(f16);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmemRequest);
   if (err != cudaSuccess) {
     set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", kFSmemRequest, cudaGetErrorString(err));
@@ -728,13 +722,8 @@ int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_ac
   cp.head_dim = p.head_dim;
   cp.scale = p.softmax_scale;
   const unsigned tiles = static_cast<unsigned>(acc_rows / kTile);
-  if (kd == 64) {
-    if (f16) bwd_dq_convert_kernel<64, true><<<tiles, 256, 0, stream>>>(cp);
-    else bwd_dq_convert_kernel<64, false><<<tiles, 256, 0, stream>>>(cp);
-  } else {
-    if (f16) bwd_dq_convert_kernel<128, true><<<tiles, 256, 0, stream>>>(cp);
-    else bwd_dq_convert_kernel<128, false><<<tiles, 256, 0, stream>>>(cp);
-  }
+  if (f16) bwd_dq_convert_kernel<true><<<tiles, 256, 0, stream>>>(cp);
+  else bwd_dq_convert_kernel<false><<<tiles, 256, 0, stream>>>(cp);
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("backward dQ conversion: launch failed: %s", cudaGetErrorString(err));

@@ -945,7 +945,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   if (p.dq_acc != nullptr) {
     // 64 rows of an accumulator tile: per 4-column group 1 KB of consecutive floats, a thread per row. The stores need no
     // registers and go out under the loads below: one launch instead of two and 45 us instead of 58 at 64 K rows of 128
-    const int groups = p.head_dim <= 64 ? 16 : 32;
+    constexpr int groups = 16;
     const int row = blockIdx.y * kPreRows + (threadIdx.x & (kPreRows - 1));
     if (row < len_q) {
       const size_t acc_row = kPacked ? static_cast<size_t>(h) * p.dq_acc_rows + q_off + row
@@ -1084,9 +1084,8 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 //  * head_dim 65 to 128, more key blocks: dS through the workspace and a GEMM for dQ (use_ds_backward). One pass over the scores where
 //    the two kernels make two, and no reductions. (Step of B8 H16 L2048 695, two kernels 757, fused 752; with dropout 875, 940, 925;
 //    B2 H16 L8192 2115, 2295, 2290; B16 H32 L512 310, 365, 360; D80 B8 H16 L2048 alone 438, 533, 545; grouped B8 H32/8 L2048 alone
-//    860, 1100, 1130, B16 H16/4 L700 165, 208, 206; B3 H50 L128, the smallest of these grids, 28.8, 28.8, 32.8.)
-//    Short sequences that fill the SMs about once (up to 160 key blocks of at most two tiles) stay with the fused kernel, or, grouped
-//    and without dropout, the two: nothing but launches shows in a step there (B3 H50 L128 77.3 each way).
+//    860, 1100, 1130, B16 H16/4 L700 165, 208, 206.) The smallest of these grids, replayed from a graph: B3 H50 L128 alone 23.1, 22.3,
+//    27.0, B2 H80 L256 45.3, 46.0, 53.8, grouped B2 H80/40 L256 41.1, 42.9, 43.0, with dropout 45.7, 47.3, 58.3.
 // A packed call counts the key blocks of its grid, every sequence at the longest length, whether they have keys or not. The number
 // of SMs is the B200's, not the current device's: workspace queries and launches must agree.
 int64_t key_blocks(const sdpa_b200_params& p) {
@@ -1095,14 +1094,11 @@ int64_t key_blocks(const sdpa_b200_params& p) {
 constexpr int64_t kSms = 148;
 
 bool use_ds_backward(const sdpa_b200_params& p) {
-  if (p.head_dim <= 64 || p.dbias != nullptr || key_blocks(p) <= kSms) return false;
-  const bool one_round = key_blocks(p) <= 160 && p.max_seqlen_q <= 2 * kTile && p.max_seqlen_k <= 2 * kTile;
-  return !one_round;
+  return p.head_dim > 64 && p.dbias == nullptr && key_blocks(p) > kSms;
 }
 
 bool use_fused_backward(const sdpa_b200_params& p) {
-  if (p.deterministic != 0 || p.bias != nullptr || key_blocks(p) <= kSms) return false;
-  return p.head_dim <= 64 || (!use_ds_backward(p) && (p.heads_q == p.heads_kv || p.dropout_p > 0.f));
+  return p.head_dim <= 64 && p.deterministic == 0 && p.bias == nullptr && key_blocks(p) > kSms;
 }
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
@@ -1110,10 +1106,10 @@ size_t bwd_vector_bytes(const sdpa_b200_params& p) {
   return (bytes + 255) / 256 * 256;
 }
 
-// What a call needs: lse2 and delta, then the fp32 dQ accumulator of the fused kernel: for every call without a bias that does not ask
-// for a fixed order, whatever path its sizes take, so that one workspace serves calls that differ in dropout or sizes.
+// What a call needs: lse2 and delta, then the fp32 dQ accumulator of the fused kernel: for every call up to head_dim 64 without a bias
+// that does not ask for a fixed order, whatever path its sizes take, so that one workspace serves calls that differ in sizes.
 size_t bwd_workspace_min_bytes(const sdpa_b200_params& p) {
-  const bool acc = p.deterministic == 0 && p.bias == nullptr;
+  const bool acc = p.head_dim <= 64 && p.deterministic == 0 && p.bias == nullptr;
   return bwd_vector_bytes(p) + (acc ? bwd_fused_workspace_bytes(p, lq_padded(p)) : 0);
 }
 
@@ -1190,10 +1186,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   if ((st = make_tensor_map_16(f16, &tm_do, p.dout, p.head_dim, rows_q, p.heads_q, nb, p.do_row_stride,
                                  p.do_head_stride, p.do_batch_stride, kTile)) != SDPA_B200_OK)
     return st;
-  CUtensorMap tm_dq, tm_dk, tm_dv;  // outputs, stored tile by tile from the epilogue's staging buffers
-  if ((st = make_tensor_map_16(f16, &tm_dq, p.dq, p.head_dim, rows_q, p.heads_q, nb, p.dq_row_stride, p.dq_head_stride,
-                                 p.dq_batch_stride, kTile)) != SDPA_B200_OK)
-    return st;
+  CUtensorMap tm_dk, tm_dv;  // outputs, stored tile by tile from the epilogue's staging buffers
   if ((st = make_tensor_map_16(f16, &tm_dk, p.dk, p.head_dim, rows_k, p.heads_kv, nb, p.dk_row_stride, p.dk_head_stride,
                                  p.dk_batch_stride, kTile)) != SDPA_B200_OK)
     return st;
@@ -1292,6 +1285,10 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   }
   const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, p.batch * p.heads_kv, rows_q_all);
   if (fused) return launch_bwd_fused(p, kp, dq_acc, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk);
+  CUtensorMap tm_dq;
+  if ((st = make_tensor_map_16(f16, &tm_dq, p.dq, p.head_dim, rows_q, p.heads_q, nb, p.dq_row_stride, p.dq_head_stride,
+                                 p.dq_batch_stride, kTile)) != SDPA_B200_OK)
+    return st;
   if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
                                /*overlap_previous=*/true)) != SDPA_B200_OK)
     return st;
