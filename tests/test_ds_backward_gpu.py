@@ -156,6 +156,48 @@ def test_infinite_gradient_of_hidden_queries(cuda_device, native_lib, packed):
         assert torch.isfinite(torch.cat((dq[:10], dq[11:]))).all()
 
 
+@pytest.mark.parametrize("native", [True, False])
+def test_short_of_memory(cuda_device, native_lib, native):
+    """178 MB of dS where torch may have 128 more: the same bits, and its pool, which empties its cache before it refuses, is asked once."""
+    dev = cuda_device
+    gen = torch.Generator(device=dev).manual_seed(10)
+    q, k, v, dout = (torch.randn(1, 40, 2048, 128, generator=gen, device=dev, dtype=torch.bfloat16) for _ in range(4))
+    out, lse = ops.gqa_prefill(q, k, v, is_causal=True)
+
+    def backward():
+        if native:
+            return ops._dense_backward(dout, q, k, v, out, lse, True, 128 ** -0.5)
+        grads = [torch.empty_like(t) for t in (q, k, v)]
+        p = ops._dense_params(q, k, v, out, lse, True, 128 ** -0.5)
+        set_bwd(p, dout, *grads, packed=False)
+        ops._run_bwd(p, dev)
+        return grads
+
+    want = backward()
+    ops._Workspace._bufs.clear()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    ooms = lambda: torch.cuda.memory_stats(dev)["num_ooms"]
+    before = ooms()
+    total = torch.cuda.get_device_properties(dev).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(dev) + (128 << 20)) / total, dev)
+    try:
+        for _ in range(3):
+            for a, b in zip(backward(), want):
+                assert torch.equal(a, b)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, dev)
+    assert ooms() == before + 1
+    # a thousand such calls later there is room, and it is used again
+    for _ in range(1000 - 2 - 1):
+        backward()
+    torch.cuda.synchronize()
+    for room in (False, True):
+        torch.cuda.reset_peak_memory_stats(dev)
+        used = torch.cuda.memory_allocated(dev)
+        backward()
+        assert (torch.cuda.max_memory_allocated(dev) - used > (178 << 20)) == room
+
 def test_several_passes_over_the_workspace(cuda_device, native_lib):
     """2.7 GB of dS: two passes of ten heads give the bits of two calls with ten heads each."""
     gen = torch.Generator(device=cuda_device).manual_seed(7)

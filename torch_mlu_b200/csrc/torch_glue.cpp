@@ -20,6 +20,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
+#include <atomic>
 #include <cmath>
 #include <memory>
 #include <mutex>
@@ -167,20 +168,36 @@ int64_t device_status(int64_t device) {
   return st;
 }
 
+// A backward runs without room for dS too, with the same bits. Before torch's pool refuses such room it returns its cached blocks and waits
+// for the device, so it is not asked for as much again for the next thousand of these calls. By device, shared by all threads.
+struct Refusal {
+  std::atomic<size_t> bytes{0};
+  std::atomic<int> calls{0};
+  bool take(size_t wanted) { return calls.load() > 0 && wanted >= bytes.load() && calls.fetch_sub(1) > 0; }
+  void note(size_t wanted) {
+    bytes = wanted;
+    calls = 1000;
+  }
+};
+Refusal refusals[64];  // status_word() checks the index
+
 void run(sdpa_b200_params& p, bool backward, const Tensor& like) {
   p.device_status = reinterpret_cast<uint32_t*>(status_word(like.get_device()).data_ptr());
-  size_t bytes = 0;
+  size_t bytes = 0, least = 0;
   check_status(backward ? sdpa_b200_bwd_workspace_bytes(&p, &bytes) : sdpa_b200_fwd_workspace_bytes(&p, &bytes),
                "workspace query");
+  least = bytes;
+  if (backward) check_status(sdpa_b200_bwd_workspace_least_bytes(&p, &least), "workspace query");
   // from torch's stream-ordered pool, and back to it at the end of this call
+  Refusal& refusal = refusals[like.get_device()];
   c10::DataPtr ws;
+  if (least < bytes && refusal.take(bytes)) bytes = least;
   try {
     ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
   } catch (const c10::OutOfMemoryError&) {
-    // the backward runs without room for dS too
-    const size_t best = bytes;
-    if (backward) check_status(sdpa_b200_bwd_workspace_least_bytes(&p, &bytes), "workspace query");
-    if (bytes >= best) throw;
+    if (bytes <= least) throw;
+    refusal.note(bytes);
+    bytes = least;
     ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
   }
   void* stream = at::cuda::getCurrentCUDAStream(like.get_device()).stream();

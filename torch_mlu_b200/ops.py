@@ -85,6 +85,17 @@ class _Workspace:
     _KEEP_BYTES = 256 << 20
     _bufs: dict = {}
     _status: dict = {}
+    # device -> [bytes, calls]: a backward runs without room for dS too, with the same bits. Before torch's pool refuses such room it returns
+    # its cached blocks and waits for the device, so it is not asked for as much again for so many of these calls
+    _refused: dict = {}
+
+    @classmethod
+    def was_refused(cls, device: torch.device, nbytes: int) -> bool:
+        refused = cls._refused.get(device.index)
+        if refused is None or refused[1] <= 0 or nbytes < refused[0]:
+            return False
+        refused[1] -= 1
+        return True
 
     @classmethod
     def get(cls, device: torch.device, nbytes: int) -> torch.Tensor:
@@ -113,16 +124,18 @@ def workspace_for(params: _cabi.SdpaParams, backward: bool, device: torch.device
     need = ctypes.c_size_t(0)
     fn = lib.sdpa_b200_bwd_workspace_bytes if backward else lib.sdpa_b200_fwd_workspace_bytes
     _cabi.check(fn(ctypes.byref(params), ctypes.byref(need)), "workspace query")
+    least = ctypes.c_size_t(need.value)
+    if backward:
+        _cabi.check(lib.sdpa_b200_bwd_workspace_least_bytes(ctypes.byref(params), ctypes.byref(least)), "workspace query")
+    if least.value < need.value and _Workspace.was_refused(device, need.value):
+        return _Workspace.get(device, least.value)
     try:
         return _Workspace.get(device, need.value)
     except torch.cuda.OutOfMemoryError:
-        # the backward runs without room for dS too
-        best = need.value
-        if backward:
-            _cabi.check(lib.sdpa_b200_bwd_workspace_least_bytes(ctypes.byref(params), ctypes.byref(need)), "workspace query")
-        if need.value >= best:
+        if least.value >= need.value:
             raise
-    return _Workspace.get(device, need.value)
+    _Workspace._refused[device.index] = [need.value, 1000]
+    return _Workspace.get(device, least.value)
 
 
 def _run(p: _cabi.SdpaParams, device: torch.device, backward: bool) -> None:
