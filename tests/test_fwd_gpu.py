@@ -15,6 +15,20 @@ from torch_mlu_b200 import _cabi, ops, workloads
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("B,H,Lq,counter", [(4, 32, 256, False), (5, 32, 256, True), (1, 149, 100, True)])
+def test_units_are_claimed_from_a_counter_where_there_are_more_than_sms(cuda_device, native_lib, B, H, Lq, counter):
+    """A CTA that starts late, because another stream's kernel holds its SM, must leave its units to the others. Read from the clearing of
+    the counter."""
+    from torch.profiler import ProfilerActivity, profile
+    q, k, v = (torch.randn(B, H, Lq, 64, device=cuda_device, dtype=torch.bfloat16) for _ in range(3))
+    ops.gqa_prefill(q, k, v)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        ops.gqa_prefill(q, k, v)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    assert any("fwd_prefill_kernel" in n for n in names) and any("Memset" in n for n in names) == counter, names
+
+
 def run_dense(dev, q, k, v, causal, scale=None):
     out, lse = ops.gqa_prefill(q.to(dev), k.to(dev), v.to(dev), is_causal=causal, scale=scale)
     assert ops.device_status() == 0

@@ -87,7 +87,7 @@ struct FwdKernelParams {
   const int32_t* cu_q;
   const int32_t* cu_k;
   uint32_t* status;
-  uint32_t* unit_counter;  // zeroed before the launch, or null: CTA i of n takes the slots i and 2 n - 1 - i
+  uint32_t* unit_counter;  // zeroed before the launch, or null: every CTA takes the one slot of its own index
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int seqlen_q, seqlen_k, total_q, heads_q, kv_group;
   int head_dim;  // <= kD: the real row length, for the paths that write rows without TMA
@@ -469,7 +469,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
         bool lazy = false;
         bool last_runs = false;  // the unit published last has key blocks (and so a Q-free phase)
         uint32_t ucnt = 0;       // such units published so far
-        int own = 0;             // without a counter: the CTA's own slots that have been taken
+        bool own_taken = false;  // without a counter: the CTA's own slot has been claimed
         for (uint32_t n = 0; ok; ++n) {
           const uint32_t e = n % kUnitRing;
           ok = mbar_wait(bar + kBarUnitEmpty + 8 * e, ((n / kUnitRing) & 1u) ^ 1u, abort_flag);
@@ -479,12 +479,11 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           u.done = 1;
           for (;;) {
             const int slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
-                             : own == 0                ? static_cast<int>(blockIdx.x)
-                             : own == 1                ? 2 * static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)
-                                                       : p.num_slots;
-            ++own;
+                             : own_taken               ? p.num_slots
+                                                       : static_cast<int>(blockIdx.x);
+            own_taken = true;
             if (slot >= p.num_slots) break;
-            if (p.unit_counter != nullptr && slot >= p.num_slots - 2 * static_cast<int>(gridDim.x)) lazy = true;
+            if (slot >= p.num_slots - 2 * static_cast<int>(gridDim.x)) lazy = true;
             if (decode_unit(p, slot, u)) break;  // padding slots and row-less units are skipped
             u.done = 1;
           }
@@ -901,12 +900,14 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   // one persistent CTA per SM (shared memory and TMEM allow no second one), less the SMs the caller wants left free
   const int usable = sms - p.sm_margin > 1 ? sms - p.sm_margin : 1;
   dim3 grid(kp.num_slots < usable ? kp.num_slots : usable, 1, 1);
-  // The unit counter is workspace header word 1. Where every slot has a CTA of its own, or every CTA at most two and all units are
-  // alike, there is nothing to count, and the launch that clears the counter, about two microseconds, is left out (B4 H16 L700 D64
-  // unmasked 31.6 -> 30.7 us). Not for causal units: B2 H32/8 L1000 D128 32.5 us with a counter, 40.1 without. (Without a
-  // device_status the header has been cleared already.)
+  // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
+  // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
+  // cleared already.) Not for two units per CTA, dealt out by index: alone that is faster (B8 H12 L512 D64 unmasked, eager, 22.6 us against
+  // 24.6), but a CTA whose SM another stream's kernel holds then starts both its units late (beside a call on 8 SMs 32.9 us against 24.6,
+  // B5 H8 L1024 D128 57.4 against 41.0), and units are not alike where the last one of a head has a single tile (B8 H12 L300 D128 24.6
+  // against 23.0).
   kp.unit_counter = nullptr;
-  if (kp.num_slots > (varlen || p.is_causal ? usable : 2 * usable)) {
+  if (kp.num_slots > usable) {
     kp.unit_counter = static_cast<uint32_t*>(workspace) + 1;
     if (p.device_status != nullptr && (err = cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, stream)) != cudaSuccess) {
       set_error("prefill: clearing the unit counter failed: %s", cudaGetErrorString(err));
