@@ -118,7 +118,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // CTA order (1-D grid): (batch, head) pairs in groups of `heads_per_wave` whose streamed tensors
   // fit L2 together; inside a group the 128-row blocks go heaviest first across all its heads
   // (dK/dV: key block 0 sees every query; dQ: the last query block sees every key), so the launch
-  // ends on its lightest blocks. Packed: blocks with the same number of blocks behind (dQ: in front of) them in their own
+  // ends on its lightest blocks. Packed, causal: blocks with the same number of blocks behind (dQ: in front of) them in their own
   // sequence count as equally heavy, so that a short sequence's first key block does not go before a long one's second.
   int b, hx, xb;
   {
@@ -143,7 +143,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
-    if (kMode == kModeDKDV) xb -= p.num_row_blocks - (len_k + kTile - 1) / kTile;
+    if (kMode == kModeDKDV && p.is_causal) xb -= p.num_row_blocks - (len_k + kTile - 1) / kTile;
   }
   const int causal_off = len_k - len_q;
   const int len_x = (kMode == kModeDKDV) ? len_k : len_q;
@@ -1255,8 +1255,8 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
     kp.heads_x = heads_x;
     kp.num_bh = num_bh;
     const double row_bytes = 2.0 * p.head_dim * 2;
-    kp.heads_per_wave = varlen && !fused ? heads_per_packed_group(row_bytes * packed_rows, num_bh)
-                                         : heads_per_l2_group(row_bytes * rows_streamed * streams_per_head, num_bh);
+    kp.heads_per_wave = varlen && !fused && p.is_causal ? heads_per_packed_group(row_bytes * packed_rows, num_bh)
+                                                        : heads_per_l2_group(row_bytes * rows_streamed * streams_per_head, num_bh);
     const int groups = (num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
     return groups * kp.heads_per_wave * kp.num_row_blocks;
   };

@@ -598,7 +598,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
   }
 
   // CTA order as in the forward: groups of heads whose streamed tensors fit L2, heaviest row blocks first
-  // (key block 0 sees every query; the last query block sees every key; packed key blocks by the number of blocks behind them)
+  // (key block 0 sees every query; the last query block sees every key; under a mask packed key blocks by the number of blocks behind them)
   int b, hx, xb;
   {
     const int per_group = p.heads_per_wave * p.num_row_blocks;
@@ -619,7 +619,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
-    if (kKeys) xb -= p.num_row_blocks - (len_k + kRowsA - 1) / kRowsA;
+    if (kKeys && p.is_causal) xb -= p.num_row_blocks - (len_k + kRowsA - 1) / kRowsA;
   }
   const int causal_off = len_k - len_q;
   const int len_x = kKeys ? len_k : len_q;
@@ -1355,7 +1355,7 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace
     // bytes one stationary head streams: Q + dO of its group (keys), or K + V (queries)
     const double streamed = 2.0 * (keys ? p.max_seqlen_q : p.max_seqlen_k) * p.head_dim * 2 * (keys ? kp.kv_group : 1);
     const double packed = 2.0 * p.head_dim * 2 * (keys ? static_cast<double>(p.total_q) * p.heads_q : static_cast<double>(p.total_k) * p.heads_kv);
-    kp.heads_per_wave = varlen ? heads_per_packed_group(packed, kp.num_bh) : heads_per_l2_group(streamed, kp.num_bh);
+    kp.heads_per_wave = varlen && p.is_causal ? heads_per_packed_group(packed, kp.num_bh) : heads_per_l2_group(streamed, kp.num_bh);
     const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
     const int grid = groups * kp.heads_per_wave * kp.num_row_blocks;
     kernel<<<grid, kBwdThreads, kSmemBytesBwd256, stream>>>(x2, y1, y2, out, kp);
@@ -1439,8 +1439,9 @@ int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   kp.num_m_blocks = (p.max_seqlen_q + kRowsA - 1) / kRowsA;
   kp.num_bh = p.batch * p.heads_q;
   const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  kp.heads_per_wave = heads_per_forward_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh, varlen,
-                                              kv_row_bytes * p.total_k * p.heads_kv);
+  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q)
+                          ? kp.num_bh
+                          : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
   kp.scale_log2 = p.softmax_scale * 1.4426950408889634f;
   kp.is_causal = p.is_causal;
   const bool drop = p.dropout_p > 0.f;

@@ -888,8 +888,9 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.num_bh = p.batch * p.heads_q;
   // K+V bytes one query head streams, shared by the heads of its GQA group
   const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  kp.heads_per_wave = heads_per_forward_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh, varlen,
-                                              kv_row_bytes * p.total_k * p.heads_kv);
+  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q)
+                          ? kp.num_bh
+                          : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
   const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
   kp.num_slots = groups * kp.heads_per_wave * kp.num_m_blocks;
   const int sms = sm_count();

@@ -42,18 +42,25 @@ inline int heads_per_l2_group(double bytes_per_head, int num_heads) {
   return n > num_heads ? num_heads : n;
 }
 
-// Packed, from what all sequences together stream: the longest one says little about it, and in fewer and larger groups fewer long
-// chains start late. The backward's groups stream 112 MB, except in the fused kernel, which also adds into its accumulator (20 sequences of
-// 100 to 3000 tokens, D64: step 1048 us by the longest, 1074 so) (dK/dV kernel of 12 sequences of 64 to 2048 tokens, 16/4 heads: 153 us in
-// five groups, the last 50 of them with idle SMs, 134 in one; step 365 -> 350, with 64 MB 360). The forward, whose dynamic units
-// leave no such tail, takes one group if K and V are at most 48 MB and otherwise goes by the longest sequence (16 sequences of 512
-// to 4096 tokens, 139 MB: 16 groups 907 us, three 921, two 929, one 958).
+// Packed backward under a causal mask, from what all sequences together stream: the longest one says little about it, and in fewer and
+// larger groups fewer long chains start late. Groups stream 112 MB, except in the fused kernel, which also adds into its accumulator (20
+// sequences of 100 to 3000 tokens, D64: step 1048 us by the longest, 1074 so) (dK/dV kernel of 12 sequences of 64 to 2048 tokens, 16/4
+// heads: 153 us in five groups, the last 50 of them with idle SMs, 134 in one; step 365 -> 350, with 64 MB 360). Without a mask all blocks
+// of a sequence are equally heavy, and the order by block index in groups by the longest sequence is the faster one (step of 20
+// sequences of 300 to 3000 tokens, 16/4 heads, D128: 2909 us, by all bytes and by the blocks behind 3066; 6 of 50 to 4000, 32/8: 2905,
+// 2983; 12 of 500 to 1000, 16/16: 451, 468). The dS GEMM, which takes its units from a counter, always goes by all bytes.
 inline int heads_per_packed_group(double all_bytes, int num_heads) {
   const int groups = 1 + static_cast<int>(all_bytes / (112.0 * 1024 * 1024));
   return (num_heads + groups - 1) / groups;
 }
-inline int heads_per_forward_group(double bytes_per_head, int num_heads, bool packed, double all_bytes) {
-  return packed && all_bytes <= 48.0 * 1024 * 1024 ? num_heads : heads_per_l2_group(bytes_per_head, num_heads);
+
+// Packed forward. Its dynamic units leave no such tail, but under a causal mask one group is the faster order where K and V are at most
+// 48 MB (16 sequences of 100 to 1000 tokens, 16/16 heads, D64: 56 us, by the longest 64; 8 of 200 to 2000, 16/4, D128: 109, 120; 139 MB, 16 of
+// 512 to 4096: 958, 907; 52 to 92 MB level). Not without a mask (6 of 300 to 2900, 8/1: 128, 117; 8 of 200 to 2000, 16/4: 190, 184), and not
+// for more heads than SMs of at most two 256-row units, whose first round of claims then finds mostly nothing (32 of 16 to 300, 32/8: 56.2,
+// 55.0; of 66 to 274: 63.0, 60.5).
+inline bool one_forward_group(double all_bytes, int num_heads, bool causal, int longest) {
+  return causal && all_bytes <= 48.0 * 1024 * 1024 && (longest > 512 || num_heads <= 148);
 }
 
 // Number of SMs of the current device (cached per device), <= 0 on error.
