@@ -601,7 +601,8 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       int j_lo = 0, j_hi = kTile;
       if (kMode == kModeDKDV) {
         if (p.is_causal) j_lo = xr - causal_off - y0;
-        if (kD > 64 && xr >= len_x) j_lo = kTile;  // a row past the last key: its dS must be zero
+        // a row past the last key: its dS in the workspace must be zero (nothing else reads it, and the element mask costs time)
+        if (kD > 64 && p.ds.data != nullptr && xr >= len_x) j_lo = kTile;
       } else {
         j_hi = len_k - y0;
         if (p.is_causal) j_hi = min(j_hi, xr + causal_off + 1 - y0);
