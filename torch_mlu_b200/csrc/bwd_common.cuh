@@ -57,7 +57,7 @@ struct BwdKernelParams {
   DsTiles ds;
   uint32_t* ds_counter;
   int bh0;  // first (batch, head) pair of this launch
-  int ds_call;  // dS of this call goes through the workspace where there is room for it: see the exponentials of bwd_tile_kernel
+  int ds_call;  // kDsCall of bwd_tile_kernel
   int dq_acc_rows;  // packed: rows per head (total_q rounded up to 128, plus 128)
 #ifdef SDPA_BWD_STAMPS
   float* stamps;  // [mode 2][role 4][item 24][event 8] SM cycles since CTA start, one CTA per mode

@@ -90,7 +90,10 @@ constexpr uint32_t kSmemAbort = kSmemTmemPtr + 4;
 // launches: 61.5 us; in the fused kernel, whose dQ varies in its last bits from call to call, 60.3.
 enum BiasKind { kNoBias = 0, kFullBias = 1, kKeyBias = 2 };
 
-template <int kMode, int kD, bool kF16, bool kDrop, int kBias>
+// kDsCall: the call's dS goes through the workspace where there is room (launch_bwd). An instance of its own, since with both kinds of
+// exponentials and the dS stores behind branches the calls without dS were slower (dK/dV and dQ kernel of 6 packed sequences of 50 to 4000
+// tokens, 32/8 heads, unmasked: 1222 + 1076 us, so 1137 + 1019).
+template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -109,7 +112,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // pre-pass's tail; its vectors are read behind the wait for it. The kernel behind (the dQ kernel, which depends on nothing
   // written here, or the dQ GEMM, which waits for this grid) is let in by every CTA behind that wait, so that it too finds the
   // vectors complete. CTAs without work wait as well: a grid must not complete before the one in front of it.
-  if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
+  if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
     *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid; here, since block 0 may be one without work
   constexpr int kStages = stages_for(kMode);
   constexpr uint32_t kSmemVec = smem_vec_off(kMode);
@@ -486,17 +489,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       my_nlse2 = p.nlse2[vec];
       my_ndelta = p.ndelta[vec];
     }
-    // dK/dV with a dQ GEMM behind it: tile (query tile 0, this key block) of the group's first query head, and what leads from it
-    // to the others
-    uint32_t ds_tile0 = 0, ds_per_head = 0;
-    int ds_key_tiles = 0, ds_shift_rows = 0;
-    if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) {
+    // dK/dV with a dQ GEMM behind it: the dS tile of the next item. One running register, since more of them spill
+    uint32_t ds_tile = 0;
+    if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr) {
       wait_for_previous_grid();  // DsTiles::seq_base comes from the pre-pass
-      const DsHead dh = ds_head(p.ds, b, hx * p.kv_group, p.heads_q, len_q, len_k, p.is_causal != 0);
-      ds_tile0 = static_cast<uint32_t>(dh.base + xb);
-      ds_per_head = static_cast<uint32_t>(ds_tiles_per_head(len_q, len_k, p.is_causal != 0));
-      ds_key_tiles = dh.key_tiles;
-      ds_shift_rows = dh.shift;
+      ds_tile = ds_head(p.ds, b, hx * p.kv_group, p.heads_q, len_q, len_k, p.is_causal != 0).tile(y_lo, xb);
     }
     for (int i = 0; i < n_items; ++i) {
       const int s = (2 * i) % kStages;  // ring slot of Y1(i), which carries the per-query vectors
@@ -602,7 +599,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (kMode == kModeDKDV) {
         if (p.is_causal) j_lo = xr - causal_off - y0;
         // a row past the last key: its dS in the workspace must be zero (nothing else reads it, and the element mask costs time)
-        if (kD > 64 && p.ds.data != nullptr && xr >= len_x) j_lo = kTile;
+        if (kDsCall && p.ds.data != nullptr && xr >= len_x) j_lo = kTile;
       } else {
         j_hi = len_k - y0;
         if (p.is_causal) j_hi = min(j_hi, xr + causal_off + 1 - y0);
@@ -664,39 +661,33 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // cap, where none to two take the same time (step of B8 H16 L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed
         // 64 to 2048 tokens 369, 368, 364), and none is the most exact. Such a call without room for dS takes these two kernels, and its
         // bits must not tell: none here either, and the same roundings in both kernels (a key bias joins with one).
-        const bool ds_call = kD > 64 && p.ds_call != 0;
-        auto exponentials = [&](auto kDsCall) {
-          constexpr bool kOfDsCall = decltype(kDsCall)::value;
-          constexpr int kPolyOf4 = kOfDsCall ? 0 : kMode == kModeDQ ? 1 : 2;
+        constexpr int kPolyOf4 = kDsCall ? 0 : kMode == kModeDQ ? 1 : 2;
 #pragma unroll
-          for (int j4 = 0; j4 < 16; ++j4) {
-            const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
-            uint2 kb = make_uint2(0u, 0u);
-            if constexpr (kBias == kKeyBias && kMode == kModeDQ) kb = *reinterpret_cast<const uint2*>(key_bias_row + 2 * j4);
+        for (int j4 = 0; j4 < 16; ++j4) {
+          const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
+          uint2 kb = make_uint2(0u, 0u);
+          if constexpr (kBias == kKeyBias && kMode == kModeDQ) kb = *reinterpret_cast<const uint2*>(key_bias_row + 2 * j4);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int j = 4 * j4 + 2 * h;
-              float2 nl = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
-              if constexpr (kBias == kKeyBias) {
-                const float2 kb2 = unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), log2e = make_float2(kLog2e, kLog2e);
-                nl = kMode == kModeDQ ? fma2(kb2, log2e, nl)
-                     : kOfDsCall      ? fma2(make_float2(key_bias, key_bias), log2e, nl)
-                                      : add2(nl, make_float2(key_bias_log2, key_bias_log2));
-              }
-              const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl);
-              if (((j >> 1) & 3) < kPolyOf4) {
-                const float2 e = exp2_poly3_x2(x);
-                pr[j] = e.x;
-                pr[j + 1] = e.y;
-              } else {
-                pr[j] = ex2_approx(x.x);
-                pr[j + 1] = ex2_approx(x.y);
-              }
+          for (int h = 0; h < 2; ++h) {
+            const int j = 4 * j4 + 2 * h;
+            float2 nl = h == 0 ? make_float2(l.x, l.y) : make_float2(l.z, l.w);
+            if constexpr (kBias == kKeyBias) {
+              const float2 kb2 = unpack_16x2<kF16>(h == 0 ? kb.x : kb.y), log2e = make_float2(kLog2e, kLog2e);
+              nl = kMode == kModeDQ ? fma2(kb2, log2e, nl)
+                   : kDsCall        ? fma2(make_float2(key_bias, key_bias), log2e, nl)
+                                    : add2(nl, make_float2(key_bias_log2, key_bias_log2));
+            }
+            const float2 x = score_exponents<kDrop>(a[j], a[j + 1], c, nl);
+            if (((j >> 1) & 3) < kPolyOf4) {
+              const float2 e = exp2_poly3_x2(x);
+              pr[j] = e.x;
+              pr[j + 1] = e.y;
+            } else {
+              pr[j] = ex2_approx(x.x);
+              pr[j + 1] = ex2_approx(x.y);
             }
           }
-        };
-        if (ds_call) exponentials(std::true_type{});
-        else exponentials(std::false_type{});
+        }
         // only tiles on the causal diagonal or past the end of the keys need the element mask
         if (__any_sync(0xffffffffu, j_lo > 0 || j_hi < 64)) {
 #pragma unroll
@@ -776,17 +767,19 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(bar + kBarPFull);
       BWD_STAMP(half, i, 7);
-      if (kMode == kModeDKDV && kD > 64 && p.ds.data != nullptr) {
+      if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr) {
         // dS for the dQ GEMM: 16 bytes (8 queries) per store, 512 contiguous bytes per warp. Behind the arrival, so that the
         // dK GEMM does not wait for the stores to issue
-        const uint32_t tile = ds_tile0 + static_cast<uint32_t>(hi) * ds_per_head +
-                              static_cast<uint32_t>(ds_row_start(y0 / kTile, ds_key_tiles, ds_shift_rows));
-        if (tile < p.ds.capacity) {
-          uint4* dst = ds_group(p.ds, tile, half * 8, r);
+        if (ds_tile < p.ds.capacity) {
+          uint4* dst = ds_group(p.ds, ds_tile, half * 8, r);
 #pragma unroll
           for (int ch = 0; ch < 8; ++ch)
             dst[ch * kDsTile] = make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]);
         }
+        // past this row of tiles; behind the last one the next head's tiles begin
+        const DsHead rows{0, (len_k + kTile - 1) / kTile, ds_shift(len_q, len_k, p.is_causal != 0)};
+        ds_tile += min(max(y0 / kTile + rows.shift, 0), rows.key_tiles);
+        if (i + 1 == (hi + 1) * tiles_per_head) ds_tile += rows.tile(y_lo, 0);
       }
     }
 
@@ -1009,22 +1002,25 @@ using TileKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensor
                             const CUtensorMap, const CUtensorMap, const BwdKernelParams);
 
 template <int kMode, bool kDrop, int kBias>
-TileKernel pick_tile_kernel(int head_dim, bool f16) {
+TileKernel pick_tile_kernel(int head_dim, bool f16, bool ds_call) {
   if (head_dim <= 64)
-    return f16 ? bwd_tile_kernel<kMode, 64, true, kDrop, kBias> : bwd_tile_kernel<kMode, 64, false, kDrop, kBias>;
-  return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias>;
+    return f16 ? bwd_tile_kernel<kMode, 64, true, kDrop, kBias, false> : bwd_tile_kernel<kMode, 64, false, kDrop, kBias, false>;
+  if (ds_call)
+    return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, true> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, true>;
+  return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, false> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, false>;
 }
 
 template <int kMode, bool kDrop>
-TileKernel pick_tile_kernel(BiasKind bias, int head_dim, bool f16) {
-  if (bias == kKeyBias) return pick_tile_kernel<kMode, kDrop, kKeyBias>(head_dim, f16);
-  return bias == kFullBias ? pick_tile_kernel<kMode, kDrop, kFullBias>(head_dim, f16)
-                           : pick_tile_kernel<kMode, kDrop, kNoBias>(head_dim, f16);
+TileKernel pick_tile_kernel(BiasKind bias, int head_dim, bool f16, bool ds_call) {
+  if (bias == kKeyBias) return pick_tile_kernel<kMode, kDrop, kKeyBias>(head_dim, f16, ds_call);
+  return bias == kFullBias ? pick_tile_kernel<kMode, kDrop, kFullBias>(head_dim, f16, ds_call)
+                           : pick_tile_kernel<kMode, kDrop, kNoBias>(head_dim, f16, ds_call);
 }
 
 template <int kMode>
-TileKernel pick_tile_kernel(bool drop, BiasKind bias, int head_dim, bool f16) {
-  return drop ? pick_tile_kernel<kMode, true>(bias, head_dim, f16) : pick_tile_kernel<kMode, false>(bias, head_dim, f16);
+TileKernel pick_tile_kernel(bool drop, BiasKind bias, int head_dim, bool f16, bool ds_call) {
+  return drop ? pick_tile_kernel<kMode, true>(bias, head_dim, f16, ds_call)
+              : pick_tile_kernel<kMode, false>(bias, head_dim, f16, ds_call);
 }
 
 // `overlap_previous`: launch with programmatic stream serialization, so that this grid's CTAs may start as soon as
@@ -1040,8 +1036,8 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
   const BiasKind bias = kp.bias == nullptr                                                                    ? kNoBias
                         : kp.bias_row_stride == 0 && (mode == kModeDKDV || kp.dbias == nullptr) ? kKeyBias
                                                                                                               : kFullBias;
-  TileKernel kernel = mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16)
-                                        : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16);
+  TileKernel kernel = mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16, kp.ds_call != 0)
+                                        : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16, kp.ds_call != 0);
   const uint32_t smem = smem_bytes_for(mode, bias == kKeyBias);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) {
