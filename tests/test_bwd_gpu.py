@@ -11,6 +11,7 @@ import torch
 
 from oracle import sdpa_oracle as orc
 from test_oracle import GOLDEN, load_golden
+from tests.test_ds_backward_gpu import run as run_with_workspace
 from torch_mlu_b200 import ops, workloads
 
 pytestmark = pytest.mark.gpu
@@ -120,9 +121,9 @@ def test_backward_varlen(cuda_device, native_lib, lens, Hq, Hkv, causal):
 
 
 def test_backward_is_deterministic(cuda_device, native_lib):
-    """With `deterministic` every gradient comes back with the same bits on every call (the dK/dV and dQ kernels sum
-    in a fixed order). The fused kernel keeps that promise for dK and dV; its dQ sums are formed by floating-point
-    reductions in global memory and repeat only to fp32 rounding."""
+    """With `deterministic` every gradient comes back with the same bits on every call. Without it that holds for every kernel but the
+    fused one (head_dim 64, more key blocks than SMs), whose dQ sums are formed by floating-point reductions in global memory and
+    repeat only to fp32 rounding."""
     q, k, v, dout = (rand((1, 4, 640, 128), s) for s in (1, 2, 3, 4))
     a = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=True)
     b = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=True)
@@ -130,10 +131,15 @@ def test_backward_is_deterministic(cuda_device, native_lib):
         assert torch.equal(x, y)
     c = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=False)
     d = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=False)
-    assert torch.equal(c[3], d[3]) and torch.equal(c[4], d[4])
-    assert orc.error_stats(c[2], d[2])[0] <= 2e-2 and orc.error_stats(c[2], a[2])[0] <= 2e-2
-    # the same with 300 key blocks, which the fused kernel serves
+    for x, y, z in zip(a, c, d):
+        assert torch.equal(x, y) and torch.equal(x, z)
+    # 300 key blocks: dS through the workspace, in a fixed order either way
     many = [rand((1, 60, 640, 128), s) for s in (5, 6, 7, 8)]
+    f, h, i = (run_fwd_bwd(cuda_device, *many, True, deterministic=det) for det in (False, False, True))
+    for x, y, z in zip(f, h, i):
+        assert torch.equal(x, y) and torch.equal(x, z)
+    # and the fused kernel
+    many = [rand((1, 60, 640, 64), s) for s in (5, 6, 7, 8)]
     f, h, i = (run_fwd_bwd(cuda_device, *many, True, deterministic=det) for det in (False, False, True))
     assert torch.equal(f[3], h[3]) and torch.equal(f[4], h[4])
     assert orc.error_stats(f[2], h[2])[0] <= 2e-2 and orc.error_stats(f[2], i[2])[0] <= 2e-2
@@ -191,8 +197,13 @@ def test_config3_sampled_heads_and_linearity(cuda_device, native_lib):
         sl = (slice(b, b + 1), slice(h, h + 1))
         o_ref, l_ref = orc.cpu_sdpa_forward(c.q[sl], c.k[sl], c.v[sl], causal=True, scale=c.softmax_scale)
         wants[sl] = orc.cpu_sdpa_backward(c.dout[sl], c.q[sl], c.k[sl], c.v[sl], o_ref, l_ref, causal=True, scale=c.softmax_scale)
-    for deterministic in (False, True):  # the fused kernel, then the dK/dV + dQ pair
-        dq, dk, dv = ops._dense_backward(dd, qd, kd, vd, out, lse, True, c.softmax_scale, deterministic=deterministic)
+    def least_workspace(dout):
+        p = ops._dense_params(qd, kd, vd, out, lse, True, c.softmax_scale)
+        return run_with_workspace(native_lib, p, qd, kd, vd, dout, False, True)
+
+    for path, backward in (("dS GEMM", lambda g: ops._dense_backward(g, qd, kd, vd, out, lse, True, c.softmax_scale)),
+                           ("dK/dV and dQ kernel", least_workspace)):
+        dq, dk, dv = backward(dd)
         assert ops.device_status() == 0
         for sl, want in wants.items():
             check_grads((dq[sl], dk[sl], dv[sl]), want)
@@ -200,15 +211,11 @@ def test_config3_sampled_heads_and_linearity(cuda_device, native_lib):
             # values bf16 cannot hold to 2e-2 (at most one element in a thousand may need it)
             for name, g, w in zip(("dq", "dk", "dv"), (dq[sl], dk[sl], dv[sl]), want):
                 rep = orc.grad_error_report(g, w)
-                print(f"config 3 {name}{tuple((x.start for x in sl))} deterministic={deterministic}: {rep}")
+                print(f"config 3 {name}{tuple((x.start for x in sl))} {path}: {rep}")
                 assert rep["max_abs_where_want_le_2"] <= 2e-2, (name, rep)
                 assert rep["beyond_abs_bound"] <= rep["elements"] // 1000, (name, rep)
-        dq2, dk2, dv2 = ops._dense_backward(dd * 2, qd, kd, vd, out, lse, True, c.softmax_scale, deterministic=deterministic)
-        assert torch.equal(dk2, dk * 2) and torch.equal(dv2, dv * 2)
-        if deterministic:
-            assert torch.equal(dq2, dq * 2)
-        else:  # the order of the fused kernel's dQ reductions varies: equal up to fp32 rounding of the sums
-            assert orc.error_stats(dq2, dq.float() * 2)[0] <= 2e-2
+        dq2, dk2, dv2 = backward(dd * 2)
+        assert torch.equal(dq2, dq * 2) and torch.equal(dk2, dk * 2) and torch.equal(dv2, dv * 2)
         for t in (dq, dk, dv):
             assert torch.isfinite(t.float()).all()
 
@@ -239,15 +246,15 @@ def test_reference_tests_own_tolerance_rule(cuda_device, native_lib, dtype, B, H
 
 @pytest.mark.parametrize("lens,Hq,Hkv,D,causal", [
     ([200, 200], 38, 38, 128, True),          # dense, one key block past a tile, 152 key blocks
-    ([129, 129], 74, 37, 128, False),         # dense, grouped queries: 148 key blocks, one short of the fused kernel
+    ([129, 129], 74, 37, 128, False),         # dense, grouped queries: 148 key blocks, as many as SMs
     ([257, 257], 100, 25, 64, True),          # dense, grouped queries at head_dim 64: 150
     ([1, 300, 513, 64], 32, 8, 128, True),    # packed, grouped queries
     ([70, 700, 129], 16, 16, 64, True),       # packed, ragged ends, most tiles of the grid empty
     ([513, 2, 385], 12, 12, 104, False),      # packed, padded head_dim: 180
 ])
 def test_backward_on_both_sides_of_the_dispatch(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
-    """Calls with more key blocks than SMs, which the fused kernel serves (except grouped queries at head_dim 128), and calls
-    just below, against the oracle; dense ones in the fixed order too; tolerances as above."""
+    """Calls with more key blocks than SMs, which the fused kernel (head_dim 64) and the dS GEMM serve, and calls just below, against the
+    oracle; dense ones in the fixed order too; tolerances as above."""
     dev = cuda_device
     total, cu = sum(lens), [sum(lens[:i]) for i in range(len(lens) + 1)]
     q, k, v, dout = rand((total, Hq, D), 1), rand((total, Hkv, D), 2), rand((total, Hkv, D), 3), rand((total, Hq, D), 4)

@@ -89,7 +89,7 @@ def test_forward_with_dropout_matches_oracle_with_the_returned_mask(cuda_device,
     (1, 2, 200, 333, 128, False, 0.48),
     (1, 3, 300, 130, 64, True, 0.22),
     (2, 2, 129, 257, 96, False, 0.1),
-    # more key blocks than SMs: the fused kernel
+    # more key blocks than SMs: dS through the workspace, or (head_dim 64) the fused kernel
     (2, 40, 200, 257, 128, True, 0.22),
     (3, 26, 130, 129, 64, False, 0.48),
     (1, 75, 300, 130, 96, True, 0.1),
@@ -158,7 +158,7 @@ def test_manual_seed_repeats_the_pattern(cuda_device, native_lib):
     ([100, 300, 257], [100, 300, 257], 4, 2, True, 0.22),
     ([512, 64, 130], [200, 333, 130], 2, 2, False, 0.48),
     ([1, 129, 255], [70, 129, 400], 4, 1, True, 0.1),
-    # more key blocks than SMs: the fused kernel, with grouped queries too
+    # more key blocks than SMs: dS through the workspace, with grouped queries too
     ([100, 300, 257], [100, 300, 257], 36, 18, True, 0.22),
     ([512, 64, 130], [200, 333, 130], 18, 18, False, 0.48),
 ])

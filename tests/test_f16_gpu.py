@@ -84,7 +84,7 @@ def test_f16_varlen(cuda_device, native_lib):
     (3, 26, 26, 130, 129, 104, False),
 ])
 def test_f16_backward_with_more_key_blocks_than_sms(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
-    """The fused backward kernel."""
+    """dS through the workspace, and the fused backward kernel (head_dim 64)."""
     dev = cuda_device
     q, k, v, dout = rand((B, Hq, Lq, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3), rand((B, Hq, Lq, D), 4)
     qd, kd, vd = q.to(dev), k.to(dev), v.to(dev)

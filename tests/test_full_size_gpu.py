@@ -93,12 +93,10 @@ def test_config4_backward_full_size(cuda_device, native_lib, config4):
             orc.assert_close_grad_bf16(dk[lo:hi, kvh:kvh + 1].transpose(0, 1).unsqueeze(0), dk_r, "dk " + tag)
             orc.assert_close_grad_bf16(dv[lo:hi, kvh:kvh + 1].transpose(0, 1).unsqueeze(0), dv_r, "dv " + tag)
     # linearity in dO on the whole tensors: doubling dO doubles every gradient exactly (powers of two commute with
-    # every rounding on the way); dQ is compared at the gradient tolerance, which holds for either backward path (these
-    # grouped queries at head_dim 128 take the two kernels, the fused one would sum dQ in a varying order)
+    # every rounding on the way, and above head_dim 64 every sum is in a fixed order)
     dq2, dk2, dv2 = ops._flash_attention_backward(dout * 2, q, k, v, out, lse, cu, cu, mx, mx, 0.0, True, e, e,
                                                   scale=c.softmax_scale)
-    assert torch.equal(dk2, dk * 2) and torch.equal(dv2, dv * 2)
-    orc.assert_close_grad_bf16(dq2, dq.float() * 2, "dq linearity")
+    assert torch.equal(dq2, dq * 2) and torch.equal(dk2, dk * 2) and torch.equal(dv2, dv * 2)
 
 
 def test_config5_decode_full_size(cuda_device, native_lib):

@@ -8,14 +8,16 @@ from torch_mlu_b200 import ops
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B,H", [
-    (2, 4),
-    (4, 26),   # 312 forward units and 624 key blocks: the forward's unit counter, the fused backward and its accumulator's clearing
+@pytest.mark.parametrize("B,H,D", [
+    (2, 4, 128),
+    (4, 26, 128),  # 312 forward units and 624 key blocks: the forward's unit counter, the dS GEMM and its unit counter
+    (4, 26, 64),   # the fused backward and its accumulator's clearing
+    (1, 2, 256),
 ])
-def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib, B, H):
+def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib, B, H, D):
     dev = cuda_device
     g = torch.Generator().manual_seed(41)
-    L, D = 768, 128
+    L = 768
     scale = D ** -0.5
     make = lambda: torch.randn(B, H, L, D, generator=g).bfloat16().to(dev)
     q, k, v, do = make(), make(), make(), make()
@@ -40,7 +42,7 @@ def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib, B, H):
         want = [o2, l2, *ops._dense_backward(do, q, k, v, o2, l2, True, scale)]
         assert ops.device_status() == 0
         for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), got, want):
-            if name == "dq" and B * H * (L // 128) > 148:
+            if name == "dq" and D == 64:
                 # the fused kernel sums dQ in a varying order: two roundings to 16 bits of nearly the same sum
                 assert float((a.float() - b.float()).norm() / b.float().norm()) <= 1e-3
             else:

@@ -82,7 +82,7 @@ def set_bwd(p, dout, dq, dk, dv, packed):
     (2, 2, 2, 1, 300, 128, False),     # one query row: the tile kernel's smallest case
     (1, 4, 2, 200, 333, 160, True),    # head dims above 128: the kernels that stage 256-column tiles
     (2, 2, 1, 129, 70, 256, False),
-    (2, 40, 40, 200, 257, 128, True),   # more key blocks than SMs: the fused backward, and more units than SMs in the forward
+    (2, 40, 40, 200, 257, 128, True),   # more key blocks than SMs: dS through the workspace (head_dim 64: the fused backward)
     (3, 26, 26, 333, 130, 80, False),
     (1, 150, 75, 129, 257, 64, True),
 ])
@@ -122,7 +122,7 @@ def test_dense_forward_and_backward_write_nothing_outside_their_outputs(cuda_dev
     ([300, 45], 8, 2, 96, True),
     ([130, 70, 1, 255], 4, 2, 256, True),
     ([128, 129], 2, 2, 136, False),
-    ([130, 70, 1, 255], 20, 20, 128, True),   # more key blocks than SMs: the fused backward
+    ([130, 70, 1, 255], 20, 20, 128, True),   # more key blocks than SMs: dS through the workspace (head_dim 64: the fused backward)
     ([128, 129, 127], 26, 26, 64, False),
     ([300, 45], 50, 25, 64, True),
 ])
@@ -273,4 +273,4 @@ def test_packed_gradients_of_tokens_outside_every_sequence_are_zero(cuda_device,
         assert not got[:front].any() and not got[front + n:].any(), name
         # the fused kernel sums dQ in a varying order: two roundings to 16 bits of nearly the same sum
         err = (got[cut].float() - ref.float()).norm() / ref.float().norm()
-        assert float(err) <= (0.0 if deterministic or name != "dq" else 1e-3), (name, float(err))
+        assert float(err) <= (0.0 if deterministic or D != 64 or name != "dq" else 1e-3), (name, float(err))

@@ -32,14 +32,14 @@ def draw_case(rng: random.Random):
 
 
 def draw_case_with_many_heads(rng: random.Random):
-    """As draw_case, with enough key blocks for the fused backward (more than SMs) and the forward's unit counter."""
+    """As draw_case, with more key blocks than SMs, for the fused backward and the dS GEMM, and the forward's unit counter."""
     c = draw_case(rng)
     group = rng.choice([1, 1, 2])
     c["Hkv"] = rng.choice([50, 75])
     c["Hq"] = c["Hkv"] * group
     c["B"] = 3
     if group > 1:
-        c["D"] = rng.choice([64, 32])  # grouped queries at head_dim 128 take the two kernels
+        c["D"] = rng.choice([64, 32])  # the fused backward's; grouped queries of the dS GEMM have tests of their own
     return c
 
 
