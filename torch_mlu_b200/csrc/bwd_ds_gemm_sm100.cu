@@ -43,16 +43,9 @@ static_assert(kAbort + 4 <= 512 && smem_bytes(128) <= 232448 && smem_bytes(256) 
 constexpr uint32_t kFlagTile0 = 1, kFlagTile1 = 2, kFlagFirst = 4, kFlagLast = 8, kFlagStop = 16, kFlagKeys = 32;
 constexpr int kUnitStop = 2;
 
-struct Unit {
-  int kind;     // 0 dQ, 1 dK, kUnitStop
-  int row0;     // first output row within the sequence
-  int rows;     // output rows of the sequence
-  int row_off;  // of the sequence in a packed tensor
-  int head, batch;
-  int has;      // bit t: some contraction row contributes to tile t
-  int unused;
-};
-static_assert(sizeof(Unit) == 32, "the table holds 32 bytes per unit");
+// A unit in the table is two int4:
+//   kind (0 dQ, 1 dK, kUnitStop), first output row within the sequence, output rows of the sequence, its first row in a packed tensor
+//   head, batch, bit t: some contraction row contributes to tile t, unused
 
 // D[tmem] (+)= A[smem, no swizzle] * B[smem, 128-byte swizzle]
 __device__ __forceinline__ void umma_ss_plain_a(uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t idesc,
@@ -391,7 +384,8 @@ Kernel pick_kernel(int head_dim, bool f16) {
 
 // dS of a call (half of B H Lq Lk elements of two bytes under a causal mask) may take this much of the workspace; a dense call with
 // more of it goes through it in several passes over its KV heads. One pass is best (step of B8 H16 L2048, 0.57 GB of dS: 673 us in
-// one pass, 709 in two, 766 in six, where a pass's dS would stay in L2; B2 H16 L8192, 2.1 GB: 2115 in one, 2189 in two).
+// one pass, 709 in two, 766 in six, where a pass's dS would stay in L2; B2 H16 L8192, 2.18 GB: 2189 in its two passes, 2115 in one
+// with room for it).
 constexpr size_t kDsBytesMax = size_t{2} << 30;
 
 DsPlan ds_plan(const sdpa_b200_params& p) {
@@ -412,7 +406,11 @@ DsPlan ds_plan(const sdpa_b200_params& p) {
   const int64_t passes = (kv_heads * per_kv_head + cap - 1) / cap;
   int64_t per_pass = (kv_heads + passes - 1) / passes;
   if (per_pass * per_kv_head > cap) per_pass = cap / per_kv_head;
-  if (passes > 1 && per_pass * key_tiles < 3 * 148) return plan;  // a pass must fill the SMs a few times over
+  // A pass must fill the SMs a few times over, or its launches' tails cost more than the second pass over the scores: step of B1 H32/8
+  // L8192 D128 causal (two passes of 256 CTAs) 2270 us with the two kernels, 2510 so; B2 (three of 384) 4524 and 4500, B1 H32/4 unmasked (two of 128)
+  // 4290 and 4195. Above head_dim 128, where the alternative are three kernels, the line lies too high (B1 H32/8 L8192 D256 causal 5283, in
+  // passes 4627; B2 H16/4 unmasked 9546, 7636).
+  if (passes > 1 && per_pass * key_tiles < 3 * 148) return plan;
   plan.kv_heads = static_cast<int>(per_pass);
   plan.tiles = static_cast<uint32_t>(per_pass * per_kv_head);
   return plan;

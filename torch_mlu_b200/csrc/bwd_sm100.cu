@@ -1080,7 +1080,7 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 //    the two kernels (B8 H12 L512 with a mask 61.5; fused 60.3, and through dS level).
 //  * head_dim 65 to 128, more key blocks: dS through the workspace and a GEMM for dQ (use_ds_backward). One pass over the scores where
 //    the two kernels make two, and no reductions. (Step of B8 H16 L2048 695, two kernels 757, fused 752; with dropout 875, 940, 925;
-//    B2 H16 L8192 2115, 2295, 2290; B16 H32 L512 310, 365, 360; D80 B8 H16 L2048 alone 438, 533, 545; grouped B8 H32/8 L2048 alone
+//    B2 H16 L8192, in two passes, 2189, 2295, 2290; B16 H32 L512 310, 365, 360; D80 B8 H16 L2048 alone 438, 533, 545; grouped B8 H32/8 L2048 alone
 //    860, 1100, 1130, B16 H16/4 L700 165, 208, 206.) The smallest of these grids, replayed from a graph: B3 H50 L128 alone 23.1, 22.3,
 //    27.0, B2 H80 L256 45.3, 46.0, 53.8, grouped B2 H80/40 L256 41.1, 42.9, 43.0, with dropout 45.7, 47.3, 58.3.
 // A packed call counts the key blocks of its grid, every sequence at the longest length, whether they have keys or not. The number
