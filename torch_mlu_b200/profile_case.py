@@ -32,7 +32,7 @@ def main() -> None:
     ap.add_argument("--launches", type=int, default=3)
     ap.add_argument("--non-causal", action="store_true")
     ap.add_argument("--head-dim", type=int, default=128)
-    ap.add_argument("--deterministic", action="store_true", help="backward: the dK/dV + dQ kernels instead of the fused one")
+    ap.add_argument("--deterministic", action="store_true", help="backward: a fixed summation order (head_dim 64: the dK/dV and dQ kernels instead of the fused one)")
     a = ap.parse_args()
     D = a.head_dim
     dev = torch.device("cuda", 0)
