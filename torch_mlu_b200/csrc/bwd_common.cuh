@@ -116,7 +116,7 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src,
 __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Four consecutive per-query values from shared memory. One 16-byte read; in the dropout instances four reads, because there
-// the quads (and packed arithmetic on them) spill: fused backward of B8 H16 L2048 D128 causal 446 -> 440 us without dropout,
+// the quads (and packed arithmetic on them) spill: fused backward, when it served head_dim 128, of B8 H16 L2048 causal 446 -> 440 us without dropout,
 // but 522 -> 542 with it.
 template <bool kDrop>
 __device__ __forceinline__ float4 read_vec4(const float* v) {

@@ -2,7 +2,7 @@
 // has left in the workspace (ds_tiles.cuh).
 //
 // Bound by memory: every dS tile is read once, 32 KB for 128 x 128 x head_dim multiply-adds. Two 128-row tiles per unit share each B
-// block (48 KB per step of 64 at head_dim 128 where single tiles would read 64). B8 H16 L2048 D128 causal: 0.57 GB of dS in about 120 us.
+// block (48 KB per step of 64 at head_dim 128 where single tiles would read 64). B8 H16 L2048 D128 causal: 0.57 GB of dS in 130 us.
 //
 // Persistent: one CTA per SM takes units of 256 output rows (two 128-row tiles that share every B block) of one head from a
 // counter, heaviest first inside a group of heads. Per 64 rows of the contraction a stage brings B (64 rows of K or Q, 128-byte

@@ -16,12 +16,11 @@
 // a small kernel scales and converts the accumulator afterwards. Those reductions arrive in an order that varies from
 // launch to launch, so dQ is reproducible only to fp32 rounding; dK and dV are summed in a fixed order.
 //
-// What bounds it (time stamps of the profiling build, B8 H16 L2048 causal): the reductions. One item adds 64 KB into
-// the accumulator; with every SM sending them, the L2 takes about 20 bytes per clock and SM (a stand-alone test reaches
+// What bounds it (time stamps of the profiling build at head_dim 128, which it served at first; B8 H16 L2048 causal): the reductions. One item
+// adds 64 KB into the accumulator (32 KB at head_dim 64, for half the tensor work as well); with every SM sending them, the L2 takes about 20 bytes per clock and SM (a stand-alone test reaches
 // 5.5 TB/s = 706 floats per clock over the chip with red.v4 and with cp.reduce.async.bulk alike, 3.6 TB/s once the
 // accumulator exceeds L2), i.e. ~3400 cycles per item against 2560 cycles of tensor work, and a reduce warp needs
-// ~90 cycles per red.v4. With the issuers at the pipe's rate and packed arithmetic the kernel takes 438 us at B8 H16 L2048
-// causal, whether none or three quarters of the exponentials run on the FMA pipe: the compute warps no longer bound it.
+// ~90 cycles per red.v4. With the issuers at the pipe's rate and packed arithmetic the kernel took 438 us there, whether none or three quarters of the exponentials run on the FMA pipe: the compute warps no longer bound it.
 // When it is the faster path, with figures: use_fused_backward() in bwd_sm100.cu.
 //
 // TMEM (512 columns): T1 [0,128) T2 [128,256) dV [256,384) dK [384,512). Item i has S in T[i&1] and dP in the other
@@ -46,7 +45,7 @@ constexpr int kFThreads = 512;  // warps 0-3 / 4-7 compute, 8 TMA, 9 score GEMMs
 // the shrinking warpgroups release must cover what the growing ones take.
 constexpr int kRegsLaunch = 128;
 constexpr int kRegsCompute = 152;
-constexpr int kRegsReduce = 144;  // a thread holds a whole row of the dQ tile (up to 128 floats)
+constexpr int kRegsReduce = 144;  // a thread holds a whole row of the dQ tile (64 floats)
 constexpr int kRegsUtil = 64;
 static_assert(kRegsCompute >= kRegsLaunch && kRegsReduce >= kRegsLaunch && kRegsUtil <= kRegsLaunch &&
                   (kRegsCompute - kRegsLaunch) * 2 + (kRegsReduce - kRegsLaunch) <= (kRegsLaunch - kRegsUtil),
