@@ -227,3 +227,24 @@ def test_config4_varlen_gqa_scaled_down(cuda_device, native_lib):
     o_ref, l_ref = orc.varlen_forward(c.q, c.k, c.v, cu, cu, causal=True, scale=c.softmax_scale)
     orc.assert_close_bf16(out, o_ref, "out")
     orc.assert_close_lse(lse, l_ref)
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,D,causal", [
+    ([193, 769, 342], 32, 32, 128, True),   # up to two rounds of units, claimed late throughout; one group of heads
+    ([300, 1, 700, 64], 64, 8, 64, False),  # the same without a mask: groups by the longest sequence
+    ([200, 62, 234], 40, 8, 128, True),     # one unit per head
+    ([134, 282, 200] * 4, 16, 4, 64, True),  # two at most
+    ([128, 888, 150, 130] * 4, 16, 16, 64, True),   # three rounds in mostly empty slots
+    ([700, 900, 888, 600] * 2, 32, 8, 64, True),    # in mostly filled ones
+])
+def test_packed_orders(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
+    """Every side of the rules that order the units of a packed call, against the oracle."""
+    gen = torch.Generator().manual_seed(11)
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    q, k, v = (torch.randn(cu[-1], h, D, generator=gen).bfloat16() for h in (Hq, Hkv, Hkv))
+    cu_d = torch.tensor(cu, dtype=torch.int32, device=cuda_device)
+    out, lse, *_ = ops._flash_attention_forward(*(t.to(cuda_device) for t in (q, k, v)), cu_d, cu_d, max(lens), max(lens), 0.0, causal, False)
+    assert ops.device_status() == 0
+    o_ref, l_ref = orc.varlen_forward(q, k, v, cu, cu, causal=causal)
+    orc.assert_close_bf16(out, o_ref, "out")
+    orc.assert_close_lse(lse, l_ref)

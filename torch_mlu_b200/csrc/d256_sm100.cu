@@ -1439,7 +1439,8 @@ int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   kp.num_m_blocks = (p.max_seqlen_q + kRowsA - 1) / kRowsA;
   kp.num_bh = p.batch * p.heads_q;
   const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q)
+  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q,
+                                                  packed_units(p, kRowsA), static_cast<double>(kp.num_bh) * kp.num_m_blocks, 148)
                           ? kp.num_bh
                           : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
   kp.scale_log2 = p.softmax_scale * 1.4426950408889634f;

@@ -101,6 +101,7 @@ struct FwdKernelParams {
   int64_t bias_batch_stride, bias_head_stride, bias_row_stride;
   float inv_scale;  // 1 / softmax_scale: the bias joins the raw scores as bias / scale
   int num_m_blocks, num_bh, heads_per_wave, num_slots;  // work-unit order, see decode_unit()
+  int lazy_from;  // slot from which units are claimed late, see the unit scheduler
   float scale_log2;
   int is_causal;
 #ifdef SDPA_FWD_STAMPS
@@ -464,7 +465,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
         bool ok = true;
         // Claiming ahead hides the claim (atomic + decode) and lets the producer prefetch the next Q
         // tiles, but near the end of the list a unit claimed early by a busy CTA is a unit an idle CTA
-        // cannot take. For the last two rounds of the grid the scheduler therefore claims late: only
+        // cannot take. For the last two rounds of the grid (`lazy_from`) the scheduler therefore claims late: only
         // once the last QK^T of the unit it published before has been issued (the Q-free barrier).
         bool lazy = false;
         bool last_runs = false;  // the unit published last has key blocks (and so a Q-free phase)
@@ -483,7 +484,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
                                                        : static_cast<int>(blockIdx.x);
             own_taken = true;
             if (slot >= p.num_slots) break;
-            if (slot >= p.num_slots - 2 * static_cast<int>(gridDim.x)) lazy = true;
+            if (slot >= p.lazy_from) lazy = true;
             if (decode_unit(p, slot, u)) break;  // padding slots and row-less units are skipped
             u.done = 1;
           }
@@ -886,13 +887,6 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   }
   kp.num_m_blocks = (p.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM);
   kp.num_bh = p.batch * p.heads_q;
-  // K+V bytes one query head streams, shared by the heads of its GQA group
-  const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q)
-                          ? kp.num_bh
-                          : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
-  const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
-  kp.num_slots = groups * kp.heads_per_wave * kp.num_m_blocks;
   const int sms = sm_count();
   if (sms <= 0) {
     set_error("prefill: cannot read the SM count of the current device");
@@ -900,7 +894,20 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   }
   // one persistent CTA per SM (shared memory and TMEM allow no second one), less the SMs the caller wants left free
   const int usable = sms - p.sm_margin > 1 ? sms - p.sm_margin : 1;
+  // K+V bytes one query head streams, shared by the heads of its GQA group
+  const double kv_row_bytes = 2.0 * p.head_dim * 2;
+  const double units = varlen ? packed_units(p, 2 * kBlockM) : 0;
+  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q, units,
+                                                  static_cast<double>(kp.num_bh) * kp.num_m_blocks, usable)
+                          ? kp.num_bh
+                          : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
+  const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
+  kp.num_slots = groups * kp.heads_per_wave * kp.num_m_blocks;
   dim3 grid(kp.num_slots < usable ? kp.num_slots : usable, 1, 1);
+  // A packed call of up to two rounds of units claims late throughout: its slots are partly empty, so the last two rounds of slots say nothing
+  // about the units (3 sequences of 193 to 769 tokens, 32 heads, D128 35.0 us in one group, 26.2 so; 6 of 390 to 1117, 16/4, D64 35.6, 25.0; 6 of
+  // 309 to 2900, 8/1, unmasked 117, 88). With more units that costs more than it gives (8 of 306 to 1102, 16/16, D64 42.1, 46.2).
+  kp.lazy_from = varlen && units <= 2.0 * usable ? 0 : kp.num_slots - 2 * static_cast<int>(grid.x);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
   // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
   // cleared already.) Not for two units per CTA, dealt out by index: alone that is faster (B8 H12 L512 D64 unmasked, eager, 22.6 us against

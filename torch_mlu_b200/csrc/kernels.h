@@ -54,13 +54,22 @@ inline int heads_per_packed_group(double all_bytes, int num_heads) {
   return (num_heads + groups - 1) / groups;
 }
 
+// Units that the sequences of a packed forward hold, with `rows` queries each: half of a last unit per sequence on average. The lengths are on
+// the device.
+inline double packed_units(const sdpa_b200_params& p, int rows) {
+  return p.heads_q * (p.total_q / static_cast<double>(rows) + 0.5 * p.batch);
+}
+
 // Packed forward. Its dynamic units leave no such tail, but under a causal mask one group is the faster order where K and V are at most
-// 48 MB (16 sequences of 100 to 1000 tokens, 16/16 heads, D64: 56 us, by the longest 64; 8 of 200 to 2000, 16/4, D128: 109, 120; 139 MB, 16 of
-// 512 to 4096: 958, 907; 52 to 92 MB level). Not without a mask (6 of 300 to 2900, 8/1: 128, 117; 8 of 200 to 2000, 16/4: 190, 184), and not
-// for more heads than SMs of at most two 256-row units, whose first round of claims then finds mostly nothing (32 of 16 to 300, 32/8: 56.2,
-// 55.0; of 66 to 274: 63.0, 60.5).
-inline bool one_forward_group(double all_bytes, int num_heads, bool causal, int longest) {
-  return causal && all_bytes <= 48.0 * 1024 * 1024 && (longest > 512 || num_heads <= 148);
+// 48 MB (16 sequences of 100 to 1000 tokens, 16/16 heads, D64: 56 us, by the longest 64; 8 of 200 to 2000, 16/4, D128: 109, 118; 139 MB, 16 of
+// 512 to 4096: 958, 907; 52 to 92 MB level). Not without a mask (6 of 300 to 2900, 8/1: 128, 117; 8 of 200 to 2000, 16/4: 190, 184), not
+// for two 256-row units at most (32 of 16 to 300, 32/8: 56.2, 55.0; 5 of 134 to 282, 16/4: 15.5, 14.6; but one unit each, without the slots that
+// fill up a last group: 6 of 62 to 234, 12/12, D64 10.8, 12.1), and not where slots without a unit, which one group puts in front, are many and
+// rounds few (9 of 29 to 2820, 8/1, D64, 424 units in 864 slots: 89, 76; 13 of 128 to 888, 16/16, 480 in 832: 43.1, 41.5; but 30 of 64 to 4000, 8/1,
+// fourteen rounds: 445, 464).
+inline bool one_forward_group(double all_bytes, int num_heads, bool causal, int longest, double units, double slots, int sms) {
+  return causal && all_bytes <= 48.0 * 1024 * 1024 && (longest > 512 || (longest <= 256 && num_heads <= sms)) &&
+         (units <= 2.0 * sms || units >= 8.0 * sms || units >= 0.6 * slots);
 }
 
 // Number of SMs of the current device (cached per device), <= 0 on error.
