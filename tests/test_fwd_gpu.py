@@ -248,3 +248,14 @@ def test_packed_orders(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
     o_ref, l_ref = orc.varlen_forward(q, k, v, cu, cu, causal=causal)
     orc.assert_close_bf16(out, o_ref, "out")
     orc.assert_close_lse(lse, l_ref)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D", [
+    (3, 16, 16, 600, 600, 64),    # three ranks of 256 rows, one of them behind two groups of heads, the second one short
+    (2, 40, 8, 257, 1100, 128),   # a cached prefix: all ranks have many keys
+    (3, 12, 12, 1030, 700, 64),   # units without keys among the lightest
+])
+def test_causal_ranks_behind_all_groups(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D):
+    """More heads than a group holds, so that the lightest ranks run behind all groups, against the oracle."""
+    q, k, v = rand((B, Hq, Lq, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3)
+    check_dense(cuda_device, q, k, v, True)

@@ -4,6 +4,7 @@
 
 #include <cuda_bf16.h>
 
+#include "block_order.cuh"
 #include "ds_tiles.cuh"
 #include "kernels.h"
 #include "ptx_sm100.cuh"
@@ -28,8 +29,8 @@ struct BwdKernelParams {
   int64_t dk_batch_stride, dk_head_stride, dk_row_stride;
   int64_t dv_batch_stride, dv_head_stride, dv_row_stride;
   int seqlen_q, seqlen_k, heads_q, heads_kv, kv_group, lq_pad;
-  int num_row_blocks;  // blocks of 128 stationary rows (keys for dK/dV, queries for dQ)
-  int num_bh, heads_x, heads_per_wave;  // CTA order, see the top of bwd_tile_kernel
+  BlockOrder order;  // of the blocks of 128 stationary rows (keys for dK/dV, queries for dQ)
+  int heads_x;
   float scale, scale_log2;
   int is_causal;
   int head_dim;  // <= kD (the kernels are built for 64 and 128 columns; TMA pads loads and clips stores)

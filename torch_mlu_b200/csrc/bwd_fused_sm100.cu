@@ -143,17 +143,11 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     return;
   }
 
-  // CTA order (1-D grid): (batch, kv head) pairs in groups of `heads_per_wave` whose streamed tensors fit L2 together;
-  // inside a group the key blocks go heaviest first across all its heads (key block 0 sees every query).
+  // CTA order (1-D grid, block_order.cuh): heaviest blocks first (key block 0 sees every query).
   int b, hx, xb;
   {
-    const int per_group = p.heads_per_wave * p.num_row_blocks;
-    const int grp = blockIdx.x / per_group;
-    const int w = blockIdx.x - grp * per_group;
-    const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
-    const int rank = w / size;
-    const int bh = grp * p.heads_per_wave + (w - rank * size);
-    if (rank >= p.num_row_blocks) return;  // padding slots of a short last group
+    int rank, bh;
+    if (!block_of_slot(p.order, blockIdx.x, rank, bh)) return;
     xb = rank;
     b = bh / p.heads_x;
     hx = bh - b * p.heads_x;

@@ -118,24 +118,18 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   constexpr uint32_t kSmemVec = smem_vec_off(kMode);
   constexpr uint32_t kSmemBar = smem_bar_off(kMode);
 
-  // CTA order (1-D grid): (batch, head) pairs in groups of `heads_per_wave` whose streamed tensors
-  // fit L2 together; inside a group the 128-row blocks go heaviest first across all its heads
-  // (dK/dV: key block 0 sees every query; dQ: the last query block sees every key), so the launch
-  // ends on its lightest blocks. Packed, causal: blocks with the same number of blocks behind (dQ: in front of) them in their own
+  // CTA order (1-D grid, block_order.cuh): heaviest blocks first (dK/dV: key block 0 sees every query; dQ: the last query block sees
+  // every key). Packed, causal: blocks with the same number of blocks behind (dQ: in front of) them in their own
   // sequence count as equally heavy, so that a short sequence's first key block does not go before a long one's second.
   int b, hx, xb;
   {
-    const int per_group = p.heads_per_wave * p.num_row_blocks;
-    const int grp = blockIdx.x / per_group;
-    const int w = blockIdx.x - grp * per_group;
-    const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
-    const int rank = w / size;
-    const int bh = p.bh0 + grp * p.heads_per_wave + (w - rank * size);
-    if (rank >= p.num_row_blocks) {  // padding slots of a short last group
+    int rank, bh;
+    if (!block_of_slot(p.order, blockIdx.x, rank, bh)) {
       wait_for_previous_grid();
       return;
     }
-    xb = (kMode == kModeDKDV) ? rank : p.num_row_blocks - 1 - rank;
+    bh += p.bh0;
+    xb = (kMode == kModeDKDV) ? rank : p.order.ranks - 1 - rank;
     b = bh / p.heads_x;
     hx = bh - b * p.heads_x;
   }
@@ -146,7 +140,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
-    if (kMode == kModeDKDV && p.is_causal) xb -= p.num_row_blocks - (len_k + kTile - 1) / kTile;
+    if (kMode == kModeDKDV && p.is_causal) xb -= p.order.ranks - (len_k + kTile - 1) / kTile;
   }
   const int causal_off = len_k - len_q;
   const int len_x = (kMode == kModeDKDV) ? len_k : len_q;
@@ -286,7 +280,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const long long t_start = clock64();
   // a long-running block of batch 0, head 0 (non-causal: any; causal: the heaviest)
   const bool stamp_on = p.stamps != nullptr && b == 0 && hx == 0 &&
-                        xb == ((kMode == kModeDKDV) ? 0 : p.num_row_blocks - 1) && (lane == 0) &&
+                        xb == ((kMode == kModeDKDV) ? 0 : p.order.ranks - 1) && (lane == 0) &&
                         (warp == 0 || warp == 4 || warp == 9 || warp == 10);
 #endif
 
@@ -1248,17 +1242,16 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
 #endif
 
   // streamed: q + dO of the group, or k + v
-  auto set_order = [&](int heads_x, int rows_streamed, int streams_per_head, int num_bh, double packed_rows) {
+  // `rows`: what the stationary blocks divide; a head streams `rows_streamed` rows of `streams` heads
+  auto set_order = [&](int heads_x, int rows, int heads, int rows_streamed, int streams, double packed_rows) {
     kp.heads_x = heads_x;
-    kp.num_bh = num_bh;
     const double row_bytes = 2.0 * p.head_dim * 2;
-    kp.heads_per_wave = varlen && !fused && p.is_causal ? heads_per_packed_group(row_bytes * packed_rows, num_bh)
-                                                        : heads_per_l2_group(row_bytes * rows_streamed * streams_per_head, num_bh);
-    const int groups = (num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
-    return groups * kp.heads_per_wave * kp.num_row_blocks;
+    kp.order = block_order(heads, (rows + kTile - 1) / kTile,
+                           varlen && !fused && p.is_causal ? heads_per_packed_group(row_bytes * packed_rows, heads)
+                                                           : heads_per_l2_group(row_bytes * rows_streamed * streams, heads));
+    return kp.order.slots;
   };
   const double rows_q_all = static_cast<double>(p.total_q) * p.heads_q, rows_k_all = static_cast<double>(p.total_k) * p.heads_kv;
-  kp.num_row_blocks = (p.max_seqlen_k + kTile - 1) / kTile;
   kp.bh0 = 0;
   kp.ds.data = nullptr;
   kp.ds_call = plan.tiles > 0;
@@ -1272,7 +1265,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
       const int n = kv_heads - first < plan.kv_heads ? kv_heads - first : plan.kv_heads;
       kp.bh0 = first;
       kp.ds.head0 = first * kp.kv_group;
-      const int grid = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, n, rows_q_all);
+      const int grid = set_order(p.heads_kv, p.max_seqlen_k, n, p.max_seqlen_q, kp.kv_group, rows_q_all);
       if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
                                    /*overlap_previous=*/first == 0)) != SDPA_B200_OK)
         return st;
@@ -1280,7 +1273,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
     }
     return SDPA_B200_OK;
   }
-  const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_q, kp.kv_group, p.batch * p.heads_kv, rows_q_all);
+  const int grid_dkdv = set_order(p.heads_kv, p.max_seqlen_k, p.batch * p.heads_kv, p.max_seqlen_q, kp.kv_group, rows_q_all);
   if (fused) return launch_bwd_fused(p, kp, dq_acc, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk);
   CUtensorMap tm_dq;
   if ((st = make_tensor_map_16(f16, &tm_dq, p.dq, p.head_dim, rows_q, p.heads_q, nb, p.dq_row_stride, p.dq_head_stride,
@@ -1289,8 +1282,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
                                /*overlap_previous=*/true)) != SDPA_B200_OK)
     return st;
-  kp.num_row_blocks = (p.max_seqlen_q + kTile - 1) / kTile;
-  const int grid_dq = set_order(p.heads_q, p.max_seqlen_k, 1, p.batch * p.heads_q, rows_k_all);
+  const int grid_dq = set_order(p.heads_q, p.max_seqlen_q, p.batch * p.heads_q, p.max_seqlen_k, 1, rows_k_all);
   return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kp,
                             /*overlap_previous=*/true);
 }

@@ -20,6 +20,7 @@
 // behind PV(j), so the next block's scores are formed while this block is exponentiated.
 #include <cuda_bf16.h>
 
+#include "block_order.cuh"
 #include "bwd_ds_gemm.h"
 #include "kernels.h"
 #include "packed_grads.cuh"
@@ -60,7 +61,7 @@ struct D256Params {
   int64_t q_batch_stride, q_head_stride, q_row_stride;
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int seqlen_q, seqlen_k, total_q, heads_q, kv_group, head_dim;
-  int num_m_blocks, num_bh, heads_per_wave;
+  BlockOrder order;  // of the 128-row blocks
   float scale_log2;
   int is_causal;
   // dropout (kernels built with kDrop): one keep bit per (query, key) pair, see dropout_mask.cu
@@ -125,18 +126,11 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  // CTA order: (batch, head) pairs in groups of `heads_per_wave` whose K/V fit L2 together; inside a group the 128-row
-  // blocks go heaviest first (with a causal mask the last block sees the most keys) across all its heads.
   int b, h, mb;
   {
-    const int per_group = p.heads_per_wave * p.num_m_blocks;
-    const int grp = blockIdx.x / per_group;
-    const int w = blockIdx.x - grp * per_group;
-    const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
-    const int rank = w / size;
-    const int bh = grp * p.heads_per_wave + (w - rank * size);
-    if (rank >= p.num_m_blocks) return;  // padding slots of a short last group
-    mb = p.num_m_blocks - 1 - rank;
+    int rank, bh;
+    if (!block_of_slot(p.order, blockIdx.x, rank, bh)) return;
+    mb = p.order.ranks - 1 - rank;  // with a causal mask the last block sees the most keys
     b = bh / p.heads_q;
     h = bh - b * p.heads_q;
   }
@@ -498,7 +492,8 @@ struct Bwd256Params {
   int64_t x1_batch_stride, x1_head_stride, x1_row_stride;
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int seqlen_q, seqlen_k, heads_q, heads_kv, kv_group, head_dim, lq_pad;
-  int num_row_blocks, num_bh, heads_x, heads_per_wave;
+  BlockOrder order;  // of the 128-row blocks
+  int heads_x;
   float scale, scale_log2;
   int is_causal;
   // dropout (kernels built with kDrop): P is recomputed without it; dV takes P o M / (1 - p), dS = P o (M o dP / (1 - p) - delta)
@@ -597,18 +592,13 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 
-  // CTA order as in the forward: groups of heads whose streamed tensors fit L2, heaviest row blocks first
-  // (key block 0 sees every query; the last query block sees every key; under a mask packed key blocks by the number of blocks behind them)
+  // key block 0 sees every query; the last query block sees every key; under a mask packed key blocks go by the number of blocks behind them
   int b, hx, xb;
   {
-    const int per_group = p.heads_per_wave * p.num_row_blocks;
-    const int grp = blockIdx.x / per_group;
-    const int w = blockIdx.x - grp * per_group;
-    const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
-    const int rank = w / size;
-    const int bh = (kMode == kDVS ? p.bh0 : 0) + grp * p.heads_per_wave + (w - rank * size);
-    if (rank >= p.num_row_blocks) return;
-    xb = kKeys ? rank : p.num_row_blocks - 1 - rank;
+    int rank, bh;
+    if (!block_of_slot(p.order, blockIdx.x, rank, bh)) return;
+    if (kMode == kDVS) bh += p.bh0;
+    xb = kKeys ? rank : p.order.ranks - 1 - rank;
     b = bh / p.heads_x;
     hx = bh - b * p.heads_x;
   }
@@ -619,7 +609,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
-    if (kKeys && p.is_causal) xb -= p.num_row_blocks - (len_k + kRowsA - 1) / kRowsA;
+    if (kKeys && p.is_causal) xb -= p.order.ranks - (len_k + kRowsA - 1) / kRowsA;
   }
   const int causal_off = len_k - len_q;
   const int len_x = kKeys ? len_k : len_q;
@@ -1350,14 +1340,13 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace
     }
     const bool keys = mode != kDQ;
     kp.heads_x = keys ? p.heads_kv : p.heads_q;
-    kp.num_bh = mode == kDVS ? kv_heads : p.batch * kp.heads_x;
-    kp.num_row_blocks = ((keys ? p.max_seqlen_k : p.max_seqlen_q) + kRowsA - 1) / kRowsA;
+    const int heads = mode == kDVS ? kv_heads : p.batch * kp.heads_x;
+    const int ranks = ((keys ? p.max_seqlen_k : p.max_seqlen_q) + kRowsA - 1) / kRowsA;
     // bytes one stationary head streams: Q + dO of its group (keys), or K + V (queries)
     const double streamed = 2.0 * (keys ? p.max_seqlen_q : p.max_seqlen_k) * p.head_dim * 2 * (keys ? kp.kv_group : 1);
     const double packed = 2.0 * p.head_dim * 2 * (keys ? static_cast<double>(p.total_q) * p.heads_q : static_cast<double>(p.total_k) * p.heads_kv);
-    kp.heads_per_wave = varlen && p.is_causal ? heads_per_packed_group(packed, kp.num_bh) : heads_per_l2_group(streamed, kp.num_bh);
-    const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
-    const int grid = groups * kp.heads_per_wave * kp.num_row_blocks;
+    kp.order = block_order(heads, ranks, varlen && p.is_causal ? heads_per_packed_group(packed, heads) : heads_per_l2_group(streamed, heads));
+    const int grid = kp.order.slots;
     kernel<<<grid, kBwdThreads, kSmemBytesBwd256, stream>>>(x2, y1, y2, out, kp);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1436,13 +1425,9 @@ int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   kp.heads_q = p.heads_q;
   kp.kv_group = p.heads_q / p.heads_kv;
   kp.head_dim = p.head_dim;
-  kp.num_m_blocks = (p.max_seqlen_q + kRowsA - 1) / kRowsA;
-  kp.num_bh = p.batch * p.heads_q;
   const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q,
-                                                  packed_units(p, kRowsA), static_cast<double>(kp.num_bh) * kp.num_m_blocks, 148)
-                          ? kp.num_bh
-                          : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
+  const int heads = p.batch * p.heads_q, ranks = (p.max_seqlen_q + kRowsA - 1) / kRowsA;
+  kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes));
   kp.scale_log2 = p.softmax_scale * 1.4426950408889634f;
   kp.is_causal = p.is_causal;
   const bool drop = p.dropout_p > 0.f;
@@ -1457,9 +1442,7 @@ int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
     set_error("head_dim 256 forward: cudaFuncSetAttribute(%u bytes smem): %s", kSmemBytesD256, cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
   }
-  const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
-  const int grid = groups * kp.heads_per_wave * kp.num_m_blocks;
-  kernel<<<grid, 192, kSmemBytesD256, stream>>>(tm_k, tm_v, tm_o, kp);
+  kernel<<<kp.order.slots, 192, kSmemBytesD256, stream>>>(tm_k, tm_v, tm_o, kp);
   err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("head_dim 256 forward: launch failed: %s", cudaGetErrorString(err));

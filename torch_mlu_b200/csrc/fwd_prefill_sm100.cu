@@ -29,6 +29,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "block_order.cuh"
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
@@ -68,7 +69,8 @@ constexpr uint32_t kBarPFull = kBarSFull + 16;             // 2 tiles x 2 halves
 constexpr uint32_t kBarOFull = kBarPFull + 32;             // 2
 constexpr uint32_t kBarOFree = kBarOFull + 16;             // 2: the epilogue has read O_t (persistent loop)
 constexpr uint32_t kBarQFree = kBarOFree + 16;             // the unit's last QK^T has read the Q tiles
-constexpr uint32_t kBarUnitFull = kBarQFree + 8;           // kUnitRing: the scheduler has written the entry
+constexpr uint32_t kBarClaim = kBarQFree + 8;              // the issuer is kClaimAhead blocks from the end of its unit
+constexpr uint32_t kBarUnitFull = kBarClaim + 8;           // kUnitRing: the scheduler has written the entry
 constexpr uint32_t kBarUnitEmpty = kBarUnitFull + 16;      // kUnitRing: every reader has copied the entry
 constexpr uint32_t kBarStageFree = kBarUnitEmpty + 16;     // 2: the warpgroup's staging buffer may be rewritten
 constexpr uint32_t kBarStageFull = kBarStageFree + 16;     // 2: all four warps have written their rows
@@ -100,8 +102,7 @@ struct FwdKernelParams {
   const uint16_t* bias;
   int64_t bias_batch_stride, bias_head_stride, bias_row_stride;
   float inv_scale;  // 1 / softmax_scale: the bias joins the raw scores as bias / scale
-  int num_m_blocks, num_bh, heads_per_wave, num_slots;  // work-unit order, see decode_unit()
-  int lazy_from;  // slot from which units are claimed late, see the unit scheduler
+  BlockOrder order;  // of the work units
   float scale_log2;
   int is_causal;
 #ifdef SDPA_FWD_STAMPS
@@ -155,18 +156,11 @@ struct Unit {
 };
 static_assert(sizeof(Unit) == 64, "Unit is copied through shared memory as four 16-byte words");
 
-// Unit order. (batch, head) pairs are taken in groups of `heads_per_wave` whose K/V fit L2
-// together; inside a group the 256-row units go heaviest first (largest m_block, i.e. most causal
-// key blocks) across all its heads. Returns false for padding slots and units without rows.
+// Returns false for padding slots and units without rows.
 __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, Unit& u) {
-  const int per_group = p.heads_per_wave * p.num_m_blocks;
-  const int grp = slot / per_group;
-  const int w = slot - grp * per_group;
-  const int size = min(p.heads_per_wave, p.num_bh - grp * p.heads_per_wave);
-  const int rank = w / size;
-  const int bh = grp * p.heads_per_wave + (w - rank * size);
-  if (rank >= p.num_m_blocks) return false;  // padding slots of a short last group
-  const int m_block = p.num_m_blocks - 1 - rank;
+  int rank, bh;
+  if (!block_of_slot(p.order, slot, rank, bh)) return false;
+  const int m_block = p.order.ranks - 1 - rank;
   u.b = bh / p.heads_q;
   u.h = bh - u.b * p.heads_q;
   u.hk = u.h / p.kv_group;
@@ -206,6 +200,9 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
 // counts, so the loads, the first QK^T and the softmax of the next unit start while this unit's
 // epilogue runs.
 constexpr int kUnitRing = 2;
+// A unit is claimed when the one in front of it has this many key blocks left: late, since a unit that a busy CTA has claimed is one that
+// an idle CTA cannot take, and early enough for the claim (atomic, decode, about 1500 cycles) to pass before the Q tiles are free.
+constexpr int kClaimAhead = 3;
 constexpr uint32_t kUnitReaders = 10;  // producer + issuer + 8 softmax warps
 
 // Copies ring entry (n mod kUnitRing) into `u` and releases it. All lanes of the calling warp (or its
@@ -304,6 +301,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bar + kBarStageFree + 8 * t, 1);
       mbar_init(bar + kBarStageFull + 8 * t, 4);
     }
+    mbar_init(bar + kBarClaim, 1);
     for (int e = 0; e < kUnitRing; ++e) {
       mbar_init(bar + kBarUnitFull + 8 * e, 1);
       mbar_init(bar + kBarUnitEmpty + 8 * e, kUnitReaders);
@@ -407,6 +405,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (n_iter == 1) umma_commit(bar + kBarQFree);
           FWD_STAMP(2, ucnt, 2);
           for (int j = 0; ok && j < n_iter; ++j) {
+            if (j == max(0, n_iter - kClaimAhead)) mbar_arrive(bar + kBarClaim);
             const uint32_t iv = kv_base + 2 * j + 1;  // ring position of V(j)
             const uint32_t ik = kv_base + 2 * j + 2;  // ring position of K(j+1)
             const uint32_t v_smem = kv_smem(iv);
@@ -463,33 +462,27 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       // ------------------------------------------------------------------ unit scheduler
       if (lane == 0) {
         bool ok = true;
-        // Claiming ahead hides the claim (atomic + decode) and lets the producer prefetch the next Q
-        // tiles, but near the end of the list a unit claimed early by a busy CTA is a unit an idle CTA
-        // cannot take. For the last two rounds of the grid (`lazy_from`) the scheduler therefore claims late: only
-        // once the last QK^T of the unit it published before has been issued (the Q-free barrier).
-        bool lazy = false;
-        bool last_runs = false;  // the unit published last has key blocks (and so a Q-free phase)
-        uint32_t ucnt = 0;       // such units published so far
+        uint32_t runs = 0;      // units published so far that have key blocks
+        bool last_runs = false;  // the one published last is among them
         bool own_taken = false;  // without a counter: the CTA's own slot has been claimed
         for (uint32_t n = 0; ok; ++n) {
           const uint32_t e = n % kUnitRing;
           ok = mbar_wait(bar + kBarUnitEmpty + 8 * e, ((n / kUnitRing) & 1u) ^ 1u, abort_flag);
-          if (ok && lazy && last_runs) ok = mbar_wait(bar + kBarQFree, (ucnt - 1) & 1, abort_flag);
+          if (ok && last_runs) ok = mbar_wait(bar + kBarClaim, (runs - 1) & 1, abort_flag);
           if (!ok) break;
           Unit u;
           u.done = 1;
           for (;;) {
             const int slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
-                             : own_taken               ? p.num_slots
+                             : own_taken               ? p.order.slots
                                                        : static_cast<int>(blockIdx.x);
             own_taken = true;
-            if (slot >= p.num_slots) break;
-            if (slot >= p.lazy_from) lazy = true;
+            if (slot >= p.order.slots) break;
             if (decode_unit(p, slot, u)) break;  // padding slots and row-less units are skipped
             u.done = 1;
           }
           last_runs = !u.done && u.n_iter > 0;
-          if (last_runs) ++ucnt;
+          if (last_runs) ++runs;
           write_unit(smem, e, u);
           mbar_arrive(bar + kBarUnitFull + 8 * e);  // release: the entry is visible to whoever sees the phase
           if (u.done) break;
@@ -885,8 +878,6 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
     set_error("prefill: cudaFuncSetAttribute(%u bytes smem): %s", kSmemBytes, cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
   }
-  kp.num_m_blocks = (p.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM);
-  kp.num_bh = p.batch * p.heads_q;
   const int sms = sm_count();
   if (sms <= 0) {
     set_error("prefill: cannot read the SM count of the current device");
@@ -896,18 +887,10 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   const int usable = sms - p.sm_margin > 1 ? sms - p.sm_margin : 1;
   // K+V bytes one query head streams, shared by the heads of its GQA group
   const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  const double units = varlen ? packed_units(p, 2 * kBlockM) : 0;
-  kp.heads_per_wave = varlen && one_forward_group(kv_row_bytes * p.total_k * p.heads_kv, kp.num_bh, p.is_causal != 0, p.max_seqlen_q, units,
-                                                  static_cast<double>(kp.num_bh) * kp.num_m_blocks, usable)
-                          ? kp.num_bh
-                          : heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, kp.num_bh);
-  const int groups = (kp.num_bh + kp.heads_per_wave - 1) / kp.heads_per_wave;
-  kp.num_slots = groups * kp.heads_per_wave * kp.num_m_blocks;
-  dim3 grid(kp.num_slots < usable ? kp.num_slots : usable, 1, 1);
-  // A packed call of up to two rounds of units claims late throughout: its slots are partly empty, so the last two rounds of slots say nothing
-  // about the units (3 sequences of 193 to 769 tokens, 32 heads, D128 35.0 us in one group, 26.2 so; 6 of 390 to 1117, 16/4, D64 35.6, 25.0; 6 of
-  // 309 to 2900, 8/1, unmasked 117, 88). With more units that costs more than it gives (8 of 306 to 1102, 16/16, D64 42.1, 46.2).
-  kp.lazy_from = varlen && units <= 2.0 * usable ? 0 : kp.num_slots - 2 * static_cast<int>(grid.x);
+  const int heads = p.batch * p.heads_q, ranks = (p.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM);
+  kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes),
+                         p.is_causal ? tail_ranks(ranks, kv_row_bytes * (2 * kBlockM) * p.batch * p.heads_kv) : 0);
+  dim3 grid(kp.order.slots < usable ? kp.order.slots : usable, 1, 1);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
   // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
   // cleared already.) Not for two units per CTA, dealt out by index: alone that is faster (B8 H12 L512 D64 unmasked, eager, 22.6 us against
@@ -915,7 +898,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   // B5 H8 L1024 D128 57.4 against 41.0), and units are not alike where the last one of a head has a single tile (B8 H12 L300 D128 24.6
   // against 23.0).
   kp.unit_counter = nullptr;
-  if (kp.num_slots > usable) {
+  if (kp.order.slots > usable) {
     kp.unit_counter = static_cast<uint32_t*>(workspace) + 1;
     if (p.device_status != nullptr && (err = cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, stream)) != cudaSuccess) {
       set_error("prefill: clearing the unit counter failed: %s", cudaGetErrorString(err));

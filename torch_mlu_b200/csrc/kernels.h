@@ -36,10 +36,29 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace
 
 // Kernels take (batch, head) pairs in groups whose streamed tensors stay in L2 together, and the blocks of a group heaviest first.
 // Heads per group, from the bytes that one head streams (packed: at the longest length).
-inline int heads_per_l2_group(double bytes_per_head, int num_heads) {
-  int n = static_cast<int>((48.0 * 1024 * 1024) / bytes_per_head);
+inline int heads_per_l2_group(double bytes_per_head, int num_heads, double group_bytes = 48.0 * 1024 * 1024) {
+  int n = static_cast<int>(group_bytes / bytes_per_head);
   n = n > 32 ? 32 : (n < 1 ? 1 : n);
   return n > num_heads ? num_heads : n;
+}
+
+// Forward: smaller groups, so that more CTAs read the same K and V at a time (B4 H32 L4096 D128 causal 539 us with groups of 48 MB, 531 of 32,
+// 527 of 16; unmasked, 16 heads 503, 497, 491; B2 H32 L8192 causal 1022, 998, 996; but B2 H16 L3000 causal 89.1, 88.6, 91.7;
+// head_dim 256, B4 H16 L4096 causal 544, 534).
+constexpr double kForwardGroupBytes = 32.0 * 1024 * 1024;
+
+// Forward under a causal mask, up to head_dim 128: how many of the lightest ranks of blocks come behind all groups, over all heads. With whole
+// groups to the end the CTAs that had taken the last group's heavy blocks ran on alone: the longest-running CTA against the mean 280 to 233
+// thousand cycles at B8 H16 L2048 D128, 911 to 825 at B4 H32 L4096; now 240 to 231 and 821 to 806. Calls over seconds, with the late claims of
+// the forward: these two 172 us -> 166 and 568 -> 533, B2 H16 L3000 101 -> 88.6, B4 H32/8 L1000 57.7 -> 51.4, 9 packed sequences of 29 to 2820
+// tokens, 8/1, D64 92.8 -> 72.8. As many as half, and as stay in L2 together, since heads do not share K and V at a time there: `bytes_per_rank`
+// are those that one more rank makes all heads stream (limit of 128 MB: 555 us at L4096, 64: 539, 32: 538; B8 H16 L2048 170, 169, 166). Not
+// where the hardware deals out CTAs of single blocks: it claims as late as can be, and the kernel ends within 2 % of the mean CTA as it is
+// (head_dim 256 forward, B4 H16 L4096 534 without, 533 with; B8 H16 L644 80, 82; backward, step of B4 H16 L1024 D256 227, 231, of B8 H12 L1000
+// D64 135, 159).
+inline int tail_ranks(int ranks, double bytes_per_rank) {
+  const int fit = static_cast<int>(32.0 * 1024 * 1024 / bytes_per_rank);
+  return fit < ranks / 2 ? fit : ranks / 2;
 }
 
 // Packed backward under a causal mask, from what all sequences together stream: the longest one says little about it, and in fewer and
@@ -52,24 +71,6 @@ inline int heads_per_l2_group(double bytes_per_head, int num_heads) {
 inline int heads_per_packed_group(double all_bytes, int num_heads) {
   const int groups = 1 + static_cast<int>(all_bytes / (112.0 * 1024 * 1024));
   return (num_heads + groups - 1) / groups;
-}
-
-// Units that the sequences of a packed forward hold, with `rows` queries each: half of a last unit per sequence on average. The lengths are on
-// the device.
-inline double packed_units(const sdpa_b200_params& p, int rows) {
-  return p.heads_q * (p.total_q / static_cast<double>(rows) + 0.5 * p.batch);
-}
-
-// Packed forward. Its dynamic units leave no such tail, but under a causal mask one group is the faster order where K and V are at most
-// 48 MB (16 sequences of 100 to 1000 tokens, 16/16 heads, D64: 56 us, by the longest 64; 8 of 200 to 2000, 16/4, D128: 109, 118; 139 MB, 16 of
-// 512 to 4096: 958, 907; 52 to 92 MB level). Not without a mask (6 of 300 to 2900, 8/1: 128, 117; 8 of 200 to 2000, 16/4: 190, 184), not
-// for two 256-row units at most (32 of 16 to 300, 32/8: 56.2, 55.0; 5 of 134 to 282, 16/4: 15.5, 14.6; but one unit each, without the slots that
-// fill up a last group: 6 of 62 to 234, 12/12, D64 10.8, 12.1), and not where slots without a unit, which one group puts in front, are many and
-// rounds few (9 of 29 to 2820, 8/1, D64, 424 units in 864 slots: 89, 76; 13 of 128 to 888, 16/16, 480 in 832: 43.1, 41.5; but 30 of 64 to 4000, 8/1,
-// fourteen rounds: 445, 464).
-inline bool one_forward_group(double all_bytes, int num_heads, bool causal, int longest, double units, double slots, int sms) {
-  return causal && all_bytes <= 48.0 * 1024 * 1024 && (longest > 512 || (longest <= 256 && num_heads <= sms)) &&
-         (units <= 2.0 * sms || units >= 8.0 * sms || units >= 0.6 * slots);
 }
 
 // Number of SMs of the current device (cached per device), <= 0 on error.
