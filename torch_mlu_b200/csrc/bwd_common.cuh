@@ -110,12 +110,6 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src,
                : "memory");
 }
 
-// A grid launched with programmatic stream serialization may start before the grid in front of it has finished. This
-// wait returns once that grid has completed and its stores are visible; a CTA that executes it before it exits keeps its
-// own grid from completing first, so whatever follows in the stream is ordered behind BOTH grids, as it would be without
-// the overlap. (A no-op for a grid launched the ordinary way.)
-__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Four consecutive per-query values from shared memory. One 16-byte read; in the dropout instances four reads, because there
 // the quads (and packed arithmetic on them) spill: fused backward, when it served head_dim 128, of B8 H16 L2048 causal 446 -> 440 us without dropout,
 // but 522 -> 542 with it.

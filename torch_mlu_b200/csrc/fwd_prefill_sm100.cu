@@ -26,7 +26,6 @@
 // (only when a row maximum grows by more than 2^8), by the softmax thread that owns the row.
 #include <cuda_bf16.h>
 
-#include <cstdlib>
 #include <type_traits>
 
 #include "block_order.cuh"
@@ -105,22 +104,7 @@ struct FwdKernelParams {
   BlockOrder order;  // of the work units
   float scale_log2;
   int is_causal;
-#ifdef SDPA_FWD_STAMPS
-  float* stamps;  // [role 4][unit 16][event 8] SM cycles since CTA start, CTA 0 only
-#endif
 };
-
-// Profiling builds (-DSDPA_FWD_STAMPS) time-stamp events of CTA 0's first units; role 0/1 = lane 0 of
-// the first warp of each softmax warpgroup, 2 = MMA issuer, 3 = TMA producer.
-#ifdef SDPA_FWD_STAMPS
-#define FWD_STAMP(role, unit, ev)                                                                  \
-  do {                                                                                             \
-    if (p.stamps != nullptr && blockIdx.x == 0 && (unit) < 16)                                     \
-      p.stamps[((role) * 16 + (unit)) * 8 + (ev)] = static_cast<float>(clock64() - t_start);        \
-  } while (0)
-#else
-#define FWD_STAMP(role, unit, ev) do {} while (0)
-#endif
 
 template <bool kF16>
 constexpr uint32_t kIdescQK = umma_idesc_16(kBlockM, kBlockN, false, false, kF16);
@@ -191,9 +175,20 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
   return true;
 }
 
+// The next unit of the list (u.done: there is none). Without a counter every CTA has the slot of its own index.
+__device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first, Unit& u) {
+  for (;; first = false) {
+    const int slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
+                     : first                   ? static_cast<int>(blockIdx.x)
+                                               : p.order.slots;
+    u.done = slot >= p.order.slots;
+    if (u.done || decode_unit(p, slot, u)) return;  // padding slots and row-less units are skipped
+  }
+}
+
 // Persistent kernel: gridDim.x CTAs (one per SM) take units off a global counter in list order, which
 // balances the uneven causal units the way the hardware block scheduler would. Warp 10 is the unit
-// scheduler: it claims the next slot, decodes it (integer divisions, cu_seqlens loads) off everyone's
+// scheduler: it claims the next slot (the first one is the producer's), decodes it (integer divisions, cu_seqlens loads) off everyone's
 // critical path and publishes the Unit through a two-entry shared-memory ring; the producer, the MMA
 // issuer and the eight softmax warps each copy the entry and release it at once, so the scheduler
 // runs one unit ahead. Barriers, TMEM and the K/V ring live across units; every role keeps running use
@@ -285,7 +280,38 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemAbort);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemTmemPtr);
 
-  if (threadIdx.x == 0) {
+  // The kernel may have been launched under the tail of the grid in front of it (launch_fwd_prefill): set-up and, for dense tensors, the first
+  // unit's coordinates come before the wait for that grid, everything that reads or writes global memory behind it. The producer thread
+  // does all of this and starts the first loads at once, so that they run under the TMEM allocation and the other warps' set-up.
+  if (threadIdx.x == 0) launch_dependents();
+  const bool producer = warp == kProducerWarp && elect_one();
+  uint32_t preloaded = 0;  // producer: ring tiles of the first unit that have been asked for
+  auto load_q = [&](int q_row, int h, int bcoord) {
+    constexpr uint32_t kLoadBytes = kBlockN * kD * 2;  // bytes one Q/K/V tile brings in
+    mbar_arrive_expect_tx(bar + kBarQFull, 2 * kLoadBytes);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const uint32_t dst = base + kSmemQ + t * kTileBytes;
+      tma_load_4d(dst, &tm_q, bar + kBarQFull, 0, q_row + t * kBlockM, h, bcoord);
+      if (kD > 64) tma_load_4d(dst + kHalfBytes, &tm_q, bar + kBarQFull, 64, q_row + t * kBlockM, h, bcoord);
+    }
+  };
+  // tile `cnt` of the ring, tile i of its unit: K(i/2) if even, V(i/2) if odd
+  auto load_kv = [&](uint32_t cnt, int i, int k_row, int hk, int bcoord) {
+    constexpr uint32_t kLoadBytes = kBlockN * kD * 2;
+    const uint32_t s = cnt % kStages;
+    const uint32_t full = bar + kBarKVFull + 8 * s;
+    const uint32_t dst = base + kSmemKV + s * kTileBytes;
+    const CUtensorMap* tm = (i & 1) ? &tm_v : &tm_k;
+    const int row = k_row + (i >> 1) * kBlockN;
+    mbar_arrive_expect_tx(full, kLoadBytes);
+    tma_load_4d(dst, tm, full, 0, row, hk, bcoord);
+    if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, full, 64, row, hk, bcoord);
+  };
+  if (producer) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
     mbar_init(bar + kBarQFull, 1);
     mbar_init(bar + kBarQFree, 1);
     for (int s = 0; s < kStages; ++s) {
@@ -308,29 +334,34 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
     *abort_flag = 0;
     fence_mbar_init();
+    const bool packed = p.cu_q != nullptr;  // the lengths are in memory
+    if (packed) wait_for_previous_grid();
+    Unit u;
+    claim_unit(p, true, u);
+    write_unit(smem, 0, u);
+    mbar_arrive(bar + kBarUnitFull);
+    if (!packed) wait_for_previous_grid();
+    if (!u.done && u.n_iter > 0) {
+      load_q(u.m0 + u.q_off, u.h, u.bcoord);
+      for (; preloaded < kStages && preloaded < 2u * u.n_iter; ++preloaded) load_kv(preloaded, preloaded, u.k_off, u.hk, u.bcoord);
+    }
   }
   if (warp == 0) {
     __syncwarp();
     tmem_alloc(base + kSmemBar + kSmemTmemPtr, 512);
     tmem_relinquish();
   }
+  wait_for_previous_grid();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-#ifdef SDPA_FWD_STAMPS
-  const long long t_start = clock64();
-#endif
 
   if (warp >= 8) {
     reg_decrease<kRegsOther>();
     if (warp == kProducerWarp) {
       // ------------------------------------------------------------------ TMA producer
-      if (elect_one()) {
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_k);
-        tma_prefetch_desc(&tm_v);
-        constexpr uint32_t kLoadBytes = kBlockN * kD * 2;  // bytes one Q/K/V tile brings in
+      if (producer) {
         uint32_t kv_cnt = 0;  // K/V tiles loaded so far (ring position)
         uint32_t ucnt = 0;    // units started so far
         bool ok = true;
@@ -339,33 +370,19 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           ok = read_unit_coords(smem, bar, n, abort_flag, q_row, k_row, h, hk, bcoord, n_iter, done);
           if (!ok || done) break;
           if (n_iter == 0) continue;
-          FWD_STAMP(3, ucnt, 0);
-          // the Q tiles are free once the last QK^T of the previous unit has read them
-          if (ucnt > 0) ok = mbar_wait(bar + kBarQFree, (ucnt - 1) & 1, abort_flag);
-          if (!ok) break;
-          FWD_STAMP(3, ucnt, 1);
-          mbar_arrive_expect_tx(bar + kBarQFull, 2 * kLoadBytes);
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const uint32_t dst = base + kSmemQ + t * kTileBytes;
-            tma_load_4d(dst, &tm_q, bar + kBarQFull, 0, q_row + t * kBlockM, h, bcoord);
-            if (kD > 64) tma_load_4d(dst + kHalfBytes, &tm_q, bar + kBarQFull, 64, q_row + t * kBlockM, h, bcoord);
-          }
-          for (int i = 0; i < 2 * n_iter; ++i, ++kv_cnt) {  // K(i/2) if even, V(i/2) if odd
-            const uint32_t s = kv_cnt % kStages;
-            const uint32_t use = kv_cnt / kStages;
-            ok = mbar_wait(bar + kBarKVEmpty + 8 * s, (use & 1u) ^ 1u, abort_flag);
+          if (n > 0) {
+            // the Q tiles are free once the last QK^T of the previous unit has read them
+            if (ucnt > 0) ok = mbar_wait(bar + kBarQFree, (ucnt - 1) & 1, abort_flag);
             if (!ok) break;
-            const uint32_t full = bar + kBarKVFull + 8 * s;
-            const uint32_t dst = base + kSmemKV + s * kTileBytes;
-            const CUtensorMap* tm = (i & 1) ? &tm_v : &tm_k;
-            const int row = k_row + (i >> 1) * kBlockN;
-            mbar_arrive_expect_tx(full, kLoadBytes);
-            tma_load_4d(dst, tm, full, 0, row, hk, bcoord);
-            if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, full, 64, row, hk, bcoord);
-            if (i == 0) FWD_STAMP(3, ucnt, 2);
+            load_q(q_row, h, bcoord);
           }
-          FWD_STAMP(3, ucnt, 3);
+          for (int i = n == 0 ? preloaded : 0; i < 2 * n_iter; ++i) {
+            const uint32_t cnt = kv_cnt + i;
+            ok = mbar_wait(bar + kBarKVEmpty + 8 * (cnt % kStages), ((cnt / kStages) & 1u) ^ 1u, abort_flag);
+            if (!ok) break;
+            load_kv(cnt, i, k_row, hk, bcoord);
+          }
+          kv_cnt += 2 * n_iter;
           ++ucnt;
         }
         drain_after_abort(abort_flag);
@@ -387,9 +404,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           ok = read_unit_counts(smem, bar, n, abort_flag, nblk0, nblk1, n_iter, done);
           if (!ok || done) break;
           if (n_iter == 0) continue;
-          FWD_STAMP(2, ucnt, 0);
           ok = mbar_wait(bar + kBarQFull, ucnt & 1, abort_flag);
-          FWD_STAMP(2, ucnt, 1);
           ok = ok && kv_full(kv_base);
           if (!ok) break;
           tc_fence_after_sync();
@@ -403,7 +418,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           }
           kv_release(kv_base);
           if (n_iter == 1) umma_commit(bar + kBarQFree);
-          FWD_STAMP(2, ucnt, 2);
           for (int j = 0; ok && j < n_iter; ++j) {
             if (j == max(0, n_iter - kClaimAhead)) mbar_arrive(bar + kBarClaim);
             const uint32_t iv = kv_base + 2 * j + 1;  // ring position of V(j)
@@ -422,7 +436,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
                 const uint32_t par = (cnt + j) & 1;
                 // the first PV of a unit overwrites O_t: the previous unit's epilogue must have read it
                 if (j == 0 && ucnt > 0 && !mbar_wait(bar + kBarOFree + 8 * t, (ucnt - 1) & 1, abort_flag)) return false;
-                if (j == 0 && t == 0) FWD_STAMP(2, ucnt, 3);
                 // P arrives in two halves so the first four MMAs overlap the second half's exponentials
                 if (!mbar_wait(bar + kBarPFull + 16 * t, par, abort_flag)) return false;
                 tc_fence_after_sync();
@@ -451,7 +464,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
               if (j + 2 == n_iter) umma_commit(bar + kBarQFree);  // that was the unit's last QK^T
             }
           }
-          FWD_STAMP(2, ucnt, 4);
           cnt0 += nblk0;
           cnt1 += nblk1;
           kv_base += 2 * n_iter;
@@ -462,30 +474,23 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       // ------------------------------------------------------------------ unit scheduler
       if (lane == 0) {
         bool ok = true;
-        uint32_t runs = 0;      // units published so far that have key blocks
-        bool last_runs = false;  // the one published last is among them
-        bool own_taken = false;  // without a counter: the CTA's own slot has been claimed
-        for (uint32_t n = 0; ok; ++n) {
+        // unit 0 has been published by the producer
+        const int* first = reinterpret_cast<const int*>(smem + kSmemBar + kSmemUnits);
+        bool last_runs = !first[13] && first[12] > 0;  // the unit published last has key blocks
+        uint32_t runs = last_runs;                     // such units so far
+        bool done = first[13] != 0;
+        for (uint32_t n = 1; ok && !done; ++n) {
           const uint32_t e = n % kUnitRing;
           ok = mbar_wait(bar + kBarUnitEmpty + 8 * e, ((n / kUnitRing) & 1u) ^ 1u, abort_flag);
           if (ok && last_runs) ok = mbar_wait(bar + kBarClaim, (runs - 1) & 1, abort_flag);
           if (!ok) break;
           Unit u;
-          u.done = 1;
-          for (;;) {
-            const int slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
-                             : own_taken               ? p.order.slots
-                                                       : static_cast<int>(blockIdx.x);
-            own_taken = true;
-            if (slot >= p.order.slots) break;
-            if (decode_unit(p, slot, u)) break;  // padding slots and row-less units are skipped
-            u.done = 1;
-          }
+          claim_unit(p, false, u);
+          done = u.done;
           last_runs = !u.done && u.n_iter > 0;
           if (last_runs) ++runs;
           write_unit(smem, e, u);
           mbar_arrive(bar + kBarUnitFull + 8 * e);  // release: the entry is visible to whoever sees the phase
-          if (u.done) break;
         }
       }
     }
@@ -552,7 +557,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
 
       float m_run = neg_inf;
       float l_run = 0.f;
-      if (row_in_tile == 0) FWD_STAMP(t, ucnt, 0);
       const uint16_t* bias_row = nullptr;  // this row's bias values, or null for a row past the sequence
       if constexpr (kBias) {
         if (row < u.len_q)
@@ -592,7 +596,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
         // warp-uniform, because the arrivals below are made by one lane on behalf of its warp
         ok = __all_sync(0xffffffffu, mbar_wait(bar_s, par, abort_flag));
         if (!ok) break;
-        if (row_in_tile == 0 && j == 0) FWD_STAMP(t, ucnt, 1);
         tc_fence_after_sync();
 
         float s[kBlockN];
@@ -703,14 +706,12 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
         if (lane == 0) mbar_arrive(bar_p + 8);
       }
       if (!ok) break;
-      if (row_in_tile == 0) FWD_STAMP(t, ucnt, 2);
 
       // ---- epilogue: O / l -> 16-bit, LSE
       if (my_blocks > 0) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar_o, (cnt + my_blocks - 1) & 1, abort_flag));
         if (!ok) break;
       }
-      if (row_in_tile == 0) FWD_STAMP(t, ucnt, 3);
       const int u_q_off = info[0], u_h = info[1], u_b = info[2], u_len_q = info[3];
       if (row_lo < u_len_q) {
         tc_fence_after_sync();
@@ -736,7 +737,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar + kBarOFree + 8 * t);
-        if (row_in_tile == 0) FWD_STAMP(t, ucnt, 4);
         const bool valid = row < u_len_q;
         // A whole 128-row tile goes out as TMA stores (64 columns at a time through a 16 KB staging
         // buffer per warpgroup): asynchronous and fully coalesced. Dense tensors are clipped by the
@@ -789,7 +789,6 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
         __syncwarp();
         if (lane == 0) mbar_arrive(bar + kBarOFree + 8 * t);
       }
-      if (row_in_tile == 0) FWD_STAMP(t, ucnt, 5);
       cnt += my_blocks;
       ++ucnt;
     }
@@ -856,12 +855,6 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.inv_scale = 1.f / p.softmax_scale;
   kp.scale_log2 = p.softmax_scale * 1.4426950408889634f;
   kp.is_causal = p.is_causal;
-#ifdef SDPA_FWD_STAMPS
-  {
-    const char* env = getenv("SDPA_FWD_STAMPS_PTR");
-    kp.stamps = env ? reinterpret_cast<float*>(strtoull(env, nullptr, 10)) : nullptr;
-  }
-#endif
 
   auto pick = [&](auto drop_tag, auto bias_tag) {
     constexpr bool kDrop = decltype(drop_tag)::value;
@@ -905,8 +898,10 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
       return SDPA_B200_LAUNCH_FAILED;
     }
   }
-  kernel<<<grid, kNumThreads, kSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_o, kp);
-  err = cudaGetLastError();
+  // Without the clearing launch in front, the grid may start under the tail of the one before it in the stream, whichever that is. Calls back
+  // to back, with the first unit's loads asked for before the set-up barrier: B2 H8 L256 D64 10.2 us -> 7.5, B1 H32/8 L300 D128 12.3 -> 10.1, 3
+  // packed sequences of 100 to 200 tokens, D64 10.7 -> 8.6.
+  err = launch_behind(kernel, grid, kNumThreads, kSmemBytes, stream, kp.unit_counter == nullptr && p.device_status != nullptr, tm_q, tm_k, tm_v, tm_o, kp);
   if (err != cudaSuccess) {
     set_error("prefill: launch failed: %s", cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;

@@ -138,6 +138,16 @@ __device__ __forceinline__ void reg_decrease() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
 
+// A grid launched with programmatic stream serialization may start before the grid in front of it has finished. This
+// wait returns once that grid has completed and its stores are visible; a CTA that executes it before it exits keeps its
+// own grid from completing first, so whatever follows in the stream is ordered behind BOTH grids, as it would be without
+// the overlap. (A no-op for a grid launched the ordinary way.)
+__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next grid in the stream start, if it is launched so, once every CTA of this one has said this (or left). It finds nothing
+// that this grid writes before its own wait.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // two fp32 -> packed bf16x2 (lo in the low half), round to nearest even
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;
