@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from oracle import sdpa_oracle as orc
-from torch_mlu_b200 import ops, workloads
+from torch_mlu_b200 import _cabi, ops, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -46,6 +46,31 @@ def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D):
     dev = cuda_device
     out, lse = ops.decode_attention(q.to(dev), k.to(dev), v.to(dev))
     assert ops.device_status() == 0
+    o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=False)
+    orc.assert_close_bf16(out, o_ref, "out")
+    orc.assert_close_lse(lse, l_ref)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Lk,D,launches", [
+    (1, 32, 8, 1000, 128, 1),   # clusters of 8, two tiles each, the last one short
+    (1, 20, 2, 321, 64, 1),     # clusters of 4 over six tiles: the last CTA has none; ten heads: both fragment row halves
+    (2, 40, 1, 600, 128, 1),    # the same with head chunks of 16, 16 and 8
+    (12, 12, 12, 100, 128, 1),  # clusters of 2
+    (1, 32, 8, 5000, 128, 2),   # too long for a cluster
+    (30, 8, 8, 200, 64, 1),     # a nearly full wave of whole units
+    (19, 8, 8, 130, 128, 2),    # half a wave of them
+    (60, 16, 8, 130, 64, 1),    # two waves of whole units
+    (68, 16, 16, 100, 64, 2),   # four waves of two tiles
+    (35, 8, 8, 4097, 64, 1),    # several waves of clusters, 33 and 32 tiles each
+])
+def test_decode_without_a_merge_kernel(cuda_device, native_lib, B, Hq, Hkv, Lk, D, launches):
+    """Each side of the rule that chooses whole units, clusters or equal shares. Tolerances as above; the kernels are counted so that
+    every case is on the side that it stands for."""
+    q, k, v = rand((B, Hq, 1, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3)
+    dev = cuda_device
+    before = _cabi.launch_count()
+    out, lse = ops.decode_attention(q.to(dev), k.to(dev), v.to(dev))
+    assert ops.device_status() == 0 and _cabi.launch_count() - before == launches
     o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=False)
     orc.assert_close_bf16(out, o_ref, "out")
     orc.assert_close_lse(lse, l_ref)

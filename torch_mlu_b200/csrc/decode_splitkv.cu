@@ -7,7 +7,8 @@
 // mma.sync.m16n8k16, so K/V bytes are read once per group. The keys of all units, cut into tiles of 64, form one list that is
 // dealt out in equal contiguous shares to a grid that fits the GPU in one wave (two CTAs per SM): every SM streams the same
 // number of bytes whatever the batch, the number of heads and the length are, and the loads of a CTA run on across unit
-// boundaries. (One CTA per (unit, split) left the last wave nearly empty - 512 CTAs on 444 places ran at 4.3 TB/s - and paid
+// boundaries. Where they fit as well without, whole units or clusters of CTAs that share one and merge their parts through shared memory save the
+// second launch (cluster_size). (One CTA per (unit, split) left the last wave nearly empty - 512 CTAs on 444 places ran at 4.3 TB/s - and paid
 // the pipeline's fill and the merge of four warps once per split.) A unit whose tiles belong to several CTAs leaves partial
 // (O, lse) rows in the workspace, at most two per CTA, and a second kernel merges them.
 //
@@ -19,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.h"
 #include "ptx_sm100.cuh"
@@ -32,6 +34,7 @@ constexpr int kKeysPerStep = 16;                        // keys one warp handles
 constexpr int kTileKeys = kDecWarps * kKeysPerStep;     // 64
 constexpr int kMaxSplits = 128;
 constexpr int kCtasPerSm = 2;
+constexpr int kMaxCluster = 8;
 constexpr uint32_t kBoxRowBytes = 128;                  // one 64-column box row
 constexpr uint32_t kBoxBytes = kKeysPerStep * kBoxRowBytes;
 
@@ -130,6 +133,22 @@ __device__ __forceinline__ void mma_rows(float (&c)[4], const uint32_t (&a)[4], 
   else mma_16816_lo<kF16>(c[0], c[1], a[0], a[2], b0, b1);
 }
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared memory of CTA `rank` of the cluster, at this CTA's address `addr`
+__device__ __forceinline__ float cluster_ld_f32(uint32_t addr, int rank) {
+  float v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 cluster_ld_f32x2(uint32_t addr, int rank) {
+  float2 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %2, %3;\n\tld.shared::cluster.v2.f32 {%0, %1}, [a];\n\t}\n"
+               : "=f"(v.x), "=f"(v.y) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float quad_max(float x) {
   x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
   x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
@@ -157,7 +176,7 @@ __host__ __device__ constexpr uint32_t decode_smem_bytes() {
 }
 
 // kHi: a unit has more than 8 query heads, so fragment rows 8-15 are in use too.
-template <bool kHi, int kD, bool kF16>
+template <bool kHi, int kD, bool kF16, bool kCluster>
 __global__ void __launch_bounds__(kDecThreads, kCtasPerSm)
 decode_splitkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const DecodeParams p) {
   constexpr int kKSteps = kD / 16;   // MMAs over head_dim for Q K^T
@@ -170,6 +189,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   float* merge = reinterpret_cast<float*>(smem_raw + (base - raw_addr) + kDecWarps * kSt * kStageBytes);
+  // kCluster: this CTA's part, [16 heads][kD] and their log2 sums, in the ring, which is idle by then
+  float* cl_o = reinterpret_cast<float*>(smem_raw + (base - raw_addr));
+  float* cl_lse = cl_o + 16 * kD;
+  static_assert(16 * (kD + 1) * 4 <= kDecWarps * kSt * kStageBytes, "a part does not fit the ring");
   const uint32_t bars = smem_u32(merge + (kDecWarps - 1) * kMergeFloats);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(merge + (kDecWarps - 1) * kMergeFloats + kDecWarps * kSt * 2);
 
@@ -430,7 +453,13 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         const float l = hi ? l_hi : l_lo, mm = hi ? mm_hi : mm_lo;
         const float inv = (l > 0.f) ? 1.f / l : 0.f;
         const float lse2 = (l == 0.f) ? -INFINITY : mm + log2f(l);  // a NaN sum stays visible to the merge
-        if (whole) {
+        if constexpr (kCluster) {
+          float* dst = cl_o + r * kD + 2 * t;
+#pragma unroll
+          for (int nb = 0; nb < kNBlocks; ++nb)
+            *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(o[nb][2 * hi] * inv, o[nb][2 * hi + 1] * inv);
+          if (t == 0) cl_lse[r] = lse2;
+        } else if (whole) {
           uint16_t* dst = p.out + b * p.o_batch_stride + (head0 + r) * p.o_head_stride + 2 * t;
 #pragma unroll
           for (int nb = 0; nb < kNBlocks; ++nb)
@@ -447,8 +476,48 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       }
     }
   }
+  if constexpr (kCluster) {
+    // ---- merge over the cluster: every CTA takes a share of the columns of all parts, out of the others' shared memory
+    const int size = p.num_splits, rank = static_cast<int>(blockIdx.x) % size;
+    if (n_tiles == 0 && threadIdx.x < 16) cl_lse[threadIdx.x] = -INFINITY;
+    cluster_sync();
+    const int u = blockIdx.x / size, hc = u / p.chunks, b = hc / p.heads_kv;
+    const int head0 = (hc - b * p.heads_kv) * p.group + (u - hc * p.chunks) * 16;
+    const int nheads = min(16, p.group - (u - hc * p.chunks) * 16);
+    const int pairs = kD / 2 / size;  // column pairs of this CTA
+    for (int e = threadIdx.x; e < nheads * pairs; e += kDecThreads) {
+      const int r = e / pairs, col = 2 * (rank * pairs + e - r * pairs);
+      const uint32_t o_addr = smem_u32(cl_o + r * kD + col), lse_addr = smem_u32(cl_lse + r);
+      float ls[kMaxCluster];
+      float2 x[kMaxCluster];
+#pragma unroll
+      for (int j = 0; j < kMaxCluster; ++j) {
+        ls[j] = -INFINITY;
+        x[j] = make_float2(0.f, 0.f);
+        if (j < size) {
+          ls[j] = cluster_ld_f32(lse_addr, j);
+          if (ls[j] != -INFINITY) x[j] = cluster_ld_f32x2(o_addr, j);  // an empty part has written no row; a NaN part is not one
+        }
+      }
+      float m = ls[0];
+#pragma unroll
+      for (int j = 1; j < kMaxCluster; ++j) m = fmaxf(m, ls[j]);
+      float l = 0.f, v0 = 0.f, v1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < kMaxCluster; ++j) {
+        const float w = (ls[j] == -INFINITY) ? 0.f : exp2f(ls[j] - m);
+        l += w;
+        v0 += w * x[j].x;
+        v1 += w * x[j].y;
+      }
+      const float inv = (l > 0.f) ? 1.f / l : 0.f;
+      *reinterpret_cast<uint32_t*>(p.out + b * p.o_batch_stride + (head0 + r) * p.o_head_stride + col) = pack_16x2<kF16>(v0 * inv, v1 * inv);
+      if (col == 0) p.lse[static_cast<int64_t>(b) * p.heads_q + head0 + r] = (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : INFINITY;
+    }
+    cluster_sync();  // the others have read this CTA's part
+  }
   // a fixed split without keys (more splits than tiles): its merge partner finds an empty part
-  if (n_tiles == 0 && p.num_splits > 1) {
+  if (!kCluster && n_tiles == 0 && p.num_splits > 1) {
     const int u = blockIdx.x / p.num_splits, hc = u / p.chunks, b = hc / p.heads_kv;
     const int chunk = u - hc * p.chunks;
     if (static_cast<int>(threadIdx.x) < min(16, p.group - chunk * 16))
@@ -565,6 +634,35 @@ void plan_decode(const sdpa_b200_params& p, int sms, DecodeParams& d) {
   }
 }
 
+// CTAs per unit of a launch that needs no merge kernel: 1 (units stay whole), or a cluster of 2 to 8 that merges in shared memory; 0: equal shares
+// over one wave and the merge kernel, whose second launch costs about 3 us. Figures in us, calls back to back, H32/8 D128 unless said, equal
+// shares | so:
+//  * One wave of clusters, where its longest share is not much longer than an equal one: B1 Lk 1000 8.8 | 6.6, Lk 2000 8.7 | 7.9 (but Lk 4000 8.8 |
+//    10.1), B8 Lk 1000 10.2 | 8.8, Lk 4096 27.3 | 26.0, B16 Lk 1000 12.5 | 11.0. Clusters of 8 (and so 4) find room for 256 CTAs at once, not for 296: B3
+//    H12/12 Lk 4000 in 288 CTAs 13.1 | 20.4.
+//  * One nearly full wave of whole units: B32 Lk 500 12.5 | 9.1, B30 Lk 300 D64 9.0 | 6.3, B34 Lk 900 26.4 | 23.1 (192 units, B24 Lk 3000 51.8 | 52.4).
+//  * Several waves whose last one is more than half full. The hardware deals them out, where the slowest SM ends an equal share: B64 Lk 32768
+//    1249 | 1164, Lk 1500 66.6 | 59.7, Lk 300 16.1 | 13.2 (last wave nearly empty: B30 H12/12 Lk 2000 60.9 | 63.7, B44 Lk 300 11.8 | 12.3; many waves of a
+//    few tiles: B64 H32/32 Lk 64 19.0 | 22.6). A wave of
+//    clusters costs 3 to 4 us, so those take long shares only: B32 Lk 16384 in twos 316 | 300, B16 in fours 316 | 310, B8 Lk 32768 in eights 164 | 160 (B16
+//    Lk 1000 in fours 12.5 | 16.6).
+int cluster_size(const DecodeParams& d) {
+  constexpr int kWave = kCtasPerSm * 148;
+  const int64_t units = d.units;
+  const int tiles = d.tiles_per_unit;
+  for (int size = kMaxCluster; size > 1; size /= 2) {
+    if (size > tiles || units * size > (size > 2 ? 256 : kWave)) continue;
+    if ((tiles + size - 1) / size - static_cast<double>(units) * tiles / kWave <= 3.5) return size;
+    break;
+  }
+  if (units <= kWave && units >= kWave * 4 / 5 && tiles < 63) return 1;
+  for (int size = 1; size <= kMaxCluster; size *= 2) {
+    const int64_t ctas = units * size, last = ctas % kWave;
+    if (ctas >= kWave && (last == 0 || last >= 160) && (size == 1 ? tiles > ctas / kWave : (tiles + size - 1) / size >= 32)) return size;
+  }
+  return 0;
+}
+
 // Rows of partial results the workspace must hold (0: every unit stays whole).
 size_t partial_rows(const sdpa_b200_params& p, const DecodeParams& d) {
   if (d.num_splits == 1) return 0;
@@ -585,13 +683,13 @@ size_t decode_workspace_bytes(const sdpa_b200_params& p) {
 
 namespace {
 
-template <bool kHi, int kD, bool kF16>
+template <bool kHi, int kD, bool kF16, bool kCluster = false>
 cudaError_t launch_split(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const DecodeParams& d, bool overlap, cudaStream_t stream) {
   constexpr uint32_t kSmem = decode_smem_bytes<kHi, kD>();
-  auto kernel = decode_splitkv_kernel<kHi, kD, kF16>;
+  auto kernel = decode_splitkv_kernel<kHi, kD, kF16, kCluster>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (err != cudaSuccess) return err;
-  return launch_behind(kernel, dim3(d.grid), kDecThreads, kSmem, stream, overlap, tm_k, tm_v, d);
+  return launch_behind(kernel, dim3(d.grid), kDecThreads, kSmem, stream, overlap, kCluster ? d.num_splits : 1, tm_k, tm_v, d);
 }
 
 template <int kD>
@@ -638,25 +736,38 @@ int launch_decode(const sdpa_b200_params& p, DecodeParams& d, float* scratch, ui
   st = make_tensor_map_16(f16, &tm_v, p.v, p.head_dim, p.max_seqlen_k, p.heads_kv, p.batch, p.v_row_stride,
                           one_head ? p.v_row_stride : p.v_head_stride, p.v_batch_stride, kKeysPerStep);
   if (st != SDPA_B200_OK) return st;
+  const int cluster = p.num_splits > 0 ? 0 : cluster_size(d);
+  if (cluster > 0) {
+    d.num_splits = cluster;
+    d.tiles_per_split = (d.tiles_per_unit + cluster - 1) / cluster;
+    d.grid = d.units * cluster;
+  }
   const bool hi = d.rows > 8;
   // under the tail of whatever is in front, unless that is the launch that clears the status word (calls back to back: B64 H32/8 Lk 84 D64
   // 12.3 us -> 9.7, B8 Lk 4096 D128 29.7 -> 27.4, B1 Lk 1000 9.0 -> 8.6)
   const bool overlap = p.device_status != nullptr;
   cudaError_t err;
-  if (p.head_dim == 64) {
-    err = hi ? (f16 ? launch_split<true, 64, true>(tm_k, tm_v, d, overlap, stream) : launch_split<true, 64, false>(tm_k, tm_v, d, overlap, stream))
-             : (f16 ? launch_split<false, 64, true>(tm_k, tm_v, d, overlap, stream) : launch_split<false, 64, false>(tm_k, tm_v, d, overlap, stream));
-  } else {
-    err = hi ? (f16 ? launch_split<true, 128, true>(tm_k, tm_v, d, overlap, stream) : launch_split<true, 128, false>(tm_k, tm_v, d, overlap, stream))
-             : (f16 ? launch_split<false, 128, true>(tm_k, tm_v, d, overlap, stream) : launch_split<false, 128, false>(tm_k, tm_v, d, overlap, stream));
-  }
+  auto launch = [&](auto hi_tag, auto dim_tag, auto f16_tag) {
+    constexpr bool kHi = decltype(hi_tag)::value, kF16 = decltype(f16_tag)::value;
+    constexpr int kD = decltype(dim_tag)::value;
+    return cluster > 1 ? launch_split<kHi, kD, kF16, true>(tm_k, tm_v, d, overlap, stream) : launch_split<kHi, kD, kF16, false>(tm_k, tm_v, d, overlap, stream);
+  };
+  auto launch_type = [&](auto hi_tag, auto dim_tag) {
+    return f16 ? launch(hi_tag, dim_tag, std::true_type{}) : launch(hi_tag, dim_tag, std::false_type{});
+  };
+  using Dim64 = std::integral_constant<int, 64>;
+  using Dim128 = std::integral_constant<int, 128>;
+  if (p.head_dim == 64)
+    err = hi ? launch_type(std::true_type{}, Dim64{}) : launch_type(std::false_type{}, Dim64{});
+  else
+    err = hi ? launch_type(std::true_type{}, Dim128{}) : launch_type(std::false_type{}, Dim128{});
   if (err != cudaSuccess) {
     set_error("%s: launch failed: %s", who, cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
   }
   count_launch();
   // no merge when the shares' borders coincide with the units'
-  const bool shared = d.num_splits > 0 ? d.num_splits > 1 : (d.tiles_per_unit > 1 && d.units % d.grid != 0);
+  const bool shared = cluster > 0 ? false : d.num_splits > 0 ? d.num_splits > 1 : (d.tiles_per_unit > 1 && d.units % d.grid != 0);
   if (shared) {
     const int out_rows = p.batch * p.heads_q;
     err = p.head_dim == 64 ? launch_combine<64>(d, out_rows, stream) : launch_combine<128>(d, out_rows, stream);

@@ -73,11 +73,11 @@ inline int heads_per_packed_group(double all_bytes, int num_heads) {
   return (num_heads + groups - 1) / groups;
 }
 
-// Launches `kernel`; with `overlap` so that its CTAs may start as soon as every CTA of the grid in front of it in the stream has said that it may
+// Launches `kernel` in clusters of `cluster` CTAs; with `overlap` so that its CTAs may start as soon as every CTA of the grid in front of it in the stream has said that it may
 // (launch_dependents) or has left, and an SM has room: its launch and set-up then pass under that grid's tail. The kernel waits
 // (wait_for_previous_grid) before it touches global memory. Not under stream capture, where what stands in front may be no kernel.
 template <typename... Params, typename... Args>
-cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool overlap, const Args&... args) {
+cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool overlap, int cluster, const Args&... args) {
   if (overlap) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     overlap = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
@@ -88,11 +88,18 @@ cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, siz
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
+  if (overlap) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, args...);
   return err == cudaSuccess ? cudaGetLastError() : err;
 }
