@@ -259,3 +259,15 @@ def test_causal_ranks_behind_all_groups(cuda_device, native_lib, B, Hq, Hkv, Lq,
     """More heads than a group holds, so that the lightest ranks run behind all groups, against the oracle."""
     q, k, v = rand((B, Hq, Lq, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3)
     check_dense(cuda_device, q, k, v, True)
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,D,causal", [
+    (1, 148, 128, 130, 64, False),  # single tiles on every SM
+    (1, 74, 129, 129, 128, True),   # the last ones of a row with one query each
+    (1, 75, 129, 200, 64, True),    # two tiles more than SMs: pairs again
+    (2, 3, 300, 200, 128, True),    # tiles without keys
+])
+def test_single_tile_units(cuda_device, native_lib, B, H, Lq, Lk, D, causal):
+    """Both sides of the rule that gives every 128-row tile an SM of its own, against the oracle."""
+    q, k, v = rand((B, H, Lq, D), 1), rand((B, H, Lk, D), 2), rand((B, H, Lk, D), 3)
+    check_dense(cuda_device, q, k, v, causal)

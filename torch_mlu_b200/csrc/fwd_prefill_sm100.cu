@@ -10,7 +10,7 @@
 // key) pair from dropout_mask.cu) and the additive bias of the memory-efficient operators (kBias:
 // softmax(scale * Q K^T + bias), mem_eff_fwd, FlashAttention_internal.cpp:485-690).
 //
-// A work unit is 256 query rows of one (batch, head): two 128-row Q tiles. One persistent CTA per SM
+// A work unit is 256 query rows of one (batch, head): two 128-row Q tiles (one where there are few). One persistent CTA per SM
 // walks the unit list; its barriers, TMEM and K/V ring live across units, so the next unit's loads
 // and first QK^T overlap this unit's epilogue. Roles:
 //   warps 0-3  softmax warpgroup for Q tile 0  (thread = one query row = one TMEM lane)
@@ -102,6 +102,8 @@ struct FwdKernelParams {
   int64_t bias_batch_stride, bias_head_stride, bias_row_stride;
   float inv_scale;  // 1 / softmax_scale: the bias joins the raw scores as bias / scale
   BlockOrder order;  // of the work units
+  int unit_tiles;    // Q tiles per unit: 2, or 1 where every tile has an SM of its own
+  int tile1;         // first row of a unit's second tile in the unit; behind every sequence where there is none
   float scale_log2;
   int is_causal;
 };
@@ -130,7 +132,7 @@ __device__ __forceinline__ void issue_pv_half(uint32_t t_o, uint32_t t_p, uint32
   if constexpr (kI + 1 < 4) issue_pv_half<kD, kF16, kHalf, kI + 1>(t_o, t_p, b_lo, accumulate);
 }
 
-// One work unit: 256 query rows (two 128-row tiles) of one (batch, head).
+// One work unit: 256 query rows (two 128-row tiles) of one (batch, head), or 128 rows (FwdKernelParams::unit_tiles).
 struct Unit {
   int b, h, hk, m0, q_off, k_off, len_q, len_k, bcoord, causal_off;
   int nblk[2];  // key blocks each Q tile visits
@@ -160,12 +162,12 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
     u.len_k = p.cu_k[u.b + 1] - u.k_off;
     u.bcoord = 0;
   }
-  u.m0 = m_block * (2 * kBlockM);
+  u.m0 = m_block * (p.unit_tiles * kBlockM);
   if (u.m0 >= u.len_q) return false;
   u.causal_off = u.len_k - u.len_q;  // bottom-right alignment
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int row_lo = u.m0 + t * kBlockM;
+    const int row_lo = u.m0 + t * p.tile1;
     int vis_end = u.len_k;
     if (p.is_causal) vis_end = min(u.len_k, row_lo + kBlockM + u.causal_off);
     u.nblk[t] = (row_lo < u.len_q && vis_end > 0) ? (vis_end + kBlockN - 1) / kBlockN : 0;
@@ -288,9 +290,8 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint32_t preloaded = 0;  // producer: ring tiles of the first unit that have been asked for
   auto load_q = [&](int q_row, int h, int bcoord) {
     constexpr uint32_t kLoadBytes = kBlockN * kD * 2;  // bytes one Q/K/V tile brings in
-    mbar_arrive_expect_tx(bar + kBarQFull, 2 * kLoadBytes);
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
+    mbar_arrive_expect_tx(bar + kBarQFull, p.unit_tiles * kLoadBytes);
+    for (int t = 0; t < p.unit_tiles; ++t) {
       const uint32_t dst = base + kSmemQ + t * kTileBytes;
       tma_load_4d(dst, &tm_q, bar + kBarQFull, 0, q_row + t * kBlockM, h, bcoord);
       if (kD > 64) tma_load_4d(dst + kHalfBytes, &tm_q, bar + kBarQFull, 64, q_row + t * kBlockM, h, bcoord);
@@ -518,7 +519,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       if (!ok || u.done) break;
       // everything the block loop needs from the unit, so that `u` dies here; what only the epilogue
       // needs waits in shared memory (one slot per warp), not in registers
-      const int row_lo = u.m0 + t * kBlockM;
+      const int row_lo = u.m0 + t * p.tile1;
       const int row = row_lo + row_in_tile;
       const int my_blocks = u.nblk[t];
       int* info = reinterpret_cast<int*>(smem + kSmemBar + kSmemStash) + 8 * warp;
@@ -880,9 +881,15 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   const int usable = sms - p.sm_margin > 1 ? sms - p.sm_margin : 1;
   // K+V bytes one query head streams, shared by the heads of its GQA group
   const double kv_row_bytes = 2.0 * p.head_dim * 2;
-  const int heads = p.batch * p.heads_q, ranks = (p.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM);
+  const int heads = p.batch * p.heads_q, tiles = (p.max_seqlen_q + kBlockM - 1) / kBlockM;
+  // Where every Q tile can have an SM of its own, a unit is one tile: two share K and V, but also the exponential unit and the tensor core, and
+  // what one of them gains from the other's waits is less than a second SM gives (pairs | single tiles, us: B2 H8 L256 D64 7.6 | 6.5, B1 H8 L2048 D128
+  // 32.4 | 29.9, B1 H12 L1500 D64 24.5 | 20.0, B1 H32/8 L512 14.0 | 12.0; with two rounds of single tiles against one of pairs it is the other way round).
+  kp.unit_tiles = static_cast<int64_t>(heads) * tiles <= usable ? 1 : 2;
+  kp.tile1 = kp.unit_tiles == 2 ? kBlockM : 1 << 30;
+  const int unit_rows = kp.unit_tiles * kBlockM, ranks = (p.max_seqlen_q + unit_rows - 1) / unit_rows;
   kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes),
-                         p.is_causal ? tail_ranks(ranks, kv_row_bytes * (2 * kBlockM) * p.batch * p.heads_kv) : 0);
+                         p.is_causal ? tail_ranks(ranks, kv_row_bytes * unit_rows * p.batch * p.heads_kv) : 0);
   dim3 grid(kp.order.slots < usable ? kp.order.slots : usable, 1, 1);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
   // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
