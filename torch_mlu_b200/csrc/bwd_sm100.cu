@@ -31,6 +31,8 @@
 #include <cstdlib>
 #endif
 
+#include <type_traits>
+
 #include "bwd_common.cuh"
 #include "bwd_ds_gemm.h"
 #include "packed_grads.cuh"
@@ -904,24 +906,27 @@ struct PreParams {
   PackedGrads grads;
 };
 
-// 16 bytes (8 elements) per thread and head_dim / 8 threads per row; a 256-thread block covers 64 rows of
-// the padded sequence in up to four passes whose loads are all issued before the first use.
-constexpr int kPreRows = 64;
-template <bool kF16, bool kPacked>
+// 16 bytes (8 elements) per thread and kD / 8 threads per row; a 256-thread block covers two passes of rows of the padded sequence. HBM-bound:
+// all loads of a block, the logsumexp among them, are issued before the first use, and the rows' sums go through shared memory, so
+// that a block has one memory latency instead of two and writes whole lines (with the logsumexp read behind the sums by one lane per row
+// and four passes per block, 134 MB at B8 H16 L2048 D128 29.8 us; so 22.6, 5.9 TB/s; four passes 23.0, one 24.6).
+template <int kD>
+constexpr int kPreRows = 2 * 256 * 8 / kD;  // 64 or 32
+template <int kD, bool kF16, bool kPacked>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) {
   if (kPacked && static_cast<int>(blockIdx.x) == p.heads_q) {
     clear_uncovered_rows(p.grads, p.heads_q);
     return;
   }
-  if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // see bwd_tile_kernel
+  if (threadIdx.x == 0) launch_dependents();  // see bwd_tile_kernel
+  constexpr int kRows = kPreRows<kD>, kPerPass = kRows / 2, kThreadsPerRow = kD / 8;
+  __shared__ float sums[kRows];
   // heads vary fastest across the grid: with the usual [batch, row, head, dim] memory order the blocks
   // that run together then read neighbouring 256-byte pieces of the same rows
   const int h = blockIdx.x, b = blockIdx.z;
-  const int tpr = p.head_dim <= 64 ? 8 : 16;  // threads per row (head dims in between leave lanes without data)
-  const int rows_per_pass = 256 / tpr;      // 16 or 32
-  const int passes = kPreRows / rows_per_pass;  // 4 or 2
-  const int sub = threadIdx.x % tpr;
-  const int r_in_pass = threadIdx.x / tpr;
+  const int row0 = blockIdx.y * kRows;
+  const int col = threadIdx.x % kThreadsPerRow * 8;
+  const int r_in_pass = threadIdx.x / kThreadsPerRow;
   int q_off = 0, len_q = p.seqlen_q;
   if (kPacked) {
     q_off = p.cu_q[b];
@@ -930,67 +935,58 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   if (kPacked && p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0) {
     write_seq_base(p.ds_seq_base, p.cu_q, p.cu_k, b, p.is_causal != 0);
   }
-  if (p.dq_acc != nullptr) {
+  uint4 ov[2], dv[2];
+#pragma unroll
+  for (int ps = 0; ps < 2; ++ps) {
+    ov[ps] = make_uint4(0u, 0u, 0u, 0u);
+    dv[ps] = make_uint4(0u, 0u, 0u, 0u);
+    const int row = row0 + ps * kPerPass + r_in_pass;
+    if (row < len_q && col < p.head_dim) {
+      const int64_t at = (kPacked ? q_off : 0) + static_cast<int64_t>(row);
+      const uint16_t* o = p.out + (kPacked ? 0 : b * p.o_batch_stride) + h * p.o_head_stride + at * p.o_row_stride + col;
+      const uint16_t* dout = p.dout + (kPacked ? 0 : b * p.do_batch_stride) + h * p.do_head_stride + at * p.do_row_stride + col;
+      ov[ps] = __ldcs(reinterpret_cast<const uint4*>(o));  // not read again, unlike dO
+      dv[ps] = *reinterpret_cast<const uint4*>(dout);
+    }
+  }
+  const int my_row = row0 + threadIdx.x;  // of the first kRows threads: the row whose values they write
+  const bool have = threadIdx.x < kRows && my_row < len_q;
+  float lse = 0.f;
+  if (have)
+    lse = kPacked ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + my_row]
+                  : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + my_row];
+  if (kD == 64 && p.dq_acc != nullptr) {
     // 64 rows of an accumulator tile: per 4-column group 1 KB of consecutive floats, a thread per row. The stores need no
-    // registers and go out under the loads below: one launch instead of two and 45 us instead of 58 at 64 K rows of 128
+    // registers and go out under the loads above
     constexpr int groups = 16;
-    const int row = blockIdx.y * kPreRows + (threadIdx.x & (kPreRows - 1));
+    const int row = row0 + (threadIdx.x & (kRows - 1));
     if (row < len_q) {
       const size_t acc_row = kPacked ? static_cast<size_t>(h) * p.dq_acc_rows + q_off + row
                                                : (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
       float4* dst = reinterpret_cast<float4*>(p.dq_acc + (acc_row >> 7) * (static_cast<size_t>(groups) * 512)) + (acc_row & 127);
-      for (int g = threadIdx.x / kPreRows; g < groups; g += 256 / kPreRows) dst[g * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  uint4 ov[4], dv[4];
-#pragma unroll
-  for (int ps = 0; ps < 4; ++ps) {
-    ov[ps] = make_uint4(0u, 0u, 0u, 0u);
-    dv[ps] = make_uint4(0u, 0u, 0u, 0u);
-    const int row = blockIdx.y * kPreRows + ps * rows_per_pass + r_in_pass;
-    if (ps < passes && row < len_q) {
-      const uint16_t* o;
-      const uint16_t* dout;
-      if (kPacked) {
-        o = p.out + static_cast<int64_t>(q_off + row) * p.o_row_stride + h * p.o_head_stride;
-        dout = p.dout + static_cast<int64_t>(q_off + row) * p.do_row_stride + h * p.do_head_stride;
-      } else {
-        o = p.out + b * p.o_batch_stride + h * p.o_head_stride + static_cast<int64_t>(row) * p.o_row_stride;
-        dout = p.dout + b * p.do_batch_stride + h * p.do_head_stride + static_cast<int64_t>(row) * p.do_row_stride;
-      }
-      if (sub * 8 < p.head_dim) {
-        ov[ps] = *reinterpret_cast<const uint4*>(o + sub * 8);
-        dv[ps] = *reinterpret_cast<const uint4*>(dout + sub * 8);
-      }
+      for (int g = threadIdx.x / kRows; g < groups; g += 256 / kRows) dst[g * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
 #pragma unroll
-  for (int ps = 0; ps < 4; ++ps) {
-    if (ps >= passes) break;
-    const int row = blockIdx.y * kPreRows + ps * rows_per_pass + r_in_pass;
+  for (int ps = 0; ps < 2; ++ps) {
     const float2 o0 = unpack_16x2<kF16>(ov[ps].x), o1 = unpack_16x2<kF16>(ov[ps].y);
     const float2 o2 = unpack_16x2<kF16>(ov[ps].z), o3 = unpack_16x2<kF16>(ov[ps].w);
     const float2 d0 = unpack_16x2<kF16>(dv[ps].x), d1 = unpack_16x2<kF16>(dv[ps].y);
     const float2 d2 = unpack_16x2<kF16>(dv[ps].z), d3 = unpack_16x2<kF16>(dv[ps].w);
     float acc = (o0.x * d0.x + o0.y * d0.y) + (o1.x * d1.x + o1.y * d1.y) + (o2.x * d2.x + o2.y * d2.y) +
                 (o3.x * d3.x + o3.y * d3.y);
-    // the tpr threads of a row are consecutive lanes of one warp
-    for (int off = tpr >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (sub == 0 && row < p.lq_pad) {
-      const size_t dst = (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
-      if (row < len_q) {
-        const float lse = (kPacked) ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + row]
-                                              : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + row];
-        p.nlse2[dst] = lse * -1.4426950408889634f;
-        p.ndelta[dst] = -acc;
-      } else {
-        p.nlse2[dst] = -INFINITY;
-        p.ndelta[dst] = 0.f;
-      }
-    }
+    // the threads of a row are consecutive lanes of one warp
+#pragma unroll
+    for (int off = kThreadsPerRow >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (col == 0) sums[ps * kPerPass + r_in_pass] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x < kRows && my_row < p.lq_pad) {
+    const size_t dst = (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + my_row;
+    p.nlse2[dst] = have ? lse * -1.4426950408889634f : -INFINITY;
+    p.ndelta[dst] = have ? -sums[threadIdx.x] : 0.f;
   }
 }
-
 
 using TileKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                             const CUtensorMap, const CUtensorMap, const BwdKernelParams);
@@ -1149,9 +1145,13 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   float* dq_acc = fused ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p)) : nullptr;
   pre.dq_acc = dq_acc;
   pre.dq_acc_rows = fused && varlen ? static_cast<int>(bwd_fused_acc_rows(p, lq_pad) / p.heads_q) : 0;
-  const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), lq_pad / kPreRows, p.batch);
-  auto pre_kernel = varlen ? (f16 ? bwd_preprocess_kernel<true, true> : bwd_preprocess_kernel<false, true>)
-                           : (f16 ? bwd_preprocess_kernel<true, false> : bwd_preprocess_kernel<false, false>);
+  const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), lq_pad / (p.head_dim <= 64 ? kPreRows<64> : kPreRows<128>), p.batch);
+  auto pick_pre = [&](auto dim_tag) {
+    constexpr int kD = decltype(dim_tag)::value;
+    return varlen ? (f16 ? bwd_preprocess_kernel<kD, true, true> : bwd_preprocess_kernel<kD, false, true>)
+                  : (f16 ? bwd_preprocess_kernel<kD, true, false> : bwd_preprocess_kernel<kD, false, false>);
+  };
+  auto pre_kernel = p.head_dim <= 64 ? pick_pre(std::integral_constant<int, 64>{}) : pick_pre(std::integral_constant<int, 128>{});
   pre_kernel<<<pre_grid, 256, 0, stream>>>(pre);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
