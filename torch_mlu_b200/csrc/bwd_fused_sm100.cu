@@ -67,14 +67,14 @@ constexpr uint32_t kFBarYEmpty = 40;   // 2 pairs: behind dK(i), the last reader
 constexpr uint32_t kFBarSFull = 56;
 constexpr uint32_t kFBarDFull = 64;
 constexpr uint32_t kFBarDFree = 72;    // 8: all compute warps have read dP out of TMEM
-constexpr uint32_t kFBarP1Full = 80;   // 8: all compute warps have stored P
-constexpr uint32_t kFBarDSFull = 88;   // 8: all compute warps have stored dS in shared memory
-constexpr uint32_t kFBarQFull = 96;    // dQ(i) is in TMEM
-constexpr uint32_t kFBarQFree = 104;   // 4: all reduce warps have read dQ(i)
-constexpr uint32_t kFBarAccFull = 112;
-constexpr uint32_t kFBarEpiFull = 120; // 8
-constexpr uint32_t kFSmemTmemPtr = 128;
-constexpr uint32_t kFSmemAbort = 132;
+constexpr uint32_t kFBarP1Full = 80;   // 2 (item parity: P(i+1) may be complete before the issuer has looked at P(i)), 8: all compute warps have stored P
+constexpr uint32_t kFBarDSFull = 96;   // 8: all compute warps have stored dS in shared memory
+constexpr uint32_t kFBarQFull = 104;   // dQ(i) is in TMEM
+constexpr uint32_t kFBarQFree = 112;   // 4: all reduce warps have read dQ(i)
+constexpr uint32_t kFBarAccFull = 120;
+constexpr uint32_t kFBarEpiFull = 128; // 8
+constexpr uint32_t kFSmemTmemPtr = 136;
+constexpr uint32_t kFSmemAbort = 140;
 
 // Profiling builds (-DSDPA_BWD_STAMPS) time-stamp pipeline events of one CTA: roles 0/1 = lane 0 of the first warp of each
 // compute warpgroup, 2 / 3 = the two MMA issuers, 4 = lane 0 of the first reduce warp; [role 5][item 24][event 8] floats.
@@ -219,6 +219,7 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(bar + kFBarDFull, 1);
     mbar_init(bar + kFBarDFree, 8);  // one arrival per compute warp
     mbar_init(bar + kFBarP1Full, 8);
+    mbar_init(bar + kFBarP1Full + 8, 8);
     mbar_init(bar + kFBarDSFull, 8);
     mbar_init(bar + kFBarQFull, 1);
     mbar_init(bar + kFBarQFree, 4);  // one arrival per reduce warp
@@ -354,7 +355,7 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           // the tiles landed long ago (the other issuer has used them); these waits make the copies visible here too
           FSTAMP(3, i, 0);
           ok = mbar_wait(bar + kFBarYFull + 8 * s0, par, abort_flag) && mbar_wait(bar + kFBarYFull + 8 * (s0 + 1), par, abort_flag) &&
-               mbar_wait(bar + kFBarP1Full, i & 1, abort_flag);
+               mbar_wait(bar + kFBarP1Full + 8 * (i & 1), (i >> 1) & 1, abort_flag);
           if (!ok) break;
           FSTAMP(3, i, 1);
           tc_fence_after_sync();
@@ -461,7 +462,7 @@ bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar + kFBarP1Full);
+        if (lane == 0) mbar_arrive(bar + kFBarP1Full + 8 * (i & 1));
       }
       FSTAMP(half, i, 3);
       // phase 2 (needs dP): dS = P o (dP - delta) into this thread's row of the shared-memory tile

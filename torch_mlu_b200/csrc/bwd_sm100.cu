@@ -64,14 +64,18 @@ constexpr uint32_t kBarYEmpty = kBarYFull + 8 * kMaxStages;
 constexpr uint32_t kBarSFull = kBarYEmpty + 8 * kMaxStages;   // 2: first score GEMM (X1 Y1^T) of an item done
 constexpr uint32_t kBarDFull = kBarSFull + 16;             // second score GEMM (X2 Y2^T) done
 constexpr uint32_t kBarDFree = kBarDFull + 8;              // all compute warps have read dP out of TMEM
-constexpr uint32_t kBarPFull = kBarDFree + 16;             // all compute warps have stored P / dS
+// Of the next two there is one per item parity: in the dQ kernel the compute warps can complete the next item's P / dS, in the dK/dV kernel its
+// P, before the accumulation issuer has looked at this one's, and to a wait on a parity two phases further on read "not yet". The item
+// after that needs the issuer first.
+constexpr uint32_t kBarPFull = kBarDFree + 16;             // 2: all compute warps have stored P / dS
 constexpr uint32_t kBarAccFull = kBarPFull + 16;
-constexpr uint32_t kBarP1Full = kBarAccFull + 8;           // dK/dV: all compute warps have stored P (dS still to come)
-constexpr uint32_t kBarWFree = kBarP1Full + 8;             // 2 (item parity): the accumulation GEMMs have read P / dS
+constexpr uint32_t kBarP1Full = kBarAccFull + 8;           // 2, dK/dV: all compute warps have stored P (dS still to come)
+constexpr uint32_t kBarWFree = kBarP1Full + 16;            // 2 (item parity): the accumulation GEMMs have read P / dS
 constexpr uint32_t kBarSIssued = kBarWFree + 16;           // dK/dV: the next item's score GEMM is in the pipe
 constexpr uint32_t kBarEpiFull = kBarSIssued + 8;           // all compute warps have staged their output rows
 constexpr uint32_t kSmemTmemPtr = kBarEpiFull + 8;
 constexpr uint32_t kSmemAbort = kSmemTmemPtr + 4;
+static_assert(kSmemAbort + 4 <= 256, "the barriers reach into the key bias");
 
 // Profiling builds (-DSDPA_BWD_STAMPS) time-stamp pipeline events of one CTA per kernel; role 0/1 =
 // lane 0 of the first warp of each compute warpgroup, roles 2 and 3 = the MMA issuer.
@@ -247,7 +251,9 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     mbar_init(bar + kBarDFull, 1);
     mbar_init(bar + kBarDFree, 8);  // one arrival per compute warp
     mbar_init(bar + kBarPFull, 8);
+    mbar_init(bar + kBarPFull + 8, 8);
     mbar_init(bar + kBarP1Full, 8);
+    mbar_init(bar + kBarP1Full + 8, 8);
     mbar_init(bar + kBarWFree, 1);
     mbar_init(bar + kBarWFree + 8, 1);
     mbar_init(bar + kBarSIssued, 1);
@@ -441,14 +447,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           if (!ok) break;
           if (kMode == kModeDKDV) {
             // dV needs P only, which is stored a whole dS pass before the item is complete
-            ok = mbar_wait(bar + kBarP1Full, i & 1, abort_flag);
+            ok = mbar_wait(bar + kBarP1Full + 8 * (i & 1), (i >> 1) & 1, abort_flag);
             if (!ok) break;
             tc_fence_after_sync();
             issue_wy_half<kD, kF16>(acc1, sbuf, y2, 0, i > 0);       // dV += P^T dO
             issue_wy_half<kD, kF16>(acc1, sbuf + 64, y2, 1, true);
           }
           BWD_STAMP(3, i, 0);
-          ok = mbar_wait(bar + kBarPFull, i & 1, abort_flag);
+          ok = mbar_wait(bar + kBarPFull + 8 * (i & 1), (i >> 1) & 1, abort_flag);
           if (!ok) break;
           BWD_STAMP(3, i, 1);
           tc_fence_after_sync();
@@ -705,7 +711,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tmem_wait_st();
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar + kBarP1Full);
+          if (lane == 0) mbar_arrive(bar + kBarP1Full + 8 * (i & 1));
         }
       }
       // phase 2 (needs dP): dS = P o (dP - delta) into the second half of this thread's columns
@@ -761,7 +767,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tmem_wait_st();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar + kBarPFull);
+      if (lane == 0) mbar_arrive(bar + kBarPFull + 8 * (i & 1));
       BWD_STAMP(half, i, 7);
       if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr) {
         // dS for the dQ GEMM: 16 bytes (8 queries) per store, 512 contiguous bytes per warp. Behind the arrival, so that the

@@ -473,8 +473,8 @@ constexpr uint32_t kBX2Full = kBAReady + 8;
 constexpr uint32_t kBTFull = kBX2Full + 8;     // 2: the score GEMM into T[b] has finished (kDK, kDQ: S, dP)
 constexpr uint32_t kBSFree = kBTFull + 16;     // 8 warps: the scores have been read out of TMEM (kDK, kDQ)
 constexpr uint32_t kBDFree = kBSFree + 8;      // 8 warps: dP has been read out of TMEM (kDK, kDQ)
-constexpr uint32_t kBWFull = kBDFree + 8;      // 8 warps: the 16-bit P is in TMEM / the 16-bit dS in shared memory
-constexpr uint32_t kBWRead = kBWFull + 8;      // 2 (kDV: item parity): the accumulation GEMM of an item has read its P / dS
+constexpr uint32_t kBWFull = kBDFree + 8;      // 2 (kDV: item parity), 8 warps: the 16-bit P is in TMEM / the 16-bit dS in shared memory
+constexpr uint32_t kBWRead = kBWFull + 16;     // 2 (kDV: item parity): the accumulation GEMM of an item has read its P / dS
 constexpr uint32_t kBAccFull = kBWRead + 16;
 constexpr uint32_t kBStageB = kBAccFull + 8;   // 4 warps
 constexpr uint32_t kTmemPtrB = kBStageB + 8;
@@ -655,6 +655,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
     mbar_init(bar + kBSFree, 8);
     mbar_init(bar + kBDFree, 8);
     mbar_init(bar + kBWFull, 8);
+    mbar_init(bar + kBWFull + 8, 8);
     mbar_init(bar + kBWRead, 1);
     mbar_init(bar + kBWRead + 8, 1);
     mbar_init(bar + kBAccFull, 1);
@@ -790,7 +791,9 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
           // ---------------- accumulations: dV += P^T(i) dO
           for (int i = 0; ok && i < n_items; ++i) {
             const int t = 2 * i + 1, s = t % kRingDV;
-            ok = mbar_wait(bar + kBWFull, i & 1, abort_flag) &&
+            // a barrier per parity: P(i+1) can be complete before this thread has looked at P(i), and to a wait on a parity two phases
+            // further on read "not yet"; P(i+2) needs WRead(i)
+            ok = mbar_wait(bar + kBWFull + 8 * (i & 1), (i >> 1) & 1, abort_flag) &&
                  mbar_wait(bar + kBFull + 8 * s, static_cast<uint32_t>(t / kRingDV) & 1u, abort_flag);
             if (!ok) break;
             tc_fence_after_sync();
@@ -1035,7 +1038,7 @@ bwd_d256_kernel(const __grid_constant__ CUtensorMap tm_x2, const __grid_constant
       auto w_full = [&]() {
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar + kBWFull);
+        if (lane == 0) mbar_arrive(bar + kBWFull + (kMode == kDV ? 8 * (i & 1) : 0));
       };
       if constexpr (kMode == kDV) {
         // over the front of this thread's OWN score columns (16 columns = 32 streamed rows): the other warpgroup may still be
