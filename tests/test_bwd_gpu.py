@@ -275,3 +275,23 @@ def test_backward_on_both_sides_of_the_dispatch(cuda_device, native_lib, lens, H
     if len(set(lens)) == 1:
         check_grads(run(True), want)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("L,dropout,path", [(1024, False, "two"), (1025, False, "fused"), (1025, True, "two")])
+def test_short_rows_and_dropout_at_head_dim_64(cuda_device, native_lib, L, dropout, path):
+    test_which_backward_kernels_run(cuda_device, native_lib, 1, 20, 20, L, 64, dropout, False, False, path)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D,causal", [
+    (1, 2, 2, 65, 190, 64, False),   # one row in the last streamed tile of 64
+    (1, 2, 2, 190, 65, 64, True),    # rows without keys
+    (1, 4, 2, 64, 129, 64, True),    # whole tiles of queries, one key in the last block
+    (2, 2, 2, 1, 63, 40, False),
+    (1, 6, 3, 321, 449, 64, True),   # offsets that are no multiple of 128
+])
+def test_streamed_tiles_of_64_rows(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
+    """The two kernels up to head_dim 64, whose streamed tiles are half as high as the blocks, against the oracle; tolerances as above."""
+    q, k, v, dout = (rand((B, h, n, D), s) for s, h, n in ((1, Hq, Lq), (2, Hkv, Lk), (3, Hkv, Lk), (4, Hq, Lq)))
+    out, lse, *grads = run_fwd_bwd(cuda_device, q, k, v, dout, causal, deterministic=True)
+    o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=causal)
+    check_grads(grads, orc.cpu_sdpa_backward(dout, q, k, v, o_ref, l_ref, causal=causal))

@@ -74,21 +74,21 @@ int launch_bwd_fused(const sdpa_b200_params& p, BwdKernelParams kp, float* dq_ac
                      const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                      const CUtensorMap& tm_dv, const CUtensorMap& tm_dk);
 
-template <bool kF16>
-constexpr uint32_t kIdescSS = umma_idesc_16(kTile, kTile, false, false, kF16);
+template <bool kF16, int kY>
+constexpr uint32_t kIdescSS = umma_idesc_16(kTile, kY, false, false, kF16);
 template <int kD, bool kF16>
 constexpr uint32_t kIdescTS = umma_idesc_16(kTile, kD, false, true, kF16);
 
-// T = X Y^T, contraction over head_dim, both operands K-major in shared memory
-template <int kD, bool kF16>
+// T = X Y^T (kY rows of Y), contraction over head_dim, both operands K-major in shared memory
+template <int kD, bool kF16, int kY = kTile>
 __device__ __forceinline__ void issue_xyT(uint32_t t, uint32_t x_smem, uint32_t y_smem) {
   const uint32_t a_lo = umma_desc_lo_kmajor(x_smem);
   const uint32_t b_lo = umma_desc_lo_kmajor(y_smem);
-  umma_ss_lo<kIdescSS<kF16>, false>(t, a_lo, b_lo);
+  umma_ss_lo<kIdescSS<kF16, kY>, false>(t, a_lo, b_lo);
 #pragma unroll
   for (int ks = 1; ks < kD / 16; ++ks) {
     const uint32_t off = ((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4;
-    umma_ss_lo<kIdescSS<kF16>, true>(t, a_lo + off, b_lo + off);
+    umma_ss_lo<kIdescSS<kF16, kY>, true>(t, a_lo + off, b_lo + off);
   }
 }
 
@@ -102,6 +102,17 @@ __device__ __forceinline__ void issue_wy_half(uint32_t acc, uint32_t w, uint32_t
     const int ks = half * 4 + i;
     umma_ts_lo<kIdescTS<kD, kF16>>(acc, w + i * 8, b_lo + ks * (2048 >> 4), (accumulate || ks > 0) ? 1u : 0u);
   }
+}
+
+// ACC (+)= W Y over all kY rows of the Y tile. Two warpgroups have written W for half of the rows each, to the columns of their own scores: the
+// second half begins kY / 2 columns behind `w`.
+template <int kD, bool kF16, int kY>
+__device__ __forceinline__ void issue_wy(uint32_t acc, uint32_t w, uint32_t y_smem, bool accumulate) {
+  const uint32_t b_lo = umma_desc_lo_mnmajor(y_smem, kHalfBytes);
+  constexpr int kHalfSteps = kY / 32;
+#pragma unroll
+  for (int ks = 0; ks < 2 * kHalfSteps; ++ks)
+    umma_ts_lo<kIdescTS<kD, kF16>>(acc, w + ks / kHalfSteps * (kY / 2) + ks % kHalfSteps * 8, b_lo + ks * (2048 >> 4), (accumulate || ks > 0) ? 1u : 0u);
 }
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {

@@ -14,16 +14,16 @@
 //      [batch, heads_q, ceil128(max_seqlen_q)] workspace (rows past a sequence get lse = +inf,
 //      which later turns their P into exact zeros).
 //   2. bwd_tile_kernel<kModeDKDV>: one CTA per (batch, kv head, 128-key block). K and V tiles
-//      stay in shared memory; (Q, dO) tiles stream through a 2-stage TMA ring. Per Q tile:
+//      stay in shared memory; (Q, dO) tiles (of 128 rows, or 64 up to head_dim 64) stream through a TMA ring. Per Q tile:
 //      S^T = K Q^T and dP^T = V dO^T on tcgen05 into TMEM, two compute warpgroups (thread = key
-//      row = TMEM lane, one warpgroup per 64-query half of the tile) form P^T and dS^T, write
+//      row = TMEM lane, one warpgroup per half of the tile's queries) form P^T and dS^T, write
 //      them back to TMEM as bf16, and MMAs with the TMEM operand accumulate dV += P^T dO and
-//      dK += dS^T Q half by half (the streamed tiles are re-read in place as MN-major operands).
+//      dK += dS^T Q (the streamed tiles are re-read in place as MN-major operands).
 //   3. dQ, one of: bwd_tile_kernel<kModeDQ>, one CTA per (batch, query head, 128-query block); Q and dO
 //      stay, (K, V) stream; S = Q K^T, dP = dO V^T, dS -> TMEM, dQ += dS K. Or, where launch 2 has left its dS
 //      in the workspace as well (8 stores of 16 bytes per thread and item: 281 -> 308 us at B8 H16 L2048 D128
 //      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> 130).
-// TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512). The bf16 P and dS of an item both
+// TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512), or four times 64 columns. The bf16 P and dS of an item both
 // live in the item's score buffer, so the buffer that held dP is free as soon as it has been read;
 // the MMA issuer uses that (and, for dQ, the unused ACC2) to run the next item's score GEMMs and
 // exponentials under the current item's accumulation MMAs (buffer schedule at the issuer).
@@ -40,23 +40,40 @@
 namespace sdpa_b200 {
 namespace {
 
-// Ring of 32 KB streamed tiles Y1(0), Y2(0), Y1(1), Y2(1), ...: 4 slots for dK/dV (which also stages
-// the per-query vectors), 5 for dQ so that K(i+2) can land while item i is still accumulating.
-constexpr int kMaxStages = 5;
-__host__ __device__ constexpr int stages_for(int mode) { return mode == 1 ? 5 : 4; }
-constexpr int kThreads = 352;  // warps 0-3 / 4-7 compute (column halves), warp 8 TMA, warps 9 and 10 MMA issuers
+// Streamed tiles. Up to head_dim 64 they have 64 rows, so that a CTA's score buffers and accumulators take half of the tensor memory and two
+// CTAs share an SM: the one's exponentials run under the other's MMAs and waits, set-ups and epilogues. Above, the accumulators leave
+// no room for that. One chain of 128-row items per SM took as long as at head_dim 128. (Step of B8 H12 L512 with a mask 94.3 -> 88.9 us, B16
+// 153 -> 134, B8 H16 L2048 579 -> 526, B4 H12 L600 with a learned bias 152 -> 144. One warpgroup with 64 columns instead: 97.)
+template <int kD>
+constexpr int kRowsY = kD == 64 ? 64 : kTile;
+constexpr int kComputeWarps = 8;  // two warpgroups, each with half of an item's columns
+template <int kD>
+constexpr int kThreads = (kComputeWarps + (kD == 64 ? 4 : 3)) * 32;  // compute, TMA producer, two MMA issuers (and an idle warp)
+// Register hand-over of the instances with two CTAs per SM (setmaxnreg; launched with 80). What the third warpgroup releases
+// covers what the other two take, or the increase would wait forever.
+constexpr int kRegsCompute = 96, kRegsOther = 48;
+static_assert(2 * kRegsCompute + kRegsOther <= 3 * 80, "setmaxnreg.inc would wait forever");
+
+// Ring of streamed tiles Y1(0), Y2(0), Y1(1), Y2(1), ...: 4 slots of 32 KB (8 of 8 KB) for dK/dV, which also stages
+// the per-query vectors, 5 for dQ so that K(i+2) can land while item i is still accumulating.
+constexpr int kMaxStages = 8;
+__host__ __device__ constexpr int stages_for(int mode, int d) { return mode == 1 ? 5 : d == 64 ? 8 : 4; }
 constexpr int kModeDKDV = 0;
 constexpr int kModeDQ = 1;
 
-constexpr uint32_t kSmemX = 0;                                   // stationary pair, 64 KB
-constexpr uint32_t kSmemY = 2 * kTileBytes;                      // stages x 32 KB
-__host__ __device__ constexpr uint32_t smem_vec_off(int mode) { return kSmemY + stages_for(mode) * kTileBytes; }
+__host__ __device__ constexpr uint32_t x_bytes(int d) { return kTile * d * 2; }                     // one stationary tile
+__host__ __device__ constexpr uint32_t y_bytes(int d) { return (d == 64 ? 64 : kTile) * d * 2; }    // one streamed tile
+constexpr uint32_t kSmemX = 0;                                   // stationary pair
+__host__ __device__ constexpr uint32_t smem_y_off(int d) { return 2 * x_bytes(d); }
+__host__ __device__ constexpr uint32_t smem_vec_off(int mode, int d) { return smem_y_off(d) + stages_for(mode, d) * y_bytes(d); }
 // per-slot (lse2[128], delta[128]), dK/dV only
-__host__ __device__ constexpr uint32_t smem_bar_off(int mode) { return smem_vec_off(mode) + (mode == 1 ? 0 : stages_for(mode) * 1024); }
+__host__ __device__ constexpr uint32_t smem_bar_off(int mode, int d) { return smem_vec_off(mode, d) + (mode == 1 ? 0 : stages_for(mode, d) * 1024); }
 // behind the barriers, dQ with a key bias only: 64 16-bit bias values per compute warp
-__host__ __device__ constexpr uint32_t smem_key_bias_off(int mode) { return smem_bar_off(mode) + 256; }
-__host__ __device__ constexpr uint32_t smem_bytes_for(int mode, bool key_bias) {
-  return smem_key_bias_off(mode) + (mode == 1 && key_bias ? 8 * 128 : 0) + 1024;
+__host__ __device__ constexpr uint32_t smem_key_bias_off(int mode, int d) { return smem_bar_off(mode, d) + 256; }
+// at least 80 KB: a third CTA on the SM would wait for tensor memory
+__host__ __device__ constexpr uint32_t smem_bytes_for(int mode, int d, bool key_bias) {
+  const uint32_t used = smem_key_bias_off(mode, d) + (mode == 1 && key_bias ? 8 * 128 : 0) + 1024;
+  return used > 80 * 1024 ? used : 80 * 1024;
 }
 constexpr uint32_t kBarXFull = 0;
 constexpr uint32_t kBarYFull = 8;
@@ -100,7 +117,7 @@ enum BiasKind { kNoBias = 0, kFullBias = 1, kKeyBias = 2 };
 // exponentials and the dS stores behind branches the calls without dS were slower (dK/dV and dQ kernel of 6 packed sequences of 50 to 4000
 // tokens, 32/8 heads, unmasked: 1222 + 1076 us, so 1137 + 1019).
 template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads<kD>, kD == 64 ? 2 : 1)
 bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_o1, const __grid_constant__ CUtensorMap tm_o2,
@@ -120,9 +137,15 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // vectors complete. CTAs without work wait as well: a grid must not complete before the one in front of it.
   if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
     *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid; here, since block 0 may be one without work
-  constexpr int kStages = stages_for(kMode);
-  constexpr uint32_t kSmemVec = smem_vec_off(kMode);
-  constexpr uint32_t kSmemBar = smem_bar_off(kMode);
+  constexpr int kStages = stages_for(kMode, kD);
+  constexpr int kY = kRowsY<kD>;
+  constexpr int kC = kY / 2;  // columns per compute warpgroup, i.e. per thread
+  constexpr int kTmaWarp = kComputeWarps, kScoreWarp = kTmaWarp + 1, kAccWarp = kTmaWarp + 2;
+  constexpr uint32_t kTmemCols = 2 * kY + 2 * kD;
+  constexpr uint32_t kXBytes = x_bytes(kD), kYBytes = y_bytes(kD);
+  constexpr uint32_t kSmemY = smem_y_off(kD);
+  constexpr uint32_t kSmemVec = smem_vec_off(kMode, kD);
+  constexpr uint32_t kSmemBar = smem_bar_off(kMode, kD);
 
   // CTA order (1-D grid, block_order.cuh): heaviest blocks first (dK/dV: key block 0 sees every query; dQ: the last query block sees
   // every key). Packed, causal: blocks with the same number of blocks behind (dQ: in front of) them in their own
@@ -156,16 +179,16 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     return;
   }
 
-  // streamed tile range [y_lo, y_hi) (in tiles of 128) per head, and heads per CTA
+  // streamed tile range [y_lo, y_hi) (in tiles of kY rows) per head, and heads per CTA
   int y_lo = 0, y_hi = 0;
   if (kMode == kModeDKDV) {
-    y_hi = (len_q + kTile - 1) / kTile;
-    if (p.is_causal) y_lo = max(0, (x0 - causal_off) / kTile);  // first query tile with a row >= x0 - off
+    y_hi = (len_q + kY - 1) / kY;
+    if (p.is_causal) y_lo = max(0, (x0 - causal_off) / kY);  // first query tile with a row >= x0 - off
     if (p.is_causal && x0 - causal_off > len_q - 1) y_lo = y_hi;
   } else {
     int vis_end = len_k;
     if (p.is_causal) vis_end = min(len_k, x0 + kTile + causal_off);
-    y_hi = vis_end > 0 ? (vis_end + kTile - 1) / kTile : 0;
+    y_hi = vis_end > 0 ? (vis_end + kY - 1) / kY : 0;
   }
   const int tiles_per_head = max(0, y_hi - y_lo);
   const int heads_here = (kMode == kModeDKDV) ? p.kv_group : 1;
@@ -184,8 +207,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const CUtensorMap* tmy2 = (kMode == kModeDKDV) ? &tm_do : &tm_v;
   const int x_row = ((kMode == kModeDKDV) ? k_off : q_off) + x0;
   const int y_off = (kMode == kModeDKDV) ? q_off : k_off;
-  constexpr uint32_t kLoadBytes = kTile * kD * 2;  // bytes one tile brings in
-  constexpr int kPreloaded = 4;
+  constexpr int kPreloaded = kMode == kModeDQ ? 4 : kStages;
   // ring tile idx: Y1(idx/2) if even, Y2(idx/2) if odd; false when a wait gave up
   auto load_tile = [&](int idx) -> bool {
         const int i = idx >> 1;
@@ -218,16 +240,16 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // dK/dV streams the query heads of this KV head; dQ streams the KV head of this query head
         const int hy = (kMode == kModeDKDV) ? hx * p.kv_group + hi : hx / p.kv_group;
         const uint32_t full = bar + kBarYFull + 8 * s;
-        const uint32_t dst = base + kSmemY + s * kTileBytes;
-        const int row = y_off + yt * kTile;
+        const uint32_t dst = base + kSmemY + s * kYBytes;
+        const int row = y_off + yt * kY;
         const bool first = (idx & 1) == 0;
         if (kMode == kModeDKDV && first) {
-          mbar_arrive_expect_tx(full, kLoadBytes + 1024);
-          const size_t vec = (static_cast<size_t>(b) * p.heads_q + hy) * p.lq_pad + static_cast<size_t>(yt) * kTile;
-          bulk_load_1d(base + kSmemVec + s * 1024, p.nlse2 + vec, 512, full);
-          bulk_load_1d(base + kSmemVec + s * 1024 + 512, p.ndelta + vec, 512, full);
+          mbar_arrive_expect_tx(full, kYBytes + 2 * kY * 4);
+          const size_t vec = (static_cast<size_t>(b) * p.heads_q + hy) * p.lq_pad + static_cast<size_t>(yt) * kY;
+          bulk_load_1d(base + kSmemVec + s * 1024, p.nlse2 + vec, kY * 4, full);
+          bulk_load_1d(base + kSmemVec + s * 1024 + 512, p.ndelta + vec, kY * 4, full);
         } else {
-          mbar_arrive_expect_tx(full, kLoadBytes);
+          mbar_arrive_expect_tx(full, kYBytes);
         }
         const CUtensorMap* tm = first ? tmy1 : tmy2;
         tma_load_4d(dst, tm, full, 0, row, hy, bcoord);
@@ -235,7 +257,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     return true;
   };
 
-  if (warp == 8 && lane == 0) {
+  if (warp == kTmaWarp && lane == 0) {
     // descriptor fetches run under the barrier initialisation
     tma_prefetch_desc(tmx1);
     tma_prefetch_desc(tmy1);
@@ -249,24 +271,28 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     mbar_init(bar + kBarSFull, 1);
     mbar_init(bar + kBarSFull + 8, 1);
     mbar_init(bar + kBarDFull, 1);
-    mbar_init(bar + kBarDFree, 8);  // one arrival per compute warp
-    mbar_init(bar + kBarPFull, 8);
-    mbar_init(bar + kBarPFull + 8, 8);
-    mbar_init(bar + kBarP1Full, 8);
-    mbar_init(bar + kBarP1Full + 8, 8);
+    mbar_init(bar + kBarDFree, kComputeWarps);  // one arrival per compute warp
+    mbar_init(bar + kBarPFull, kComputeWarps);
+    mbar_init(bar + kBarPFull + 8, kComputeWarps);
+    mbar_init(bar + kBarP1Full, kComputeWarps);
+    mbar_init(bar + kBarP1Full + 8, kComputeWarps);
     mbar_init(bar + kBarWFree, 1);
     mbar_init(bar + kBarWFree + 8, 1);
     mbar_init(bar + kBarSIssued, 1);
-    mbar_init(bar + kBarEpiFull, 8);
+    mbar_init(bar + kBarEpiFull, kComputeWarps);
     mbar_init(bar + kBarAccFull, 1);
     *abort_flag = 0;
     fence_mbar_init();
     if (n_items > 0) {
-      mbar_arrive_expect_tx(bar + kBarXFull, 2 * kLoadBytes);
-      tma_load_4d(base + kSmemX, tmx1, bar + kBarXFull, 0, x_row, hx, bcoord);
-      if (kD > 64) tma_load_4d(base + kSmemX + kHalfBytes, tmx1, bar + kBarXFull, 64, x_row, hx, bcoord);
-      tma_load_4d(base + kSmemX + kTileBytes, tmx2, bar + kBarXFull, 0, x_row, hx, bcoord);
-      if (kD > 64) tma_load_4d(base + kSmemX + kTileBytes + kHalfBytes, tmx2, bar + kBarXFull, 64, x_row, hx, bcoord);
+      mbar_arrive_expect_tx(bar + kBarXFull, 2 * kXBytes);
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const CUtensorMap* tm = x == 0 ? tmx1 : tmx2;
+        const uint32_t dst = base + kSmemX + x * kXBytes;
+        tma_load_4d(dst, tm, bar + kBarXFull, 0, x_row, hx, bcoord);
+        if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, bar + kBarXFull, 64, x_row, hx, bcoord);
+        else tma_load_4d(dst + kYBytes, tm, bar + kBarXFull, 0, x_row + kY, hx, bcoord);  // the maps' boxes have kY rows
+      }
     }
     if (kMode == kModeDKDV) {
       wait_for_previous_grid();
@@ -276,213 +302,214 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   if (warp == 0) {
     __syncwarp();
-    tmem_alloc(base + kSmemBar + kSmemTmemPtr, 512);
+    tmem_alloc(base + kSmemBar + kSmemTmemPtr, kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  const uint32_t t1 = tmem_base, t2 = tmem_base + 128, acc1 = tmem_base + 256, acc2 = tmem_base + 384;
+  const uint32_t t1 = tmem_base, t2 = tmem_base + kY, acc1 = tmem_base + 2 * kY, acc2 = tmem_base + 2 * kY + kD;
 #ifdef SDPA_BWD_STAMPS
   const long long t_start = clock64();
   // a long-running block of batch 0, head 0 (non-causal: any; causal: the heaviest)
   const bool stamp_on = p.stamps != nullptr && b == 0 && hx == 0 &&
                         xb == ((kMode == kModeDKDV) ? 0 : p.order.ranks - 1) && (lane == 0) &&
-                        (warp == 0 || warp == 4 || warp == 9 || warp == 10);
+                        (warp == 0 || warp == 4 || warp == kScoreWarp || warp == kAccWarp);
 #endif
 
-  if (warp == 8) {
-    // ------------------------------------------------------------------ TMA producer (rest of the ring)
-    if (n_items > 0 && elect_one()) {
-      for (int idx = kPreloaded; idx < 2 * n_items; ++idx)
-        if (!load_tile(idx)) break;
-      drain_after_abort(abort_flag);
-    }
-  } else if (warp == 9 || warp == 10) {
-    // ------------------------------------------------------------------ MMA issuers
-    // One thread needs ~50-65 cycles to issue an MMA and ~70 for every barrier wait or commit, about
-    // as long as the tensor pipe needs to execute it, and an item has 24 (dQ) or 32 (dK/dV) MMAs
-    // plus half a dozen waits: a single issuer is the bottleneck. So two threads issue:
-    //   warp 9  the score GEMMs   S = X1 Y1^T, dP = X2 Y2^T            (operands in shared memory)
-    //   warp 10 the accumulations dV += P^T dO, dK += dS^T Q / dQ += dS K (A operand in TMEM)
-    // What the in-order pipe would guarantee between the two groups is a barrier here: `W free`
-    // (warp 10 commits it behind an item's accumulation MMAs; warp 9 waits for it before a score GEMM
-    // overwrites that item's P / dS buffer). There is one per item parity, so that the barrier a wait
-    // looks at cannot be a whole phase further on: its next phase belongs to item i+2, whose scores
-    // only exist after this wait.
-    if (n_items > 0 && elect_one()) {
-      // Where the score GEMMs of item i land:
-      //   dK/dV: S(i) in T[i&1], dP(i) in T[(i&1)^1]. The compute warpgroups put BOTH 16-bit results
-      //          (P and dS) into the S buffer, so the dP buffer is free once it has been read and
-      //          takes S(i+1) right away; dP(i+1) goes into the S buffer behind the accumulations.
-      //   dQ:    ACC2 is unused, so S alternates between T1 and ACC2 and dP always uses T2: S(i+2)
-      //          follows the accumulation of item i, dP(i+1) goes out as soon as dP(i) is read.
-      // Either way the next item's scores and exponentials run under this item's accumulation.
-      const uint32_t x1 = base + kSmemX, x2 = base + kSmemX + kTileBytes;
-      auto s_buf = [&](int i) { return kMode == kModeDKDV ? ((i & 1) ? t2 : t1) : ((i & 1) ? acc2 : t1); };
-      auto d_buf = [&](int i) { return kMode == kModeDKDV ? ((i & 1) ? t1 : t2) : t2; };
-      auto s_bar = [&](int i) { return bar + kBarSFull + (kMode == kModeDQ ? 8 * (i & 1) : 0); };
-      // ring position of tile 2i, kept incrementally (no division in the issue loop): slot = (2i) mod
-      // kStages, lap = (2i) / kStages. Tiles 2i + k, k < kStages, follow from it with one wrap.
-      // dQ splits its five slots into a K ring (slots 0-2) and a V ring (slots 3-4): a K tile lives
-      // from its score GEMM to its accumulation GEMM two items later, a V tile only for one GEMM, so a
-      // shared round-robin would free the slot V(i+1) needs too late to hide the load latency.
-      int ring_slot = 0, ring_lap = 0;  // dK/dV: position of tile 2i; dQ: i mod 3 and i / 3
-      int item = 0;
-      auto pos = [&](int k, int& slot, int& lap) {
-        if (kMode == kModeDKDV) {
-          slot = ring_slot + k;
-          lap = ring_lap;
-          if (slot >= kStages) { slot -= kStages; ++lap; }
-        } else if ((k & 1) == 0) {  // K(item + k/2)
-          slot = ring_slot + (k >> 1);
-          lap = ring_lap;
-          if (slot >= 3) { slot -= 3; ++lap; }
-        } else {  // V(item + k/2)
-          const int j = item + (k >> 1);
-          slot = 3 + (j & 1);
-          lap = j >> 1;
-        }
-      };
-      auto advance = [&]() {
-        ++item;
-        if (kMode == kModeDKDV) {
-          ring_slot += 2;
-          if (ring_slot >= kStages) { ring_slot -= kStages; ++ring_lap; }
-        } else if (++ring_slot == 3) {
-          ring_slot = 0;
-          ++ring_lap;
-        }
-      };
-      auto y_slot_k = [&](int k) { int sl, lp; pos(k, sl, lp); return base + kSmemY + sl * kTileBytes; };
-      auto y_wait_k = [&](int k) { int sl, lp; pos(k, sl, lp); return mbar_wait(bar + kBarYFull + 8 * sl, lp & 1, abort_flag); };
-      auto y_free_k = [&](int k) { int sl, lp; pos(k, sl, lp); umma_commit(bar + kBarYEmpty + 8 * sl); };
-      bool ok = true;
-      if (warp == 9) {
-        // ---------------- score GEMMs
+  if (warp >= kTmaWarp) {
+    if constexpr (kD == 64) reg_decrease<kRegsOther>();
+    if (warp == kTmaWarp) {
+      // ------------------------------------------------------------------ TMA producer (rest of the ring)
+      if (n_items > 0 && elect_one()) {
+        for (int idx = kPreloaded; idx < 2 * n_items; ++idx)
+          if (!load_tile(idx)) break;
+        drain_after_abort(abort_flag);
+      }
+    } else if (warp == kScoreWarp || warp == kAccWarp) {
+      // ------------------------------------------------------------------ MMA issuers
+      // One thread needs ~50-65 cycles to issue an MMA and ~70 for every barrier wait or commit, about
+      // as long as the tensor pipe needs to execute it, and an item has 24 (dQ) or 32 (dK/dV) MMAs
+      // plus half a dozen waits: a single issuer is the bottleneck. So two threads issue:
+      //   kScoreWarp the score GEMMs   S = X1 Y1^T, dP = X2 Y2^T            (operands in shared memory)
+      //   kAccWarp   the accumulations dV += P^T dO, dK += dS^T Q / dQ += dS K (A operand in TMEM)
+      // What the in-order pipe would guarantee between the two groups is a barrier here: `W free`
+      // (committed behind an item's accumulation MMAs; the score warp waits for it before a score GEMM
+      // overwrites that item's P / dS buffer). There is one per item parity, so that the barrier a wait
+      // looks at cannot be a whole phase further on: its next phase belongs to item i+2, whose scores
+      // only exist after this wait.
+      if (n_items > 0 && elect_one()) {
+        // Where the score GEMMs of item i land:
+        //   dK/dV: S(i) in T[i&1], dP(i) in T[(i&1)^1]. The compute warpgroups put BOTH 16-bit results
+        //          (P and dS) into the S buffer, so the dP buffer is free once it has been read and
+        //          takes S(i+1) right away; dP(i+1) goes into the S buffer behind the accumulations.
+        //   dQ:    ACC2 is unused, so S alternates between T1 and ACC2 and dP always uses T2: S(i+2)
+        //          follows the accumulation of item i, dP(i+1) goes out as soon as dP(i) is read.
+        // Either way the next item's scores and exponentials run under this item's accumulation.
+        const uint32_t x1 = base + kSmemX, x2 = base + kSmemX + kXBytes;
+        auto s_buf = [&](int i) { return kMode == kModeDKDV ? ((i & 1) ? t2 : t1) : ((i & 1) ? acc2 : t1); };
+        auto d_buf = [&](int i) { return kMode == kModeDKDV ? ((i & 1) ? t1 : t2) : t2; };
+        auto s_bar = [&](int i) { return bar + kBarSFull + (kMode == kModeDQ ? 8 * (i & 1) : 0); };
+        // ring position of tile 2i, kept incrementally (no division in the issue loop): slot = (2i) mod
+        // kStages, lap = (2i) / kStages. Tiles 2i + k, k < kStages, follow from it with one wrap.
+        // dQ splits its five slots into a K ring (slots 0-2) and a V ring (slots 3-4): a K tile lives
+        // from its score GEMM to its accumulation GEMM two items later, a V tile only for one GEMM, so a
+        // shared round-robin would free the slot V(i+1) needs too late to hide the load latency.
+        int ring_slot = 0, ring_lap = 0;  // dK/dV: position of tile 2i; dQ: i mod 3 and i / 3
+        int item = 0;
+        auto pos = [&](int k, int& slot, int& lap) {
+          if (kMode == kModeDKDV) {
+            slot = ring_slot + k;
+            lap = ring_lap;
+            if (slot >= kStages) { slot -= kStages; ++lap; }
+          } else if ((k & 1) == 0) {  // K(item + k/2)
+            slot = ring_slot + (k >> 1);
+            lap = ring_lap;
+            if (slot >= 3) { slot -= 3; ++lap; }
+          } else {  // V(item + k/2)
+            const int j = item + (k >> 1);
+            slot = 3 + (j & 1);
+            lap = j >> 1;
+          }
+        };
+        auto advance = [&]() {
+          ++item;
+          if (kMode == kModeDKDV) {
+            ring_slot += 2;
+            if (ring_slot >= kStages) { ring_slot -= kStages; ++ring_lap; }
+          } else if (++ring_slot == 3) {
+            ring_slot = 0;
+            ++ring_lap;
+          }
+        };
+        auto y_slot_k = [&](int k) { int sl, lp; pos(k, sl, lp); return base + kSmemY + sl * kYBytes; };
+        auto y_wait_k = [&](int k) { int sl, lp; pos(k, sl, lp); return mbar_wait(bar + kBarYFull + 8 * sl, lp & 1, abort_flag); };
+        auto y_free_k = [&](int k) { int sl, lp; pos(k, sl, lp); umma_commit(bar + kBarYEmpty + 8 * sl); };
+        bool ok = true;
+        if (warp == kScoreWarp) {
+          // ---------------- score GEMMs
 #ifdef SDPA_BWD_STAMPS
-        if (stamp_on) p.stamps[((kMode * 4 + 2) * 24 + 23) * 8 + 0] = static_cast<float>(t_start - t_entry);
+          if (stamp_on) p.stamps[((kMode * 4 + 2) * 24 + 23) * 8 + 0] = static_cast<float>(t_start - t_entry);
 #endif
-        ok = mbar_wait(bar + kBarXFull, 0, abort_flag) && y_wait_k(0);
-        BWD_STAMP(2, 23, 1);
-        if (ok) {
-          tc_fence_after_sync();
-          issue_xyT<kD, kF16>(s_buf(0), x1, y_slot_k(0));
-          umma_commit(s_bar(0));
-        }
-        BWD_STAMP(2, 23, 2);
-        ok = ok && y_wait_k(1);
-        if (ok) {
-          tc_fence_after_sync();
-          issue_xyT<kD, kF16>(d_buf(0), x2, y_slot_k(1));
-          umma_commit(bar + kBarDFull);
-        }
-        if (kMode == kModeDQ && ok && n_items > 1) {
-          ok = y_wait_k(2);
+          ok = mbar_wait(bar + kBarXFull, 0, abort_flag) && y_wait_k(0);
+          BWD_STAMP(2, 23, 1);
           if (ok) {
             tc_fence_after_sync();
-            issue_xyT<kD, kF16>(s_buf(1), x1, y_slot_k(2));
-            umma_commit(s_bar(1));
+            issue_xyT<kD, kF16, kY>(s_buf(0), x1, y_slot_k(0));
+            umma_commit(s_bar(0));
           }
-        }
-        for (int i = 0; ok && i < n_items; ++i, advance()) {
-          const uint32_t sbuf = s_buf(i);
-          const bool more = i + 1 < n_items;
-          BWD_STAMP(2, i, 0);
-          // dP(i) has left TMEM once all compute warps have read it
-          ok = mbar_wait(bar + kBarDFree, i & 1, abort_flag);
-          if (!ok) break;
-          BWD_STAMP(2, i, 1);
-          if (kMode == kModeDKDV) {
-            if (!more) {
-              mbar_arrive(bar + kBarSIssued);
-              continue;
-            }
-            ok = y_wait_k(2);
-            if (!ok) break;
+          BWD_STAMP(2, 23, 2);
+          ok = ok && y_wait_k(1);
+          if (ok) {
             tc_fence_after_sync();
-            issue_xyT<kD, kF16>(d_buf(i), x1, y_slot_k(2));  // S(i+1) into the buffer dP(i) has just left
-            umma_commit(s_bar(i + 1));
-            // S(i+1) is what the compute warps wait for; dK(i) is not urgent. The other issuer holds
-            // dK(i) back until this arrival, so the two GEMMs do not share the pipe MMA by MMA.
-            mbar_arrive(bar + kBarSIssued);
-            BWD_STAMP(2, i, 2);
-            ok = mbar_wait(bar + kBarWFree + 8 * (i & 1), (i >> 1) & 1, abort_flag) && y_wait_k(3);
-            if (!ok) break;
-            BWD_STAMP(2, i, 3);
-            tc_fence_after_sync();
-            issue_xyT<kD, kF16>(sbuf, x2, y_slot_k(3));  // dP(i+1) into the buffer P(i), dS(i) have left
+            issue_xyT<kD, kF16, kY>(d_buf(0), x2, y_slot_k(1));
             umma_commit(bar + kBarDFull);
-            BWD_STAMP(2, i, 4);
-          } else {
-            if (more) {
-              ok = y_wait_k(3);
+          }
+          if (kMode == kModeDQ && ok && n_items > 1) {
+            ok = y_wait_k(2);
+            if (ok) {
+              tc_fence_after_sync();
+              issue_xyT<kD, kF16, kY>(s_buf(1), x1, y_slot_k(2));
+              umma_commit(s_bar(1));
+            }
+          }
+          for (int i = 0; ok && i < n_items; ++i, advance()) {
+            const uint32_t sbuf = s_buf(i);
+            const bool more = i + 1 < n_items;
+            BWD_STAMP(2, i, 0);
+            // dP(i) has left TMEM once all compute warps have read it
+            ok = mbar_wait(bar + kBarDFree, i & 1, abort_flag);
+            if (!ok) break;
+            BWD_STAMP(2, i, 1);
+            if (kMode == kModeDKDV) {
+              if (!more) {
+                mbar_arrive(bar + kBarSIssued);
+                continue;
+              }
+              ok = y_wait_k(2);
               if (!ok) break;
               tc_fence_after_sync();
-              issue_xyT<kD, kF16>(t2, x2, y_slot_k(3));  // dP(i+1)
-              umma_commit(bar + kBarDFull);
-            }
-            BWD_STAMP(2, i, 2);
-            if (i + 2 < n_items) {
-              ok = mbar_wait(bar + kBarWFree + 8 * (i & 1), (i >> 1) & 1, abort_flag) && y_wait_k(4);
+              issue_xyT<kD, kF16, kY>(d_buf(i), x1, y_slot_k(2));  // S(i+1) into the buffer dP(i) has just left
+              umma_commit(s_bar(i + 1));
+              // S(i+1) is what the compute warps wait for; dK(i) is not urgent. The other issuer holds
+              // dK(i) back until this arrival, so the two GEMMs do not share the pipe MMA by MMA.
+              mbar_arrive(bar + kBarSIssued);
+              BWD_STAMP(2, i, 2);
+              ok = mbar_wait(bar + kBarWFree + 8 * (i & 1), (i >> 1) & 1, abort_flag) && y_wait_k(3);
               if (!ok) break;
               BWD_STAMP(2, i, 3);
               tc_fence_after_sync();
-              issue_xyT<kD, kF16>(sbuf, x1, y_slot_k(4));  // S(i+2) into the buffer dS(i) has left
-              umma_commit(s_bar(i + 2));
+              issue_xyT<kD, kF16, kY>(sbuf, x2, y_slot_k(3));  // dP(i+1) into the buffer P(i), dS(i) have left
+              umma_commit(bar + kBarDFull);
               BWD_STAMP(2, i, 4);
+            } else {
+              if (more) {
+                ok = y_wait_k(3);
+                if (!ok) break;
+                tc_fence_after_sync();
+                issue_xyT<kD, kF16, kY>(t2, x2, y_slot_k(3));  // dP(i+1)
+                umma_commit(bar + kBarDFull);
+              }
+              BWD_STAMP(2, i, 2);
+              if (i + 2 < n_items) {
+                ok = mbar_wait(bar + kBarWFree + 8 * (i & 1), (i >> 1) & 1, abort_flag) && y_wait_k(4);
+                if (!ok) break;
+                BWD_STAMP(2, i, 3);
+                tc_fence_after_sync();
+                issue_xyT<kD, kF16, kY>(sbuf, x1, y_slot_k(4));  // S(i+2) into the buffer dS(i) has left
+                umma_commit(s_bar(i + 2));
+                BWD_STAMP(2, i, 4);
+              }
             }
           }
-        }
-      } else {
-        // ---------------- accumulation GEMMs
-        ok = mbar_wait(bar + kBarXFull, 0, abort_flag);
-        for (int i = 0; ok && i < n_items; ++i, advance()) {
-          const uint32_t y1 = y_slot_k(0), y2 = y_slot_k(1);
-          const uint32_t sbuf = s_buf(i);
-          // the tiles have landed long ago (the other issuer has used them); this wait makes the
-          // copies visible to this thread's MMAs as well
-          ok = y_wait_k(0) && (kMode == kModeDQ || y_wait_k(1));
-          if (!ok) break;
-          if (kMode == kModeDKDV) {
-            // dV needs P only, which is stored a whole dS pass before the item is complete
-            ok = mbar_wait(bar + kBarP1Full + 8 * (i & 1), (i >> 1) & 1, abort_flag);
+        } else {
+          // ---------------- accumulation GEMMs
+          ok = mbar_wait(bar + kBarXFull, 0, abort_flag);
+          for (int i = 0; ok && i < n_items; ++i, advance()) {
+            const uint32_t y1 = y_slot_k(0), y2 = y_slot_k(1);
+            const uint32_t sbuf = s_buf(i);
+            // the tiles have landed long ago (the other issuer has used them); this wait makes the
+            // copies visible to this thread's MMAs as well
+            ok = y_wait_k(0) && (kMode == kModeDQ || y_wait_k(1));
             if (!ok) break;
+            if (kMode == kModeDKDV) {
+              // dV needs P only, which is stored a whole dS pass before the item is complete
+              ok = mbar_wait(bar + kBarP1Full + 8 * (i & 1), (i >> 1) & 1, abort_flag);
+              if (!ok) break;
+              tc_fence_after_sync();
+              issue_wy<kD, kF16, kY>(acc1, sbuf, y2, i > 0);  // dV += P^T dO
+            }
+            BWD_STAMP(3, i, 0);
+            ok = mbar_wait(bar + kBarPFull + 8 * (i & 1), (i >> 1) & 1, abort_flag);
+            if (!ok) break;
+            BWD_STAMP(3, i, 1);
             tc_fence_after_sync();
-            issue_wy_half<kD, kF16>(acc1, sbuf, y2, 0, i > 0);       // dV += P^T dO
-            issue_wy_half<kD, kF16>(acc1, sbuf + 64, y2, 1, true);
+            if (kMode == kModeDKDV) {
+              ok = mbar_wait(bar + kBarSIssued, i & 1, abort_flag);
+              if (!ok) break;
+              issue_wy<kD, kF16, kY>(acc2, sbuf + kC / 2, y1, i > 0);  // dK += dS^T Q
+              y_free_k(0);  // releases the slot pair Q(i), dO(i)
+            } else {
+              issue_wy<kD, kF16, kY>(acc1, sbuf + kC / 2, y1, i > 0);  // dQ += dS K
+            }
+            umma_commit(bar + kBarWFree + 8 * (i & 1));
+            if (i == n_items - 1) umma_commit(bar + kBarAccFull);
+            BWD_STAMP(3, i, 2);
+            if (i == 0) BWD_STAMP(3, 23, 0);
+            if (i == n_items - 1) BWD_STAMP(3, 23, 1);
           }
-          BWD_STAMP(3, i, 0);
-          ok = mbar_wait(bar + kBarPFull + 8 * (i & 1), (i >> 1) & 1, abort_flag);
-          if (!ok) break;
-          BWD_STAMP(3, i, 1);
-          tc_fence_after_sync();
-          if (kMode == kModeDKDV) {
-            ok = mbar_wait(bar + kBarSIssued, i & 1, abort_flag);
-            if (!ok) break;
-            issue_wy_half<kD, kF16>(acc2, sbuf + 32, y1, 0, i > 0);  // dK += dS^T Q
-            issue_wy_half<kD, kF16>(acc2, sbuf + 96, y1, 1, true);
-            y_free_k(0);  // releases the slot pair Q(i), dO(i)
-          } else {
-            issue_wy_half<kD, kF16>(acc1, sbuf + 32, y1, 0, i > 0);  // dQ += dS K
-            issue_wy_half<kD, kF16>(acc1, sbuf + 96, y1, 1, true);
-          }
-          umma_commit(bar + kBarWFree + 8 * (i & 1));
-          if (i == n_items - 1) umma_commit(bar + kBarAccFull);
-          BWD_STAMP(3, i, 2);
-          if (i == 0) BWD_STAMP(3, 23, 0);
-          if (i == n_items - 1) BWD_STAMP(3, 23, 1);
         }
       }
     }
-  } else if (warp < 8) {
+  } else {
     // ------------------------------------------------------------------ compute warpgroups
-    // warps 0-3 own streamed columns [0,64) of every stationary row, warps 4-7 columns [64,128)
+    if constexpr (kD == 64) reg_increase<kRegsCompute>();
+    // warps 0-3 own the first kC streamed columns of every stationary row, warps 4-7 the others
     const int half = warp >> 2;
     const int r = (warp & 3) * 32 + lane;  // stationary row in the tile = TMEM lane
     const int xr = x0 + r;                 // key index (dK/dV) or query index (dQ) within the sequence
-    const uint32_t lane_base = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * 64;
+    const uint32_t lane_base = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * kC;
     const float c = p.scale_log2;
     bool ok = true;
     float my_nlse2 = 0.f, my_ndelta = 0.f;
@@ -500,11 +527,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int i = 0; i < n_items; ++i) {
       const int s = (2 * i) % kStages;  // ring slot of Y1(i), which carries the per-query vectors
       const int hi = i / tiles_per_head;
-      const int y0 = (y_lo + (i - hi * tiles_per_head)) * kTile;
+      const int y0 = (y_lo + (i - hi * tiles_per_head)) * kY;
       const uint32_t sbuf = (kMode == kModeDKDV ? ((i & 1) ? t2 : t1) : ((i & 1) ? acc2 : t1)) + lane_base;
       const uint32_t dbuf = (kMode == kModeDKDV ? ((i & 1) ? t1 : t2) : t2) + lane_base;
       BWD_STAMP(half, i, 0);
-      // keep bits of this thread's 64 (row, column) pairs, in flight under the waits below
+      // keep bits of this thread's kC (row, column) pairs, in flight under the waits below
       uint2 keep = make_uint2(0u, 0u);
       if constexpr (kDrop) {
         const uint32_t* words =
@@ -516,13 +543,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                                      ? static_cast<size_t>(hx * p.kv_group + hi) * p.keep_k_rows + k_off + xr
                                      : static_cast<size_t>(b * p.heads_q + hx * p.kv_group + hi) * p.keep_k_rows + xr) *
                                     (p.keep_lq_pad >> 5);
-        keep = *reinterpret_cast<const uint2*>(words + ((y0 + half * 64) >> 5));
+        if constexpr (kC == 64) keep = *reinterpret_cast<const uint2*>(words + ((y0 + half * kC) >> 5));
+        else keep.x = words[(y0 + half * kC) >> 5];
       }
-      uint32_t key_bias_raw = 0u;  // dK/dV: this key's value; dQ: the values of two of the 64 keys
+      uint32_t key_bias_raw = 0u;  // dK/dV: this key's value; dQ: the values of two of the kC keys
       if constexpr (kBias == kKeyBias) {
         const uint16_t* head = p.bias + b * p.bias_batch_stride + (kMode == kModeDQ ? hx : hx * p.kv_group + hi) * p.bias_head_stride;
-        const int key = y0 + half * 64 + 2 * lane;
-        if (kMode == kModeDQ && key < len_k) key_bias_raw = *reinterpret_cast<const uint32_t*>(head + key);
+        const int key = y0 + half * kC + 2 * lane;
+        if (kMode == kModeDQ && 2 * lane < kC && key < len_k) key_bias_raw = *reinterpret_cast<const uint32_t*>(head + key);
         if (kMode == kModeDKDV && xr < len_k) key_bias_raw = head[xr];
       }
       if constexpr (kBias == kFullBias) {
@@ -530,13 +558,13 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // row; dK/dV: 64 query rows, two per lane, 64 bytes each around this warp's keys)
         if (i + 1 < n_items && xr < len_x) {
           const int hn = (i + 1) / tiles_per_head;
-          const int cn = (y_lo + (i + 1 - hn * tiles_per_head)) * kTile + half * 64;
+          const int cn = (y_lo + (i + 1 - hn * tiles_per_head)) * kY + half * kC;
           if (kMode == kModeDQ) {
             const uint16_t* nx = p.bias + b * p.bias_batch_stride + hx * p.bias_head_stride +
                                  static_cast<int64_t>(xr) * p.bias_row_stride + cn;
             if (cn < len_k) {  // only addresses inside the row
               prefetch_l2(nx);
-              prefetch_l2(nx + min(63, len_k - 1 - cn));
+              prefetch_l2(nx + min(kC - 1, len_k - 1 - cn));
             }
           } else {
             if (p.bias_t != nullptr) {
@@ -544,11 +572,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                                    static_cast<int64_t>(xr) * p.bias_t_row_stride + cn;
               if (cn < len_q) {
                 prefetch_l2(nx);
-                prefetch_l2(nx + min(63, len_q - 1 - cn));
+                prefetch_l2(nx + min(kC - 1, len_q - 1 - cn));
               }
             } else {
               const uint16_t* nx = p.bias + b * p.bias_batch_stride + (hx * p.kv_group + hn) * p.bias_head_stride + xr;
-              const int q = cn + 2 * lane;
+              const int q = 2 * lane < kC ? cn + 2 * lane : len_q;
               if (q < len_q) prefetch_l2(nx + static_cast<int64_t>(q) * p.bias_row_stride);
               if (q + 1 < len_q) prefetch_l2(nx + static_cast<int64_t>(q + 1) * p.bias_row_stride);
             }
@@ -558,10 +586,10 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // This item's bias values where they are contiguous for this thread (dQ: its query row; dK/dV: its key's row
       // of the transposed copy): eight 16-byte loads issued before the waits, so their latency passes under the
       // score GEMM. A chunk that starts past the end is skipped (zeros); one that straddles it reads row padding.
-      uint4 bw[kBias == kFullBias ? 8 : 1];
+      uint4 bw[kBias == kFullBias ? kC / 8 : 1];
       bool bias_in_regs = false;
       if constexpr (kBias == kFullBias) {
-        const int col0 = y0 + half * 64;
+        const int col0 = y0 + half * kC;
         const uint16_t* vrow = nullptr;
         int vlen = 0;
         if (kMode == kModeDQ) {
@@ -575,7 +603,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         bias_in_regs = vrow != nullptr;
         if (bias_in_regs) {
 #pragma unroll
-          for (int ch = 0; ch < 8; ++ch) {
+          for (int ch = 0; ch < kC / 8; ++ch) {
             bw[ch] = make_uint4(0u, 0u, 0u, 0u);
             if (xr < len_x && col0 + ch * 8 < vlen) bw[ch] = *reinterpret_cast<const uint4*>(vrow + col0 + ch * 8);
           }
@@ -592,7 +620,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!ok) break;
       tc_fence_after_sync();
       BWD_STAMP(half, i, 1);
-      const float* vec_nlse = reinterpret_cast<const float*>(smem + kSmemVec + s * 1024) + half * 64;
+      const float* vec_nlse = reinterpret_cast<const float*>(smem + kSmemVec + s * 1024) + half * kC;
       const float* vec_ndelta = vec_nlse + 128;
       // visibility of element (row xr, column y0 + j)
       //   dK/dV: key xr, query y0+j : visible iff xr <= y0 + j + off  <=>  j >= xr - off - y0
@@ -606,23 +634,23 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         j_hi = len_k - y0;
         if (p.is_causal) j_hi = min(j_hi, xr + causal_off + 1 - y0);
       }
-      j_lo -= half * 64;  // relative to this thread's 64 columns
-      j_hi -= half * 64;
+      j_lo -= half * kC;  // relative to this thread's columns
+      j_hi -= half * kC;
 
       // phase 1 (needs S only): P = exp2(S c - lse2), masked; its bf16 copy goes back at once
-      float pr[64];
+      float pr[kC];
       {
-        uint32_t a[64];
+        uint32_t a[kC];
         tmem_ld_x32_at<0>(sbuf, a);
-        tmem_ld_x32_at<32>(sbuf + 32, a);
+        if constexpr (kC > 32) tmem_ld_x32_at<32>(sbuf + 32, a);
         tmem_wait_ld();
         BWD_STAMP(half, i, 2);
         if constexpr (kBias == kFullBias) {
           // S <- S + bias / scale (then x = S c - lse2 as without bias)
-          const int col0 = y0 + half * 64;
+          const int col0 = y0 + half * kC;
           if (bias_in_regs) {
 #pragma unroll
-            for (int ch = 0; ch < 8; ++ch) {
+            for (int ch = 0; ch < kC / 8; ++ch) {
               const uint32_t ww[4] = {bw[ch].x, bw[ch].y, bw[ch].z, bw[ch].w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -632,11 +660,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               }
             }
           } else if (kMode == kModeDKDV && xr < len_x) {
-            // no transposed copy: this key in 64 consecutive query rows, 64 two-byte loads (consecutive lanes on
+            // no transposed copy: this key in kC consecutive query rows, as many two-byte loads (consecutive lanes on
             // consecutive keys)
             const uint16_t* bcol = p.bias + b * p.bias_batch_stride + (hx * p.kv_group + hi) * p.bias_head_stride + xr;
 #pragma unroll
-            for (int j = 0; j < 64; ++j) {
+            for (int j = 0; j < kC; ++j) {
               if (col0 + j < len_q) {
                 const uint32_t raw = bcol[static_cast<int64_t>(col0 + j) * p.bias_row_stride];
                 const float bv = unpack_16x2<kF16>(raw).x;
@@ -647,25 +675,25 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         constexpr float kLog2e = 1.4426950408889634f;
         float key_bias = 0.f, key_bias_log2 = 0.f;  // dK/dV
-        uint32_t* key_bias_row = reinterpret_cast<uint32_t*>(smem + smem_key_bias_off(kMode) + warp * 128);  // dQ
+        uint32_t* key_bias_row = reinterpret_cast<uint32_t*>(smem + smem_key_bias_off(kMode, kD) + warp * 128);  // dQ
         if constexpr (kBias == kKeyBias) {
           if (kMode == kModeDKDV) {
             key_bias = unpack_16x2<kF16>(key_bias_raw).x;
             key_bias_log2 = key_bias * kLog2e;
           } else {
-            key_bias_row[lane] = key_bias_raw;  // the previous item's values were read before this warp's last __syncwarp
+            if (2 * lane < kC) key_bias_row[lane] = key_bias_raw;  // the previous item's values were read before this warp's last __syncwarp
             __syncwarp();
           }
         }
         // x = S c - lse2. kPolyOf4 of every four column pairs take their 2^x from the FMA pipe (exp2_poly3_x2). dQ: one; two already
-        // cost issue slots. dK/dV: two, which shortens the chain of an item (step of B8 H12 L512 D64 with a mask 96.3 us, without any
-        // 97.5; B1 H8 L2048 D128 78.7, 82.0) - but none where dS goes through the workspace: those grids are full and run at the power
+        // cost issue slots. dK/dV: two, which shortens the chain of an item (step of B1 H8 L2048 D128 78.7 us, without any 82.0). None up to
+        // head_dim 64: with two CTAs per SM one of four takes the same time (B8 H12 L1000 126, 126). And none where dS goes through the workspace: those grids are full and run at the power
         // cap, where none to two take the same time (step of B8 H16 L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed
         // 64 to 2048 tokens 369, 368, 364), and none is the most exact. Such a call without room for dS takes these two kernels, and its
         // bits must not tell: none here either, and the same roundings in both kernels (a key bias joins with one).
-        constexpr int kPolyOf4 = kDsCall ? 0 : kMode == kModeDQ ? 1 : 2;
+        constexpr int kPolyOf4 = kDsCall || kD == 64 ? 0 : kMode == kModeDQ ? 1 : 2;
 #pragma unroll
-        for (int j4 = 0; j4 < 16; ++j4) {
+        for (int j4 = 0; j4 < kC / 4; ++j4) {
           const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_nlse + 4 * j4) : make_float4(my_nlse2, my_nlse2, my_nlse2, my_nlse2);
           uint2 kb = make_uint2(0u, 0u);
           if constexpr (kBias == kKeyBias && kMode == kModeDQ) kb = *reinterpret_cast<const uint2*>(key_bias_row + 2 * j4);
@@ -691,14 +719,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         // only tiles on the causal diagonal or past the end of the keys need the element mask
-        if (__any_sync(0xffffffffu, j_lo > 0 || j_hi < 64)) {
+        if (__any_sync(0xffffffffu, j_lo > 0 || j_hi < kC)) {
 #pragma unroll
-          for (int j = 0; j < 64; ++j) pr[j] = (j >= j_lo && j < j_hi) ? pr[j] : 0.f;
+          for (int j = 0; j < kC; ++j) pr[j] = (j >= j_lo && j < j_hi) ? pr[j] : 0.f;
         }
         if (kMode == kModeDKDV) {
-          uint32_t pw[32];
+          uint32_t pw[kC / 2];
 #pragma unroll
-          for (int j2 = 0; j2 < 32; ++j2) {
+          for (int j2 = 0; j2 < kC / 2; ++j2) {
             if constexpr (kDrop) {
               const uint32_t word = j2 < 16 ? keep.x : keep.y;
               pw[j2] = pack_16x2<kF16>(kept(word, (2 * j2) & 31, pr[2 * j2]), kept(word, (2 * j2 + 1) & 31, pr[2 * j2 + 1]));
@@ -707,7 +735,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
           }
           tmem_st_x16(sbuf, pw);
-          tmem_st_x16(sbuf + 16, pw + 16);
+          if constexpr (kC > 32) tmem_st_x16(sbuf + 16, pw + 16);
           tmem_wait_st();
           tc_fence_before_sync();
           __syncwarp();
@@ -720,18 +748,18 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!ok) break;
       tc_fence_after_sync();
       BWD_STAMP(half, i, 4);
-      uint32_t dw[32];
+      uint32_t dw[kC / 2];
       {
-        uint32_t d[64];
+        uint32_t d[kC];
         tmem_ld_x32_at<0>(dbuf, d);
-        tmem_ld_x32_at<32>(dbuf + 32, d);
+        if constexpr (kC > 32) tmem_ld_x32_at<32>(dbuf + 32, d);
         tmem_wait_ld();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar + kBarDFree);  // the dP buffer may be overwritten
         BWD_STAMP(half, i, 5);
 #pragma unroll
-        for (int j4 = 0; j4 < 16; ++j4) {
+        for (int j4 = 0; j4 < kC / 4; ++j4) {
           const float4 l = (kMode == kModeDKDV) ? read_vec4<kDrop>(vec_ndelta + 4 * j4) : make_float4(my_ndelta, my_ndelta, my_ndelta, my_ndelta);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -748,16 +776,16 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             dw[j >> 1] = pack_16x2<kF16>(e.x, e.y);
           }
         }
-        tmem_st_x16(sbuf + 32, dw);
-        tmem_st_x16(sbuf + 48, dw + 16);
+        tmem_st_x16(sbuf + kC / 2, dw);
+        if constexpr (kC > 32) tmem_st_x16(sbuf + kC / 2 + 16, dw + 16);
         if constexpr (kBias == kFullBias && kMode == kModeDQ) {
-          // dbias = dS: this thread's 64 keys of its query row, already packed for the dQ GEMM
-          const int col0 = y0 + half * 64;
+          // dbias = dS: this thread's keys of its query row, already packed for the dQ GEMM
+          const int col0 = y0 + half * kC;
           if (p.dbias != nullptr && xr < len_x) {
             uint16_t* drow = p.dbias + b * p.dbias_batch_stride + hx * p.dbias_head_stride +
                              static_cast<int64_t>(xr) * p.dbias_row_stride + col0;
 #pragma unroll
-            for (int ch = 0; ch < 8; ++ch)
+            for (int ch = 0; ch < kC / 8; ++ch)
               if (col0 + ch * 8 < len_k)
                 *reinterpret_cast<uint4*>(drow + ch * 8) = make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]);
           }
@@ -775,7 +803,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (ds_tile < p.ds.capacity) {
           uint4* dst = ds_group(p.ds, ds_tile, half * 8, r);
 #pragma unroll
-          for (int ch = 0; ch < 8; ++ch)
+          for (int ch = 0; ch < kC / 8; ++ch)
             dst[ch * kDsTile] = make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]);
         }
         // past this row of tiles; behind the last one the next head's tiles begin
@@ -798,6 +826,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // last rows would spill into the next sequence and is written row by row instead.
       const bool use_tma = (p.cu_q == nullptr) || (x0 + kTile <= len_x);
       const int n_out = (kMode == kModeDKDV) ? 2 : 1;
+      constexpr int kColumns = kD / 2;  // head_dim columns per warpgroup
 #pragma unroll
       for (int which = 0; which < n_out; ++which) {
         uint16_t* dst;
@@ -823,11 +852,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           acc = acc2;
         }
 #pragma unroll
-        // this warpgroup converts head_dim columns [half * kD/2, (half + 1) * kD/2)
-        for (int cc = 0; cc < kD / 64; ++cc) {
+        // this warpgroup converts its share of the head_dim columns
+        for (int cc = 0; cc < kColumns / 32; ++cc) {
           uint32_t v[32];
           if (n_items > 0) {
-            tmem_ld_x32(acc + (lane_base - half * 64) + half * (kD / 2) + cc * 32, v);
+            tmem_ld_x32(acc + (lane_base - half * kC) + half * kColumns + cc * 32, v);
             tmem_wait_ld();
           } else {
 #pragma unroll
@@ -841,11 +870,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             w[j].z = pack_16x2<kF16>(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul);
             w[j].w = pack_16x2<kF16>(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul);
           }
-          const int col = half * (kD / 2) + cc * 32;  // first of this thread's 32 columns
+          const int col = half * kColumns + cc * 32;  // first of this thread's 32 columns
           if (use_tma) {
-            // output tile `which` is staged in ring slot `which`: two 64-column halves of 128-byte rows
+            // output tile `which` is staged in the ring: 64-column halves of 128-byte rows
             // in the 128-byte-swizzled layout the tensor map expects
-            uint8_t* row = smem + kSmemY + which * kTileBytes + (col >> 6) * kHalfBytes + r * 128;
+            uint8_t* row = smem + kSmemY + which * kXBytes + (col >> 6) * kHalfBytes + r * 128;
             const int chunk0 = (col & 63) >> 3;
 #pragma unroll
             for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(row + (((chunk0 + j) ^ (r & 7)) << 4)) = w[j];
@@ -869,7 +898,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const CUtensorMap* tm = (which == 0) ? &tm_o1 : &tm_o2;
 #pragma unroll
               for (int ht = 0; ht < kD / 64; ++ht)
-                tma_store_4d(tm, base + kSmemY + which * kTileBytes + ht * kHalfBytes, ht * 64, row0, hx, bcoord);
+                tma_store_4d(tm, base + kSmemY + which * kXBytes + ht * kHalfBytes, ht * 64, row0, hx, bcoord);
             }
             tma_store_commit();
             tma_store_wait_read();  // the shared memory must outlive the stores' reads of it
@@ -879,12 +908,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   }
 
-  if (warp < 8) BWD_STAMP(warp >> 2, 23, 1);
+  if (warp < kTmaWarp) BWD_STAMP(warp >> 2, 23, 1);
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, kTmemCols);
   }
   if (warp == 0) BWD_STAMP(0, 23, 2);
   if (threadIdx.x == 0 && *abort_flag != 0) atomicExch(p.status, SDPA_B200_DEVICE_TIMEOUT);
@@ -1034,7 +1063,8 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
                                                                                                               : kFullBias;
   TileKernel kernel = mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16, kp.ds_call != 0)
                                         : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16, kp.ds_call != 0);
-  const uint32_t smem = smem_bytes_for(mode, bias == kKeyBias);
+  const int dim = head_dim <= 64 ? 64 : 128;  // the instance
+  const uint32_t smem = smem_bytes_for(mode, dim, bias == kKeyBias);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) {
     set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", smem, cudaGetErrorString(err));
@@ -1042,7 +1072,7 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(dim == 64 ? kThreads<64> : kThreads<128>);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -1070,10 +1100,11 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 //    the dK/dV kernel waits for a whole chain of items while SMs are idle. (B1 H8 L2048 D128 step 85, through dS 95, fused 103; B4
 //    H8/1 L4096 545, 564, 800; the other way round only where few key blocks meet many queries: B2 H32/8 L1024 unmasked 124, 112.)
 //  * a bias gradient: the same two, since the dQ kernel, whose threads own query rows, writes it.
-//  * head_dim 64, more key blocks, no bias, no fixed order asked for: the fused kernel. Its items are cheap against a second pass over
-//    the scores or over dS, whose traffic is the same as at 128 for half the work. (Step of B8 H16 L2048 490, through dS 530, two
-//    kernels 554; B4 H16 L1024 unmasked 141, 146, 142; grouped B8 H32/8 L2048 623, two kernels 735.) With a bias or in a fixed order:
-//    the two kernels (B8 H12 L512 with a mask 61.5; fused 60.3, and through dS level).
+//  * head_dim 64, more key blocks, no bias, no fixed order asked for: the fused kernel where rows are long or query heads grouped, the two kernels
+//    where they are short, since their two CTAs per SM hide set-up and epilogue, and with dropout, where the fused kernel reads keep
+//    bits on its chain. (Step, fused | two kernels: B8 H16 L2048 471 | 476, B2 H16 L4096 unmasked 727 | 787, B8 H16 L1500 unmasked 485 | 505, packed
+//    30 to 300 tokens, 32/8 heads 133 | 137; B16 H16 L1024 318 | 305, L500 131 | 121, B8 H12 L1000 unmasked 197 | 187, packed 100 to 600 tokens 203 | 192;
+//    dropout B32 H12 L300 unmasked 208 | 180, B8 H16 L2000 693 | 675. Through dS, when its kernels had one CTA per SM: B8 H16 L2048 530.)
 //  * head_dim 65 to 128, more key blocks: dS through the workspace and a GEMM for dQ (use_ds_backward). One pass over the scores where
 //    the two kernels make two, and no reductions. (Step of B8 H16 L2048 695, two kernels 757, fused 752; with dropout 875, 940, 925;
 //    B2 H16 L8192, in two passes, 2189, 2295, 2290; B16 H32 L512 310, 365, 360; D80 B8 H16 L2048 alone 438, 533, 545; grouped B8 H32/8 L2048 alone
@@ -1091,7 +1122,9 @@ bool use_ds_backward(const sdpa_b200_params& p) {
 }
 
 bool use_fused_backward(const sdpa_b200_params& p) {
-  return p.head_dim <= 64 && p.deterministic == 0 && p.bias == nullptr && key_blocks(p) > kSms;
+  const int longest = p.max_seqlen_q > p.max_seqlen_k ? p.max_seqlen_q : p.max_seqlen_k;
+  const bool short_rows = p.heads_q == p.heads_kv && longest <= (p.dropout_p > 0.f ? 2048 : 1024);
+  return p.head_dim <= 64 && p.deterministic == 0 && p.bias == nullptr && key_blocks(p) > kSms && !short_rows;
 }
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
@@ -1171,17 +1204,18 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   const int64_t rows_k = varlen ? p.total_k : p.max_seqlen_k;
   const int64_t nb = varlen ? 1 : p.batch;
   int st;
+  const int box = p.head_dim <= 64 && !fused ? kRowsY<64> : kTile;  // rows of the streamed tiles; stationary ones take two
   if ((st = make_tensor_map_16(f16, &tm_q, p.q, p.head_dim, rows_q, p.heads_q, nb, p.q_row_stride, p.q_head_stride,
-                                 p.q_batch_stride, kTile)) != SDPA_B200_OK)
+                                 p.q_batch_stride, box)) != SDPA_B200_OK)
     return st;
   if ((st = make_tensor_map_16(f16, &tm_k, p.k, p.head_dim, rows_k, p.heads_kv, nb, p.k_row_stride, p.k_head_stride,
-                                 p.k_batch_stride, kTile)) != SDPA_B200_OK)
+                                 p.k_batch_stride, box)) != SDPA_B200_OK)
     return st;
   if ((st = make_tensor_map_16(f16, &tm_v, p.v, p.head_dim, rows_k, p.heads_kv, nb, p.v_row_stride, p.v_head_stride,
-                                 p.v_batch_stride, kTile)) != SDPA_B200_OK)
+                                 p.v_batch_stride, box)) != SDPA_B200_OK)
     return st;
   if ((st = make_tensor_map_16(f16, &tm_do, p.dout, p.head_dim, rows_q, p.heads_q, nb, p.do_row_stride,
-                                 p.do_head_stride, p.do_batch_stride, kTile)) != SDPA_B200_OK)
+                                 p.do_head_stride, p.do_batch_stride, box)) != SDPA_B200_OK)
     return st;
   CUtensorMap tm_dk, tm_dv;  // outputs, stored tile by tile from the epilogue's staging buffers
   if ((st = make_tensor_map_16(f16, &tm_dk, p.dk, p.head_dim, rows_k, p.heads_kv, nb, p.dk_row_stride, p.dk_head_stride,
