@@ -49,7 +49,7 @@ def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib, B, H, 
                 assert torch.equal(a, b), name
 
 
-@pytest.mark.parametrize("call", ["prefill", "packed", "decode", "decode_shared"])
+@pytest.mark.parametrize("call", ["prefill", "prefill_d256", "packed", "packed_d256", "decode", "decode_shared"])
 @pytest.mark.parametrize("captured", [False, True])
 def test_calls_launched_under_the_kernel_in_front_of_them(cuda_device, native_lib, call, captured):
     """Small forwards and decodes start under the tail of whatever is in front of them in the stream: they must see what that writes, and
@@ -57,8 +57,9 @@ def test_calls_launched_under_the_kernel_in_front_of_them(cuda_device, native_li
     dev = cuda_device
     gen = torch.Generator(device=dev).manual_seed(5)
     randn = lambda *s: torch.randn(*s, generator=gen, device=dev, dtype=torch.bfloat16)
+    call, D = call.replace("_d256", ""), 256 if call.endswith("d256") else 64
     B, H, Lq, Lk = {"prefill": (2, 4, 200, 200), "packed": (1, 4, 300, 300), "decode": (64, 8, 1, 64), "decode_shared": (2, 8, 1, 1500)}[call]
-    shape = (lambda L: (L, H, 64)) if call == "packed" else (lambda L: (B, H, L, 64))
+    shape = (lambda L: (L, H, D)) if call == "packed" else (lambda L: (B, H, L, D))
     src, q, k, v = randn(*shape(Lq)), randn(*shape(Lq)), randn(*shape(Lk)), randn(*shape(Lk))
     k0 = k.clone()
     cu = torch.tensor([0, 130, 300], dtype=torch.int32, device=dev)
