@@ -295,3 +295,35 @@ def test_streamed_tiles_of_64_rows(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, 
     out, lse, *grads = run_fwd_bwd(cuda_device, q, k, v, dout, causal, deterministic=True)
     o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=causal)
     check_grads(grads, orc.cpu_sdpa_backward(dout, q, k, v, o_ref, l_ref, causal=causal))
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,D,causal", [
+    ([700], 8, 1, 128, True),            # clusters of four
+    ([513, 513], 6, 1, 64, False),       # of two: three heads each
+    ([2000], 4, 2, 96, True),            # of two, padded head_dim
+    ([130, 1, 900, 257], 8, 2, 64, True),   # packed, of four, with a sequence of one
+    ([1200, 77], 16, 4, 128, True),      # packed, of four, ragged ends
+    ([900, 300], 12, 2, 128, False),     # packed, of two
+    ([2048] + [63] * 9, 2, 1, 128, True),   # dS through the workspace
+])
+def test_clusters_share_a_group_of_query_heads(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
+    """Grouped calls whose longest chain of items is far above an SM's average: against the oracle, tolerances as above, and twice with
+    the same bits."""
+    dev = cuda_device
+    total, cu = sum(lens), [sum(lens[:i]) for i in range(len(lens) + 1)]
+    q, k, v, dout = rand((total, Hq, D), 1), rand((total, Hkv, D), 2), rand((total, Hkv, D), 3), rand((total, Hq, D), 4)
+    want = orc.varlen_backward(dout, q, k, v, cu, cu, causal=causal)
+    qd, kd, vd, dd = (t.to(dev) for t in (q, k, v, dout))
+    if len(set(lens)) == 1:
+        split = lambda t: t.view(len(lens), lens[0], -1, D).transpose(1, 2)
+        qd, kd, vd, dd = (split(t) for t in (qd, kd, vd, dd))
+        out, lse = ops.gqa_prefill(qd, kd, vd, is_causal=causal)
+        run = lambda: [t.transpose(1, 2).reshape(total, -1, D) for t in ops._dense_backward(dd, qd, kd, vd, out, lse, causal, D ** -0.5)]
+    else:
+        cu_t = torch.tensor(cu, dtype=torch.int32, device=dev)
+        out, lse, seed, off, _ = ops._flash_attention_forward(qd, kd, vd, cu_t, cu_t, max(lens), max(lens), 0.0, causal, False)
+        run = lambda: ops._flash_attention_backward(dd, qd, kd, vd, out, lse, cu_t, cu_t, max(lens), max(lens), 0.0, causal, seed, off)
+    first, second = run(), run()
+    check_grads(first, want)
+    assert all(torch.equal(a, b) for a, b in zip(first, second))
+    assert ops.device_status() == 0

@@ -161,6 +161,7 @@ def test_manual_seed_repeats_the_pattern(cuda_device, native_lib):
     # more key blocks than SMs: dS through the workspace, with grouped queries too
     ([100, 300, 257], [100, 300, 257], 36, 18, True, 0.22),
     ([512, 64, 130], [200, 333, 130], 18, 18, False, 0.48),
+    ([700, 300], [650, 401], 8, 1, True, 0.2),   # clusters that share the query heads
 ])
 def test_packed_varlen_forward_and_backward_with_dropout(cuda_device, native_lib, lens_q, lens_k, Hq, Hkv, causal, p):
     """_flash_attention_forward / _backward with dropout_p > 0 (the path the reference's dense wrapper runs on,

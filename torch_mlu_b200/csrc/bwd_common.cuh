@@ -60,6 +60,7 @@ struct BwdKernelParams {
   int bh0;  // first (batch, head) pair of this launch
   int ds_call;  // kDsCall of bwd_tile_kernel
   int dq_acc_rows;  // packed: rows per head (total_q rounded up to 128, plus 128)
+  int split;  // dK/dV: CTAs (a cluster) that share the query heads of a key block, see bwd_split()
 #ifdef SDPA_BWD_STAMPS
   float* stamps;  // [mode 2][role 4][item 24][event 8] SM cycles since CTA start, one CTA per mode
 #endif

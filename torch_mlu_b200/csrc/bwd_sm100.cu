@@ -13,7 +13,8 @@
 //   1. bwd_preprocess_kernel: delta and the log2-domain logsumexp into a padded
 //      [batch, heads_q, ceil128(max_seqlen_q)] workspace (rows past a sequence get lse = +inf,
 //      which later turns their P into exact zeros).
-//   2. bwd_tile_kernel<kModeDKDV>: one CTA per (batch, kv head, 128-key block). K and V tiles
+//   2. bwd_tile_kernel<kModeDKDV>: one CTA, or a cluster that shares the query heads (bwd_split), per (batch, kv head,
+//      128-key block). K and V tiles
 //      stay in shared memory; (Q, dO) tiles (of 128 rows, or 64 up to head_dim 64) stream through a TMA ring. Per Q tile:
 //      S^T = K Q^T and dP^T = V dO^T on tcgen05 into TMEM, two compute warpgroups (thread = key
 //      row = TMEM lane, one warpgroup per half of the tile's queries) form P^T and dS^T, write
@@ -116,7 +117,7 @@ enum BiasKind { kNoBias = 0, kFullBias = 1, kKeyBias = 2 };
 // kDsCall: the call's dS goes through the workspace where there is room (launch_bwd). An instance of its own, since with both kinds of
 // exponentials and the dS stores behind branches the calls without dS were slower (dK/dV and dQ kernel of 6 packed sequences of 50 to 4000
 // tokens, 32/8 heads, unmasked: 1222 + 1076 us, so 1137 + 1019).
-template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall>
+template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall, bool kSplit>
 __global__ void __launch_bounds__(kThreads<kD>, kD == 64 ? 2 : 1)
 bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -153,7 +154,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   int b, hx, xb;
   {
     int rank, bh;
-    if (!block_of_slot(p.order, blockIdx.x, rank, bh)) {
+    if (!block_of_slot(p.order, kSplit ? blockIdx.x / p.split : blockIdx.x, rank, bh)) {
       wait_for_previous_grid();
       return;
     }
@@ -191,7 +192,10 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     y_hi = vis_end > 0 ? (vis_end + kY - 1) / kY : 0;
   }
   const int tiles_per_head = max(0, y_hi - y_lo);
-  const int heads_here = (kMode == kModeDKDV) ? p.kv_group : 1;
+  // dK/dV: the CTAs of a cluster (kSplit) take equal shares of the group's query heads
+  const int cluster_rank = kSplit ? static_cast<int>(blockIdx.x) % p.split : 0;
+  const int heads_here = kSplit ? p.kv_group / p.split : (kMode == kModeDKDV) ? p.kv_group : 1;
+  const auto query_head = [&](int hi) { return hx * p.kv_group + (kSplit ? cluster_rank * heads_here : 0) + hi; };
   const int n_items = tiles_per_head * heads_here;
 
   const uint32_t bar = base + kSmemBar;
@@ -238,7 +242,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int hi = i / tiles_per_head;
         const int yt = y_lo + (i - hi * tiles_per_head);
         // dK/dV streams the query heads of this KV head; dQ streams the KV head of this query head
-        const int hy = (kMode == kModeDKDV) ? hx * p.kv_group + hi : hx / p.kv_group;
+        const int hy = (kMode == kModeDKDV) ? query_head(hi) : hx / p.kv_group;
         const uint32_t full = bar + kBarYFull + 8 * s;
         const uint32_t dst = base + kSmemY + s * kYBytes;
         const int row = y_off + yt * kY;
@@ -347,7 +351,9 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         //   dQ:    ACC2 is unused, so S alternates between T1 and ACC2 and dP always uses T2: S(i+2)
         //          follows the accumulation of item i, dP(i+1) goes out as soon as dP(i) is read.
         // Either way the next item's scores and exponentials run under this item's accumulation.
-        const uint32_t x1 = base + kSmemX, x2 = base + kSmemX + kXBytes;
+        // operand descriptors hold 18 bits of the address; in a cluster the bits above say which CTA it belongs to
+        const uint32_t op_base = kSplit ? base & 0x3ffffu : base;
+        const uint32_t x1 = op_base + kSmemX, x2 = op_base + kSmemX + kXBytes;
         auto s_buf = [&](int i) { return kMode == kModeDKDV ? ((i & 1) ? t2 : t1) : ((i & 1) ? acc2 : t1); };
         auto d_buf = [&](int i) { return kMode == kModeDKDV ? ((i & 1) ? t1 : t2) : t2; };
         auto s_bar = [&](int i) { return bar + kBarSFull + (kMode == kModeDQ ? 8 * (i & 1) : 0); };
@@ -383,7 +389,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             ++ring_lap;
           }
         };
-        auto y_slot_k = [&](int k) { int sl, lp; pos(k, sl, lp); return base + kSmemY + sl * kYBytes; };
+        auto y_slot_k = [&](int k) { int sl, lp; pos(k, sl, lp); return op_base + kSmemY + sl * kYBytes; };
         auto y_wait_k = [&](int k) { int sl, lp; pos(k, sl, lp); return mbar_wait(bar + kBarYFull + 8 * sl, lp & 1, abort_flag); };
         auto y_free_k = [&](int k) { int sl, lp; pos(k, sl, lp); umma_commit(bar + kBarYEmpty + 8 * sl); };
         bool ok = true;
@@ -502,6 +508,11 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
       }
     }
+    if constexpr (kSplit) {  // the compute warps sum over the cluster
+      __syncwarp();
+      cluster_sync();
+      cluster_sync();
+    }
   } else {
     // ------------------------------------------------------------------ compute warpgroups
     if constexpr (kD == 64) reg_increase<kRegsCompute>();
@@ -522,7 +533,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     uint32_t ds_tile = 0;
     if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr) {
       wait_for_previous_grid();  // DsTiles::seq_base comes from the pre-pass
-      ds_tile = ds_head(p.ds, b, hx * p.kv_group, p.heads_q, len_q, len_k, p.is_causal != 0).tile(y_lo, xb);
+      ds_tile = ds_head(p.ds, b, query_head(0), p.heads_q, len_q, len_k, p.is_causal != 0).tile(y_lo, xb);
     }
     for (int i = 0; i < n_items; ++i) {
       const int s = (2 * i) % kStages;  // ring slot of Y1(i), which carries the per-query vectors
@@ -540,15 +551,15 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                                                    : static_cast<size_t>(b * p.heads_q + hx) * p.keep_q_rows + xr) *
                                     (p.keep_lk_pad >> 5)
                 : p.keep_cols + (p.cu_q != nullptr
-                                     ? static_cast<size_t>(hx * p.kv_group + hi) * p.keep_k_rows + k_off + xr
-                                     : static_cast<size_t>(b * p.heads_q + hx * p.kv_group + hi) * p.keep_k_rows + xr) *
+                                     ? static_cast<size_t>(query_head(hi)) * p.keep_k_rows + k_off + xr
+                                     : static_cast<size_t>(b * p.heads_q + query_head(hi)) * p.keep_k_rows + xr) *
                                     (p.keep_lq_pad >> 5);
         if constexpr (kC == 64) keep = *reinterpret_cast<const uint2*>(words + ((y0 + half * kC) >> 5));
         else keep.x = words[(y0 + half * kC) >> 5];
       }
       uint32_t key_bias_raw = 0u;  // dK/dV: this key's value; dQ: the values of two of the kC keys
       if constexpr (kBias == kKeyBias) {
-        const uint16_t* head = p.bias + b * p.bias_batch_stride + (kMode == kModeDQ ? hx : hx * p.kv_group + hi) * p.bias_head_stride;
+        const uint16_t* head = p.bias + b * p.bias_batch_stride + (kMode == kModeDQ ? hx : query_head(hi)) * p.bias_head_stride;
         const int key = y0 + half * kC + 2 * lane;
         if (kMode == kModeDQ && 2 * lane < kC && key < len_k) key_bias_raw = *reinterpret_cast<const uint32_t*>(head + key);
         if (kMode == kModeDKDV && xr < len_k) key_bias_raw = head[xr];
@@ -568,14 +579,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
           } else {
             if (p.bias_t != nullptr) {
-              const uint16_t* nx = p.bias_t + b * p.bias_t_batch_stride + (hx * p.kv_group + hn) * p.bias_t_head_stride +
+              const uint16_t* nx = p.bias_t + b * p.bias_t_batch_stride + query_head(hn) * p.bias_t_head_stride +
                                    static_cast<int64_t>(xr) * p.bias_t_row_stride + cn;
               if (cn < len_q) {
                 prefetch_l2(nx);
                 prefetch_l2(nx + min(kC - 1, len_q - 1 - cn));
               }
             } else {
-              const uint16_t* nx = p.bias + b * p.bias_batch_stride + (hx * p.kv_group + hn) * p.bias_head_stride + xr;
+              const uint16_t* nx = p.bias + b * p.bias_batch_stride + query_head(hn) * p.bias_head_stride + xr;
               const int q = 2 * lane < kC ? cn + 2 * lane : len_q;
               if (q < len_q) prefetch_l2(nx + static_cast<int64_t>(q) * p.bias_row_stride);
               if (q + 1 < len_q) prefetch_l2(nx + static_cast<int64_t>(q + 1) * p.bias_row_stride);
@@ -596,7 +607,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           vrow = p.bias + b * p.bias_batch_stride + hx * p.bias_head_stride + static_cast<int64_t>(xr) * p.bias_row_stride;
           vlen = len_k;
         } else if (p.bias_t != nullptr) {
-          vrow = p.bias_t + b * p.bias_t_batch_stride + (hx * p.kv_group + hi) * p.bias_t_head_stride +
+          vrow = p.bias_t + b * p.bias_t_batch_stride + query_head(hi) * p.bias_t_head_stride +
                  static_cast<int64_t>(xr) * p.bias_t_row_stride;
           vlen = len_q;
         }
@@ -662,7 +673,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           } else if (kMode == kModeDKDV && xr < len_x) {
             // no transposed copy: this key in kC consecutive query rows, as many two-byte loads (consecutive lanes on
             // consecutive keys)
-            const uint16_t* bcol = p.bias + b * p.bias_batch_stride + (hx * p.kv_group + hi) * p.bias_head_stride + xr;
+            const uint16_t* bcol = p.bias + b * p.bias_batch_stride + query_head(hi) * p.bias_head_stride + xr;
 #pragma unroll
             for (int j = 0; j < kC; ++j) {
               if (col0 + j < len_q) {
@@ -816,7 +827,66 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // ---- epilogue: accumulators -> scale -> 16-bit -> global
     if (ok && n_items > 0) ok = mbar_wait(bar + kBarAccFull, 0, abort_flag);
     BWD_STAMP(half, 23, 0);
-    if (ok) {
+    if constexpr (kSplit) {
+      // this CTA's part, fp32, for the sum over the cluster: 16 bytes (4 columns) per row, [column / 4][128 rows]; dV where K and V were, dK in
+      // the ring, which is idle by now too
+      if (ok) {
+        tc_fence_after_sync();
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+          float4* part = reinterpret_cast<float4*>(smem + (which == 0 ? kSmemX : kSmemY)) + r;
+#pragma unroll
+          for (int cc = 0; cc < kD / 64; ++cc) {
+            const int col = half * (kD / 2) + cc * 32;
+            uint32_t v[32];
+            if (n_items > 0) {
+              tmem_ld_x32((which == 0 ? acc1 : acc2) + (lane_base - half * kC) + col, v);
+              tmem_wait_ld();
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              part[(col / 4 + j) * kTile] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
+                                                        __uint_as_float(v[4 * j + 3]));
+          }
+        }
+      }
+      // Sum over the cluster: every CTA takes its share of the rows out of all parts, in the order of the ranks. A CTA that has given up takes
+      // part in the barriers.
+      cluster_sync();
+      const int rows = kTile / p.split;  // a multiple of 16
+      for (int e = threadIdx.x; e < rows * (kD / 16) * 2; e += kComputeWarps * 32) {
+        const int row = cluster_rank * rows + e % rows, chunk = e / rows;  // 16 columns of dV or dK
+        const int which = chunk / (kD / 16), col = chunk % (kD / 16) * 16;
+        const uint32_t part = base + (which == 0 ? kSmemX : kSmemY) + (col / 4 * kTile + row) * 16;
+        float4 sum[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[j] = cluster_ld_f32x4(part + j * kTile * 16, 0);
+        for (int other = 1; other < p.split; ++other) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 x = cluster_ld_f32x4(part + j * kTile * 16, other);
+            sum[j] = make_float4(sum[j].x + x.x, sum[j].y + x.y, sum[j].z + x.z, sum[j].w + x.w);
+          }
+        }
+        if (x0 + row >= len_x) continue;
+        const float mul = which == 1 ? p.scale : kDrop ? p.keep_scale : 1.f;
+        const int64_t row_stride = which == 0 ? p.dv_row_stride : p.dk_row_stride;
+        uint16_t* dst = which == 0 ? p.dv + hx * p.dv_head_stride : p.dk + hx * p.dk_head_stride;
+        dst += (p.cu_q != nullptr ? k_off + x0 + row : static_cast<int64_t>(x0 + row)) * row_stride + col;
+        if (p.cu_q == nullptr) dst += b * (which == 0 ? p.dv_batch_stride : p.dk_batch_stride);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (col + 8 * j >= p.head_dim) break;
+          const float4 lo = sum[2 * j], hi = sum[2 * j + 1];
+          *reinterpret_cast<uint4*>(dst + 8 * j) = make_uint4(pack_16x2<kF16>(lo.x * mul, lo.y * mul), pack_16x2<kF16>(lo.z * mul, lo.w * mul),
+                                                              pack_16x2<kF16>(hi.x * mul, hi.y * mul), pack_16x2<kF16>(hi.z * mul, hi.w * mul));
+        }
+      }
+      cluster_sync();  // the others have read this CTA's part
+    } else if (ok) {
       tc_fence_after_sync();
       const bool valid = xr < len_x;
       // A whole 128-row tile leaves through shared memory and TMA stores (the ring slots are idle by
@@ -1026,13 +1096,13 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
 using TileKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                             const CUtensorMap, const CUtensorMap, const BwdKernelParams);
 
-template <int kMode, bool kDrop, int kBias>
+template <int kMode, bool kDrop, int kBias, bool kSplit = false>
 TileKernel pick_tile_kernel(int head_dim, bool f16, bool ds_call) {
   if (head_dim <= 64)
-    return f16 ? bwd_tile_kernel<kMode, 64, true, kDrop, kBias, false> : bwd_tile_kernel<kMode, 64, false, kDrop, kBias, false>;
+    return f16 ? bwd_tile_kernel<kMode, 64, true, kDrop, kBias, false, kSplit> : bwd_tile_kernel<kMode, 64, false, kDrop, kBias, false, kSplit>;
   if (ds_call)
-    return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, true> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, true>;
-  return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, false> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, false>;
+    return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, true, kSplit> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, true, kSplit>;
+  return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, false, kSplit> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, false, kSplit>;
 }
 
 template <int kMode, bool kDrop>
@@ -1061,7 +1131,10 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
   const BiasKind bias = kp.bias == nullptr                                                                    ? kNoBias
                         : kp.bias_row_stride == 0 && (mode == kModeDKDV || kp.dbias == nullptr) ? kKeyBias
                                                                                                               : kFullBias;
-  TileKernel kernel = mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16, kp.ds_call != 0)
+  const bool split = mode == kModeDKDV && kp.split > 1;
+  TileKernel kernel = split ? (drop ? pick_tile_kernel<kModeDKDV, true, kNoBias, true>(head_dim, f16, kp.ds_call != 0)
+                                    : pick_tile_kernel<kModeDKDV, false, kNoBias, true>(head_dim, f16, kp.ds_call != 0))
+                      : mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16, kp.ds_call != 0)
                                         : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16, kp.ds_call != 0);
   const int dim = head_dim <= 64 ? 64 : 128;  // the instance
   const uint32_t smem = smem_bytes_for(mode, dim, bias == kKeyBias);
@@ -1071,15 +1144,22 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
     return SDPA_B200_LAUNCH_FAILED;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = dim3(split ? grid * kp.split : grid);
   cfg.blockDim = dim3(dim == 64 ? kThreads<64> : kThreads<128>);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = overlap_previous ? 1 : 0;
+  if (overlap_previous) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (split) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = kp.split;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   err = cudaLaunchKernelEx(&cfg, kernel, tm_q, tm_k, tm_v, tm_do, tm_o1, tm_o2, kp);
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -1101,7 +1181,7 @@ int lq_padded(const sdpa_b200_params& p) { return ((p.max_seqlen_q + kTile - 1) 
 //    H8/1 L4096 545, 564, 800; the other way round only where few key blocks meet many queries: B2 H32/8 L1024 unmasked 124, 112.)
 //  * a bias gradient: the same two, since the dQ kernel, whose threads own query rows, writes it.
 //  * head_dim 64, more key blocks, no bias, no fixed order asked for: the fused kernel where rows are long or query heads grouped, the two kernels
-//    where they are short, since their two CTAs per SM hide set-up and epilogue, and with dropout, where the fused kernel reads keep
+//    where clusters share a group of query heads (bwd_split) and where rows are short, since their two CTAs per SM hide set-up and epilogue, and with dropout, where the fused kernel reads keep
 //    bits on its chain. (Step, fused | two kernels: B8 H16 L2048 471 | 476, B2 H16 L4096 unmasked 727 | 787, B8 H16 L1500 unmasked 485 | 505, packed
 //    30 to 300 tokens, 32/8 heads 133 | 137; B16 H16 L1024 318 | 305, L500 131 | 121, B8 H12 L1000 unmasked 197 | 187, packed 100 to 600 tokens 203 | 192;
 //    dropout B32 H12 L300 unmasked 208 | 180, B8 H16 L2000 693 | 675. Through dS, when its kernels had one CTA per SM: B8 H16 L2048 530.)
@@ -1117,6 +1197,30 @@ int64_t key_blocks(const sdpa_b200_params& p) {
 }
 constexpr int64_t kSms = 148;
 
+// CTAs that share the query heads of a key block (calls without bias). One CTA sums a whole group, in a chain of group x query tiles items;
+// where the longest chain is a multiple (the ratio below) of what an SM has to do on average, a cluster takes the heads in shares and sums
+// its parts through shared memory. A packed call counts lengths spread between the mean and the longest. (Step in us, one CTA | two | four;
+// packed, causal unless said. Up to head_dim 64, "one" the fused kernel where it would run: ratio 1, 3 sequences of 200 to 3000 tokens, 16/4
+// heads, unmasked 402 | 377 | 363; 1, 8 of 64 to 2000, 16/4 331 | 295 | 331; 2.1, 16 of 64 to 2000, 8/1 374 | 321 | 296; 2.3, chain of 36, 4 of 64 to
+// 1280, 32/8 132 | 122 | 137; 4.5, 4 of 64 to 1280, 16/4 121 | 93 | 83; rows of nearly one length, whose chains fill the SMs more evenly: 1.24,
+// 2 of 1900 to 2000, 16/4, unmasked 260 | 225, and 1.4, 5 of 900 to 1700 191 | 184; but 1.18, 4 of 2000 to 2100 244 | 255; also 0.6, 8 of 500 to
+// 1500, 32/8 374 | 404, and 1.5, chain of 20, 12 of 64 to 700, 32/8 138 | 141. D128: 2.3, 16 of 100 to 2500, 8/1 489 | 405 | 433; 4.6, 2 of 300 to 2000, 16/4 151 | 112 | 120; 8, 6 of 200 to 1500, 8/1
+// 232 | 154 | 116, eight 152; but 1, 12 of 64 to 2048, 16/4 326 | 351, and 2.4, chain of 20, 8 of 64 to 700, 16/4, unmasked 103.5 | 108.5: a cluster
+// waits for SMs that are free together and for its slowest part.)
+int bwd_split(const sdpa_b200_params& p) {
+  const int group = p.heads_q / p.heads_kv;
+  const double query_tiles = (p.max_seqlen_q + kTile - 1) / kTile;
+  const double mean_tiles = p.cu_seqlens_q != nullptr ? static_cast<double>(p.total_q) / p.batch / kTile : query_tiles;
+  const double key_tiles = p.cu_seqlens_q != nullptr ? mean_tiles : (p.max_seqlen_k + kTile - 1) / kTile;
+  const double items = static_cast<double>(p.batch) * p.heads_q * key_tiles * (mean_tiles + query_tiles) / 2 * (p.is_causal ? 0.5 : 1.0);
+  const double ratio = group * query_tiles * kSms / (items > 1 ? items : 1);
+  const bool narrow = p.head_dim <= 64;
+  const double chain = group * query_tiles;
+  if (p.bias != nullptr || chain < (narrow ? 24 : 32)) return 1;
+  if (group % 4 == 0 && ratio >= (narrow ? (chain < 64 ? 3.0 : 2.0) : 6.0)) return 4;
+  return group % 2 == 0 && ratio >= (!narrow ? 2.0 : mean_tiles < 0.75 * query_tiles ? 0.9 : 1.2) ? 2 : 1;
+}
+
 bool use_ds_backward(const sdpa_b200_params& p) {
   return p.head_dim > 64 && p.dbias == nullptr && key_blocks(p) > kSms;
 }
@@ -1124,7 +1228,7 @@ bool use_ds_backward(const sdpa_b200_params& p) {
 bool use_fused_backward(const sdpa_b200_params& p) {
   const int longest = p.max_seqlen_q > p.max_seqlen_k ? p.max_seqlen_q : p.max_seqlen_k;
   const bool short_rows = p.heads_q == p.heads_kv && longest <= (p.dropout_p > 0.f ? 2048 : 1024);
-  return p.head_dim <= 64 && p.deterministic == 0 && p.bias == nullptr && key_blocks(p) > kSms && !short_rows;
+  return p.head_dim <= 64 && p.deterministic == 0 && p.bias == nullptr && key_blocks(p) > kSms && !short_rows && bwd_split(p) == 1;
 }
 
 size_t bwd_vector_bytes(const sdpa_b200_params& p) {
@@ -1293,6 +1397,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   };
   const double rows_q_all = static_cast<double>(p.total_q) * p.heads_q, rows_k_all = static_cast<double>(p.total_k) * p.heads_kv;
   kp.bh0 = 0;
+  kp.split = bwd_split(p);
   kp.ds.data = nullptr;
   kp.ds_call = plan.tiles > 0;
   if (through_ds) {

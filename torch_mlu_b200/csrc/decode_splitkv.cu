@@ -133,22 +133,6 @@ __device__ __forceinline__ void mma_rows(float (&c)[4], const uint32_t (&a)[4], 
   else mma_16816_lo<kF16>(c[0], c[1], a[0], a[2], b0, b1);
 }
 
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared memory of CTA `rank` of the cluster, at this CTA's address `addr`
-__device__ __forceinline__ float cluster_ld_f32(uint32_t addr, int rank) {
-  float v;
-  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
-  return v;
-}
-__device__ __forceinline__ float2 cluster_ld_f32x2(uint32_t addr, int rank) {
-  float2 v;
-  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %2, %3;\n\tld.shared::cluster.v2.f32 {%0, %1}, [a];\n\t}\n"
-               : "=f"(v.x), "=f"(v.y) : "r"(addr), "r"(rank) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ float quad_max(float x) {
   x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
   x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));

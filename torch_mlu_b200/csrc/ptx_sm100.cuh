@@ -148,6 +148,29 @@ __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddep
 // that this grid writes before its own wait.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Barrier over all threads of the cluster; shared memory written before it is visible to the others behind it
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared memory of CTA `rank` of the cluster, at this CTA's address `addr`
+__device__ __forceinline__ float cluster_ld_f32(uint32_t addr, int rank) {
+  float v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 cluster_ld_f32x2(uint32_t addr, int rank) {
+  float2 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %2, %3;\n\tld.shared::cluster.v2.f32 {%0, %1}, [a];\n\t}\n"
+               : "=f"(v.x), "=f"(v.y) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 cluster_ld_f32x4(uint32_t addr, int rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}\n"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+
 // two fp32 -> packed bf16x2 (lo in the low half), round to nearest even
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;
