@@ -1454,7 +1454,7 @@ int launch_fwd_d256(const sdpa_b200_params& p, void* workspace, cudaStream_t str
   }
   // under the tail of the grid in front, unless that is the launch that clears the status word (calls back to back: B3 H16/4 L227
   // 14.3 us -> 11.3, B1 H8 L128 12.3 -> 9.6, B8 H16 L644 79.9 -> 77.1)
-  err = launch_behind(kernel, dim3(kp.order.slots), 192, kSmemBytesD256, stream, p.device_status != nullptr, 1, tm_k, tm_v, tm_o, kp);
+  err = launch_behind(kernel, dim3(kp.order.slots), 192, kSmemBytesD256, stream, p.device_status != nullptr && short_forward(p), 1, tm_k, tm_v, tm_o, kp);
   if (err != cudaSuccess) {
     set_error("head_dim 256 forward: launch failed: %s", cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;

@@ -908,7 +908,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   // Without the clearing launch in front, the grid may start under the tail of the one before it in the stream, whichever that is. Calls back
   // to back, with the first unit's loads asked for before the set-up barrier: B2 H8 L256 D64 10.2 us -> 7.5, B1 H32/8 L300 D128 12.3 -> 10.1, 3
   // packed sequences of 100 to 200 tokens, D64 10.7 -> 8.6.
-  err = launch_behind(kernel, grid, kNumThreads, kSmemBytes, stream, kp.unit_counter == nullptr && p.device_status != nullptr, 1, tm_q, tm_k, tm_v, tm_o, kp);
+  err = launch_behind(kernel, grid, kNumThreads, kSmemBytes, stream, kp.unit_counter == nullptr && p.device_status != nullptr && short_forward(p), 1, tm_q, tm_k, tm_v, tm_o, kp);
   if (err != cudaSuccess) {
     set_error("prefill: launch failed: %s", cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;

@@ -104,6 +104,16 @@ cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, siz
   return err == cudaSuccess ? cudaGetLastError() : err;
 }
 
+// Forwards that are launched behind the kernel in front of them: up to 1e11 operations. Longer ones have little to hide and run into the power
+// cap, where the gap costs nothing and filling it does. (Calls back to back, early | plain start, us: 1.3e11 operations, D128, B2 H32/8, 512 rows of 8192
+// 126 | 122, B1 H32/8, 1024 of 8192 122 | 120; 6e10, B2 H32/8, 512 of 4096 66.9 | 67.0; but 8e10, B1 H9 L4096 unmasked 66.5 | 68.1; 7e10, D256, B3 H12,
+// 1479 of 2047 95.3 | 97.5; 3e10, D128, B1 H32/8, 512 of 4096 55.3 | 56.1.)
+inline bool short_forward(const sdpa_b200_params& p) {
+  const double rows = p.cu_seqlens_q != nullptr ? p.total_q : static_cast<double>(p.batch) * p.max_seqlen_q;
+  const double hidden = p.is_causal ? (p.max_seqlen_q < p.max_seqlen_k ? p.max_seqlen_q : p.max_seqlen_k) / 2.0 : 0.0;
+  return 4.0 * p.head_dim * p.heads_q * rows * (p.max_seqlen_k - hidden) <= 1e11;
+}
+
 // Number of SMs of the current device (cached per device), <= 0 on error.
 int sm_count();
 
