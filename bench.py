@@ -43,9 +43,9 @@ sys.path.insert(0, ROOT)
 METRIC = "SDPA TFLOP/s per B200 (fwd, fwd+bwd) at 1/2/4/8 GPUs; decode HBM GB/s"
 WORKLOAD = "bf16 causal prefill forward B=4 per GPU Hq=Hkv=32 L=4096 D=128 (batch slice r drawn from seed 1+r)"
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
-# DRAM bytes per launch of the prefill kernel on the headline workload: 2 x the 316 MB an ncu capture of half the
+# DRAM bytes per launch of the prefill kernel on the headline workload: 2 x the 286 MB an ncu capture of half the
 # batch measured (profiles/fwd_prefill_kernel_b2_h32_l4096_causal.md; traffic grows in proportion to the batch)
-NCU_TRAFFIC_BYTES = {"prefill_c2": 6.32e8}
+NCU_TRAFFIC_BYTES = {"prefill_c2": 5.72e8}
 PER_GPU_BATCH = 4
 
 
