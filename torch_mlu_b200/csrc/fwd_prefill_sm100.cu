@@ -284,10 +284,10 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   // The kernel may have been launched under the tail of the grid in front of it (launch_fwd_prefill): set-up and, for dense tensors, the first
   // unit's coordinates come before the wait for that grid, everything that reads or writes global memory behind it. The producer thread
-  // does all of this and starts the first loads at once, so that they run under the TMEM allocation and the other warps' set-up.
+  // does all of this and starts the first loads at once, so that they run under the TMEM allocation and the other warps' set-up. Nothing of it
+  // outlives the branch: values that every role keeps cost the softmax warps registers that they do not have (a flag and a count of the tiles asked for here
+  // took the instances with dropout or a bias from 0 to 60 bytes of spills to 44 to 96).
   if (threadIdx.x == 0) launch_dependents();
-  const bool producer = warp == kProducerWarp && elect_one();
-  uint32_t preloaded = 0;  // producer: ring tiles of the first unit that have been asked for
   auto load_q = [&](int q_row, int h, int bcoord) {
     constexpr uint32_t kLoadBytes = kBlockN * kD * 2;  // bytes one Q/K/V tile brings in
     mbar_arrive_expect_tx(bar + kBarQFull, p.unit_tiles * kLoadBytes);
@@ -309,7 +309,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     tma_load_4d(dst, tm, full, 0, row, hk, bcoord);
     if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, full, 64, row, hk, bcoord);
   };
-  if (producer) {
+  if (warp == kProducerWarp && elect_one()) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
@@ -344,7 +344,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     if (!packed) wait_for_previous_grid();
     if (!u.done && u.n_iter > 0) {
       load_q(u.m0 + u.q_off, u.h, u.bcoord);
-      for (; preloaded < kStages && preloaded < 2u * u.n_iter; ++preloaded) load_kv(preloaded, preloaded, u.k_off, u.hk, u.bcoord);
+      for (int i = 0; i < min(kStages, 2 * u.n_iter); ++i) load_kv(i, i, u.k_off, u.hk, u.bcoord);
     }
   }
   if (warp == 0) {
@@ -362,7 +362,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     reg_decrease<kRegsOther>();
     if (warp == kProducerWarp) {
       // ------------------------------------------------------------------ TMA producer
-      if (producer) {
+      if (elect_one()) {
         uint32_t kv_cnt = 0;  // K/V tiles loaded so far (ring position)
         uint32_t ucnt = 0;    // units started so far
         bool ok = true;
@@ -377,7 +377,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
             if (!ok) break;
             load_q(q_row, h, bcoord);
           }
-          for (int i = n == 0 ? preloaded : 0; i < 2 * n_iter; ++i) {
+          for (int i = n == 0 ? min(kStages, 2 * n_iter) : 0; i < 2 * n_iter; ++i) {  // unit 0: behind the tiles asked for at the start
             const uint32_t cnt = kv_cnt + i;
             ok = mbar_wait(bar + kBarKVEmpty + 8 * (cnt % kStages), ((cnt / kStages) & 1u) ^ 1u, abort_flag);
             if (!ok) break;
