@@ -327,3 +327,29 @@ def test_clusters_share_a_group_of_query_heads(cuda_device, native_lib, lens, Hq
     check_grads(first, want)
     assert all(torch.equal(a, b) for a, b in zip(first, second))
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_more_rows_than_one_grid_of_the_prepass_covers(cuda_device, native_lib, packed):
+    """2 097 281 query rows: one block of 32 rows more than 65 535. Against fp32 math on the device. P, dS and the results are rounded to bf16
+    (2^-9 at most, 1.7e-3 in the 2-norm), independently in every term of a sum: 1e-2 leaves room for three of them and the inputs' own."""
+    L, D = 65535 * 32 + 161, 72
+    gen = torch.Generator(device=cuda_device).manual_seed(3)
+    q, k, v, dout = (torch.randn(1, 1, n, D, generator=gen, device=cuda_device).bfloat16() for n in (L, 64, 64, L))
+    if packed:
+        flat = lambda t: t.view(-1, 1, D)
+        cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=cuda_device) for n in (L, 64))
+        out, lse, seed, off, _ = ops._flash_attention_forward(flat(q), flat(k), flat(v), cu_q, cu_k, L, 64, 0.0, False, False)
+        grads = ops._flash_attention_backward(flat(dout), flat(q), flat(k), flat(v), out, lse, cu_q, cu_k, L, 64, 0.0, False, seed, off)
+    else:
+        out, lse = ops.gqa_prefill(q, k, v, is_causal=False)
+        grads = ops._dense_backward(dout, q, k, v, out, lse, False, D ** -0.5)
+    assert ops.device_status() == 0
+    qf, kf, vf, df = (t.view(-1, D).float() for t in (q, k, v, dout))
+    p = torch.softmax(qf @ kf.T * D ** -0.5, -1)
+    dp = df @ vf.T
+    ds = p * (dp - (dp * p).sum(-1, keepdim=True)) * D ** -0.5
+    for name, got, want in zip(("out", "dq", "dk", "dv"), (out, *grads), (p @ vf, ds @ kf, ds.T @ qf, p.T @ df)):
+        err = float((got.reshape(-1, D).float() - want).norm() / want.norm())
+        assert err <= 1e-2, (name, err)
+    assert float((grads[0].reshape(-1, D)[-200:].float() - (ds @ kf)[-200:]).norm() / (ds @ kf)[-200:].norm()) <= 1e-2

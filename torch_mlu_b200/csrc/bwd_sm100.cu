@@ -1003,6 +1003,7 @@ struct PreParams {
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int64_t do_batch_stride, do_head_stride, do_row_stride;
   int seqlen_q, total_q, heads_q, lq_pad, head_dim;
+  int block0;       // first block of rows of this launch
   float* dq_acc;    // fused kernel: its dQ accumulator, whose existing rows are cleared here; else null
   int dq_acc_rows;  // as in BwdKernelParams
   int32_t* ds_seq_base;  // packed, dS for a dQ GEMM: DsTiles::seq_base, written here; else null
@@ -1017,6 +1018,7 @@ struct PreParams {
 // and four passes per block, 134 MB at B8 H16 L2048 D128 29.8 us; so 22.6, 5.9 TB/s; four passes 23.0, one 24.6).
 template <int kD>
 constexpr int kPreRows = 2 * 256 * 8 / kD;  // 64 or 32
+constexpr int kMaxGridY = 65535;
 template <int kD, bool kF16, bool kPacked>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) {
   if (kPacked && static_cast<int>(blockIdx.x) == p.heads_q) {
@@ -1029,7 +1031,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   // heads vary fastest across the grid: with the usual [batch, row, head, dim] memory order the blocks
   // that run together then read neighbouring 256-byte pieces of the same rows
   const int h = blockIdx.x, b = blockIdx.z;
-  const int row0 = blockIdx.y * kRows;
+  const int row0 = (p.block0 + blockIdx.y) * kRows;
   const int col = threadIdx.x % kThreadsPerRow * 8;
   const int r_in_pass = threadIdx.x / kThreadsPerRow;
   int q_off = 0, len_q = p.seqlen_q;
@@ -1037,7 +1039,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     q_off = p.cu_q[b];
     len_q = p.cu_q[b + 1] - q_off;
   }
-  if (kPacked && p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0) {
+  if (kPacked && p.ds_seq_base != nullptr && h == 0 && row0 == 0) {
     write_seq_base(p.ds_seq_base, p.cu_q, p.cu_k, b, p.is_causal != 0);
   }
   uint4 ov[2], dv[2];
@@ -1288,20 +1290,24 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   float* dq_acc = fused ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceHeaderBytes + bwd_vector_bytes(p)) : nullptr;
   pre.dq_acc = dq_acc;
   pre.dq_acc_rows = fused && varlen ? static_cast<int>(bwd_fused_acc_rows(p, lq_pad) / p.heads_q) : 0;
-  const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), lq_pad / (p.head_dim <= 64 ? kPreRows<64> : kPreRows<128>), p.batch);
   auto pick_pre = [&](auto dim_tag) {
     constexpr int kD = decltype(dim_tag)::value;
     return varlen ? (f16 ? bwd_preprocess_kernel<kD, true, true> : bwd_preprocess_kernel<kD, false, true>)
                   : (f16 ? bwd_preprocess_kernel<kD, true, false> : bwd_preprocess_kernel<kD, false, false>);
   };
   auto pre_kernel = p.head_dim <= 64 ? pick_pre(std::integral_constant<int, 64>{}) : pick_pre(std::integral_constant<int, 128>{});
-  pre_kernel<<<pre_grid, 256, 0, stream>>>(pre);
-  cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) {
-    set_error("backward preprocess: launch failed: %s", cudaGetErrorString(err));
-    return SDPA_B200_LAUNCH_FAILED;
+  const int pre_blocks = lq_pad / (p.head_dim <= 64 ? kPreRows<64> : kPreRows<128>);
+  for (pre.block0 = 0; pre.block0 < pre_blocks; pre.block0 += kMaxGridY) {  // one launch up to 2 M rows
+    const int rest = pre_blocks - pre.block0;
+    const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), rest < kMaxGridY ? rest : kMaxGridY, p.batch);
+    pre_kernel<<<pre_grid, 256, 0, stream>>>(pre);
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) {
+      set_error("backward preprocess: launch failed: %s", cudaGetErrorString(err));
+      return SDPA_B200_LAUNCH_FAILED;
+    }
+    count_launch();
   }
-  count_launch();
 
   CUtensorMap tm_q, tm_k, tm_v, tm_do;
   const int64_t rows_q = varlen ? p.total_q : p.max_seqlen_q;
