@@ -53,6 +53,7 @@ def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D):
 
 @pytest.mark.parametrize("B,Hq,Hkv,Lk,D,launches", [
     (1, 32, 8, 1000, 128, 1),   # clusters of 8, two tiles each, the last one short
+    (1, 5, 1, 600, 64, 1),      # clusters of 8 that merge 20 column pairs each: part of a warp
     (1, 20, 2, 321, 64, 1),     # clusters of 4 over six tiles: the last CTA has none; ten heads: both fragment row halves
     (2, 40, 1, 600, 128, 1),    # the same with head chunks of 16, 16 and 8
     (12, 12, 12, 100, 128, 1),  # clusters of 2

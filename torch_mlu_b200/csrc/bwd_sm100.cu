@@ -509,7 +509,6 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
     if constexpr (kSplit) {  // the compute warps sum over the cluster
-      __syncwarp();
       cluster_sync();
       cluster_sync();
     }

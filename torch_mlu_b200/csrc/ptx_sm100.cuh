@@ -148,8 +148,10 @@ __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddep
 // that this grid writes before its own wait.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Barrier over all threads of the cluster; shared memory written before it is visible to the others behind it
+// Barrier over all threads of the cluster; shared memory written before it is visible to the others behind it. The aligned forms want every warp to arrive as
+// one, and callers come out of loops and branches that part its lanes.
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // shared memory of CTA `rank` of the cluster, at this CTA's address `addr`
