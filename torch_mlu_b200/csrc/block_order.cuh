@@ -28,7 +28,7 @@ inline BlockOrder block_order(int heads, int ranks, int heads_per_group, int tai
 }
 
 // False for a slot without a block.
-__device__ __forceinline__ bool block_of_slot(const BlockOrder& o, int slot, int& rank, int& head) {
+__host__ __device__ __forceinline__ bool block_of_slot(const BlockOrder& o, int slot, int& rank, int& head) {
   if (slot >= o.front_slots) {
     const int w = slot - o.front_slots;
     rank = w / o.heads;

@@ -888,8 +888,10 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.unit_tiles = static_cast<int64_t>(heads) * tiles <= usable ? 1 : 2;
   kp.tile1 = kp.unit_tiles == 2 ? kBlockM : 1 << 30;
   const int unit_rows = kp.unit_tiles * kBlockM, ranks = (p.max_seqlen_q + unit_rows - 1) / unit_rows;
+  const double all_heads_row = kv_row_bytes * p.batch * p.heads_kv;
+  const int prefix = p.max_seqlen_k > p.max_seqlen_q ? p.max_seqlen_k - p.max_seqlen_q : 0;
   kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes),
-                         p.is_causal ? tail_ranks(ranks, kv_row_bytes * unit_rows * p.batch * p.heads_kv) : 0);
+                         p.is_causal ? tail_ranks(ranks, all_heads_row * unit_rows, all_heads_row * prefix) : 0);
   dim3 grid(kp.order.slots < usable ? kp.order.slots : usable, 1, 1);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
   // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been

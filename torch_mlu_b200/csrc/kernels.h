@@ -57,13 +57,16 @@ constexpr double kForwardGroupBytes = 32.0 * 1024 * 1024;
 // thousand cycles at B8 H16 L2048 D128, 911 to 825 at B4 H32 L4096; now 240 to 231 and 821 to 806. Calls over seconds, with the late claims of
 // the forward: these two 172 us -> 166 and 568 -> 533, B2 H16 L3000 101 -> 88.6, B4 H32/8 L1000 57.7 -> 51.4, 9 packed sequences of 29 to 2820
 // tokens, 8/1, D64 92.8 -> 72.8. As many as half, and as stay in L2 together, since heads do not share K and V at a time there: `bytes_per_rank`
-// are those that one more rank makes all heads stream (limit of 128 MB: 555 us at L4096, 64: 539, 32: 538; B8 H16 L2048 170, 169, 166). Not
+// are those that one more rank makes all heads stream, `prefix_bytes` those that every rank does, since the keys in front of the first query are
+// visible to all (limit of 128 MB: 555 us at L4096, 64: 539, 32: 538; B8 H16 L2048 170, 169, 166. With the prefix left out of the count, 512 rows behind a
+// cached prefix read all of K and V twice, us, so | counted: B7 H32 512 of 1297 102.5 | 92.6, B8 H32 512 of 2048 156.8 | 147.1, B4 H32 1024 of 4096
+// 282 | 259, B8 H32 1152 of 1984 D96 267 | 259). Not
 // where the hardware deals out CTAs of single blocks: it claims as late as can be, and the kernel ends within 2 % of the mean CTA as it is
 // (head_dim 256 forward, B4 H16 L4096 534 without, 533 with; B8 H16 L644 80, 82; backward, step of B4 H16 L1024 D256 227, 231, of B8 H12 L1000
 // D64 135, 159).
-inline int tail_ranks(int ranks, double bytes_per_rank) {
-  const int fit = static_cast<int>(32.0 * 1024 * 1024 / bytes_per_rank);
-  return fit < ranks / 2 ? fit : ranks / 2;
+inline int tail_ranks(int ranks, double bytes_per_rank, double prefix_bytes) {
+  const double fit = (32.0 * 1024 * 1024 - prefix_bytes) / bytes_per_rank;
+  return fit < 1 ? 0 : fit < ranks / 2 ? static_cast<int>(fit) : ranks / 2;
 }
 
 // Packed backward under a causal mask, from what all sequences together stream: the longest one says little about it, and in fewer and
