@@ -68,7 +68,7 @@ constexpr uint32_t kBarPFull = kBarSFull + 16;             // 2 tiles x 2 halves
 constexpr uint32_t kBarOFull = kBarPFull + 32;             // 2
 constexpr uint32_t kBarOFree = kBarOFull + 16;             // 2: the epilogue has read O_t (persistent loop)
 constexpr uint32_t kBarQFree = kBarOFree + 16;             // the unit's last QK^T has read the Q tiles
-constexpr uint32_t kBarClaim = kBarQFree + 8;              // the issuer is kClaimAhead blocks from the end of its unit
+constexpr uint32_t kBarClaim = kBarQFree + 8;              // the issuer is claim_ahead() blocks from the end of its unit
 constexpr uint32_t kBarUnitFull = kBarClaim + 8;           // kUnitRing: the scheduler has written the entry
 constexpr uint32_t kBarUnitEmpty = kBarUnitFull + 16;      // kUnitRing: every reader has copied the entry
 constexpr uint32_t kBarStageFree = kBarUnitEmpty + 16;     // 2: the warpgroup's staging buffer may be rewritten
@@ -102,6 +102,7 @@ struct FwdKernelParams {
   int64_t bias_batch_stride, bias_head_stride, bias_row_stride;
   float inv_scale;  // 1 / softmax_scale: the bias joins the raw scores as bias / scale
   BlockOrder order;  // of the work units
+  int claim_ahead;   // see claim_ahead(), at least 1
   int unit_tiles;    // Q tiles per unit: 2, or 1 where every tile has an SM of its own
   int tile1;         // first row of a unit's second tile in the unit; behind every sequence where there is none
   float scale_log2;
@@ -197,9 +198,17 @@ __device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first,
 // counts, so the loads, the first QK^T and the softmax of the next unit start while this unit's
 // epilogue runs.
 constexpr int kUnitRing = 2;
-// A unit is claimed when the one in front of it has this many key blocks left: late, since a unit that a busy CTA has claimed is one that
-// an idle CTA cannot take, and early enough for the claim (atomic, decode, about 1500 cycles) to pass before the Q tiles are free.
-constexpr int kClaimAhead = 3;
+// A unit is claimed when the one in front of it has claim_ahead() key blocks left: late, since a unit that a busy CTA has claimed is one that
+// an idle CTA cannot take, and early enough for the claim (atomic, decode, about 1500 cycles) to pass before the Q tiles are free: three blocks. A packed claim
+// takes longer, since it reads the lengths, and once more for every slot without a unit: eight where the list is long, so that few units of it are
+// its end. In a packed list of up to two rounds every unit is its end, and lengths differ: one. (us, claims a whole unit ahead | eight | three | one; long lists, D64: 28
+// sequences of 64 to 3008 tokens, 64/8 heads 1424 | 1424 | 1448, 32 of 192 to 1321, 64/8 - | 478 | 486 | 536, 12 of 64 to 3000, 16/16, 2304 slots 177 | 165 | 165; short
+// ones: 8 of 100 to 900, 16/16, 512 slots - | 28.0 | 23.5 | 23.7, 10 of 47 to 605, 12/12, D128, 360 slots - | 22.1 | 22.0 | 22.9, 7 of 19 to 448, 16/16, unmasked, 224
+// slots - | 18.5 | 18.4 | 17.1; dense: B4 H32/8 L700 D64 - | 31.1 | 28.4 | 28.6, B8 H16 L512 D128, 256 slots - | 22.3 | 21.6 | 22.2.)
+inline int claim_ahead(bool packed, int slots, int ctas) {
+  if (!packed) return 3;
+  return slots <= 2 * ctas ? 1 : slots >= 16 * ctas ? 8 : 3;
+}
 constexpr uint32_t kUnitReaders = 10;  // producer + issuer + 8 softmax warps
 
 // Copies ring entry (n mod kUnitRing) into `u` and releases it. All lanes of the calling warp (or its
@@ -420,7 +429,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           kv_release(kv_base);
           if (n_iter == 1) umma_commit(bar + kBarQFree);
           for (int j = 0; ok && j < n_iter; ++j) {
-            if (j == max(0, n_iter - kClaimAhead)) mbar_arrive(bar + kBarClaim);
+            if (j == max(0, n_iter - p.claim_ahead)) mbar_arrive(bar + kBarClaim);
             const uint32_t iv = kv_base + 2 * j + 1;  // ring position of V(j)
             const uint32_t ik = kv_base + 2 * j + 2;  // ring position of K(j+1)
             const uint32_t v_smem = kv_smem(iv);
@@ -893,6 +902,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes),
                          p.is_causal ? tail_ranks(ranks, all_heads_row * unit_rows, all_heads_row * prefix) : 0);
   dim3 grid(kp.order.slots < usable ? kp.order.slots : usable, 1, 1);
+  kp.claim_ahead = claim_ahead(varlen, kp.order.slots, usable);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
   // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
   // cleared already.) Not for two units per CTA, dealt out by index: alone that is faster (B8 H12 L512 D64 unmasked, eager, 22.6 us against
