@@ -1397,7 +1397,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
     const double row_bytes = 2.0 * p.head_dim * 2;
     kp.order = block_order(heads, (rows + kTile - 1) / kTile,
                            varlen && !fused && p.is_causal ? heads_per_packed_group(row_bytes * packed_rows, heads)
-                                                           : heads_per_l2_group(row_bytes * rows_streamed * streams, heads, 48.0 * 1024 * 1024, !fused));
+                                                           : heads_per_l2_group(row_bytes * rows_streamed * streams, heads, 48.0 * 1024 * 1024, !fused && !varlen));
     return kp.order.slots;
   };
   const double rows_q_all = static_cast<double>(p.total_q) * p.heads_q, rows_k_all = static_cast<double>(p.total_k) * p.heads_kv;

@@ -1355,7 +1355,7 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace
     // bytes one stationary head streams: Q + dO of its group (keys), or K + V (queries)
     const double streamed = 2.0 * (keys ? p.max_seqlen_q : p.max_seqlen_k) * p.head_dim * 2 * (keys ? kp.kv_group : 1);
     const double packed = 2.0 * p.head_dim * 2 * (keys ? static_cast<double>(p.total_q) * p.heads_q : static_cast<double>(p.total_k) * p.heads_kv);
-    kp.order = block_order(heads, ranks, varlen && p.is_causal ? heads_per_packed_group(packed, heads) : heads_per_l2_group(streamed, heads));
+    kp.order = block_order(heads, ranks, varlen && p.is_causal ? heads_per_packed_group(packed, heads) : heads_per_l2_group(streamed, heads, 48.0 * 1024 * 1024, !varlen));
     const int grid = kp.order.slots;
     kernel<<<grid, kBwdThreads, kSmemBytesBwd256, stream>>>(x2, y1, y2, out, kp);
     e = cudaGetLastError();

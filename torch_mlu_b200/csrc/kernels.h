@@ -38,7 +38,9 @@ int launch_bwd_d256(const sdpa_b200_params& p, void* workspace, size_t workspace
 // Heads per group, from the bytes that one head streams (packed: at the longest length). The groups are of one size, as far as that goes: a small
 // last group puts its few heavy blocks where no light ones are left to fill up behind them (us, filled up | even: forward D256, B3 H12, 1479 rows of
 // 2047, 15 + 15 + 6 heads or 3 x 12 95.3 | 89.2, 12 packed sequences of 300 to 2000, 16/4 332 | 312, D128, 16 of 512 to 4096, 32/8 915 | 885; step of
-// B3 H12 L1479 D128 143 | 133, of B5 H8 L2500 D192 551 | 544). Not in the fused kernel (`even`; step of B5 H12 L1500 D64 154.6 | 156.4).
+// B3 H12 L1479 D128 143 | 133, of B5 H8 L2500 D192 551 | 544). Not (`even`) in the fused kernel (step of B5 H12 L1500 D64 154.6 | 156.4), nor in packed backwards
+// without a mask, whose heads stand by sequence: even groups cut the sequences elsewhere, and where the last group begins inside the longest one it has
+// the longest chains (722, 529, 2016 and 843 tokens, 32/8 heads, D128, 12 + 12 + 8 or 11 + 11 + 10 heads: dK/dV 197 | 252 us).
 inline int heads_per_l2_group(double bytes_per_head, int num_heads, double group_bytes = 48.0 * 1024 * 1024, bool even = true) {
   int n = static_cast<int>(group_bytes / bytes_per_head);
   n = n > 32 ? 32 : (n < 1 ? 1 : n);
