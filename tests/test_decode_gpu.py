@@ -32,20 +32,24 @@ def test_decode_matches_oracle(cuda_device, native_lib, B, Hq, Hkv, Lk, splits):
     orc.assert_close_lse(lse, l_ref)
 
 
-@pytest.mark.parametrize("B,Hq,Hkv,Lk,D", [
-    (1, 8, 1, 20000, 128),    # one unit over every CTA of the grid
-    (5, 24, 1, 130, 64),      # head chunks of 16 and 8, a tile of two keys
-    (75, 8, 4, 64, 128),      # one tile per unit, more units than CTAs: nothing is shared
-    (50, 8, 8, 65, 64),       # 400 units of two tiles: shares that begin and end inside units
-    (37, 12, 12, 700, 128),   # 444 units: CTAs with whole units between two shared ones
+@pytest.mark.parametrize("B,Hq,Hkv,Lk,D,launches", [
+    (1, 8, 1, 20000, 128, 2),    # one unit over every CTA of the grid
+    (5, 24, 1, 130, 64, 1),      # head chunks of 16 and 8, a tile of two keys: as clusters of two
+    (1, 24, 1, 20000, 64, 2),    # head chunks of 16 and 8 in equal shares
+    (1, 40, 2, 8192, 128, 2),    # of 16 and 4
+    (7, 32, 2, 9000, 128, 2),    # 16 heads: a full chunk
+    (75, 8, 4, 64, 128, 1),      # one tile per unit, more units than CTAs: nothing is shared
+    (50, 8, 8, 65, 64, 2),       # 400 units of two tiles: shares that begin and end inside units
+    (37, 12, 12, 700, 128, 2),   # 444 units: CTAs with whole units between two shared ones
 ])
-def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D):
+def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D, launches):
     """The automatic split deals 64-key tiles of all (batch, kv head) units out in equal contiguous shares: shapes whose
-    shares begin, end or lie entirely inside units. Tolerances as above (16-bit output, fp32 logsumexp)."""
+    shares begin, end or lie entirely inside units. Two launches tell that shares were merged. Tolerances as above (16-bit output, fp32 logsumexp)."""
     q, k, v = rand((B, Hq, 1, D), 1), rand((B, Hkv, Lk, D), 2), rand((B, Hkv, Lk, D), 3)
     dev = cuda_device
+    before = _cabi.launch_count()
     out, lse = ops.decode_attention(q.to(dev), k.to(dev), v.to(dev))
-    assert ops.device_status() == 0
+    assert ops.device_status() == 0 and _cabi.launch_count() - before == launches
     o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=False)
     orc.assert_close_bf16(out, o_ref, "out")
     orc.assert_close_lse(lse, l_ref)
@@ -80,7 +84,9 @@ def test_decode_without_a_merge_kernel(cuda_device, native_lib, B, Hq, Hkv, Lk, 
 @pytest.mark.parametrize("what", ["query", "key", "value", "score"])
 @pytest.mark.parametrize("B,Hq,Hkv,Lk,splits,D", [
     (1, 8, 2, 4096, 0, 128),    # every unit shared between CTAs
-    (1, 40, 2, 1000, 0, 64),    # shared, head chunks of 16 and 4
+    (1, 40, 2, 1000, 0, 64),    # clusters of eight, head chunks of 16 and 4
+    (1, 40, 2, 8192, 0, 128),   # equal shares, the same chunks
+    (1, 24, 2, 20000, 0, 64),   # of 12 heads
     (1, 8, 2, 4096, 4, 128),    # fixed splits
     (1, 8, 2, 200, 6, 64),      # fixed splits, some of them without keys
     (2, 8, 2, 4096, 1, 128),    # one CTA per unit
