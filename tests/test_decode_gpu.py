@@ -67,6 +67,9 @@ def test_decode_equal_shares(cuda_device, native_lib, B, Hq, Hkv, Lk, D, launche
     (60, 16, 8, 130, 64, 1),    # two waves of whole units
     (68, 16, 16, 100, 64, 2),   # four waves of two tiles
     (35, 8, 8, 4097, 64, 1),    # several waves of clusters, 33 and 32 tiles each
+    (30, 4, 4, 8129, 128, 1),   # nearly two waves of clusters of four
+    (30, 4, 4, 8129, 64, 2),    # too few bytes in a share for them
+    (9, 8, 8, 16385, 64, 2),    # not in waves of clusters of eight: equal shares
 ])
 def test_decode_without_a_merge_kernel(cuda_device, native_lib, B, Hq, Hkv, Lk, D, launches):
     """Each side of the rule that chooses whole units, clusters or equal shares. Tolerances as above; the kernels are counted so that

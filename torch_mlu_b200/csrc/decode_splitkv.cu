@@ -622,14 +622,17 @@ void plan_decode(const sdpa_b200_params& p, int sms, DecodeParams& d) {
 // over one wave and the merge kernel, whose second launch costs about 3 us. Figures in us, calls back to back, H32/8 D128 unless said, equal
 // shares | so:
 //  * One wave of clusters, where its longest share is not much longer than an equal one: B1 Lk 1000 8.8 | 6.6, Lk 2000 8.7 | 7.9 (but Lk 4000 8.8 |
-//    10.1), B8 Lk 1000 10.2 | 8.8, Lk 4096 27.3 | 26.0, B16 Lk 1000 12.5 | 11.0. Clusters of 8 (and so 4) find room for 256 CTAs at once, not for 296: B3
-//    H12/12 Lk 4000 in 288 CTAs 13.1 | 20.4.
-//  * One nearly full wave of whole units: B32 Lk 500 12.5 | 9.1, B30 Lk 300 D64 9.0 | 6.3, B34 Lk 900 26.4 | 23.1 (192 units, B24 Lk 3000 51.8 | 52.4).
-//  * Several waves whose last one is more than half full. The hardware deals them out, where the slowest SM ends an equal share: B64 Lk 32768
+//    10.1), B8 Lk 1000 10.2 | 8.8, Lk 4096 27.3 | 26.0, B16 Lk 1000 12.5 | 11.0. Clusters of 8 find room for 256 CTAs at once, not for 296: B3
+//    H12/12 Lk 4000 in 288 CTAs 13.1 | 20.4; so for fours too, which come after them.
+//  * One nearly full wave of whole units, up to where a second wave of clusters has long enough shares: B32 Lk 500 12.5 | 9.1, B30 Lk 300 D64 9.0 | 6.3, B34 Lk 900
+//    26.4 | 23.1, B30 Lk 3900 80.1 | 78.5 (192 units, B24 Lk 3000 51.8 | 52.4).
+//  * Several waves whose last one has at least 160 of 296 CTAs. The hardware deals them out, where the slowest SM ends an equal share: B64 Lk 32768
 //    1249 | 1164, Lk 1500 66.6 | 59.7, Lk 300 16.1 | 13.2 (last wave nearly empty: B30 H12/12 Lk 2000 60.9 | 63.7, B44 Lk 300 11.8 | 12.3; many waves of a
-//    few tiles: B64 H32/32 Lk 64 19.0 | 22.6). A wave of
-//    clusters costs 3 to 4 us, so those take long shares only: B32 Lk 16384 in twos 316 | 300, B16 in fours 316 | 310, B8 Lk 32768 in eights 164 | 160 (B16
-//    Lk 1000 in fours 12.5 | 16.6).
+//    few tiles: B64 H32/32 Lk 64 19.0 | 22.6).
+//  * The same in clusters of two or four. A wave of clusters costs 3 to 4 us, so those take long shares only: B32 Lk 16384 in twos 316 | 300, B57 H16/4 Lk
+//    9000 162 | 152, B16 Lk 16384 in fours 316 | 310, B30 H16/4 Lk 18000 170 | 160, D64 91.0 | 86.5 (B16 Lk 1000 in fours 12.5 | 16.6; with 104 CTAs in the last wave, B25
+//    H16/4 Lk 8300 D64 39.6 | 44.6, with 80, B42 61.9 | 67.1; in shares of half the bytes, B18 H12/12
+//    Lk 9684 D64 89.7 | 94.3). Not in eights, which find room for 256 CTAs: two full waves of those, B8 Lk 20000 D64 57.2 | 60.0, 2.25 of them, B9 Lk 17000 57 | 65.
 int cluster_size(const DecodeParams& d) {
   constexpr int kWave = kCtasPerSm * 148;
   const int64_t units = d.units;
@@ -640,9 +643,10 @@ int cluster_size(const DecodeParams& d) {
     break;
   }
   if (units <= kWave && units >= kWave * 4 / 5 && tiles < 63) return 1;
-  for (int size = 1; size <= kMaxCluster; size *= 2) {
+  for (int size = 1; size <= 4; size *= 2) {
     const int64_t ctas = units * size, last = ctas % kWave;
-    if (ctas >= kWave && (last == 0 || last >= 160) && (size == 1 ? tiles > ctas / kWave : (tiles + size - 1) / size >= 32)) return size;
+    const int least = size == 4 && d.head_dim == 64 ? 64 : 32;  // tiles of a cluster's share
+    if (ctas >= kWave && (last == 0 || last >= 160) && (size == 1 ? tiles > ctas / kWave : (tiles + size - 1) / size >= least)) return size;
   }
   return 0;
 }
