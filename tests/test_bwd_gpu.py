@@ -122,8 +122,8 @@ def test_backward_varlen(cuda_device, native_lib, lens, Hq, Hkv, causal):
 
 def test_backward_is_deterministic(cuda_device, native_lib):
     """With `deterministic` every gradient comes back with the same bits on every call. Without it that holds for every kernel but the
-    fused one (head_dim 64, more key blocks than SMs), whose dQ sums are formed by floating-point reductions in global memory and
-    repeat only to fp32 rounding."""
+    fused one (head_dim 64, more key blocks than SMs, rows above 1024 or grouped heads), whose dQ sums are formed by floating-point
+    reductions in global memory and repeat only to fp32 rounding."""
     q, k, v, dout = (rand((1, 4, 640, 128), s) for s in (1, 2, 3, 4))
     a = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=True)
     b = run_fwd_bwd(cuda_device, q, k[:, :2], v[:, :2], dout, True, deterministic=True)
@@ -138,8 +138,13 @@ def test_backward_is_deterministic(cuda_device, native_lib):
     f, h, i = (run_fwd_bwd(cuda_device, *many, True, deterministic=det) for det in (False, False, True))
     for x, y, z in zip(f, h, i):
         assert torch.equal(x, y) and torch.equal(x, z)
-    # and the fused kernel
+    # the dK/dV and the dQ kernel at head_dim 64
     many = [rand((1, 60, 640, 64), s) for s in (5, 6, 7, 8)]
+    f, h, i = (run_fwd_bwd(cuda_device, *many, True, deterministic=det) for det in (False, False, True))
+    for x, y, z in zip(f, h, i):
+        assert torch.equal(x, y) and torch.equal(x, z)
+    # and the fused kernel
+    many = [rand((1, 20, 1100, 64), s) for s in (5, 6, 7, 8)]
     f, h, i = (run_fwd_bwd(cuda_device, *many, True, deterministic=det) for det in (False, False, True))
     assert torch.equal(f[3], h[3]) and torch.equal(f[4], h[4])
     assert orc.error_stats(f[2], h[2])[0] <= 2e-2 and orc.error_stats(f[2], i[2])[0] <= 2e-2
@@ -249,12 +254,14 @@ def test_reference_tests_own_tolerance_rule(cuda_device, native_lib, dtype, B, H
     ([129, 129], 74, 37, 128, False),         # dense, grouped queries: 148 key blocks, as many as SMs
     ([257, 257], 100, 25, 64, True),          # dense, grouped queries at head_dim 64: 150
     ([1, 300, 513, 64], 32, 8, 128, True),    # packed, grouped queries
+    ([1100, 1100], 10, 10, 64, True),         # dense, rows above 1024 at head_dim 64: the fused kernel without groups
     ([70, 700, 129], 16, 16, 64, True),       # packed, ragged ends, most tiles of the grid empty
+    ([70, 700, 129], 32, 16, 64, True),       # the same, grouped: the fused kernel
     ([513, 2, 385], 12, 12, 104, False),      # packed, padded head_dim: 180
 ])
 def test_backward_on_both_sides_of_the_dispatch(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
-    """Calls with more key blocks than SMs, which the fused kernel (head_dim 64) and the dS GEMM serve, and calls just below, against the
-    oracle; dense ones in the fixed order too; tolerances as above."""
+    """Calls with more key blocks than SMs, which the fused kernel (head_dim 64, grouped or long rows), two CTAs per SM (head_dim 64 otherwise) and
+    the dS GEMM serve, and calls just below, against the oracle; dense ones in the fixed order too; tolerances as above."""
     dev = cuda_device
     total, cu = sum(lens), [sum(lens[:i]) for i in range(len(lens) + 1)]
     q, k, v, dout = rand((total, Hq, D), 1), rand((total, Hkv, D), 2), rand((total, Hkv, D), 3), rand((total, Hq, D), 4)

@@ -89,9 +89,10 @@ def test_forward_with_dropout_matches_oracle_with_the_returned_mask(cuda_device,
     (1, 2, 200, 333, 128, False, 0.48),
     (1, 3, 300, 130, 64, True, 0.22),
     (2, 2, 129, 257, 96, False, 0.1),
-    # more key blocks than SMs: dS through the workspace, or (head_dim 64) the fused kernel
+    # more key blocks than SMs: dS through the workspace, or (head_dim 64, short rows) the dK/dV and the dQ kernel
     (2, 40, 200, 257, 128, True, 0.22),
     (3, 26, 130, 129, 64, False, 0.48),
+    (1, 9, 130, 2100, 64, False, 0.48),   # the fused kernel
     (1, 75, 300, 130, 96, True, 0.1),
     (1, 150, 129, 70, 128, False, 0.1),
 ])

@@ -230,15 +230,15 @@ def test_config4_varlen_gqa_scaled_down(cuda_device, native_lib):
 
 
 @pytest.mark.parametrize("lens,Hq,Hkv,D,causal", [
-    ([193, 769, 342], 32, 32, 128, True),   # up to two rounds of units, claimed late throughout; one group of heads
-    ([300, 1, 700, 64], 64, 8, 64, False),  # the same without a mask: groups by the longest sequence
+    ([193, 769, 342], 32, 32, 128, True),   # three groups of heads, one of four ranks behind them
+    ([300, 1, 700, 64], 64, 8, 64, False),  # without a mask: no ranks behind
     ([200, 62, 234], 40, 8, 128, True),     # one unit per head
     ([134, 282, 200] * 4, 16, 4, 64, True),  # two at most
-    ([128, 888, 150, 130] * 4, 16, 16, 64, True),   # three rounds in mostly empty slots
-    ([700, 900, 888, 600] * 2, 32, 8, 64, True),    # in mostly filled ones
+    ([128, 888, 150, 130] * 4, 16, 16, 64, True),   # mostly empty slots
+    ([700, 900, 888, 600] * 2, 32, 8, 64, True),    # mostly filled ones
 ])
 def test_packed_orders(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
-    """Every side of the rules that order the units of a packed call, against the oracle."""
+    """Packed calls whose list of units has groups, ranks behind them and slots without a unit, against the oracle."""
     gen = torch.Generator().manual_seed(11)
     cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
     q, k, v = (torch.randn(cu[-1], h, D, generator=gen).bfloat16() for h in (Hq, Hkv, Hkv))
@@ -251,7 +251,8 @@ def test_packed_orders(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D", [
-    (3, 16, 16, 600, 600, 64),    # three ranks of 256 rows, one of them behind two groups of heads, the second one short
+    (3, 16, 16, 600, 600, 64),    # three ranks of 256 rows, one of them behind two groups of 24 heads
+    (3, 11, 11, 1100, 1100, 64),  # five ranks, two of them behind groups of 17 and 16 heads: slots without a unit in the second one
     (2, 40, 8, 257, 1100, 128),   # a cached prefix: all ranks have many keys
     (3, 12, 12, 1030, 700, 64),   # units without keys among the lightest
 ])

@@ -82,7 +82,7 @@ def set_bwd(p, dout, dq, dk, dv, packed):
     (2, 2, 2, 1, 300, 128, False),     # one query row: the tile kernel's smallest case
     (1, 4, 2, 200, 333, 160, True),    # head dims above 128: the kernels that stage 256-column tiles
     (2, 2, 1, 129, 70, 256, False),
-    (2, 40, 40, 200, 257, 128, True),   # more key blocks than SMs: dS through the workspace (head_dim 64: the fused backward)
+    (2, 40, 40, 200, 257, 128, True),   # more key blocks than SMs: dS through the workspace (grouped at head_dim 64: the fused backward)
     (3, 26, 26, 333, 130, 80, False),
     (1, 150, 75, 129, 257, 64, True),
 ])
@@ -122,7 +122,7 @@ def test_dense_forward_and_backward_write_nothing_outside_their_outputs(cuda_dev
     ([300, 45], 8, 2, 96, True),
     ([130, 70, 1, 255], 4, 2, 256, True),
     ([128, 129], 2, 2, 136, False),
-    ([130, 70, 1, 255], 20, 20, 128, True),   # more key blocks than SMs: dS through the workspace (head_dim 64: the fused backward)
+    ([130, 70, 1, 255], 20, 20, 128, True),   # more key blocks than SMs: dS through the workspace (grouped at head_dim 64: the fused backward)
     ([128, 129, 127], 26, 26, 64, False),
     ([300, 45], 50, 25, 64, True),
 ])
@@ -240,6 +240,7 @@ def test_backward_with_a_key_bias_needs_no_accumulator(cuda_device, native_lib):
 @pytest.mark.parametrize("Hq,Hkv,D,lens,front,tail", [
     (4, 4, 128, (100, 60), 3, 70),         # few key blocks
     (16, 16, 64, (300, 1, 129) * 6, 5, 1),  # more key blocks than SMs
+    (16, 8, 64, (300, 1, 129) * 7, 5, 1),   # the fused backward
     (40, 8, 128, (200, 300) * 8, 1, 200),   # grouped query heads
     (4, 2, 256, (100, 60), 9, 130),
     (2, 1, 72, (100, 60), 0, 0),            # no such rows
