@@ -284,6 +284,23 @@ def test_backward_on_both_sides_of_the_dispatch(cuda_device, native_lib, lens, H
     assert ops.device_status() == 0
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,L,path", [
+    (8, 64, 8, 381, "fused"),    # a chain of 24 items, 1.5 times an SM's average
+    (1, 32, 8, 2880, "two"),     # of 92, 1.6 times: clusters
+])
+def test_clusters_at_head_dim_64_are_for_long_chains(cuda_device, native_lib, B, Hq, Hkv, L, path):
+    """Under a causal mask, read from the names of the kernels that ran."""
+    from torch.profiler import ProfilerActivity, profile
+    dev = cuda_device
+    q, k, v, do = (rand((B, h, L, 64), s).to(dev) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
+    out, lse = ops.gqa_prefill(q, k, v, is_causal=True)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        ops._dense_backward(do, q, k, v, out, lse, True, 0.125)
+        torch.cuda.synchronize()
+    names = " ".join(e.name for e in prof.events())
+    assert ("bwd_fused_kernel" in names, "bwd_tile_kernel" in names) == (path == "fused", path == "two"), names
+
+
 @pytest.mark.parametrize("L,dropout,path", [(1024, False, "two"), (1025, False, "fused"), (1025, True, "two")])
 def test_short_rows_and_dropout_at_head_dim_64(cuda_device, native_lib, L, dropout, path):
     test_which_backward_kernels_run(cuda_device, native_lib, 1, 20, 20, L, 64, dropout, False, False, path)
