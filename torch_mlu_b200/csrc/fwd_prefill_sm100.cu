@@ -201,13 +201,13 @@ constexpr int kUnitRing = 2;
 // A unit is claimed when the one in front of it has claim_ahead() key blocks left: late, since a unit that a busy CTA has claimed is one that
 // an idle CTA cannot take, and early enough for the claim (atomic, decode, about 1500 cycles) to pass before the Q tiles are free: three blocks. A packed claim
 // takes longer, since it reads the lengths, and once more for every slot without a unit: eight where the list is long, so that few units of it are
-// its end. In a packed list of up to two rounds every unit is its end, and lengths differ: one. (us, claims a whole unit ahead | eight | three | one; long lists, D64: 28
-// sequences of 64 to 3008 tokens, 64/8 heads 1424 | 1424 | 1448, 32 of 192 to 1321, 64/8 - | 478 | 486 | 536, 12 of 64 to 3000, 16/16, 2304 slots 177 | 165 | 165; short
-// ones: 8 of 100 to 900, 16/16, 512 slots - | 28.0 | 23.5 | 23.7, 10 of 47 to 605, 12/12, D128, 360 slots - | 22.1 | 22.0 | 22.9, 7 of 19 to 448, 16/16, unmasked, 224
-// slots - | 18.5 | 18.4 | 17.1; dense: B4 H32/8 L700 D64 - | 31.1 | 28.4 | 28.6, B8 H16 L512 D128, 256 slots - | 22.3 | 21.6 | 22.2.)
-inline int claim_ahead(bool packed, int slots, int ctas) {
+// its end. In an unmasked packed list of up to two rounds every unit is its end, and the heaviest are not in front: one. (us, claims a whole unit ahead | eight | three |
+// one; long lists, D64: 28 sequences of 64 to 3008 tokens, 64/8 heads 1424 | 1424 | 1448, 32 of 192 to 1321, 64/8 - | 478 | 486 | 536, 12 of 64 to 3000, 16/16, 2304 slots
+// 177 | 165 | 165; short ones: 8 of 100 to 900, 16/16, 512 slots - | 28.0 | 23.5 | 23.7, 23 of 51 to 236, 12/12, D128, 276 slots - | 19.5 | 19.5 | 20.4, 7 of 19 to 448, 16/16,
+// unmasked, 224 slots - | 18.5 | 18.4 | 17.1; dense: B4 H32/8 L700 D64 - | 31.1 | 28.4 | 28.6, B8 H16 L512 D128, 256 slots - | 22.3 | 21.6 | 22.2.)
+inline int claim_ahead(bool packed, bool causal, int slots, int ctas) {
   if (!packed) return 3;
-  return slots <= 2 * ctas ? 1 : slots >= 16 * ctas ? 8 : 3;
+  return slots >= 16 * ctas ? 8 : slots > 2 * ctas || causal ? 3 : 1;
 }
 constexpr uint32_t kUnitReaders = 10;  // producer + issuer + 8 softmax warps
 
@@ -902,7 +902,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes),
                          p.is_causal ? tail_ranks(ranks, all_heads_row * unit_rows, all_heads_row * prefix) : 0);
   dim3 grid(kp.order.slots < usable ? kp.order.slots : usable, 1, 1);
-  kp.claim_ahead = claim_ahead(varlen, kp.order.slots, usable);
+  kp.claim_ahead = claim_ahead(varlen, p.is_causal != 0, kp.order.slots, usable);
   // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
   // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
   // cleared already.) Not for two units per CTA, dealt out by index: alone that is faster (B8 H12 L512 D64 unmasked, eager, 22.6 us against
