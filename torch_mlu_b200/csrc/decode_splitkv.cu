@@ -733,7 +733,12 @@ int launch_decode(const sdpa_b200_params& p, DecodeParams& d, float* scratch, ui
   const bool hi = d.rows > 8;
   // under the tail of whatever is in front, unless that is the launch that clears the status word (calls back to back: B64 H32/8 Lk 84 D64
   // 12.3 us -> 9.7, B8 Lk 4096 D128 29.7 -> 27.4, B1 Lk 1000 9.0 -> 8.6)
-  const bool overlap = p.device_status != nullptr;
+  // But not a fixed split into long shares with CTAs for more than a quarter of the SMs (half of them, where the merge kernel stands between two such grids) and fewer than
+  // fill them twice: those that start early find part of the SMs taken, share others in pairs and stream at half the rate to the end (calls back to back, early | plain start:
+  // H16/16, Lk 5857, one split, D64 B4 43.4 | 37.4, B9 44.9 | 40.1, B12 51.9 | 49.3, D128 B6 58.3 | 52.2, B5 H8/8 Lk 9000 D64, 40 CTAs, 62.8 | 55.3, three splits, B2 18.8 | 18.5; but one
+  // split, 32 CTAs, B2 H16/16 Lk 3000 D64 19.4 | 20.8, three, 48 CTAs, B1 Lk 9000 D64 22.2 | 24.6, four, 23 tiles, B2 Lk 5857 15.4 | 16.4).
+  const bool pairs_up = p.num_splits > 0 && d.tiles_per_split >= 28 && d.grid > (p.num_splits > 1 ? 74 : 37) && d.grid < kCtasPerSm * 148;
+  const bool overlap = p.device_status != nullptr && !pairs_up;
   cudaError_t err;
   auto launch = [&](auto hi_tag, auto dim_tag, auto f16_tag) {
     constexpr bool kHi = decltype(hi_tag)::value, kF16 = decltype(f16_tag)::value;
