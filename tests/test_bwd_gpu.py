@@ -307,14 +307,24 @@ def test_short_rows_and_dropout_at_head_dim_64(cuda_device, native_lib, L, dropo
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D,causal", [
-    (1, 2, 2, 65, 190, 64, False),   # one row in the last streamed tile of 64
+    # few blocks, or long chains: streamed tiles of 128 rows
+    (1, 2, 2, 65, 190, 64, False),   # one row in the last 64 of a streamed tile
     (1, 2, 2, 190, 65, 64, True),    # rows without keys
-    (1, 4, 2, 64, 129, 64, True),    # whole tiles of queries, one key in the last block
+    (1, 4, 2, 64, 129, 64, True),    # half a tile of queries, one key in the last block
     (2, 2, 2, 1, 63, 40, False),
     (1, 6, 3, 321, 449, 64, True),   # offsets that are no multiple of 128
+    (1, 37, 37, 129, 129, 64, True),   # 74 blocks, as many as pairs of SMs
+    (1, 37, 37, 700, 300, 64, True),   # 111 key blocks with a chain of six tiles, 222 query blocks of three: one kernel of each kind
+    # more: of 64 rows
+    (1, 80, 80, 65, 190, 64, False),
+    (1, 80, 80, 190, 65, 64, True),
+    (1, 80, 40, 64, 129, 64, True),
+    (2, 75, 75, 1, 63, 40, False),
+    (1, 80, 40, 321, 449, 64, True),
+    (1, 75, 75, 129, 129, 64, True),
 ])
-def test_streamed_tiles_of_64_rows(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
-    """The two kernels up to head_dim 64, whose streamed tiles are half as high as the blocks, against the oracle; tolerances as above."""
+def test_streamed_tiles_of_64_and_128_rows(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
+    """The two kernels up to head_dim 64 with streamed tiles half as high as the blocks and as high, against the oracle; tolerances as above."""
     q, k, v, dout = (rand((B, h, n, D), s) for s, h, n in ((1, Hq, Lq), (2, Hkv, Lk), (3, Hkv, Lk), (4, Hq, Lq)))
     out, lse, *grads = run_fwd_bwd(cuda_device, q, k, v, dout, causal, deterministic=True)
     o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=causal)

@@ -205,6 +205,7 @@ def _bias_reference(q, k, v, bias, do, causal_top_left, dtype=torch.float32):
     (300, 300, 64, True, (2, 1, 300, 300)),      # head broadcast with the causal mask
     (130, 257, 128, True, (1, 1, 1, 257)),       # one bias row for every query; top-left causal with Lq < Lk
     (257, 130, 96, True, (2, 3, 257, 130)),      # top-left causal with Lq > Lk: two kernel calls
+    (130, 70, 64, False, (2, 40, 130, 70)),      # blocks for more than half of the SMs at head_dim 64: two CTAs per SM
 ])
 def test_attn_bias_forward_and_backward(cuda_device, native_lib, dtype, Lq, Lk, D, causal, bias_shape):
     """Additive bias through the memory-efficient operators, as the reference tests exercise it (a random
@@ -212,7 +213,7 @@ def test_attn_bias_forward_and_backward(cuda_device, native_lib, dtype, Lq, Lk, 
     all four gradients against autograd through the fp32 math, held to that suite's own tolerance rule, and to
     the fixed tolerances where values are of order one."""
     dev = cuda_device
-    B, H = 2, 3
+    B, H = 2, max(3, bias_shape[1])
     g = torch.Generator().manual_seed(7)
     q, k, v = (torch.randn(s, generator=g).to(dtype) for s in ((B, H, Lq, D), (B, H, Lk, D), (B, H, Lk, D)))
     bias = torch.rand(bias_shape, generator=g).to(dtype)

@@ -41,15 +41,14 @@
 namespace sdpa_b200 {
 namespace {
 
-// Streamed tiles. Up to head_dim 64 they have 64 rows, so that a CTA's score buffers and accumulators take half of the tensor memory and two
-// CTAs share an SM: the one's exponentials run under the other's MMAs and waits, set-ups and epilogues. Above, the accumulators leave
+// Streamed tiles (kY rows). Up to head_dim 64 they have 64 rows where launches fill the GPU, so that a CTA's score buffers and accumulators take half of the tensor memory and
+// two CTAs share an SM: the one's exponentials run under the other's MMAs and waits, set-ups and epilogues. Above, the accumulators leave
 // no room for that. One chain of 128-row items per SM took as long as at head_dim 128. (Step of B8 H12 L512 with a mask 94.3 -> 88.9 us, B16
-// 153 -> 134, B8 H16 L2048 579 -> 526, B4 H12 L600 with a learned bias 152 -> 144. One warpgroup with 64 columns instead: 97.)
-template <int kD>
-constexpr int kRowsY = kD == 64 ? 64 : kTile;
+// 153 -> 134, B8 H16 L2048 579 -> 526, B4 H12 L600 with a learned bias 152 -> 144. One warpgroup with 64 columns instead: 97.) Where CTAs are few, a chain of 128-row items has
+// half as many and is over sooner: wide_tiles().
 constexpr int kComputeWarps = 8;  // two warpgroups, each with half of an item's columns
-template <int kD>
-constexpr int kThreads = (kComputeWarps + (kD == 64 ? 4 : 3)) * 32;  // compute, TMA producer, two MMA issuers (and an idle warp)
+template <int kY>
+constexpr int kThreads = (kComputeWarps + (kY == 64 ? 4 : 3)) * 32;  // compute, TMA producer, two MMA issuers (and an idle warp)
 // Register hand-over of the instances with two CTAs per SM (setmaxnreg; launched with 80). What the third warpgroup releases
 // covers what the other two take, or the increase would wait forever.
 constexpr int kRegsCompute = 96, kRegsOther = 48;
@@ -63,17 +62,17 @@ constexpr int kModeDKDV = 0;
 constexpr int kModeDQ = 1;
 
 __host__ __device__ constexpr uint32_t x_bytes(int d) { return kTile * d * 2; }                     // one stationary tile
-__host__ __device__ constexpr uint32_t y_bytes(int d) { return (d == 64 ? 64 : kTile) * d * 2; }    // one streamed tile
+__host__ __device__ constexpr uint32_t y_bytes(int d, int y) { return y * d * 2; }            // one streamed tile
 constexpr uint32_t kSmemX = 0;                                   // stationary pair
 __host__ __device__ constexpr uint32_t smem_y_off(int d) { return 2 * x_bytes(d); }
-__host__ __device__ constexpr uint32_t smem_vec_off(int mode, int d) { return smem_y_off(d) + stages_for(mode, d) * y_bytes(d); }
+__host__ __device__ constexpr uint32_t smem_vec_off(int mode, int d, int y) { return smem_y_off(d) + stages_for(mode, d) * y_bytes(d, y); }
 // per-slot (lse2[128], delta[128]), dK/dV only
-__host__ __device__ constexpr uint32_t smem_bar_off(int mode, int d) { return smem_vec_off(mode, d) + (mode == 1 ? 0 : stages_for(mode, d) * 1024); }
+__host__ __device__ constexpr uint32_t smem_bar_off(int mode, int d, int y) { return smem_vec_off(mode, d, y) + (mode == 1 ? 0 : stages_for(mode, d) * 1024); }
 // behind the barriers, dQ with a key bias only: 64 16-bit bias values per compute warp
-__host__ __device__ constexpr uint32_t smem_key_bias_off(int mode, int d) { return smem_bar_off(mode, d) + 256; }
+__host__ __device__ constexpr uint32_t smem_key_bias_off(int mode, int d, int y) { return smem_bar_off(mode, d, y) + 256; }
 // at least 80 KB: a third CTA on the SM would wait for tensor memory
-__host__ __device__ constexpr uint32_t smem_bytes_for(int mode, int d, bool key_bias) {
-  const uint32_t used = smem_key_bias_off(mode, d) + (mode == 1 && key_bias ? 8 * 128 : 0) + 1024;
+__host__ __device__ constexpr uint32_t smem_bytes_for(int mode, int d, int y, bool key_bias) {
+  const uint32_t used = smem_key_bias_off(mode, d, y) + (mode == 1 && key_bias ? 8 * 128 : 0) + 1024;
   return used > 80 * 1024 ? used : 80 * 1024;
 }
 constexpr uint32_t kBarXFull = 0;
@@ -117,8 +116,8 @@ enum BiasKind { kNoBias = 0, kFullBias = 1, kKeyBias = 2 };
 // kDsCall: the call's dS goes through the workspace where there is room (launch_bwd). An instance of its own, since with both kinds of
 // exponentials and the dS stores behind branches the calls without dS were slower (dK/dV and dQ kernel of 6 packed sequences of 50 to 4000
 // tokens, 32/8 heads, unmasked: 1222 + 1076 us, so 1137 + 1019).
-template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall, bool kSplit>
-__global__ void __launch_bounds__(kThreads<kD>, kD == 64 ? 2 : 1)
+template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall, bool kSplit, int kY>
+__global__ void __launch_bounds__(kThreads<kY>, kY == 64 ? 2 : 1)
 bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_o1, const __grid_constant__ CUtensorMap tm_o2,
@@ -139,14 +138,16 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
     *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid; here, since block 0 may be one without work
   constexpr int kStages = stages_for(kMode, kD);
-  constexpr int kY = kRowsY<kD>;
   constexpr int kC = kY / 2;  // columns per compute warpgroup, i.e. per thread
   constexpr int kTmaWarp = kComputeWarps, kScoreWarp = kTmaWarp + 1, kAccWarp = kTmaWarp + 2;
-  constexpr uint32_t kTmemCols = 2 * kY + 2 * kD;
-  constexpr uint32_t kXBytes = x_bytes(kD), kYBytes = y_bytes(kD);
+  constexpr uint32_t kTmemCols = kY == 64 ? 256 : 512;
+  static_assert(2 * kY + 2 * kD <= static_cast<int>(kTmemCols), "score buffers and accumulators");
+  constexpr uint32_t kXBytes = x_bytes(kD), kYBytes = y_bytes(kD, kY);
   constexpr uint32_t kSmemY = smem_y_off(kD);
-  constexpr uint32_t kSmemVec = smem_vec_off(kMode, kD);
-  constexpr uint32_t kSmemBar = smem_bar_off(kMode, kD);
+  constexpr uint32_t kSmemVec = smem_vec_off(kMode, kD, kY);
+  constexpr uint32_t kSmemBar = smem_bar_off(kMode, kD, kY);
+  constexpr int kBoxRows = kD == 64 ? 64 : kTile;  // of the maps that load; a tile of 128 rows takes two boxes of 64
+  constexpr uint32_t kBoxBytes = kBoxRows * kD * 2;
 
   // CTA order (1-D grid, block_order.cuh): heaviest blocks first (dK/dV: key block 0 sees every query; dQ: the last query block sees
   // every key). Packed, causal: blocks with the same number of blocks behind (dQ: in front of) them in their own
@@ -258,6 +259,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const CUtensorMap* tm = first ? tmy1 : tmy2;
         tma_load_4d(dst, tm, full, 0, row, hy, bcoord);
         if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, full, 64, row, hy, bcoord);
+        else if (kY > kBoxRows) tma_load_4d(dst + kBoxBytes, tm, full, 0, row + kBoxRows, hy, bcoord);
     return true;
   };
 
@@ -295,7 +297,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t dst = base + kSmemX + x * kXBytes;
         tma_load_4d(dst, tm, bar + kBarXFull, 0, x_row, hx, bcoord);
         if (kD > 64) tma_load_4d(dst + kHalfBytes, tm, bar + kBarXFull, 64, x_row, hx, bcoord);
-        else tma_load_4d(dst + kYBytes, tm, bar + kBarXFull, 0, x_row + kY, hx, bcoord);  // the maps' boxes have kY rows
+        else tma_load_4d(dst + kBoxBytes, tm, bar + kBarXFull, 0, x_row + kBoxRows, hx, bcoord);
       }
     }
     if (kMode == kModeDKDV) {
@@ -323,7 +325,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #endif
 
   if (warp >= kTmaWarp) {
-    if constexpr (kD == 64) reg_decrease<kRegsOther>();
+    if constexpr (kY == 64) reg_decrease<kRegsOther>();
     if (warp == kTmaWarp) {
       // ------------------------------------------------------------------ TMA producer (rest of the ring)
       if (n_items > 0 && elect_one()) {
@@ -514,7 +516,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------------ compute warpgroups
-    if constexpr (kD == 64) reg_increase<kRegsCompute>();
+    if constexpr (kY == 64) reg_increase<kRegsCompute>();
     // warps 0-3 own the first kC streamed columns of every stationary row, warps 4-7 the others
     const int half = warp >> 2;
     const int r = (warp & 3) * 32 + lane;  // stationary row in the tile = TMEM lane
@@ -685,7 +687,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         constexpr float kLog2e = 1.4426950408889634f;
         float key_bias = 0.f, key_bias_log2 = 0.f;  // dK/dV
-        uint32_t* key_bias_row = reinterpret_cast<uint32_t*>(smem + smem_key_bias_off(kMode, kD) + warp * 128);  // dQ
+        uint32_t* key_bias_row = reinterpret_cast<uint32_t*>(smem + smem_key_bias_off(kMode, kD, kY) + warp * 128);  // dQ
         if constexpr (kBias == kKeyBias) {
           if (kMode == kModeDKDV) {
             key_bias = unpack_16x2<kF16>(key_bias_raw).x;
@@ -1097,33 +1099,39 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
 using TileKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                             const CUtensorMap, const CUtensorMap, const BwdKernelParams);
 
+template <int kMode, bool kDrop, int kBias, bool kSplit, int kD, bool kDsCall, int kY>
+TileKernel pick_tile_kernel(bool f16) {
+  return f16 ? bwd_tile_kernel<kMode, kD, true, kDrop, kBias, kDsCall, kSplit, kY> : bwd_tile_kernel<kMode, kD, false, kDrop, kBias, kDsCall, kSplit, kY>;
+}
+
 template <int kMode, bool kDrop, int kBias, bool kSplit = false>
-TileKernel pick_tile_kernel(int head_dim, bool f16, bool ds_call) {
-  if (head_dim <= 64)
-    return f16 ? bwd_tile_kernel<kMode, 64, true, kDrop, kBias, false, kSplit> : bwd_tile_kernel<kMode, 64, false, kDrop, kBias, false, kSplit>;
-  if (ds_call)
-    return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, true, kSplit> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, true, kSplit>;
-  return f16 ? bwd_tile_kernel<kMode, 128, true, kDrop, kBias, false, kSplit> : bwd_tile_kernel<kMode, 128, false, kDrop, kBias, false, kSplit>;
+TileKernel pick_tile_kernel(int head_dim, bool f16, bool ds_call, bool wide) {
+  if (head_dim <= 64) {
+    if constexpr (!kSplit)
+      if (wide) return pick_tile_kernel<kMode, kDrop, kBias, kSplit, 64, false, kTile>(f16);
+    return pick_tile_kernel<kMode, kDrop, kBias, kSplit, 64, false, 64>(f16);
+  }
+  return ds_call ? pick_tile_kernel<kMode, kDrop, kBias, kSplit, 128, true, kTile>(f16) : pick_tile_kernel<kMode, kDrop, kBias, kSplit, 128, false, kTile>(f16);
 }
 
 template <int kMode, bool kDrop>
-TileKernel pick_tile_kernel(BiasKind bias, int head_dim, bool f16, bool ds_call) {
-  if (bias == kKeyBias) return pick_tile_kernel<kMode, kDrop, kKeyBias>(head_dim, f16, ds_call);
-  return bias == kFullBias ? pick_tile_kernel<kMode, kDrop, kFullBias>(head_dim, f16, ds_call)
-                           : pick_tile_kernel<kMode, kDrop, kNoBias>(head_dim, f16, ds_call);
+TileKernel pick_tile_kernel(BiasKind bias, int head_dim, bool f16, bool ds_call, bool wide) {
+  if (bias == kKeyBias) return pick_tile_kernel<kMode, kDrop, kKeyBias>(head_dim, f16, ds_call, wide);
+  return bias == kFullBias ? pick_tile_kernel<kMode, kDrop, kFullBias>(head_dim, f16, ds_call, wide)
+                           : pick_tile_kernel<kMode, kDrop, kNoBias>(head_dim, f16, ds_call, wide);
 }
 
 template <int kMode>
-TileKernel pick_tile_kernel(bool drop, BiasKind bias, int head_dim, bool f16, bool ds_call) {
-  return drop ? pick_tile_kernel<kMode, true>(bias, head_dim, f16, ds_call)
-              : pick_tile_kernel<kMode, false>(bias, head_dim, f16, ds_call);
+TileKernel pick_tile_kernel(bool drop, BiasKind bias, int head_dim, bool f16, bool ds_call, bool wide) {
+  return drop ? pick_tile_kernel<kMode, true>(bias, head_dim, f16, ds_call, wide)
+              : pick_tile_kernel<kMode, false>(bias, head_dim, f16, ds_call, wide);
 }
 
 // `overlap_previous`: launch with programmatic stream serialization, so that this grid's CTAs may start as soon as
 // every CTA of the kernel before it in the stream has signalled launch_dependents and an SM has room. Used for the dK/dV kernel
 // behind the pre-pass, and for the dQ kernel, which needs nothing the dK/dV kernel writes: its CTAs fill the SMs the last, partly
-// empty wave of dK/dV CTAs leaves idle.
-int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t stream, const CUtensorMap& tm_q,
+// empty wave of dK/dV CTAs leaves idle. `wide`, up to head_dim 64: streamed tiles of 128 rows, one CTA per SM.
+int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, bool wide, cudaStream_t stream, const CUtensorMap& tm_q,
                        const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                        const CUtensorMap& tm_o1, const CUtensorMap& tm_o2, const BwdKernelParams& kp,
                        bool overlap_previous = false) {
@@ -1133,12 +1141,12 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
                         : kp.bias_row_stride == 0 && (mode == kModeDKDV || kp.dbias == nullptr) ? kKeyBias
                                                                                                               : kFullBias;
   const bool split = mode == kModeDKDV && kp.split > 1;
-  TileKernel kernel = split ? (drop ? pick_tile_kernel<kModeDKDV, true, kNoBias, true>(head_dim, f16, kp.ds_call != 0)
-                                    : pick_tile_kernel<kModeDKDV, false, kNoBias, true>(head_dim, f16, kp.ds_call != 0))
-                      : mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16, kp.ds_call != 0)
-                                        : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16, kp.ds_call != 0);
-  const int dim = head_dim <= 64 ? 64 : 128;  // the instance
-  const uint32_t smem = smem_bytes_for(mode, dim, bias == kKeyBias);
+  TileKernel kernel = split ? (drop ? pick_tile_kernel<kModeDKDV, true, kNoBias, true>(head_dim, f16, kp.ds_call != 0, false)
+                                    : pick_tile_kernel<kModeDKDV, false, kNoBias, true>(head_dim, f16, kp.ds_call != 0, false))
+                      : mode == kModeDKDV ? pick_tile_kernel<kModeDKDV>(drop, bias, head_dim, f16, kp.ds_call != 0, wide)
+                                        : pick_tile_kernel<kModeDQ>(drop, bias, head_dim, f16, kp.ds_call != 0, wide);
+  const int dim = head_dim <= 64 ? 64 : 128, rows = dim == 64 && (split || !wide) ? 64 : kTile;  // the instance
+  const uint32_t smem = smem_bytes_for(mode, dim, rows, bias == kKeyBias);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) {
     set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", smem, cudaGetErrorString(err));
@@ -1146,7 +1154,7 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, cudaStream_t 
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(split ? grid * kp.split : grid);
-  cfg.blockDim = dim3(dim == 64 ? kThreads<64> : kThreads<128>);
+  cfg.blockDim = dim3(rows == 64 ? kThreads<64> : kThreads<kTile>);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -1197,6 +1205,12 @@ int64_t key_blocks(const sdpa_b200_params& p) {
   return static_cast<int64_t>(p.batch) * p.heads_kv * ((static_cast<int64_t>(p.max_seqlen_k) + kTile - 1) / kTile);
 }
 constexpr int64_t kSms = 148;
+
+// Up to head_dim 64: streamed tiles of 128 rows, from the blocks of a launch and the longest chain of such items. With blocks for at most half of the SMs every block has a pair
+// of SMs to itself, and with one per SM long chains are worth it still. (Backward alone, 64 rows | 128, us; up to 74 blocks: B1 H8 L1051 unmasked 30.7 | 23.8, B6 H8/1 L197
+// unmasked 41.0 | 32.8, B2 H8 L453 20.5 | 16.4, B1 H16 L308 15.7 | 14.4; up to 148: B3 H32/8 L457 unmasked 57.2 | 47.6, B5 H16/4 L709 86.3 | 73.9, B1 H16 L656 causal, a chain of 6, 23.1 |
+// 18.5; but chains of 5, 4, 3 and 1: B1 H16 L539 21.4 | 24.6, B2 H16 L475 21.5 | 23.9, B4 H12 L285 18.5 | 22.3, B7 H16 L75 12.6 | 14.4.)
+bool wide_tiles(double blocks, int chain) { return blocks <= kSms / 2 || (blocks <= kSms && chain >= 6); }
 
 // CTAs that share the query heads of a key block (calls without bias). One CTA sums a whole group, in a chain of group x query tiles items;
 // where the longest chain is a multiple (the ratio below) of what an SM has to do on average, a cluster takes the heads in shares and sums
@@ -1315,7 +1329,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   const int64_t rows_k = varlen ? p.total_k : p.max_seqlen_k;
   const int64_t nb = varlen ? 1 : p.batch;
   int st;
-  const int box = p.head_dim <= 64 && !fused ? kRowsY<64> : kTile;  // rows of the streamed tiles; stationary ones take two
+  const int box = p.head_dim <= 64 && !fused ? 64 : kTile;  // rows; tiles of 128 take two
   if ((st = make_tensor_map_16(f16, &tm_q, p.q, p.head_dim, rows_q, p.heads_q, nb, p.q_row_stride, p.q_head_stride,
                                  p.q_batch_stride, box)) != SDPA_B200_OK)
     return st;
@@ -1418,7 +1432,7 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
       kp.bh0 = first;
       kp.ds.head0 = first * kp.kv_group;
       const int grid = set_order(p.heads_kv, p.max_seqlen_k, n, p.max_seqlen_q, kp.kv_group, rows_q_all);
-      if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
+      if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid, true, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
                                    /*overlap_previous=*/first == 0)) != SDPA_B200_OK)
         return st;
       if ((st = launch_bwd_ds_gemm(p, kp.ds, first, n, false, kp.ds_counter, kp.status, stream)) != SDPA_B200_OK) return st;
@@ -1431,11 +1445,15 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   if ((st = make_tensor_map_16(f16, &tm_dq, p.dq, p.head_dim, rows_q, p.heads_q, nb, p.dq_row_stride, p.dq_head_stride,
                                  p.dq_batch_stride, kTile)) != SDPA_B200_OK)
     return st;
-  if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
+  // a packed call's blocks are those with rows: half a block more per sequence and head than the rows fill
+  const auto blocks = [&](int grid, int heads, int rows) { return varlen ? heads * (rows / static_cast<double>(kTile) + 0.5 * p.batch) : grid; };
+  const auto tiles = [](int rows) { return (rows + kTile - 1) / kTile; };
+  const bool wide_dkdv = wide_tiles(blocks(grid_dkdv, p.heads_kv, p.total_k), kp.kv_group * tiles(p.max_seqlen_q));
+  if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, wide_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
                                /*overlap_previous=*/true)) != SDPA_B200_OK)
     return st;
   const int grid_dq = set_order(p.heads_q, p.max_seqlen_q, p.batch * p.heads_q, p.max_seqlen_k, 1, rows_k_all);
-  return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kp,
+  return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, wide_tiles(blocks(grid_dq, p.heads_q, p.total_q), tiles(p.max_seqlen_k)), stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kp,
                             /*overlap_previous=*/true);
 }
 
