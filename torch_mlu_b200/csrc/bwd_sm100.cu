@@ -1219,7 +1219,8 @@ bool wide_tiles(double blocks, int chain) { return blocks <= kSms / 2 || (blocks
 // heads, unmasked 402 | 377 | 363; 1, 8 of 64 to 2000, 16/4 331 | 295 | 331; 2.1, 16 of 64 to 2000, 8/1 374 | 321 | 296; 2.3, chain of 36, 4 of 64 to
 // 1280, 32/8 132 | 122 | 137; 4.5, 4 of 64 to 1280, 16/4 121 | 93 | 83; rows of nearly one length, whose chains fill the SMs more evenly: 1.24,
 // 2 of 1900 to 2000, 16/4, unmasked 260 | 225, and 1.4, 5 of 900 to 1700 191 | 184; but 1.18, 4 of 2000 to 2100 244 | 255; also 0.6, 8 of 500 to
-// 1500, 32/8 374 | 404. Chains of less than 48 want a ratio of two there as well, since the fused kernel is the better one for them: backward alone, 1.23, chain of 32, 32 of 197
+// 1500, 32/8 374 | 404. Chains of less than 48 want a ratio of two there as well where the fused kernel is the other choice, which is the better one for them (but against one CTA per block, up to
+// 148 of them: 1.2, chain of 24, 5 of 654, 16/4 backward alone 70 | 64): backward alone, 1.23, chain of 32, 32 of 197
 // to 397, 64/8 165 | 184, 1.71, 24, 8 of 175 to 708, 32/8 80 | 88, 1.41, 44, 4 of 636 to 1336, 32/8 111 | 122; but 2.4, 30, 32 of 136 to 631, 12/2 97 | 94, and longer ones 1.25, 60, 10 of
 // 385 to 1850 178 | 175, 1.1, 144, 32 of 328 to 2297, 8/1 486 | 388. D128: 2.3, 16 of 100 to 2500, 8/1 489 | 405 | 433; 4.6, 2 of 300 to 2000, 16/4 151 | 112 | 120; 8, 6 of 200 to 1500, 8/1
 // 232 | 154 | 116, eight 152; but 1, 12 of 64 to 2048, 16/4 326 | 351, and 2.4, chain of 20, 8 of 64 to 700, 16/4, unmasked 103.5 | 108.5: a cluster
@@ -1235,7 +1236,8 @@ int bwd_split(const sdpa_b200_params& p) {
   const double chain = group * query_tiles;
   if (p.bias != nullptr || chain < (narrow ? 24 : 32)) return 1;
   if (group % 4 == 0 && ratio >= (narrow ? (chain < 64 ? 3.0 : 2.0) : 6.0)) return 4;
-  return group % 2 == 0 && ratio >= (!narrow || chain < 48 ? 2.0 : mean_tiles < 0.75 * query_tiles ? 0.9 : 1.2) ? 2 : 1;
+  const bool or_fused = p.deterministic == 0 && key_blocks(p) > kSms;  // what the call would take instead
+  return group % 2 == 0 && ratio >= (!narrow || (or_fused && chain < 48) ? 2.0 : mean_tiles < 0.75 * query_tiles ? 0.9 : 1.2) ? 2 : 1;
 }
 
 bool use_ds_backward(const sdpa_b200_params& p) {
