@@ -15,7 +15,7 @@
 //      which later turns their P into exact zeros).
 //   2. bwd_tile_kernel<kModeDKDV>: one CTA, or a cluster that shares the query heads (bwd_split), per (batch, kv head,
 //      128-key block). K and V tiles
-//      stay in shared memory; (Q, dO) tiles (of 128 rows, or 64 up to head_dim 64) stream through a TMA ring. Per Q tile:
+//      stay in shared memory; (Q, dO) tiles (of 128 rows, up to head_dim 64 of 64 unless wide_tiles()) stream through a TMA ring. Per Q tile:
 //      S^T = K Q^T and dP^T = V dO^T on tcgen05 into TMEM, two compute warpgroups (thread = key
 //      row = TMEM lane, one warpgroup per half of the tile's queries) form P^T and dS^T, write
 //      them back to TMEM as bf16, and MMAs with the TMEM operand accumulate dV += P^T dO and
@@ -24,7 +24,7 @@
 //      stay, (K, V) stream; S = Q K^T, dP = dO V^T, dS -> TMEM, dQ += dS K. Or, where launch 2 has left its dS
 //      in the workspace as well (8 stores of 16 bytes per thread and item: 281 -> 308 us at B8 H16 L2048 D128
 //      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> 130).
-// TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512), or four times 64 columns. The bf16 P and dS of an item both
+// TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512); up to head_dim 64 accumulators of 64 columns, with tiles of 64 rows four times 64. The bf16 P and dS of an item both
 // live in the item's score buffer, so the buffer that held dP is free as soon as it has been read;
 // the MMA issuer uses that (and, for dQ, the unused ACC2) to run the next item's score GEMMs and
 // exponentials under the current item's accumulation MMAs (buffer schedule at the issuer).
@@ -699,7 +699,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         // x = S c - lse2. kPolyOf4 of every four column pairs take their 2^x from the FMA pipe (exp2_poly3_x2). dQ: one; two already
         // cost issue slots. dK/dV: two, which shortens the chain of an item (step of B1 H8 L2048 D128 78.7 us, without any 82.0). None up to
-        // head_dim 64: with two CTAs per SM one of four takes the same time (B8 H12 L1000 126, 126). And none where dS goes through the workspace: those grids are full and run at the power
+        // head_dim 64: with two CTAs per SM one of four takes the same time (B8 H12 L1000 126, 126), and with one per SM, where two would save 0 to 6 %, the bits are to be the same. And none where dS goes through the workspace: those grids are full and run at the power
         // cap, where none to two take the same time (step of B8 H16 L2048 695, 694, 696 us, with dropout 858, 872, 870; B12 packed
         // 64 to 2048 tokens 369, 368, 364), and none is the most exact. Such a call without room for dS takes these two kernels, and its
         // bits must not tell: none here either, and the same roundings in both kernels (a key bias joins with one).
