@@ -2,7 +2,10 @@
 // has left in the workspace (ds_tiles.cuh).
 //
 // Bound by memory: every dS tile is read once, 32 KB for 128 x 128 x head_dim multiply-adds. Two 128-row tiles per unit share each B
-// block (48 KB per step of 64 at head_dim 128 where single tiles would read 64). B8 H16 L2048 D128 causal: 0.57 GB of dS in 130 us.
+// block (48 KB per step of 64 at head_dim 128 where single tiles would read 64). B8 H16 L2048 D128 causal: 0.57 GB of dS in 118 us. What the kernel in front
+// wrote last is read first, from L2, which is asked to keep dS in front of what streams past it when it is written and to give it up when it has been read
+// (up to head_dim 128, where it is read once): 603 MB from memory instead of 666, 130 us -> 118, and 0.9 % of a step at the power cap (B8 H16 L2048 687 -> 682 us,
+// packed 12 of 64 to 2048 tokens, 16/4 heads, 339 -> 336). Above, where dK and dQ read it and L2 keeps it for neither, the hints changed nothing.
 //
 // Persistent: one CTA per SM takes units of 256 output rows (two 128-row tiles that share every B block) of one head from a
 // counter, heaviest first inside a group of heads. Per 64 rows of the contraction a stage brings B (64 rows of K or Q, 128-byte
@@ -131,6 +134,7 @@ bwd_ds_gemm_kernel(const __grid_constant__ CUtensorMap tm_ds_q, const __grid_con
       // everything above runs under the tail of the grid that writes dS and clears the counter
       asm volatile("griddepcontrol.wait;" ::: "memory");
       const uint32_t boxes = (p.head_dim + 63) / 64;
+      const uint64_t read_once = l2_drop();
       uint32_t stage = 0, unit_count = 0;
       bool ok = true;
       uint32_t u = atomicAdd(p.counter, 1u);
@@ -218,7 +222,8 @@ bwd_ds_gemm_kernel(const __grid_constant__ CUtensorMap tm_ds_q, const __grid_con
                     tma_load_4d(a_dst, &tm_ds_k, full, 0, tile * 16 + (ks & 1) * 8, 0, 0);
                   } else {
                     const int tile = static_cast<int>(ds.tile(x, ks >> 1));
-                    tma_load_4d(a_dst, &tm_ds_q, full, (ks & 1) * 128, tile * 16, 0, 0);
+                    if constexpr (kD == 128) tma_load_4d_hint(a_dst, &tm_ds_q, full, (ks & 1) * 128, tile * 16, 0, 0, read_once);
+                    else tma_load_4d(a_dst, &tm_ds_q, full, (ks & 1) * 128, tile * 16, 0, 0);
                   }
                 }
                 for (uint32_t c = 0; c < boxes; ++c) tma_load_4d(dst + c * kBoxBytes, tm_b, full, c * 64, b_row, b_head, bcoord);

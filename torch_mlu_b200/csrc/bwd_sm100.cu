@@ -811,12 +811,12 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       BWD_STAMP(half, i, 7);
       if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr) {
         // dS for the dQ GEMM: 16 bytes (8 queries) per store, 512 contiguous bytes per warp. Behind the arrival, so that the
-        // dK GEMM does not wait for the stores to issue
+        // dK GEMM does not wait for the stores to issue. L2 is asked to keep them for that GEMM (figures there)
         if (ds_tile < p.ds.capacity) {
           uint4* dst = ds_group(p.ds, ds_tile, half * 8, r);
 #pragma unroll
           for (int ch = 0; ch < kC / 8; ++ch)
-            dst[ch * kDsTile] = make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]);
+            st_global_hint(dst + ch * kDsTile, make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]), l2_keep());
         }
         // past this row of tiles; behind the last one the next head's tiles begin
         const DsHead rows{0, (len_k + kTile - 1) / kTile, ds_shift(len_q, len_k, p.is_causal != 0)};
