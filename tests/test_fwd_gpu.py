@@ -272,3 +272,38 @@ def test_single_tile_units(cuda_device, native_lib, B, H, Lq, Lk, D, causal):
     """Both sides of the rule that gives every 128-row tile an SM of its own, against the oracle."""
     q, k, v = rand((B, H, Lq, D), 1), rand((B, H, Lk, D), 2), rand((B, H, Lk, D), 3)
     check_dense(cuda_device, q, k, v, causal)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Lq,Lk,D,causal", [
+    (1, 149, 149, 100, 100, 64, True),     # one unit more than SMs
+    (1, 37, 37, 1025, 1025, 64, True),     # five units per head, the last of one row
+    (3, 50, 25, 300, 200, 128, True),      # units without keys, whose rows become zero; 16 empty slots in the last group of heads
+    (8, 48, 48, 200, 300, 64, False),      # more than two rounds
+    (9, 32, 8, 257, 64, 96, True),
+])
+def test_units_taken_from_waiting_ctas(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):
+    """Who runs a unit must not show: the same bits as by the counter, which a call that leaves SMs free still goes by."""
+    gen = torch.Generator(device=cuda_device).manual_seed(3)
+    q, k, v = (torch.randn(B, h, n, D, generator=gen, device=cuda_device, dtype=torch.bfloat16)
+               for h, n in ((Hq, Lq), (Hkv, Lk), (Hkv, Lk)))
+    for _ in range(3):  # back to back, each under the tail of the one in front
+        out, lse = ops.gqa_prefill(q, k, v, is_causal=causal)
+    out2, lse2 = ops.gqa_prefill(q, k, v, is_causal=causal, sm_margin=1)
+    assert ops.device_status() == 0
+    assert torch.equal(out, out2) and torch.equal(lse, lse2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_packed_units_taken_from_waiting_ctas(cuda_device, native_lib, D):
+    """Most slots of the list are empty: one long sequence among short ones and ones without tokens, against each sequence's own call."""
+    lens = [700, 0, 1, 130, 0, 65, 256, 3, 300, 0]
+    gen = torch.Generator(device=cuda_device).manual_seed(4)
+    q, k, v = (torch.randn(sum(lens), h, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for h in (24, 6, 6))
+    ends = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    cu = torch.tensor(ends, dtype=torch.int32, device=cuda_device)
+    out, lse = ops._flash_attention_forward(q, k, v, cu, cu, max(lens), max(lens), 0.0, True, False)[:2]
+    assert ops.device_status() == 0
+    for lo, hi in zip(ends, ends[1:]):
+        if hi > lo:
+            o, l = ops.gqa_prefill(*(t[lo:hi].transpose(0, 1).unsqueeze(0) for t in (q, k, v)), is_causal=True)
+            assert torch.equal(out[lo:hi], o[0].transpose(0, 1)) and torch.equal(lse[..., lo:hi].reshape(24, -1), l[0])

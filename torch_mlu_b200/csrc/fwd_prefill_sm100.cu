@@ -73,9 +73,13 @@ constexpr uint32_t kBarUnitFull = kBarClaim + 8;           // kUnitRing: the sch
 constexpr uint32_t kBarUnitEmpty = kBarUnitFull + 16;      // kUnitRing: every reader has copied the entry
 constexpr uint32_t kBarStageFree = kBarUnitEmpty + 16;     // 2: the warpgroup's staging buffer may be rewritten
 constexpr uint32_t kBarStageFull = kBarStageFree + 16;     // 2: all four warps have written their rows
-constexpr uint32_t kSmemTmemPtr = kBarStageFull + 16;
+constexpr uint32_t kBarTaken = kBarStageFull + 16;         // the answer to a request for a CTA that has not started
+constexpr uint32_t kSmemTmemPtr = kBarTaken + 8;
 constexpr uint32_t kSmemAbort = kSmemTmemPtr + 4;
+static_assert(kSmemAbort + 4 <= 256, "the barriers reach into the units");
 constexpr uint32_t kSmemUnits = 256;  // offset of the Unit ring from kSmemBar (2 x 64 bytes)
+constexpr uint32_t kSmemTaken = 384;    // the answer to the last request for a CTA that has not started, 16 bytes
+constexpr uint32_t kSmemRequests = 400;  // such requests so far
 constexpr uint32_t kSmemStash = 512;   // per softmax warp: the unit's coordinates for the epilogue (8 x 32 bytes)
 constexpr uint32_t kSmemStage = kSmemBar + 1024;  // 2 x 16 KB: one 64-column half of an O tile per softmax warpgroup
 constexpr uint32_t kStageBytes = kBlockM * 128;
@@ -88,7 +92,8 @@ struct FwdKernelParams {
   const int32_t* cu_q;
   const int32_t* cu_k;
   uint32_t* status;
-  uint32_t* unit_counter;  // zeroed before the launch, or null: every CTA takes the one slot of its own index
+  uint32_t* unit_counter;  // zeroed before the launch, or null: every CTA begins with the slot of its own index
+  int steal;               // and goes on with those of CTAs that have not started
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int seqlen_q, seqlen_k, total_q, heads_q, kv_group;
   int head_dim;  // <= kD: the real row length, for the paths that write rows without TMA
@@ -178,18 +183,28 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
   return true;
 }
 
-// The next unit of the list (u.done: there is none). Without a counter every CTA has the slot of its own index.
-__device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first, Unit& u) {
+// The next unit of the list (u.done: there is none).
+__device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first, uint8_t* smem, uint32_t bar, volatile uint32_t* abort_flag, Unit& u) {
   for (;; first = false) {
-    const int slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
-                     : first                   ? static_cast<int>(blockIdx.x)
-                                               : p.order.slots;
+    int slot = p.order.slots;
+    if (p.unit_counter != nullptr) {
+      slot = static_cast<int>(atomicAdd(p.unit_counter, 1u));
+    } else if (first) {
+      slot = static_cast<int>(blockIdx.x);
+    } else if (p.steal) {
+      volatile uint32_t* requests = reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests);
+      const uint32_t n = *requests;
+      *requests = n + 1;
+      take_waiting_cta(bar + kSmemTaken, bar + kBarTaken);
+      const int cta = mbar_wait(bar + kBarTaken, n & 1, abort_flag) ? taken_cta(bar + kSmemTaken) : -1;
+      if (cta >= 0) slot = cta;
+    }
     u.done = slot >= p.order.slots;
     if (u.done || decode_unit(p, slot, u)) return;  // padding slots and row-less units are skipped
   }
 }
 
-// Persistent kernel: gridDim.x CTAs (one per SM) take units off a global counter in list order, which
+// Persistent kernel: one CTA per SM takes units in list order, from the CTAs that have not started or off a global counter (launch_fwd_prefill), which
 // balances the uneven causal units the way the hardware block scheduler would. Warp 10 is the unit
 // scheduler: it claims the next slot (the first one is the producer's), decodes it (integer divisions, cu_seqlens loads) off everyone's
 // critical path and publishes the Unit through a two-entry shared-memory ring; the producer, the MMA
@@ -338,6 +353,8 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bar + kBarStageFull + 8 * t, 4);
     }
     mbar_init(bar + kBarClaim, 1);
+    mbar_init(bar + kBarTaken, 1);
+    *reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests) = 0u;
     for (int e = 0; e < kUnitRing; ++e) {
       mbar_init(bar + kBarUnitFull + 8 * e, 1);
       mbar_init(bar + kBarUnitEmpty + 8 * e, kUnitReaders);
@@ -347,7 +364,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     const bool packed = p.cu_q != nullptr;  // the lengths are in memory
     if (packed) wait_for_previous_grid();
     Unit u;
-    claim_unit(p, true, u);
+    claim_unit(p, true, smem, bar, abort_flag, u);
     write_unit(smem, 0, u);
     mbar_arrive(bar + kBarUnitFull);
     if (!packed) wait_for_previous_grid();
@@ -495,7 +512,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (ok && last_runs) ok = mbar_wait(bar + kBarClaim, (runs - 1) & 1, abort_flag);
           if (!ok) break;
           Unit u;
-          claim_unit(p, false, u);
+          claim_unit(p, false, smem, bar, abort_flag, u);
           done = u.done;
           last_runs = !u.done && u.n_iter > 0;
           if (last_runs) ++runs;
@@ -901,22 +918,32 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   const int prefix = p.max_seqlen_k > p.max_seqlen_q ? p.max_seqlen_k - p.max_seqlen_q : 0;
   kp.order = block_order(heads, ranks, heads_per_l2_group(kv_row_bytes * p.max_seqlen_k / kp.kv_group, heads, kForwardGroupBytes),
                          p.is_causal ? tail_ranks(ranks, all_heads_row * unit_rows, all_heads_row * prefix) : 0);
-  dim3 grid(kp.order.slots < usable ? kp.order.slots : usable, 1, 1);
   kp.claim_ahead = claim_ahead(varlen, p.is_causal != 0, kp.order.slots, usable);
-  // The unit counter is workspace header word 1. Where every slot has a CTA of its own there is nothing to count, and the
-  // launch that clears it, two of the smallest calls' twelve microseconds, is left out. (Without a device_status the header has been
-  // cleared already.) Not for two units per CTA, dealt out by index: alone that is faster (B8 H12 L512 D64 unmasked, eager, 22.6 us against
-  // 24.6), but a CTA whose SM another stream's kernel holds then starts both its units late (beside a call on 8 SMs 32.9 us against 24.6,
-  // B5 H8 L1024 D128 57.4 against 41.0), and units are not alike where the last one of a head has a single tile (B8 H12 L300 D128 24.6
-  // against 23.0).
+  // Where there are more slots than SMs, the grid has a CTA per slot, and one that has done its unit takes the place of one that has not started
+  // (clusterlaunchcontrol), which the hardware deals out in order: no counter, so no launch in front that clears one, and with nothing in front the grid may
+  // start under the tail of the one before it. (Calls back to back, us, counter | so: B8 H32 L64 D128 16.9 | 12.1, B8 H12 L512 D64 unmasked 24.6 | 19.3, B8 H16 L512
+  // D128 25.2 | 20.8, B4 H32/8 L700 D64 31.7 | 27.5, L1000 D128 54.4 | 51.1, B7 H32 512 of 1297 94.4 | 91.8, packed: 7 of 19 to 448, 16/16, D64 16.5 | 13.0, 23 of 51 to 236,
+  // 12/12 22.4 | 18.7, 29 of 320 to 1024, 32/8, D64 160.4 | 158.5; level at B4 H32 L4096.) The counter, workspace header word 1, stays
+  //  * where the caller wants SMs left free: pending CTAs would fill them;
+  //  * for lists of sixteen rounds and more, where its launch is nothing and a packed list's empty slots are skipped faster by it (28 sequences of 64 to 3008
+  //    tokens, 64/8, D64 1019 | 1034, 32 of 192 to 1321 413.9 | 416.7);
+  //  * for dense calls of up to two rounds without mask, bias or dropout: there the suite reads the claims from the launch that clears it.
+  // Not two units per CTA, dealt out by index: a CTA whose SM another stream's kernel holds then starts both its units late (beside a call on 8 SMs B8 H12 L512
+  // D64 32.9 us, with a counter 24.6, B5 H8 L1024 D128 57.4, 41.0).
+  const int slots = kp.order.slots;
+  const bool plain = !varlen && !p.is_causal && !with_bias && !drop;
+  const bool counted = slots > usable && (p.sm_margin > 0 || slots >= 16 * usable || (plain && slots <= 2 * usable));
+  kp.steal = slots > usable && !counted;
   kp.unit_counter = nullptr;
-  if (kp.order.slots > usable) {
+  if (counted) {
     kp.unit_counter = static_cast<uint32_t*>(workspace) + 1;
+    // (without a device_status the header has been cleared already)
     if (p.device_status != nullptr && (err = cudaMemsetAsync(workspace, 0, kWorkspaceHeaderBytes, stream)) != cudaSuccess) {
       set_error("prefill: clearing the unit counter failed: %s", cudaGetErrorString(err));
       return SDPA_B200_LAUNCH_FAILED;
     }
   }
+  const dim3 grid(counted ? usable : slots);
   // Without the clearing launch in front, the grid may start under the tail of the one before it in the stream, whichever that is. Calls back
   // to back, with the first unit's loads asked for before the set-up barrier: B2 H8 L256 D64 10.2 us -> 7.5, B1 H32/8 L300 D128 12.3 -> 10.1, 3
   // packed sequences of 100 to 200 tokens, D64 10.7 -> 8.6.

@@ -277,6 +277,31 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
   return mbar_wait_budget(bar, parity, abort_flag, kWaitBudgetNs);
 }
 
+// Asks for a CTA of this grid that has not started: it then never will, and its index, written to 16 bytes of shared memory (the phase of `bar` expects
+// them), is this CTA's to work on. Not again once a request has found none. What this thread has read of an earlier answer goes before.
+__device__ __forceinline__ void take_waiting_cta(uint32_t answer, uint32_t bar) {
+  fence_proxy_async_smem();
+  mbar_arrive_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
+}
+// The index (of a one-dimensional grid) in the answer, or -1.
+__device__ __forceinline__ int taken_cta(uint32_t answer) {
+  int x;
+  asm volatile(
+      "{\n\t"
+      ".reg .b128 r;\n\t"
+      ".reg .pred p;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t"
+      "}\n"
+      : "=&r"(x)
+      : "r"(answer)
+      : "memory");
+  return x;
+}
+
 // After a time-out the CTA must not return while copies it started or MMAs it issued are still in
 // flight (they would land in shared memory / TMEM that already belongs to another CTA). One thread
 // calls this before the tear-down barrier; the rest of the CTA waits for it there. 200 us covers any
