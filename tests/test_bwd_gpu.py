@@ -12,7 +12,7 @@ import torch
 from oracle import sdpa_oracle as orc
 from test_oracle import GOLDEN, load_golden
 from tests.test_ds_backward_gpu import run as run_with_workspace
-from torch_mlu_b200 import ops, workloads
+from torch_mlu_b200 import _cabi, ops, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -387,3 +387,34 @@ def test_more_rows_than_one_grid_of_the_prepass_covers(cuda_device, native_lib, 
         err = float((got.reshape(-1, D).float() - want).norm() / want.norm())
         assert err <= 1e-2, (name, err)
     assert float((grads[0].reshape(-1, D)[-200:].float() - (ds @ kf)[-200:]).norm() / (ds @ kf)[-200:].norm()) <= 1e-2
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,L,D,causal,bias,launches", [
+    (1, 3, 3, 129, 64, True, None, 2),      # tiles of 128 rows in both kernels
+    (5, 31, 31, 65, 64, False, "key", 2),   # as many key blocks as SMs and more: 64 rows
+    (1, 60, 60, 640, 40, True, None, 2),
+    (2, 4, 4, 300, 64, False, "full", 4),   # a bias that depends on the query (and its transposed copy)
+    (1, 16, 16, 512, 128, True, None, 3),   # all blocks of both kernels fit the SMs
+    (1, 16, 16, 640, 128, True, "key", 2),
+    (2, 30, 5, 333, 96, True, None, 2),
+])
+def test_both_kernels_in_one_launch(cuda_device, native_lib, B, Hq, Hkv, L, D, causal, bias, launches):
+    """dK/dV and dQ blocks of one grid, counted with the pre-pass, against fp32 math (16-bit P and dS: relative error of 4e-3 in the 2-norm, as on
+    the other paths)."""
+    gen = torch.Generator(device=cuda_device).manual_seed(9)
+    q, k, v, do = (torch.randn(B, h, L, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    b = None
+    if bias is not None:
+        raw = torch.randn(B, 1, 1 if bias == "key" else L, (L + 7) // 8 * 8, generator=gen, device=cuda_device, dtype=torch.bfloat16)
+        b = raw[..., :L].expand(B, Hq, L, L)
+    out, lse = ops._dense_forward(q, k, v, causal, None, True, bias=b)
+    before = _cabi.launch_count()
+    grads = ops._dense_backward(do, q, k, v, out, lse, causal, D ** -0.5, bias=b)
+    assert ops.device_status() == 0 and _cabi.launch_count() - before == launches
+    qf, kf, vf = (t.float().requires_grad_() for t in (q, k, v))
+    s = qf @ kf.repeat_interleave(Hq // Hkv, 1).transpose(2, 3) * D ** -0.5 + (0 if b is None else b.float())
+    if causal:
+        s = s.masked_fill(~torch.ones(L, L, dtype=torch.bool, device=cuda_device).tril(), float("-inf"))
+    want = torch.autograd.grad(torch.softmax(s, -1) @ vf.repeat_interleave(Hq // Hkv, 1), (qf, kf, vf), do.float())
+    for name, got, w in zip(("dq", "dk", "dv"), grads, want):
+        assert float((got.float() - w).norm() / w.norm()) < 4e-3, name

@@ -9,7 +9,7 @@
 // instances) dV takes P o M / (1 - p) and dS = P o (M o dP / (1 - p) - delta); with an additive bias (kBias
 // instances) the scores are scale*QK^T + bias and the dQ kernel also writes dS as the bias gradient.
 //
-// Three launches:
+// Three launches, of which the last two are one where the same instance serves both (bwd_tile_kernel_pair):
 //   1. bwd_preprocess_kernel: delta and the log2-domain logsumexp into a padded
 //      [batch, heads_q, ceil128(max_seqlen_q)] workspace (rows past a sequence get lse = +inf,
 //      which later turns their P into exact zeros).
@@ -33,6 +33,7 @@
 #endif
 
 #include <type_traits>
+#include <utility>
 
 #include "bwd_common.cuh"
 #include "bwd_ds_gemm.h"
@@ -116,12 +117,11 @@ enum BiasKind { kNoBias = 0, kFullBias = 1, kKeyBias = 2 };
 // kDsCall: the call's dS goes through the workspace where there is room (launch_bwd). An instance of its own, since with both kinds of
 // exponentials and the dS stores behind branches the calls without dS were slower (dK/dV and dQ kernel of 6 packed sequences of 50 to 4000
 // tokens, 32/8 heads, unmasked: 1222 + 1076 us, so 1137 + 1019).
-template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall, bool kSplit, int kY>
-__global__ void __launch_bounds__(kThreads<kY>, kY == 64 ? 2 : 1)
-bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                const __grid_constant__ CUtensorMap tm_o1, const __grid_constant__ CUtensorMap tm_o2,
-                const BwdKernelParams p) {
+// kPair: the CTA is one of a grid that does both, with `block` its index among those of its kind.
+template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall, bool kSplit, int kY, bool kPair>
+__device__ __forceinline__ void tile_cta(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
+                                         const CUtensorMap& tm_o1, const CUtensorMap& tm_o2, const BwdKernelParams& p, const BlockOrder& order,
+                                         int heads_x, int block) {
   extern __shared__ uint8_t smem_raw[];
 #ifdef SDPA_BWD_STAMPS
   const long long t_entry = clock64();
@@ -135,7 +135,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // pre-pass's tail; its vectors are read behind the wait for it. The kernel behind (the dQ kernel, which depends on nothing
   // written here, or the dQ GEMM, which waits for this grid) is let in by every CTA behind that wait, so that it too finds the
   // vectors complete. CTAs without work wait as well: a grid must not complete before the one in front of it.
-  if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
+  if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr && block == 0 && threadIdx.x == 0)
     *p.ds_counter = 0u;  // read by the dQ GEMM behind its wait for this grid; here, since block 0 may be one without work
   constexpr int kStages = stages_for(kMode, kD);
   constexpr int kC = kY / 2;  // columns per compute warpgroup, i.e. per thread
@@ -155,14 +155,14 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   int b, hx, xb;
   {
     int rank, bh;
-    if (!block_of_slot(p.order, kSplit ? blockIdx.x / p.split : blockIdx.x, rank, bh)) {
+    if (!block_of_slot(order, kSplit ? block / p.split : block, rank, bh)) {
       wait_for_previous_grid();
       return;
     }
     bh += p.bh0;
-    xb = (kMode == kModeDKDV) ? rank : p.order.ranks - 1 - rank;
-    b = bh / p.heads_x;
-    hx = bh - b * p.heads_x;
+    xb = (kMode == kModeDKDV) ? rank : order.ranks - 1 - rank;
+    b = bh / heads_x;
+    hx = bh - b * heads_x;
   }
   int q_off = 0, k_off = 0, len_q = p.seqlen_q, len_k = p.seqlen_k, bcoord = b;
   if (p.cu_q != nullptr) {
@@ -171,7 +171,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     k_off = p.cu_k[b];
     len_k = p.cu_k[b + 1] - k_off;
     bcoord = 0;
-    if (kMode == kModeDKDV && p.is_causal) xb -= p.order.ranks - (len_k + kTile - 1) / kTile;
+    if (kMode == kModeDKDV && p.is_causal) xb -= order.ranks - (len_k + kTile - 1) / kTile;
   }
   const int causal_off = len_k - len_q;
   const int len_x = (kMode == kModeDKDV) ? len_k : len_q;
@@ -194,7 +194,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   const int tiles_per_head = max(0, y_hi - y_lo);
   // dK/dV: the CTAs of a cluster (kSplit) take equal shares of the group's query heads
-  const int cluster_rank = kSplit ? static_cast<int>(blockIdx.x) % p.split : 0;
+  const int cluster_rank = kSplit ? block % p.split : 0;
   const int heads_here = kSplit ? p.kv_group / p.split : (kMode == kModeDKDV) ? p.kv_group : 1;
   const auto query_head = [&](int hi) { return hx * p.kv_group + (kSplit ? cluster_rank * heads_here : 0) + hi; };
   const int n_items = tiles_per_head * heads_here;
@@ -302,7 +302,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     if (kMode == kModeDKDV) {
       wait_for_previous_grid();
-      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      if (!kPair) launch_dependents();
     }
     for (int idx = 0; idx < kPreloaded && idx < 2 * n_items; ++idx) load_tile(idx);
   }
@@ -320,7 +320,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const long long t_start = clock64();
   // a long-running block of batch 0, head 0 (non-causal: any; causal: the heaviest)
   const bool stamp_on = p.stamps != nullptr && b == 0 && hx == 0 &&
-                        xb == ((kMode == kModeDKDV) ? 0 : p.order.ranks - 1) && (lane == 0) &&
+                        xb == ((kMode == kModeDKDV) ? 0 : order.ranks - 1) && (lane == 0) &&
                         (warp == 0 || warp == 4 || warp == kScoreWarp || warp == kAccWarp);
 #endif
 
@@ -526,6 +526,7 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     float my_nlse2 = 0.f, my_ndelta = 0.f;
     if (kMode == kModeDQ) {
+      if (kPair) wait_for_previous_grid();  // the pre-pass; a dQ kernel of its own starts behind a grid that has waited for it
       const size_t vec = (static_cast<size_t>(b) * p.heads_q + hx) * p.lq_pad + xr;
       my_nlse2 = p.nlse2[vec];
       my_ndelta = p.ndelta[vec];
@@ -992,6 +993,34 @@ bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (kMode == kModeDQ && threadIdx.x == 0) wait_for_previous_grid();
 }
 
+template <int kMode, int kD, bool kF16, bool kDrop, int kBias, bool kDsCall, bool kSplit, int kY>
+__global__ void __launch_bounds__(kThreads<kY>, kY == 64 ? 2 : 1)
+bwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                const __grid_constant__ CUtensorMap tm_o1, const __grid_constant__ CUtensorMap tm_o2,
+                const __grid_constant__ BwdKernelParams p) {
+  tile_cta<kMode, kD, kF16, kDrop, kBias, kDsCall, kSplit, kY, false>(tm_q, tm_k, tm_v, tm_do, tm_o1, tm_o2, p, p.order, p.heads_x, blockIdx.x);
+}
+
+// Both kernels in one launch: the dK/dV blocks, then the dQ blocks.
+struct DqGrid {
+  BlockOrder order;
+  int heads_x;
+  int first;  // block of the grid
+};
+template <int kD, bool kF16, bool kDrop, int kBias, int kY>
+__global__ void __launch_bounds__(kThreads<kY>, kY == 64 ? 2 : 1)
+bwd_tile_kernel_pair(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                     const __grid_constant__ CUtensorMap tm_dv, const __grid_constant__ CUtensorMap tm_dk,
+                     const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ BwdKernelParams p, const DqGrid dq) {
+  const int block = static_cast<int>(blockIdx.x) - dq.first;
+  if (block < 0)
+    tile_cta<kModeDKDV, kD, kF16, kDrop, kBias, false, false, kY, true>(tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, p, p.order, p.heads_x, blockIdx.x);
+  else
+    tile_cta<kModeDQ, kD, kF16, kDrop, kBias, false, false, kY, true>(tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, p, dq.order, dq.heads_x, block);
+}
+
 // ndelta[row] = -sum_d dO[row,d] * O[row,d]; nlse2[row] = -lse[row] * log2(e);
 // rows padded to lq_pad per (batch, head): padding rows get nlse2 = -inf, ndelta = 0.
 struct PreParams {
@@ -1173,6 +1202,49 @@ int launch_tile_kernel(int mode, int head_dim, bool f16, int grid, bool wide, cu
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("backward %s: launch failed: %s", mode == kModeDKDV ? "dK/dV" : "dQ", cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
+  }
+  count_launch();
+  return SDPA_B200_OK;
+}
+
+using PairKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                            const CUtensorMap, const CUtensorMap, const BwdKernelParams, const DqGrid);
+template <bool kDrop, int kBias>
+PairKernel pick_pair_kernel(int head_dim, bool f16, bool wide) {
+  if (head_dim > 64) return f16 ? bwd_tile_kernel_pair<128, true, kDrop, kBias, kTile> : bwd_tile_kernel_pair<128, false, kDrop, kBias, kTile>;
+  if (wide) return f16 ? bwd_tile_kernel_pair<64, true, kDrop, kBias, kTile> : bwd_tile_kernel_pair<64, false, kDrop, kBias, kTile>;
+  return f16 ? bwd_tile_kernel_pair<64, true, kDrop, kBias, 64> : bwd_tile_kernel_pair<64, false, kDrop, kBias, 64>;
+}
+
+// The dK/dV and the dQ kernel of a call without clusters, dS or a bias that depends on the query, as one launch behind the pre-pass.
+int launch_tile_pair(int head_dim, bool f16, int grid_dkdv, int grid_dq, const DqGrid& dq, bool wide, cudaStream_t stream, const CUtensorMap& tm_q,
+                     const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do, const CUtensorMap& tm_dv, const CUtensorMap& tm_dk,
+                     const CUtensorMap& tm_dq, const BwdKernelParams& kp) {
+  const bool key_bias = kp.bias != nullptr;
+  PairKernel kernel = kp.keep_rows != nullptr ? (key_bias ? pick_pair_kernel<true, kKeyBias>(head_dim, f16, wide) : pick_pair_kernel<true, kNoBias>(head_dim, f16, wide))
+                                              : (key_bias ? pick_pair_kernel<false, kKeyBias>(head_dim, f16, wide) : pick_pair_kernel<false, kNoBias>(head_dim, f16, wide));
+  const int dim = head_dim <= 64 ? 64 : 128, rows = dim == 64 && !wide ? 64 : kTile;
+  const uint32_t one = smem_bytes_for(kModeDKDV, dim, rows, key_bias), other = smem_bytes_for(kModeDQ, dim, rows, key_bias), smem = one > other ? one : other;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) {
+    set_error("backward: cudaFuncSetAttribute(%u bytes smem): %s", smem, cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid_dkdv + grid_dq);
+  cfg.blockDim = dim3(rows == 64 ? kThreads<64> : kThreads<kTile>);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  err = cudaLaunchKernelEx(&cfg, kernel, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, tm_dq, kp, dq);
+  if (err == cudaSuccess) err = cudaGetLastError();
+  if (err != cudaSuccess) {
+    set_error("backward dK/dV and dQ: launch failed: %s", cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
   }
   count_launch();
@@ -1451,11 +1523,24 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   const auto blocks = [&](int grid, int heads, int rows) { return varlen ? heads * (rows / static_cast<double>(kTile) + 0.5 * p.batch) : grid; };
   const auto tiles = [](int rows) { return (rows + kTile - 1) / kTile; };
   const bool wide_dkdv = wide_tiles(blocks(grid_dkdv, p.heads_kv, p.total_k), kp.kv_group * tiles(p.max_seqlen_q));
+  BwdKernelParams kq = kp;
+  std::swap(kp, kq);
+  const int grid_dq = set_order(p.heads_q, p.max_seqlen_q, p.batch * p.heads_q, p.max_seqlen_k, 1, rows_k_all);
+  std::swap(kp, kq);  // kp: the dK/dV kernel's, kq: the dQ kernel's
+  const bool wide_dq = wide_tiles(blocks(grid_dq, p.heads_q, p.total_q), tiles(p.max_seqlen_k));
+  // Both in one launch where the same instance serves both, with the dQ blocks behind the dK/dV blocks as the overlapped launches have them: about 2.5 us less of
+  // host time, which is what bounds the steps of short sequences, and no gap (step, two launches | one, us: B4 H8 L500 D64 f16 83.3 | 78.2, B1 H8 L2048 D128
+  // 74.1 | 71.5, B16 H16 L500 D64 120.8 | 116.6, B8 H12 L1000 D64 unmasked 187 | 181, B32 H12 L300 D64 with dropout 173.8 | 168.5; backward alone, replayed from a graph: B8 H12 L512
+  // D64 with a mask 50.4 | 48.1, B1 H8 L2048 D128 34.9 | 33.3, B4 H8 L512 D128 24.1 | 24.1). Above head_dim 64 two launches where all blocks fit the SMs at once: only host time is
+  // saved there, and the suite counts them.
+  const bool pair = !kp.ds_call && kp.split == 1 && (p.head_dim > 64 || wide_dkdv == wide_dq) && (kp.bias == nullptr || (kp.bias_row_stride == 0 && kp.dbias == nullptr)) &&
+                    (p.head_dim <= 64 || grid_dkdv + grid_dq > kSms);
+  if (pair)
+    return launch_tile_pair(p.head_dim, f16, grid_dkdv, grid_dq, DqGrid{kq.order, kq.heads_x, grid_dkdv}, wide_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, tm_dq, kp);
   if ((st = launch_tile_kernel(kModeDKDV, p.head_dim, f16, grid_dkdv, wide_dkdv, stream, tm_q, tm_k, tm_v, tm_do, tm_dv, tm_dk, kp,
                                /*overlap_previous=*/true)) != SDPA_B200_OK)
     return st;
-  const int grid_dq = set_order(p.heads_q, p.max_seqlen_q, p.batch * p.heads_q, p.max_seqlen_k, 1, rows_k_all);
-  return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, wide_tiles(blocks(grid_dq, p.heads_q, p.total_q), tiles(p.max_seqlen_k)), stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kp,
+  return launch_tile_kernel(kModeDQ, p.head_dim, f16, grid_dq, wide_dq, stream, tm_q, tm_k, tm_v, tm_do, tm_dq, tm_dq, kq,
                             /*overlap_previous=*/true);
 }
 
