@@ -270,6 +270,19 @@ SDPA_B200_API int sdpa_b200_mask_to_bias(const void* mask, int64_t batch_stride,
                                          int64_t key_stride, int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k,
                                          void* out, int64_t out_row_stride, int32_t dtype, void* stream);
 
+/* Copies a bias of 16-bit elements (element strides, 0 for a broadcast dimension, any key stride) into rows that sdpa_b200_params.bias can be read
+ * from: out is [batch][heads][seqlen_q][out_row_stride], contiguous, out_row_stride a multiple of 8 that holds seqlen_k; the padding is zero-filled. */
+SDPA_B200_API int sdpa_b200_pad_bias(const void* bias, int64_t batch_stride, int64_t head_stride, int64_t row_stride,
+                                     int64_t key_stride, int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k,
+                                     void* out, int64_t out_row_stride, void* stream);
+
+/* Sums a bias gradient (sdpa_b200_params.dbias: 16-byte aligned, strides that are multiples of 8, unit key stride, rows readable to the next multiple
+ * of 8 keys) over the batches and / or the heads that the bias is broadcast along, in fp32. out is [batch or 1][heads or 1][seqlen_q][seqlen_k],
+ * contiguous, of `dtype`. */
+SDPA_B200_API int sdpa_b200_sum_bias_grad(const void* grad, int64_t batch_stride, int64_t head_stride, int64_t row_stride,
+                                          int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t over_batch,
+                                          int32_t over_heads, void* out, int32_t dtype, void* stream);
+
 /* How many of this library's kernels the calling process has launched so far. */
 SDPA_B200_API uint64_t sdpa_b200_launch_count(void);
 

@@ -397,3 +397,28 @@ def test_bias_goes_through_saved_tensor_hooks(cuda_device, native_lib, Lk, boole
         assert any(s[:3] == (2, 1, 96) for s in packed), packed
         for a, b in zip(*grads):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("B,H,L,shape,dtype", [
+    (3, 2, 67, (1, 2, 67, 67), torch.bfloat16),     # summed over batches, odd rows
+    (9, 3, 64, (9, 1, 64, 64), torch.float16),      # over heads; rows as they are
+    (5, 4, 130, (130, 130), torch.bfloat16),        # over both: 20 gradients per element, no multiple of eight
+    (2, 3, 33, (3, 33, 33), torch.float16),
+    (2, 2, 70, (2, 2, 1, 70), torch.bfloat16),      # also over the queries: not by this kernel
+    (1, 2, 71, (1, 2, 71, 71), torch.bfloat16),     # nothing to sum
+])
+def test_gradient_of_a_broadcast_bias(cuda_device, native_lib, B, H, L, shape, dtype):
+    """The padded copy and the summed gradient, through the package's entry point, against fp32 math. The gradient is a sum of 16-bit dS (relative error
+    2^-9 or 2^-12 each, their sum rounded once more): 1e-2 in the 2-norm as in the other gradient tests."""
+    gen = torch.Generator(device=cuda_device).manual_seed(12)
+    q, k, v, do = (torch.randn(B, H, L, 64, generator=gen, device=cuda_device, dtype=dtype) for _ in range(4))
+    wide = torch.randn(*shape[:-1], shape[-1] + 3, generator=gen, device=cuda_device, dtype=dtype)
+    bias = wide[..., 1:1 + shape[-1]].detach().requires_grad_()  # rows that begin at odd addresses
+    q, k, v = (t.requires_grad_() for t in (q, k, v))
+    out = sdp_choice.scaled_dot_product_attention(q, k, v, attn_mask=bias)
+    got = torch.autograd.grad(out, (q, k, v, bias), do)
+    f = [t.detach().float().requires_grad_() for t in (q, k, v, bias)]
+    ref = torch.softmax(f[0] @ f[1].transpose(2, 3) * 64 ** -0.5 + f[3], -1) @ f[2]
+    for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, torch.autograd.grad(ref, f, do.float())):
+        assert g.shape == w.shape and float((g.float() - w).norm() / w.norm()) < 1e-2, name
+    assert float((out.float() - ref).norm() / ref.norm()) < 1e-2

@@ -34,6 +34,8 @@ EXPORTED_SYMBOLS = (
     "sdpa_b200_dropout_keep_mask_varlen",
     "sdpa_b200_transpose_bias",
     "sdpa_b200_mask_to_bias",
+    "sdpa_b200_pad_bias",
+    "sdpa_b200_sum_bias_grad",
     "sdpa_b200_launch_count",
 )
 STATIC_SCRATCH_BYTES = 16 << 20
@@ -123,6 +125,12 @@ def load() -> ctypes.CDLL:
     lib.sdpa_b200_mask_to_bias.restype = c_int
     lib.sdpa_b200_mask_to_bias.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32, c_void_p,
                                            c_int64, c_int32, c_void_p]
+    lib.sdpa_b200_pad_bias.restype = c_int
+    lib.sdpa_b200_pad_bias.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32, c_void_p, c_int64,
+                                       c_void_p]
+    lib.sdpa_b200_sum_bias_grad.restype = c_int
+    lib.sdpa_b200_sum_bias_grad.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p,
+                                            c_int32, c_void_p]
     _lib = lib
     return lib
 

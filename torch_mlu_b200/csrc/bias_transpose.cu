@@ -1,10 +1,12 @@
-// Preparation of attention biases: a boolean mask as a bias (mask_to_bias_kernel), and the transposed copy for the backward
+// Preparation of attention biases: a boolean mask as a bias (mask_to_bias_kernel), a bias with rows of a multiple of 8 keys
+// (bias_pad_kernel), its gradient summed over what it is broadcast along (bias_grad_sum_kernel), and the transposed copy for the backward
 // pass: [.., Lq, Lk] -> [.., Lk, ld >= Lq].
 //
 // The dK/dV kernel's threads own keys and walk over queries, so it reads a bias stored query-major two bytes
 // at a time; with this copy (sdpa_b200_params.bias_t) it reads 16 bytes at a time. HBM-bound: every element is
 // read once and written once through a 64 x 64 shared-memory tile, 16 bytes per thread on both sides.
 #include "kernels.h"
+#include "ptx_sm100.cuh"
 
 namespace sdpa_b200 {
 namespace {
@@ -81,6 +83,75 @@ __global__ void __launch_bounds__(256) mask_to_bias_kernel(const MaskParams p, i
     w[j] = x;
   }
   p.out[i] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The same for a bias in its own type, whose rows the attention kernels cannot read where they lie: bound by memory, one launch where filling and copying took
+// two and wrote the copy twice (12 heads of 594 x 594 20 + 12 us -> 4).
+struct PadParams {
+  const uint16_t* bias;
+  uint4* out;
+  int64_t batch_stride, head_stride, row_stride, key_stride;
+  int heads, seqlen_q, seqlen_k, groups;
+};
+__global__ void __launch_bounds__(256) bias_pad_kernel(const PadParams p, int64_t total) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const int64_t row = i / p.groups;
+  const int k0 = static_cast<int>(i - row * p.groups) * 8;
+  const int64_t bh = row / p.seqlen_q;
+  const int64_t b = bh / p.heads;
+  const uint16_t* src = p.bias + b * p.batch_stride + (bh - b * p.heads) * p.head_stride + (row - bh * p.seqlen_q) * p.row_stride;
+  uint32_t v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = k0 + j < p.seqlen_k ? src[(k0 + j) * p.key_stride] : 0u;
+  p.out[i] = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+}
+
+// Sums a [batch, heads, seqlen_q, seqlen_k] gradient over batches and / or heads, eight keys per thread, fp32, in the order of the indexes. Bound by memory: a
+// thread's reads do not depend on one another, eight are in flight (16 batches of 12 heads of 594 x 594 135 MB in 27 us; the tensor library's sum 52).
+struct GradSumParams {
+  const uint16_t* grad;
+  uint16_t* out;  // contiguous
+  int64_t batch_stride, head_stride, row_stride;
+  int out_heads, sum_batches, sum_heads;  // heads of the result; batches and heads per element of it
+  int seqlen_q, seqlen_k, groups;
+};
+template <bool kF16>
+__global__ void __launch_bounds__(256) bias_grad_sum_kernel(const GradSumParams p, int64_t total) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const int64_t row = i / p.groups;
+  const int k0 = static_cast<int>(i - row * p.groups) * 8;
+  const int64_t bh = row / p.seqlen_q;
+  const int64_t b = bh / p.out_heads;
+  const uint16_t* src = p.grad + b * p.batch_stride + (bh - b * p.out_heads) * p.head_stride + (row - bh * p.seqlen_q) * p.row_stride + k0;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  const int n = p.sum_batches * p.sum_heads;
+  for (int first = 0; first < n; first += 8) {
+    uint4 w[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int at = min(first + u, n - 1), sb = at / p.sum_heads;
+      w[u] = __ldcs(reinterpret_cast<const uint4*>(src + sb * p.batch_stride + (at - sb * p.sum_heads) * p.head_stride));
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (first + u >= n) break;
+      const uint32_t ww[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 x = unpack_16x2<kF16>(ww[j]);
+        acc[2 * j] += x.x;
+        acc[2 * j + 1] += x.y;
+      }
+    }
+  }
+  uint16_t* dst = p.out + row * p.seqlen_k + k0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (k0 + j < p.seqlen_k) dst[j] = to_16<kF16>(acc[j]);
 }
 
 }  // namespace
@@ -161,6 +232,81 @@ extern "C" SDPA_B200_API int sdpa_b200_transpose_bias(const void* bias, int64_t 
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("transpose_bias: launch failed: %s", cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
+  }
+  count_launch();
+  return SDPA_B200_OK;
+}
+
+extern "C" SDPA_B200_API int sdpa_b200_pad_bias(const void* bias, int64_t batch_stride, int64_t head_stride, int64_t row_stride, int64_t key_stride,
+                                                int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, void* out,
+                                                int64_t out_row_stride, void* stream) {
+  if (bias == nullptr || out == nullptr || (reinterpret_cast<uintptr_t>(bias) & 1u) || (reinterpret_cast<uintptr_t>(out) & 15u) || batch <= 0 ||
+      heads <= 0 || seqlen_q <= 0 || seqlen_k <= 0 || batch_stride < 0 || head_stride < 0 || row_stride < 0 || key_stride < 0 ||
+      (out_row_stride % 8) != 0 || out_row_stride < seqlen_k) {
+    set_error("pad_bias: non-NULL pointers, a 16-byte aligned output, positive sizes, strides that are not negative and an output row stride that is a "
+              "multiple of 8 and holds seqlen_k");
+    return SDPA_B200_INVALID_ARG;
+  }
+  PadParams m;
+  m.bias = static_cast<const uint16_t*>(bias);
+  m.out = static_cast<uint4*>(out);
+  m.batch_stride = batch_stride;
+  m.head_stride = head_stride;
+  m.row_stride = row_stride;
+  m.key_stride = key_stride;
+  m.heads = heads;
+  m.seqlen_q = seqlen_q;
+  m.seqlen_k = seqlen_k;
+  m.groups = static_cast<int>(out_row_stride / 8);
+  const int64_t total = static_cast<int64_t>(batch) * heads * seqlen_q * m.groups, blocks = (total + 255) / 256;
+  if (blocks > 0x7fffffff) {
+    set_error("pad_bias: too many elements");
+    return SDPA_B200_INVALID_ARG;
+  }
+  bias_pad_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(m, total);
+  const cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) {
+    set_error("pad_bias: launch failed: %s", cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
+  }
+  count_launch();
+  return SDPA_B200_OK;
+}
+
+extern "C" SDPA_B200_API int sdpa_b200_sum_bias_grad(const void* grad, int64_t batch_stride, int64_t head_stride, int64_t row_stride, int32_t batch,
+                                                     int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t over_batch, int32_t over_heads,
+                                                     void* out, int32_t dtype, void* stream) {
+  auto bad = [](int64_t s) { return s < 0 || (s % 8) != 0; };
+  if (grad == nullptr || out == nullptr || (reinterpret_cast<uintptr_t>(grad) & 15u) || (reinterpret_cast<uintptr_t>(out) & 1u) || batch <= 0 ||
+      heads <= 0 || seqlen_q <= 0 || seqlen_k <= 0 || bad(batch_stride) || bad(head_stride) || bad(row_stride) || row_stride < seqlen_k ||
+      (dtype != SDPA_B200_BF16 && dtype != SDPA_B200_F16)) {
+    set_error("sum_bias_grad: non-NULL pointers, a 16-byte aligned gradient, positive sizes and strides that are multiples of 8, with rows that are readable "
+              "to the next multiple of 8 keys");
+    return SDPA_B200_INVALID_ARG;
+  }
+  GradSumParams m;
+  m.grad = static_cast<const uint16_t*>(grad);
+  m.out = static_cast<uint16_t*>(out);
+  m.batch_stride = batch_stride;
+  m.head_stride = head_stride;
+  m.row_stride = row_stride;
+  m.out_heads = over_heads ? 1 : heads;
+  m.sum_batches = over_batch ? batch : 1;
+  m.sum_heads = over_heads ? heads : 1;
+  m.seqlen_q = seqlen_q;
+  m.seqlen_k = seqlen_k;
+  m.groups = (seqlen_k + 7) / 8;
+  const int64_t total = static_cast<int64_t>(over_batch ? 1 : batch) * m.out_heads * seqlen_q * m.groups, blocks = (total + 255) / 256;
+  if (blocks > 0x7fffffff) {
+    set_error("sum_bias_grad: too many elements");
+    return SDPA_B200_INVALID_ARG;
+  }
+  auto kernel = dtype == SDPA_B200_F16 ? bias_grad_sum_kernel<true> : bias_grad_sum_kernel<false>;
+  kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(m, total);
+  const cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) {
+    set_error("sum_bias_grad: launch failed: %s", cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
   }
   count_launch();

@@ -47,15 +47,39 @@ bool dispatcher_may_be_skipped() {
 // ------------------------------------------------------------------------- additive bias
 int64_t ceil8(int64_t n) { return (n + 7) / 8 * 8; }
 
-// A copy of the bias with rows padded to a multiple of 8 keys.
+// A copy of the bias (of q's type and device) with rows padded to a multiple of 8 keys.
 Tensor padded_copy(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k) {
   std::vector<int64_t> sizes(attn_bias.sizes().begin(), attn_bias.sizes().end());
-  sizes.back() = seqlen_k;
-  const Tensor src = attn_bias.expand(sizes);
   sizes.back() = ceil8(seqlen_k);
-  Tensor buf = at::zeros(sizes, q.options());
-  buf.narrow(-1, 0, seqlen_k).copy_(src);
+  int64_t own[4] = {1, 1, 1, seqlen_k}, strides[4] = {0, 0, 0, attn_bias.size(-1) == 1 ? 0 : attn_bias.stride(-1)};
+  const int64_t d = attn_bias.dim();
+  for (int64_t i = 4 - d, j = 0; i < 3; ++i, ++j) {
+    own[i] = attn_bias.size(j);
+    strides[i] = attn_bias.stride(j);
+  }
+  Tensor buf = at::detail::empty_cuda(sizes, q.scalar_type(), q.device(), c10::nullopt);
+  check_status(sdpa_b200_pad_bias(attn_bias.data_ptr(), strides[0], strides[1], strides[2], strides[3], static_cast<int32_t>(own[0]),
+                                  static_cast<int32_t>(own[1]), static_cast<int32_t>(own[2]), static_cast<int32_t>(seqlen_k), buf.data_ptr(),
+                                  sizes.back(), at::cuda::getCurrentCUDAStream(q.get_device()).stream()),
+               "sdpa_b200_pad_bias");
   return buf;
+}
+
+// The gradient of a bias of shape `sizes` out of that of its expansion: summed over what it is broadcast along.
+Tensor summed_bias_gradient(const Tensor& dbias, const std::vector<int64_t>& sizes) {
+  const int64_t d = static_cast<int64_t>(sizes.size());
+  int64_t own[4] = {1, 1, 1, 1};
+  for (int64_t i = 4 - d, j = 0; j < d; ++i, ++j) own[i] = sizes[j];
+  const bool over_batch = own[0] != dbias.size(0), over_heads = own[1] != dbias.size(1);
+  if (!(over_batch || over_heads) || own[2] != dbias.size(2) || own[3] != dbias.size(3)) return at::sum_to(dbias, sizes);
+  c10::cuda::CUDAGuard device_guard(dbias.device());
+  Tensor sum = at::detail::empty_cuda(sizes, dbias.scalar_type(), dbias.device(), c10::nullopt);
+  check_status(sdpa_b200_sum_bias_grad(dbias.data_ptr(), dbias.stride(0), dbias.stride(1), dbias.stride(2), static_cast<int32_t>(dbias.size(0)),
+                                       static_cast<int32_t>(dbias.size(1)), static_cast<int32_t>(dbias.size(2)), static_cast<int32_t>(dbias.size(3)),
+                                       over_batch, over_heads, sum.data_ptr(), dbias.scalar_type() == at::kHalf ? SDPA_B200_F16 : SDPA_B200_BF16,
+                                       at::cuda::getCurrentCUDAStream(dbias.get_device()).stream()),
+               "sdpa_b200_sum_bias_grad");
+  return sum;
 }
 
 // The additive bias as a [B, H, Lq, Lk] view the kernels can read: broadcast dimensions keep stride 0, rows start 16-byte
@@ -122,8 +146,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> bias_backward(const Tensor& grad_out,
   c10::cuda::CUDAGuard device_guard(q.device());
   const Tensor view = prepare_bias(bias, q, k.size(2), bias_padded);
   Tensor dbias;
-  if (want_dbias)  // zero-filled: the kernels skip what the causal mask hides
-    dbias = at::zeros({q.size(0), q.size(1), q.size(2), ceil8(k.size(2))}, q.options()).narrow(-1, 0, k.size(2));
+  if (want_dbias) {
+    const int64_t sizes[4] = {q.size(0), q.size(1), q.size(2), ceil8(k.size(2))};
+    // under a causal mask zero-filled, since the kernels skip what it hides; else they write every pair
+    dbias = (causal ? at::zeros(sizes, q.options()) : at::empty(sizes, q.options())).narrow(-1, 0, k.size(2));
+  }
   const Tensor bias_t = transposed_bias(view);
   BackwardOptions opt;
   opt.bias = &view;
@@ -175,11 +202,12 @@ variable_list run_backward(const Tensor& go, const BackwardCall& c, const Backwa
     if (direct && plain(t.bias)) {
       at::AutoDispatchBelowADInplaceOrView guard;
       std::tie(dq, dk, dv, dbias) = bias_backward(go, t.q, t.k, t.v, t.bias, t.out, t.lse, c.bias_padded, c.causal, c.want_dbias, c.scale);
+      if (c.want_dbias) result[3] = summed_bias_gradient(dbias, c.bias_sizes);
     } else {
       static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("b200_sdpa::_bias_attention_backward", "").typed<decltype(bias_backward)>();
       std::tie(dq, dk, dv, dbias) = op.call(go, t.q, t.k, t.v, t.bias, t.out, t.lse, c.bias_padded, c.causal, c.want_dbias, c.scale);
     }
-    if (c.want_dbias) result[3] = at::sum_to(dbias, c.bias_sizes);
+    if (c.want_dbias && !result[3].defined()) result[3] = at::sum_to(dbias, c.bias_sizes);
   } else if (!direct) {
     if (c.packed) {
       static auto op = c10::Dispatcher::singleton()
