@@ -1061,7 +1061,6 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   // heads vary fastest across the grid: with the usual [batch, row, head, dim] memory order the blocks
   // that run together then read neighbouring 256-byte pieces of the same rows
   const int h = blockIdx.x, b = blockIdx.z;
-  const int row0 = (p.block0 + blockIdx.y) * kRows;
   const int col = threadIdx.x % kThreadsPerRow * 8;
   const int r_in_pass = threadIdx.x / kThreadsPerRow;
   int q_off = 0, len_q = p.seqlen_q;
@@ -1069,59 +1068,66 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
     q_off = p.cu_q[b];
     len_q = p.cu_q[b + 1] - q_off;
   }
-  if (kPacked && p.ds_seq_base != nullptr && h == 0 && row0 == 0) {
+  if (kPacked && p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0 && p.block0 == 0) {
     write_seq_base(p.ds_seq_base, p.cu_q, p.cu_k, b, p.is_causal != 0);
   }
-  uint4 ov[2], dv[2];
+  // Packed: as many blocks per sequence as one of the mean length has, which go on where there are more rows, up to the last row that a tile of the kernels
+  // behind has; with blocks for the longest one in all of them half were empty (12 sequences of 64 to 2048 tokens, 16 heads, D128 25.0 us, so 18.5; 20 of 100 to 3000, D64 with the accumulator 44.7, 39.1).
+  const int rows = kPacked ? min((len_q + kTile - 1) / kTile * kTile, p.lq_pad) : p.lq_pad;
+  for (int row0 = (p.block0 + blockIdx.y) * kRows; row0 < rows; row0 += gridDim.y * kRows) {
+    uint4 ov[2], dv[2];
 #pragma unroll
-  for (int ps = 0; ps < 2; ++ps) {
-    ov[ps] = make_uint4(0u, 0u, 0u, 0u);
-    dv[ps] = make_uint4(0u, 0u, 0u, 0u);
-    const int row = row0 + ps * kPerPass + r_in_pass;
-    if (row < len_q && col < p.head_dim) {
-      const int64_t at = (kPacked ? q_off : 0) + static_cast<int64_t>(row);
-      const uint16_t* o = p.out + (kPacked ? 0 : b * p.o_batch_stride) + h * p.o_head_stride + at * p.o_row_stride + col;
-      const uint16_t* dout = p.dout + (kPacked ? 0 : b * p.do_batch_stride) + h * p.do_head_stride + at * p.do_row_stride + col;
-      ov[ps] = __ldcs(reinterpret_cast<const uint4*>(o));  // not read again, unlike dO
-      dv[ps] = *reinterpret_cast<const uint4*>(dout);
+    for (int ps = 0; ps < 2; ++ps) {
+      ov[ps] = make_uint4(0u, 0u, 0u, 0u);
+      dv[ps] = make_uint4(0u, 0u, 0u, 0u);
+      const int row = row0 + ps * kPerPass + r_in_pass;
+      if (row < len_q && col < p.head_dim) {
+        const int64_t at = (kPacked ? q_off : 0) + static_cast<int64_t>(row);
+        const uint16_t* o = p.out + (kPacked ? 0 : b * p.o_batch_stride) + h * p.o_head_stride + at * p.o_row_stride + col;
+        const uint16_t* dout = p.dout + (kPacked ? 0 : b * p.do_batch_stride) + h * p.do_head_stride + at * p.do_row_stride + col;
+        ov[ps] = __ldcs(reinterpret_cast<const uint4*>(o));  // not read again, unlike dO
+        dv[ps] = *reinterpret_cast<const uint4*>(dout);
+      }
     }
-  }
-  const int my_row = row0 + threadIdx.x;  // of the first kRows threads: the row whose values they write
-  const bool have = threadIdx.x < kRows && my_row < len_q;
-  float lse = 0.f;
-  if (have)
-    lse = kPacked ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + my_row]
-                  : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + my_row];
-  if (kD == 64 && p.dq_acc != nullptr) {
-    // 64 rows of an accumulator tile: per 4-column group 1 KB of consecutive floats, a thread per row. The stores need no
-    // registers and go out under the loads above
-    constexpr int groups = 16;
-    const int row = row0 + (threadIdx.x & (kRows - 1));
-    if (row < len_q) {
-      const size_t acc_row = kPacked ? static_cast<size_t>(h) * p.dq_acc_rows + q_off + row
-                                               : (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
-      float4* dst = reinterpret_cast<float4*>(p.dq_acc + (acc_row >> 7) * (static_cast<size_t>(groups) * 512)) + (acc_row & 127);
-      for (int g = threadIdx.x / kRows; g < groups; g += 256 / kRows) dst[g * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int my_row = row0 + threadIdx.x;  // of the first kRows threads: the row whose values they write
+    const bool have = threadIdx.x < kRows && my_row < len_q;
+    float lse = 0.f;
+    if (have)
+      lse = kPacked ? p.lse[static_cast<size_t>(h) * p.total_q + q_off + my_row]
+                    : p.lse[(static_cast<size_t>(b) * p.heads_q + h) * p.seqlen_q + my_row];
+    if (kD == 64 && p.dq_acc != nullptr) {
+      // 64 rows of an accumulator tile: per 4-column group 1 KB of consecutive floats, a thread per row. The stores need no
+      // registers and go out under the loads above
+      constexpr int groups = 16;
+      const int row = row0 + (threadIdx.x & (kRows - 1));
+      if (row < len_q) {
+        const size_t acc_row = kPacked ? static_cast<size_t>(h) * p.dq_acc_rows + q_off + row
+                                                 : (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + row;
+        float4* dst = reinterpret_cast<float4*>(p.dq_acc + (acc_row >> 7) * (static_cast<size_t>(groups) * 512)) + (acc_row & 127);
+        for (int g = threadIdx.x / kRows; g < groups; g += 256 / kRows) dst[g * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
     }
-  }
 #pragma unroll
-  for (int ps = 0; ps < 2; ++ps) {
-    const float2 o0 = unpack_16x2<kF16>(ov[ps].x), o1 = unpack_16x2<kF16>(ov[ps].y);
-    const float2 o2 = unpack_16x2<kF16>(ov[ps].z), o3 = unpack_16x2<kF16>(ov[ps].w);
-    const float2 d0 = unpack_16x2<kF16>(dv[ps].x), d1 = unpack_16x2<kF16>(dv[ps].y);
-    const float2 d2 = unpack_16x2<kF16>(dv[ps].z), d3 = unpack_16x2<kF16>(dv[ps].w);
-    float acc = (o0.x * d0.x + o0.y * d0.y) + (o1.x * d1.x + o1.y * d1.y) + (o2.x * d2.x + o2.y * d2.y) +
-                (o3.x * d3.x + o3.y * d3.y);
-    // the threads of a row are consecutive lanes of one warp
+    for (int ps = 0; ps < 2; ++ps) {
+      const float2 o0 = unpack_16x2<kF16>(ov[ps].x), o1 = unpack_16x2<kF16>(ov[ps].y);
+      const float2 o2 = unpack_16x2<kF16>(ov[ps].z), o3 = unpack_16x2<kF16>(ov[ps].w);
+      const float2 d0 = unpack_16x2<kF16>(dv[ps].x), d1 = unpack_16x2<kF16>(dv[ps].y);
+      const float2 d2 = unpack_16x2<kF16>(dv[ps].z), d3 = unpack_16x2<kF16>(dv[ps].w);
+      float acc = (o0.x * d0.x + o0.y * d0.y) + (o1.x * d1.x + o1.y * d1.y) + (o2.x * d2.x + o2.y * d2.y) +
+                  (o3.x * d3.x + o3.y * d3.y);
+      // the threads of a row are consecutive lanes of one warp
 #pragma unroll
-    for (int off = kThreadsPerRow >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (col == 0) sums[ps * kPerPass + r_in_pass] = acc;
-  }
-  __syncthreads();
-  if (threadIdx.x < kRows && my_row < p.lq_pad) {
-    const size_t dst = (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + my_row;
-    p.nlse2[dst] = have ? lse * -1.4426950408889634f : -INFINITY;
-    p.ndelta[dst] = have ? -sums[threadIdx.x] : 0.f;
+      for (int off = kThreadsPerRow >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      if (col == 0) sums[ps * kPerPass + r_in_pass] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x < kRows && my_row < p.lq_pad) {
+      const size_t dst = (static_cast<size_t>(b) * p.heads_q + h) * p.lq_pad + my_row;
+      p.nlse2[dst] = have ? lse * -1.4426950408889634f : -INFINITY;
+      p.ndelta[dst] = have ? -sums[threadIdx.x] : 0.f;
+    }
+    if (!kPacked) break;
+    __syncthreads();  // the sums have been read
   }
 }
 
@@ -1385,7 +1391,13 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
                   : (f16 ? bwd_preprocess_kernel<kD, true, false> : bwd_preprocess_kernel<kD, false, false>);
   };
   auto pre_kernel = p.head_dim <= 64 ? pick_pre(std::integral_constant<int, 64>{}) : pick_pre(std::integral_constant<int, 128>{});
-  const int pre_blocks = lq_pad / (p.head_dim <= 64 ? kPreRows<64> : kPreRows<128>);
+  const int pre_rows = p.head_dim <= 64 ? kPreRows<64> : kPreRows<128>;
+  int pre_blocks = lq_pad / pre_rows;
+  if (varlen) {  // the mean length's, but a third of the longest one's, since a block that goes on pays one memory latency each time
+    const int mean = p.total_q / p.batch / pre_rows + 1, third = (pre_blocks + 2) / 3, enough = mean > third ? mean : third;
+    pre_blocks = enough < pre_blocks ? enough : pre_blocks;
+    pre_blocks = pre_blocks < kMaxGridY ? pre_blocks : kMaxGridY;
+  }
   for (pre.block0 = 0; pre.block0 < pre_blocks; pre.block0 += kMaxGridY) {  // one launch up to 2 M rows
     const int rest = pre_blocks - pre.block0;
     const dim3 pre_grid(p.heads_q + (varlen ? 1 : 0), rest < kMaxGridY ? rest : kMaxGridY, p.batch);
