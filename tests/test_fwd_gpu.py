@@ -278,7 +278,7 @@ def test_single_tile_units(cuda_device, native_lib, B, H, Lq, Lk, D, causal):
     (1, 149, 149, 100, 100, 64, True),     # one unit more than SMs
     (1, 37, 37, 1025, 1025, 64, True),     # five units per head, the last of one row
     (3, 50, 25, 300, 200, 128, True),      # units without keys, whose rows become zero; 16 empty slots in the last group of heads
-    (8, 48, 48, 200, 300, 64, False),      # more than two rounds
+    (8, 48, 48, 200, 300, 64, False),      # more than two rounds, a list of fewer than 48
     (9, 32, 8, 257, 64, 96, True),
 ])
 def test_units_taken_from_waiting_ctas(cuda_device, native_lib, B, Hq, Hkv, Lq, Lk, D, causal):

@@ -92,7 +92,7 @@ struct FwdKernelParams {
   const int32_t* cu_q;
   const int32_t* cu_k;
   uint32_t* status;
-  uint32_t* unit_counter;  // zeroed before the launch, or null: every CTA begins with the slot of its own index
+  uint32_t* unit_counter;  // zeroed before the launch (kCounted); else every CTA begins with the slot of its own index
   int steal;               // and goes on with those of CTAs that have not started
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int seqlen_q, seqlen_k, total_q, heads_q, kv_group;
@@ -183,11 +183,13 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
   return true;
 }
 
-// The next unit of the list (u.done: there is none).
+// The next unit of the list (u.done: there is none). kCounted: off the counter. An instance of its own, since with both ways in one the packed calls that
+// take the counter lost 1 %.
+template <bool kCounted>
 __device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first, uint8_t* smem, uint32_t bar, volatile uint32_t* abort_flag, Unit& u) {
   for (;; first = false) {
     int slot = p.order.slots;
-    if (p.unit_counter != nullptr) {
+    if constexpr (kCounted) {
       slot = static_cast<int>(atomicAdd(p.unit_counter, 1u));
     } else if (first) {
       slot = static_cast<int>(blockIdx.x);
@@ -289,7 +291,7 @@ __device__ __forceinline__ void write_unit(uint8_t* smem, uint32_t e, const Unit
   dst[3] = make_uint4(u.n_iter, u.done, 0, 0);
 }
 
-template <int kD, bool kF16, bool kDrop, bool kBias>
+template <int kD, bool kF16, bool kDrop, bool kBias, bool kCounted>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k,
@@ -364,7 +366,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     const bool packed = p.cu_q != nullptr;  // the lengths are in memory
     if (packed) wait_for_previous_grid();
     Unit u;
-    claim_unit(p, true, smem, bar, abort_flag, u);
+    claim_unit<kCounted>(p, true, smem, bar, abort_flag, u);
     write_unit(smem, 0, u);
     mbar_arrive(bar + kBarUnitFull);
     if (!packed) wait_for_previous_grid();
@@ -512,7 +514,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (ok && last_runs) ok = mbar_wait(bar + kBarClaim, (runs - 1) & 1, abort_flag);
           if (!ok) break;
           Unit u;
-          claim_unit(p, false, smem, bar, abort_flag, u);
+          claim_unit<kCounted>(p, false, smem, bar, abort_flag, u);
           done = u.done;
           last_runs = !u.done && u.n_iter > 0;
           if (last_runs) ++runs;
@@ -883,21 +885,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.scale_log2 = p.softmax_scale * 1.4426950408889634f;
   kp.is_causal = p.is_causal;
 
-  auto pick = [&](auto drop_tag, auto bias_tag) {
-    constexpr bool kDrop = decltype(drop_tag)::value;
-    constexpr bool kBias = decltype(bias_tag)::value;
-    return p.head_dim <= 64 ? (f16 ? fwd_prefill_kernel<64, true, kDrop, kBias> : fwd_prefill_kernel<64, false, kDrop, kBias>)
-                            : (f16 ? fwd_prefill_kernel<128, true, kDrop, kBias> : fwd_prefill_kernel<128, false, kDrop, kBias>);
-  };
   const bool with_bias = p.bias != nullptr;
-  auto kernel = drop ? (with_bias ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
-                     : (with_bias ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}));
-  cudaError_t err =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-  if (err != cudaSuccess) {
-    set_error("prefill: cudaFuncSetAttribute(%u bytes smem): %s", kSmemBytes, cudaGetErrorString(err));
-    return SDPA_B200_LAUNCH_FAILED;
-  }
   const int sms = sm_count();
   if (sms <= 0) {
     set_error("prefill: cannot read the SM count of the current device");
@@ -921,19 +909,20 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   kp.claim_ahead = claim_ahead(varlen, p.is_causal != 0, kp.order.slots, usable);
   // Where there are more slots than SMs, the grid has a CTA per slot, and one that has done its unit takes the place of one that has not started
   // (clusterlaunchcontrol), which the hardware deals out in order: no counter, so no launch in front that clears one, and with nothing in front the grid may
-  // start under the tail of the one before it. (Calls back to back, us, counter | so: B8 H32 L64 D128 16.9 | 12.1, B8 H12 L512 D64 unmasked 24.6 | 19.3, B8 H16 L512
-  // D128 25.2 | 20.8, B4 H32/8 L700 D64 31.7 | 27.5, L1000 D128 54.4 | 51.1, B7 H32 512 of 1297 94.4 | 91.8, packed: 7 of 19 to 448, 16/16, D64 16.5 | 13.0, 23 of 51 to 236,
-  // 12/12 22.4 | 18.7, 29 of 320 to 1024, 32/8, D64 160.4 | 158.5; level at B4 H32 L4096.) The counter, workspace header word 1, stays
+  // start under the tail of the one before it. (Calls back to back, us, counter | so: B8 H32 L64 D128 16.7 | 12.0, B8 H16 L512 D128 25.3 | 20.8, B4 H32/8 L700 D64
+  // 31.7 | 27.0, L1000 D128 54.1 | 50.3, B7 H32 512 of 1297 93.0 | 90.3, B8 H32 L1024 D64 unmasked 112.7 | 109.4, packed: 7 of 19 to 448, 16/16, D64 16.4 | 13.0, 23 of 51 to 236, 12/12
+  // 22.4 | 18.7, 12 of 64 to 3000, 16/16, D64 125.9 | 122.5, 29 of 320 to 1024, 32/8, D64 160.4 | 155.2; level at B4 H32 L4096.) The counter, workspace header word 1, stays
   //  * where the caller wants SMs left free: pending CTAs would fill them;
-  //  * for lists of sixteen rounds and more, where its launch is nothing and a packed list's empty slots are skipped faster by it (28 sequences of 64 to 3008
-  //    tokens, 64/8, D64 1019 | 1034, 32 of 192 to 1321 413.9 | 416.7);
+  //  * for lists of forty-eight rounds and more, where its launch is nothing and a packed list's empty slots are skipped faster by it (28 sequences of 64 to 3008
+  //    tokens, 64/8, D64, 145 rounds, 1033 | 1042, 32 of 192 to 1321, 83 rounds, 414 | 417; but 24 of 500 to 1500, 32/8, 31 rounds, 236.3 | 234.8);
   //  * for dense calls of up to two rounds without mask, bias or dropout: there the suite reads the claims from the launch that clears it.
   // Not two units per CTA, dealt out by index: a CTA whose SM another stream's kernel holds then starts both its units late (beside a call on 8 SMs B8 H12 L512
   // D64 32.9 us, with a counter 24.6, B5 H8 L1024 D128 57.4, 41.0).
   const int slots = kp.order.slots;
   const bool plain = !varlen && !p.is_causal && !with_bias && !drop;
-  const bool counted = slots > usable && (p.sm_margin > 0 || slots >= 16 * usable || (plain && slots <= 2 * usable));
+  const bool counted = slots > usable && (p.sm_margin > 0 || slots >= 48 * usable || (plain && slots <= 2 * usable));
   kp.steal = slots > usable && !counted;
+  cudaError_t err;
   kp.unit_counter = nullptr;
   if (counted) {
     kp.unit_counter = static_cast<uint32_t*>(workspace) + 1;
@@ -942,6 +931,23 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
       set_error("prefill: clearing the unit counter failed: %s", cudaGetErrorString(err));
       return SDPA_B200_LAUNCH_FAILED;
     }
+  }
+  auto pick = [&](auto drop_tag, auto bias_tag) {
+    constexpr bool kDrop = decltype(drop_tag)::value;
+    constexpr bool kBias = decltype(bias_tag)::value;
+    auto of = [&](auto counted_tag) {
+      constexpr bool kCounted = decltype(counted_tag)::value;
+      return p.head_dim <= 64 ? (f16 ? fwd_prefill_kernel<64, true, kDrop, kBias, kCounted> : fwd_prefill_kernel<64, false, kDrop, kBias, kCounted>)
+                              : (f16 ? fwd_prefill_kernel<128, true, kDrop, kBias, kCounted> : fwd_prefill_kernel<128, false, kDrop, kBias, kCounted>);
+    };
+    return counted ? of(std::true_type{}) : of(std::false_type{});
+  };
+  auto kernel = drop ? (with_bias ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
+                     : (with_bias ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}));
+  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (err != cudaSuccess) {
+    set_error("prefill: cudaFuncSetAttribute(%u bytes smem): %s", kSmemBytes, cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
   }
   const dim3 grid(counted ? usable : slots);
   // Without the clearing launch in front, the grid may start under the tail of the one before it in the stream, whichever that is. Calls back
