@@ -92,8 +92,7 @@ struct FwdKernelParams {
   const int32_t* cu_q;
   const int32_t* cu_k;
   uint32_t* status;
-  uint32_t* unit_counter;  // zeroed before the launch (kCounted); else every CTA begins with the slot of its own index
-  int steal;               // and goes on with those of CTAs that have not started
+  uint32_t* unit_counter;  // zeroed before the launch, or null: every CTA takes the slot of its own index, and with kSteal those of CTAs that have not started
   int64_t o_batch_stride, o_head_stride, o_row_stride;
   int seqlen_q, seqlen_k, total_q, heads_q, kv_group;
   int head_dim;  // <= kD: the real row length, for the paths that write rows without TMA
@@ -183,23 +182,26 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
   return true;
 }
 
-// The next unit of the list (u.done: there is none). kCounted: off the counter. An instance of its own, since with both ways in one the packed calls that
-// take the counter lost 1 %.
-template <bool kCounted>
+// The next unit of the list (u.done: there is none). kSteal: from a CTA that has not started; else off the counter, or, without one, none but the slot of the
+// CTA's own index. Instances of their own, since with both ways in one the calls that do not steal lost up to 1 %.
+template <bool kSteal>
 __device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first, uint8_t* smem, uint32_t bar, volatile uint32_t* abort_flag, Unit& u) {
   for (;; first = false) {
-    int slot = p.order.slots;
-    if constexpr (kCounted) {
-      slot = static_cast<int>(atomicAdd(p.unit_counter, 1u));
-    } else if (first) {
+    int slot;
+    if constexpr (kSteal) {
       slot = static_cast<int>(blockIdx.x);
-    } else if (p.steal) {
-      volatile uint32_t* requests = reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests);
-      const uint32_t n = *requests;
-      *requests = n + 1;
-      take_waiting_cta(bar + kSmemTaken, bar + kBarTaken);
-      const int cta = mbar_wait(bar + kBarTaken, n & 1, abort_flag) ? taken_cta(bar + kSmemTaken) : -1;
-      if (cta >= 0) slot = cta;
+      if (!first) {
+        volatile uint32_t* requests = reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests);
+        const uint32_t n = *requests;
+        *requests = n + 1;
+        take_waiting_cta(bar + kSmemTaken, bar + kBarTaken);
+        slot = mbar_wait(bar + kBarTaken, n & 1, abort_flag) ? taken_cta(bar + kSmemTaken) : -1;
+        if (slot < 0) slot = p.order.slots;
+      }
+    } else {
+      slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
+             : first                   ? static_cast<int>(blockIdx.x)
+                                       : p.order.slots;
     }
     u.done = slot >= p.order.slots;
     if (u.done || decode_unit(p, slot, u)) return;  // padding slots and row-less units are skipped
@@ -291,7 +293,7 @@ __device__ __forceinline__ void write_unit(uint8_t* smem, uint32_t e, const Unit
   dst[3] = make_uint4(u.n_iter, u.done, 0, 0);
 }
 
-template <int kD, bool kF16, bool kDrop, bool kBias, bool kCounted>
+template <int kD, bool kF16, bool kDrop, bool kBias, bool kSteal>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k,
@@ -355,8 +357,10 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bar + kBarStageFull + 8 * t, 4);
     }
     mbar_init(bar + kBarClaim, 1);
-    mbar_init(bar + kBarTaken, 1);
-    *reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests) = 0u;
+    if constexpr (kSteal) {
+      mbar_init(bar + kBarTaken, 1);
+      *reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests) = 0u;
+    }
     for (int e = 0; e < kUnitRing; ++e) {
       mbar_init(bar + kBarUnitFull + 8 * e, 1);
       mbar_init(bar + kBarUnitEmpty + 8 * e, kUnitReaders);
@@ -366,7 +370,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     const bool packed = p.cu_q != nullptr;  // the lengths are in memory
     if (packed) wait_for_previous_grid();
     Unit u;
-    claim_unit<kCounted>(p, true, smem, bar, abort_flag, u);
+    claim_unit<kSteal>(p, true, smem, bar, abort_flag, u);
     write_unit(smem, 0, u);
     mbar_arrive(bar + kBarUnitFull);
     if (!packed) wait_for_previous_grid();
@@ -514,7 +518,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (ok && last_runs) ok = mbar_wait(bar + kBarClaim, (runs - 1) & 1, abort_flag);
           if (!ok) break;
           Unit u;
-          claim_unit<kCounted>(p, false, smem, bar, abort_flag, u);
+          claim_unit<kSteal>(p, false, smem, bar, abort_flag, u);
           done = u.done;
           last_runs = !u.done && u.n_iter > 0;
           if (last_runs) ++runs;
@@ -921,7 +925,7 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   const int slots = kp.order.slots;
   const bool plain = !varlen && !p.is_causal && !with_bias && !drop;
   const bool counted = slots > usable && (p.sm_margin > 0 || slots >= 48 * usable || (plain && slots <= 2 * usable));
-  kp.steal = slots > usable && !counted;
+  const bool steal = slots > usable && !counted;
   cudaError_t err;
   kp.unit_counter = nullptr;
   if (counted) {
@@ -935,12 +939,12 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   auto pick = [&](auto drop_tag, auto bias_tag) {
     constexpr bool kDrop = decltype(drop_tag)::value;
     constexpr bool kBias = decltype(bias_tag)::value;
-    auto of = [&](auto counted_tag) {
-      constexpr bool kCounted = decltype(counted_tag)::value;
-      return p.head_dim <= 64 ? (f16 ? fwd_prefill_kernel<64, true, kDrop, kBias, kCounted> : fwd_prefill_kernel<64, false, kDrop, kBias, kCounted>)
-                              : (f16 ? fwd_prefill_kernel<128, true, kDrop, kBias, kCounted> : fwd_prefill_kernel<128, false, kDrop, kBias, kCounted>);
+    auto of = [&](auto steal_tag) {
+      constexpr bool kSteal = decltype(steal_tag)::value;
+      return p.head_dim <= 64 ? (f16 ? fwd_prefill_kernel<64, true, kDrop, kBias, kSteal> : fwd_prefill_kernel<64, false, kDrop, kBias, kSteal>)
+                              : (f16 ? fwd_prefill_kernel<128, true, kDrop, kBias, kSteal> : fwd_prefill_kernel<128, false, kDrop, kBias, kSteal>);
     };
-    return counted ? of(std::true_type{}) : of(std::false_type{});
+    return steal ? of(std::true_type{}) : of(std::false_type{});
   };
   auto kernel = drop ? (with_bias ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
                      : (with_bias ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}));
