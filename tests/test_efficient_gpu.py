@@ -422,3 +422,20 @@ def test_gradient_of_a_broadcast_bias(cuda_device, native_lib, B, H, L, shape, d
     for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, torch.autograd.grad(ref, f, do.float())):
         assert g.shape == w.shape and float((g.float() - w).norm() / w.norm()) < 1e-2, name
     assert float((out.float() - ref).norm() / ref.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("D,last", [(128, 0.0), (72, -0.0), (128, float("-inf")), (128, 1.5)])
+def test_bias_with_blocks_of_zeros(cuda_device, native_lib, D, last):
+    """A bias that is the same for every query: a block of 128 keys of zeros, one with a single other value in its last key (minus zero counts as one,
+    and adds nothing), a ragged one. Against fp32 math; where the bias adds nothing at all, the bits of the call without one."""
+    gen = torch.Generator(device=cuda_device).manual_seed(2)
+    q, k, v = (torch.randn(2, 3, 300, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for _ in range(3))
+    bias = torch.zeros(2, 1, 1, 304, device=cuda_device, dtype=torch.bfloat16)
+    bias[1, ..., 255] = last
+    out, lse = ops._dense_forward(q, k, v, False, None, True, bias=bias[..., :300].expand(2, 3, 300, 300))
+    s = q.float() @ k.float().transpose(2, 3) * D ** -0.5 + bias[..., :300].float()
+    want = torch.softmax(s, -1) @ v.float()
+    assert float((out.float() - want).norm() / want.norm()) < 4e-3 and float((lse - s.logsumexp(-1)).abs().max()) < 1e-5
+    if last == 0:
+        plain, plain_lse = ops._dense_forward(q, k, v, False, None, True)
+        assert torch.equal(out, plain) and torch.equal(lse, plain_lse)
