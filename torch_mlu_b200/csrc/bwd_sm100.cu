@@ -23,7 +23,7 @@
 //   3. dQ, one of: bwd_tile_kernel<kModeDQ>, one CTA per (batch, query head, 128-query block); Q and dO
 //      stay, (K, V) stream; S = Q K^T, dP = dO V^T, dS -> TMEM, dQ += dS K. Or, where launch 2 has left its dS
 //      in the workspace as well (8 stores of 16 bytes per thread and item: 281 -> 308 us at B8 H16 L2048 D128
-//      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> 130).
+//      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> 118).
 // TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512); up to head_dim 64 accumulators of 64 columns, with tiles of 64 rows four times 64. The bf16 P and dS of an item both
 // live in the item's score buffer, so the buffer that held dP is free as soon as it has been read;
 // the MMA issuer uses that (and, for dQ, the unused ACC2) to run the next item's score GEMMs and
