@@ -307,3 +307,22 @@ def test_packed_units_taken_from_waiting_ctas(cuda_device, native_lib, D):
         if hi > lo:
             o, l = ops.gqa_prefill(*(t[lo:hi].transpose(0, 1).unsqueeze(0) for t in (q, k, v)), is_causal=True)
             assert torch.equal(out[lo:hi], o[0].transpose(0, 1)) and torch.equal(lse[..., lo:hi].reshape(24, -1), l[0])
+
+
+def test_units_taken_from_waiting_ctas_on_two_streams(cuda_device, native_lib):
+    """Two grids whose CTAs wait for the same SMs: each takes units of its own only."""
+    gen = torch.Generator(device=cuda_device).manual_seed(6)
+    calls = [tuple(torch.randn(B, 12, L, 64, generator=gen, device=cuda_device, dtype=torch.bfloat16) for _ in range(3)) for B, L in ((8, 512), (11, 300))]
+    want = [ops.gqa_prefill(*c, is_causal=True) for c in calls]
+    streams = [torch.cuda.Stream(cuda_device) for _ in calls]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(8):
+        for i, c in enumerate(calls):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(ops.gqa_prefill(*c, is_causal=True))
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for w, results in zip(want, got):
+        for out, lse in results:
+            assert torch.equal(out, w[0]) and torch.equal(lse, w[1])
