@@ -9,7 +9,7 @@ import torch
 import torch.nn.functional as F
 
 from oracle import sdpa_oracle as orc
-from torch_mlu_b200 import backends, ops, sdp_choice
+from torch_mlu_b200 import backends, ops, sdp_choice, torch_glue
 from torch_mlu_b200.backends import SDPBackend
 
 pytestmark = pytest.mark.gpu
@@ -439,3 +439,22 @@ def test_bias_with_blocks_of_zeros(cuda_device, native_lib, D, last):
     if last == 0:
         plain, plain_lse = ops._dense_forward(q, k, v, False, None, True)
         assert torch.equal(out, plain) and torch.equal(lse, plain_lse)
+
+
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("shape", [(2, 3, 40, 32), (40, 2), (2, 3, 40, 39), (2, 3, 40, 48), (1, 2, 3, 40, 40), ()])
+def test_bias_of_another_number_of_keys_is_refused(cuda_device, native_lib, shape, padded):
+    """The registered backward, called by itself: a bias with fewer or more keys than key has, or of no or five dimensions, raises before a kernel
+    reads it. Padded rows may be longer."""
+    torch_glue.load()
+    q, k, v, out, do = (torch.zeros(2, 3, 40, 64, device=cuda_device, dtype=torch.bfloat16) for _ in range(5))
+    lse = torch.zeros(2, 3, 40, device=cuda_device)
+    bias = torch.zeros(shape, device=cuda_device, dtype=torch.bfloat16)
+    call = lambda b: torch.ops.b200_sdpa._bias_attention_backward(do, q, k, v, b, out, lse, padded, False, True, 0.125)
+    for b in (bias, torch.cat((bias, bias), -1)[..., 1:1 + shape[-1]] if shape else bias):  # rows as they are, and rows that begin at odd addresses
+        if padded and shape[-1:] == (48,):
+            assert call(b)[3].shape == (2, 3, 40, 40)
+        else:
+            with pytest.raises((RuntimeError, IndexError)):
+                call(b)
+    assert ops.device_status() == 0

@@ -47,8 +47,11 @@ bool dispatcher_may_be_skipped() {
 // ------------------------------------------------------------------------- additive bias
 int64_t ceil8(int64_t n) { return (n + 7) / 8 * 8; }
 
-// A copy of the bias (of q's type and device) with rows padded to a multiple of 8 keys.
+// A copy of the bias (of q's type and device) with rows padded to a multiple of 8 keys. The kernel reads `seqlen_k` keys of every row, so the
+// bias must have them, or one for all.
 Tensor padded_copy(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k) {
+  TORCH_CHECK(attn_bias.size(-1) == 1 || attn_bias.size(-1) == seqlen_k, "attn_bias must have one key or the ", seqlen_k, " of key, it has ",
+              attn_bias.size(-1));
   std::vector<int64_t> sizes(attn_bias.sizes().begin(), attn_bias.sizes().end());
   sizes.back() = ceil8(seqlen_k);
   int64_t own[4] = {1, 1, 1, seqlen_k}, strides[4] = {0, 0, 0, attn_bias.size(-1) == 1 ? 0 : attn_bias.stride(-1)};
@@ -102,6 +105,7 @@ Tensor readable_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k,
 }
 
 Tensor prepare_bias(const Tensor& attn_bias, const Tensor& q, int64_t seqlen_k, bool padded) {
+  TORCH_CHECK(attn_bias.dim() >= 1 && attn_bias.dim() <= 4, "attn_bias must have one to four dimensions, it has ", attn_bias.dim());
   const Tensor view = readable_bias(attn_bias, q, seqlen_k, padded);
   if (view.defined()) return view;
   return readable_bias(padded_copy(padded ? attn_bias.narrow(-1, 0, seqlen_k) : attn_bias, q, seqlen_k), q, seqlen_k, true);
