@@ -200,6 +200,11 @@ SDPA_B200_API int sdpa_b200_read_device_status(const void* workspace, void* stre
  * nothing back from the device. */
 SDPA_B200_API int sdpa_b200_selftest_wait_timeout(uint32_t* device_status, uint32_t budget_us, void* stream);
 
+/* The same for a forward's grid with several CTAs per SM: each of `ctas` CTAs, one at a time per SM, adds 1 to *started and waits for at most `budget_us`
+ * (up to 1000) microseconds; those that give up take the CTAs that have not started with them, so that the grid ends after one budget and *started
+ * has grown by no more than the number of SMs. */
+SDPA_B200_API int sdpa_b200_selftest_grid_timeout(uint32_t* device_status, uint32_t* started, uint32_t ctas, uint32_t budget_us, void* stream);
+
 /* Split-KV decode (dense tensors, seqlen_q == 1) for callers that cannot allocate device memory
  * where they call it - inside an allocator or memory-pool callback, or after the process has
  * frozen its memory plan. No counterpart in the reference: its attention calls always take a

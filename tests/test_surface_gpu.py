@@ -223,3 +223,22 @@ def test_sm_margin_leaves_the_result_alone(cuda_device, native_lib, margin):
     o_ref, l_ref = orc.cpu_sdpa_forward(q, k, v, causal=True)
     orc.assert_close_bf16(out1, o_ref, "out")
     orc.assert_close_lse(lse1, l_ref)
+
+
+@pytest.mark.parametrize("rounds", [1, 3, 30])
+def test_a_grid_whose_waits_run_out_ends_after_one_budget(cuda_device, native_lib, rounds):
+    """A grid with several CTAs per SM, as a forward has them, in which every wait runs out: those that give up take the CTAs that have not started with
+    them, so that each SM starts one. The next call is clean."""
+    dev = cuda_device
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    words = torch.zeros(2, dtype=torch.int32, device=dev)
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    _cabi.check(native_lib.sdpa_b200_selftest_grid_timeout(words.data_ptr(), words.data_ptr() + 4, rounds * sms, 200, stream), "selftest")
+    status, started = words.tolist()
+    assert status == _cabi.DEVICE_TIMEOUT and 1 <= started <= sms
+    for ctas, budget in ((0, 200), (148, 0), (148, 1001), (100001, 200)):
+        assert native_lib.sdpa_b200_selftest_grid_timeout(words.data_ptr(), words.data_ptr() + 4, ctas, budget, stream) == _cabi.INVALID_ARG
+    q = rand((8, 64, 256, 128), 1).to(dev)
+    out, lse = ops.gqa_prefill(q, q, q, is_causal=True)
+    again = ops.gqa_prefill(q, q, q, is_causal=True, sm_margin=1)
+    assert ops.device_status(dev) == 0 and torch.equal(out, again[0]) and torch.equal(lse, again[1])

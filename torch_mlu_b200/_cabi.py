@@ -28,6 +28,7 @@ EXPORTED_SYMBOLS = (
     "sdpa_b200_bwd",
     "sdpa_b200_read_device_status",
     "sdpa_b200_selftest_wait_timeout",
+    "sdpa_b200_selftest_grid_timeout",
     "sdpa_b200_decode_static",
     "sdpa_b200_merge_partial",
     "sdpa_b200_dropout_keep_mask",
@@ -108,6 +109,8 @@ def load() -> ctypes.CDLL:
     lib.sdpa_b200_read_device_status.argtypes = [c_void_p, c_void_p, POINTER(c_int)]
     lib.sdpa_b200_selftest_wait_timeout.restype = c_int
     lib.sdpa_b200_selftest_wait_timeout.argtypes = [c_void_p, ctypes.c_uint32, c_void_p]
+    lib.sdpa_b200_selftest_grid_timeout.restype = c_int
+    lib.sdpa_b200_selftest_grid_timeout.argtypes = [c_void_p, c_void_p, ctypes.c_uint32, ctypes.c_uint32, c_void_p]
     lib.sdpa_b200_decode_static.restype = c_int
     lib.sdpa_b200_decode_static.argtypes = [POINTER(SdpaParams), c_void_p]
     lib.sdpa_b200_merge_partial.restype = c_int

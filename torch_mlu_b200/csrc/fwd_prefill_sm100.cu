@@ -182,6 +182,8 @@ __device__ __forceinline__ bool decode_unit(const FwdKernelParams& p, int slot, 
   return true;
 }
 
+__device__ __forceinline__ volatile uint32_t* requests_word(uint8_t* smem) { return reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests); }
+
 // The next unit of the list (u.done: there is none). kSteal: from a CTA that has not started; else off the counter, or, without one, none but the slot of the
 // CTA's own index. Instances of their own, since with both ways in one the calls that do not steal lost up to 1 %.
 template <bool kSteal>
@@ -189,15 +191,8 @@ __device__ __forceinline__ void claim_unit(const FwdKernelParams& p, bool first,
   for (;; first = false) {
     int slot;
     if constexpr (kSteal) {
-      slot = static_cast<int>(blockIdx.x);
-      if (!first) {
-        volatile uint32_t* requests = reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests);
-        const uint32_t n = *requests;
-        *requests = n + 1;
-        take_waiting_cta(bar + kSmemTaken, bar + kBarTaken);
-        slot = mbar_wait(bar + kBarTaken, n & 1, abort_flag) ? taken_cta(bar + kSmemTaken) : -1;
-        if (slot < 0) slot = p.order.slots;
-      }
+      slot = first ? static_cast<int>(blockIdx.x) : take_waiting_cta(bar + kSmemTaken, bar + kBarTaken, requests_word(smem), abort_flag);
+      if (slot < 0) slot = p.order.slots;
     } else {
       slot = p.unit_counter != nullptr ? static_cast<int>(atomicAdd(p.unit_counter, 1u))
              : first                   ? static_cast<int>(blockIdx.x)
@@ -359,7 +354,7 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
     mbar_init(bar + kBarClaim, 1);
     if constexpr (kSteal) {
       mbar_init(bar + kBarTaken, 1);
-      *reinterpret_cast<volatile uint32_t*>(smem + kSmemBar + kSmemRequests) = 0u;
+      *requests_word(smem) = 0u;
     }
     for (int e = 0; e < kUnitRing; ++e) {
       mbar_init(bar + kBarUnitFull + 8 * e, 1);
@@ -525,6 +520,9 @@ fwd_prefill_kernel(const __grid_constant__ CUtensorMap tm_q,
           write_unit(smem, e, u);
           mbar_arrive(bar + kBarUnitFull + 8 * e);  // release: the entry is visible to whoever sees the phase
         }
+        // given up: up to 48 CTAs behind this one on its SM would each wait the 2 s; their rows stay unwritten, as this one's do
+        if constexpr (kSteal)
+          if (!ok) discard_waiting_ctas(bar + kSmemTaken, bar + kBarTaken, requests_word(smem), abort_flag);
       }
     }
   } else {

@@ -277,15 +277,26 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
   return mbar_wait_budget(bar, parity, abort_flag, kWaitBudgetNs);
 }
 
-// Asks for a CTA of this grid that has not started: it then never will, and its index, written to 16 bytes of shared memory (the phase of `bar` expects
-// them), is this CTA's to work on. Not again once a request has found none. What this thread has read of an earlier answer goes before.
-__device__ __forceinline__ void take_waiting_cta(uint32_t answer, uint32_t bar) {
-  fence_proxy_async_smem();
+// The index (of a one-dimensional grid) of a CTA of this grid that has not started, and now never will: its work is this CTA's; or -1: there is none, or no answer has
+// come after the budget, which sets the flag. For one thread at a time, and not again behind a -1. `answer`: 16 bytes of shared memory for the hardware's answer,
+// `bar`: a barrier of one arrival of its own, `requests`: a word of shared memory, 0 at first. An answer on its way is waited for also where the CTA has given up
+// meanwhile: a CTA must not end before it is there, nor without the work that it brings.
+__device__ __forceinline__ int take_waiting_cta(uint32_t answer, uint32_t bar, volatile uint32_t* requests, volatile uint32_t* abort_flag,
+                                                uint64_t budget_ns = kWaitBudgetNs) {
+  const uint32_t n = *requests;
+  *requests = n + 1;
+  fence_proxy_async_smem();  // what this thread has read of an earlier answer goes before
   mbar_arrive_expect_tx(bar, 16);
   asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
-}
-// The index (of a one-dimensional grid) in the answer, or -1.
-__device__ __forceinline__ int taken_cta(uint32_t answer) {
+  if (!mbar_test(bar, n & 1)) {
+    const uint64_t t0 = global_timer_ns();
+    while (!mbar_test(bar, n & 1)) {
+      if (global_timer_ns() - t0 > budget_ns) {
+        *abort_flag = 1;
+        return -1;
+      }
+    }
+  }
   int x;
   asm volatile(
       "{\n\t"
@@ -300,6 +311,13 @@ __device__ __forceinline__ int taken_cta(uint32_t answer) {
       : "r"(answer)
       : "memory");
   return x;
+}
+// For a CTA that has given up, instead of the work behind its last one: takes all CTAs that have not started with it. Each of them would wait the whole budget in its
+// turn, one behind the other on an SM, before the status could be read.
+__device__ __forceinline__ void discard_waiting_ctas(uint32_t answer, uint32_t bar, volatile uint32_t* requests, volatile uint32_t* abort_flag,
+                                                     uint64_t budget_ns = kWaitBudgetNs) {
+  while (take_waiting_cta(answer, bar, requests, abort_flag, budget_ns) >= 0) {
+  }
 }
 
 // After a time-out the CTA must not return while copies it started or MMAs it issued are still in

@@ -320,6 +320,25 @@ __global__ void selftest_wait_timeout_kernel(uint32_t* status, uint64_t budget_n
   __syncwarp();
   if (threadIdx.x == 0 && (!ok || abort_word != 0)) atomicExch(status, static_cast<uint32_t>(SDPA_B200_DEVICE_TIMEOUT));
 }
+
+// The same in each CTA of a grid of several per SM, as the forward's are: counted when they start, they give up, and take those that wait with them.
+constexpr uint32_t kSelftestSmem = 200 * 1024;  // one CTA per SM
+__global__ void selftest_grid_timeout_kernel(uint32_t* status, uint32_t* started, uint64_t budget_ns) {
+  extern __shared__ uint8_t one_cta_per_sm[];
+  __shared__ __align__(16) uint8_t answer[16];
+  __shared__ uint64_t barriers[2];
+  __shared__ uint32_t abort_word, requests;
+  if (threadIdx.x != 0) return;
+  mbar_init(smem_u32(&barriers[0]), 1);
+  mbar_init(smem_u32(&barriers[1]), 1);
+  abort_word = 0;
+  requests = 0;
+  fence_mbar_init();
+  atomicAdd(started, 1u);
+  if (!mbar_wait_budget(smem_u32(&barriers[0]), 0, &abort_word, budget_ns))
+    discard_waiting_ctas(smem_u32(answer), smem_u32(&barriers[1]), &requests, &abort_word);
+  if (abort_word != 0) atomicExch(status, static_cast<uint32_t>(SDPA_B200_DEVICE_TIMEOUT));
+}
 }  // namespace
 }  // namespace sdpa_b200
 
@@ -341,6 +360,31 @@ int sdpa_b200_selftest_wait_timeout(uint32_t* device_status, uint32_t budget_us,
   selftest_wait_timeout_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(device_status,
                                                                                 static_cast<uint64_t>(budget_us) * 1000ull);
   cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) {
+    set_error("selftest: launch failed: %s", cudaGetErrorString(err));
+    return SDPA_B200_LAUNCH_FAILED;
+  }
+  count_launch();
+  return SDPA_B200_OK;
+}
+
+int sdpa_b200_selftest_grid_timeout(uint32_t* device_status, uint32_t* started, uint32_t ctas, uint32_t budget_us, void* stream) {
+  if (device_status == nullptr || started == nullptr || ((reinterpret_cast<uintptr_t>(device_status) | reinterpret_cast<uintptr_t>(started)) & 3u) != 0) {
+    set_error("device_status and started must be 4-byte aligned device pointers");
+    return SDPA_B200_INVALID_ARG;
+  }
+  if (budget_us == 0 || budget_us > 1000u || ctas == 0 || ctas > 100000u) {
+    set_error("budget_us must be between 1 and 1000, ctas between 1 and 100000 (got %u, %u)", budget_us, ctas);
+    return SDPA_B200_INVALID_ARG;
+  }
+  int st = check_device();
+  if (st != SDPA_B200_OK) return st;
+  cudaError_t err = cudaFuncSetAttribute(selftest_grid_timeout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelftestSmem);
+  if (err == cudaSuccess) {
+    selftest_grid_timeout_kernel<<<ctas, 32, kSelftestSmem, static_cast<cudaStream_t>(stream)>>>(device_status, started,
+                                                                                                 static_cast<uint64_t>(budget_us) * 1000ull);
+    err = cudaGetLastError();
+  }
   if (err != cudaSuccess) {
     set_error("selftest: launch failed: %s", cudaGetErrorString(err));
     return SDPA_B200_LAUNCH_FAILED;
