@@ -2,10 +2,11 @@
 // has left in the workspace (ds_tiles.cuh).
 //
 // Bound by memory: every dS tile is read once, 32 KB for 128 x 128 x head_dim multiply-adds. Two 128-row tiles per unit share each B
-// block (48 KB per step of 64 at head_dim 128 where single tiles would read 64). B8 H16 L2048 D128 causal: 0.57 GB of dS in 118 us. What the kernel in front
-// wrote last is read first, from L2, which is asked to keep dS in front of what streams past it when it is written and to give it up when it has been read
-// (up to head_dim 128, where it is read once): 603 MB from memory instead of 666, 130 us -> 118, and 0.9 % of a step at the power cap (B8 H16 L2048 687 -> 682 us,
-// packed 12 of 64 to 2048 tokens, 16/4 heads, 339 -> 336). Above, where dK and dQ read it and L2 keeps it for neither, the hints changed nothing.
+// block (48 KB per step of 64 at head_dim 128 where single tiles would read 64). B8 H16 L2048 D128 causal: 0.57 GB of dS in 122 us. What the kernel in front
+// wrote last is read first, from L2, which is asked to give dS up when it has been read (up to head_dim 128, where it is read once): 130 us -> 122 there, packed 12 of 64 to
+// 2048 tokens, 16/4 heads, 78 -> 72. Above, where dK and dQ read it and L2 keeps it for neither, the hint changed nothing. Stores of dS that ask L2 to keep it save
+// 3 us more here (119), but neither the read nor its hint takes that back: the lines stay in L2 when the call is over, and every kernel behind has less of it
+// (the pre-pass of B8 H16 L2048 21.5 -> 22.7 us; an addition over 48 + 48 MB, repeated, 12.5 -> 13.7; a product of two 4096 x 4096 matrices 88.9 -> 90.1).
 //
 // Persistent: one CTA per SM takes units of 256 output rows (two 128-row tiles that share every B block) of one head from a
 // counter, heaviest first inside a group of heads. Per 64 rows of the contraction a stage brings B (64 rows of K or Q, 128-byte

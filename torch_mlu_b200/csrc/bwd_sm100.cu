@@ -23,7 +23,7 @@
 //   3. dQ, one of: bwd_tile_kernel<kModeDQ>, one CTA per (batch, query head, 128-query block); Q and dO
 //      stay, (K, V) stream; S = Q K^T, dP = dO V^T, dS -> TMEM, dQ += dS K. Or, where launch 2 has left its dS
 //      in the workspace as well (8 stores of 16 bytes per thread and item: 281 -> 308 us at B8 H16 L2048 D128
-//      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> 118).
+//      causal), the GEMM of bwd_ds_gemm_sm100.cu, which forms no scores (221 us -> 122).
 // TMEM: T1 [0,128) T2 [128,256) ACC1 [256,384) ACC2 [384,512); up to head_dim 64 accumulators of 64 columns, with tiles of 64 rows four times 64. The bf16 P and dS of an item both
 // live in the item's score buffer, so the buffer that held dP is free as soon as it has been read;
 // the MMA issuer uses that (and, for dQ, the unused ACC2) to run the next item's score GEMMs and
@@ -812,12 +812,12 @@ __device__ __forceinline__ void tile_cta(const CUtensorMap& tm_q, const CUtensor
       BWD_STAMP(half, i, 7);
       if (kMode == kModeDKDV && kDsCall && p.ds.data != nullptr) {
         // dS for the dQ GEMM: 16 bytes (8 queries) per store, 512 contiguous bytes per warp. Behind the arrival, so that the
-        // dK GEMM does not wait for the stores to issue. L2 is asked to keep them for that GEMM (figures there)
+        // dK GEMM does not wait for the stores to issue. Without a hint to L2 (see bwd_ds_gemm_sm100.cu)
         if (ds_tile < p.ds.capacity) {
           uint4* dst = ds_group(p.ds, ds_tile, half * 8, r);
 #pragma unroll
           for (int ch = 0; ch < kC / 8; ++ch)
-            st_global_hint(dst + ch * kDsTile, make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]), l2_keep());
+            dst[ch * kDsTile] = make_uint4(dw[4 * ch], dw[4 * ch + 1], dw[4 * ch + 2], dw[4 * ch + 3]);
         }
         // past this row of tiles; behind the last one the next head's tiles begin
         const DsHead rows{0, (len_k + kTile - 1) / kTile, ds_shift(len_q, len_k, p.is_causal != 0)};

@@ -349,19 +349,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst_smem, const CUtensorMap
       : "memory");
 }
 
-// How long L2 is to keep the lines that an access brings in or writes: longer than others, or no longer than until it needs the room.
-__device__ __forceinline__ uint64_t l2_keep() {
-  uint64_t policy;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
-  return policy;
-}
+// For an access whose lines L2 need not keep: they make room first.
 __device__ __forceinline__ uint64_t l2_drop() {
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   return policy;
-}
-__device__ __forceinline__ void st_global_hint(uint4* dst, uint4 v, uint64_t policy) {
-  asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void tma_load_4d_hint(uint32_t dst_smem, const CUtensorMap* m, uint32_t bar,
                                                  int c0, int c1, int c2, int c3, uint64_t policy) {
