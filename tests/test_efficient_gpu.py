@@ -9,7 +9,7 @@ import torch
 import torch.nn.functional as F
 
 from oracle import sdpa_oracle as orc
-from torch_mlu_b200 import backends, ops, sdp_choice, torch_glue
+from torch_mlu_b200 import _cabi, backends, ops, sdp_choice, torch_glue
 from torch_mlu_b200.backends import SDPBackend
 
 pytestmark = pytest.mark.gpu
@@ -458,3 +458,56 @@ def test_bias_of_another_number_of_keys_is_refused(cuda_device, native_lib, shap
             with pytest.raises((RuntimeError, IndexError)):
                 call(b)
     assert ops.device_status() == 0
+
+
+def _summed(lib, grad, keys, over_batch, over_heads):
+    B, H, L, _ = grad.shape
+    out = torch.full((1 if over_batch else B, 1 if over_heads else H, L, keys), float("nan"), device=grad.device, dtype=grad.dtype)
+    _cabi.check(lib.sdpa_b200_sum_bias_grad(grad.data_ptr(), *grad.stride()[:3], B, H, L, keys, int(over_batch), int(over_heads), out.data_ptr(),
+                                            _cabi.DTYPE_F16 if grad.dtype == torch.float16 else _cabi.DTYPE_BF16,
+                                            torch.cuda.current_stream(grad.device).cuda_stream), "sum_bias_grad")
+    return out
+
+
+@pytest.mark.parametrize("B,H,L,over_batch,over_heads", [
+    (15, 1, 9, True, False),     # one thread per element
+    (16, 1, 9, True, False),     # two, of eight summands each
+    (31, 1, 16, True, False),
+    (5, 13, 33, True, True),     # four and 65 summands
+    (1, 128, 40, False, True),   # sixteen
+    (257, 2, 7, True, True),     # 32, and two more summands than they divide
+    (1030, 3, 49, True, False),  # more eights than threads
+    (3, 8, 700, True, True),     # enough elements for one thread each
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_summed_bias_gradient(cuda_device, native_lib, B, H, L, over_batch, over_heads, dtype):
+    """The kernel alone, at the edges of the split of an element's summands over threads, against the sum in 64 bits: one rounding to 16 bits, and an fp32 error of
+    2^-24 per addition, each of at most the sum of magnitudes. Padding holds NaN and takes no part."""
+    gen = torch.Generator(device=cuda_device).manual_seed(13)
+    grad = torch.randn(B, H, L, (L + 7) // 8 * 8, generator=gen, device=cuda_device, dtype=dtype)
+    grad[..., L:] = float("nan")
+    got = _summed(native_lib, grad, L, over_batch, over_heads).double()
+    x = grad[..., :L].double()
+    want, size = x.sum_to_size(got.shape), x.abs().sum_to_size(got.shape)
+    unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert bool(((got - want).abs() <= unit * want.abs() + B * H * 2.0 ** -24 * size + 2.0 ** -24).all())
+
+
+def test_summed_bias_gradient_of_short_sequences_takes_no_longer_than_the_general_sum(cuda_device, native_lib):
+    """Few elements with many summands each: with all of an element's in one thread 20 to 40 times the tensor library's time, which three times cannot reach
+    by noise."""
+    from torch.profiler import ProfilerActivity, profile
+    for B, H, L, over_batch, over_heads in [(1024, 4, 49, True, False), (64, 12, 128, True, True)]:
+        grad = torch.randn(B, H, L, (L + 7) // 8 * 8, device=cuda_device, dtype=torch.bfloat16)
+        sizes = (1 if over_batch else B, 1 if over_heads else H, L, L)
+        times = []
+        for call in (lambda: _summed(native_lib, grad, L, over_batch, over_heads), lambda: grad[..., :L].sum_to_size(sizes)):
+            call()
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                for _ in range(15):
+                    call()
+                torch.cuda.synchronize()
+            each = sorted(e.device_time for e in prof.events() if "bias_grad_sum" in e.name or "reduce_kernel" in e.name)
+            assert len(each) == 15
+            times.append(each[7])
+        assert times[0] <= 3 * times[1], (B, H, L, times)

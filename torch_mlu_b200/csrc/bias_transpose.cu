@@ -107,48 +107,100 @@ __global__ void __launch_bounds__(256) bias_pad_kernel(const PadParams p, int64_
   p.out[i] = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
 }
 
-// Sums a [batch, heads, seqlen_q, seqlen_k] gradient over batches and / or heads, eight keys per thread, fp32, in the order of the indexes. Bound by memory: a
-// thread's reads do not depend on one another, eight are in flight (16 batches of 12 heads of 594 x 594 135 MB in 27 us; the tensor library's sum 52).
+// Sums a [batch, heads, seqlen_q, seqlen_k] gradient over batches and / or heads, eight keys per thread, fp32. Bound by memory and, behind it, by instructions: eight
+// reads are in flight per thread, addresses are counted on instead of divided out. (Behind the kernel that writes the gradient, tensor library's sum | one thread per
+// element | so: 16 batches of 12 heads of 594 x 594, 135 MB, 52 us | 42 | 38; 2 of 8 of 2000 x 2000 114 | 85 | 72; 40 of 12 of 384 x 384 36 | 47 | 47, with
+// 128-byte reads per thread too short for its many streams.) Where the result is small, `slices` threads share an element's summands, every slices-th eight of them, and
+// their sums meet in shared memory, in the order of the threads: in one thread, the 512 summands of a [64, 64] bias of B32 H16 are 64 memory latencies one behind the
+// other on two SMs (16 | 163 | 8; [197, 197] of B16 H12 20 | 65 | 6.6; 256 batches of 8 heads of 100 x 100 14.6 | 106 | 15.8).
 struct GradSumParams {
   const uint16_t* grad;
   uint16_t* out;  // contiguous
   int64_t batch_stride, head_stride, row_stride;
   int out_heads, sum_batches, sum_heads;  // heads of the result; batches and heads per element of it
   int seqlen_q, seqlen_k, groups;
+  int slices;       // a power of two up to kSumThreads / 8
+  bool wide_rows;   // rows of the result are whole groups at 16-byte addresses
 };
+constexpr int kSumThreads = 256;
 template <bool kF16>
-__global__ void __launch_bounds__(256) bias_grad_sum_kernel(const GradSumParams p, int64_t total) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int64_t row = i / p.groups;
-  const int k0 = static_cast<int>(i - row * p.groups) * 8;
-  const int64_t bh = row / p.seqlen_q;
-  const int64_t b = bh / p.out_heads;
-  const uint16_t* src = p.grad + b * p.batch_stride + (bh - b * p.out_heads) * p.head_stride + (row - bh * p.seqlen_q) * p.row_stride + k0;
+__global__ void __launch_bounds__(kSumThreads) bias_grad_sum_kernel(const GradSumParams p, int64_t total) {
+  __shared__ float4 sums[2][kSumThreads];
+  const int elements = kSumThreads / p.slices;  // groups of eight keys per block
+  const int slice = threadIdx.x / elements;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * elements + (threadIdx.x - slice * elements);
+  int64_t row, b;
+  int h, q, k0;
+  if (total <= 0xffffffffll) {  // divisions of 64 bits take as long as the loads
+    const uint32_t r = static_cast<uint32_t>(i) / p.groups, bh = r / p.seqlen_q;
+    k0 = static_cast<int>(static_cast<uint32_t>(i) - r * p.groups) * 8;
+    q = static_cast<int>(r - bh * p.seqlen_q);
+    row = r;
+    b = bh / p.out_heads;
+    h = static_cast<int>(bh - static_cast<uint32_t>(b) * p.out_heads);
+  } else {
+    row = i / p.groups;
+    k0 = static_cast<int>(i - row * p.groups) * 8;
+    const int64_t bh = row / p.seqlen_q;
+    q = static_cast<int>(row - bh * p.seqlen_q);
+    b = bh / p.out_heads;
+    h = static_cast<int>(bh - b * p.out_heads);
+  }
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  const int n = p.sum_batches * p.sum_heads;
-  for (int first = 0; first < n; first += 8) {
-    uint4 w[8];
+  if (i < total) {
+    const uint16_t* src = p.grad + b * p.batch_stride + h * p.head_stride + q * p.row_stride + k0;
+    const int n = p.sum_batches * p.sum_heads;
+    const int64_t next_batch = p.batch_stride - static_cast<int64_t>(p.sum_heads - 1) * p.head_stride;
+    for (int first = slice * 8; first < n; first += p.slices * 8) {
+      const int sb = first / p.sum_heads;
+      int sh = first - sb * p.sum_heads;
+      const uint16_t* at = src + sb * p.batch_stride + sh * p.head_stride;
+      uint4 w[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int at = min(first + u, n - 1), sb = at / p.sum_heads;
-      w[u] = __ldcs(reinterpret_cast<const uint4*>(src + sb * p.batch_stride + (at - sb * p.sum_heads) * p.head_stride));
-    }
+      for (int u = 0; u < 8; ++u) {
+        w[u] = first + u < n ? __ldg(reinterpret_cast<const uint4*>(at)) : make_uint4(0u, 0u, 0u, 0u);
+        const bool last = ++sh == p.sum_heads;
+        at += last ? next_batch : p.head_stride;
+        sh = last ? 0 : sh;
+      }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      if (first + u >= n) break;
-      const uint32_t ww[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t ww[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 x = unpack_16x2<kF16>(ww[j]);
-        acc[2 * j] += x.x;
-        acc[2 * j + 1] += x.y;
+        for (int j = 0; j < 4; ++j) {
+          const float2 x = unpack_16x2<kF16>(ww[j]);
+          acc[2 * j] += x.x;
+          acc[2 * j + 1] += x.y;
+        }
       }
     }
   }
+  if (p.slices > 1) {
+    sums[0][threadIdx.x] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    sums[1][threadIdx.x] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    __syncthreads();
+    if (slice != 0) return;
+    for (int other = threadIdx.x + elements; other < kSumThreads; other += elements) {
+      const float4 x = sums[0][other], y = sums[1][other];
+      acc[0] += x.x;
+      acc[1] += x.y;
+      acc[2] += x.z;
+      acc[3] += x.w;
+      acc[4] += y.x;
+      acc[5] += y.y;
+      acc[6] += y.z;
+      acc[7] += y.w;
+    }
+  }
+  if (i >= total) return;
   uint16_t* dst = p.out + row * p.seqlen_k + k0;
+  if (p.wide_rows) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(pack_16x2<kF16>(acc[0], acc[1]), pack_16x2<kF16>(acc[2], acc[3]), pack_16x2<kF16>(acc[4], acc[5]),
+                                                pack_16x2<kF16>(acc[6], acc[7]));
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     if (k0 + j < p.seqlen_k) dst[j] = to_16<kF16>(acc[j]);
@@ -297,13 +349,19 @@ extern "C" SDPA_B200_API int sdpa_b200_sum_bias_grad(const void* grad, int64_t b
   m.seqlen_q = seqlen_q;
   m.seqlen_k = seqlen_k;
   m.groups = (seqlen_k + 7) / 8;
-  const int64_t total = static_cast<int64_t>(over_batch ? 1 : batch) * m.out_heads * seqlen_q * m.groups, blocks = (total + 255) / 256;
+  const int64_t total = static_cast<int64_t>(over_batch ? 1 : batch) * m.out_heads * seqlen_q * m.groups;
+  m.wide_rows = seqlen_k % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  // until every thread has one eight of summands, or the SMs the threads that they hold: beyond, a thread costs more than its shorter chain gives (figures above)
+  m.slices = 1;
+  while (m.slices < kSumThreads / 8 && total * m.slices < 148 * 2048 && static_cast<int64_t>(m.sum_batches) * m.sum_heads > 8 * m.slices) m.slices *= 2;
+  const int per_block = kSumThreads / m.slices;
+  const int64_t blocks = (total + per_block - 1) / per_block;
   if (blocks > 0x7fffffff) {
     set_error("sum_bias_grad: too many elements");
     return SDPA_B200_INVALID_ARG;
   }
   auto kernel = dtype == SDPA_B200_F16 ? bias_grad_sum_kernel<true> : bias_grad_sum_kernel<false>;
-  kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(m, total);
+  kernel<<<static_cast<unsigned>(blocks), kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(m, total);
   const cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     set_error("sum_bias_grad: launch failed: %s", cudaGetErrorString(err));
