@@ -418,3 +418,35 @@ def test_both_kernels_in_one_launch(cuda_device, native_lib, B, Hq, Hkv, L, D, c
     want = torch.autograd.grad(torch.softmax(s, -1) @ vf.repeat_interleave(Hq // Hkv, 1), (qf, kf, vf), do.float())
     for name, got, w in zip(("dq", "dk", "dv"), grads, want):
         assert float((got.float() - w).norm() / w.norm()) < 4e-3, name
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,D,causal", [
+    ([1100, 0, 3, 40], 2, 1, 128, True),                 # fewer blocks than the SMs hold: one for every row
+    ([3000, 20, 1], 16, 4, 96, True),                    # as many as they hold
+    ([1500] + [7] * 30, 8, 8, 128, False),               # a third of the longest one's, three rounds
+    ([700, 600, 500, 400, 300, 200, 100, 65, 0], 32, 8, 64, True),  # the mean's, with the fused kernel's accumulator
+])
+def test_packed_prepass_blocks_that_go_on(cuda_device, native_lib, lens, Hq, Hkv, D, causal):
+    """Gradients of packed sequences of very different lengths, whose pre-pass has fewer blocks than rows, against fp32 math (relative error in the 2-norm as on the
+    other paths)."""
+    gen = torch.Generator(device=cuda_device).manual_seed(21)
+    q, k, v, do = (torch.randn(sum(lens), h, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    ends = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    cu = torch.tensor(ends, dtype=torch.int32, device=cuda_device)
+    out, lse = ops._flash_attention_forward(q, k, v, cu, cu, max(lens), max(lens), 0.0, causal, False)[:2]
+    none = torch.empty(0, dtype=torch.int64)
+    got = ops._flash_attention_backward(do, q, k, v, out, lse, cu, cu, max(lens), max(lens), 0.0, causal, none, none)
+    assert ops.device_status() == 0
+    want = [torch.zeros_like(t, dtype=torch.float32) for t in (q, k, v)]
+    for lo, hi in zip(ends, ends[1:]):
+        if hi == lo:
+            continue
+        f = [t[lo:hi].float().transpose(0, 1).detach().requires_grad_() for t in (q, k, v)]
+        s = f[0] @ f[1].repeat_interleave(Hq // Hkv, 0).transpose(1, 2) * D ** -0.5
+        if causal:
+            s = s.masked_fill(~torch.ones_like(s[0], dtype=torch.bool).tril(), float("-inf"))
+        ref = torch.softmax(s, -1) @ f[2].repeat_interleave(Hq // Hkv, 0)
+        for w, g in zip(want, torch.autograd.grad(ref, f, do[lo:hi].float().transpose(0, 1))):
+            w[lo:hi] = g.transpose(0, 1)
+    for name, g, w in zip(("dq", "dk", "dv"), got, want):
+        assert float((g.float() - w).norm() / w.norm()) < 4e-3, name

@@ -32,6 +32,7 @@
 #include <cstdlib>
 #endif
 
+#include <algorithm>
 #include <type_traits>
 #include <utility>
 
@@ -1049,8 +1050,11 @@ struct PreParams {
 template <int kD>
 constexpr int kPreRows = 2 * 256 * 8 / kD;  // 64 or 32
 constexpr int kMaxGridY = 65535;
+// Blocks per SM: 32 registers dense, 40 packed. (Packed without the limit, above head_dim 64, 47 registers and five blocks: 12 sequences of 64 to 2048 tokens, 16 heads 20.6 us, so 18.5.)
+template <bool kPacked>
+constexpr int kPreBlocks = kPacked ? 6 : 8;
 template <int kD, bool kF16, bool kPacked>
-__global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) {
+__global__ void __launch_bounds__(256, kPreBlocks<kPacked>) bwd_preprocess_kernel(const PreParams p) {
   if (kPacked && static_cast<int>(blockIdx.x) == p.heads_q) {
     clear_uncovered_rows(p.grads, p.heads_q);
     return;
@@ -1071,8 +1075,9 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
   if (kPacked && p.ds_seq_base != nullptr && h == 0 && blockIdx.y == 0 && p.block0 == 0) {
     write_seq_base(p.ds_seq_base, p.cu_q, p.cu_k, b, p.is_causal != 0);
   }
-  // Packed: as many blocks per sequence as one of the mean length has, which go on where there are more rows, up to the last row that a tile of the kernels
-  // behind has; with blocks for the longest one in all of them half were empty (12 sequences of 64 to 2048 tokens, 16 heads, D128 25.0 us, so 18.5; 20 of 100 to 3000, D64 with the accumulator 44.7, 39.1).
+  // Packed: as many blocks per sequence as one of the mean length has (launch_bwd), which go on where there are more rows, up to the last row that a tile of the kernels
+  // behind has; with blocks for the longest one in all of them half were empty (12 sequences of 64 to 2048 tokens, 16 heads, D128 25.3 us, so 18.5; 20 of 100 to 3000, D64 with the
+  // accumulator 47.7, 46.1; one of 4096 among 7 of 16, D64 16.3, 7.9).
   const int rows = kPacked ? min((len_q + kTile - 1) / kTile * kTile, p.lq_pad) : p.lq_pad;
   for (int row0 = (p.block0 + blockIdx.y) * kRows; row0 < rows; row0 += gridDim.y * kRows) {
     uint4 ov[2], dv[2];
@@ -1393,10 +1398,13 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   auto pre_kernel = p.head_dim <= 64 ? pick_pre(std::integral_constant<int, 64>{}) : pick_pre(std::integral_constant<int, 128>{});
   const int pre_rows = p.head_dim <= 64 ? kPreRows<64> : kPreRows<128>;
   int pre_blocks = lq_pad / pre_rows;
-  if (varlen) {  // the mean length's, but a third of the longest one's, since a block that goes on pays one memory latency each time
-    const int mean = p.total_q / p.batch / pre_rows + 1, third = (pre_blocks + 2) / 3, enough = mean > third ? mean : third;
-    pre_blocks = enough < pre_blocks ? enough : pre_blocks;
-    pre_blocks = pre_blocks < kMaxGridY ? pre_blocks : kMaxGridY;
+  if (varlen) {
+    // The mean length's, but a third of the longest one's, since a block that goes on pays one memory latency each time, and no fewer than the SMs hold at once: below
+    // that a latency is all there is (all rows' blocks at once | by the mean and the third | so, us: 4 of 64 to 2048, 2 heads, D128 3.5 | 4.4 | 3.5, 1024 + 64, one head 2.7 | 3.3 | 2.9,
+    // 3000 + 100, 8 heads, D64 3.4 | 3.9 | 3.3, one of 2048 among 3 of 16, 8 heads, D128 6.1 | 5.7 | 5.4).
+    const int64_t mean = p.total_q / p.batch / pre_rows + 1, third = (pre_blocks + 2) / 3;
+    const int64_t held = kPreBlocks<true> * kSms / (static_cast<int64_t>(p.heads_q) * p.batch);
+    pre_blocks = static_cast<int>(std::min<int64_t>({std::max({mean, third, held}), pre_blocks, kMaxGridY}));
   }
   for (pre.block0 = 0; pre.block0 < pre_blocks; pre.block0 += kMaxGridY) {  // one launch up to 2 M rows
     const int rest = pre_blocks - pre.block0;
