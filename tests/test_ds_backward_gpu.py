@@ -231,8 +231,8 @@ def test_the_backward_leaves_l2_to_the_kernels_behind_it(cuda_device, native_lib
             adds = sorted((e for e in prof.events() if "CUDAFunctor" in e.name and "add" in e.name.lower()), key=lambda e: e.time_range.start)
             if i >= 3:
                 times += [e.device_time for e in adds[2:]]
-        assert len(times) == 49
-        return sorted(times)[24]
+        assert len(times) >= 35  # the profiler may lose some
+        return sorted(times)[len(times) // 2]
 
     backward = behind(lambda: ops._dense_backward(do, q, k, v, out, lse, True, 128 ** -0.5))
     fill = behind(lambda: big.fill_(1))

