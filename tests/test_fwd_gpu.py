@@ -326,3 +326,60 @@ def test_units_taken_from_waiting_ctas_on_two_streams(cuda_device, native_lib):
     for w, results in zip(want, got):
         for out, lse in results:
             assert torch.equal(out, w[0]) and torch.equal(lse, w[1])
+
+
+@pytest.mark.parametrize("kind", ["plain", "causal", "bias", "dropout", "bias_dropout"])
+@pytest.mark.parametrize("B,counter", [(100, False), (111, True)])  # 64 heads on 148 SMs: fewer than 48 rounds of units, and 48
+@pytest.mark.parametrize("D", [64, 128])
+def test_long_lists_of_units(cuda_device, native_lib, B, counter, D, kind):
+    """Lists on either side of the line above which units come off the counter, in every instance, against fp32 math. 16-bit P: relative error of 4e-3 in the
+    2-norm as on the other paths."""
+    from torch.profiler import ProfilerActivity, profile
+    from torch_mlu_b200 import dropout
+    H, L = 64, 40
+    gen = torch.Generator(device=cuda_device).manual_seed(5)
+    q, k, v = (torch.randn(B, H, L, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for _ in range(3))
+    bias = torch.randn(B, 1, 1, L, generator=gen, device=cuda_device, dtype=torch.bfloat16).expand(B, H, L, L) if "bias" in kind else None
+    keep = dropout.KeepMasks(3, 1, 0.2, B, H, L, L, cuda_device) if "dropout" in kind else None
+    causal = kind == "causal"
+    call = lambda: ops._dense_forward(q, k, v, causal, None, False, _cabi.KERNEL_PREFILL, 0, keep, bias)
+    call()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        out, lse = call()
+        torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert any("Memset" in e.name for e in prof.events()) == counter
+    s = q.float() @ k.float().transpose(2, 3) * D ** -0.5 + (0 if bias is None else bias.float())
+    if causal:
+        s = s.masked_fill(~torch.ones(L, L, dtype=torch.bool, device=cuda_device).tril(), float("-inf"))
+    p = torch.softmax(s, -1)
+    if keep is not None:
+        p = p.masked_fill(~keep.dense(), 0.0) / 0.8
+    want = p @ v.float()
+    assert float((out.float() - want).norm() / want.norm()) < 4e-3
+    assert float((lse - s.logsumexp(-1)).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("B,counter", [(30, False), (40, True)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_long_packed_lists_with_empty_slots(cuda_device, native_lib, B, counter, D, causal):
+    """One sequence of three units per head among short and empty ones: two in three slots of a list on either side of that line hold no unit. Against each
+    sequence's own call."""
+    from torch.profiler import ProfilerActivity, profile
+    lens = [700] + [(0, 5, 33, 1)[i % 4] for i in range(B - 1)]
+    gen = torch.Generator(device=cuda_device).manual_seed(8)
+    q, k, v = (torch.randn(sum(lens), h, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for h in (64, 16, 16))
+    ends = [sum(lens[:i]) for i in range(B + 1)]
+    cu = torch.tensor(ends, dtype=torch.int32, device=cuda_device)
+    call = lambda: ops._flash_attention_forward(q, k, v, cu, cu, 700, 700, 0.0, causal, False)[:2]
+    call()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        out, lse = call()
+        torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert any("Memset" in e.name for e in prof.events()) == counter
+    for lo, hi in zip(ends, ends[1:]):
+        if hi > lo:
+            o, l = ops.gqa_prefill(*(t[lo:hi].transpose(0, 1).unsqueeze(0) for t in (q, k, v)), is_causal=causal)
+            assert torch.equal(out[lo:hi], o[0].transpose(0, 1)) and torch.equal(lse[..., lo:hi].reshape(64, -1), l[0])

@@ -155,3 +155,53 @@ def test_chains_of_calls_that_feed_one_another(cuda_device, native_lib, chain):
         assert ops.device_status() == 0
         for i, (a, b) in enumerate(zip(got, want)):
             assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("B,H,D,L,causal", [(4, 26, 128, 768, True), (5, 32, 64, 256, False)])
+def test_units_by_the_counter_replay_in_a_cuda_graph(cuda_device, native_lib, B, H, D, L, causal):
+    """A call that leaves an SM free takes its units off the counter, whose clearing is a graph node too: two replays on new inputs, against the bits of the call
+    that takes them from waiting CTAs or has none to leave."""
+    dev = cuda_device
+    gen = torch.Generator(device=dev).manual_seed(43)
+    make = lambda: torch.randn(B, H, L, D, generator=gen, device=dev, dtype=torch.bfloat16)
+    q, k, v = make(), make(), make()
+    call = lambda margin: ops.gqa_prefill(q, k, v, is_causal=causal, sm_margin=margin)
+    side = torch.cuda.Stream(dev)
+    side.wait_stream(torch.cuda.current_stream(dev))
+    with torch.cuda.stream(side):
+        call(1)
+    torch.cuda.current_stream(dev).wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out, lse = call(1)
+    for _ in range(2):
+        for t in (q, k, v):
+            t.copy_(make())
+        graph.replay()
+        torch.cuda.synchronize()
+        want = call(0)
+        assert ops.device_status() == 0
+        assert torch.equal(out, want[0]) and torch.equal(lse, want[1])
+
+
+def test_chain_of_calls_by_the_counter(cuda_device, native_lib):
+    """The counter's clearing stands between calls of which each one's output is the next one's query: the bits are those of the same calls with the device waited for."""
+    gen = torch.Generator(device=cuda_device).manual_seed(7)
+    x0, k, v = (torch.randn(2, 80, 300, 128, generator=gen, device=cuda_device, dtype=torch.bfloat16) for _ in range(3))
+
+    def run(wait, margin):
+        x, outs = x0, []
+        for _ in range(12):
+            x = ops.gqa_prefill(x, k, v, is_causal=True, sm_margin=margin)[0]
+            wait()
+            outs.append(x)
+        return outs
+
+    want = run(torch.cuda.synchronize, 0)
+    for _ in range(3):
+        got = run(lambda: None, 1)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert torch.equal(a, b), i
