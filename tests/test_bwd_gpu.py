@@ -450,3 +450,55 @@ def test_packed_prepass_blocks_that_go_on(cuda_device, native_lib, lens, Hq, Hkv
             w[lo:hi] = g.transpose(0, 1)
     for name, g, w in zip(("dq", "dk", "dv"), got, want):
         assert float((g.float() - w).norm() / w.norm()) < 4e-3, name
+
+
+@pytest.mark.parametrize("dtype,bound", [(torch.bfloat16, 4e-3), (torch.float16, 1e-3)])
+@pytest.mark.parametrize("Hq,Hkv,L,D,causal,launches", [
+    (16, 16, 640, 128, True, 2),
+    (18, 6, 900, 96, False, 2),
+    (12, 4, 900, 96, False, 3),  # all blocks of both kernels fit the SMs
+])
+def test_both_kernels_in_one_launch_with_dropout(cuda_device, native_lib, Hq, Hkv, L, D, causal, launches, dtype, bound):
+    """Above head_dim 64, up to 148 key blocks and more blocks than SMs: the pre-pass and one launch, against fp32 math with the same pattern."""
+    from torch_mlu_b200 import dropout
+    gen = torch.Generator(device=cuda_device).manual_seed(10)
+    q, k, v, do = (torch.randn(1, h, L, D, generator=gen, device=cuda_device, dtype=dtype) for h in (Hq, Hkv, Hkv, Hq))
+    keep = dropout.KeepMasks(11, 2, 0.15, 1, Hq, L, L, cuda_device)
+    out, lse = ops._dense_forward(q, k, v, causal, None, True, keep=keep)
+    before = _cabi.launch_count()
+    grads = ops._dense_backward(do, q, k, v, out, lse, causal, D ** -0.5, keep=keep)
+    assert ops.device_status() == 0 and _cabi.launch_count() - before == launches
+    f = [t.float().requires_grad_() for t in (q, k, v)]
+    s = f[0] @ f[1].repeat_interleave(Hq // Hkv, 1).transpose(2, 3) * D ** -0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(L, L, dtype=torch.bool, device=cuda_device).tril(), float("-inf"))
+    p = torch.softmax(s, -1).masked_fill(~keep.dense(), 0.0) / 0.85
+    want = torch.autograd.grad(p @ f[2].repeat_interleave(Hq // Hkv, 1), f, do.float())
+    for name, got, w in zip(("dq", "dk", "dv"), grads, want):
+        assert float((got.float() - w).norm() / w.norm()) < bound, name
+
+
+@pytest.mark.parametrize("D", [128, 72])
+@pytest.mark.parametrize("causal", [True, False])
+def test_both_kernels_in_one_launch_packed(cuda_device, native_lib, D, causal):
+    """The same for packed sequences, some without tokens, against each sequence's own backward."""
+    lens, Hq, Hkv = [640, 0, 65, 3], 8, 4
+    gen = torch.Generator(device=cuda_device).manual_seed(12)
+    q, k, v, do = (torch.randn(sum(lens), h, D, generator=gen, device=cuda_device, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    ends = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    cu = torch.tensor(ends, dtype=torch.int32, device=cuda_device)
+    none = torch.empty(0, dtype=torch.int64)
+    out, lse = ops._flash_attention_forward(q, k, v, cu, cu, 640, 640, 0.0, causal, False)[:2]
+    before = _cabi.launch_count()
+    got = ops._flash_attention_backward(do, q, k, v, out, lse, cu, cu, 640, 640, 0.0, causal, none, none)
+    assert ops.device_status() == 0 and _cabi.launch_count() - before == 2
+    for lo, hi in zip(ends, ends[1:]):
+        if hi == lo:
+            continue
+        f = [t[lo:hi].float().transpose(0, 1).detach().requires_grad_() for t in (q, k, v)]
+        s = f[0] @ f[1].repeat_interleave(Hq // Hkv, 0).transpose(1, 2) * D ** -0.5
+        if causal:
+            s = s.masked_fill(~torch.ones_like(s[0], dtype=torch.bool).tril(), float("-inf"))
+        ref = torch.softmax(s, -1) @ f[2].repeat_interleave(Hq // Hkv, 0)
+        for name, g, w in zip(("dq", "dk", "dv"), got, torch.autograd.grad(ref, f, do[lo:hi].float().transpose(0, 1))):
+            assert float((g[lo:hi].float().transpose(0, 1) - w).norm() / w.norm()) < 4e-3, (name, lo)
