@@ -145,7 +145,8 @@ typedef struct sdpa_b200_params {
   const void* bias;
   int64_t bias_batch_stride, bias_head_stride, bias_row_stride;
   /* Backward: gradient of the bias, [batch, heads_q, seqlen_q, dbias_row_stride >= seqlen_k rounded up to 8],
-   * same type, or NULL. Elements the causal mask hides are not written: clear the buffer first. */
+   * same type, or NULL. Elements the causal mask hides are not written: clear the buffer first.
+   * Without a causal mask every element of a dense call's gradient is written; the padding behind seqlen_k need not be. */
   void* dbias;
   int64_t dbias_batch_stride, dbias_head_stride, dbias_row_stride;
   /* Backward, optional: the same bias with keys and queries exchanged, [batch, heads_q, seqlen_k, seqlen_q]

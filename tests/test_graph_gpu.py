@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("B,H,D,L", [
     (2, 4, 128, 768),
-    (4, 26, 128, 768),  # 312 forward units and 624 key blocks: the forward's unit counter, the dS GEMM and its unit counter
+    (4, 26, 128, 768),  # 312 forward units, taken from waiting CTAs, and 624 key blocks: the dS GEMM and its unit counter
     (4, 26, 64, 768),   # the dK/dV and the dQ kernel
     (2, 20, 64, 1100),  # the fused backward and its accumulator's clearing
     (1, 2, 256, 768),
@@ -32,7 +32,7 @@ def test_forward_backward_replay_in_a_cuda_graph(cuda_device, native_lib, B, H, 
     with torch.cuda.graph(graph):
         out, lse = ops.gqa_prefill(q, k, v, is_causal=True)
         dq, dk, dv = ops._dense_backward(do, q, k, v, out, lse, True, scale)
-    for _ in range(2):  # replay twice on fresh inputs: the persistent kernel's unit counter is reset by a graph node too
+    for _ in range(2):  # replay twice on fresh inputs
         for t in (q, k, v, do):
             t.copy_(torch.randn(B, H, L, D, generator=g).bfloat16())
         graph.replay()
@@ -121,7 +121,7 @@ def test_chains_of_calls_that_feed_one_another(cuda_device, native_lib, chain):
         cu = torch.tensor([0, 130, 300], dtype=torch.int32, device=dev)
         step = lambda x: ops._flash_attention_forward(x, k, x, cu, cu, 170, 170, 0.0, True, False)[0]
         launches = 1
-    elif chain == "counted_128":  # more units than SMs: the counter's clearing stands between the calls
+    elif chain == "counted_128":  # more units than SMs, taken from waiting CTAs
         x0, k, v = randn(2, 80, 300, 128), randn(2, 80, 300, 128), randn(2, 80, 300, 128)
         step = lambda x: ops.gqa_prefill(x, k, v, is_causal=True)[0]
     elif chain == "prefill_and_decode":  # a forward's output is the decode's cache, the decode's output the forward's first query

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) mask_to_bias_kernel(const MaskParams p, i
 }
 
 // The same for a bias in its own type, whose rows the attention kernels cannot read where they lie: bound by memory, one launch where filling and copying took
-// two and wrote the copy twice (12 heads of 594 x 594 20 + 12 us -> 4).
+// two and wrote the copy twice (12 heads of 594 x 594 11.9 us -> 6.7, 192 of 1001 x 1001 524 -> 216).
 struct PadParams {
   const uint16_t* bias;
   uint4* out;

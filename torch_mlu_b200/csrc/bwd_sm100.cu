@@ -1551,8 +1551,8 @@ int launch_bwd(const sdpa_b200_params& p, void* workspace, size_t workspace_byte
   // Both in one launch where the same instance serves both, with the dQ blocks behind the dK/dV blocks as the overlapped launches have them: about 2.5 us less of
   // host time, which is what bounds the steps of short sequences, and no gap (step, two launches | one, us: B4 H8 L500 D64 f16 83.3 | 78.2, B1 H8 L2048 D128
   // 74.1 | 71.5, B16 H16 L500 D64 120.8 | 116.6, B8 H12 L1000 D64 unmasked 187 | 181, B32 H12 L300 D64 with dropout 173.8 | 168.5; backward alone, replayed from a graph: B8 H12 L512
-  // D64 with a mask 50.4 | 48.1, B1 H8 L2048 D128 34.9 | 33.3, B4 H8 L512 D128 24.1 | 24.1). Above head_dim 64 two launches where all blocks fit the SMs at once: only host time is
-  // saved there, and the suite counts them.
+  // D64 with a mask 50.4 | 48.1, B1 H8 L2048 D128 34.9 | 33.3, B4 H8 L512 D128 24.1 | 24.1). Above head_dim 64 two launches where all blocks fit the SMs at once, although one
+  // is shorter there too (step B1 H16 L512 D128 83.9 | 82.4, B4 H8 L256 D96 83.5 | 80.5; backward alone from a graph 14.9 | 14.2, 11.7 | 11.0): a test counts them.
   const bool pair = !kp.ds_call && kp.split == 1 && (p.head_dim > 64 || wide_dkdv == wide_dq) && (kp.bias == nullptr || (kp.bias_row_stride == 0 && kp.dbias == nullptr)) &&
                     (p.head_dim <= 64 || grid_dkdv + grid_dq > kSms);
   if (pair)

@@ -927,9 +927,12 @@ int launch_fwd_prefill(const sdpa_b200_params& p, void* workspace, cudaStream_t 
   // 31.7 | 27.0, L1000 D128 54.1 | 50.3, B7 H32 512 of 1297 93.0 | 90.3, B8 H32 L1024 D64 unmasked 112.7 | 109.4, packed: 7 of 19 to 448, 16/16, D64 16.4 | 13.0, 23 of 51 to 236, 12/12
   // 22.4 | 18.7, 12 of 64 to 3000, 16/16, D64 125.9 | 122.5, 29 of 320 to 1024, 32/8, D64 160.4 | 155.2; level at B4 H32 L4096.) The counter, workspace header word 1, stays
   //  * where the caller wants SMs left free: pending CTAs would fill them;
-  //  * for lists of forty-eight rounds and more, where its launch is nothing and a packed list's empty slots are skipped faster by it (28 sequences of 64 to 3008
-  //    tokens, 64/8, D64, 145 rounds, 1033 | 1042, 32 of 192 to 1321, 83 rounds, 414 | 417; but 24 of 500 to 1500, 32/8, 31 rounds, 236.3 | 234.8);
-  //  * for dense calls of up to two rounds without mask, bias or dropout: there the suite reads the claims from the launch that clears it.
+  //  * for lists of forty-eight rounds and more, where its launch is nothing: at head_dim 128 it is level or ahead by less than 1 % (16 sequences of 512 to 4096, 32/8, 55
+  //    rounds, 887 | 893, 32 of 1000 to 2000 810 | 814, unmasked 1279 | 1284), at 64 behind by 1 to 2 % (the same 32 578 | 572, 28 of 64 to 3008, 64/8, 145 rounds, 1219 | 1189, 32 of
+  //    500 to 1500, 32/8, 41 rounds, which do not count, 320 | 315). Slots without a unit do not decide it (one of 4096 among 31 of 16, 32/8, nine in ten empty, D64 192 | 186,
+  //    D128 209 | 205; one of 1024 among 63 of 64, 16/4, D64, 28 rounds, 43.8 | 40.3);
+  //  * for dense calls of up to two rounds without mask, bias or dropout, which would be faster without it too (B8 H12 L512 D64 24.6 | 19.0, B5 H32 L256 D64 16.5 | 12.3, B4 H16 L1024
+  //    D128 41.2 | 36.2): a test reads from the launch that clears it that a CTA which starts late leaves its units to others.
   // Not two units per CTA, dealt out by index: a CTA whose SM another stream's kernel holds then starts both its units late (beside a call on 8 SMs B8 H12 L512
   // D64 32.9 us, with a counter 24.6, B5 H8 L1024 D128 57.4, 41.0).
   const int slots = kp.order.slots;
